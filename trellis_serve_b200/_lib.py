@@ -9,11 +9,13 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libexl3_b200.so")
+TORCH_LIB_PATH = os.path.join(_HERE, "libexl3_b200_torch.so")
 
 F16, BF16, F32 = 0, 1, 2
 CB_3INST, CB_MCG, CB_MUL1 = 0, 1, 2
 
 _lib = None
+_native = None
 _initialised: set[int] = set()
 
 _vp, _i, _sz, _i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_int64
@@ -50,6 +52,7 @@ SIGNATURES = {
     "exl3_decode_attention": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp, ctypes.c_float, _vp, _sz, _vp, _vp, _i, _vp, _sz, _vp]),
     "exl3_rope_decode_attention": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, ctypes.c_float, _vp, _sz, _vp, _vp, _i, _vp, _sz,
                                         _vp]),
+    "exl3_prefers_decode": (_i, [_i, _i, _i, _i]),
     "exl3_gemm_tc_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "exl3_linear_tc": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_linear_static": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp]),
@@ -100,6 +103,20 @@ def load() -> ctypes.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+def native():
+    """torch.ops.exl3_b200: the operators of libexl3_b200_torch.so over the C ABI; raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        if not os.path.exists(TORCH_LIB_PATH):
+            raise ImportError(f"{TORCH_LIB_PATH} is missing: build it with `python -m trellis_serve_b200.csrc.build`; there is "
+                              f"no fallback implementation")
+        import torch
+        torch.ops.load_library(TORCH_LIB_PATH)
+        _native = torch.ops.exl3_b200
+    return _native
 
 
 def check(status: int, where: str) -> None:

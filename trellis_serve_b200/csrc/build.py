@@ -3,7 +3,8 @@
     python -m trellis_serve_b200.csrc.build [--force] [--verbose]
 
 One object per source; the decode GEMV is compiled once per bit rate (-DEXL3_GEMV_K=2..8) so the seven
-instantiation sets build in parallel.  Output: trellis_serve_b200/libexl3_b200.so.
+instantiation sets build in parallel.  Output: trellis_serve_b200/libexl3_b200.so, and libexl3_b200_torch.so beside it (the
+torch operators over the C ABI, host code only).
 """
 from __future__ import annotations
 
@@ -17,6 +18,7 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 OUT = os.environ.get("EXL3_B200_BUILD_OUT") or os.path.join(PKG, "libexl3_b200.so")
+TORCH_OUT = os.path.join(os.path.dirname(OUT), "libexl3_b200_torch.so")
 OBJ = os.environ.get("EXL3_B200_BUILD_OBJ") or os.path.join(HERE, "build")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -43,13 +45,30 @@ def _jobs():
 
 
 def _sources_mtime() -> float:
-    files = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".cu", ".cuh", ".h"))]
+    files = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".cu", ".cuh", ".h", ".cpp"))]
     files.append(os.path.join(os.path.dirname(PKG), "include", "exl3_b200.h"))
     return max(os.path.getmtime(f) for f in files)
 
 
+def build_torch() -> str:
+    """libexl3_b200_torch.so: csrc/exl3_torch.cpp against the installed torch and the C-ABI library beside it."""
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(nvcc())), "include")
+    includes = [f"-I{p}" for p in dict.fromkeys([*include_paths(), cuda])]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *includes,
+           os.path.join(HERE, "exl3_torch.cpp"), "-o", TORCH_OUT, f"-L{os.path.dirname(OUT)}", f"-l:{os.path.basename(OUT)}", f"-L{lib}",
+           "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("building libexl3_b200_torch.so failed")
+    return TORCH_OUT
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and os.path.exists(OUT) and os.path.getmtime(OUT) >= _sources_mtime():
+    if not force and all(os.path.exists(f) and os.path.getmtime(f) >= _sources_mtime() for f in (OUT, TORCH_OUT)):
         return OUT
     os.makedirs(OBJ, exist_ok=True)
     exe = nvcc()
@@ -78,6 +97,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("linking libexl3_b200.so failed")
+    build_torch()
     return OUT
 
 

@@ -610,6 +610,35 @@ exl3_status exl3_rope_decode_attention(const void* qkv, int dtype, int rows, int
 
 static size_t tc_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// Fitted to measurements on B200 (microseconds).  The decode kernel streams the weights once per 16 rows: ~14 + 0.38 per million
+// weights for a full chunk, ~0.8 of that for a last chunk of up to 8 rows.  The tensor-core kernel works through its tiles in
+// waves over the SMs at ~1.1 per 64-deep reduction block (~1.6 for the 512-row tiles used above 256 rows); when the tiles are
+// fewer than the SMs the reduction of each is cut into up to 8 parts on CTAs of their own; ~12 more for the two rotation
+// launches, ~8 for adding the parts.
+int exl3_prefers_decode(int rows, int k, int n_total, int sms)
+{
+    const double chunk = 14.0 + 0.38 * ((double)k * n_total / 1e6);
+    const int rem = rows % 16;
+    const double decode = rows / 16 * chunk + (rem == 0 ? 0.0 : chunk * (rem <= 8 ? 0.8 : 1.0));
+    long long tiles;
+    double per_block;
+    if (rows <= 256) {
+        tiles = (long long)((rows + 255) / 256) * (n_total / 256 > 1 ? n_total / 256 : 1);
+        per_block = 1.1;
+    } else {
+        tiles = (long long)((rows + 511) / 512) * (n_total / 128);
+        per_block = 1.6;
+    }
+    const long long one = tiles > 1 ? tiles : 1;
+    long long parts = sms / one;
+    if (parts > 8) parts = 8;
+    if (parts > k / 64) parts = k / 64;
+    if (parts < 1) parts = 1;
+    const long long waves = sms > 0 ? (tiles + sms - 1) / sms : tiles;
+    const double tensor = (double)waves * (k / 64.0) / (double)parts * per_block + 12.0 + (parts > 1 ? 8.0 : 0.0) + 0.08 * (rows < 256 ? rows : 256);
+    return decode <= tensor;
+}
+
 size_t exl3_gemm_tc_workspace_bytes(int rows, int k, int n_total, int n_shards)
 {
     if (rows < 0 || k < 0 || n_total < 0 || n_shards < 1) return 0;

@@ -23,8 +23,28 @@ from .. import _lib
 from .base import BackendStatus
 
 MAX_ROWS = 64            # rows the per-device workspace is sized for at load time (marlin.py:24-27)
-_workspace: dict[int, torch.Tensor] = {}
-_tc_workspace: dict[int, torch.Tensor] = {}
+
+
+class _Scratch:
+    """Zero-filled scratch per device that calls without a workspace of their own share; it lives in the native operators, which
+    use the same one (kind 0: decode kernels, 1: many-row kernels)."""
+
+    def __init__(self, kind: int):
+        self.kind = kind
+
+    def reserve(self, device: int, nbytes: int) -> torch.Tensor:
+        return _lib.native().scratch(self.kind, device, nbytes)
+
+    def get(self, device: int) -> torch.Tensor | None:
+        t = _lib.native().scratch(self.kind, device, 0)
+        return t if t.numel() else None
+
+    def clear(self) -> None:
+        _lib.native().scratch_clear(self.kind)
+
+
+_workspace = _Scratch(0)
+_tc_workspace = _Scratch(1)
 
 
 def _dtype_code(t: torch.Tensor, allow_f32: bool = False) -> int:
@@ -62,11 +82,7 @@ def workspace_bytes(rows: int, k: int, n_total: int, shards: int) -> int:
 def reserve_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """Zero-filled, reused per-device scratch (activation fragments, split-k partial sums, counters).  Sized at load
     time so the run path never allocates and CUDA graphs see a fixed address."""
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    cur = _workspace.get(idx)
-    if cur is None or cur.numel() < nbytes:
-        cur = _workspace[idx] = torch.zeros(nbytes, dtype=torch.uint8, device=torch.device("cuda", idx))
-    return cur
+    return _workspace.reserve(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
 
 def probe() -> BackendStatus:
@@ -102,20 +118,22 @@ def supports_matrix(trellis: torch.Tensor) -> tuple[bool, str]:
     return True, ""
 
 
-def prepare_matrix(trellis: torch.Tensor) -> torch.Tensor:
-    """int16 (k/16, n/16, 16K) -> resident int32 (n/128, k/128, 8, 2, K, 32): the same bits, lane-major."""
+def _check_matrix(trellis: torch.Tensor) -> None:
     _require_cuda(trellis, "trellis")
     ok, why = supports_matrix(trellis)
     if not ok:
         raise RuntimeError(f"cannot prepare this matrix: {why}")
-    lib = _lib.load()
+
+
+def prepare_matrix(trellis: torch.Tensor) -> torch.Tensor:
+    """int16 (k/16, n/16, 16K) -> resident int32 (n/128, k/128, 8, 2, K, 32): the same bits, lane-major."""
+    _check_matrix(trellis)
     _lib.init_device(trellis.device.index)
     t = trellis.contiguous()
     kt, nt, words = t.shape
-    K = words // 16
-    packed = torch.empty((nt // 8, kt // 8, 8, 2, K, 32), dtype=torch.int32, device=t.device)
+    packed = torch.empty((nt // 8, kt // 8, 8, 2, words // 16, 32), dtype=torch.int32, device=t.device)
     with torch.cuda.device(t.device):
-        _lib.check(lib.exl3_repack(_ptr(t), kt * 16, nt * 16, K, _ptr(packed), _stream(t.device)), "exl3_repack")
+        _lib.check(_lib.load().exl3_repack(_ptr(t), kt * 16, nt * 16, words // 16, _ptr(packed), _stream(t.device)), "exl3_repack")
     return packed
 
 
@@ -132,18 +150,17 @@ def unprepare_matrix(packed: torch.Tensor) -> torch.Tensor:
 
 def prepare(trellis: list[torch.Tensor], suh: list[torch.Tensor], svh: list[torch.Tensor]):
     """-> (packed int32 [n_total/128, k/128, 8, 2, K, 32], suh_cat [shards, k], svh_cat [n_total], shard_ends)."""
-    b = torch.cat([prepare_matrix(t) for t in trellis], dim=0).contiguous()
+    for t in trellis:
+        _check_matrix(t)
+        if t.shape[0] != trellis[0].shape[0] or t.shape[2] != trellis[0].shape[2]:
+            raise RuntimeError("the matrices of a fused group share input width and bitrate")
     ends, total = [], 0
     for t in trellis[:-1]:
         total += t.shape[1] * 16
         ends.append(total)
-    k = trellis[0].shape[0] * 16
-    n_total = sum(t.shape[1] * 16 for t in trellis)
-    reserve_workspace(b.device, workspace_bytes(MAX_ROWS, k, n_total, len(trellis)))
-    suh_cat, svh_cat = torch.stack(suh).contiguous(), torch.cat(svh).contiguous()
-    # The run path starts fetching the resident weights and sign vectors while the kernel ahead of it is still running
-    # (programmatic dependent launch), so they must be complete before the first `run` is enqueued: load time pays for that.
-    torch.cuda.current_stream(b.device).synchronize()
+    # Repacked into the group's column blocks and complete on return: the run path starts fetching the resident weights and sign
+    # vectors while the kernel ahead of it is still running (programmatic dependent launch).
+    b, suh_cat, svh_cat = _lib.native().prepare_group(trellis, suh, svh, MAX_ROWS)
     return b, suh_cat, svh_cat, ends
 
 
@@ -152,18 +169,14 @@ def _geometry(packed: torch.Tensor) -> tuple[int, int, int]:
     return kg * 128, nb * 128, K
 
 
-def _own_or_given(workspace: torch.Tensor | None, device: torch.device, need: int, table: dict) -> torch.Tensor:
+def _own_or_given(workspace: torch.Tensor | None, device: torch.device, need: int, table: _Scratch) -> torch.Tensor:
     """The caller's scratch when one is handed in (it must be large enough: nothing is allocated on its behalf), else the
     per-device one of this module, grown if needed."""
     if workspace is not None:
         if workspace.numel() * workspace.element_size() < need:
             raise RuntimeError(f"workspace holds {workspace.numel() * workspace.element_size()} bytes, this call needs {need}")
         return workspace
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    cur = table.get(idx)
-    if cur is None or cur.numel() < need:
-        cur = table[idx] = torch.zeros(need, dtype=torch.uint8, device=torch.device("cuda", idx))
-    return cur
+    return table.reserve(device.index if device.index is not None else torch.cuda.current_device(), need)
 
 
 def run(x: torch.Tensor, b: torch.Tensor, suh_cat: torch.Tensor, svh_cat: torch.Tensor, shard_ends: list[int],

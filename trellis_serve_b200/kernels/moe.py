@@ -21,7 +21,7 @@ import torch
 
 from .. import _lib
 from .base import BackendStatus
-from .linear import _dtype_code, _ptr, _require_cuda, _stream, prepare_matrix
+from .linear import _dtype_code, _ptr, _require_cuda, _stream, supports_matrix
 
 BLOCK_SIZES = (8, 128)
 # Average routed rows per expert from which a class goes through the grouped tensor-core GEMM (128-row blocks, every
@@ -50,12 +50,31 @@ def sorted_ids_capacity(tokens: int, top_k: int, num_experts: int, block: int = 
     return int(_lib.load().exl3_moe_sorted_capacity(tokens * top_k, num_experts))
 
 
-def stack_repacked(trellis: list[torch.Tensor]) -> torch.Tensor:
-    """E x int16 [k/16, n/16, 16K] -> int32 [E, n/128, k/128, 8, 2, K, 32]: a pure permutation of the stored words."""
+def _one_shape(trellis: list[torch.Tensor]) -> tuple[int, int, int]:
     shapes = {tuple(t.shape) for t in trellis}
     if len(shapes) != 1:
         raise ValueError(f"experts must share one shape and bitrate, got {sorted(shapes)}")
-    return torch.stack([prepare_matrix(t if t.is_cuda else t.cuda()) for t in trellis]).contiguous()
+    ok, why = supports_matrix(trellis[0])
+    if not ok:
+        raise RuntimeError(f"cannot prepare this matrix: {why}")
+    return shapes.pop()
+
+
+def stack_repacked(trellis: list[torch.Tensor], *more: list[torch.Tensor]) -> torch.Tensor:
+    """E x int16 [k/16, n/16, 16K] -> int32 [E, n/128, k/128, 8, 2, K, 32]: a pure permutation of the stored words.  `more`: further
+    projections of the same experts, side by side along n."""
+    projections = [trellis, *more]
+    shapes = [_one_shape(t) for t in projections]
+    if len({(kt, words) for kt, _, words in shapes}) != 1 or len({len(t) for t in projections}) != 1:
+        raise ValueError(f"projections must share input width, bitrate and experts, got {shapes}")
+    kt, _, words = shapes[0]
+    dev = trellis[0].device if trellis[0].is_cuda else torch.device("cuda", torch.cuda.current_device())
+    out = torch.empty((len(trellis), sum(nt for _, nt, _ in shapes) // 8, kt // 8, 8, 2, words // 16, 32), dtype=torch.int32, device=dev)
+    nb = 0
+    for t, (_, nt, _) in zip(projections, shapes):
+        _lib.native().repack_experts(t, out, nb)
+        nb += nt // 8
+    return out
 
 
 def bits_of_stack(stack: torch.Tensor) -> int:
@@ -100,7 +119,7 @@ def prepare(gate, up, down, codebook: int) -> ExpertPack:
     if dev.type != "cuda":
         dev = torch.device("cuda", torch.cuda.current_device())
     _lib.init_device(dev.index)
-    w13 = torch.cat([stack_repacked(gate[0]), stack_repacked(up[0])], dim=1).contiguous()
+    w13 = stack_repacked(gate[0], up[0])
     w2 = stack_repacked(down[0])
     suh13 = torch.stack([torch.stack(gate[1]), torch.stack(up[1])], dim=1).contiguous().to(dev)
     svh13 = torch.cat([torch.stack(gate[2]), torch.stack(up[2])], dim=1).contiguous().to(dev)

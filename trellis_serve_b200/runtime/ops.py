@@ -6,7 +6,8 @@ Same schema as the reference's custom op (ops.py:133):
     linear(Tensor x, Tensor[] trellis, Tensor[] suh, Tensor[] svh, Tensor[] dense, Tensor[] sliced, int sliced_min_rows,
            Tensor[] marlin_w, int[] marlin_ends, int[] codebooks, int[] out_widths) -> Tensor
 
-registered as `torch.ops.exl3_b200.linear`, with a fake (meta) implementation so tracing compilers see only shapes.
+registered as `torch.ops.exl3_b200.linear` (native: csrc/exl3_torch.cpp), with a fake (meta) implementation so tracing
+compilers see only shapes.
 `marlin_w` carries the output of `kernels.linear.prepare`: [packed, suh_cat, svh_cat]; `marlin_ends` its shard ends.
 `trellis`, `suh`, `svh` (the stored tensors) are optional here: the resident layout alone serves every path.
 `dense` may hold resident decoded fp16 weights per matrix; `sliced` is accepted for schema compatibility and unused.
@@ -26,38 +27,51 @@ any other dtype is computed in fp16 and cast back.
 from __future__ import annotations
 
 import os
+import sys
+import types
 
 import torch
 
-from .._lib import sm_count as lib_sm_count
+from .. import _lib as _native_lib
 from ..kernels import linear as lin
 
+_ops = _native_lib.native()
 _lib = torch.library.Library("exl3_b200", "FRAGMENT")       # must stay alive at module scope
 
-# Row count from which the many-row path is taken; 0 = decide per call with `prefers_decode` (the crossover depends on the
-# shape and, since narrow outputs split their reduction over the idle SMs, lies at 17 rows for the 27B-shape groups).
-DENSE_ROWS = int(os.environ.get("EXL3_B200_DENSE_ROWS", "0"))
+
+class _Module(types.ModuleType):
+    """Measurement knobs, module attributes that live in the native operator.
+
+    DENSE_ROWS: row count from which the many-row path is taken; 0 = decide per call with `prefers_decode` (the crossover depends
+    on the shape).  PREFILL: "tc" = fused tcgen05 kernel; "library" = decode to fp16 + library GEMM (the reference's sequence), for
+    comparisons."""
+
+    @property
+    def DENSE_ROWS(self) -> int:
+        return _ops.knob(0, -1)
+
+    @DENSE_ROWS.setter
+    def DENSE_ROWS(self, rows: int) -> None:
+        _ops.knob(0, int(rows))
+
+    @property
+    def PREFILL(self) -> str:
+        return "library" if _ops.knob(1, -1) else "tc"
+
+    @PREFILL.setter
+    def PREFILL(self, path: str) -> None:
+        _ops.knob(1, int(path == "library"))
+
+
+sys.modules[__name__].__class__ = _Module
+_ops.knob(0, int(os.environ.get("EXL3_B200_DENSE_ROWS", "0")))
+_ops.knob(1, int(os.environ.get("EXL3_B200_PREFILL", "tc") == "library"))
 
 
 def prefers_decode(rows: int, k: int, n_total: int, sms: int = 148) -> bool:
-    """Cost model fitted to measurements on B200 (microseconds); `sms` is the device's multiprocessor count.  The decode kernel streams the weights once per 16 rows:
-    ~14 + 0.38 per million weights for a full chunk, ~0.8 of that for a last chunk of up to 8 rows.  The tensor-core kernel
-    works through its tiles in waves over the SMs at ~1.1 per 64-deep reduction block (~1.6 for the 512-row tiles used above
-    256 rows); when the tiles are fewer than the SMs the reduction of each is cut into up to 8 parts on CTAs of their own;
-    ~12 more for the two rotation launches, ~8 for adding the parts."""
-    mw = k * n_total / 1e6
-    chunk = 14.0 + 0.38 * mw
-    full, rem = divmod(rows, 16)
-    decode = full * chunk + (0.0 if rem == 0 else chunk * (0.8 if rem <= 8 else 1.0))
-    if rows <= 256:
-        tiles, per_block = -(-rows // 256) * max(n_total // 256, 1), 1.1
-    else:
-        tiles, per_block = -(-rows // 512) * (n_total // 128), 1.6
-    parts = max(1, min(8, sms // max(tiles, 1), k // 64))
-    tensor = -(-tiles // sms) * (k / 64) / parts * per_block + 12.0 + (8.0 if parts > 1 else 0.0) + 0.08 * min(rows, 256)
-    return decode <= tensor
-# "tc": fused tcgen05 kernel; "library": decode to fp16 + library GEMM (the reference's sequence), for comparisons.
-PREFILL = os.environ.get("EXL3_B200_PREFILL", "tc")
+    """Whether the decode kernel is expected to be faster than the tensor-core kernel for these sizes; `sms` is the device's
+    multiprocessor count."""
+    return bool(_native_lib.load().exl3_prefers_decode(rows, k, n_total, sms))
 
 
 def dense_group(x: torch.Tensor, packed: torch.Tensor, suh_cat: torch.Tensor, svh_cat: torch.Tensor, shard_ends: list[int],
@@ -77,53 +91,19 @@ def dense_group(x: torch.Tensor, packed: torch.Tensor, suh_cat: torch.Tensor, sv
     return out
 
 
-def _linear(x: torch.Tensor, trellis: list[torch.Tensor], suh: list[torch.Tensor], svh: list[torch.Tensor],
-            dense: list[torch.Tensor], sliced: list[torch.Tensor], sliced_min_rows: int, marlin_w: list[torch.Tensor],
-            marlin_ends: list[int], codebooks: list[int], out_widths: list[int]) -> torch.Tensor:
-    if len(marlin_w) != 3:
-        raise RuntimeError("marlin_w must be [packed, suh_cat, svh_cat] from kernels.linear.prepare")
-    if len(set(codebooks)) != 1:
-        raise RuntimeError("one codebook per fused group")
+def _dense_linear(h: torch.Tensor, dense: list[torch.Tensor], marlin_w: list[torch.Tensor], marlin_ends: list[int], codebook: int) -> torch.Tensor:
+    """The branch of `linear` for resident decoded weights (`dense`) and for the library sequence."""
     packed, suh_cat, svh_cat = marlin_w
-    ends = list(marlin_ends)
-    k, n_total = packed.shape[1] * 128, packed.shape[0] * 128
-    rows = x.reshape(-1, x.shape[-1])
-    h = rows if rows.dtype in (torch.float16, torch.bfloat16) else rows.to(torch.float16)
-    if h.shape[1] > k:
-        raise RuntimeError(f"input width {h.shape[1]} exceeds the stored width {k}")
-    if h.shape[1] < k:                                   # stored input width is padded to 128
-        h = torch.nn.functional.pad(h, (0, k - h.shape[1]))
-    h = h.contiguous()
-    sms = lib_sm_count(h.device.index if h.device.index is not None else torch.cuda.current_device())
-    if (h.shape[0] < DENSE_ROWS) if DENSE_ROWS > 0 else prefers_decode(h.shape[0], k, n_total, sms):
-        y = lin.run(h, packed, suh_cat, svh_cat, ends, codebooks[0])
-    elif dense or PREFILL == "library":
-        y = torch.empty((h.shape[0], n_total), dtype=h.dtype, device=h.device)
-        dense_group(h, packed, suh_cat, svh_cat, ends, codebooks[0], y, list(dense) if dense else None)
-    else:
-        y = lin.run_tc(h, packed, suh_cat, svh_cat, ends, codebooks[0])
-    bounds = [0, *ends, n_total]
-    stored = [b - a for a, b in zip(bounds[:-1], bounds[1:])]
-    if any(w > s for w, s in zip(out_widths, stored)):   # logical widths beyond the stored ones read as zeros (ops.py:117-121)
-        padded = torch.zeros((y.shape[0], sum(out_widths)), dtype=y.dtype, device=y.device)
-        col = 0
-        for a, w, s in zip(bounds[:-1], out_widths, stored):
-            keep = min(w, s)
-            padded[:, col:col + keep] = y[:, a:a + keep]
-            col += w
-        y = padded
-    elif list(out_widths) != stored:                     # stored output columns beyond the true width are dropped
-        y = torch.cat([y[:, a:a + w] for a, w in zip(bounds[:-1], out_widths)], dim=1)
-    return y.to(x.dtype).view(*x.shape[:-1], y.shape[1])
+    y = torch.empty((h.shape[0], packed.shape[0] * 128), dtype=h.dtype, device=h.device)
+    return dense_group(h, packed, suh_cat, svh_cat, list(marlin_ends), codebook, y, list(dense) if dense else None)
 
 
 def _linear_fake(x, trellis, suh, svh, dense, sliced, sliced_min_rows, marlin_w, marlin_ends, codebooks, out_widths):
     return x.new_empty((*x.shape[:-1], sum(out_widths)))
 
 
-_lib.define("linear(Tensor x, Tensor[] trellis, Tensor[] suh, Tensor[] svh, Tensor[] dense, Tensor[] sliced, int sliced_min_rows, "
-            "Tensor[] marlin_w, int[] marlin_ends, int[] codebooks, int[] out_widths) -> Tensor")
-_lib.impl("linear", _linear, "CUDA")
+_lib.define("dense_linear(Tensor h, Tensor[] dense, Tensor[] marlin_w, int[] marlin_ends, int codebook) -> Tensor")
+_lib.impl("dense_linear", _dense_linear, "CUDA")
 torch.library.register_fake("exl3_b200::linear", _linear_fake, lib=_lib)
 
 linear = torch.ops.exl3_b200.linear
