@@ -1,0 +1,50 @@
+"""The decode GEMV / skinny GEMM at the edges of its row pitches (1-2, 3-8, 9-16, 17-32, 33-64 rows) and of its stage ring (ranges of
+one unit, ranges that wrap the ring several times), with and without the rotation inside, against a plain fp32 product on the decoded
+weights."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from trellis_serve_b200.kernels import linear as lin
+from trellis_serve_b200.runtime.layerset import random_packed, random_signs
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _had128(x: torch.Tensor) -> torch.Tensor:
+    h = torch.ones((1, 1), device=x.device)
+    while h.shape[0] < 128:
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    return (x.view(x.shape[0], -1, 128) @ (h / 128 ** 0.5)).reshape(x.shape)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 8, 9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("k,ns,K,cb", [(128, [128], 3, 0), (384, [256, 128], 8, 1), (5120, [5120, 1024, 1024], 3, 0), (17408, [2048], 2, 2),
+                                       (2176, [17408], 8, 0), (5120, [10240], 5, 1)])
+def test_rows_and_ring_edges(rows, k, ns, K, cb):
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(rows + k)
+    packed = torch.cat([random_packed(k, n, K, gen, DEV) for n in ns])
+    suh, svh = random_signs(k, gen, DEV, len(ns)), (random_signs(sum(ns), gen, DEV).view(-1) / 64).half()
+    ends = [sum(ns[:i + 1]) for i in range(len(ns) - 1)]
+    dtype = torch.bfloat16 if rows % 2 else torch.float16
+    x = torch.randn((rows, k), device=DEV, generator=gen).to(dtype)
+    y = torch.empty((rows, sum(ns)), dtype=torch.float32, device=DEV)
+    lin.run(x, packed, suh, svh, ends, cb, out=y)
+    again = torch.empty_like(y)
+    lin.run(x, packed, suh, svh, ends, cb, out=again)
+    torch.cuda.synchronize()
+    lin.device_error(DEV)
+    assert torch.equal(y, again)
+    xh = lin.had_in_group(x, suh).float()
+    col = 0
+    torch.backends.cuda.matmul.allow_tf32 = False
+    for s, n in enumerate(ns):
+        w = lin.reconstruct_packed(packed[col // 128:(col + n) // 128].contiguous(), cb).float()
+        want = _had128(xh[s * rows:(s + 1) * rows] @ w) * svh[col:col + n].float()
+        got = y[:, col:col + n]
+        assert float((got - want).norm() / want.norm()) <= 1e-3
+        assert float((got - want).abs().max() / want.pow(2).mean().sqrt()) <= 2e-3
+        col += n

@@ -2,7 +2,7 @@
 
     python -m trellis_serve_b200.csrc.build [--force] [--verbose]
 
-One object per source; the decode GEMV is compiled once per bit rate (-DEXL3_GEMV_K=2..8) so the seven
+One object per source; the decode GEMV is compiled once per bit rate (-DEXL3_SKINNY_K=2..8) so the seven
 instantiation sets build in parallel.  Output: trellis_serve_b200/libexl3_b200.so, and libexl3_b200_torch.so beside it (the
 torch operators over the C ABI, host code only).
 """
@@ -25,8 +25,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", 
          "--expt-relaxed-constexpr", "-Xptxas", "-v", *os.environ.get("EXL3_B200_NVCC_FLAGS", "").split()]
 
-PLAIN = ["exl3_api.cu", "exl3_kernels.cu", "exl3_gemv.cu", "exl3_moe.cu", "exl3_moe_tc.cu", "exl3_gemm_tc.cu", "exl3_allreduce.cu", "exl3_step.cu"]
-PER_K = [("exl3_gemv_inst.cu", "EXL3_GEMV_K", range(2, 9)), ("exl3_moe_inst.cu", "EXL3_MOE_K", range(2, 9))]
+PLAIN = ["exl3_api.cu", "exl3_kernels.cu", "exl3_skinny.cu", "exl3_moe.cu", "exl3_moe_tc.cu", "exl3_gemm_tc.cu", "exl3_allreduce.cu", "exl3_step.cu"]
+PER_K = [("exl3_skinny_inst.cu", "EXL3_SKINNY_K", range(2, 9)), ("exl3_moe_inst.cu", "EXL3_MOE_K", range(2, 9))]
 
 
 def nvcc() -> str:

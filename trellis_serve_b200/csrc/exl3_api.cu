@@ -5,6 +5,7 @@
 
 #include "exl3_internal.h"
 #include "exl3_moe_kernel.cuh"
+#include "exl3_skinny_kernel.cuh"
 
 namespace exl3 {
 
@@ -92,7 +93,7 @@ exl3_status exl3_init_device(int device)
         if (rc == EXL3_OK) rc = cuda_status(cudaDeviceGetAttribute(&d.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         if (rc == EXL3_OK) {
             d.ready = true;
-            rc = gemv_init_device();
+            rc = skinny_init_device();
             if (rc == EXL3_OK) rc = moe_init_device();
             if (rc == EXL3_OK) rc = attention_init_device();
             if (rc == EXL3_OK) rc = gemm_tc_init_device();
@@ -201,7 +202,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
     memset(&a, 0, sizeof(a));
     if (int rc = fill_shards(a, shard_ends, n_shards, n_total)) return rc;
     if (!rotated && !prerotated && x_dtype != EXL3_F16 && x_dtype != EXL3_BF16) return EXL3_ERR_UNSUPPORTED_DTYPE;
-    if (prerotated && rows > GEMV_MAX_ROWS) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (prerotated && rows > PREROTATED_MAX_ROWS) return EXL3_ERR_UNSUPPORTED_ROWS;
     if (y_dtype != EXL3_F16 && y_dtype != EXL3_F32 && !(y_dtype == EXL3_BF16 && !rotated)) return EXL3_ERR_UNSUPPORTED_DTYPE;
     if (rows == 0 || k == 0 || n_total == 0) return EXL3_OK;
     if ((size_t)(n_total / 128) > WS_MAX_COUNTERS) return EXL3_ERR_BAD_SHAPE;
@@ -213,7 +214,10 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
     if (prerotated ? !aligned(svh_cat, 8)
                    : rotated ? !aligned(xh_rowmajor, 2) : (!aligned(x, 2) || !aligned(suh_cat, 2) || !aligned(svh_cat, 8)))
         return EXL3_ERR_BAD_POINTER;
-    const WorkspaceLayout wl = workspace_layout(rows, k, n_total, n_shards);
+    // Rows per launch: as many as the kernels take and the workspace holds; a workspace sized for 16 rows serves any row count.
+    int most = tp ? PREROTATED_MAX_ROWS : SKINNY_MAX_ROWS;
+    while (most > PREROTATED_MAX_ROWS && workspace_layout(rows < most ? rows : most, k, n_total, n_shards).total > workspace_bytes) most -= 16;
+    const WorkspaceLayout wl = workspace_layout(rows < most ? rows : most, k, n_total, n_shards);
     if (!aligned(workspace, 256) || workspace_bytes < wl.total) return EXL3_ERR_WORKSPACE;
     unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
 
@@ -232,8 +236,9 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
     a.rotated = rotated ? 1 : 0;
     if (tp) a.tp = *tp;
     const size_t esz = 2, osz = y_dtype == EXL3_F32 ? 4 : 2;
-    for (int r0 = 0; r0 < rows; r0 += GEMV_MAX_ROWS) {
-        const int r = rows - r0 < GEMV_MAX_ROWS ? rows - r0 : GEMV_MAX_ROWS;
+    const int layout = rotated_layout(a.mode);
+    for (int r0 = 0, r; r0 < rows; r0 += r) {
+        r = rows - r0 < most ? rows - r0 : most;
         a.rows = r;
         a.out = y ? reinterpret_cast<unsigned char*>(y) + (size_t)r0 * n_total * osz : nullptr;
         if (res) {
@@ -243,18 +248,14 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
         }
         int rc;
         if (prerotated) {
-            // The fragments are in the workspace already (exl3_rotate_fragments, exl3_rmsnorm_rotate, exl3_silu_mul_rotate):
-            // up to two rows the kernel copies those of its units into shared memory once, else it reads them tile by tile.
-            a.x = nullptr;
-            a.xf_staged = 1;
-            if (!gemv_rotates_input(a)) a.xf_staged = 0;
-            if (res && !a.xf_staged) {          // more rows than the residual epilogue serves: plain GEMV, then the stream kernel
+            // The rotated input is in the workspace already (exl3_rotate_fragments, exl3_rmsnorm_rotate, exl3_silu_mul_rotate).
+            if (res && r > SK_FUSED_ROWS) {     // more rows than the residual epilogue serves: plain launch, then the stream kernel
                 if (!y) return EXL3_ERR_BAD_POINTER;
+                void* res_out = a.res_out;
                 a.res_out = nullptr;
-                rc = launch_gemv(a, st);
+                rc = launch_skinny(a, st);
                 if (rc) return rc;
-                rc = launch_residual_ssq(a.out, a.res_in, y_dtype == EXL3_BF16, r, n_total, reinterpret_cast<unsigned char*>(res->res_out) + (size_t)r0 * n_total * 2,
-                                         res->ssq_out + (size_t)r0 * (n_total / 128), st);
+                rc = launch_residual_ssq(a.out, a.res_in, y_dtype == EXL3_BF16, r, n_total, res_out, a.ssq_out, st);
                 if (rc) return rc;
                 continue;
             }
@@ -262,12 +263,12 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
             // shard s reads slab s of xh: rows [s*rows + r0, s*rows + r0 + r)
             for (int s = 0; s < n_shards; s++) {
                 const __half* src = reinterpret_cast<const __half*>(xh_rowmajor) + ((size_t)s * rows + r0) * k;
-                uint32_t* dst = const_cast<uint32_t*>(a.xf) + (size_t)s * (k / 16) * r * 4 * gemv_frag_words(a.mode);
-                rc = launch_to_fragments(src, 1, r, k, dst, a.mode == GEMV_SPLIT ? 1 : 2, st);
+                uint32_t* dst = const_cast<uint32_t*>(a.xf) + (size_t)s * (k / 16) * operand_pitch(r) * 4 * gemv_frag_words(a.mode);
+                rc = launch_to_fragments(src, 1, r, k, dst, layout, st);
                 if (rc) return rc;
             }
         } else {
-            // Up to two rows: the GEMV rotates its own input (one launch); otherwise the rotation kernel runs ahead of it.
+            // Few rows: the kernel rotates its own input (one launch); otherwise the rotation kernel runs ahead of it.
             // glu: x is gate | up with rows of 2k values and the input proper is silu(gate) * up.
             const unsigned char* xr = reinterpret_cast<const unsigned char*>(x) + (size_t)r0 * (glu ? 2 * k : k) * esz;
             a.x = xr;
@@ -279,41 +280,31 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
                 a.ssq_in = norm->ssq + (size_t)r0 * (k / 128);
                 a.norm_eps = norm->eps;
             }
-            if (!gemv_rotates_input(a)) {
+            if (!skinny_rotates_input(a)) {
+                // The rotation, normalisation or activation kernel ahead of the product, and behind it the stream kernel where the
+                // epilogue does not add the residual.
                 a.x = nullptr;
-                if (norm || res) {
-                    // more rows than the kernel rotates itself: the normalisation / activation kernel ahead of a plain GEMV, and
-                    // the stream kernel behind it where the epilogue would have added the residual
-                    a.norm_weight = nullptr;
+                a.norm_weight = nullptr;
+                const __half* signs = reinterpret_cast<const __half*>(suh_cat);
+                uint32_t* xf = const_cast<uint32_t*>(a.xf);
+                const bool x16 = x_dtype == EXL3_BF16;
+                rc = norm  ? launch_rmsnorm_rotate(xr, nullptr, norm->weight, norm->eps, x16, signs, n_shards, r, k, nullptr, xf, layout, st)
+                     : glu ? launch_silu_mul_rotate(xr, x16, signs, r, k, nullptr, xf, layout, st)
+                           : launch_had_in(xr, x16, signs, n_shards, r, k, xf, layout, st);
+                if (rc) return rc;
+                if (res && r > SK_FUSED_ROWS) {
+                    if (!y) return EXL3_ERR_BAD_POINTER;
                     void* res_out = a.res_out;
                     a.res_out = nullptr;
-                    if (res && !y) return EXL3_ERR_BAD_POINTER;
-                    if (norm)
-                        rc = launch_rmsnorm_rotate(xr, nullptr, norm->weight, norm->eps, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat),
-                                                   n_shards, r, k, nullptr, const_cast<uint32_t*>(a.xf), a.mode == GEMV_SPLIT ? 1 : 2, st);
-                    else if (glu)
-                        rc = launch_silu_mul_rotate(xr, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat), r, k, nullptr,
-                                                    const_cast<uint32_t*>(a.xf), a.mode == GEMV_SPLIT ? 1 : 2, st);
-                    else
-                        rc = launch_had_in(xr, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat), n_shards, r, k,
-                                           const_cast<uint32_t*>(a.xf), a.mode == GEMV_SPLIT ? 1 : 2, st);
+                    rc = launch_skinny(a, st);
                     if (rc) return rc;
-                    rc = launch_gemv(a, st);
+                    rc = launch_residual_ssq(a.out, a.res_in, y_dtype == EXL3_BF16, r, n_total, res_out, a.ssq_out, st);
                     if (rc) return rc;
-                    if (res) {
-                        rc = launch_residual_ssq(a.out, a.res_in, y_dtype == EXL3_BF16, r, n_total, res_out, a.ssq_out, st);
-                        if (rc) return rc;
-                    }
                     continue;
                 }
-                rc = glu ? launch_silu_mul_rotate(xr, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat), r, k, nullptr,
-                                                  const_cast<uint32_t*>(a.xf), a.mode == GEMV_SPLIT ? 1 : 2, st)
-                         : launch_had_in(xr, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat), n_shards, r, k,
-                                         const_cast<uint32_t*>(a.xf), a.mode == GEMV_SPLIT ? 1 : 2, st);
-                if (rc) return rc;
             }
         }
-        rc = launch_gemv(a, st);
+        rc = launch_skinny(a, st);
         if (rc) return rc;
     }
     return EXL3_OK;
@@ -337,7 +328,7 @@ exl3_status exl3_linear_allreduce(const void* x, int x_dtype, const uint32_t* pa
         return linear_common(x, x_dtype, nullptr, packed, K, codebook, suh_cat, svh_cat, shard_ends, n_shards, rows, k, n_total, y,
                              y_dtype, workspace, workspace_bytes, (cudaStream_t)stream, false);
     if (y_dtype != EXL3_F16 && y_dtype != EXL3_BF16) return EXL3_ERR_UNSUPPORTED_DTYPE;
-    const size_t chunk_rows = rows < GEMV_MAX_ROWS ? (rows < 0 ? 0 : rows) : GEMV_MAX_ROWS;
+    const size_t chunk_rows = rows < PREROTATED_MAX_ROWS ? (rows < 0 ? 0 : rows) : PREROTATED_MAX_ROWS;
     const size_t slot_bytes = (max_elems * 4 + 255) & ~(size_t)255;
     if (chunk_rows * (size_t)(n_total < 0 ? 0 : n_total) > max_elems || slot_bytes > 0xFFFFFFFFu) return EXL3_ERR_BAD_SHAPE;
     if (!peer_regions || !state || !aligned(state, 4)) return EXL3_ERR_BAD_POINTER;
@@ -392,11 +383,11 @@ exl3_status exl3_device_error(void* workspace, size_t workspace_bytes, void* str
 
 /* ---- decode step: rotated fragments written by the kernel ahead of the linear -------------------------------------- */
 
-static int fragment_mode(int codebook) { return gemv_default_mode(codebook) == GEMV_SPLIT ? 1 : 2; }
+static int fragment_mode(int codebook) { return rotated_layout(gemv_default_mode(codebook)); }
 
 static int fragment_region(int rows, int k, int n_shards, void* workspace, size_t workspace_bytes, uint32_t** xf)
 {
-    if (rows < 0 || rows > GEMV_MAX_ROWS) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (rows < 0 || rows > PREROTATED_MAX_ROWS) return EXL3_ERR_UNSUPPORTED_ROWS;
     if (k < 0 || (k % 128) || n_shards < 1 || n_shards > GEMV_MAX_SHARDS) return EXL3_ERR_BAD_SHAPE;
     const WorkspaceLayout wl = workspace_layout(rows, k, 128, n_shards);
     if (!aligned(workspace, 256) || workspace_bytes < wl.partials_off) return EXL3_ERR_WORKSPACE;

@@ -212,8 +212,8 @@ __device__ __forceinline__ LaneRegs<K> lane_regs(const uint32_t (&own)[2], uint3
 }
 
 // 16-bit trellis state of element P (0..7) of the lane, bits above it cleared.
-template <int K, int P>
-__device__ __forceinline__ uint32_t window_low(const LaneRegs<K>& R, const Pow2& pw)
+template <int K, int P, typename Powers>
+__device__ __forceinline__ uint32_t window_low(const LaneRegs<K>& R, const Powers& pw)
 {
     constexpr int lo = K * (7 - P);
     constexpr int j = lo / 16;

@@ -1,4 +1,4 @@
-// Pieces shared by the dense decode GEMV (exl3_gemv_kernel.cuh) and the grouped MoE GEMV (exl3_moe_kernel.cuh): the
+// Pieces shared by the dense decode GEMV (exl3_skinny_kernel.cuh) and the grouped MoE GEMV (exl3_moe_kernel.cuh): the
 // even, contiguous split of a unit list over persistent CTAs, the register-level decode of one 16x16 tile into MMA
 // operands, and the tensor-parallel exchange that a row-parallel linear runs in its epilogue.
 #pragma once
@@ -20,14 +20,10 @@ __device__ __forceinline__ unsigned long long tl_now()
     return t;
 }
 #define EXL3_STAMP(i) do { if (threadIdx.x == 0) p.tl[(blockIdx.x) * TL_POINTS + (i)] = tl_now(); } while (0)
-#define EXL3_STAMP_ANY(i) do { if ((threadIdx.x & 31) == 0) p.tl[(blockIdx.x) * TL_POINTS + (i)] = tl_now(); } while (0)
-#define EXL3_STAMP_CLK(i) do { if (threadIdx.x == 0) p.tl[(blockIdx.x) * TL_POINTS + (i)] = (unsigned long long)clock64(); } while (0)
-#define EXL3_STAMP_SM(i) do { if (threadIdx.x == 0) { unsigned s_; asm volatile("mov.u32 %0, %%smid;" : "=r"(s_)); p.tl[(blockIdx.x) * TL_POINTS + (i)] = s_; } } while (0)
+#define EXL3_STAMP_LANE(which, i) do { if ((which) && (threadIdx.x & 31) == 0) p.tl[(blockIdx.x) * TL_POINTS + (i)] = tl_now(); } while (0)
 #else
 #define EXL3_STAMP(i) do { } while (0)
-#define EXL3_STAMP_ANY(i) do { } while (0)
-#define EXL3_STAMP_CLK(i) do { } while (0)
-#define EXL3_STAMP_SM(i) do { } while (0)
+#define EXL3_STAMP_LANE(which, i) do { } while (0)
 #endif
 
 // Unit indices fit 32 bits (the host refuses matrices with 2^31 or more units).
@@ -39,8 +35,8 @@ __device__ __forceinline__ int gemv_cta_of_unit(long long u, int q, int r)
     return u < boundary ? (int)(u / (q + 1)) : r + (int)((u - boundary) / q);
 }
 
-template <int K, int MODE, int FAM>
-__device__ __forceinline__ void decode_tile_regs(const LaneRegs<K>& R, const Pow2& pw, CodebookConst cbc, uint32_t (&w)[8])
+template <int K, int MODE, int FAM, typename Powers>
+__device__ __forceinline__ void decode_tile_regs(const LaneRegs<K>& R, const Powers& pw, CodebookConst cbc, uint32_t (&w)[8])
 {
     uint32_t s[8];
     s[0] = window_low<K, 0>(R, pw); s[1] = window_low<K, 1>(R, pw); s[2] = window_low<K, 2>(R, pw); s[3] = window_low<K, 3>(R, pw);
@@ -57,29 +53,6 @@ __device__ __forceinline__ void decode_tile_regs(const LaneRegs<K>& R, const Pow
     }
 }
 
-__device__ __forceinline__ float gemv_load_x(const void* p, long long idx, bool bf16)
-{
-    // bf16 inputs are first converted to fp16 (round to nearest even), as the stand-alone rotation kernel does.
-    if (bf16) return __half2float(__float2half_rn(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[idx])));
-    return __half2float(reinterpret_cast<const __half*>(p)[idx]);
-}
-
-// The same for a down projection fed straight from gate | up (row stride 2k): the activation silu(gate) * up, rounded to the
-// activation type as the stand-alone activation kernel stores it, then taken as fp16.
-__device__ __forceinline__ float gemv_load_glu(const void* p, long long idx, int k, bool bf16)
-{
-    float g, u;
-    if (bf16) {
-        g = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[idx]);
-        u = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[idx + k]);
-    } else {
-        g = __half2float(reinterpret_cast<const __half*>(p)[idx]);
-        u = __half2float(reinterpret_cast<const __half*>(p)[idx + k]);
-    }
-    const float act = g / (1.0f + __expf(-g)) * u;
-    return __half2float(__float2half_rn(bf16 ? __bfloat162float(__float2bfloat16_rn(act)) : act));
-}
-
 __device__ __forceinline__ float gemv_raw(const void* p, long long idx, bool bf16)
 {
     return bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[idx]) : __half2float(reinterpret_cast<const __half*>(p)[idx]);
@@ -88,14 +61,6 @@ __device__ __forceinline__ float gemv_raw(const void* p, long long idx, bool bf1
 __device__ __forceinline__ float gemv_round_act(float v, bool bf16)
 {
     return bf16 ? __bfloat162float(__float2bfloat16_rn(v)) : __half2float(__float2half_rn(v));
-}
-
-// The normalised activation z * rstd * weight, rounded to the activation type (as the stand-alone normalisation kernel stores
-// it) and taken as fp16.
-__device__ __forceinline__ float gemv_load_norm(const void* z, const void* weight, long long idx, long long col, float rstd, bool bf16)
-{
-    const float a = gemv_round_act(gemv_raw(z, idx, bf16) * rstd * gemv_raw(weight, col, bf16), bf16);
-    return __half2float(__float2half_rn(a));
 }
 
 // 1 / sqrt(mean square + eps) of a row of the residual stream from its per-block sums of squares (one warp, every lane gets
@@ -114,9 +79,10 @@ __device__ __forceinline__ float gemv_row_rstd(const float* ssq_row, int blocks,
 // the same words of all ranks are awaited here (bounded), added in rank order in fp32 and rounded once: the bits a
 // separate all-reduce of the rounded outputs gives.  Kept out of line: it runs once per 128 outputs and must not
 // weigh on the register allocation of the decode loop.
-static __device__ __noinline__ void gemv_exchange_store(const TpExchange& tp, uint32_t tp_epoch, bool bf, const float (&v)[4], long long o,
+static __device__ __noinline__ void gemv_exchange_store(const TpExchange& tp, uint32_t tp_epoch, bool bf, float4 vv, long long o,
                                                  uint16_t* out, int* err)
 {
+    const float v[4] = {vv.x, vv.y, vv.z, vv.w};
     uint32_t w2[2];
 #pragma unroll
     for (int e = 0; e < 2; e++) {
@@ -190,13 +156,14 @@ static __device__ __noinline__ void gemv_exchange_store(const TpExchange& tp, ui
 // Residual epilogue of one row's block of 128 outputs (one warp, four columns per lane): y -- summed over the ranks first, if
 // there is an exchange -- rounded as it would be stored, plus the residual stream: the new stream goes to res_out, this block's
 // share of its mean square to ssq_out, y itself to `out` only if that is set.  Out of line: once per 128 outputs.
-static __device__ __noinline__ void gemv_residual_store(const GemvArgs& a, uint32_t tp_epoch, const float (&v)[4], long long o, int m, int fnb,
+static __device__ __noinline__ void gemv_residual_store(const GemvArgs& a, uint32_t tp_epoch, float4 vv, long long o, int m, int fnb,
                                                         int lane)
 {
+    const float v[4] = {vv.x, vv.y, vv.z, vv.w};
     const bool bf = a.out_dtype == EXL3_BF16;
     float y[4];
     if (a.tp.world > 1) {
-        gemv_exchange_store(a.tp, tp_epoch, bf, v, o, reinterpret_cast<uint16_t*>(a.out), a.err);
+        gemv_exchange_store(a.tp, tp_epoch, bf, vv, o, reinterpret_cast<uint16_t*>(a.out), a.err);
 #pragma unroll
         for (int e = 0; e < 4; e++) y[e] = gemv_raw(a.out, o + e, bf);       // what the exchange stored
     } else {
@@ -221,6 +188,40 @@ static __device__ __noinline__ void gemv_residual_store(const GemvArgs& a, uint3
 #pragma unroll
     for (int m2 = 16; m2 > 0; m2 >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, m2);
     if (lane == 0) a.ssq_out[(size_t)m * (a.n_total >> 7) + fnb] = ss;
+}
+
+// One row's block of 128 outputs (one warp, four columns per lane) from the fp32 sums: the rotated-basis product as it is, or
+// Had128 * svh in the output type, summed over the ranks where there is an exchange.  EPI 1: with the residual stream.
+template <int EPI>
+__device__ __forceinline__ void gemv_finish_row(const GemvArgs& a, uint32_t tp_epoch, float4 v, int m, int nb, int lane)
+{
+    const long long o = (long long)m * a.n_total + nb * 128 + 4 * lane;
+    if (EPI == 1 || !a.rotated) {
+        fwht128(v.x, v.y, v.z, v.w, lane);
+        const uint2 sv = *reinterpret_cast<const uint2*>(a.svh + nb * 128 + 4 * lane);
+        const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
+        v.x *= HAD_SCALE * __low2float(s01);
+        v.y *= HAD_SCALE * __high2float(s01);
+        v.z *= HAD_SCALE * __low2float(s23);
+        v.w *= HAD_SCALE * __high2float(s23);
+    }
+    if constexpr (EPI == 1) {
+        gemv_residual_store(a, tp_epoch, v, o, m, nb, lane);
+        return;
+    }
+    if (a.out_dtype == EXL3_F32) {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) = v;
+    } else if (!a.rotated && a.tp.world > 1) {
+        gemv_exchange_store(a.tp, tp_epoch, a.out_dtype == EXL3_BF16, v, o, reinterpret_cast<uint16_t*>(a.out), a.err);
+    } else {
+        const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+        uint2 w = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+        if (!a.rotated && a.out_dtype == EXL3_BF16) {
+            const __nv_bfloat162 b0 = __floats2bfloat162_rn(__low2float(h0), __high2float(h0)), b1 = __floats2bfloat162_rn(__low2float(h1), __high2float(h1));
+            w = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
+        }
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(a.out) + o) = w;
+    }
 }
 
 }  // namespace exl3

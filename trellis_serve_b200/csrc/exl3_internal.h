@@ -32,7 +32,7 @@ int launch_to_fragments(const __half* xh, int shards, int rows, int k, uint32_t*
 int launch_had_out(const void* y, int y_f32, const __half* svh, int rows, int n, void* out, long long out_stride, int out_bf16,
                    cudaStream_t st);
 
-// exl3_gemv.cu -------------------------------------------------------------------------------------------
+// exl3_skinny.cu -----------------------------------------------------------------------------------------
 
 // How decoded weights enter the tensor-core product.
 //   GEMV_SPLIT   hash codebooks: each weight occupies two k slots of the MMA as its two fp16 summands, the
@@ -40,11 +40,12 @@ int launch_had_out(const void* y, int y_f32, const __half* svh, int rows, int n,
 //   GEMV_PAIRED  any codebook: weights are rounded to fp16 and packed two per register.
 enum { GEMV_SPLIT = 0, GEMV_PAIRED = 1 };
 
-constexpr int GEMV_MAX_ROWS = 16;          // rows per launch
+constexpr int SKINNY_MAX_ROWS = 64;        // rows per launch
+constexpr int PREROTATED_MAX_ROWS = 16;    // rows whose rotated input a kernel ahead may have left in the workspace
 constexpr int GEMV_MAX_GRID = 512;         // upper bound of persistent CTAs assumed when sizing workspaces
 constexpr int GEMV_MAX_SHARDS = 4;
 
-// Words per lane of one activation fragment (four k values of a 16-row tile) in each mode.
+// Words per lane of one activation fragment (four k values of a 16-row tile) of the grouped MoE GEMV in each mode.
 __host__ __device__ constexpr int gemv_frag_words(int mode) { return mode == GEMV_SPLIT ? 4 : 2; }
 
 // Tensor-parallel exchange fused into the GEMV (row-parallel linears): peer regions laid out as for the one-shot
@@ -60,7 +61,7 @@ struct TpExchange {
 
 struct GemvArgs {
     const uint32_t* packed;     // resident weights, n-blocks of all shards concatenated
-    const uint32_t* xf;         // activation fragments [shard][k/16][rows][4][frag_words]
+    const uint32_t* xf;         // rotated activations, layout of had_in_kernel modes 1 / 2 (unless x is set)
     const void* x;              // in-kernel rotation (rows <= 2): raw activations [rows, k], else nullptr
     const __half* suh;          //   and the input sign vectors [n_shards][k]
     int x_bf16;
@@ -76,8 +77,6 @@ struct GemvArgs {
     const void* res_in;
     void* res_out;
     float* ssq_out;
-    int xf_staged;              // rows <= 2 without x: the fragments in xf are copied to shared memory once (bulk copies)
-                                //   instead of being read from global memory tile by tile
     const __half* svh;          // [n_total]; unused when rotated
     void* out;                  // [rows, n_total]
     float* partials;            // [(grid + NB)][rows][128]
@@ -95,11 +94,16 @@ struct GemvArgs {
 // Preferred mode for a codebook (split for the hash codebooks, paired for MUL1).
 int gemv_default_mode(int codebook);
 void gemv_set_mode_override(int mode);      // -1 = default; test / measurement knob
-// With a.x set the GEMV rotates the input itself (no rotation launch ahead of it); gemv_rotates_input() tells whether
-// that variant can serve the problem (row count, shared-memory budget) and launch_gemv() then requires it to.
-bool gemv_rotates_input(const GemvArgs& a);
-int launch_gemv(const GemvArgs& a, cudaStream_t st);
-int gemv_init_device();
+// With a.x set the kernel rotates the input itself (no rotation launch ahead of it); skinny_rotates_input() tells whether that
+// variant can serve the problem (row count, alignment, shared-memory budget) and launch_skinny() then requires it to.
+bool skinny_rotates_input(const GemvArgs& a);
+int launch_skinny(const GemvArgs& a, cudaStream_t st);
+int skinny_init_device();
+// Rows that a core-matrix column of the rotated input is laid out for (the kernels' B operand; the padding rows are never written and
+// their products never looked at): a constant of each kernel instance, so that descriptors advance by constants.
+__host__ __device__ inline int operand_pitch(int rows) { return rows <= 2 ? 2 : rows <= 8 ? 8 : rows <= 16 ? 16 : rows <= 32 ? 32 : 64; }
+// Layout of the rotated input that the kernel reads (mode of had_in_kernel).
+inline int rotated_layout(int gemv_mode) { return gemv_mode == GEMV_SPLIT ? 1 : 2; }
 
 // exl3_moe.cu -------------------------------------------------------------------------------------------
 struct MoeGemmLaunch;

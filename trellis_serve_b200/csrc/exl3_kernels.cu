@@ -176,12 +176,24 @@ __device__ __forceinline__ float load_as_f16_value(const void* p, long long idx,
     return __half2float(reinterpret_cast<const __half*>(p)[idx]);
 }
 
+// Four k values of a row into the B operand of the decode GEMV / skinny GEMM; at4 = (k / 4) counted over all shards.
+template <int MODE>
+__device__ __forceinline__ void store_operand(void* out, long long at4, int rows, int row, const __half (&h)[4])
+{
+    const int pitch = operand_pitch(rows);
+    uint32_t v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = __half_as_ushort(h[e]);
+    if constexpr (MODE == 1)
+        reinterpret_cast<uint4*>(out)[at4 * pitch + row] = make_uint4(v[0] * 0x10001u, v[1] * 0x10001u, v[2] * 0x10001u, v[3] * 0x10001u);
+    else
+        reinterpret_cast<uint2*>(out)[((at4 >> 1) * pitch + row) * 2 + (at4 & 1)] = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+}
+
 // xh = Had128(fp16(x) * suh[s]) for every shard s.  One warp per (shard, row, 128-block).
 // MODE 0: row-major fp16 [shards*rows, k] (slab s = rows s*rows..).
-// MODE 1: B-operand fragments for the split-pair MMA: [shard][k/16][rows][4 lanes q][4 words], every word one
-//         fp16 value duplicated in both halves; word order x[2q], x[2q+1], x[2q+8], x[2q+9] of the 16-row tile.
-// MODE 2: B-operand fragments for the paired MMA: [shard][k/16][rows][4 lanes q][2 words]:
-//         (x[2q], x[2q+1]), (x[2q+8], x[2q+9]).
+// MODE 1: B operand of the decode GEMV / skinny GEMM, split: [shard][k/4][pitch][8 halves], every value twice (8 k slots of one
+//         row are one 16-byte row of a core matrix).  MODE 2: paired: [shard][k/8][pitch][8 halves].  pitch = operand_pitch(rows).
 template <int MODE>
 __global__ void had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int rows, int k,
                               void* __restrict__ out)
@@ -213,55 +225,21 @@ __global__ void had_in_kernel(const void* __restrict__ x, int x_bf16, const __ha
             (uint32_t)__half_as_ushort(h[0]) | ((uint32_t)__half_as_ushort(h[1]) << 16),
             (uint32_t)__half_as_ushort(h[2]) | ((uint32_t)__half_as_ushort(h[3]) << 16));
     } else {
-        // lane holds tile-local rows r = 4*(lane&3) + e of 16-row tile kt = kg*8 + lane/4
-        const int kt = kg * 8 + (lane >> 2);
-        const int rbase = 4 * (lane & 3);
-        if constexpr (MODE == 1) {
-            uint32_t* o = reinterpret_cast<uint32_t*>(out) + (((long long)s * (k >> 4) + kt) * rows + row) * 16;
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int r = rbase + e;
-                int q = (r & 7) >> 1;
-                int slot = (r & 1) + 2 * (r >> 3);
-                uint32_t hv = __half_as_ushort(h[e]);
-                o[q * 4 + slot] = hv | (hv << 16);
-            }
-        } else {
-            uint32_t* o = reinterpret_cast<uint32_t*>(out) + (((long long)s * (k >> 4) + kt) * rows + row) * 8;
-#pragma unroll
-            for (int e = 0; e < 4; e += 2) {
-                int r = rbase + e;
-                int q = (r & 7) >> 1;
-                int slot = r >> 3;
-                o[q * 2 + slot] = (uint32_t)__half_as_ushort(h[e]) | ((uint32_t)__half_as_ushort(h[e + 1]) << 16);
-            }
-        }
+        store_operand<MODE>(out, ((long long)s * kgs + kg) * 32 + lane, rows, row, h);
     }
 }
 
-// Row-major fp16 xh [shards*rows, k] (already rotated) -> fragment layouts of had_in_kernel MODE 1 / 2.
+// Row-major fp16 xh [shards*rows, k] (already rotated) -> layouts of had_in_kernel MODE 1 / 2; one thread per four values.
 template <int MODE>
 __global__ void to_fragments_kernel(const __half* __restrict__ xh, int shards, int rows, int k, uint32_t* __restrict__ out)
 {
-    long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;      // one thread per (s, row, kt, q)
-    const int kts = k >> 4;
-    if (idx >= (long long)shards * rows * kts * 4) return;
-    int q = (int)(idx & 3);
-    long long r = idx >> 2;
-    int kt = (int)(r % kts);
-    r /= kts;
-    int row = (int)(r % rows);
-    int s = (int)(r / rows);
-    const __half* src = xh + ((long long)s * rows + row) * k + kt * 16;
-    uint32_t a = __half_as_ushort(src[2 * q]), b = __half_as_ushort(src[2 * q + 1]);
-    uint32_t c = __half_as_ushort(src[2 * q + 8]), d = __half_as_ushort(src[2 * q + 9]);
-    if constexpr (MODE == 1) {
-        uint4* o = reinterpret_cast<uint4*>(out) + (((long long)s * kts + kt) * rows + row) * 4 + q;
-        *o = make_uint4(a | (a << 16), b | (b << 16), c | (c << 16), d | (d << 16));
-    } else {
-        uint2* o = reinterpret_cast<uint2*>(out) + (((long long)s * kts + kt) * rows + row) * 4 + q;
-        *o = make_uint2(a | (b << 16), c | (d << 16));
-    }
+    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int k4 = k >> 2;
+    if (idx >= (long long)shards * rows * k4) return;
+    const int at = (int)(idx % k4), row = (int)((idx / k4) % rows), s = (int)(idx / ((long long)k4 * rows));
+    const __half* src = xh + ((long long)s * rows + row) * k + 4 * at;
+    const __half h[4] = {src[0], src[1], src[2], src[3]};
+    store_operand<MODE>(out, (long long)s * k4 + at, rows, row, h);
 }
 
 __device__ __forceinline__ void store_out4(void* out, long long idx, const float (&v)[4], bool bf16)
@@ -451,16 +429,16 @@ int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (mode == 0) return cuda_status(cudaLaunchKernelEx(&cfg, had_in_kernel<0>, x, x_bf16, suh, shards, rows, k, out));
-    if (mode == 1) return cuda_status(cudaLaunchKernelEx(&cfg, had_in_kernel<1>, x, x_bf16, suh, shards, rows, k, out));
-    return cuda_status(cudaLaunchKernelEx(&cfg, had_in_kernel<2>, x, x_bf16, suh, shards, rows, k, out));
+    auto kernel = mode == 1 ? had_in_kernel<1> : had_in_kernel<2>;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, x, x_bf16, suh, shards, rows, k, out));
 }
 
 int launch_to_fragments(const __half* xh, int shards, int rows, int k, uint32_t* out, int mode, cudaStream_t st)
 {
-    long long items = (long long)shards * rows * (k / 16) * 4;
+    long long items = (long long)shards * rows * (k / 4);
     if (items == 0) return EXL3_OK;
-    if (mode == 1) to_fragments_kernel<1><<<blocks_for(items, 256), 256, 0, st>>>(xh, shards, rows, k, out);
-    else to_fragments_kernel<2><<<blocks_for(items, 256), 256, 0, st>>>(xh, shards, rows, k, out);
+    auto kernel = mode == 1 ? to_fragments_kernel<1> : to_fragments_kernel<2>;
+    kernel<<<blocks_for(items, 256), 256, 0, st>>>(xh, shards, rows, k, out);
     return cuda_status(cudaGetLastError());
 }
 

@@ -296,7 +296,7 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     if (ups > UB) ups = UB;
     l.units_per_stage = ups;
     l.stage_stride = (uint32_t)ups * (unit_bytes + frag_bytes);
-    const size_t fixed = 256 + GEMV_MAX_ROWS * 128 * 4;
+    const size_t fixed = 256 + MOE_BLOCK_ROWS * 128 * 4;
     int stages = (int)((96u * 1024u) / l.stage_stride);
     const int cap = (int)((d->max_smem_optin / MOE_CTAS_PER_SM - 2048 - fixed) / l.stage_stride);
     if (stages > cap) stages = cap;

@@ -6,7 +6,7 @@
 // cuda/csrc/exl3_marlin_moe.cu:542-594); this kernel multiplies each block by its expert's matrix.  It replaces the
 // reference's grouped Marlin instances (cuda/csrc/exl3_marlin_moe_template.h, launch at exl3_marlin_moe.cu:376-408).
 //
-// Same machinery as the dense decode GEMV (exl3_gemv_kernel.cuh): persistent CTAs that split the unit list
+// Same machinery as the dense decode GEMV (exl3_skinny_kernel.cuh): persistent CTAs that split the unit list
 // (moe block, column block, row block) evenly and contiguously, a producer thread streaming weights through a ring of
 // bulk-copy stages, 16 consumer warps decoding in registers into transposed m16n8k16 MMAs, split-k partial sums
 // finished by the last CTA to arrive.  Differences: the number of blocks is read on the device (CUDA-graph safe), a
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(MOE_THREADS, MOE_CTAS_PER_SM) moe_gemm_kernel(
     uint64_t* empty = full + MOE_MAX_STAGES;
     int* flag = reinterpret_cast<int*>(smem + 2 * MOE_MAX_STAGES * 8);
     float* P = reinterpret_cast<float*>(smem + 256);                              // [8][128]
-    unsigned char* stage0 = smem + 256 + GEMV_MAX_ROWS * 128 * 4;
+    unsigned char* stage0 = smem + 256 + MOE_BLOCK_ROWS * 128 * 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cta = blockIdx.x;

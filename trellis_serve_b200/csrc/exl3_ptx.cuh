@@ -30,38 +30,50 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  : "memory");
 }
 
-// A waiting warp is suspended by the hardware for up to this many nanoseconds per poll instead of burning issue slots.
-constexpr uint32_t MBAR_SUSPEND_NS = 20000;
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
+// A waiting warp is suspended by the hardware until the phase completes or a time of its own choosing has passed.  (Giving it a
+// time hint instead compiles into a polling loop with sleeps.)
+__device__ __forceinline__ bool mbar_try_wait_addr(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity), "r"(MBAR_SUSPEND_NS)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait_addr(smem_addr(bar), parity); }
 
-// Bounded wait: about a second of polling at most, then gives up.
-constexpr uint32_t MBAR_MAX_POLLS = 1u << 16;
+// Bounded waits: how long a failed poll suspends the warp is up to the hardware, so the bound is a time, not a number of polls.
+constexpr uint64_t MBAR_MAX_NS = 2000000000ull;
+
+__device__ __forceinline__ uint64_t time_ns()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity)
 {
-    for (uint32_t i = 0; i < MBAR_MAX_POLLS; i++)
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = time_ns();
+    do {
         if (mbar_try_wait(bar, parity)) return true;
+    } while (time_ns() - t0 < MBAR_MAX_NS);
     return false;
 }
 
-// Bounded wait for a thread that is in no hurry (a copy producer far ahead of its consumers): sleeps between polls
-// so that it does not take issue slots from the warps doing the work.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity)
+// For a thread that is in no hurry (a copy producer far ahead of its consumers): sleeps between polls so that it does not take
+// issue slots from the warps doing the work.
+__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, uint32_t sleep_ns = 256)
 {
-    for (uint32_t i = 0; i < MBAR_MAX_POLLS; i++) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = time_ns();
+    do {
+        __nanosleep(sleep_ns);
         if (mbar_try_wait(bar, parity)) return true;
-        __nanosleep(256);
-    }
+    } while (time_ns() - t0 < MBAR_MAX_NS);
     return false;
 }
 
@@ -91,15 +103,16 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta)
 // Bounded wait on a barrier of this CTA that threads of the other CTA arrive on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity)
 {
-    for (uint32_t i = 0; i < MBAR_MAX_POLLS; i++) {
+    const uint64_t t0 = time_ns();
+    do {
         uint32_t ok;
         asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
             : "=r"(ok)
-            : "r"(smem_addr(bar)), "r"(parity), "r"(MBAR_SUSPEND_NS)
+            : "r"(smem_addr(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
-    }
+    } while (time_ns() - t0 < MBAR_MAX_NS);
     return false;
 }
 
@@ -108,6 +121,14 @@ __device__ __forceinline__ int atom_add_acq_rel_cta_shared(int* addr, int v)
 {
     int old;
     asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_addr(addr)), "r"(v) : "memory");
+    return old;
+}
+
+// Global counter update with acquire-release semantics between the CTAs of the device.
+__device__ __forceinline__ int atom_add_acq_rel_gpu(int* addr, int v)
+{
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(addr), "r"(v) : "memory");
     return old;
 }
 

@@ -1,0 +1,145 @@
+// Host side of the decode GEMV / skinny GEMM: work split, shared-memory plan, dispatch on K.
+#include <cstring>
+
+#include "exl3_skinny_kernel.cuh"
+
+namespace exl3 {
+
+static int g_mode_override = -1;
+[[maybe_unused]] static int g_tl_next_slot = 0;
+
+#ifdef EXL3_TIMELINE
+__device__ unsigned long long g_timeline[TL_SLOTS][TL_CTAS][TL_POINTS];
+static unsigned long long* g_tl_base = nullptr;
+extern "C" int exl3_debug_timeline(unsigned long long* host_out, int* next_slot)
+{
+    if (next_slot) *next_slot = g_tl_next_slot;
+    return (int)cudaMemcpyFromSymbol(host_out, g_timeline, sizeof(g_timeline));
+}
+extern "C" void exl3_debug_timeline_reset(void) { g_tl_next_slot = 0; }
+#endif
+
+int gemv_default_mode(int codebook)
+{
+    if (codebook_family(codebook) == FAM_MUL1) return GEMV_PAIRED;
+    return g_mode_override >= 0 ? g_mode_override : GEMV_SPLIT;
+}
+
+void gemv_set_mode_override(int mode) { g_mode_override = mode; }
+
+WorkspaceLayout workspace_layout(int rows, int k, int n_total, int n_shards)
+{
+    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+    const int r = rows < SKINNY_MAX_ROWS ? (rows < 1 ? 1 : rows) : SKINNY_MAX_ROWS;
+    WorkspaceLayout w;
+    w.err_off = 0;
+    w.counters_off = WS_HEADER_BYTES;
+    w.xf_off = WS_SCRATCH_OFF;
+    w.partials_off = up(w.xf_off + (size_t)n_shards * k * operand_pitch(r) * 2 * sizeof(__half));
+    w.total = up(w.partials_off + (size_t)(GEMV_MAX_GRID + n_total / 128) * r * 128 * sizeof(float));
+    return w;
+}
+
+int skinny_init_device()
+{
+    const DeviceInfo* d = current_device_info();
+    if (!d) return EXL3_ERR_NOT_INITIALISED;
+    int rc = skinny_set_attributes_for_k<2>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<3>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<4>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<5>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<6>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<7>(d->max_smem_optin);
+    if (rc == EXL3_OK) rc = skinny_set_attributes_for_k<8>(d->max_smem_optin);
+    return rc;
+}
+
+// Work split and shared-memory plan of one launch; `x`: SK_STREAM or one of the modes that keep a slot of activations per unit.
+static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaunch& l, size_t& smem)
+{
+    memset(&l, 0, sizeof(l));
+    l.a = a;
+    l.KG = a.k / 128;
+    l.NB = a.n_total / 128;
+    const long long units = (long long)l.KG * l.NB;
+    l.grid = units < d->sm_count ? (int)units : d->sm_count;
+    if (l.grid > GEMV_MAX_GRID) l.grid = GEMV_MAX_GRID;
+    l.units_q = (int)(units / l.grid);
+    l.units_r = (int)(units % l.grid);
+    // Stages of whole units.  A bulk copy costs a few hundred nanoseconds whatever its size: copies of 24 KB of weights or a little
+    // more, as long as three such stages fit; a short range travels as one copy.
+    const size_t w = 2048u * (size_t)a.K, f = (size_t)operand_pitch(a.rows) * (a.mode == GEMV_SPLIT ? 512 : 256);
+    const size_t most = (size_t)(l.units_q + (l.units_r ? 1 : 0));
+    const SkRaw raw = sk_raw_planes(x, a.x_glu);
+    const size_t planes = x == SK_STREAM ? 0 : (size_t)(raw.planes_const + a.rows * raw.planes_row);
+    const size_t fixed = SK_BAR_BYTES + (x == SK_STREAM ? 0 : most * f + planes * (most * 256 + 16)) + (size_t)a.rows * 512 + 1024;
+    if (fixed >= (size_t)d->max_smem_optin) return EXL3_ERR_UNSUPPORTED_ROWS;
+    const size_t budget = (size_t)d->max_smem_optin - fixed, unit = w + (x == SK_STREAM ? f : 0);
+    size_t ups = (24 * 1024 + w - 1) / w;
+    if (ups > most) ups = most;
+    while (ups > 2 && budget / (ups * unit) < 3) ups--;      // a ring needs stages of two units or more (see SkWalk)
+    size_t stages = budget / (ups * unit);
+    if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+    const size_t fills = (most + ups - 1) / ups;
+    if (stages < 2 && stages < fills) return EXL3_ERR_UNSUPPORTED_ROWS;
+    // From three rows up the rotation inside saves a launch (3 us) as long as it is one pass of the decode warps and leaves the ring
+    // its three stages: 5120 x 5120, 4 rows: 13.3 against 15.9 us; 17408 x 5120, 4 rows: 34.1 against 29.1 us.
+    if (x == SK_ROTATE && a.rows > SK_FUSED_ROWS && (most > SK_DECODE_WARPS || (stages < 3 && stages < fills))) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (stages > fills) stages = fills;
+    l.stages = (int)stages;
+    l.units_per_stage = (int)ups;
+    l.x_off = (uint32_t)(SK_BAR_BYTES + stages * ups * w);
+    l.r_off = (uint32_t)(l.x_off + (x == SK_STREAM ? stages * ups : most) * f);
+    l.r_plane = (uint32_t)(most * 256 + 16);              // 16 bytes apart in the banks: eight rows are read together
+    l.p_off = (uint32_t)(l.r_off + planes * l.r_plane);
+    // Rows behind the last real one are read from whatever follows (their products are dropped): never past the allocation.
+    smem = l.p_off + (size_t)a.rows * 512 + 1024;
+    const CodebookConst c = codebook_const(a.codebook);
+    l.mul = c.mul;
+    l.add = c.add;
+    l.xf_shard_stride = (long long)l.KG * (long long)f;
+    return EXL3_OK;
+}
+
+bool skinny_rotates_input(const GemvArgs& a)
+{
+    const DeviceInfo* d = current_device_info();
+    if (!d || !a.x || !a.suh || a.rotated || a.rows < 1 || a.rows > SK_ROTATE_ROWS || a.k < 128 || a.n_total < 128) return false;
+    if (a.rows > SK_FUSED_ROWS && (a.norm_weight || a.res_out || a.x_glu)) return false;
+    auto odd = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) != 0; };     // the raw input travels by bulk copies
+    if (odd(a.x) || odd(a.suh) || odd(a.norm_weight)) return false;
+    SkinnyLaunch l;
+    size_t smem;
+    return plan_skinny(a, d, a.norm_weight ? SK_NORM : SK_ROTATE, l, smem) == EXL3_OK;
+}
+
+int launch_skinny(const GemvArgs& a, cudaStream_t st)
+{
+    const DeviceInfo* d = current_device_info();
+    if (!d) return EXL3_ERR_NOT_INITIALISED;
+    if (a.rows < 1 || a.rows > SKINNY_MAX_ROWS) return EXL3_ERR_UNSUPPORTED_ROWS;
+    const long long units = (long long)(a.k / 128) * (a.n_total / 128);
+    if (units == 0) return EXL3_OK;
+    if (units >= (1ll << 30)) return EXL3_ERR_BAD_SHAPE;
+    SkinnyLaunch l;
+    size_t smem = 0;
+    const int x = !a.x ? SK_STREAM : a.norm_weight ? SK_NORM : SK_ROTATE;
+    if (int rc = plan_skinny(a, d, x, l, smem)) return rc;
+#ifdef EXL3_TIMELINE
+    if (!g_tl_base) cudaGetSymbolAddress(reinterpret_cast<void**>(&g_tl_base), g_timeline);
+    l.tl = g_tl_base + (size_t)(g_tl_next_slot++ % TL_SLOTS) * TL_CTAS * TL_POINTS;
+#endif
+    const int pitch = operand_pitch(a.rows);
+    switch (a.K) {
+        case 2: return launch_skinny_for_k<2>(l, pitch, x, smem, st);
+        case 3: return launch_skinny_for_k<3>(l, pitch, x, smem, st);
+        case 4: return launch_skinny_for_k<4>(l, pitch, x, smem, st);
+        case 5: return launch_skinny_for_k<5>(l, pitch, x, smem, st);
+        case 6: return launch_skinny_for_k<6>(l, pitch, x, smem, st);
+        case 7: return launch_skinny_for_k<7>(l, pitch, x, smem, st);
+        case 8: return launch_skinny_for_k<8>(l, pitch, x, smem, st);
+    }
+    return EXL3_ERR_UNSUPPORTED_K;
+}
+
+}  // namespace exl3

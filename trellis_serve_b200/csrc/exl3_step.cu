@@ -55,7 +55,7 @@ __device__ __forceinline__ void load_act4(const void* p, long long i, bool bf16,
 
 // One warp, one (shard, row, 128 block): a[e] are activation values already rounded to the activation type.  They are
 // converted to fp16 as the rotation kernel does, scaled by suh, rotated and stored as fragments.
-// mode 1: split-pair fragments (4 words per lane q), mode 2: paired (2 words); layouts of had_in_kernel.
+// mode 1: split (every value twice), mode 2: paired; layouts of had_in_kernel.
 __device__ __forceinline__ void rotate_store(const float (&a)[4], const __half* suh_blk, uint32_t* xf, int mode, int s, int kts, int rows,
                                              int row, int kg, int lane)
 {
@@ -70,23 +70,12 @@ __device__ __forceinline__ void rotate_store(const float (&a)[4], const __half* 
     uint32_t hv[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) hv[e] = __half_as_ushort(__float2half_rn(v[e] * HAD_SCALE));
-    const int kt = kg * 8 + (lane >> 2);
-    const int rbase = 4 * (lane & 3);
-    if (mode == 1) {
-        uint32_t* o = xf + (((long long)s * kts + kt) * rows + row) * 16;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int r = rbase + e;
-            o[((r & 7) >> 1) * 4 + (r & 1) + 2 * (r >> 3)] = hv[e] | (hv[e] << 16);
-        }
-    } else {
-        uint32_t* o = xf + (((long long)s * kts + kt) * rows + row) * 8;
-#pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-            const int r = rbase + e;
-            o[((r & 7) >> 1) * 2 + (r >> 3)] = hv[e] | (hv[e + 1] << 16);
-        }
-    }
+    const long long at4 = (long long)s * kts * 4 + kg * 32 + lane;
+    const int pitch = operand_pitch(rows);
+    if (mode == 1)
+        reinterpret_cast<uint4*>(xf)[at4 * pitch + row] = make_uint4(hv[0] * 0x10001u, hv[1] * 0x10001u, hv[2] * 0x10001u, hv[3] * 0x10001u);
+    else
+        reinterpret_cast<uint2*>(xf)[((at4 >> 1) * pitch + row) * 2 + (at4 & 1)] = make_uint2(hv[0] | (hv[1] << 16), hv[2] | (hv[3] << 16));
 }
 
 // grid = rows, block = STEP_THREADS.  x [rows, k]; residual [rows, k] or null (in / out); weight [k]; suh [shards, k];

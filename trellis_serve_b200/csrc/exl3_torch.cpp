@@ -141,7 +141,7 @@ at::Tensor linear(const at::Tensor& x, at::TensorList trellis, at::TensorList su
         y = at::empty({rows, n_total}, h.options());
         if (rows > 0) {
             void* st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-            const size_t need = decode ? exl3_linear_workspace_bytes((int)std::min<int64_t>(rows, 16), (int)k, (int)n_total, shards)
+            const size_t need = decode ? exl3_linear_workspace_bytes((int)rows, (int)k, (int)n_total, shards)
                                        : exl3_gemm_tc_workspace_bytes((int)rows, (int)k, (int)n_total, shards);
             const at::Tensor ws = scratch(decode ? 0 : 1, x.device().index(), (int64_t)need);
             auto fn = decode ? exl3_linear : exl3_linear_tc;
@@ -187,7 +187,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> prepare_group(at::TensorList trel
         dst += c.numel() / 2;
     }
     at::Tensor suh_cat = at::stack(suh), svh_cat = at::cat(svh);
-    scratch(0, device.index(), (int64_t)exl3_linear_workspace_bytes((int)std::min<int64_t>(max_rows, 16), (int)kt * 16, (int)nt * 16, (int)trellis.size()));
+    scratch(0, device.index(), (int64_t)exl3_linear_workspace_bytes((int)max_rows, (int)kt * 16, (int)nt * 16, (int)trellis.size()));
     stream.synchronize();
     return {packed, suh_cat, svh_cat};
 }

@@ -76,7 +76,7 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
 
 
 def workspace_bytes(rows: int, k: int, n_total: int, shards: int) -> int:
-    return int(_lib.load().exl3_linear_workspace_bytes(min(rows, 16), k, n_total, shards))
+    return int(_lib.load().exl3_linear_workspace_bytes(rows, k, n_total, shards))
 
 
 def reserve_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
