@@ -48,3 +48,26 @@ def test_rows_and_ring_edges(rows, k, ns, K, cb):
         assert float((got - want).norm() / want.norm()) <= 1e-3
         assert float((got - want).abs().max() / want.pow(2).mean().sqrt()) <= 2e-3
         col += n
+
+
+@pytest.mark.parametrize("rows", [1, 9, 57, 65, 130])
+@pytest.mark.parametrize("x_cols,widths", [(1000, [1000, 130]), (1021, [128, 1]), (8, [7, 256]), (1024, [900, 255])])
+def test_true_sizes_below_the_stored_ones(rows, x_cols, widths):
+    from trellis_serve_b200.runtime import ops
+
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(rows * 7 + x_cols)
+    k, K = 1024, 4
+    ns = [(w + 127) // 128 * 128 for w in widths]
+    trellis = [torch.randint(-32768, 32767, (k // 16, n // 16, 16 * K), dtype=torch.int16, device=DEV, generator=gen) for n in ns]
+    suh = [random_signs(k, gen, DEV, 1).view(-1) for _ in ns]
+    svh = [(random_signs(n, gen, DEV).view(-1) / 64).half() for n in ns]
+    x = torch.randn((rows, x_cols), device=DEV, generator=gen).half()
+    padded = torch.nn.functional.pad(x, (0, k - x_cols))
+    packed, suh_cat, svh_cat, ends = lin.prepare(trellis, suh, svh)
+    whole = ops.linear(padded, [], [], [], [], [], 0, [packed, suh_cat, svh_cat], ends, [0, 0], ns)
+    got = ops.linear(x, [], [], [], [], [], 0, [packed, suh_cat, svh_cat], ends, [0, 0], widths)
+    torch.cuda.synchronize()
+    lin.device_error(DEV)
+    want = torch.cat([whole[:, sum(ns[:i]):sum(ns[:i]) + w] for i, w in enumerate(widths)], 1)
+    assert torch.equal(got, want)

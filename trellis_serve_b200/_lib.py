@@ -52,8 +52,10 @@ SIGNATURES = {
     "exl3_decode_attention": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp, ctypes.c_float, _vp, _sz, _vp, _vp, _i, _vp, _sz, _vp]),
     "exl3_rope_decode_attention": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, ctypes.c_float, _vp, _sz, _vp, _vp, _i, _vp, _sz,
                                         _vp]),
+    "exl3_linear_ragged": (_i, [_vp, _i, _i, _vp, _i, _i, _vp, _vp, _ip, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_prefers_decode": (_i, [_i, _i, _i, _i]),
     "exl3_gemm_tc_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "exl3_linear_tc_padded": (_i, [_vp, _i, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_linear_tc": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_linear_static": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp]),
     "exl3_static_workspace_bytes": (_sz, []),

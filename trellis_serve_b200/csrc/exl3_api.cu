@@ -183,6 +183,10 @@ struct NormArgs {                // consumer of a residual stream: x = z, normal
     const float* ssq;            // [rows, k/128]
     float eps;
 };
+struct RaggedArgs {              // true sizes that are not the stored, padded ones (exl3_linear_ragged)
+    int x_cols;
+    const int* out_widths;       // [n_shards]
+};
 struct ResidualArgs {            // producer: the epilogue adds res_in, writes the new stream and its sums of squares
     const void* res_in;
     void* res_out;
@@ -194,7 +198,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
                          const uint16_t* suh_cat, const uint16_t* svh_cat, const int* shard_ends, int n_shards, int rows, int k,
                          int n_total, void* y, int y_dtype, void* workspace, size_t workspace_bytes, cudaStream_t st, bool rotated,
                          const TpExchange* tp = nullptr, bool prerotated = false, bool glu = false, const NormArgs* norm = nullptr,
-                         const ResidualArgs* res = nullptr)
+                         const ResidualArgs* res = nullptr, const RaggedArgs* ragged = nullptr)
 {
     if (int rc = check_matrix(k, n_total, K, codebook)) return rc;
     if (rows < 0) return EXL3_ERR_BAD_SHAPE;
@@ -208,6 +212,20 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
     if ((size_t)(n_total / 128) > WS_MAX_COUNTERS) return EXL3_ERR_BAD_SHAPE;
     if (!current_device_info()) return EXL3_ERR_NOT_INITIALISED;
     if (!aligned(packed, 16) || (!aligned(y, 16) && !(res && y == nullptr))) return EXL3_ERR_BAD_POINTER;
+    const int x_cols = ragged ? ragged->x_cols : k;
+    int ld_y = n_total;
+    if (ragged) {
+        ld_y = 0;
+        for (int s = 0; s < n_shards; s++) {
+            const int stored = 128 * (a.shard_end_blocks[s] - (s > 0 ? a.shard_end_blocks[s - 1] : 0)), width = ragged->out_widths[s];
+            if (width < 0 || width > stored) return EXL3_ERR_BAD_SHAPE;
+            a.out_first[s] = ld_y;
+            a.out_width[s] = width;
+            ld_y += width;
+        }
+        a.ragged = ld_y != n_total;
+        a.ld_out = ld_y;
+    }
     if (res && (!aligned(res->res_in, 8) || !aligned(res->res_out, 8) || !aligned(res->ssq_out, 4) || res->res_in == res->res_out ||
                 (y_dtype != EXL3_F16 && y_dtype != EXL3_BF16)))
         return EXL3_ERR_BAD_POINTER;
@@ -240,7 +258,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
     for (int r0 = 0, r; r0 < rows; r0 += r) {
         r = rows - r0 < most ? rows - r0 : most;
         a.rows = r;
-        a.out = y ? reinterpret_cast<unsigned char*>(y) + (size_t)r0 * n_total * osz : nullptr;
+        a.out = y ? reinterpret_cast<unsigned char*>(y) + (size_t)r0 * ld_y * osz : nullptr;
         if (res) {
             a.res_in = reinterpret_cast<const unsigned char*>(res->res_in) + (size_t)r0 * n_total * 2;
             a.res_out = reinterpret_cast<unsigned char*>(res->res_out) + (size_t)r0 * n_total * 2;
@@ -270,7 +288,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
         } else {
             // Few rows: the kernel rotates its own input (one launch); otherwise the rotation kernel runs ahead of it.
             // glu: x is gate | up with rows of 2k values and the input proper is silu(gate) * up.
-            const unsigned char* xr = reinterpret_cast<const unsigned char*>(x) + (size_t)r0 * (glu ? 2 * k : k) * esz;
+            const unsigned char* xr = reinterpret_cast<const unsigned char*>(x) + (size_t)r0 * (glu ? 2 * k : x_cols) * esz;
             a.x = xr;
             a.suh = reinterpret_cast<const __half*>(suh_cat);
             a.x_bf16 = x_dtype == EXL3_BF16;
@@ -280,7 +298,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
                 a.ssq_in = norm->ssq + (size_t)r0 * (k / 128);
                 a.norm_eps = norm->eps;
             }
-            if (!skinny_rotates_input(a)) {
+            if (x_cols != k || !skinny_rotates_input(a)) {
                 // The rotation, normalisation or activation kernel ahead of the product, and behind it the stream kernel where the
                 // epilogue does not add the residual.
                 a.x = nullptr;
@@ -290,7 +308,7 @@ static int linear_common(const void* x, int x_dtype, const uint16_t* xh_rowmajor
                 const bool x16 = x_dtype == EXL3_BF16;
                 rc = norm  ? launch_rmsnorm_rotate(xr, nullptr, norm->weight, norm->eps, x16, signs, n_shards, r, k, nullptr, xf, layout, st)
                      : glu ? launch_silu_mul_rotate(xr, x16, signs, r, k, nullptr, xf, layout, st)
-                           : launch_had_in(xr, x16, signs, n_shards, r, k, xf, layout, st);
+                           : launch_had_in(xr, x16, signs, n_shards, r, k, xf, layout, st, x_cols);
                 if (rc) return rc;
                 if (res && r > SK_FUSED_ROWS) {
                     if (!y) return EXL3_ERR_BAD_POINTER;
@@ -316,6 +334,18 @@ exl3_status exl3_linear(const void* x, int x_dtype, const uint32_t* packed, int 
 {
     return linear_common(x, x_dtype, nullptr, packed, K, codebook, suh_cat, svh_cat, shard_ends, n_shards, rows, k, n_total, y,
                          y_dtype, workspace, workspace_bytes, (cudaStream_t)stream, false);
+}
+
+exl3_status exl3_linear_ragged(const void* x, int x_dtype, int x_cols, const uint32_t* packed, int K, int codebook, const uint16_t* suh_cat,
+                               const uint16_t* svh_cat, const int* shard_ends, const int* out_widths, int n_shards, int rows, int k, int n_total,
+                               void* y, int y_dtype, void* workspace, size_t workspace_bytes, void* stream)
+{
+    if (x_cols < 0 || x_cols > k) return EXL3_ERR_BAD_SHAPE;
+    if (!out_widths) return EXL3_ERR_BAD_POINTER;
+    if (y_dtype != EXL3_F16 && y_dtype != EXL3_BF16) return EXL3_ERR_UNSUPPORTED_DTYPE;
+    const RaggedArgs ragged = {x_cols, out_widths};
+    return linear_common(x, x_dtype, nullptr, packed, K, codebook, suh_cat, svh_cat, shard_ends, n_shards, rows, k, n_total, y, y_dtype, workspace,
+                         workspace_bytes, (cudaStream_t)stream, false, nullptr, false, false, nullptr, nullptr, &ragged);
 }
 
 exl3_status exl3_linear_allreduce(const void* x, int x_dtype, const uint32_t* packed, int K, int codebook, const uint16_t* suh_cat,
@@ -601,33 +631,15 @@ exl3_status exl3_rope_decode_attention(const void* qkv, int dtype, int rows, int
 
 static size_t tc_up(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// Fitted to measurements on B200 (microseconds).  The decode kernel streams the weights once per 16 rows: ~14 + 0.38 per million
-// weights for a full chunk, ~0.8 of that for a last chunk of up to 8 rows.  The tensor-core kernel works through its tiles in
-// waves over the SMs at ~1.1 per 64-deep reduction block (~1.6 for the 512-row tiles used above 256 rows); when the tiles are
-// fewer than the SMs the reduction of each is cut into up to 8 parts on CTAs of their own; ~12 more for the two rotation
-// launches, ~8 for adding the parts.
+// Up to 64 rows the decode kernel passes over the weights once and is bound by their decode; measured (microseconds, decode kernel
+// against the tensor-core kernel at 64 rows): 5120 x 5120 25.4 / 30.6, 17408 x 5120 43.8 / 61, 5120 x 34816 76.8 / 118.  From 65 rows
+// up it would pass twice: 5120 x 5120 at 96 rows 48 / 33.
 int exl3_prefers_decode(int rows, int k, int n_total, int sms)
 {
-    const double chunk = 14.0 + 0.38 * ((double)k * n_total / 1e6);
-    const int rem = rows % 16;
-    const double decode = rows / 16 * chunk + (rem == 0 ? 0.0 : chunk * (rem <= 8 ? 0.8 : 1.0));
-    long long tiles;
-    double per_block;
-    if (rows <= 256) {
-        tiles = (long long)((rows + 255) / 256) * (n_total / 256 > 1 ? n_total / 256 : 1);
-        per_block = 1.1;
-    } else {
-        tiles = (long long)((rows + 511) / 512) * (n_total / 128);
-        per_block = 1.6;
-    }
-    const long long one = tiles > 1 ? tiles : 1;
-    long long parts = sms / one;
-    if (parts > 8) parts = 8;
-    if (parts > k / 64) parts = k / 64;
-    if (parts < 1) parts = 1;
-    const long long waves = sms > 0 ? (tiles + sms - 1) / sms : tiles;
-    const double tensor = (double)waves * (k / 64.0) / (double)parts * per_block + 12.0 + (parts > 1 ? 8.0 : 0.0) + 0.08 * (rows < 256 ? rows : 256);
-    return decode <= tensor;
+    (void)k;
+    (void)n_total;
+    (void)sms;
+    return rows <= SKINNY_MAX_ROWS;
 }
 
 size_t exl3_gemm_tc_workspace_bytes(int rows, int k, int n_total, int n_shards)
@@ -641,11 +653,20 @@ exl3_status exl3_linear_tc(const void* x, int x_dtype, const uint32_t* packed, i
                            const uint16_t* svh_cat, const int* shard_ends, int n_shards, int rows, int k, int n_total, void* y,
                            int y_dtype, void* workspace, size_t workspace_bytes, void* stream)
 {
+    return exl3_linear_tc_padded(x, x_dtype, k, packed, K, codebook, suh_cat, svh_cat, shard_ends, n_shards, rows, k, n_total, y, y_dtype, workspace,
+                                 workspace_bytes, stream);
+}
+
+exl3_status exl3_linear_tc_padded(const void* x, int x_dtype, int x_cols, const uint32_t* packed, int K, int codebook, const uint16_t* suh_cat,
+                                  const uint16_t* svh_cat, const int* shard_ends, int n_shards, int rows, int k, int n_total, void* y,
+                                  int y_dtype, void* workspace, size_t workspace_bytes, void* stream)
+{
     if (int rc = check_matrix(k, n_total, K, codebook)) return rc;
     if (rows < 0) return EXL3_ERR_BAD_SHAPE;
     GemvArgs a;
     memset(&a, 0, sizeof(a));
     if (int rc = fill_shards(a, shard_ends, n_shards, n_total)) return rc;
+    if (x_cols < 0 || x_cols > k || (x_cols % 8)) return EXL3_ERR_BAD_SHAPE;
     if ((x_dtype != EXL3_F16 && x_dtype != EXL3_BF16) || (y_dtype != EXL3_F16 && y_dtype != EXL3_BF16)) return EXL3_ERR_UNSUPPORTED_DTYPE;
     if (rows == 0 || k == 0 || n_total == 0) return EXL3_OK;
     if (!current_device_info()) return EXL3_ERR_NOT_INITIALISED;
@@ -657,7 +678,7 @@ exl3_status exl3_linear_tc(const void* x, int x_dtype, const uint32_t* packed, i
     __half* rot = reinterpret_cast<__half*>(ws + 256 + tc_up(gemm_tc_activation_bytes(rows, k, n_shards)));
     float* part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(rot) + tc_up((size_t)rows * n_total * sizeof(__half)));
     TcSplit split = {1, 0, 0, 0};
-    if (int rc = launch_gemm_tc(x, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh_cat), packed, K, codebook, a.shard_end_blocks,
+    if (int rc = launch_gemm_tc(x, x_dtype == EXL3_BF16, x_cols, reinterpret_cast<const __half*>(suh_cat), packed, K, codebook, a.shard_end_blocks,
                                 n_shards, rows, k, n_total, xa, rot, part, y, reinterpret_cast<const __half*>(svh_cat), y_dtype == EXL3_BF16,
                                 &split, reinterpret_cast<int*>(ws), st))
         return rc;

@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
 // lanes that share a column range fill a 128-byte core matrix.  Rows beyond `rows` inside the last group are written as
 // zeros; those up to the next multiple of 512 must have been zero-filled by the caller.
 constexpr int HAD_IN_TC_ROWS = 8;
-__global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int rows, int k,
+__global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_cols, const __half* __restrict__ suh, int shards, int rows, int k,
                                  __half* __restrict__ xa, long long shard_stride)
 {
     const int lane = threadIdx.x & 31;
@@ -734,7 +734,9 @@ __global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, const _
     if (row < rows) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint4 raw = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * k + col)[i];
+            // rows of x are x_cols (a multiple of 8) long, zeros from there to k
+            const uint4 raw = col + 8 * i < x_cols ? reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * x_cols + col)[i]
+                                                   : make_uint4(0u, 0u, 0u, 0u);
             const uint4 sraw = reinterpret_cast<const uint4*>(suh + (long long)s * k + col)[i];
             const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w}, sw[4] = {sraw.x, sraw.y, sraw.z, sraw.w};
 #pragma unroll
@@ -921,7 +923,7 @@ size_t gemm_tc_part_bytes(int rows, int n_total)
     return want < cap ? want : cap;
 }
 
-int launch_gemm_tc(const void* x, int x_bf16, const __half* suh_cat, const uint32_t* packed, int K, int codebook, const int* shard_end_blocks,
+int launch_gemm_tc(const void* x, int x_bf16, int x_cols, const __half* suh_cat, const uint32_t* packed, int K, int codebook, const int* shard_end_blocks,
                    int n_shards, int rows, int k, int n_total, __half* xa, __half* out, float* part, void* y, const __half* svh, int y_bf16, TcSplit* split_out, int* err,
                    cudaStream_t st)
 {
@@ -948,7 +950,7 @@ int launch_gemm_tc(const void* x, int x_bf16, const __half* suh_cat, const uint3
     if (rows % TC_ROWS != 0)
         if (int rc = cuda_status(cudaMemsetAsync(xa, 0, gemm_tc_activation_bytes(rows, k, n_shards), st))) return rc;
     const long long items = (long long)n_shards * ((rows + HAD_IN_TC_ROWS - 1) / HAD_IN_TC_ROWS) * (k / 128);
-    had_in_tc_kernel<<<(unsigned)((items + 7) / 8), 256, 0, st>>>(x, x_bf16, suh_cat, n_shards, rows, k, xa, l.xa_shard_stride);
+    had_in_tc_kernel<<<(unsigned)((items + 7) / 8), 256, 0, st>>>(x, x_bf16, x_cols, suh_cat, n_shards, rows, k, xa, l.xa_shard_stride);
     if (int rc = cuda_status(cudaGetLastError())) return rc;
     // Wide tiles (256 x 256) need column blocks that pair up inside every shard.  They halve the rows that share a decoded
     // weight block, which makes the decode the limiter at large row counts (measured: 823 against 851 TFLOP/s at 2048

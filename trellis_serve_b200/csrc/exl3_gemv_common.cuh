@@ -209,7 +209,18 @@ __device__ __forceinline__ void gemv_finish_row(const GemvArgs& a, uint32_t tp_e
         gemv_residual_store(a, tp_epoch, v, o, m, nb, lane);
         return;
     }
-    if (a.out_dtype == EXL3_F32) {
+    if (a.ragged) {
+        int s = 0;
+        while (s < a.n_shards - 1 && nb >= a.shard_end_blocks[s]) s++;
+        const int c = (nb - (s > 0 ? a.shard_end_blocks[s - 1] : 0)) * 128 + 4 * lane;
+        const float w[4] = {v.x, v.y, v.z, v.w};
+        uint16_t* dst = reinterpret_cast<uint16_t*>(a.out) + (long long)m * a.ld_out + a.out_first[s] + c;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const __half h = __float2half_rn(w[e]);
+            if (c + e < a.out_width[s]) dst[e] = a.out_dtype == EXL3_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(h))) : __half_as_ushort(h);
+        }
+    } else if (a.out_dtype == EXL3_F32) {
         *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) = v;
     } else if (!a.rotated && a.tp.world > 1) {
         gemv_exchange_store(a.tp, tp_epoch, a.out_dtype == EXL3_BF16, v, o, reinterpret_cast<uint16_t*>(a.out), a.err);

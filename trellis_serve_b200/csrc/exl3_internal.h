@@ -27,7 +27,8 @@ int launch_repack(const uint16_t* trellis, int k, int n, int K, uint32_t* packed
 int launch_unpack(const uint32_t* packed, int k, int n, int K, uint16_t* trellis, cudaStream_t st);
 int launch_reconstruct_stored(const uint16_t* trellis, int kt, int nt, int K, int cb, __half* w, cudaStream_t st);
 int launch_reconstruct_packed(const uint32_t* packed, int k, int n, int K, int cb, __half* w, cudaStream_t st);
-int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int rows, int k, void* out, int mode, cudaStream_t st);
+int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int rows, int k, void* out, int mode, cudaStream_t st,
+                  int x_cols = -1);      // x_cols: true row length of x, zeros from there to k (default: k)
 int launch_to_fragments(const __half* xh, int shards, int rows, int k, uint32_t* out, int mode, cudaStream_t st);
 int launch_had_out(const void* y, int y_f32, const __half* svh, int rows, int n, void* out, long long out_stride, int out_bf16,
                    cudaStream_t st);
@@ -88,6 +89,10 @@ struct GemvArgs {
     int shard_end_blocks[GEMV_MAX_SHARDS];   // n-block index where shard s ends (last = NB)
     int out_dtype;              // EXL3_F16 / EXL3_BF16 / EXL3_F32 (fp32 only with the output Hadamard)
     int rotated;                // 1: store the rotated-basis product as fp16, no output Hadamard
+    // ragged: the rows of out are ld_out apart and shard s stores its first out_width[s] columns from column out_first[s] on (true
+    // output widths that are not the stored, padded ones)
+    int ragged, ld_out;
+    int out_first[GEMV_MAX_SHARDS], out_width[GEMV_MAX_SHARDS];
     TpExchange tp;              // world > 1: the output is summed over the ranks inside the kernel
 };
 
@@ -172,7 +177,7 @@ void gemm_tc_set_tiling(int t);             // -1 = choose; 0 = 512 x 128 tiles;
 int gemm_tc_pairs();                        // CTA pairs of the pair tiling that fit on the device at once (0 = tiling unavailable)
 size_t gemm_tc_part_bytes(int rows, int n_total);
 void gemm_tc_set_ksplit(int n);             // 0 = choose; n >= 1 = at most n parts of the reduction per tile
-int launch_gemm_tc(const void* x, int x_bf16, const __half* suh_cat, const uint32_t* packed, int K, int codebook, const int* shard_end_blocks,
+int launch_gemm_tc(const void* x, int x_bf16, int x_cols, const __half* suh_cat, const uint32_t* packed, int K, int codebook, const int* shard_end_blocks,
                    int n_shards, int rows, int k, int n_total, __half* xa, __half* out, float* part, void* y, const __half* svh, int y_bf16, TcSplit* split_out, int* err,
                    cudaStream_t st);
 int launch_had_out_tiles(const float* part, int parts, int tail_first, int row_tiles, const __half* svh, int rows, int n, void* out,

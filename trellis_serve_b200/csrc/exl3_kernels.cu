@@ -196,7 +196,7 @@ __device__ __forceinline__ void store_operand(void* out, long long at4, int rows
 //         row are one 16-byte row of a core matrix).  MODE 2: paired: [shard][k/8][pitch][8 halves].  pitch = operand_pitch(rows).
 template <int MODE>
 __global__ void had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int rows, int k,
-                              void* __restrict__ out)
+                              void* __restrict__ out, int x_cols)
 {
     ptx_grid_launch_dependents();              // the GEMV behind this kernel may start streaming weights already
     ptx_grid_dependency_wait();                // x may be the output of the kernel ahead
@@ -211,7 +211,7 @@ __global__ void had_in_kernel(const void* __restrict__ x, int x_bf16, const __ha
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         int col = kg * 128 + 4 * lane + e;
-        float xv = load_as_f16_value(x, (long long)row * k + col, x_bf16 != 0);
+        const float xv = col < x_cols ? load_as_f16_value(x, (long long)row * x_cols + col, x_bf16 != 0) : 0.f;
         v[e] = suh ? xv * __half2float(suh[(long long)s * k + col]) : xv;
     }
     fwht128(v[0], v[1], v[2], v[3], lane);
@@ -414,8 +414,9 @@ int launch_reconstruct_packed(const uint32_t* packed, int k, int n, int K, int c
     return EXL3_ERR_UNSUPPORTED_K;
 }
 
-int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int rows, int k, void* out, int mode, cudaStream_t st)
+int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int rows, int k, void* out, int mode, cudaStream_t st, int x_cols)
 {
+    if (x_cols < 0) x_cols = k;
     long long items = (long long)shards * rows * (k / 128);
     if (items == 0) return EXL3_OK;
     // programmatic stream serialization: see the GEMV launcher
@@ -428,9 +429,9 @@ int launch_had_in(const void* x, int x_bf16, const __half* suh, int shards, int 
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (mode == 0) return cuda_status(cudaLaunchKernelEx(&cfg, had_in_kernel<0>, x, x_bf16, suh, shards, rows, k, out));
+    if (mode == 0) return cuda_status(cudaLaunchKernelEx(&cfg, had_in_kernel<0>, x, x_bf16, suh, shards, rows, k, out, x_cols));
     auto kernel = mode == 1 ? had_in_kernel<1> : had_in_kernel<2>;
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, x, x_bf16, suh, shards, rows, k, out));
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, x, x_bf16, suh, shards, rows, k, out, x_cols));
 }
 
 int launch_to_fragments(const __half* xh, int shards, int rows, int k, uint32_t* out, int mode, cudaStream_t st)

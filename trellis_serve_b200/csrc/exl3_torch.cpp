@@ -120,42 +120,61 @@ at::Tensor linear(const at::Tensor& x, at::TensorList trellis, at::TensorList su
     at::Tensor h = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
     if (h.scalar_type() != at::kHalf && h.scalar_type() != at::kBFloat16) h = h.to(at::kHalf);
     TORCH_CHECK(h.size(1) <= k, "input width ", h.size(1), " exceeds the stored width ", k);
-    if (h.size(1) < k) h = at::constant_pad_nd(h, {0, k - h.size(1)});        // stored input width is padded to 128
-    h = h.contiguous();
     const int64_t rows = h.size(0);
     std::vector<int64_t> bounds(shards + 1, 0);
-    int ends[8];
+    int ends[8], widths[8];
     for (int s = 0; s + 1 < shards; s++) {
         bounds[s + 1] = marlin_ends[s];
         ends[s] = (int)marlin_ends[s];
     }
     bounds[shards] = n_total;
+    bool whole = (int)out_widths.size() == shards, wider = !whole;
+    int64_t n_out = 0;
+    for (int s = 0; s < shards && s < (int)out_widths.size(); s++) {
+        whole = whole && out_widths[s] == bounds[s + 1] - bounds[s];
+        wider = wider || out_widths[s] > bounds[s + 1] - bounds[s] || out_widths[s] < 0;
+        widths[s] = (int)out_widths[s];
+        n_out += out_widths[s];
+    }
+    TORCH_CHECK((int)out_widths.size() <= shards, "more output widths than matrices");
 
-    at::Tensor y;
     const bool decode = g_knob[0] > 0 ? rows < g_knob[0] : exl3_prefers_decode((int)rows, (int)k, (int)n_total, sms) != 0;
-    if (!decode && (!dense.empty() || g_knob[1] != 0)) {
+    const bool library = !decode && (!dense.empty() || g_knob[1] != 0);
+    // Stored input width is padded to 128: the kernels read rows of the true width (the many-row one in steps of eight columns).
+    h = h.contiguous();
+    if (h.size(1) < k && (library || h.size(1) == 0 || (!decode && (h.size(1) % 8 != 0 || reinterpret_cast<uintptr_t>(h.const_data_ptr()) % 16 != 0))))
+        h = at::constant_pad_nd(h, {0, k - h.size(1)});
+    const int x_cols = (int)h.size(1);
+    at::Tensor y;
+    bool trimmed = whole;                                    // y has the true output columns
+    if (library) {
         // resident decoded weights, or the decode + library GEMM sequence asked for: runtime/ops.py
         static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("exl3_b200::dense_linear", "");
         y = op.typed<at::Tensor(const at::Tensor&, at::TensorList, at::TensorList, at::IntArrayRef, int64_t)>().call(h, dense, marlin_w, marlin_ends, cb);
     } else {
-        y = at::empty({rows, n_total}, h.options());
+        const bool ragged = decode && !wider && !whole && n_out > 0;
+        y = at::empty({rows, ragged ? n_out : n_total}, h.options());
+        if (ragged) trimmed = true;
         if (rows > 0) {
             void* st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
             const size_t need = decode ? exl3_linear_workspace_bytes((int)rows, (int)k, (int)n_total, shards)
                                        : exl3_gemm_tc_workspace_bytes((int)rows, (int)k, (int)n_total, shards);
             const at::Tensor ws = scratch(decode ? 0 : 1, x.device().index(), (int64_t)need);
-            auto fn = decode ? exl3_linear : exl3_linear_tc;
-            check(fn(h.const_data_ptr(), dtype_code(h), static_cast<const uint32_t*>(packed.const_data_ptr()), K, cb, u16(suh_cat), u16(svh_cat), ends,
-                     shards, (int)rows, (int)k, (int)n_total, y.mutable_data_ptr(), dtype_code(y), ws.mutable_data_ptr(), (size_t)ws.numel(), st),
-                  decode ? "exl3_linear" : "exl3_linear_tc");
+            const uint32_t* w = static_cast<const uint32_t*>(packed.const_data_ptr());
+            if (decode) {
+                if (!ragged)
+                    for (int s = 0; s < shards; s++) widths[s] = (int)(bounds[s + 1] - bounds[s]);
+                check(exl3_linear_ragged(h.const_data_ptr(), dtype_code(h), x_cols, w, K, cb, u16(suh_cat), u16(svh_cat), ends, widths, shards, (int)rows,
+                                         (int)k, (int)n_total, y.mutable_data_ptr(), dtype_code(y), ws.mutable_data_ptr(), (size_t)ws.numel(), st),
+                      "exl3_linear");
+            } else {
+                check(exl3_linear_tc_padded(h.const_data_ptr(), dtype_code(h), x_cols, w, K, cb, u16(suh_cat), u16(svh_cat), ends, shards, (int)rows,
+                                            (int)k, (int)n_total, y.mutable_data_ptr(), dtype_code(y), ws.mutable_data_ptr(), (size_t)ws.numel(), st),
+                      "exl3_linear_tc");
+            }
         }
     }
-    bool whole = (int)out_widths.size() == shards;
-    for (int s = 0; whole && s < shards; s++) whole = out_widths[s] == bounds[s + 1] - bounds[s];
-    if (!whole) {
-        TORCH_CHECK((int)out_widths.size() <= shards, "more output widths than matrices");
-        y = trim(y, bounds, out_widths);
-    }
+    if (!trimmed) y = trim(y, bounds, out_widths);
     if (y.scalar_type() != x.scalar_type()) y = y.to(x.scalar_type());
     if (x.dim() == 2) return y;
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());

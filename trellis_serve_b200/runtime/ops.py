@@ -14,14 +14,14 @@ compilers see only shapes.
 
 Dispatch (there is a single backend, so the reference's ladder, ops.py:79-95, collapses to two paths):
 
-  few rows                  fused decode kernel (weights streamed once per 16 rows)
+  few rows                  fused decode kernel (up to 64: weights streamed once)
   many rows                 many-row path: the fused tcgen05 kernel (`kernels.linear.run_tc`: weights decoded once per
                             512 rows into the tensor-core operand); when resident decoded weights are passed in `dense`,
                             `dense_group` instead (batched input rotation, library fp16 GEMM on the resident weight,
                             output rotation), which is the reference's many-row sequence
 
-x may have any leading dims; a last dim narrower than the stored (128-padded) k is zero-padded (ops.py:98-99) and
-stored output columns beyond the true `out_widths` are dropped (ops.py:122-124).  fp16 / bf16 go through as they are;
+x may have any leading dims; a last dim narrower than the stored (128-padded) k reads as zero-padded (ops.py:98-99) and
+stored output columns beyond the true `out_widths` are dropped (ops.py:122-124), up to 64 rows without a copy for either.  fp16 / bf16 go through as they are;
 any other dtype is computed in fp16 and cast back.
 """
 from __future__ import annotations
