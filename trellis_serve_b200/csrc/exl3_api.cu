@@ -715,14 +715,13 @@ namespace exl3 {
 struct MoeWorkspace {
     size_t counters_off, partials_off, total;
 };
-static MoeWorkspace moe_workspace(int cap, int n_total)
+static MoeWorkspace moe_workspace()
 {
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t col_blocks = (size_t)(cap / MOE_BLOCK_ROWS) * (n_total / 128);
     MoeWorkspace w;
     w.counters_off = WS_HEADER_BYTES;
     w.partials_off = WS_SCRATCH_OFF;
-    w.total = up(w.partials_off + (GEMV_MAX_GRID + col_blocks) * MOE_BLOCK_ROWS * 128 * sizeof(float));
+    w.total = up(w.partials_off + (size_t)2 * MOE_MAX_GRID * MOE_BLOCK_ROWS * 128 * sizeof(float));
     return w;
 }
 }  // namespace exl3
@@ -745,8 +744,8 @@ exl3_status exl3_moe_align(const int32_t* topk_ids, int slots, int num_experts, 
     if ((size_t)cap < exl3_moe_sorted_capacity(slots, num_experts)) return EXL3_ERR_BAD_SHAPE;
     if (!aligned(num_post, 4) || (slots > 0 && !aligned(topk_ids, 4)) || (cap > 0 && (!aligned(sorted_ids, 4) || !aligned(expert_ids, 4))))
         return EXL3_ERR_BAD_POINTER;
-    return launch_moe_align(topk_ids, slots, num_experts, MOE_BLOCK_ROWS, cap, sorted_ids, expert_ids, num_post, nullptr, 0,
-                            (cudaStream_t)stream);
+    return launch_moe_align(topk_ids, slots, num_experts, MOE_BLOCK_ROWS, cap, sorted_ids, expert_ids, num_post, nullptr, 0, 0,
+                            nullptr, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 exl3_status exl3_moe_align_mapped(const int32_t* topk_ids, int slots, int num_experts, const int32_t* expert_map, int num_local,
@@ -758,7 +757,7 @@ exl3_status exl3_moe_align_mapped(const int32_t* topk_ids, int slots, int num_ex
         (cap > 0 && (!aligned(sorted_ids, 4) || !aligned(expert_ids, 4))))
         return EXL3_ERR_BAD_POINTER;
     return launch_moe_align(topk_ids, slots, num_local, MOE_BLOCK_ROWS, cap, sorted_ids, expert_ids, num_post, expert_map, num_experts,
-                            (cudaStream_t)stream);
+                            0, nullptr, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 size_t exl3_moe_fragment_bytes(int cap, int k, int shards, int codebook)
@@ -778,7 +777,8 @@ exl3_status exl3_moe_had_in(const void* x, int x_dtype, const uint16_t* suh, int
     if (!aligned(x, 2) || !aligned(suh, 2) || !aligned(xf, 16) || !aligned(sorted_ids, 4) || !aligned(expert_ids, 4) || !aligned(num_post, 4))
         return EXL3_ERR_BAD_POINTER;
     return launch_moe_had_in(x, x_dtype == EXL3_BF16, reinterpret_cast<const __half*>(suh), shards, hidden, top_k, slots, cap, sorted_ids,
-                             expert_ids, num_post, xf, gemv_default_mode(codebook), (cudaStream_t)stream);
+                             expert_ids, num_post, xf, (long long)exl3_moe_fragment_bytes(cap, hidden, 1, codebook),
+                             gemv_default_mode(codebook), (cudaStream_t)stream);
 }
 
 exl3_status exl3_moe_glu_had_in(const uint16_t* gu, const uint16_t* suh2, int inter, int slots, const int32_t* sorted_ids, int cap,
@@ -796,7 +796,7 @@ exl3_status exl3_moe_glu_had_in(const uint16_t* gu, const uint16_t* suh2, int in
 size_t exl3_moe_workspace_bytes(int cap, int n_total)
 {
     if (cap < 0 || n_total < 0) return 0;
-    return moe_workspace(cap, n_total).total;
+    return moe_workspace().total;
 }
 
 exl3_status exl3_moe_gemm(const uint32_t* xf, const uint32_t* packed, int K, int codebook, const uint16_t* svh, const int32_t* sorted_ids,
@@ -806,25 +806,25 @@ exl3_status exl3_moe_gemm(const uint32_t* xf, const uint32_t* packed, int K, int
     if (int rc = check_matrix(k, n_total, K, codebook)) return rc;
     if (cap < 0 || (cap % MOE_BLOCK_ROWS) || slots < 0 || shard_end < 0 || shard_end > n_total || (shard_end % 128)) return EXL3_ERR_BAD_SHAPE;
     if (cap == 0 || k == 0 || n_total == 0) return EXL3_OK;
-    if ((size_t)(cap / MOE_BLOCK_ROWS) * (size_t)(n_total / 128) > WS_MAX_COUNTERS) return EXL3_ERR_BAD_SHAPE;
     if (!current_device_info()) return EXL3_ERR_NOT_INITIALISED;
     if (!aligned(xf, 16) || !aligned(packed, 16) || !aligned(out, 8) || (svh && !aligned(svh, 8)) || !aligned(sorted_ids, 4) ||
         !aligned(expert_ids, 4) || !aligned(num_post, 4))
         return EXL3_ERR_BAD_POINTER;
-    const MoeWorkspace wl = moe_workspace(cap, n_total);
+    const MoeWorkspace wl = moe_workspace();
     if (!aligned(workspace, 256) || workspace_bytes < wl.total) return EXL3_ERR_WORKSPACE;
     unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
     MoeGemmLaunch l;
     memset(&l, 0, sizeof(l));
     l.packed = packed;
     l.expert_stride = (long long)k * n_total * K / 32;
-    l.xf = xf;
-    l.xf_shard_stride = (long long)(cap / MOE_BLOCK_ROWS) * (k / 16) * 32;
+    l.xf = reinterpret_cast<const unsigned char*>(xf);
+    l.xf_shard_stride = (long long)exl3_moe_fragment_bytes(cap, k, 1, codebook);
+    l.slab_rows = MOE_BLOCK_ROWS;
     l.svh = reinterpret_cast<const __half*>(svh);
     l.out = reinterpret_cast<__half*>(out);
     l.sorted_ids = sorted_ids;
     l.expert_ids = expert_ids;
-    l.num_post = num_post;
+    l.counts = num_post;
     l.partials = reinterpret_cast<float*>(ws + wl.partials_off);
     l.counters = reinterpret_cast<int*>(ws + wl.counters_off);
     l.err = reinterpret_cast<int*>(ws);

@@ -310,28 +310,58 @@ __device__ __forceinline__ void fwht128(float& v0, float& v1, float& v2, float& 
 // per warp): five stages stay inside the lane and only two cross lanes, 64 shuffles for eight rows where the layout above
 // needs 160 -- the shuffle unit is what bounds the rotation kernels of the many-row paths.  Same stage order (strides 1, 2, ...,
 // 64) and the same sums and differences, so the results are the same bits.
+// Pairs of elements travel through the packed fp32 instructions of sm_100 (a - b as fma(b, -1, a): one rounding, the same bits), which
+// halves the additions: 280 instructions per eight rows instead of 450.
+__device__ __forceinline__ unsigned long long f32x2(float a, float b)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f32x2_split(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ unsigned long long f32x2_add(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long f32x2_fma(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane)
 {
+    unsigned long long p[16];
+    const unsigned long long minus = f32x2(-1.f, -1.f);
 #pragma unroll
-    for (int stride = 1; stride < 32; stride <<= 1) {
+    for (int i = 0; i < 16; i++) p[i] = f32x2(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
+    for (int stride = 1; stride < 16; stride <<= 1) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
             if ((i & stride) == 0) {
-                const float lo = v[i], hi = v[i + stride];
-                v[i] = lo + hi;
-                v[i + stride] = lo - hi;
+                const unsigned long long lo = p[i], hi = p[i + stride];
+                p[i] = f32x2_add(lo, hi);
+                p[i + stride] = f32x2_fma(hi, minus, lo);
             }
         }
     }
 #pragma unroll
     for (int m = 1; m < 4; m <<= 1) {
-        const bool upper = (lane & m) != 0;
+        const float sign = (lane & m) != 0 ? -1.f : 1.f;
+        const unsigned long long sign2 = f32x2(sign, sign);
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
-            const float p = __shfl_xor_sync(0xFFFFFFFFu, v[i], m);
-            v[i] = upper ? p - v[i] : v[i] + p;
+        for (int i = 0; i < 16; i++) {
+            float a, b;
+            f32x2_split(p[i], a, b);
+            p[i] = f32x2_fma(p[i], sign2, f32x2(__shfl_xor_sync(0xFFFFFFFFu, a, m), __shfl_xor_sync(0xFFFFFFFFu, b, m)));
         }
     }
+#pragma unroll
+    for (int i = 0; i < 16; i++) f32x2_split(p[i], v[2 * i], v[2 * i + 1]);
 }
 
 constexpr float HAD_SCALE = 0.08838834764831845f;   // 1 / sqrt(128)

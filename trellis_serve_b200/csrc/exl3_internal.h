@@ -114,11 +114,18 @@ inline int rotated_layout(int gemv_mode) { return gemv_mode == GEMV_SPLIT ? 1 : 
 struct MoeGemmLaunch;
 int moe_init_device();
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, cudaStream_t st);
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* counters, cudaStream_t st);
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
-                      const int* sorted_ids, const int* expert_ids, const int* num_post, uint32_t* xf, int mode, cudaStream_t st);
-int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
-                          const int* expert_ids, const int* num_post, uint32_t* xf, int mode, cudaStream_t st);
+                      const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st);
+int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids, const int* expert_ids,
+                          const int* num_post, void* xf, int mode, cudaStream_t st);
+// Long items (see exl3_moe_tc.cu).
+int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
+                            const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st);
+int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
+                         const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st);
+int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
+                         const int* num_post, __half* yd, cudaStream_t st);
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,
                        int y_bf16, cudaStream_t st);
 
@@ -158,7 +165,7 @@ int launch_gemm_tc_grouped(const uint32_t* packed, long long expert_stride, int 
                            int* err, cudaStream_t st);
 // exl3_moe_tc.cu: routed experts through the grouped tensor-core GEMM (many rows per expert)
 constexpr int MOE_TC_BLOCK_ROWS = 128;
-size_t moe_tc_capacity(int slots, int num_local);
+
 size_t moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter);
 int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int inter, const int* topk_ids, int slots, int num_experts,
                           const int* expert_map, int num_local, const uint32_t* w13, const __half* suh13, const __half* svh13,

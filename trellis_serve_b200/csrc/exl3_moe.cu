@@ -21,9 +21,12 @@ __device__ __forceinline__ int moe_mapped_id(const int* topk_ids, int i, const i
     return (e >= 0 && e < E_global) ? expert_map[e] : -1;
 }
 
+// With `items`: every expert's rows are also cut into items of up to item_blocks blocks of eight rows; items[i] = (expert, first block,
+// blocks, 0), blk[b] = (first block of the item of block b, its blocks), num_post[1] = items, num_post[2] = rows of the largest one; and
+// the counters of the grouped GEMM, and its error word ahead of them, are cleared.  One CTA: bound by latency, so the ids are requested eight at a time per thread.
 __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
                                  int* __restrict__ expert_ids, int* __restrict__ num_post, const int* __restrict__ expert_map,
-                                 int E_global)
+                                 int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ counters)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -31,199 +34,419 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, in
     int* count = sh;              // [E]
     int* offset = sh + E;         // [E + 1]
     int* fill = sh + 2 * E + 1;   // [E]
+    constexpr int BATCH = 8;
+    auto each_id = [&](auto use) {                      // use(slot, expert) for every slot of an expert in [0, E)
+        for (int i0 = threadIdx.x; i0 < numel; i0 += BATCH * blockDim.x) {
+            int e[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; j++) {
+                const int i = i0 + j * blockDim.x;
+                e[j] = i < numel ? moe_mapped_id(topk_ids, i, expert_map, E_global) : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < BATCH; j++)
+                if (e[j] >= 0 && e[j] < E) use(i0 + j * (int)blockDim.x, e[j]);
+        }
+    };
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         count[e] = 0;
         fill[e] = 0;
     }
+    if (items)
+        for (int i = threadIdx.x; i < MOE_MAX_GRID + MOE_ERR_WORDS; i += blockDim.x) counters[i - MOE_ERR_WORDS] = 0;      // and the error word ahead of them
     __syncthreads();
-    for (int i = threadIdx.x; i < numel; i += blockDim.x) {
-        const int e = moe_mapped_id(topk_ids, i, expert_map, E_global);
-        if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+    each_id([&](int, int e) { atomicAdd(&count[e], 1); });
+    for (int i = threadIdx.x; i < cap; i += blockDim.x) sorted_ids[i] = numel;
+    // Exclusive prefix sums of the padded counts and (high word) of the items: warp scans by shuffle, warp totals through shared
+    // memory; experts are taken in chunks of blockDim.x with a running carry.
+    __shared__ unsigned long long warp_total[32];
+    __shared__ unsigned long long carry_sh;
+    __shared__ int largest;
+    if (threadIdx.x == 0) {
+        carry_sh = 0;
+        largest = 0;
     }
-    __syncthreads();
-    // Exclusive prefix sum of the padded counts: warp scans by shuffle, warp totals through shared memory; experts are
-    // taken in chunks of blockDim.x with a running carry.
-    __shared__ int warp_total[32];
-    __shared__ int carry_sh;
-    if (threadIdx.x == 0) carry_sh = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     for (int e0 = 0; e0 < E; e0 += blockDim.x) {
         const int e = e0 + threadIdx.x;
-        const int padded = e < E ? (count[e] + block - 1) / block * block : 0;
-        int incl = padded;
+        const int blocks = e < E ? (count[e] + block - 1) / block : 0;
+        const int n_items = items ? (blocks + item_blocks - 1) / item_blocks : 0;
+        const unsigned long long own = (unsigned long long)(blocks * block) | ((unsigned long long)n_items << 32);
+        unsigned long long incl = own;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
             if (lane >= d) incl += up;
         }
         if (lane == 31) warp_total[wid] = incl;
         __syncthreads();
         if (wid == 0) {
-            int t = lane < nwarps ? warp_total[lane] : 0;
+            unsigned long long t = lane < nwarps ? warp_total[lane] : 0;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
-                const int up = __shfl_up_sync(0xFFFFFFFFu, t, d);
+                const unsigned long long up = __shfl_up_sync(0xFFFFFFFFu, t, d);
                 if (lane >= d) t += up;
             }
             warp_total[lane] = t;                      // inclusive totals of the warps
         }
         __syncthreads();
-        const int base = carry_sh + (wid > 0 ? warp_total[wid - 1] : 0);
-        if (e < E) offset[e] = base + incl - padded;
+        const unsigned long long base = carry_sh + (wid > 0 ? warp_total[wid - 1] : 0);
+        const unsigned long long excl = base + incl - own;
+        if (e < E) {
+            const int b0 = (int)(excl & 0xFFFFFFFFu) / block;
+            offset[e] = b0 * block;
+            for (int r = 0; r < blocks; r++) expert_ids[b0 + r] = e;
+            if (items) {
+                // the expert's blocks in nearly even items
+                int at = (int)(excl >> 32), first = 0;
+                for (int i = 0; i < n_items; i++) {
+                    const int len = (blocks - first + n_items - i - 1) / (n_items - i);
+                    items[at + i] = make_int4(e, b0 + first, len, 0);
+                    for (int r = 0; r < len; r++) blk[b0 + first + r] = make_int2(b0 + first, len);
+                    if (i == 0) atomicMax(&largest, len * block);      // the first is the largest
+                    first += len;
+                }
+            }
+        }
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) carry_sh = base + incl;
         __syncthreads();
     }
+    const int total = (int)(carry_sh & 0xFFFFFFFFu);
     if (threadIdx.x == 0) {
-        offset[E] = carry_sh;
-        *num_post = carry_sh;
+        num_post[0] = total;
+        if (items) {
+            num_post[1] = (int)(carry_sh >> 32);
+            num_post[2] = largest;
+        }
     }
-    __syncthreads();
-    const int total = offset[E];
-    for (int i = threadIdx.x; i < cap; i += blockDim.x) sorted_ids[i] = numel;
-    for (int e = threadIdx.x; e < E; e += blockDim.x)
-        for (int r = offset[e]; r < offset[e + 1]; r += block) expert_ids[r / block] = e;
     for (int i = total / block + threadIdx.x; i < cap / block; i += blockDim.x) expert_ids[i] = -1;
-    __syncthreads();
-    for (int i = threadIdx.x; i < numel; i += blockDim.x) {
-        const int e = moe_mapped_id(topk_ids, i, expert_map, E_global);
-        if (e >= 0 && e < E) sorted_ids[offset[e] + atomicAdd(&fill[e], 1)] = i;
+    each_id([&](int i, int e) { sorted_ids[offset[e] + atomicAdd(&fill[e], 1)] = i; });
+}
+
+// ------------------------------------------------------------------------------------------------ rotations
+
+// A lane's 32 values of a row, four lanes per row, in the B-operand layout of the grouped GEMM (k chunk by k chunk of eight, a 16-byte word
+// per row, `rows` rows): the warp's stores fill 128-byte lines.
+__device__ __forceinline__ void moe_store_rows(unsigned char* unit, int rows, int row, int q, const float (&v)[32])
+{
+    unsigned char* dst = unit + ((size_t)(q * 4) * rows + row) * 16;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const __half2 h = __floats2half2_rn(v[8 * j + 2 * i] * HAD_SCALE, v[8 * j + 2 * i + 1] * HAD_SCALE);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(dst + (size_t)j * rows * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// ------------------------------------------------------------------------------------------------ fragments
-
-template <int MODE>
-__device__ __forceinline__ void store_fragments(uint32_t* out, long long elem_base, int lane, const __half (&h)[4])
+// 32 halves (16-byte aligned) as packed words.
+__device__ __forceinline__ void moe_load32(const void* base, long long at, uint32_t (&w)[16])
 {
-    // lane holds rows r = 4*(lane&3) + e of 16-row tile lane/4; element = ((kt * 8 + row) * 4 + q), FW words each
-    constexpr int FW = gemv_frag_words(MODE);
-    const int rbase = 4 * (lane & 3);
-    if constexpr (MODE == GEMV_SPLIT) {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int r = rbase + e, q = (r & 7) >> 1, slot = (r & 1) + 2 * (r >> 3);
-            const uint32_t hv = __half_as_ushort(h[e]);
-            out[(elem_base + q) * FW + slot] = hv | (hv << 16);
-        }
+    for (int i = 0; i < 4; i++) {
+        const uint4 r = src[i];
+        w[4 * i] = r.x;
+        w[4 * i + 1] = r.y;
+        w[4 * i + 2] = r.z;
+        w[4 * i + 3] = r.w;
+    }
+}
+__device__ __forceinline__ float moe_half(const uint32_t (&w)[16], int i)
+{
+    const __half2 h = *reinterpret_cast<const __half2*>(&w[i >> 1]);
+    return i & 1 ? __high2float(h) : __low2float(h);
+}
+
+// One row per warp, four values per lane, into the same layout (fwht128's lane order).
+template <int MODE>
+__device__ __forceinline__ void moe_store_row(unsigned char* unit, int rows, int row, int lane, const float (&v)[4])
+{
+    uint32_t h[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) h[e] = __half_as_ushort(__float2half_rn(v[e] * HAD_SCALE));
+    if constexpr (MODE == GEMV_SPLIT)
+        *reinterpret_cast<uint4*>(unit + (size_t)(lane * rows + row) * 16) = make_uint4(h[0] * 0x10001u, h[1] * 0x10001u, h[2] * 0x10001u, h[3] * 0x10001u);
+    else
+        *reinterpret_cast<uint2*>(unit + (size_t)((lane >> 1) * rows + row) * 16 + (lane & 1) * 8) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+}
+__device__ __forceinline__ void moe_load4(const void* base, long long at, bool bf16, float (&v)[4])
+{
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(base) + at;
+    uint16_t r[4];
+    if ((reinterpret_cast<uintptr_t>(src) & 7) == 0) {
+        const uint2 w = *reinterpret_cast<const uint2*>(src);
+        r[0] = (uint16_t)w.x;
+        r[1] = (uint16_t)(w.x >> 16);
+        r[2] = (uint16_t)w.y;
+        r[3] = (uint16_t)(w.y >> 16);
     } else {
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-            const int r = rbase + e, q = (r & 7) >> 1, slot = r >> 3;
-            out[(elem_base + q) * FW + slot] = (uint32_t)__half_as_ushort(h[e]) | ((uint32_t)__half_as_ushort(h[e + 1]) << 16);
-        }
+        for (int e = 0; e < 4; e++) r[e] = src[e];
     }
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = bf16 ? __half2float(__float2half_rn(__bfloat162float(__ushort_as_bfloat16(r[e])))) : __half2float(__ushort_as_half(r[e]));
 }
 
-// xf[shard][position p][k tile][q] = fragments of Had128(fp16(x[token(p)]) * suh[expert(p), shard]); zero rows for padding.
-// One warp per (shard, p, 128-block).  Positions at or beyond num_post are left untouched.
+// Decode-sized batches, where most rows of a block of eight are padding: one warp per (row, 128 columns), as little code as possible
+// (run once per launch it is bound by instruction fetch: 5 us against 7 with the form below for one token).
 template <int MODE>
-__global__ void moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int hidden, int top_k,
-                                  int numel, int cap, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
-                                  const int* __restrict__ num_post, uint32_t* __restrict__ xf)
+__global__ void __launch_bounds__(256) moe_had_in_rows_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int hidden,
+                                                              int top_k, int numel, int cap, const int* __restrict__ sorted_ids,
+                                                              const int* __restrict__ expert_ids, const int* __restrict__ num_post,
+                                                              unsigned char* __restrict__ xf, long long shard_stride)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    const int lane = threadIdx.x & 31;
-    const int kgs = hidden >> 7, KT = hidden >> 4;
-    const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long long)shards * cap * kgs) return;
-    const int kg = (int)(item % kgs);
-    const int p = (int)((item / kgs) % cap);
-    const int s = (int)(item / ((long long)kgs * cap));
-    if (p >= *num_post) return;
-    const int slot = sorted_ids[p];
-    const int b = p / MOE_BLOCK_ROWS, row = p % MOE_BLOCK_ROWS;
-    __half h[4];
-    if (slot < 0 || slot >= numel) {
-#pragma unroll
-        for (int e = 0; e < 4; e++) h[e] = __ushort_as_half(0);
-    } else {
-        const int token = slot / top_k, ex = expert_ids[b];
+    constexpr int F_ROW = MODE == GEMV_SPLIT ? 512 : 256;
+    const int lane = threadIdx.x & 31, kgs = hidden >> 7;
+    const long long at = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (at >= (long long)cap * kgs) return;
+    const int row = (int)(at / kgs), kg = (int)(at - (long long)row * kgs), b = row / MOE_BLOCK_ROWS;
+    const int post = *num_post, slot = sorted_ids[row], ex = expert_ids[b];
+    if (row >= post || slot < 0 || slot >= numel) return;
+    float a[4];
+    moe_load4(x, (long long)(slot / top_k) * hidden + kg * 128 + 4 * lane, x_bf16 != 0, a);
+    for (int s = 0; s < shards; s++) {
         float v[4];
+        moe_load4(suh, ((long long)ex * shards + s) * hidden + kg * 128 + 4 * lane, false, v);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int col = kg * 128 + 4 * lane + e;
-            float xv = x_bf16 ? __half2float(__float2half_rn(__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[(long long)token * hidden + col])))
-                              : __half2float(reinterpret_cast<const __half*>(x)[(long long)token * hidden + col]);
-            v[e] = xv * __half2float(suh[((long long)ex * shards + s) * hidden + col]);
-        }
+        for (int e = 0; e < 4; e++) v[e] *= a[e];
         fwht128(v[0], v[1], v[2], v[3], lane);
-#pragma unroll
-        for (int e = 0; e < 4; e++) h[e] = __float2half_rn(v[e] * HAD_SCALE);
+        moe_store_row<MODE>(xf + s * shard_stride + ((long long)b * kgs + kg) * MOE_BLOCK_ROWS * F_ROW, MOE_BLOCK_ROWS, row % MOE_BLOCK_ROWS, lane, v);
     }
-    const int kt = kg * 8 + (lane >> 2);
-    const long long elem_base = (((long long)s * (cap / MOE_BLOCK_ROWS) + b) * KT + kt) * 32 + row * 4;
-    store_fragments<MODE>(xf, elem_base, lane, h);
 }
 
-// xd fragments = Had128( fp16( silu(gate) * up ) * suh2[expert] ) per position; gu is [slots][2*inter] fp16.
 template <int MODE>
-__global__ void moe_glu_had_in_kernel(const __half* __restrict__ gu, const __half* __restrict__ suh2, int inter, int numel, int cap,
-                                      const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
-                                      const int* __restrict__ num_post, uint32_t* __restrict__ xf)
+__global__ void __launch_bounds__(256) moe_glu_had_in_rows_kernel(const __half* __restrict__ gu, const __half* __restrict__ suh2, int inter, int numel, int cap,
+                                                                  const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+                                                                  const int* __restrict__ num_post, unsigned char* __restrict__ xf)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    const int lane = threadIdx.x & 31;
-    const int kgs = inter >> 7, KT = inter >> 4;
-    const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long long)cap * kgs) return;
-    const int kg = (int)(item % kgs);
-    const int p = (int)(item / kgs);
-    if (p >= *num_post) return;
-    const int slot = sorted_ids[p];
-    const int b = p / MOE_BLOCK_ROWS, row = p % MOE_BLOCK_ROWS;
-    __half h[4];
-    if (slot < 0 || slot >= numel) {
+    constexpr int F_ROW = MODE == GEMV_SPLIT ? 512 : 256;
+    const int lane = threadIdx.x & 31, kgs = inter >> 7;
+    const long long at = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (at >= (long long)cap * kgs) return;
+    const int row = (int)(at / kgs), kg = (int)(at - (long long)row * kgs), b = row / MOE_BLOCK_ROWS;
+    const int post = *num_post, slot = sorted_ids[row], ex = expert_ids[b];
+    if (row >= post || slot < 0 || slot >= numel) return;
+    const int col = kg * 128 + 4 * lane;
+    float g[4], u[4], v[4];
+    moe_load4(gu, (long long)slot * 2 * inter + col, false, g);
+    moe_load4(gu, (long long)slot * 2 * inter + inter + col, false, u);
+    moe_load4(suh2, (long long)ex * inter + col, false, v);
 #pragma unroll
-        for (int e = 0; e < 4; e++) h[e] = __ushort_as_half(0);
-    } else {
-        const int ex = expert_ids[b];
-        float v[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int col = kg * 128 + 4 * lane + e;
-            const float gv = __half2float(gu[(long long)slot * 2 * inter + col]);
-            const float uv = __half2float(gu[(long long)slot * 2 * inter + inter + col]);
-            const float act = __half2float(__float2half_rn(gv / (1.0f + __expf(-gv)) * uv));
-            v[e] = act * __half2float(suh2[(long long)ex * inter + col]);
-        }
-        fwht128(v[0], v[1], v[2], v[3], lane);
-#pragma unroll
-        for (int e = 0; e < 4; e++) h[e] = __float2half_rn(v[e] * HAD_SCALE);
-    }
-    const int kt = kg * 8 + (lane >> 2);
-    const long long elem_base = (((long long)b) * KT + kt) * 32 + row * 4;
-    store_fragments<MODE>(xf, elem_base, lane, h);
+    for (int e = 0; e < 4; e++) v[e] *= __half2float(__float2half_rn(g[e] / (1.0f + __expf(-g[e])) * u[e]));
+    fwht128(v[0], v[1], v[2], v[3], lane);
+    moe_store_row<MODE>(xf + ((long long)b * kgs + kg) * MOE_BLOCK_ROWS * F_ROW, MOE_BLOCK_ROWS, row % MOE_BLOCK_ROWS, lane, v);
 }
 
-// y[t, :] = sum_j w[t, j] * yd[t*top_k + j, :] in fp32, slot order, one rounding; ids outside [0, E) are skipped.
-__global__ void moe_combine_kernel(const __half* __restrict__ yd, const float* __restrict__ w, const int* __restrict__ topk_ids, int tokens,
-                                   int top_k, int hidden, int E, void* __restrict__ y, int y_bf16)
+// 32 columns of a rotated-basis row back in the true basis: Had128(y) * svh, rounded to fp16 like the output of the linear.
+__device__ __forceinline__ void moe_unrotate32(const uint32_t (&w)[16], const uint32_t (&sw)[16], int lane, float (&v)[32])
+{
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = moe_half(w, i);
+    fwht128_quad(v, lane);
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] * (HAD_SCALE * moe_half(sw, i))));
+}
+
+// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_quad), and up to MOE_SPAN column blocks of
+// 128 of it: 16-byte loads and full-line stores, and the chain of dependent loads (block -> expert and slot -> values) is walked once
+// per span -- with one column block per warp it is what bounds these kernels (70 us instead of 22 us of traffic for 2048 tokens, top-8,
+// 2048 columns).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
+constexpr int MOE_SPAN = 4;
+struct MoeSpan {
+    int b, kg0, kg1, row, slot, ex;
+    bool valid, any;
+    __device__ __forceinline__ MoeSpan(int kgs, int cap, int numel, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+                                       const int* __restrict__ num_post)
+    {
+        const int lane = threadIdx.x & 31, spans = (kgs + MOE_SPAN - 1) / MOE_SPAN;
+        const int at = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        b = at / spans;
+        kg0 = (at - b * spans) * MOE_SPAN;
+        kg1 = kg0 + MOE_SPAN < kgs ? kg0 + MOE_SPAN : kgs;
+        any = false;
+        if (b >= cap / MOE_BLOCK_ROWS) return;
+        const int post = *num_post;
+        row = b * MOE_BLOCK_ROWS + (lane >> 2);
+        ex = expert_ids[b];
+        slot = sorted_ids[row];
+        any = b * MOE_BLOCK_ROWS < post;
+        valid = any && slot >= 0 && slot < numel;
+    }
+};
+
+// xf[shard][item][row block] = Had128(fp16(x[token(p)]) * suh[expert(p), shard]) in the B-operand layout, both shards from one load of x.
+__global__ void __launch_bounds__(256, 2) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
+                                                            int numel, int cap, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+                                                            const int* __restrict__ num_post, const int2* __restrict__ blk,
+                                                            unsigned char* __restrict__ xf, long long shard_stride)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;       // one thread per (token, 2 columns)
-    const int half_h = hidden >> 1;
-    if (idx >= (long long)tokens * half_h) return;
-    const int t = (int)(idx / half_h), c = (int)(idx % half_h) * 2;
-    float a0 = 0.f, a1 = 0.f;
-    for (int j = 0; j < top_k; j++) {
-        const int e = topk_ids[t * top_k + j];
-        if (e < 0 || e >= E) continue;
-        const __half2 v = *reinterpret_cast<const __half2*>(yd + ((long long)t * top_k + j) * hidden + c);
-        const float wt = w[t * top_k + j];
-        a0 += wt * __low2float(v);
-        a1 += wt * __high2float(v);
+    const int lane = threadIdx.x & 31, q = lane & 3, kgs = hidden >> 7;
+    const MoeSpan at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    if (!at.any) return;
+    const int2 run = blk[at.b];
+    const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
+    const long long x_row = (long long)(at.valid ? at.slot / top_k : 0) * hidden + 32 * q;
+    const __half* signs = suh + (long long)at.ex * 2 * hidden + 32 * q;
+    unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
+#pragma unroll 1
+    for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
+        uint32_t xw[16], sw[2][16];
+        moe_load32(x, x_row + kg * 128, xw);
+        moe_load32(signs, kg * 128, sw[0]);
+        moe_load32(signs, hidden + kg * 128, sw[1]);
+        if (x_bf16) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xw[i]);
+                const __half2 h = __floats2half2_rn(__low2float(bb), __high2float(bb));
+                xw[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            float v[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = moe_half(xw, i) * moe_half(sw[s], i);
+            fwht128_quad(v, lane);
+            if (at.valid) moe_store_rows(unit + s * shard_stride, rows, row, q, v);
+        }
     }
-    const __half2 h = __floats2half2_rn(a0, a1);
-    if (y_bf16) {
-        reinterpret_cast<__nv_bfloat162*>(y)[idx] = __floats2bfloat162_rn(__low2float(h), __high2float(h));
-    } else {
-        reinterpret_cast<__half2*>(y)[idx] = h;
+}
+
+// The input of the down projection: Had128( fp16( silu(gate) * up ) * suh2[expert] ) with gate | up = Had128(gu_rot[row]) * svh13[expert].
+__global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restrict__ gu_rot, const __half* __restrict__ svh13,
+                                                         const __half* __restrict__ suh2, int inter, int numel, int cap,
+                                                         const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, unsigned char* __restrict__ xf)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    const int lane = threadIdx.x & 31, q = lane & 3, kgs = inter >> 7;
+    const MoeSpan at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    if (!at.any) return;
+    const int2 run = blk[at.b];
+    const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
+    const __half* gu = gu_rot + (long long)at.row * 2 * inter + 32 * q;
+    const __half* sv = svh13 + (long long)at.ex * 2 * inter + 32 * q;
+    const __half* s2 = suh2 + (long long)at.ex * inter + 32 * q;
+    unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
+#pragma unroll 1
+    for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
+        uint32_t gw[16], uw[16], sg[16], su[16], sw[16];
+        moe_load32(gu, kg * 128, gw);
+        moe_load32(gu, inter + kg * 128, uw);
+        moe_load32(sv, kg * 128, sg);
+        moe_load32(sv, inter + kg * 128, su);
+        moe_load32(s2, kg * 128, sw);
+        float g[32], u[32];
+        moe_unrotate32(gw, sg, lane, g);
+        moe_unrotate32(uw, su, lane, u);
+#pragma unroll
+        for (int i = 0; i < 32; i++) g[i] = __half2float(__float2half_rn(g[i] / (1.0f + __expf(-g[i])) * u[i])) * moe_half(sw, i);
+        fwht128_quad(g, lane);
+        if (at.valid) moe_store_rows(unit, rows, row, q, g);
     }
+}
+
+// yd[slot(row), :] = fp16( Had128(yd_rot[row]) * svh2[expert] ).
+__global__ void __launch_bounds__(256, 2) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
+                                                         const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+                                                         const int* __restrict__ num_post, __half* __restrict__ yd)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    const MoeSpan at(hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
+    if (!at.any) return;
+    const __half* src = yd_rot + (long long)at.row * hidden + 32 * q;
+    const __half* sv = svh2 + (long long)at.ex * hidden + 32 * q;
+    __half* dst = yd + (long long)(at.valid ? at.slot : 0) * hidden + 32 * q;
+#pragma unroll 1
+    for (int kg = at.kg0; kg < at.kg1; kg++) {
+        uint32_t w[16], sw[16];
+        moe_load32(src, kg * 128, w);
+        moe_load32(sv, kg * 128, sw);
+        float v[32];
+        moe_unrotate32(w, sw, lane, v);
+        if (!at.valid) continue;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const __half2 h = __floats2half2_rn(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
+                o[j] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            reinterpret_cast<uint4*>(dst + kg * 128)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+}
+
+// y[t, :] = sum_j w[t, j] * yd[t*top_k + j, :] in fp32, slot order, one rounding; ids outside [0, E) are skipped.  V columns per
+// thread; the rows of up to eight slots are requested together (16384 slots of 2048 columns: 40 us with two columns per thread
+// and one slot at a time).
+template <int V>
+__global__ void __launch_bounds__(256) moe_combine_kernel(const __half* __restrict__ yd, const float* __restrict__ w, const int* __restrict__ topk_ids,
+                                                          int tokens, int top_k, int hidden, int E, void* __restrict__ y, int y_bf16)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    using Vec = typename std::conditional<V == 8, uint4, uint32_t>::type;
+    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;       // one thread per (token, V columns)
+    const int per = hidden / V;
+    if (idx >= (long long)tokens * per) return;
+    const int t = (int)(idx / per), c = (int)(idx - (long long)t * per) * V;
+    float a[V];
+#pragma unroll
+    for (int i = 0; i < V; i++) a[i] = 0.f;
+    for (int j0 = 0; j0 < top_k; j0 += 8) {
+        Vec r[8];
+        float wt[8];
+        bool on[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const long long slot = (long long)t * top_k + j0 + j;
+            int e = -1;
+            if (j0 + j < top_k) e = topk_ids[slot];
+            on[j] = e >= 0 && e < E;
+            if (on[j]) {
+                r[j] = *reinterpret_cast<const Vec*>(yd + slot * hidden + c);
+                wt[j] = w[slot];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (!on[j]) continue;
+            const uint32_t* words = reinterpret_cast<const uint32_t*>(&r[j]);
+#pragma unroll
+            for (int i = 0; i < V / 2; i++) {
+                const __half2 h = *reinterpret_cast<const __half2*>(&words[i]);
+                a[2 * i] += wt[j] * __low2float(h);
+                a[2 * i + 1] += wt[j] * __high2float(h);
+            }
+        }
+    }
+    Vec o;
+    uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+    for (int i = 0; i < V / 2; i++) {
+        const __half2 h = __floats2half2_rn(a[2 * i], a[2 * i + 1]);
+        const __nv_bfloat162 bb = __floats2bfloat162_rn(__low2float(h), __high2float(h));
+        ow[i] = y_bf16 ? *reinterpret_cast<const uint32_t*>(&bb) : *reinterpret_cast<const uint32_t*>(&h);
+    }
+    reinterpret_cast<Vec*>(y)[idx] = o;
 }
 
 // ------------------------------------------------------------------------------------------------ launchers
@@ -250,64 +473,94 @@ int moe_init_device()
 static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, cudaStream_t st)
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* counters, cudaStream_t st)
 {
     return launch_chained(moe_align_kernel, dim3(1), dim3(1024), (3 * E + 1) * sizeof(int), st, topk_ids, numel, E, block, cap, sorted_ids, expert_ids,
-                          num_post, expert_map, E_global);
+                          num_post, expert_map, E_global, item_blocks, items, blk, counters);
+}
+
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+static unsigned span_blocks(int cap, int cols)      // CTAs of eight warps, a warp per (block of eight rows, span)
+{
+    return blocks_for((long long)(cap / MOE_BLOCK_ROWS) * ((cols / 128 + MOE_SPAN - 1) / MOE_SPAN), 8);
 }
 
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
-                      const int* sorted_ids, const int* expert_ids, const int* num_post, uint32_t* xf, int mode, cudaStream_t st)
+                      const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st)
 {
-    const long long items = (long long)shards * cap * (hidden / 128);
-    if (items == 0) return EXL3_OK;
-    auto kernel = mode == GEMV_SPLIT ? moe_had_in_kernel<GEMV_SPLIT> : moe_had_in_kernel<GEMV_PAIRED>;
-    return launch_chained(kernel, dim3(blocks_for(items, 8)), dim3(256), 0, st, x, x_bf16, suh, shards, hidden, top_k, numel, cap, sorted_ids,
-                          expert_ids, num_post, xf);
+    return launch_chained(mode == GEMV_SPLIT ? moe_had_in_rows_kernel<GEMV_SPLIT> : moe_had_in_rows_kernel<GEMV_PAIRED>,
+                          dim3(blocks_for((long long)cap * (hidden / 128), 8)), dim3(256), 0, st, x, x_bf16, suh, shards, hidden, top_k, numel, cap,
+                          sorted_ids, expert_ids, num_post, reinterpret_cast<unsigned char*>(xf), shard_stride);
 }
 
-int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
-                          const int* expert_ids, const int* num_post, uint32_t* xf, int mode, cudaStream_t st)
+int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids, const int* expert_ids,
+                          const int* num_post, void* xf, int mode, cudaStream_t st)
 {
-    const long long items = (long long)cap * (inter / 128);
-    if (items == 0) return EXL3_OK;
-    auto kernel = mode == GEMV_SPLIT ? moe_glu_had_in_kernel<GEMV_SPLIT> : moe_glu_had_in_kernel<GEMV_PAIRED>;
-    return launch_chained(kernel, dim3(blocks_for(items, 8)), dim3(256), 0, st, gu, suh2, inter, numel, cap, sorted_ids, expert_ids, num_post, xf);
+    return launch_chained(mode == GEMV_SPLIT ? moe_glu_had_in_rows_kernel<GEMV_SPLIT> : moe_glu_had_in_rows_kernel<GEMV_PAIRED>,
+                          dim3(blocks_for((long long)cap * (inter / 128), 8)), dim3(256), 0, st, gu, suh2, inter, numel, cap, sorted_ids, expert_ids,
+                          num_post, reinterpret_cast<unsigned char*>(xf));
+}
+
+int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
+                            const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st)
+{
+    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden)), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
+                          expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride);
+}
+
+int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
+                         const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st)
+{
+    return launch_chained(moe_mid_kernel, dim3(span_blocks(cap, inter)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
+                          num_post, blk, reinterpret_cast<unsigned char*>(xf));
+}
+
+int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
+                         const int* num_post, __half* yd, cudaStream_t st)
+{
+    return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
+                          num_post, yd);
 }
 
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,
                        int y_bf16, cudaStream_t st)
 {
-    const long long items = (long long)tokens * (hidden / 2);
-    if (items == 0) return EXL3_OK;
-    return launch_chained(moe_combine_kernel, dim3(blocks_for(items, 256)), dim3(256), 0, st, yd, w, topk_ids, tokens, top_k, hidden, E, y, y_bf16);
+    // Eight columns per thread once that leaves enough threads to fill the chip; few tokens are latency, not bandwidth.
+    const bool wide = hidden % 8 == 0 && aligned16(yd) && aligned16(y) && (long long)tokens * hidden >= 8 * 64 * 1024;
+    const int v = wide ? 8 : 2;
+    return launch_chained(wide ? moe_combine_kernel<8> : moe_combine_kernel<2>, dim3(blocks_for((long long)tokens * (hidden / v), 256)), dim3(256), 0, st, yd, w,
+                          topk_ids, tokens, top_k, hidden, E, y, y_bf16);
 }
 
 int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t st)
 {
     const DeviceInfo* d = current_device_info();
     if (!d) return EXL3_ERR_NOT_INITIALISED;
-    int grid = d->sm_count * MOE_CTAS_PER_SM;
-    if (grid > GEMV_MAX_GRID) grid = GEMV_MAX_GRID;
-    const uint32_t unit_bytes = 2048u * K;
-    const uint32_t frag_bytes = 8u * MOE_BLOCK_ROWS * 4u * (uint32_t)gemv_frag_words(mode) * 4u;   // a unit's fragments ride with its weights
-    int ups = (int)((24u * 1024u + unit_bytes - 1) / unit_bytes);
-    const int UB = l.KG * l.NB;
-    if (ups > UB) ups = UB;
-    l.units_per_stage = ups;
-    l.stage_stride = (uint32_t)ups * (unit_bytes + frag_bytes);
-    const size_t fixed = 256 + MOE_BLOCK_ROWS * 128 * 4;
-    int stages = (int)((96u * 1024u) / l.stage_stride);
-    const int cap = (int)((d->max_smem_optin / MOE_CTAS_PER_SM - 2048 - fixed) / l.stage_stride);
-    if (stages > cap) stages = cap;
-    if (stages > MOE_MAX_STAGES) stages = MOE_MAX_STAGES;
-    if (stages < 2) return EXL3_ERR_UNSUPPORTED_ROWS;
-    l.stages = stages;
+    const int grid = d->sm_count < MOE_MAX_GRID ? d->sm_count : MOE_MAX_GRID;
+    // Stages of about 24 KB of weights (a bulk copy costs a few hundred nanoseconds whatever its size), two units or more per stage (see
+    // SkWalk).  Single blocks of eight rows: eight slots of activations, the rest of the shared memory for weights.  Long items: three
+    // stages of weights, the rest for activations (four slots of 128 rows and more).
+    const uint32_t unit = 2048u * (uint32_t)K, row = mode == GEMV_SPLIT ? 512u : 256u, tail = MOE_BLOCK_ROWS * 128 * 4, all = (uint32_t)d->max_smem_optin;
+    uint32_t ups = (24u * 1024u + unit - 1) / unit;
+    if (ups < 2) ups = 2;
+    uint32_t stages = 3;
+    if (!l.items) {
+        l.x_bytes = MOE_X_SLOTS * MOE_BLOCK_ROWS * row;
+        stages = (all - MOE_BAR_BYTES - tail - l.x_bytes) / (ups * unit);
+        if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+    } else {
+        l.x_bytes = (all - MOE_BAR_BYTES - tail - stages * ups * unit) & ~1023u;
+    }
+    l.units_per_stage = (int)ups;
+    l.stages = (int)stages;
+    l.x_off = MOE_BAR_BYTES + stages * ups * unit;
+    l.p_off = l.x_off + l.x_bytes;
+    if (l.p_off + tail > all || l.x_bytes < (uint32_t)l.slab_rows * row) return EXL3_ERR_UNSUPPORTED_ROWS;
     const CodebookConst c = codebook_const(codebook);
     l.mul = c.mul;
     l.add = c.add;
-    l.pw = make_pow2();
-    const size_t smem = fixed + (size_t)stages * l.stage_stride;
+    const size_t smem = l.p_off + tail;
     const int fam = codebook_family(codebook);
     switch (K) {
         case 2: return launch_moe_gemm_for_k<2>(l, mode, fam, grid, smem, st);

@@ -16,18 +16,22 @@ template <>
 int launch_moe_gemm_for_k<EXL3_MOE_K>(const MoeGemmLaunch& l, int mode, int family, int grid, size_t smem, cudaStream_t st)
 {
     constexpr int K = EXL3_MOE_K;
-    if (family == FAM_MUL1) return launch_chained(moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1>, dim3(grid), dim3(MOE_THREADS), smem, st, l);
-    if (mode == GEMV_SPLIT) return launch_chained(moe_gemm_kernel<K, GEMV_SPLIT, FAM_HASH>, dim3(grid), dim3(MOE_THREADS), smem, st, l);
-    return launch_chained(moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH>, dim3(grid), dim3(MOE_THREADS), smem, st, l);
+    const auto kernel = l.items ? (family == FAM_MUL1 ? moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1, true> : moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH, true>)
+                        : family == FAM_MUL1 ? moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1, false>
+                        : mode == GEMV_SPLIT ? moe_gemm_kernel<K, GEMV_SPLIT, FAM_HASH, false>
+                                             : moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH, false>;
+    return launch_chained(kernel, dim3(grid), dim3(SK_THREADS), smem, st, l);
 }
 
 template <>
 int moe_set_attributes_for_k<EXL3_MOE_K>(int max_smem)
 {
     constexpr int K = EXL3_MOE_K;
-    int rc = cuda_status(cudaFuncSetAttribute(moe_gemm_kernel<K, GEMV_SPLIT, FAM_HASH>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    int rc = EXL3_OK;
+    for (const auto kernel : {moe_gemm_kernel<K, GEMV_SPLIT, FAM_HASH, false>, moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH, false>,
+                              moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1, false>, moe_gemm_kernel<K, GEMV_PAIRED, FAM_HASH, true>,
+                              moe_gemm_kernel<K, GEMV_PAIRED, FAM_MUL1, true>})
+        if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     return rc;
 }
 

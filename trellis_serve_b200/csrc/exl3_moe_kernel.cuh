@@ -1,320 +1,521 @@
-// Grouped decode GEMV for routed MoE experts (sm_100a).
+// Grouped decode GEMM for routed MoE experts (sm_100a).
 //
-// Every (token, expert) slot is its own GEMV row because every expert has its own suh
-// (cuda/src/sglang_exl3/kernels/marlin_moe.py:11-13 of 0xSero/trellis-serve).  The routing step sorts the slots by
-// expert into "moe blocks" of 8 rows of one expert (sorted ids, block expert ids, padded count: the contract of
-// cuda/csrc/exl3_marlin_moe.cu:542-594); this kernel multiplies each block by its expert's matrix.  It replaces the
-// reference's grouped Marlin instances (cuda/csrc/exl3_marlin_moe_template.h, launch at exl3_marlin_moe.cu:376-408).
+// Every (token, expert) slot is its own row because every expert has its own suh
+// (cuda/src/sglang_exl3/kernels/marlin_moe.py:11-13 of 0xSero/trellis-serve).  The routing step sorts the slots by expert; an ITEM is a
+// run of up to 32 (split) or 128 (paired) rows of one expert, a multiple of eight: either the "moe blocks" of eight rows of the engine's
+// contract (cuda/csrc/exl3_marlin_moe.cu:542-594), or the longer runs that launch_moe_align lists.  This kernel multiplies each item by
+// its expert's matrix.  It replaces the reference's grouped Marlin instances (cuda/csrc/exl3_marlin_moe_template.h, launch at
+// exl3_marlin_moe.cu:376-408), for decode batches and for prefill alike.
 //
-// Same machinery as the dense decode GEMV (exl3_skinny_kernel.cuh): persistent CTAs that split the unit list
-// (moe block, column block, row block) evenly and contiguously, a producer thread streaming weights through a ring of
-// bulk-copy stages, 16 consumer warps decoding in registers into transposed m16n8k16 MMAs, split-k partial sums
-// finished by the last CTA to arrive.  Differences: the number of blocks is read on the device (CUDA-graph safe), a
-// stage never crosses a moe block (the next block is another expert's matrix), activation fragments always hold 8
-// rows per block (padding rows are zero), the epilogue uses the expert's svh and scatters rows to their slots.
+// The machinery of the dense decode GEMV (exl3_skinny_kernel.cuh): decoded registers go to tensor memory as the A operand, the rotated
+// rows are the B operand (N = rows of the item), persistent CTAs split the unit list (item, column block, row block) evenly and
+// contiguously, partial sums of column blocks cut between CTAs are added in CTA order by the last one to arrive.  Differences: item
+// list and row counts are read on the device (CUDA-graph safe), so N and the pitch of B are run-time values; the activations have a ring
+// of their own, a slot per unit, whose slot count follows the largest item; ONE warp issues the MMAs of the three decode groups in unit
+// order into one accumulator, so that 128 rows fit into tensor memory twice.  Single blocks of eight rows are finished here (output
+// rotation with the expert's svh, rows scattered to their slots); for long items that would be a third of all instructions on four of 32
+// warps (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): their rows leave in the rotated basis, as fp16, and the
+// kernels behind rotate them.
+//
+// Bound by the ALU pipe of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.
 #pragma once
-#include "exl3_gemv_common.cuh"
+#include "exl3_skinny_kernel.cuh"
 
 namespace exl3 {
 
 constexpr int MOE_BLOCK_ROWS = 8;
-constexpr int MOE_CONSUMER_WARPS = 16;
-constexpr int MOE_THREADS = (MOE_CONSUMER_WARPS + 1) * 32;        // 16 decode warps and a copy warp
-constexpr int MOE_MAX_STAGES = 12;
-constexpr int MOE_CTAS_PER_SM = 2;
+constexpr int MOE_MAX_GRID = 192;                                // CTAs of a launch (one per SM)
+constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word, then the counters
+constexpr int MOE_X_SLOTS = 8;                                   // most slots of the activation ring
+constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, then the constants of the decode loop
 // Largest expert count of one routing alignment: its single CTA keeps three counters per expert in the default 48 KB of
-// shared memory ((3 * E + 1) * 4 bytes + 132 static).
+// shared memory ((3 * E + 1) * 4 bytes + 280 static).
 constexpr int MOE_MAX_EXPERTS = 4064;
+
+__host__ __device__ constexpr int moe_item_rows(int mode) { return mode == GEMV_SPLIT ? 32 : 128; }
 
 struct MoeGemmLaunch {
     const uint32_t* packed;          // [E][NB][KG][...] resident expert stack
     long long expert_stride;         // words between experts
-    const uint32_t* xf;              // fragments [shard][moe block][k/16][8][4][FW]
-    long long xf_shard_stride;       // elements (of FW words) between shards
+    const unsigned char* xf;         // rotated rows: item at first row * KG * F, unit row block at + kg * rows * F, [k chunk][row] 16 bytes
+    long long xf_shard_stride;       // bytes between shards
     const __half* svh;               // [E][n_total]
-    __half* out;                     // [slots][n_total] fp16
-    const int* sorted_ids;           // [blocks * 8] slot of each row, >= numel for padding
-    const int* expert_ids;           // [blocks]
-    const int* num_post;             // device: padded slot count = blocks * 8
-    float* partials;
-    int* counters;
+    __half* out;                     // fp16: [slots][n_total], or with items [rows][n_total] in the rotated basis
+    const int* sorted_ids;           // slot of each row, >= numel for padding
+    const int* expert_ids;           // expert of each block of eight rows
+    const int4* items;               // (expert, first block, blocks, 0), or null: every block of eight rows is an item
+    const int* counts;               // device: [0] rows; with items: [1] items, [2] rows of the largest item
+    float* partials;                 // [2 * grid][slab_rows][128]
+    int* counters;                   // [grid]
     int* err;
     int KG, NB, n_total, numel, shard_end_block;   // shard_end_block: first column block of shard 1 (NB if one shard)
-    int stages, units_per_stage;
-    uint32_t stage_stride, mul, add;
+    int stages, units_per_stage, slab_rows;
+    uint32_t x_off, x_bytes, p_off;
+    uint32_t mul, add;
     int rotated;                     // 1: no output Hadamard / svh (identity read-out)
-    Pow2 pw;
 };
 
 int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t st);
 
-template <int K, int MODE, int FAM>
-__global__ void __launch_bounds__(MOE_THREADS, MOE_CTAS_PER_SM) moe_gemm_kernel(const MoeGemmLaunch p)
+// Rows w and w + 4 of a block of eight (w = the epilogue warp), a row per warp at a time: from staged rows (c_last < c_first), or the
+// partial sums of CTAs c_first .. c_last, added in CTA order with the loads of four CTAs in flight together.
+__device__ __forceinline__ void moe_finish_eight(const MoeGemmLaunch& p, const float* src, int c_first, int c_last, uint2 sv, const int (&slots)[2], int nb,
+                                                 int w, int lane)
 {
-    constexpr int FW = gemv_frag_words(MODE);
-    constexpr uint32_t W_BYTES = 2048u * K;
-    // Fragments of one unit (8 k-tiles x 8 rows x 4 lanes x FW words): they are copied into the stage behind its weights,
-    // [weights of units_per_stage units][fragments of units_per_stage units], so a fragment crosses the L2 once per CTA.
-    constexpr uint32_t F_BYTES = 8u * MOE_BLOCK_ROWS * 4u * FW * 4u;
-    using Frag = typename std::conditional<FW == 4, uint4, uint2>::type;
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);
-    uint64_t* empty = full + MOE_MAX_STAGES;
-    int* flag = reinterpret_cast<int*>(smem + 2 * MOE_MAX_STAGES * 8);
-    float* P = reinterpret_cast<float*>(smem + 256);                              // [8][128]
-    unsigned char* stage0 = smem + 256 + MOE_BLOCK_ROWS * 128 * 4;
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cta = blockIdx.x;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < p.stages; s++) {
-            ptx::mbar_init(&full[s], 1);
-            ptx::mbar_init(&empty[s], MOE_CONSUMER_WARPS);
-        }
-        flag[0] = 0;
-        ptx::mbar_fence_init();
-    }
-    __syncthreads();
-    // The routing lists come from kernels ahead of this one in the stream: nothing is read before they have finished.
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
-    const int UB = p.NB * p.KG;                                  // units per moe block
-    const int nblocks = *p.num_post / MOE_BLOCK_ROWS;
-    const long long total = (long long)nblocks * UB;
-    const int units_q = (int)(total / gridDim.x), units_r = (int)(total % gridDim.x);
-    const long long u0 = gemv_first_unit(cta, units_q, units_r);
-    const long long u1 = gemv_first_unit(cta + 1, units_q, units_r);
-    if (u0 >= u1) return;
-
-    // position of the first unit: moe block, unit inside the block
-    int b = (int)(u0 / UB);
-    int in_blk = (int)(u0 - (long long)b * UB);
-
-    if (warp == MOE_CONSUMER_WARPS) {
-        // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            int s = 0;
-            uint32_t wait_parity = 1;
-            bool first_lap = true;
-            long long left = u1 - u0;
-            while (left > 0) {
-                int n = p.units_per_stage;
-                if (n > UB - in_blk) n = UB - in_blk;          // a stage never crosses into the next expert's matrix
-                if (n > left) n = (int)left;
-                if (!first_lap && !ptx::mbar_wait(&empty[s], wait_parity)) {
-                    atomicExch(p.err, GEMV_ERR_EMPTY_WAIT);
-                    break;
+    constexpr int CB = 4;
+    const size_t slab = MOE_BLOCK_ROWS * 128;
+    float v[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[i][e] = 0.f;
+    const bool staged = c_last < c_first;
+#pragma unroll 1
+    for (int c = c_first; c <= (staged ? c_first : c_last); c += CB) {
+        float4 f[CB][2];
+#pragma unroll
+        for (int j = 0; j < CB; j++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                f[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                const size_t at = (staged ? 0 : (size_t)(2 * (c + j) + (c + j == c_first)) * slab) + (w + 4 * i) * 128 + 4 * lane;
+                if (staged) {
+                    if (j == 0) f[j][i] = *reinterpret_cast<const float4*>(src + at);
+                } else if (c + j <= c_last) {
+                    f[j][i] = __ldcg(reinterpret_cast<const float4*>(src + at));
                 }
-                const int e = p.expert_ids[b];
-                const uint32_t bytes = (uint32_t)n * W_BYTES;
-                ptx::mbar_arrive_expect_tx(&full[s], bytes + (uint32_t)n * F_BYTES);
-                ptx::bulk_g2s(stage0 + (size_t)s * p.stage_stride, p.packed + e * p.expert_stride + (long long)in_blk * (512ll * K), bytes,
-                              &full[s]);
-                {   // the units' fragments: consecutive row blocks of a column block are consecutive in the fragment buffer
-                    unsigned char* dst = stage0 + (size_t)s * p.stage_stride + (size_t)p.units_per_stage * W_BYTES;
-                    int at = in_blk, todo = n;
-                    while (todo > 0) {
-                        const int fnb = at / p.KG, fkg = at - fnb * p.KG;
-                        int run = p.KG - fkg;
-                        if (run > todo) run = todo;
-                        const long long shard = fnb >= p.shard_end_block ? 1 : 0;
-                        const uint32_t* src = p.xf + (shard * p.xf_shard_stride + ((long long)b * (p.KG * 8) + fkg * 8) * 32) * FW;
-                        ptx::bulk_g2s(dst, src, (uint32_t)run * F_BYTES, &full[s]);
-                        dst += (size_t)run * F_BYTES;
-                        at += run;
-                        todo -= run;
+            }
+#pragma unroll
+        for (int j = 0; j < CB; j++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                v[i][0] += f[j][i].x;
+                v[i][1] += f[j][i].y;
+                v[i][2] += f[j][i].z;
+                v[i][3] += f[j][i].w;
+            }
+    }
+    const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        if (slots[i] < 0 || slots[i] >= p.numel) continue;                  // the same for the whole warp
+        if (!p.rotated) {
+            fwht128(v[i][0], v[i][1], v[i][2], v[i][3], lane);
+            v[i][0] *= HAD_SCALE * __low2float(s01);
+            v[i][1] *= HAD_SCALE * __high2float(s01);
+            v[i][2] *= HAD_SCALE * __low2float(s23);
+            v[i][3] *= HAD_SCALE * __high2float(s23);
+        }
+        const __half2 a = __floats2half2_rn(v[i][0], v[i][1]), b = __floats2half2_rn(v[i][2], v[i][3]);
+        *reinterpret_cast<uint2*>(p.out + (long long)slots[i] * p.n_total + nb * 128 + 4 * lane) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+}
+
+// LIST: items of several blocks from the align kernel's list; otherwise every block of eight rows is an item, and row count and pitch are
+// constants of the code.
+template <int K, int MODE, int FAM, bool LIST>
+__global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_constant__ MoeGemmLaunch p)
+{
+    constexpr int NMAX = LIST ? moe_item_rows(MODE) : 16;
+    constexpr uint32_t W_BYTES = 2048u * K, HALF_BYTES = K * 128u;
+    constexpr uint32_t F_ROW = MODE == GEMV_SPLIT ? 512u : 256u;            // bytes of a row in a unit's activations
+    constexpr int A_COLS = MODE == GEMV_SPLIT ? 64 : 32, A_OFF = 2 * NMAX, MMAS = MODE == GEMV_SPLIT ? 8 : 4;
+    static_assert(A_OFF + 2 * SK_GROUPS * A_COLS <= SK_TMEM_COLS, "tensor memory");
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);                   // weights of a stage have landed
+    uint64_t* stage_empty = w_full + SK_MAX_STAGES;                         // ... have been multiplied
+    uint64_t* x_full = stage_empty + SK_MAX_STAGES;                         // activations of a unit
+    uint64_t* x_empty = x_full + MOE_X_SLOTS;
+    uint64_t* buf_empty = x_empty + MOE_X_SLOTS;                            // [group][2] multiplied
+    uint64_t* acc_done = buf_empty + 2 * SK_GROUPS;                         // [2] a column block's MMAs have completed
+    uint64_t* acc_empty = acc_done + 2;                                     // [2] read out
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    int* flag = reinterpret_cast<int*>(tmem_slot + 1);
+    unsigned char* wring = smem + MOE_BAR_BYTES;
+    unsigned char* xs = smem + p.x_off;
+    float* P = reinterpret_cast<float*>(smem + p.p_off);
+
+    const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int cta = blockIdx.x, ups = p.units_per_stage, stages = p.stages;
+    if (warp == SK_COPY_WARP) {
+        if (lane == 0) {
+            for (int s = 0; s < SK_MAX_STAGES; s++) {
+                ptx::mbar_init(&w_full[s], 1);
+                ptx::mbar_init(&stage_empty[s], 1);
+            }
+            for (int s = 0; s < MOE_X_SLOTS; s++) {
+                ptx::mbar_init(&x_full[s], 1);
+                ptx::mbar_init(&x_empty[s], 1);
+            }
+            for (int b = 0; b < 2 * SK_GROUPS; b++) ptx::mbar_init(&buf_empty[b], 1);
+            for (int d = 0; d < 2; d++) {
+                ptx::mbar_init(&acc_done[d], 1);
+                ptx::mbar_init(&acc_empty[d], 4);
+            }
+            ptx::mbar_fence_init();
+        }
+    } else if (warp == SK_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ptx::smem_addr(tmem_slot)), "r"((uint32_t)SK_TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x < 34)
+        reinterpret_cast<uint32_t*>(smem + MOE_TABLE_OFF)[threadIdx.x] = threadIdx.x < 32 ? 1u << threadIdx.x : threadIdx.x == 32 ? p.mul : p.add;
+    sk_fence_before();
+    __syncthreads();
+    sk_fence_after();
+    uint32_t failed = *tmem_slot != 0;                                      // all 512 columns are this CTA's: addresses start at 0
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();                                            // the item list comes from kernels ahead in the stream
+
+    const int UB = p.NB * p.KG;                                             // units per item
+    // Values read from memory go through a shuffle where MMA operands depend on them: warp-uniform to the compiler.
+    const int n_items = __shfl_sync(0xFFFFFFFFu, LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS, 0);
+    const long long total = (long long)n_items * UB;
+    int units_q, units_r;
+    if (total < (1ll << 31)) {                                              // the 64-bit division is a few hundred clocks of everyone's start
+        units_q = (int)((unsigned)total / gridDim.x);
+        units_r = (int)((unsigned)total % gridDim.x);
+    } else {
+        units_q = (int)(total / gridDim.x);
+        units_r = (int)(total % gridDim.x);
+    }
+    const long long u0 = gemv_first_unit(cta, units_q, units_r);
+    const int units = units_q + (cta < units_r ? 1 : 0), fills = (units + ups - 1) / ups;
+    // Activation ring: the same slot size and count for every warp.
+    const uint32_t slot_bytes = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : MOE_BLOCK_ROWS * F_ROW;
+    int x_slots = slot_bytes > 0 ? (int)(p.x_bytes / slot_bytes) : 1;
+    if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
+    int item = units <= 0 ? 0 : total < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
+    int in_item = units > 0 ? (int)(u0 - (long long)item * UB) : 0;
+    auto item_of = [&](int i) {                                             // expert, first row, rows
+        if constexpr (LIST) {
+            const int4 t = p.items[i];
+            return make_int3(t.x, t.y * MOE_BLOCK_ROWS, t.z * MOE_BLOCK_ROWS);
+        }
+        else return make_int3(p.expert_ids[i], i * MOE_BLOCK_ROWS, MOE_BLOCK_ROWS);
+    };
+
+    if (warp >= SK_DECODE_WARP) {
+        // ------------------------------------------------------------------ decode: as in the dense kernel
+        const int dw = warp - SK_DECODE_WARP, group = dw >> 3, nt = 2 * (dw & 3) + ((dw >> 2) & 1);
+        const uint32_t table = ptx::smem_addr(smem + MOE_TABLE_OFF);
+        const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132)};
+        const SkPow2<K> pw(table);
+        const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
+        const int halves = 2 * units;
+        if (halves > 0) {
+            auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
+            SkWalk at(group, ups, fills, enter);
+            uint32_t wa = ptx::smem_addr(wring) + (uint32_t)(nt * 2) * HALF_BYTES + lane * 4u + (group >> 1) * W_BYTES + (group & 1) * HALF_BYTES;
+            const uint32_t t_base = ((uint32_t)(nt * 16) << 16) + A_OFF + (uint32_t)(group * 2) * A_COLS;
+            const uint32_t empty0 = ptx::smem_addr(&buf_empty[group * 2]);
+            const int bar0 = SK_BAR_BUF + group * 2;
+            uint32_t parity = 1;
+            int h = group;
+            const uint32_t move0 = group & 1 ? 2 * W_BYTES - HALF_BYTES : W_BYTES + HALF_BYTES, move1 = 3 * W_BYTES - move0;
+            const int adv0 = 1 + (group & 1);
+            auto step = [&](auto which) {
+                constexpr int S = decltype(which)::value;
+                if (at.left <= 0 && at.settle(ups, stages, enter)) wa -= ring;
+                uint32_t L[K];
+#pragma unroll
+                for (int i = 0; i < K; i++) L[i] = ptx::lds32(wa + i * 128u);
+                constexpr int TCOLS = MODE == GEMV_SPLIT ? 16 : 8;
+                const uint32_t ta = t_base + S * A_COLS;
+                auto tile = [&](auto tconst) {
+                    constexpr int T = decltype(tconst)::value;
+                    uint32_t own[2];
+                    own_words<K, T>(L, own);
+                    const uint32_t prev0 = __shfl_sync(0xFFFFFFFFu, own[0], (lane + 31) & 31);
+                    const LaneRegs<K> R = lane_regs<K>(own, prev0);
+                    uint32_t w[8];
+                    decode_tile_regs<K, MODE, FAM>(R, pw, cbc, w);
+                    if constexpr (MODE == GEMV_SPLIT) sk_store_tile_split(ta + T * TCOLS, w);
+                    else sk_store_tile_paired(ta + T * TCOLS, w);
+                };
+                sk_wait(empty0 + S * 8u, parity, failed);
+                sk_fence_after();
+                tile(std::integral_constant<int, 0>{});
+                tile(std::integral_constant<int, 1>{});
+                tile(std::integral_constant<int, 2>{});
+                tile(std::integral_constant<int, 3>{});
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                sk_fence_before();
+                sk_bar_arrive(bar0 + S, (8 + 1) * 32);
+                wa += S == 0 ? move0 : move1;
+                at.left -= S == 0 ? adv0 : 3 - adv0;
+                h += SK_GROUPS;
+            };
+#pragma unroll 1
+            while (h < halves) {
+                step(std::integral_constant<int, 0>{});
+                if (h < halves) step(std::integral_constant<int, 1>{});
+                parity ^= 1;
+            }
+        }
+    } else if (warp == SK_MMA_WARP) {
+        // ------------------------------------------------------------------ MMA issue, all groups in unit order
+        const uint32_t s_bar = ptx::smem_addr(stage_empty), xe_bar = ptx::smem_addr(x_empty), xf_bar = ptx::smem_addr(x_full);
+        const uint32_t empty0 = ptx::smem_addr(buf_empty), done0 = ptx::smem_addr(acc_done), xs_addr = ptx::smem_addr(xs);
+        uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, accumulate = 0, acc = 0, idesc = 0, pitch = MOE_BLOCK_ROWS;
+        int left = ups, third = 0;
+        // Half `HF` (0, 1) of a unit whose number is `C` modulo three: group and buffer are constants of the code.
+        auto half = [&](auto cconst, auto hconst, uint32_t b_lo, bool stage_end) {
+            constexpr int PH = 2 * decltype(cconst)::value + decltype(hconst)::value, G = PH % 3, BUF = PH / 3;
+            ptx::named_bar_sync(SK_BAR_BUF + G * 2 + BUF, (8 + 1) * 32);
+            sk_fence_after();
+            const uint64_t b = ((uint64_t)((128u >> 4) | (1u << 14)) << 32) | b_lo;
+            if (sk_elect()) {
+#pragma unroll
+                for (int m = 0; m < MMAS; m++) sk_mma(acc, A_OFF + (G * 2 + BUF) * A_COLS + m * 8, b + m * 2u * pitch, idesc, m > 0 ? 1u : accumulate);
+                sk_commit_addr(empty0 + (G * 2 + BUF) * 8u);
+                if (decltype(hconst)::value == 1) {
+                    sk_commit_addr(xe_bar + x_slot * 8u);
+                    if (stage_end) sk_commit_addr(s_bar + stage8);
+                }
+            }
+            __syncwarp();
+            accumulate = 1;
+        };
+        auto unit = [&](auto cconst, bool stage_end) {
+            const uint32_t b_lo = (pitch << 16) | ((xs_addr + x_slot * slot_bytes) >> 4);
+            half(cconst, std::integral_constant<int, 0>{}, b_lo, false);
+            half(cconst, std::integral_constant<int, 1>{}, b_lo + pitch * (F_ROW / 32), stage_end);      // half a unit, in units of 16 bytes
+        };
+        int done = 0;
+#pragma unroll 1
+        while (done < units) {                                              // column blocks of the CTA
+            const int kg = in_item % p.KG, count = p.KG - kg < units - done ? p.KG - kg : units - done;
+            if constexpr (LIST) pitch = (uint32_t)__shfl_sync(0xFFFFFFFFu, item_of(item).z, 0);
+            const uint32_t cols = (pitch + 15u) & ~15u;
+            idesc = (1u << 4) | ((cols >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> fp32, M = 128, N = cols
+            sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
+            sk_fence_after();
+            acc = d * NMAX;
+            accumulate = 0;
+#pragma unroll 1
+            for (int u = 0; u < count; u++) {
+                sk_wait(xf_bar + x_slot * 8u, x_parity, failed);
+                left--;
+                const bool stage_end = left == 0;
+                if (third == 0) unit(std::integral_constant<int, 0>{}, stage_end);
+                else if (third == 1) unit(std::integral_constant<int, 1>{}, stage_end);
+                else unit(std::integral_constant<int, 2>{}, stage_end);
+                third = third == 2 ? 0 : third + 1;
+                if (stage_end) {
+                    left = ups;
+                    stage8 = stage8 + 8 == (uint32_t)stages * 8u ? 0 : stage8 + 8;
+                }
+                if (++x_slot == (uint32_t)x_slots) {
+                    x_slot = 0;
+                    x_parity ^= 1;
+                }
+            }
+            if (sk_elect()) sk_commit_addr(done0 + d * 8u);
+            __syncwarp();
+            d ^= 1;
+            if (d == 0) acc_parity ^= 1;
+            done += count;
+            in_item += count;
+            if (in_item == UB) {
+                in_item = 0;
+                item++;
+            }
+        }
+    } else if (warp == SK_MMA_WARP + 1) {
+        // ------------------------------------------------------------------ "column block multiplied": polls for the four epilogue warps
+        uint32_t d = 0, parity = 0;
+        int done = 0, kg = units > 0 ? in_item % p.KG : 0;
+#pragma unroll 1
+        while (done < units) {
+            if (!failed && !ptx::mbar_wait_relaxed(&acc_done[d], parity, 20)) failed = 1;
+            sk_fence_after();
+            sk_fence_before();
+            sk_bar_arrive(SK_BAR_ACC + (int)d, (1 + 4) * 32);
+            d ^= 1;
+            if (d == 0) parity ^= 1;
+            done += p.KG - kg;
+            kg = 0;
+        }
+    } else if (warp == SK_MMA_WARP + 2) {
+        // ------------------------------------------------------------------ copies of activations, a unit per slot
+        if (lane == 0 && units > 0) {
+            int slot = 0;
+            uint32_t phase = 1;                                             // the first lap's slots are free
+            int3 it = item_of(item);
+            for (int j = 0; j < units; j++) {
+                if (!failed && !ptx::mbar_wait_relaxed(&x_empty[slot], phase, 50)) failed = 1;
+                const int nb = in_item / p.KG, kg = in_item - nb * p.KG;
+                const uint32_t bytes = (uint32_t)it.z * F_ROW;
+                const unsigned char* src = p.xf + (nb >= p.shard_end_block ? p.xf_shard_stride : 0) + ((long long)it.y * p.KG + (long long)kg * it.z) * F_ROW;
+                ptx::mbar_arrive_expect_tx(&x_full[slot], bytes);
+                ptx::bulk_g2s(xs + (size_t)slot * slot_bytes, src, bytes, &x_full[slot]);
+                if (++slot == x_slots) {
+                    slot = 0;
+                    phase ^= 1;
+                }
+                if (++in_item == UB) {
+                    in_item = 0;
+                    if (j + 1 < units) it = item_of(++item);
+                }
+            }
+            for (int j = units > x_slots ? units - x_slots : 0; j < units; j++) {       // every copy has landed before the CTA may leave
+                uint32_t late = 0;
+                sk_wait(ptx::smem_addr(&x_full[j % x_slots]), (uint32_t)(j / x_slots) & 1u, late);
+                failed |= late;
+            }
+        }
+        __syncwarp();
+    } else if (warp == SK_COPY_WARP) {
+        // ------------------------------------------------------------------ copies of weights
+        if (lane == 0 && units > 0) {
+            int slot = 0, todo = units;
+            uint32_t phase = 1;
+            int e = item_of(item).x;
+            for (int j = 0; j < fills; j++) {
+                if (!failed && !ptx::mbar_wait_relaxed(&stage_empty[slot], phase, 100)) failed = 1;
+                int n = todo < ups ? todo : ups;
+                todo -= n;
+                unsigned char* dst = wring + (size_t)(slot * ups) * W_BYTES;
+                ptx::mbar_arrive_expect_tx(&w_full[slot], (uint32_t)n * W_BYTES);
+                while (n > 0) {
+                    const int run = UB - in_item < n ? UB - in_item : n;     // up to the end of this expert's matrix
+                    ptx::bulk_g2s(dst, p.packed + (long long)e * p.expert_stride + (long long)in_item * (512 * K), (uint32_t)run * W_BYTES, &w_full[slot]);
+                    dst += (size_t)run * W_BYTES;
+                    n -= run;
+                    in_item += run;
+                    if (in_item == UB) {
+                        in_item = 0;
+                        item++;
+                        if (n + todo > 0) e = item_of(item).x;
                     }
                 }
-                left -= n;
-                in_blk += n;
-                if (in_blk == UB) {
-                    in_blk = 0;
-                    b++;
-                }
-                if (++s == p.stages) {
-                    s = 0;
-                    if (first_lap) { first_lap = false; wait_parity = 0; } else wait_parity ^= 1;
+                if (++slot == stages) {
+                    slot = 0;
+                    phase ^= 1;
                 }
             }
-        }
-        return;
-    }
-
-    // ---------------------------------------------------------------------- consumers
-    const int nt = warp & 7, kq = warp >> 3;
-    const int g = lane >> 2, q = lane & 3;
-    const CodebookConst cbc = {p.mul, p.add};
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const uint32_t stage0_addr = ptx::smem_addr(stage0);
-    const uint32_t w_off = (uint32_t)((nt * 2 + kq) * K) * 128u + lane * 4u;
-    int nb = in_blk / p.KG, kg = in_blk - nb * p.KG;
-    bool aborted = false;
-
-    auto wait_stage = [&](int slot, uint32_t phase) {
-        if (!aborted && !ptx::mbar_wait(&full[slot], phase)) {
-            aborted = true;
-            if (lane == 0) atomicExch(p.err, GEMV_ERR_FULL_WAIT);
-        }
-    };
-
-    auto flush = [&]() {
-        ptx::named_bar_sync(1, MOE_CONSUMER_WARPS * 32);
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-            if (kq == half) {
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    float* dst = &P[(2 * q + (e & 1)) * 128 + nt * 16 + g + 8 * (e >> 1)];
-                    *dst = half == 0 ? acc[e] : *dst + acc[e];
-                }
-            }
-            ptx::named_bar_sync(1, MOE_CONSUMER_WARPS * 32);
-        }
-        const int gb = b * p.NB + nb;                           // global column block
-        const long long ub = (long long)gb * p.KG;
-        const int c_first = gemv_cta_of_unit(ub, units_q, units_r);
-        const int c_last = gemv_cta_of_unit(ub + p.KG - 1, units_q, units_r);
-        const int tid = threadIdx.x;
-        constexpr int nelem = MOE_BLOCK_ROWS * 128;
-        bool finish = true;
-        if (c_first != c_last) {
-            float* slot = p.partials + (size_t)(cta + gb) * nelem;
-            for (int e = tid; e < nelem; e += MOE_CONSUMER_WARPS * 32) slot[e] = P[e];
-            ptx::named_bar_sync(1, MOE_CONSUMER_WARPS * 32);
-            if (tid == 0) {
-                __threadfence();          // publishes every thread's stores (ordered before it by the barrier) ahead of the counter
-                const int old = atomicAdd(&p.counters[gb], 1);
-                const int last = (old == c_last - c_first);
-                if (last) p.counters[gb] = 0;
-                flag[0] = last;
-            }
-            ptx::named_bar_sync(1, MOE_CONSUMER_WARPS * 32);
-            finish = flag[0] != 0;
-            if (finish) {
-                __threadfence();
-                for (int e = tid; e < nelem; e += MOE_CONSUMER_WARPS * 32) {
-                    float sum = 0.f;
-                    for (int c = c_first; c <= c_last; c++) sum += __ldcg(p.partials + (size_t)(c + gb) * nelem + e);
-                    P[e] = sum;
-                }
-            }
-            ptx::named_bar_sync(1, MOE_CONSUMER_WARPS * 32);
-        }
-        if (finish && warp < MOE_BLOCK_ROWS) {
-            const int slot_id = p.sorted_ids[b * MOE_BLOCK_ROWS + warp];
-            if (slot_id >= 0 && slot_id < p.numel) {
-                float v[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) v[e] = P[warp * 128 + 4 * lane + e];
-                if (!p.rotated) {
-                    fwht128(v[0], v[1], v[2], v[3], lane);
-                    const int ex = p.expert_ids[b];
-                    const uint2 sv = *reinterpret_cast<const uint2*>(p.svh + (size_t)ex * p.n_total + nb * 128 + 4 * lane);
-                    const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
-                    v[0] *= HAD_SCALE * __low2float(s01);
-                    v[1] *= HAD_SCALE * __high2float(s01);
-                    v[2] *= HAD_SCALE * __low2float(s23);
-                    v[3] *= HAD_SCALE * __high2float(s23);
-                }
-                __half h[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) h[e] = __float2half_rn(v[e]);
-                *reinterpret_cast<uint2*>(p.out + (size_t)slot_id * p.n_total + nb * 128 + 4 * lane) = *reinterpret_cast<uint2*>(h);
+            for (int j = fills > stages ? fills - stages : 0; j < fills; j++) {
+                uint32_t late = 0;
+                sk_wait(ptx::smem_addr(&w_full[j % stages]), (uint32_t)(j / stages) & 1u, late);
+                failed |= late;
             }
         }
-#pragma unroll
-        for (int e = 0; e < 4; e++) acc[e] = 0.f;
-    };
-
-    int slot = 0, in_stage = 0;
-    uint32_t phase = 0;
-    int left = (int)(u1 - u0);
-    int stage_units = p.units_per_stage;
-    if (stage_units > UB - in_blk) stage_units = UB - in_blk;
-    if (stage_units > left) stage_units = left;
-    uint32_t waddr = stage0_addr + w_off;
-    const uint32_t f_off = (uint32_t)p.units_per_stage * W_BYTES + ((uint32_t)(g * 4 + q) + (uint32_t)(kq * 4) * 32u) * FW * 4u;
-    uint32_t faddr = stage0_addr + f_off;
-    bool dirty = false;
-    wait_stage(0, 0);
-
-    // Runs of units that end where something has to happen (stage used up, column block finished, range finished);
-    // inside a run only the two read addresses advance.
-    while (left > 0) {
-        int run = p.KG - kg;
-        if (run > stage_units - in_stage) run = stage_units - in_stage;
-        if (run > left) run = left;
-        left -= run;
-        in_blk += run;
-        in_stage += run;
-        kg += run;
-        dirty = true;
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ epilogue
+        const int ew = warp - SK_EPI_WARP, tid = (int)threadIdx.x - SK_EPI_WARP * 32;
+        int d = 0, done = 0;
 #pragma unroll 1
-        for (; run > 0; run--) {
-            uint32_t L[K];
-#pragma unroll
-            for (int i = 0; i < K; i++) L[i] = ptx::lds32(waddr + i * 128u);
-            Frag bfrag[4];
-#pragma unroll
-            for (int T = 0; T < 4; T++) {
-                if constexpr (FW == 4) bfrag[T] = ptx::lds128(faddr + T * 32u * FW * 4u);
-                else bfrag[T] = ptx::lds64(faddr + T * 32u * FW * 4u);
+        while (done < units) {
+            const int nb = in_item / p.KG, kg = in_item - nb * p.KG, count = p.KG - kg < units - done ? p.KG - kg : units - done;
+            const int3 it = item_of(item);
+            const long long first = u0 + done - kg;                         // first unit of the column block
+            const int c_first = gemv_cta_of_unit(first, units_q, units_r), c_last = gemv_cta_of_unit(first + p.KG - 1, units_q, units_r);
+            const bool shared = c_first != c_last;
+            [[maybe_unused]] uint2 sv = make_uint2(0u, 0u);
+            [[maybe_unused]] int slots[2] = {-1, -1};
+            if constexpr (!LIST) {                                          // requested while the block is still being multiplied
+                if (!p.rotated) sv = *reinterpret_cast<const uint2*>(p.svh + (long long)it.x * p.n_total + nb * 128 + 4 * lane);
+                slots[0] = p.sorted_ids[it.y + ew];
+                slots[1] = p.sorted_ids[it.y + ew + 4];
             }
-
-            auto tile = [&](auto tconst) {
-                constexpr int T = decltype(tconst)::value;
-                uint32_t own[2];
-                own_words<K, T>(L, own);
-                const uint32_t prev0 = __shfl_sync(0xFFFFFFFFu, own[0], (lane + 31) & 31);
-                const LaneRegs<K> R = lane_regs<K>(own, prev0);
-                uint32_t w[8];
-                decode_tile_regs<K, MODE, FAM>(R, p.pw, cbc, w);
-                if constexpr (MODE == GEMV_SPLIT) {
-                    const uint4 bb = bfrag[T];
-                    ptx::mma_m16n8k16(acc, w[0], w[4], w[1], w[5], bb.x, bb.y);
-                    ptx::mma_m16n8k16(acc, w[2], w[6], w[3], w[7], bb.z, bb.w);
-                } else {
-                    const uint2 bb = bfrag[T];
-                    ptx::mma_m16n8k16(acc, w[0], w[2], w[1], w[3], bb.x, bb.y);
+            __half* dst = p.out + (long long)it.y * p.n_total + nb * 128 + ew * 32 + lane;      // LIST: this lane's column
+            auto store8 = [&](int r0, const float (&v)[8]) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) dst[(long long)(r0 + e) * p.n_total] = __float2half_rn(v[e]);
+            };
+            // Tensor memory -> shared memory or the CTA's slab: lane = output column.
+            auto load_rows = [&](int c, float (&v)[8]) {
+                uint32_t r[8];
+                sk_load8(((uint32_t)(ew * 32) << 16) + (uint32_t)(d * NMAX + c), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    asm volatile("" : "+r"(r[e]));
+                    v[e] = __uint_as_float(r[e]);
                 }
             };
-            tile(std::integral_constant<int, 0>{});
-            tile(std::integral_constant<int, 1>{});
-            tile(std::integral_constant<int, 2>{});
-            tile(std::integral_constant<int, 3>{});
-            waddr += W_BYTES;
-            faddr += F_BYTES;
-        }
-        const bool stage_done = in_stage == stage_units;
-        if (stage_done) {
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&empty[slot]);
-        }
-        if (kg == p.KG) {                                        // column block of this moe block finished
-            flush();
-            dirty = false;
-            kg = 0;
-            if (++nb == p.NB) {                                  // next moe block: another expert, another 8 rows
-                nb = 0;
-                in_blk = 0;
-                b++;
+            auto read_rows = [&](int rows, float* to) {
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 8) {
+                    float v[8];
+                    load_rows(c, v);
+#pragma unroll
+                    for (int e = 0; e < 8; e++) to[(c + e) * 128] = v[e];
+                }
+            };
+            auto release = [&]() {
+                sk_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&acc_empty[d]);
+            };
+            ptx::named_bar_sync(SK_BAR_ACC + d, (1 + 4) * 32);
+            sk_fence_after();
+            if (shared) {
+                const size_t slab = (size_t)p.slab_rows * 128;
+                read_rows(it.z, p.partials + (size_t)(2 * cta + (cta == c_first)) * slab + ew * 32 + lane);
+                release();
+                ptx::named_bar_sync(SK_BAR_EPI, 128);
+                if (tid == 0) {
+                    // Ordered behind every thread's partial sums by the barrier: releases them, and acquires those of the others.
+                    const int last = ptx::atom_add_acq_rel_gpu(&p.counters[c_first], 1) == c_last - c_first;
+                    if (last) p.counters[c_first] = 0;
+                    *flag = last;
+                }
+                ptx::named_bar_sync(SK_BAR_EPI, 128);
+                if (!LIST && *flag) {
+                    moe_finish_eight(p, p.partials, c_first, c_last, sv, slots, nb, ew, lane);
+                } else if (*flag) {
+#pragma unroll 1
+                    for (int r0 = 0; r0 < it.z; r0 += 8) {
+                        float v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) v[e] = 0.f;
+#pragma unroll 1
+                        for (int c = c_first; c <= c_last; c++) {
+                            const float* src = p.partials + (size_t)(2 * c + (c == c_first)) * slab + r0 * 128 + ew * 32 + lane;
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[e] += __ldcg(src + e * 128);
+                        }
+                        store8(r0, v);
+                    }
+                }
+                ptx::named_bar_sync(SK_BAR_EPI, 128);                       // the flag may be overwritten
+            } else if (!LIST) {
+                read_rows(MOE_BLOCK_ROWS, P + ew * 32 + lane);
+                release();
+                ptx::named_bar_sync(SK_BAR_EPI, 128);
+                moe_finish_eight(p, P, 0, -1, sv, slots, nb, ew, lane);
+                ptx::named_bar_sync(SK_BAR_EPI, 128);
+            } else {
+#pragma unroll 1
+                for (int r0 = 0; r0 < it.z; r0 += 8) {
+                    float v[8];
+                    load_rows(r0, v);
+                    store8(r0, v);
+                }
+                release();
             }
-        }
-        if (stage_done && left > 0) {
-            in_stage = 0;
-            if (++slot == p.stages) {
-                slot = 0;
-                phase ^= 1;
+            d ^= 1;
+            done += count;
+            in_item += count;
+            if (in_item == UB) {
+                in_item = 0;
+                item++;
             }
-            stage_units = p.units_per_stage;
-            if (stage_units > UB - in_blk) stage_units = UB - in_blk;
-            if (stage_units > left) stage_units = left;
-            waddr = stage0_addr + (uint32_t)slot * p.stage_stride + w_off;
-            faddr = stage0_addr + (uint32_t)slot * p.stage_stride + f_off;
-            wait_stage(slot, phase);
         }
     }
-    if (dirty) flush();
+
+    if (failed && lane == 0) atomicExch(p.err, GEMV_ERR_FULL_WAIT);
+    sk_fence_before();
+    __syncthreads();
+    if (warp == SK_MMA_WARP) {
+        sk_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(0u), "r"((uint32_t)SK_TMEM_COLS));
+    }
 }
 
 }  // namespace exl3

@@ -15,6 +15,7 @@ expert (`BLOCK_SIZES`); `align` here produces the (sorted_ids, expert_ids, num_p
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass, field
 
 import torch
@@ -344,8 +345,9 @@ def _up256(n: int) -> int:
     return (n + 255) & ~255
 
 
-def _layer_regions(num_experts_per_class: list[int], hidden: int, inter: int, codebook: int, tokens: int, top_k: int):
-    """[(name, nbytes)] of one layer's temporaries, in workspace order; per class: routing triple and fragment buffers."""
+@functools.lru_cache(maxsize=256)
+def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: int, codebook: int, tokens: int, top_k: int):
+    """{name: (offset, nbytes)} of one layer's temporaries and their total; per class: routing triple and activation buffers."""
     lib = _lib.load()
     slots = tokens * top_k
     regions = [("ids32", slots * 4), ("wts", slots * 4), ("gu", slots * 2 * inter * 2), ("yd", slots * hidden * 2)]
@@ -358,12 +360,16 @@ def _layer_regions(num_experts_per_class: list[int], hidden: int, inter: int, co
         gemv = max(gemv, int(lib.exl3_moe_workspace_bytes(cap, 2 * inter)), int(lib.exl3_moe_workspace_bytes(cap, hidden)))
         if moe_block_size(tokens, top_k, e) == BLOCK_SIZES[1]:
             regions.append((f"tc{c}", int(lib.exl3_moe_tc_workspace_bytes(slots, e, hidden, inter))))
-    return [("gemv", gemv)] + regions       # the GEMV workspace first: its header and counters must stay zero
+    plan, off = {}, 0
+    for name, n in [("gemv", gemv)] + regions:       # the GEMV workspace first: its header and counters must stay zero
+        plan[name] = (off, n)
+        off += _up256(n)
+    return plan, off
 
 
 def layer_workspace_bytes(num_experts_per_class: list[int], hidden: int, inter: int, codebook: int, tokens: int, top_k: int) -> int:
     """Bytes `run_layer` needs for up to `tokens` tokens (zero-filled once by the caller)."""
-    return sum(_up256(n) for _, n in _layer_regions(num_experts_per_class, hidden, inter, codebook, tokens, top_k))
+    return _layer_regions(tuple(num_experts_per_class), hidden, inter, codebook, tokens, top_k)[1]
 
 
 def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, workspace: torch.Tensor,
@@ -381,44 +387,52 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
         return out
     dev, st = x.device, _stream(x.device)
     maps = expert_maps if expert_maps is not None else pack.expert_maps
-    views, off = {}, 0
-    for name, n in _layer_regions([p.num_experts for p in pack.packs], hidden, inter, pack.codebook, tokens, top_k):
-        views[name] = workspace[off:off + n]
-        off += _up256(n)
-    if off > workspace.numel():
-        raise RuntimeError(f"MoE workspace holds {workspace.numel()} bytes, this call needs {off}")
-    ids32, wts = views["ids32"].view(torch.int32), views["wts"].view(torch.float32)
-    ids32.copy_(topk_ids.reshape(-1))
-    wts.copy_(topk_weights.reshape(-1))
-    gu, yd, ws = views["gu"], views["yd"], views["gemv"]
+    plan, need = _layer_regions(tuple(p.num_experts for p in pack.packs), hidden, inter, pack.codebook, tokens, top_k)
+    if need > workspace.numel():
+        raise RuntimeError(f"MoE workspace holds {workspace.numel()} bytes, this call needs {need}")
+    base = workspace.data_ptr()
+
+    def at(name):
+        return ctypes.c_void_p(base + plan[name][0])
+
+    def view(name):
+        return workspace[plan[name][0]:plan[name][0] + plan[name][1]]
+
+    # Routing as the kernels want it (int32 ids, fp32 weights, contiguous) is used where it stands.
+    ids32, wts = topk_ids, topk_weights
+    if ids32.dtype != torch.int32 or not ids32.is_contiguous() or ids32.device != dev:
+        ids32 = view("ids32").view(torch.int32)
+        ids32.copy_(topk_ids.reshape(-1))
+    if wts.dtype != torch.float32 or not wts.is_contiguous() or wts.device != dev:
+        wts = view("wts").view(torch.float32)
+        wts.copy_(topk_weights.reshape(-1))
+    gu, yd, ws, ws_bytes = at("gu"), at("yd"), at("gemv"), plan["gemv"][1]
     if not pack.covers_all or expert_maps is not None:
-        yd.zero_()                        # slots of experts held elsewhere are never written and must add nothing
+        view("yd").zero_()                # slots of experts held elsewhere are never written and must add nothing
     with torch.cuda.device(dev):
         for c, (pk, emap) in enumerate(zip(pack.packs, maps)):
-            sorted_ids, expert_ids, num_post = views[f"sorted{c}"], views[f"experts{c}"], views[f"post{c}"]
-            xf13, xf2 = views[f"xf13_{c}"], views[f"xf2_{c}"]
-            cap = sorted_ids.numel() // 4
+            sorted_ids, expert_ids, num_post = at(f"sorted{c}"), at(f"experts{c}"), at(f"post{c}")
+            xf13, xf2 = at(f"xf13_{c}"), at(f"xf2_{c}")
+            cap = plan[f"sorted{c}"][1] // 4
             K = pk.bits
             if moe_block_size(tokens, top_k, pk.num_experts) == BLOCK_SIZES[1]:
-                tc = views[f"tc{c}"]
-                tc[:256].zero_()          # this region moves with the token count: its error word starts clean
                 _lib.check(lib.exl3_moe_tc_experts(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
                                                    pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
-                                                   _ptr(pk.svh2), K, pk.codebook, _ptr(yd), _ptr(tc), tc.numel(), st), "exl3_moe_tc_experts")
+                                                   _ptr(pk.svh2), K, pk.codebook, yd, at(f"tc{c}"), plan[f"tc{c}"][1], st), "exl3_moe_tc_experts")
                 continue
-            _lib.check(lib.exl3_moe_align_mapped(_ptr(ids32), slots, emap.numel(), _ptr(emap), pk.num_experts, _ptr(sorted_ids), cap,
-                                                 _ptr(expert_ids), _ptr(num_post), st), "exl3_moe_align_mapped")
-            _lib.check(lib.exl3_moe_had_in(_ptr(x), _dtype_code(x), _ptr(pk.suh13), 2, hidden, top_k, slots, _ptr(sorted_ids), cap,
-                                           _ptr(expert_ids), _ptr(num_post), pk.codebook, _ptr(xf13), st), "exl3_moe_had_in")
-            _lib.check(lib.exl3_moe_gemm(_ptr(xf13), _ptr(pk.w13), K, pk.codebook, _ptr(pk.svh13), _ptr(sorted_ids), _ptr(expert_ids),
-                                         _ptr(num_post), cap, slots, hidden, 2 * inter, inter, _ptr(gu), _ptr(ws), ws.numel(), st),
+            _lib.check(lib.exl3_moe_align_mapped(_ptr(ids32), slots, emap.numel(), _ptr(emap), pk.num_experts, sorted_ids, cap,
+                                                 expert_ids, num_post, st), "exl3_moe_align_mapped")
+            _lib.check(lib.exl3_moe_had_in(_ptr(x), _dtype_code(x), _ptr(pk.suh13), 2, hidden, top_k, slots, sorted_ids, cap,
+                                           expert_ids, num_post, pk.codebook, xf13, st), "exl3_moe_had_in")
+            _lib.check(lib.exl3_moe_gemm(xf13, _ptr(pk.w13), K, pk.codebook, _ptr(pk.svh13), sorted_ids, expert_ids,
+                                         num_post, cap, slots, hidden, 2 * inter, inter, gu, ws, ws_bytes, st),
                        "exl3_moe_gemm")
-            _lib.check(lib.exl3_moe_glu_had_in(_ptr(gu), _ptr(pk.suh2), inter, slots, _ptr(sorted_ids), cap, _ptr(expert_ids),
-                                               _ptr(num_post), pk.codebook, _ptr(xf2), st), "exl3_moe_glu_had_in")
-            _lib.check(lib.exl3_moe_gemm(_ptr(xf2), _ptr(pk.w2), K, pk.codebook, _ptr(pk.svh2), _ptr(sorted_ids), _ptr(expert_ids),
-                                         _ptr(num_post), cap, slots, inter, hidden, 0, _ptr(yd), _ptr(ws), ws.numel(), st),
+            _lib.check(lib.exl3_moe_glu_had_in(gu, _ptr(pk.suh2), inter, slots, sorted_ids, cap, expert_ids,
+                                               num_post, pk.codebook, xf2, st), "exl3_moe_glu_had_in")
+            _lib.check(lib.exl3_moe_gemm(xf2, _ptr(pk.w2), K, pk.codebook, _ptr(pk.svh2), sorted_ids, expert_ids,
+                                         num_post, cap, slots, inter, hidden, 0, yd, ws, ws_bytes, st),
                        "exl3_moe_gemm")
-        _lib.check(lib.exl3_moe_combine(_ptr(yd), _ptr(wts), _ptr(ids32), tokens, top_k, hidden, maps[0].numel(), _ptr(out),
+        _lib.check(lib.exl3_moe_combine(yd, _ptr(wts), _ptr(ids32), tokens, top_k, hidden, maps[0].numel(), _ptr(out),
                                         _dtype_code(out), st), "exl3_moe_combine")
     return out
 
