@@ -26,7 +26,7 @@ namespace exl3 {
 constexpr int MOE_BLOCK_ROWS = 8;
 constexpr int MOE_MAX_GRID = 192;                                // CTAs of a launch (one per SM)
 constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word, then the counters
-constexpr int MOE_X_SLOTS = 8;                                   // most slots of the activation ring
+constexpr int MOE_X_SLOTS = 4, MOE_X_UNITS = 4;                  // most slots of the activation ring, and units of a slot
 constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, then the constants of the decode loop
 // Largest expert count of one routing alignment: its single CTA keeps three counters per expert in the default 48 KB of
 // shared memory ((3 * E + 1) * 4 bytes + 280 static).
@@ -183,10 +183,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     }
     const long long u0 = gemv_first_unit(cta, units_q, units_r);
     const int units = units_q + (cta < units_r ? 1 : 0), fills = (units + ups - 1) / ups;
-    // Activation ring: the same slot size and count for every warp.
-    const uint32_t slot_bytes = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : MOE_BLOCK_ROWS * F_ROW;
-    int x_slots = slot_bytes > 0 ? (int)(p.x_bytes / slot_bytes) : 1;
-    if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
+    // Activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory.  A bulk
+    // copy costs a few hundred nanoseconds whatever its size: one per unit of eight rows would be slower than the decode.
+    const uint32_t x_unit = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : MOE_BLOCK_ROWS * F_ROW;
+    int x_units = MOE_X_UNITS, x_slots = MOE_X_SLOTS;
+    if (LIST && x_unit > 0) {
+        while (x_units > 1 && p.x_bytes / (x_unit * x_units) < 3) x_units--;
+        x_slots = (int)(p.x_bytes / (x_unit * x_units));
+        if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
+    }
+    const uint32_t slot_bytes = x_unit * x_units;
     int item = units <= 0 ? 0 : total < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
     int in_item = units > 0 ? (int)(u0 - (long long)item * UB) : 0;
     auto item_of = [&](int i) {                                             // expert, first row, rows
@@ -259,10 +265,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         // ------------------------------------------------------------------ MMA issue, all groups in unit order
         const uint32_t s_bar = ptx::smem_addr(stage_empty), xe_bar = ptx::smem_addr(x_empty), xf_bar = ptx::smem_addr(x_full);
         const uint32_t empty0 = ptx::smem_addr(buf_empty), done0 = ptx::smem_addr(acc_done), xs_addr = ptx::smem_addr(xs);
-        uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, accumulate = 0, acc = 0, idesc = 0, pitch = MOE_BLOCK_ROWS;
+        uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, accumulate = 0, acc = 0, idesc = 0, pitch = MOE_BLOCK_ROWS, b_lo = 0;
         int left = ups, third = 0;
         // Half `HF` (0, 1) of a unit whose number is `C` modulo three: group and buffer are constants of the code.
-        auto half = [&](auto cconst, auto hconst, uint32_t b_lo, bool stage_end) {
+        auto half = [&](auto cconst, auto hconst, uint32_t b_lo, bool run_end, bool stage_end) {
             constexpr int PH = 2 * decltype(cconst)::value + decltype(hconst)::value, G = PH % 3, BUF = PH / 3;
             ptx::named_bar_sync(SK_BAR_BUF + G * 2 + BUF, (8 + 1) * 32);
             sk_fence_after();
@@ -272,17 +278,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 for (int m = 0; m < MMAS; m++) sk_mma(acc, A_OFF + (G * 2 + BUF) * A_COLS + m * 8, b + m * 2u * pitch, idesc, m > 0 ? 1u : accumulate);
                 sk_commit_addr(empty0 + (G * 2 + BUF) * 8u);
                 if (decltype(hconst)::value == 1) {
-                    sk_commit_addr(xe_bar + x_slot * 8u);
+                    if (run_end) sk_commit_addr(xe_bar + x_slot * 8u);
                     if (stage_end) sk_commit_addr(s_bar + stage8);
                 }
             }
             __syncwarp();
             accumulate = 1;
         };
-        auto unit = [&](auto cconst, bool stage_end) {
-            const uint32_t b_lo = (pitch << 16) | ((xs_addr + x_slot * slot_bytes) >> 4);
-            half(cconst, std::integral_constant<int, 0>{}, b_lo, false);
-            half(cconst, std::integral_constant<int, 1>{}, b_lo + pitch * (F_ROW / 32), stage_end);      // half a unit, in units of 16 bytes
+        auto unit = [&](auto cconst, uint32_t b_lo, bool run_end, bool stage_end) {
+            half(cconst, std::integral_constant<int, 0>{}, b_lo, false, false);
+            half(cconst, std::integral_constant<int, 1>{}, b_lo + pitch * (F_ROW / 32), run_end, stage_end);      // half a unit, in units of 16 bytes
         };
         int done = 0;
 #pragma unroll 1
@@ -296,21 +301,29 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             acc = d * NMAX;
             accumulate = 0;
 #pragma unroll 1
-            for (int u = 0; u < count; u++) {
-                sk_wait(xf_bar + x_slot * 8u, x_parity, failed);
+            for (int u = 0, r = 0; u < count; u++) {
+                if (r == 0) {
+                    sk_wait(xf_bar + x_slot * 8u, x_parity, failed);
+                    b_lo = (pitch << 16) | ((xs_addr + x_slot * slot_bytes) >> 4);
+                }
                 left--;
-                const bool stage_end = left == 0;
-                if (third == 0) unit(std::integral_constant<int, 0>{}, stage_end);
-                else if (third == 1) unit(std::integral_constant<int, 1>{}, stage_end);
-                else unit(std::integral_constant<int, 2>{}, stage_end);
+                const bool stage_end = left == 0, run_end = r + 1 == x_units || u + 1 == count;
+                if (third == 0) unit(std::integral_constant<int, 0>{}, b_lo, run_end, stage_end);
+                else if (third == 1) unit(std::integral_constant<int, 1>{}, b_lo, run_end, stage_end);
+                else unit(std::integral_constant<int, 2>{}, b_lo, run_end, stage_end);
                 third = third == 2 ? 0 : third + 1;
                 if (stage_end) {
                     left = ups;
                     stage8 = stage8 + 8 == (uint32_t)stages * 8u ? 0 : stage8 + 8;
                 }
-                if (++x_slot == (uint32_t)x_slots) {
-                    x_slot = 0;
-                    x_parity ^= 1;
+                b_lo += pitch * (F_ROW / 16);
+                r++;
+                if (run_end) {
+                    r = 0;
+                    if (++x_slot == (uint32_t)x_slots) {
+                        x_slot = 0;
+                        x_parity ^= 1;
+                    }
                 }
             }
             if (sk_elect()) sk_commit_addr(done0 + d * 8u);
@@ -340,28 +353,35 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             kg = 0;
         }
     } else if (warp == SK_MMA_WARP + 2) {
-        // ------------------------------------------------------------------ copies of activations, a unit per slot
+        // ------------------------------------------------------------------ copies of activations, a run of units per slot
         if (lane == 0 && units > 0) {
-            int slot = 0;
+            int slot = 0, runs = 0;
             uint32_t phase = 1;                                             // the first lap's slots are free
             int3 it = item_of(item);
-            for (int j = 0; j < units; j++) {
+            int nb = in_item / p.KG, kg = in_item - nb * p.KG;
+            for (int j = 0; j < units; runs++) {
+                int n = p.KG - kg < units - j ? p.KG - kg : units - j;
+                if (n > x_units) n = x_units;
+                const uint32_t unit = (uint32_t)it.z * F_ROW, bytes = (uint32_t)n * unit;
+                const unsigned char* src = p.xf + (nb >= p.shard_end_block ? p.xf_shard_stride : 0) + ((long long)it.y * p.KG * F_ROW + (long long)kg * unit);
                 if (!failed && !ptx::mbar_wait_relaxed(&x_empty[slot], phase, 50)) failed = 1;
-                const int nb = in_item / p.KG, kg = in_item - nb * p.KG;
-                const uint32_t bytes = (uint32_t)it.z * F_ROW;
-                const unsigned char* src = p.xf + (nb >= p.shard_end_block ? p.xf_shard_stride : 0) + ((long long)it.y * p.KG + (long long)kg * it.z) * F_ROW;
                 ptx::mbar_arrive_expect_tx(&x_full[slot], bytes);
                 ptx::bulk_g2s(xs + (size_t)slot * slot_bytes, src, bytes, &x_full[slot]);
                 if (++slot == x_slots) {
                     slot = 0;
                     phase ^= 1;
                 }
-                if (++in_item == UB) {
-                    in_item = 0;
-                    if (j + 1 < units) it = item_of(++item);
+                j += n;
+                kg += n;
+                if (kg == p.KG) {
+                    kg = 0;
+                    if (++nb == p.NB) {
+                        nb = 0;
+                        if (j < units) it = item_of(++item);
+                    }
                 }
             }
-            for (int j = units > x_slots ? units - x_slots : 0; j < units; j++) {       // every copy has landed before the CTA may leave
+            for (int j = runs > x_slots ? runs - x_slots : 0; j < runs; j++) {          // every copy has landed before the CTA may leave
                 uint32_t late = 0;
                 sk_wait(ptx::smem_addr(&x_full[j % x_slots]), (uint32_t)(j / x_slots) & 1u, late);
                 failed |= late;
