@@ -539,16 +539,17 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     if (!d) return EXL3_ERR_NOT_INITIALISED;
     const int grid = d->sm_count < MOE_MAX_GRID ? d->sm_count : MOE_MAX_GRID;
     // Stages of about 24 KB of weights (a bulk copy costs a few hundred nanoseconds whatever its size), two units or more per stage (see
-    // SkWalk).  Single blocks of eight rows: four slots of activations of four units, the rest of the shared memory for weights.  Long items: three
-    // stages of weights, the rest for activations (three units of 128 rows and more).
+    // SkWalk).  Single blocks of eight rows: their activations ride with the weights, as many stages as fit.  Long items: three stages of
+    // weights, the rest for activations (three units of 128 rows and more).
     const uint32_t unit = 2048u * (uint32_t)K, row = mode == GEMV_SPLIT ? 512u : 256u, tail = MOE_BLOCK_ROWS * 128 * 4, all = (uint32_t)d->max_smem_optin;
     uint32_t ups = (24u * 1024u + unit - 1) / unit;
     if (ups < 2) ups = 2;
     uint32_t stages = 3;
     if (!l.items) {
-        l.x_bytes = MOE_X_SLOTS * MOE_X_UNITS * MOE_BLOCK_ROWS * row;
-        stages = (all - MOE_BAR_BYTES - tail - l.x_bytes) / (ups * unit);
+        const uint32_t with_rows = unit + MOE_BLOCK_ROWS * row;
+        stages = (all - MOE_BAR_BYTES - tail) / (ups * with_rows);
         if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
+        l.x_bytes = stages * ups * MOE_BLOCK_ROWS * row;
     } else {
         l.x_bytes = (all - MOE_BAR_BYTES - tail - stages * ups * unit) & ~1023u;
     }

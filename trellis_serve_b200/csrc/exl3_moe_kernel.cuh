@@ -9,13 +9,15 @@
 //
 // The machinery of the dense decode GEMV (exl3_skinny_kernel.cuh): decoded registers go to tensor memory as the A operand, the rotated
 // rows are the B operand (N = rows of the item), persistent CTAs split the unit list (item, column block, row block) evenly and
-// contiguously, partial sums of column blocks cut between CTAs are added in CTA order by the last one to arrive.  Differences: item
-// list and row counts are read on the device (CUDA-graph safe), so N and the pitch of B are run-time values; the activations have a ring
-// of their own, a slot per unit, whose slot count follows the largest item; ONE warp issues the MMAs of the three decode groups in unit
-// order into one accumulator, so that 128 rows fit into tensor memory twice.  Single blocks of eight rows are finished here (output
-// rotation with the expert's svh, rows scattered to their slots); for long items that would be a third of all instructions on four of 32
-// warps (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): their rows leave in the rotated basis, as fp16, and the
-// kernels behind rotate them.
+// contiguously, partial sums of column blocks cut between CTAs are added in CTA order by the last one to arrive.  Two forms:
+//
+//   * blocks of eight rows (decode batches): the dense kernel, but for the item list that is read on the device (CUDA-graph safe), the
+//     expert's svh and the scattering of rows to their slots;
+//   * LIST, longer items: N and the pitch of B are run-time values, the activations have a ring of their own whose slot size follows
+//     the largest item, ONE warp issues the MMAs of the three decode groups in unit order into one accumulator, so that 128 rows
+//     fit into tensor memory twice.  Rotating such rows in the epilogue would be a third of all instructions on four of 32 warps
+//     (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): they leave in the rotated basis, as fp16, and the kernels
+//     behind rotate them.
 //
 // Bound by the ALU pipe of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.
 #pragma once
@@ -117,10 +119,10 @@ __device__ __forceinline__ void moe_finish_eight(const MoeGemmLaunch& p, const f
 template <int K, int MODE, int FAM, bool LIST>
 __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_constant__ MoeGemmLaunch p)
 {
-    constexpr int NMAX = LIST ? moe_item_rows(MODE) : 16;
+    constexpr int ACCS = LIST ? 1 : SK_GROUPS, NMAX = LIST ? moe_item_rows(MODE) : 16;      // accumulators of a column block, and their columns
     constexpr uint32_t W_BYTES = 2048u * K, HALF_BYTES = K * 128u;
     constexpr uint32_t F_ROW = MODE == GEMV_SPLIT ? 512u : 256u;            // bytes of a row in a unit's activations
-    constexpr int A_COLS = MODE == GEMV_SPLIT ? 64 : 32, A_OFF = 2 * NMAX, MMAS = MODE == GEMV_SPLIT ? 8 : 4;
+    constexpr int A_COLS = MODE == GEMV_SPLIT ? 64 : 32, A_OFF = 2 * ACCS * NMAX, MMAS = MODE == GEMV_SPLIT ? 8 : 4;
     static_assert(A_OFF + 2 * SK_GROUPS * A_COLS <= SK_TMEM_COLS, "tensor memory");
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* w_full = reinterpret_cast<uint64_t*>(smem);                   // weights of a stage have landed
@@ -128,8 +130,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     uint64_t* x_full = stage_empty + SK_MAX_STAGES;                         // activations of a unit
     uint64_t* x_empty = x_full + MOE_X_SLOTS;
     uint64_t* buf_empty = x_empty + MOE_X_SLOTS;                            // [group][2] multiplied
-    uint64_t* acc_done = buf_empty + 2 * SK_GROUPS;                         // [2] a column block's MMAs have completed
-    uint64_t* acc_empty = acc_done + 2;                                     // [2] read out
+    uint64_t* acc_done = buf_empty + 2 * SK_GROUPS;                         // LIST: [2] a column block's MMAs have completed; else [group]
+    uint64_t* acc_empty = acc_done + SK_GROUPS;                             // [2] read out
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* flag = reinterpret_cast<int*>(tmem_slot + 1);
     unsigned char* wring = smem + MOE_BAR_BYTES;
@@ -142,17 +144,15 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         if (lane == 0) {
             for (int s = 0; s < SK_MAX_STAGES; s++) {
                 ptx::mbar_init(&w_full[s], 1);
-                ptx::mbar_init(&stage_empty[s], 1);
+                ptx::mbar_init(&stage_empty[s], LIST ? 1 : 2 * ups);
             }
             for (int s = 0; s < MOE_X_SLOTS; s++) {
                 ptx::mbar_init(&x_full[s], 1);
                 ptx::mbar_init(&x_empty[s], 1);
             }
             for (int b = 0; b < 2 * SK_GROUPS; b++) ptx::mbar_init(&buf_empty[b], 1);
-            for (int d = 0; d < 2; d++) {
-                ptx::mbar_init(&acc_done[d], 1);
-                ptx::mbar_init(&acc_empty[d], 4);
-            }
+            for (int g = 0; g < SK_GROUPS; g++) ptx::mbar_init(&acc_done[g], 1);
+            for (int d = 0; d < 2; d++) ptx::mbar_init(&acc_empty[d], 4);
             ptx::mbar_fence_init();
         }
     } else if (warp == SK_MMA_WARP) {
@@ -183,16 +183,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     }
     const long long u0 = gemv_first_unit(cta, units_q, units_r);
     const int units = units_q + (cta < units_r ? 1 : 0), fills = (units + ups - 1) / ups;
-    // Activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory.  A bulk
-    // copy costs a few hundred nanoseconds whatever its size: one per unit of eight rows would be slower than the decode.
-    const uint32_t x_unit = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : MOE_BLOCK_ROWS * F_ROW;
-    int x_units = MOE_X_UNITS, x_slots = MOE_X_SLOTS;
+    // LIST, activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory
+    // (a bulk copy costs a few hundred nanoseconds whatever its size).
+    const uint32_t x_unit = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : 0u;
+    [[maybe_unused]] int x_units = MOE_X_UNITS, x_slots = MOE_X_SLOTS;
     if (LIST && x_unit > 0) {
         while (x_units > 1 && p.x_bytes / (x_unit * x_units) < 3) x_units--;
         x_slots = (int)(p.x_bytes / (x_unit * x_units));
         if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
     }
-    const uint32_t slot_bytes = x_unit * x_units;
+    [[maybe_unused]] const uint32_t slot_bytes = x_unit * x_units;
     int item = units <= 0 ? 0 : total < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
     int in_item = units > 0 ? (int)(u0 - (long long)item * UB) : 0;
     auto item_of = [&](int i) {                                             // expert, first row, rows
@@ -261,7 +261,80 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 parity ^= 1;
             }
         }
-    } else if (warp == SK_MMA_WARP) {
+    } else if (!LIST && warp < SK_COPY_WARP) {
+        // ------------------------------------------------------------------ MMA issue, one warp per group: as in the dense kernel
+        auto multiply = [&](auto gconst) {
+            constexpr int group = decltype(gconst)::value;
+            constexpr uint32_t F_BYTES = MOE_BLOCK_ROWS * F_ROW, chunk = MOE_BLOCK_ROWS;
+            constexpr uint32_t IDESC = (1u << 4) | ((16u >> 3) << 17) | ((128u >> 4) << 24);           // fp16 x fp16 -> fp32, M = 128, N = 16
+            constexpr uint32_t b_hi = (128u >> 4) | (1u << 14), a_base = A_OFF + (uint32_t)(group * 2) * A_COLS;
+            const uint32_t w_bar = ptx::smem_addr(w_full), s_bar = ptx::smem_addr(stage_empty), ring = (uint32_t)(stages * ups) * F_BYTES;
+            auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
+            SkWalk at(group, ups, fills, enter);
+            uint32_t xa = ptx::smem_addr(xs) + (group >> 1) * F_BYTES + (group & 1) * (F_BYTES / 2);
+            const uint32_t empty0 = ptx::smem_addr(&buf_empty[group * 2]), done_bar = ptx::smem_addr(&acc_done[group]);
+            uint32_t d = 0, acc_parity = 1, done_parity = 0, acc = 0, accumulate = 0;
+            int h = group, done = 0, kg = in_item % p.KG;
+            auto step = [&](auto which) {
+                constexpr int S = decltype(which)::value;
+                constexpr uint32_t half = S == 0 ? group & 1 : 1 - (group & 1);
+                if (at.left <= 0 && at.settle(ups, stages, enter)) xa -= ring;
+                const uint64_t b = ((uint64_t)b_hi << 32) | (chunk << 16) | (xa >> 4);
+                ptx::named_bar_sync(SK_BAR_BUF + group * 2 + S, (8 + 1) * 32);
+                sk_fence_after();
+                if (sk_elect()) {
+#pragma unroll
+                    for (int m = 0; m < MMAS; m++) sk_mma(acc, a_base + S * A_COLS + m * 8, b + m * 2u * chunk, IDESC, m > 0 ? 1u : accumulate);
+                    sk_commit_addr(empty0 + S * 8u);
+                    sk_commit_addr(s_bar + at.slot8);
+                }
+                __syncwarp();
+                accumulate = 1;
+                xa += half ? 2 * F_BYTES - F_BYTES / 2 : F_BYTES + F_BYTES / 2;
+                at.left -= 1 + half;
+                h += SK_GROUPS;
+            };
+            bool second = false;                                            // which of the two steps comes next
+#pragma unroll 1
+            while (done < units) {                                          // column blocks of the CTA
+                done += p.KG - kg < units - done ? p.KG - kg : units - done;
+                kg = 0;
+                const int he = 2 * done;
+                sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
+                sk_fence_after();
+                acc = (d * SK_GROUPS + group) * NMAX;
+                accumulate = 0;
+#pragma unroll 1
+                while (h < he) {
+                    if (!second) {
+                        step(std::integral_constant<int, 0>{});
+                        if (h >= he) {
+                            second = true;
+                            break;
+                        }
+                    }
+                    step(std::integral_constant<int, 1>{});
+                    second = false;
+                }
+                if (accumulate) {                                           // else the group had no half unit of this block
+                    if (sk_elect()) sk_commit_addr(done_bar);
+                    __syncwarp();
+                    sk_wait(done_bar, done_parity, failed);
+                    done_parity ^= 1;
+                    sk_fence_after();
+                    sk_fence_before();
+                }
+                sk_bar_arrive(SK_BAR_ACC + (int)d, (SK_GROUPS + 4) * 32);
+                d ^= 1;
+                if (d == 0) acc_parity ^= 1;
+            }
+        };
+        if (units > 0) {
+            if (warp == SK_MMA_WARP) multiply(std::integral_constant<int, 0>{});
+            else if (warp == SK_MMA_WARP + 1) multiply(std::integral_constant<int, 1>{});
+            else multiply(std::integral_constant<int, 2>{});
+        }
+    } else if (LIST && warp == SK_MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue, all groups in unit order
         const uint32_t s_bar = ptx::smem_addr(stage_empty), xe_bar = ptx::smem_addr(x_empty), xf_bar = ptx::smem_addr(x_full);
         const uint32_t empty0 = ptx::smem_addr(buf_empty), done0 = ptx::smem_addr(acc_done), xs_addr = ptx::smem_addr(xs);
@@ -337,7 +410,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 item++;
             }
         }
-    } else if (warp == SK_MMA_WARP + 1) {
+    } else if (LIST && warp == SK_MMA_WARP + 1) {
         // ------------------------------------------------------------------ "column block multiplied": polls for the four epilogue warps
         uint32_t d = 0, parity = 0;
         int done = 0, kg = units > 0 ? in_item % p.KG : 0;
@@ -352,7 +425,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             done += p.KG - kg;
             kg = 0;
         }
-    } else if (warp == SK_MMA_WARP + 2) {
+    } else if (LIST && warp == SK_MMA_WARP + 2) {
         // ------------------------------------------------------------------ copies of activations, a run of units per slot
         if (lane == 0 && units > 0) {
             int slot = 0, runs = 0;
@@ -389,17 +462,19 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         }
         __syncwarp();
     } else if (warp == SK_COPY_WARP) {
-        // ------------------------------------------------------------------ copies of weights
+        // ------------------------------------------------------------------ copies of weights; eight rows: the activations ride with them
         if (lane == 0 && units > 0) {
             int slot = 0, todo = units;
             uint32_t phase = 1;
             int e = item_of(item).x;
+            [[maybe_unused]] int x_item = item, x_nb = in_item / p.KG, x_kg = in_item - x_nb * p.KG;
             for (int j = 0; j < fills; j++) {
                 if (!failed && !ptx::mbar_wait_relaxed(&stage_empty[slot], phase, 100)) failed = 1;
                 int n = todo < ups ? todo : ups;
                 todo -= n;
                 unsigned char* dst = wring + (size_t)(slot * ups) * W_BYTES;
-                ptx::mbar_arrive_expect_tx(&w_full[slot], (uint32_t)n * W_BYTES);
+                ptx::mbar_arrive_expect_tx(&w_full[slot], (uint32_t)n * (W_BYTES + (LIST ? 0u : MOE_BLOCK_ROWS * F_ROW)));
+                [[maybe_unused]] int xn = n;
                 while (n > 0) {
                     const int run = UB - in_item < n ? UB - in_item : n;     // up to the end of this expert's matrix
                     ptx::bulk_g2s(dst, p.packed + (long long)e * p.expert_stride + (long long)in_item * (512 * K), (uint32_t)run * W_BYTES, &w_full[slot]);
@@ -410,6 +485,25 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                         in_item = 0;
                         item++;
                         if (n + todo > 0) e = item_of(item).x;
+                    }
+                }
+                if constexpr (!LIST) {
+                    constexpr uint32_t F_BYTES = MOE_BLOCK_ROWS * F_ROW;
+                    unsigned char* to = xs + (size_t)(slot * ups) * F_BYTES;
+                    while (xn > 0) {                                        // runs of row blocks of a column block are consecutive in memory
+                        const int run = p.KG - x_kg < xn ? p.KG - x_kg : xn;
+                        const unsigned char* src = p.xf + (x_nb >= p.shard_end_block ? p.xf_shard_stride : 0) + ((long long)x_item * p.KG + x_kg) * F_BYTES;
+                        ptx::bulk_g2s(to, src, (uint32_t)run * F_BYTES, &w_full[slot]);
+                        to += (size_t)run * F_BYTES;
+                        xn -= run;
+                        x_kg += run;
+                        if (x_kg == p.KG) {
+                            x_kg = 0;
+                            if (++x_nb == p.NB) {
+                                x_nb = 0;
+                                x_item++;
+                            }
+                        }
                     }
                 }
                 if (++slot == stages) {
@@ -448,14 +542,24 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 for (int e = 0; e < 8; e++) dst[(long long)(r0 + e) * p.n_total] = __float2half_rn(v[e]);
             };
             // Tensor memory -> shared memory or the CTA's slab: lane = output column.
+            const int hb = 2 * done, he = 2 * (done + count);
             auto load_rows = [&](int c, float (&v)[8]) {
-                uint32_t r[8];
-                sk_load8(((uint32_t)(ew * 32) << 16) + (uint32_t)(d * NMAX + c), r);
+                uint32_t r[ACCS][8];
+#pragma unroll
+                for (int g = 0; g < ACCS; g++) sk_load8(((uint32_t)(ew * 32) << 16) + (uint32_t)((d * ACCS + g) * NMAX + c), r[g]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    asm volatile("" : "+r"(r[e]));
-                    v[e] = __uint_as_float(r[e]);
+                for (int g = 0; g < ACCS; g++)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) asm volatile("" : "+r"(r[g][e]));       // no use of the registers moves ahead of the wait
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = LIST ? __uint_as_float(r[0][e]) : 0.f;
+                if constexpr (!LIST) {
+#pragma unroll
+                    for (int g = 0; g < ACCS; g++)
+                        if (hb + (g + 3 - hb % 3) % 3 < he)                 // else the group had no half unit of this block
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[e] += __uint_as_float(r[g][e]);
                 }
             };
             auto read_rows = [&](int rows, float* to) {
@@ -472,7 +576,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&acc_empty[d]);
             };
-            ptx::named_bar_sync(SK_BAR_ACC + d, (1 + 4) * 32);
+            ptx::named_bar_sync(SK_BAR_ACC + d, (ACCS + 4) * 32);
             sk_fence_after();
             if (shared) {
                 const size_t slab = (size_t)p.slab_rows * 128;
