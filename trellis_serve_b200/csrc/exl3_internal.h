@@ -125,7 +125,7 @@ int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int 
 int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
                          const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st);
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
-                         const int* num_post, __half* yd, cudaStream_t st);
+                         const int* num_post, const int2* blk, __half* yd, cudaStream_t st);
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,
                        int y_bf16, cudaStream_t st);
 

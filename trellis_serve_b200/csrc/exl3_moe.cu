@@ -263,7 +263,7 @@ __device__ __forceinline__ void moe_unrotate32(const uint32_t (&w)[16], const ui
 // 2048 columns).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
 constexpr int MOE_SPAN = 4;
 struct MoeSpan {
-    int b, kg0, kg1, row, slot, ex;
+    int b, kg0, kg1, slot, ex;
     bool valid, any;
     __device__ __forceinline__ MoeSpan(int kgs, int cap, int numel, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                        const int* __restrict__ num_post)
@@ -276,16 +276,16 @@ struct MoeSpan {
         any = false;
         if (b >= cap / MOE_BLOCK_ROWS) return;
         const int post = *num_post;
-        row = b * MOE_BLOCK_ROWS + (lane >> 2);
         ex = expert_ids[b];
-        slot = sorted_ids[row];
+        slot = sorted_ids[b * MOE_BLOCK_ROWS + (lane >> 2)];
         any = b * MOE_BLOCK_ROWS < post;
         valid = any && slot >= 0 && slot < numel;
     }
 };
 
-// xf[shard][item][row block] = Had128(fp16(x[token(p)]) * suh[expert(p), shard]) in the B-operand layout, both shards from one load of x.
-__global__ void __launch_bounds__(256, 2) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
+// xf[shard][item][row block] = Had128(fp16(x[token(p)]) * suh[expert(p), shard]) in the B-operand layout; blockIdx.y = shard (both
+// shards from one load of x cost 128 registers and a third of the warps in flight).
+__global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
                                                             int numel, int cap, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                                             const int* __restrict__ num_post, const int2* __restrict__ blk,
                                                             unsigned char* __restrict__ xf, long long shard_stride)
@@ -298,14 +298,13 @@ __global__ void __launch_bounds__(256, 2) moe_had_in_kernel(const void* __restri
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
     const long long x_row = (long long)(at.valid ? at.slot / top_k : 0) * hidden + 32 * q;
-    const __half* signs = suh + (long long)at.ex * 2 * hidden + 32 * q;
-    unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
+    const __half* signs = suh + ((long long)at.ex * gridDim.y + blockIdx.y) * hidden + 32 * q;
+    unsigned char* unit = xf + blockIdx.y * shard_stride + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
-        uint32_t xw[16], sw[2][16];
+        uint32_t xw[16], sw[16];
         moe_load32(x, x_row + kg * 128, xw);
-        moe_load32(signs, kg * 128, sw[0]);
-        moe_load32(signs, hidden + kg * 128, sw[1]);
+        moe_load32(signs, kg * 128, sw);
         if (x_bf16) {
 #pragma unroll
             for (int i = 0; i < 16; i++) {
@@ -314,14 +313,11 @@ __global__ void __launch_bounds__(256, 2) moe_had_in_kernel(const void* __restri
                 xw[i] = *reinterpret_cast<const uint32_t*>(&h);
             }
         }
+        float v[32];
 #pragma unroll
-        for (int s = 0; s < 2; s++) {
-            float v[32];
-#pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = moe_half(xw, i) * moe_half(sw[s], i);
-            fwht128_quad(v, lane);
-            if (at.valid) moe_store_rows(unit + s * shard_stride, rows, row, q, v);
-        }
+        for (int i = 0; i < 32; i++) v[i] = moe_half(xw, i) * moe_half(sw, i);
+        fwht128_quad(v, lane);
+        if (at.valid) moe_store_rows(unit, rows, row, q, v);
     }
 }
 
@@ -338,15 +334,15 @@ __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restric
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
-    const __half* gu = gu_rot + (long long)at.row * 2 * inter + 32 * q;
+    const __half* gu = gu_rot + (long long)run.x * MOE_BLOCK_ROWS * 2 * inter + row * 128 + 32 * q;      // [column block][row][128]
     const __half* sv = svh13 + (long long)at.ex * 2 * inter + 32 * q;
     const __half* s2 = suh2 + (long long)at.ex * inter + 32 * q;
     unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
         uint32_t gw[16], uw[16], sg[16], su[16], sw[16];
-        moe_load32(gu, kg * 128, gw);
-        moe_load32(gu, inter + kg * 128, uw);
+        moe_load32(gu, (long long)kg * rows * 128, gw);
+        moe_load32(gu, (long long)(kgs + kg) * rows * 128, uw);
         moe_load32(sv, kg * 128, sg);
         moe_load32(sv, inter + kg * 128, su);
         moe_load32(s2, kg * 128, sw);
@@ -361,22 +357,24 @@ __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restric
 }
 
 // yd[slot(row), :] = fp16( Had128(yd_rot[row]) * svh2[expert] ).
-__global__ void __launch_bounds__(256, 2) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
+__global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
                                                          const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
-                                                         const int* __restrict__ num_post, __half* __restrict__ yd)
+                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, __half* __restrict__ yd)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3;
     const MoeSpan at(hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
-    const __half* src = yd_rot + (long long)at.row * hidden + 32 * q;
+    const int2 run = blk[at.b];
+    const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
+    const __half* src = yd_rot + (long long)run.x * MOE_BLOCK_ROWS * hidden + row * 128 + 32 * q;            // [column block][row][128]
     const __half* sv = svh2 + (long long)at.ex * hidden + 32 * q;
     __half* dst = yd + (long long)(at.valid ? at.slot : 0) * hidden + 32 * q;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++) {
         uint32_t w[16], sw[16];
-        moe_load32(src, kg * 128, w);
+        moe_load32(src, (long long)kg * rows * 128, w);
         moe_load32(sv, kg * 128, sw);
         float v[32];
         moe_unrotate32(w, sw, lane, v);
@@ -505,7 +503,7 @@ int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int n
 int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
                             const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st)
 {
-    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden)), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
+    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
                           expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride);
 }
 
@@ -517,10 +515,10 @@ int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half
 }
 
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
-                         const int* num_post, __half* yd, cudaStream_t st)
+                         const int* num_post, const int2* blk, __half* yd, cudaStream_t st)
 {
     return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
-                          num_post, yd);
+                          num_post, blk, yd);
 }
 
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,

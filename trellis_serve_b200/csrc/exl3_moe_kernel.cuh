@@ -42,7 +42,7 @@ struct MoeGemmLaunch {
     const unsigned char* xf;         // rotated rows: item at first row * KG * F, unit row block at + kg * rows * F, [k chunk][row] 16 bytes
     long long xf_shard_stride;       // bytes between shards
     const __half* svh;               // [E][n_total]
-    __half* out;                     // fp16: [slots][n_total], or with items [rows][n_total] in the rotated basis
+    __half* out;                     // fp16: [slots][n_total], or with items [item][column block][row][128] in the rotated basis
     const int* sorted_ids;           // slot of each row, >= numel for padding
     const int* expert_ids;           // expert of each block of eight rows
     const int4* items;               // (expert, first block, blocks, 0), or null: every block of eight rows is an item
@@ -340,27 +340,26 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         const uint32_t empty0 = ptx::smem_addr(buf_empty), done0 = ptx::smem_addr(acc_done), xs_addr = ptx::smem_addr(xs);
         uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, accumulate = 0, acc = 0, idesc = 0, pitch = MOE_BLOCK_ROWS, b_lo = 0;
         int left = ups, third = 0;
-        // Half `HF` (0, 1) of a unit whose number is `C` modulo three: group and buffer are constants of the code.
-        auto half = [&](auto cconst, auto hconst, uint32_t b_lo, bool run_end, bool stage_end) {
-            constexpr int PH = 2 * decltype(cconst)::value + decltype(hconst)::value, G = PH % 3, BUF = PH / 3;
-            ptx::named_bar_sync(SK_BAR_BUF + G * 2 + BUF, (8 + 1) * 32);
+        // A unit whose number is `C` modulo three: groups and buffers of its two halves are constants of the code.  A unit at a time, with as
+        // few instructions as possible: this warp gets an eighth of its scheduler's issue slots.
+        auto unit = [&](auto cconst, bool run_end, bool stage_end) {
+            constexpr int C = decltype(cconst)::value, G0 = (2 * C) % 3, B0 = (2 * C) / 3, G1 = (2 * C + 1) % 3, B1 = (2 * C + 1) / 3;
+            ptx::named_bar_sync(SK_BAR_BUF + G0 * 2 + B0, (8 + 1) * 32);
+            ptx::named_bar_sync(SK_BAR_BUF + G1 * 2 + B1, (8 + 1) * 32);
             sk_fence_after();
             const uint64_t b = ((uint64_t)((128u >> 4) | (1u << 14)) << 32) | b_lo;
             if (sk_elect()) {
 #pragma unroll
-                for (int m = 0; m < MMAS; m++) sk_mma(acc, A_OFF + (G * 2 + BUF) * A_COLS + m * 8, b + m * 2u * pitch, idesc, m > 0 ? 1u : accumulate);
-                sk_commit_addr(empty0 + (G * 2 + BUF) * 8u);
-                if (decltype(hconst)::value == 1) {
-                    if (run_end) sk_commit_addr(xe_bar + x_slot * 8u);
-                    if (stage_end) sk_commit_addr(s_bar + stage8);
-                }
+                for (int m = 0; m < 2 * MMAS; m++)
+                    sk_mma(acc, A_OFF + (m < MMAS ? (G0 * 2 + B0) * A_COLS + m * 8 : (G1 * 2 + B1) * A_COLS + (m - MMAS) * 8), b + m * 2u * pitch, idesc,
+                           m > 0 ? 1u : accumulate);
+                sk_commit_addr(empty0 + (G0 * 2 + B0) * 8u);
+                sk_commit_addr(empty0 + (G1 * 2 + B1) * 8u);
+                if (run_end) sk_commit_addr(xe_bar + x_slot * 8u);
+                if (stage_end) sk_commit_addr(s_bar + stage8);
             }
             __syncwarp();
             accumulate = 1;
-        };
-        auto unit = [&](auto cconst, uint32_t b_lo, bool run_end, bool stage_end) {
-            half(cconst, std::integral_constant<int, 0>{}, b_lo, false, false);
-            half(cconst, std::integral_constant<int, 1>{}, b_lo + pitch * (F_ROW / 32), run_end, stage_end);      // half a unit, in units of 16 bytes
         };
         int done = 0;
 #pragma unroll 1
@@ -381,9 +380,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 }
                 left--;
                 const bool stage_end = left == 0, run_end = r + 1 == x_units || u + 1 == count;
-                if (third == 0) unit(std::integral_constant<int, 0>{}, b_lo, run_end, stage_end);
-                else if (third == 1) unit(std::integral_constant<int, 1>{}, b_lo, run_end, stage_end);
-                else unit(std::integral_constant<int, 2>{}, b_lo, run_end, stage_end);
+                if (third == 0) unit(std::integral_constant<int, 0>{}, run_end, stage_end);
+                else if (third == 1) unit(std::integral_constant<int, 1>{}, run_end, stage_end);
+                else unit(std::integral_constant<int, 2>{}, run_end, stage_end);
                 third = third == 2 ? 0 : third + 1;
                 if (stage_end) {
                     left = ups;
@@ -416,7 +415,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         int done = 0, kg = units > 0 ? in_item % p.KG : 0;
 #pragma unroll 1
         while (done < units) {
-            if (!failed && !ptx::mbar_wait_relaxed(&acc_done[d], parity, 20)) failed = 1;
+            if (!failed && !ptx::mbar_wait_relaxed(&acc_done[d], parity, 60)) failed = 1;
             sk_fence_after();
             sk_fence_before();
             sk_bar_arrive(SK_BAR_ACC + (int)d, (1 + 4) * 32);
@@ -521,14 +520,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     } else {
         // ------------------------------------------------------------------ epilogue
         const int ew = warp - SK_EPI_WARP, tid = (int)threadIdx.x - SK_EPI_WARP * 32;
-        int d = 0, done = 0;
+        int d = 0, done = 0, nb = units > 0 ? in_item / p.KG : 0, kg = units > 0 ? in_item - nb * p.KG : 0;
+        int3 it = make_int3(0, 0, 0);
+        bool fresh = true;
 #pragma unroll 1
         while (done < units) {
-            const int nb = in_item / p.KG, kg = in_item - nb * p.KG, count = p.KG - kg < units - done ? p.KG - kg : units - done;
-            const int3 it = item_of(item);
-            const long long first = u0 + done - kg;                         // first unit of the column block
-            const int c_first = gemv_cta_of_unit(first, units_q, units_r), c_last = gemv_cta_of_unit(first + p.KG - 1, units_q, units_r);
-            const bool shared = c_first != c_last;
+            const int count = p.KG - kg < units - done ? p.KG - kg : units - done;
+            if (fresh) it = item_of(item);
+            const bool shared = count < p.KG;                               // the column block is cut between CTAs
+            int c_first = cta, c_last = cta;
+            if (shared) {
+                const long long first = u0 + done - kg;                     // its first unit
+                c_first = gemv_cta_of_unit(first, units_q, units_r);
+                c_last = gemv_cta_of_unit(first + p.KG - 1, units_q, units_r);
+            }
             [[maybe_unused]] uint2 sv = make_uint2(0u, 0u);
             [[maybe_unused]] int slots[2] = {-1, -1};
             if constexpr (!LIST) {                                          // requested while the block is still being multiplied
@@ -536,10 +541,11 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 slots[0] = p.sorted_ids[it.y + ew];
                 slots[1] = p.sorted_ids[it.y + ew + 4];
             }
-            __half* dst = p.out + (long long)it.y * p.n_total + nb * 128 + ew * 32 + lane;      // LIST: this lane's column
+            // LIST: rows of a column block of an item are consecutive, [item][column block][row][128]; this lane's column.
+            __half* dst = p.out + (long long)it.y * p.n_total + (long long)nb * it.z * 128 + ew * 32 + lane;
             auto store8 = [&](int r0, const float (&v)[8]) {
 #pragma unroll
-                for (int e = 0; e < 8; e++) dst[(long long)(r0 + e) * p.n_total] = __float2half_rn(v[e]);
+                for (int e = 0; e < 8; e++) dst[r0 * 128 + e * 128] = __float2half_rn(v[e]);
             };
             // Tensor memory -> shared memory or the CTA's slab: lane = output column.
             const int hb = 2 * done, he = 2 * (done + count);
@@ -625,9 +631,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             }
             d ^= 1;
             done += count;
-            in_item += count;
-            if (in_item == UB) {
-                in_item = 0;
+            kg = 0;
+            fresh = ++nb == p.NB;
+            if (fresh) {
+                nb = 0;
                 item++;
             }
         }

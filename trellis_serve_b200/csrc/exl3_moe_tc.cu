@@ -114,7 +114,7 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
     l.n_total = hidden;
     l.shard_end_block = l.NB;
     if (int rc = launch_moe_gemm(l, K, codebook, MODE, st)) return rc;
-    return launch_moe_out_items(yd_rot, svh2, hidden, slots, w.cap, sorted_ids, expert_ids, counts, yd, st);
+    return launch_moe_out_items(yd_rot, svh2, hidden, slots, w.cap, sorted_ids, expert_ids, counts, blk, yd, st);
 }
 
 }  // namespace exl3
