@@ -270,10 +270,12 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb, Codebook
 // Two hash-codebook weights rounded to fp16: half2(value(a), value(b)).
 __device__ __forceinline__ uint32_t hash_pair_rounded(uint32_t sa, uint32_t sb, CodebookConst c)
 {
-    uint32_t xa = hash_pair(sa, c), xb = hash_pair(sb, c);
-    uint32_t lo = prmt(xa, xb, 0x5410), hi = prmt(xa, xb, 0x7632);
-    __half2 v = __hadd2(*reinterpret_cast<__half2*>(&lo), *reinterpret_cast<__half2*>(&hi));
-    return *reinterpret_cast<uint32_t*>(&v);
+    // Sums inside the registers (operand selects of the add, fp16 pipe) and one permute: the other way round, two permutes and one add,
+    // loads the integer pipe that bounds the decode.
+    const uint32_t xa = hash_pair(sa, c), xb = hash_pair(sb, c);
+    const __half2 ha = *reinterpret_cast<const __half2*>(&xa), hb = *reinterpret_cast<const __half2*>(&xb);
+    const __half2 a = __hadd2(__low2half2(ha), __high2half2(ha)), b = __hadd2(__low2half2(hb), __high2half2(hb));
+    return prmt(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b), 0x5410);
 }
 
 // ---------------------------------------------------------------------------------------------- placement
@@ -358,6 +360,52 @@ __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane)
             float a, b;
             f32x2_split(p[i], a, b);
             p[i] = f32x2_fma(p[i], sign2, f32x2(__shfl_xor_sync(0xFFFFFFFFu, a, m), __shfl_xor_sync(0xFFFFFFFFu, b, m)));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) f32x2_split(p[i], v[2 * i], v[2 * i + 1]);
+}
+
+// The transform over four lanes with half the shuffles: in a cross-lane stage the two lanes of a pair exchange HALF of their values each,
+// so that every lane holds both operands of its butterflies, 32 shuffles for eight rows.  The exchange turns the layout: a row comes in
+// as 16-byte chunks dealt to the lanes in turn (v[8 i + e] of lane q is element 32 i + 8 q + e: loads of 64 consecutive bytes) and goes
+// out with 32 consecutive elements per lane (v[i] is element 32 q + i), or the other way round -- the same code.  The stages run in a
+// different order from fwht128's, with the same rounding of every sum.  Shuffles and loads share a pipe (207 of its cycles per eight rows
+// and 128 columns with fwht128_quad and 64-byte lanes, 83 % busy) that bounds the rotations of routed experts.
+__device__ __forceinline__ void fwht128_turn(float (&v)[32], int lane)
+{
+    unsigned long long p[16];
+    const unsigned long long minus = f32x2(-1.f, -1.f);
+#pragma unroll
+    for (int i = 0; i < 16; i++) p[i] = f32x2(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
+#pragma unroll
+    for (int stride = 1; stride < 16; stride <<= 1) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            if ((i & stride) == 0) {
+                const unsigned long long lo = p[i], hi = p[i + stride];
+                p[i] = f32x2_add(lo, hi);
+                p[i + stride] = f32x2_fma(hi, minus, lo);
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+        const bool upper = (lane & m) != 0;
+        const float sign = upper ? -1.f : 1.f;
+        const unsigned long long sign2 = f32x2(sign, sign), other2 = f32x2(-sign, -sign);
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            if ((i & (4 * m)) == 0) {
+                const unsigned long long send = upper ? p[i] : p[i + 4 * m], keep = upper ? p[i + 4 * m] : p[i];
+                float a, b;
+                f32x2_split(send, a, b);
+                const unsigned long long got = f32x2(__shfl_xor_sync(0xFFFFFFFFu, a, m), __shfl_xor_sync(0xFFFFFFFFu, b, m));
+                unsigned long long t;
+                asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(keep), "l"(sign2));
+                p[i] = f32x2_add(keep, got);
+                p[i + 4 * m] = f32x2_fma(got, other2, t);
+            }
         }
     }
 #pragma unroll

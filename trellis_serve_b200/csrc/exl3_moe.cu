@@ -14,17 +14,13 @@ namespace exl3 {
 // [0, E) are dropped.  The order of slots inside an expert is not specified (rows are independent).
 // With expert_map (int [E_global]: global id -> id in [0, E), or -1) the ids are translated first, so one class of a
 // mixed-bitrate expert set gets the blocks of its own slots only, with local expert ids.
-__device__ __forceinline__ int moe_mapped_id(const int* topk_ids, int i, const int* expert_map, int E_global)
-{
-    const int e = topk_ids[i];
-    if (!expert_map) return e;
-    return (e >= 0 && e < E_global) ? expert_map[e] : -1;
-}
-
 // With `items`: every expert's rows are also cut into items of up to item_blocks blocks of eight rows; items[i] = (expert, first block,
 // blocks, 0), blk[b] = (first block of the item of block b, its blocks), num_post[1] = items, num_post[2] = rows of the largest one; and
-// the counters of the grouped GEMM, and its error word ahead of them, are cleared.  One CTA: bound by latency, so the ids are requested eight at a time per thread.
-__global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
+// the counters of the grouped GEMM, and its error word ahead of them, are cleared.  One CTA: bound by latency, so the ids are requested
+// KEEP at a time per thread.  If they fit into one such pass they stay in registers, each with its rank among its expert's slots from
+// the counting pass (16384 slots 24 us with a second pass of loads and atomics, 20 without).
+template <int KEEP>
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
                                  int* __restrict__ expert_ids, int* __restrict__ num_post, const int* __restrict__ expert_map,
                                  int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ counters)
 {
@@ -34,20 +30,23 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, in
     int* count = sh;              // [E]
     int* offset = sh + E;         // [E + 1]
     int* fill = sh + 2 * E + 1;   // [E]
-    constexpr int BATCH = 8;
-    auto each_id = [&](auto use) {                      // use(slot, expert) for every slot of an expert in [0, E)
-        for (int i0 = threadIdx.x; i0 < numel; i0 += BATCH * blockDim.x) {
-            int e[BATCH];
+    const bool one = numel <= KEEP * (int)blockDim.x;
+    int e_of[KEEP], rank[KEEP];
+    auto load_ids = [&](int i0) {                       // experts of slots i0 + thread + j * threads, -1 outside [0, E)
 #pragma unroll
-            for (int j = 0; j < BATCH; j++) {
-                const int i = i0 + j * blockDim.x;
-                e[j] = i < numel ? moe_mapped_id(topk_ids, i, expert_map, E_global) : -1;
-            }
-#pragma unroll
-            for (int j = 0; j < BATCH; j++)
-                if (e[j] >= 0 && e[j] < E) use(i0 + j * (int)blockDim.x, e[j]);
+        for (int j = 0; j < KEEP; j++) {
+            const int i = i0 + threadIdx.x + j * blockDim.x;
+            e_of[j] = i < numel ? topk_ids[i] : -1;
         }
+        if (expert_map) {
+#pragma unroll
+            for (int j = 0; j < KEEP; j++) e_of[j] = e_of[j] >= 0 && e_of[j] < E_global ? expert_map[e_of[j]] : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < KEEP; j++)
+            if (e_of[j] >= E) e_of[j] = -1;
     };
+    load_ids(0);
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         count[e] = 0;
         fill[e] = 0;
@@ -55,8 +54,11 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, in
     if (items)
         for (int i = threadIdx.x; i < MOE_MAX_GRID + MOE_ERR_WORDS; i += blockDim.x) counters[i - MOE_ERR_WORDS] = 0;      // and the error word ahead of them
     __syncthreads();
-    each_id([&](int, int e) { atomicAdd(&count[e], 1); });
-    for (int i = threadIdx.x; i < cap; i += blockDim.x) sorted_ids[i] = numel;
+    for (int i0 = 0; i0 < numel; i0 += KEEP * blockDim.x) {
+        if (i0 > 0) load_ids(i0);
+#pragma unroll
+        for (int j = 0; j < KEEP; j++) rank[j] = e_of[j] >= 0 ? atomicAdd(&count[e_of[j]], 1) : 0;
+    }
     // Exclusive prefix sums of the padded counts and (high word) of the items: warp scans by shuffle, warp totals through shared
     // memory; experts are taken in chunks of blockDim.x with a running carry.
     __shared__ unsigned long long warp_total[32];
@@ -97,6 +99,7 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, in
             const int b0 = (int)(excl & 0xFFFFFFFFu) / block;
             offset[e] = b0 * block;
             for (int r = 0; r < blocks; r++) expert_ids[b0 + r] = e;
+            for (int r = count[e]; r < blocks * block; r++) sorted_ids[b0 * block + r] = numel;
             if (items) {
                 // the expert's blocks in nearly even items
                 int at = (int)(excl >> 32), first = 0;
@@ -122,16 +125,22 @@ __global__ void moe_align_kernel(const int* __restrict__ topk_ids, int numel, in
         }
     }
     for (int i = total / block + threadIdx.x; i < cap / block; i += blockDim.x) expert_ids[i] = -1;
-    each_id([&](int i, int e) { sorted_ids[offset[e] + atomicAdd(&fill[e], 1)] = i; });
+    for (int i = total + threadIdx.x; i < cap; i += blockDim.x) sorted_ids[i] = numel;
+    for (int i0 = 0; i0 < numel; i0 += KEEP * blockDim.x) {
+        if (!one) load_ids(i0);
+#pragma unroll
+        for (int j = 0; j < KEEP; j++)
+            if (e_of[j] >= 0) sorted_ids[offset[e_of[j]] + (one ? rank[j] : atomicAdd(&fill[e_of[j]], 1))] = i0 + threadIdx.x + j * blockDim.x;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ rotations
 
-// A lane's 32 values of a row, four lanes per row, in the B-operand layout of the grouped GEMM (k chunk by k chunk of eight, a 16-byte word
-// per row, `rows` rows): the warp's stores fill 128-byte lines.
+// A lane's 32 values of a row in the B-operand layout of the grouped GEMM (k chunk by k chunk of eight, a 16-byte word per row, `rows`
+// rows): the warp's stores fill 128-byte lines.  DEALT: the lane holds chunks q, q + 4, ... (see fwht128_turn), else 4 q, 4 q + 1, ...
+template <bool DEALT>
 __device__ __forceinline__ void moe_store_rows(unsigned char* unit, int rows, int row, int q, const float (&v)[32])
 {
-    unsigned char* dst = unit + ((size_t)(q * 4) * rows + row) * 16;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         uint32_t w[4];
@@ -140,17 +149,18 @@ __device__ __forceinline__ void moe_store_rows(unsigned char* unit, int rows, in
             const __half2 h = __floats2half2_rn(v[8 * j + 2 * i] * HAD_SCALE, v[8 * j + 2 * i + 1] * HAD_SCALE);
             w[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        *reinterpret_cast<uint4*>(dst + (size_t)j * rows * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(unit + ((size_t)(DEALT ? 4 * j + q : 4 * q + j) * rows + row) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// 32 halves (16-byte aligned) as packed words.
-__device__ __forceinline__ void moe_load32(const void* base, long long at, uint32_t (&w)[16])
+// A lane's 32 halves of 128 (16-byte aligned) as packed words: 32 consecutive ones, or (DEALT) 16-byte chunks q, q + 4, ...
+template <bool DEALT>
+__device__ __forceinline__ void moe_load32(const void* base, long long at, int q, uint32_t (&w)[16])
 {
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at);
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at) + (DEALT ? q : 4 * q);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint4 r = src[i];
+        const uint4 r = src[DEALT ? 4 * i : i];
         w[4 * i] = r.x;
         w[4 * i + 1] = r.y;
         w[4 * i + 2] = r.z;
@@ -252,27 +262,28 @@ __device__ __forceinline__ void moe_unrotate32(const uint32_t (&w)[16], const ui
 {
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = moe_half(w, i);
-    fwht128_quad(v, lane);
+    fwht128_turn(v, lane);
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] * (HAD_SCALE * moe_half(sw, i))));
 }
 
-// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_quad), and up to MOE_SPAN column blocks of
+// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_turn), and up to MOE_SPAN column blocks of
 // 128 of it: 16-byte loads and full-line stores, and the chain of dependent loads (block -> expert and slot -> values) is walked once
 // per span -- with one column block per warp it is what bounds these kernels (70 us instead of 22 us of traffic for 2048 tokens, top-8,
 // 2048 columns).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
-constexpr int MOE_SPAN = 4;
+constexpr int MOE_SPAN = 4, MOE_MID_SPAN = 2;
+template <int SPAN>
 struct MoeSpan {
     int b, kg0, kg1, slot, ex;
     bool valid, any;
     __device__ __forceinline__ MoeSpan(int kgs, int cap, int numel, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                        const int* __restrict__ num_post)
     {
-        const int lane = threadIdx.x & 31, spans = (kgs + MOE_SPAN - 1) / MOE_SPAN;
+        const int lane = threadIdx.x & 31, spans = (kgs + SPAN - 1) / SPAN;
         const int at = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         b = at / spans;
-        kg0 = (at - b * spans) * MOE_SPAN;
-        kg1 = kg0 + MOE_SPAN < kgs ? kg0 + MOE_SPAN : kgs;
+        kg0 = (at - b * spans) * SPAN;
+        kg1 = kg0 + SPAN < kgs ? kg0 + SPAN : kgs;
         any = false;
         if (b >= cap / MOE_BLOCK_ROWS) return;
         const int post = *num_post;
@@ -293,18 +304,18 @@ __global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restri
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3, kgs = hidden >> 7;
-    const MoeSpan at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan<MOE_SPAN> at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
-    const long long x_row = (long long)(at.valid ? at.slot / top_k : 0) * hidden + 32 * q;
-    const __half* signs = suh + ((long long)at.ex * gridDim.y + blockIdx.y) * hidden + 32 * q;
+    const long long x_row = (long long)(at.valid ? at.slot / top_k : 0) * hidden;
+    const __half* signs = suh + ((long long)at.ex * gridDim.y + blockIdx.y) * hidden;
     unsigned char* unit = xf + blockIdx.y * shard_stride + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
         uint32_t xw[16], sw[16];
-        moe_load32(x, x_row + kg * 128, xw);
-        moe_load32(signs, kg * 128, sw);
+        moe_load32<true>(x, x_row + kg * 128, q, xw);
+        moe_load32<true>(signs, kg * 128, q, sw);
         if (x_bf16) {
 #pragma unroll
             for (int i = 0; i < 16; i++) {
@@ -316,8 +327,8 @@ __global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restri
         float v[32];
 #pragma unroll
         for (int i = 0; i < 32; i++) v[i] = moe_half(xw, i) * moe_half(sw, i);
-        fwht128_quad(v, lane);
-        if (at.valid) moe_store_rows(unit, rows, row, q, v);
+        fwht128_turn(v, lane);
+        if (at.valid) moe_store_rows<false>(unit, rows, row, q, v);
     }
 }
 
@@ -330,29 +341,34 @@ __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restric
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3, kgs = inter >> 7;
-    const MoeSpan at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan<MOE_MID_SPAN> at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
-    const __half* gu = gu_rot + (long long)run.x * MOE_BLOCK_ROWS * 2 * inter + row * 128 + 32 * q;      // [column block][row][128]
-    const __half* sv = svh13 + (long long)at.ex * 2 * inter + 32 * q;
-    const __half* s2 = suh2 + (long long)at.ex * inter + 32 * q;
+    const __half* gu = gu_rot + (long long)run.x * MOE_BLOCK_ROWS * 2 * inter + row * 128;               // [column block][row][128]
+    const __half* sv = svh13 + (long long)at.ex * 2 * inter;
+    const __half* s2 = suh2 + (long long)at.ex * inter;
     unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
-        uint32_t gw[16], uw[16], sg[16], su[16], sw[16];
-        moe_load32(gu, (long long)kg * rows * 128, gw);
-        moe_load32(gu, (long long)(kgs + kg) * rows * 128, uw);
-        moe_load32(sv, kg * 128, sg);
-        moe_load32(sv, inter + kg * 128, su);
-        moe_load32(s2, kg * 128, sw);
-        float g[32], u[32];
-        moe_unrotate32(gw, sg, lane, g);
-        moe_unrotate32(uw, su, lane, u);
+        uint32_t w[16], sw[16], u[16];                        // up is fp16 by now: packed again, it leaves room for gate
+        float v[32];
+        moe_load32<true>(gu, (long long)(kgs + kg) * rows * 128, q, w);
+        moe_load32<false>(sv, inter + kg * 128, q, sw);
+        moe_unrotate32(w, sw, lane, v);
 #pragma unroll
-        for (int i = 0; i < 32; i++) g[i] = __half2float(__float2half_rn(g[i] / (1.0f + __expf(-g[i])) * u[i])) * moe_half(sw, i);
-        fwht128_quad(g, lane);
-        if (at.valid) moe_store_rows(unit, rows, row, q, g);
+        for (int i = 0; i < 16; i++) {
+            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            u[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        moe_load32<true>(gu, (long long)kg * rows * 128, q, w);
+        moe_load32<false>(sv, kg * 128, q, sw);
+        moe_unrotate32(w, sw, lane, v);
+        moe_load32<false>(s2, kg * 128, q, sw);
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] / (1.0f + __expf(-v[i])) * moe_half(u, i))) * moe_half(sw, i);
+        fwht128_turn(v, lane);
+        if (at.valid) moe_store_rows<true>(unit, rows, row, q, v);
     }
 }
 
@@ -364,18 +380,18 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3;
-    const MoeSpan at(hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan<MOE_SPAN> at(hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
-    const __half* src = yd_rot + (long long)run.x * MOE_BLOCK_ROWS * hidden + row * 128 + 32 * q;            // [column block][row][128]
-    const __half* sv = svh2 + (long long)at.ex * hidden + 32 * q;
-    __half* dst = yd + (long long)(at.valid ? at.slot : 0) * hidden + 32 * q;
+    const __half* src = yd_rot + (long long)run.x * MOE_BLOCK_ROWS * hidden + row * 128;                     // [column block][row][128]
+    const __half* sv = svh2 + (long long)at.ex * hidden;
+    __half* dst = yd + (long long)(at.valid ? at.slot : 0) * hidden + 8 * q;
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++) {
         uint32_t w[16], sw[16];
-        moe_load32(src, (long long)kg * rows * 128, w);
-        moe_load32(sv, kg * 128, sw);
+        moe_load32<false>(src, (long long)kg * rows * 128, q, w);
+        moe_load32<true>(sv, kg * 128, q, sw);
         float v[32];
         moe_unrotate32(w, sw, lane, v);
         if (!at.valid) continue;
@@ -387,7 +403,7 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
                 const __half2 h = __floats2half2_rn(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
                 o[j] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            reinterpret_cast<uint4*>(dst + kg * 128)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<uint4*>(dst + kg * 128)[4 * i] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
 }
@@ -473,15 +489,15 @@ static inline unsigned blocks_for(long long items, int per_block) { return (unsi
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
                      const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* counters, cudaStream_t st)
 {
-    return launch_chained(moe_align_kernel, dim3(1), dim3(1024), (3 * E + 1) * sizeof(int), st, topk_ids, numel, E, block, cap, sorted_ids, expert_ids,
+    return launch_chained(numel <= 2048 ? moe_align_kernel<2> : moe_align_kernel<16>, dim3(1), dim3(1024), (3 * E + 1) * sizeof(int), st, topk_ids, numel, E, block, cap, sorted_ids, expert_ids,
                           num_post, expert_map, E_global, item_blocks, items, blk, counters);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-static unsigned span_blocks(int cap, int cols)      // CTAs of eight warps, a warp per (block of eight rows, span)
+static unsigned span_blocks(int cap, int cols, int span)      // CTAs of eight warps, a warp per (block of eight rows, span)
 {
-    return blocks_for((long long)(cap / MOE_BLOCK_ROWS) * ((cols / 128 + MOE_SPAN - 1) / MOE_SPAN), 8);
+    return blocks_for((long long)(cap / MOE_BLOCK_ROWS) * ((cols / 128 + span - 1) / span), 8);
 }
 
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
@@ -503,21 +519,21 @@ int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int n
 int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
                             const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st)
 {
-    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
+    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden, MOE_SPAN), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
                           expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride);
 }
 
 int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
                          const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st)
 {
-    return launch_chained(moe_mid_kernel, dim3(span_blocks(cap, inter)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
+    return launch_chained(moe_mid_kernel, dim3(span_blocks(cap, inter, MOE_MID_SPAN)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
                           num_post, blk, reinterpret_cast<unsigned char*>(xf));
 }
 
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
                          const int* num_post, const int2* blk, __half* yd, cudaStream_t st)
 {
-    return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
+    return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden, MOE_SPAN)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
                           num_post, blk, yd);
 }
 

@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     ptx::grid_dependency_wait();                                            // the item list comes from kernels ahead in the stream
 
     const int UB = p.NB * p.KG;                                             // units per item
-    // Values read from memory go through a shuffle where MMA operands depend on them: warp-uniform to the compiler.
-    const int n_items = __shfl_sync(0xFFFFFFFFu, LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS, 0);
+    // Values read from memory go through a reduction where MMA operands depend on them: its result is a uniform register.
+    const int n_items = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)(LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS));
     const long long total = (long long)n_items * UB;
     int units_q, units_r;
     if (total < (1ll << 31)) {                                              // the 64-bit division is a few hundred clocks of everyone's start
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     const int units = units_q + (cta < units_r ? 1 : 0), fills = (units + ups - 1) / ups;
     // LIST, activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory
     // (a bulk copy costs a few hundred nanoseconds whatever its size).
-    const uint32_t x_unit = LIST ? (uint32_t)__shfl_sync(0xFFFFFFFFu, p.counts[2], 0) * F_ROW : 0u;
+    const uint32_t x_unit = LIST ? __reduce_max_sync(0xFFFFFFFFu, (unsigned)p.counts[2]) * F_ROW : 0u;
     [[maybe_unused]] int x_units = MOE_X_UNITS, x_slots = MOE_X_SLOTS;
     if (LIST && x_unit > 0) {
         while (x_units > 1 && p.x_bytes / (x_unit * x_units) < 3) x_units--;
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
 #pragma unroll 1
         while (done < units) {                                              // column blocks of the CTA
             const int kg = in_item % p.KG, count = p.KG - kg < units - done ? p.KG - kg : units - done;
-            if constexpr (LIST) pitch = (uint32_t)__shfl_sync(0xFFFFFFFFu, item_of(item).z, 0);
+            if constexpr (LIST) pitch = __reduce_max_sync(0xFFFFFFFFu, (unsigned)item_of(item).z);
             const uint32_t cols = (pitch + 15u) & ~15u;
             idesc = (1u << 4) | ((cols >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> fp32, M = 128, N = cols
             sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
