@@ -62,6 +62,10 @@ int exl3_device_sm_count(int device);
  * the stored bits.  Replaces repack_trellis / unpack_trellis (cuda/csrc/exl3_marlin.cu:344-408). */
 size_t exl3_packed_bytes(int k, int n, int K);
 exl3_status exl3_repack(const uint16_t *trellis, int k, int n, int K, uint32_t *packed, void *stream);
+/* A fused group in one launch: up to 8 matrices of one k and K side by side along n, and their sign and scale vectors copied to suh_cat
+ * [matrices, k] and svh_cat [sum(ns)]. */
+exl3_status exl3_repack_group(const uint16_t *const *trellis, const uint16_t *const *suh, const uint16_t *const *svh, const int *ns,
+                              int matrices, int k, int K, uint32_t *packed, uint16_t *suh_cat, uint16_t *svh_cat, void *stream);
 exl3_status exl3_unpack(const uint32_t *packed, int k, int n, int K, uint16_t *trellis, void *stream);
 
 /* ---- decode to dense ------------------------------------------------------------------------------------

@@ -1,0 +1,71 @@
+"""Edges of two launches that take several things at once: a fused group repacked together with its sign and scale vectors, and routed
+experts in items of up to 128 rows (an expert with one row, exactly a full item, one row more, several items; more slots than the
+alignment keeps in registers), the latter against the same layer in blocks of eight rows."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from trellis_serve_b200.kernels import linear as lin
+from trellis_serve_b200.kernels import moe
+from trellis_serve_b200.runtime.layerset import random_signs
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _trellis(k, n, K, gen, offset=0):
+    flat = torch.randint(-32768, 32767, (k // 16 * (n // 16) * 16 * K + offset,), dtype=torch.int16, device=DEV, generator=gen)
+    return flat[offset:].view(k // 16, n // 16, 16 * K)
+
+
+@pytest.mark.parametrize("ns", [[128], [256, 128], [128, 384, 128, 128, 256, 128, 128, 128]])
+@pytest.mark.parametrize("K,offset,strided", [(2, 0, False), (3, 2, False), (8, 0, True), (5, 6, True)])
+def test_group_repack_equals_its_matrices(ns, K, offset, strided):
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(K)
+    k = 384
+    trellis = [_trellis(k, n, K, gen, offset) for n in ns]
+
+    def vector(n):
+        v = torch.randn((2 * n if strided else n + 1,), device=DEV, generator=gen).half()
+        return v[::2] if strided else v[1:]
+
+    suh, svh = [vector(k) for _ in ns], [vector(n) for n in ns]
+    packed, suh_cat, svh_cat, ends = lin.prepare(trellis, suh, svh)
+    assert torch.equal(packed, torch.cat([lin.prepare_matrix(t) for t in trellis]))
+    assert torch.equal(suh_cat, torch.stack(suh)) and torch.equal(svh_cat, torch.cat(svh))
+    assert ends == [sum(ns[:i + 1]) for i in range(len(ns) - 1)]
+
+
+@pytest.mark.parametrize("rows,top_k,K,cb", [([1, 128, 129, 0], 1, 3, 0), ([700, 8, 9, 137], 1, 2, 2), ([256, 300, 255, 257], 2, 8, 1),
+                                             ([6000, 5, 11000, 900], 1, 4, 0)])
+def test_long_items_agree_with_blocks_of_eight(monkeypatch, rows, top_k, K, cb):
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(sum(rows))
+    hidden, inter, E = 384, 128, len(rows)
+
+    def proj(k, n):
+        return ([_trellis(k, n, K, gen) for _ in range(E)], [random_signs(k, gen, DEV).view(-1) for _ in range(E)],
+                [(random_signs(n, gen, DEV).view(-1) / 16).half() for _ in range(E)])
+
+    pack = moe.prepare_mixed(proj(hidden, inter), proj(hidden, inter), proj(inter, hidden), cb)
+    first = torch.cat([torch.full((r,), e, dtype=torch.int32) for e, r in enumerate(rows)]).to(DEV)
+    first = first[torch.randperm(first.numel(), device=DEV, generator=gen)]
+    ids = torch.stack([(first + j) % E for j in range(top_k)], 1).contiguous()
+    x = torch.randn((ids.shape[0], hidden), device=DEV, generator=gen).bfloat16()
+    w = torch.rand(ids.shape, device=DEV, generator=gen)
+    out = []
+    for rows_per_expert in (0, 1 << 20):
+        monkeypatch.setattr(moe, "TC_ROWS_PER_EXPERT", rows_per_expert)
+        ws = torch.zeros(moe.layer_workspace_bytes([E], hidden, inter, cb, ids.shape[0], top_k), dtype=torch.uint8, device=DEV)
+        y = torch.empty_like(x)
+        moe.run_layer(x, w, ids, pack, y, ws)
+        again = torch.empty_like(x)
+        moe.run_layer(x, w, ids, pack, again, ws)
+        torch.cuda.synchronize()
+        assert rows_per_expert or torch.equal(y, again)      # in whatever order the alignment put the rows
+        out.append(y.float())
+    scale = out[1].pow(2).mean().sqrt()
+    assert float((out[0] - out[1]).norm() / out[1].norm()) <= 6e-3
+    assert float((out[0] - out[1]).abs().max() / scale) <= 8e-2

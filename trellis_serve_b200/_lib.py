@@ -29,6 +29,7 @@ SIGNATURES = {
     "exl3_init_device": (_i, [_i]),
     "exl3_device_sm_count": (_i, [_i]),
     "exl3_packed_bytes": (_sz, [_i, _i, _i]),
+    "exl3_repack_group": (_i, [_vp, _vp, _vp, _ip, _i, _i, _i, _vp, _vp, _vp, _vp]),
     "exl3_repack": (_i, [_vp, _i, _i, _i, _vp, _vp]),
     "exl3_unpack": (_i, [_vp, _i, _i, _i, _vp, _vp]),
     "exl3_reconstruct": (_i, [_vp, _i, _i, _i, _i, _vp, _vp]),

@@ -121,7 +121,36 @@ exl3_status exl3_repack(const uint16_t* trellis, int k, int n, int K, uint32_t* 
     if (int rc = check_matrix(k, n, K, 0)) return rc;
     if ((long long)k * n == 0) return EXL3_OK;
     if (!aligned(trellis, 4) || !aligned(packed, 16)) return EXL3_ERR_BAD_POINTER;
-    return launch_repack(trellis, k, n, K, packed, (cudaStream_t)stream);
+    RepackGroup g;
+    memset(&g, 0, sizeof(g));
+    g.trellis[0] = trellis;
+    g.nb_end[0] = n / 128;
+    g.matrices = 1;
+    g.KG = k / 128;
+    return launch_repack(g, K, packed, (cudaStream_t)stream);
+}
+
+exl3_status exl3_repack_group(const uint16_t* const* trellis, const uint16_t* const* suh, const uint16_t* const* svh, const int* ns, int matrices, int k,
+                              int K, uint32_t* packed, uint16_t* suh_cat, uint16_t* svh_cat, void* stream)
+{
+    if (matrices < 1 || matrices > REPACK_MATRICES) return EXL3_ERR_BAD_SHAPE;
+    if (!trellis || !suh || !svh || !ns || !aligned(packed, 16) || !aligned(suh_cat, 2) || !aligned(svh_cat, 2)) return EXL3_ERR_BAD_POINTER;
+    RepackGroup g;
+    memset(&g, 0, sizeof(g));
+    int nb = 0;
+    for (int i = 0; i < matrices; i++) {
+        if (int rc = check_matrix(k, ns[i], K, 0)) return rc;
+        if (ns[i] > 0 && (!aligned(trellis[i], 4) || !aligned(suh[i], 2) || !aligned(svh[i], 2))) return EXL3_ERR_BAD_POINTER;
+        g.trellis[i] = trellis[i];
+        g.suh[i] = suh[i];
+        g.svh[i] = svh[i];
+        g.nb_end[i] = nb += ns[i] / 128;
+    }
+    g.suh_cat = suh_cat;
+    g.svh_cat = svh_cat;
+    g.matrices = matrices;
+    g.KG = k / 128;
+    return launch_repack(g, K, packed, (cudaStream_t)stream);
 }
 
 exl3_status exl3_unpack(const uint32_t* packed, int k, int n, int K, uint16_t* trellis, void* stream)
@@ -819,7 +848,6 @@ exl3_status exl3_moe_gemm(const uint32_t* xf, const uint32_t* packed, int K, int
     l.expert_stride = (long long)k * n_total * K / 32;
     l.xf = reinterpret_cast<const unsigned char*>(xf);
     l.xf_shard_stride = (long long)exl3_moe_fragment_bytes(cap, k, 1, codebook);
-    l.slab_rows = MOE_BLOCK_ROWS;
     l.svh = reinterpret_cast<const __half*>(svh);
     l.out = reinterpret_cast<__half*>(out);
     l.sorted_ids = sorted_ids;

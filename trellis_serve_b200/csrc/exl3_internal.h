@@ -23,7 +23,16 @@ struct DeviceInfo {
 const DeviceInfo* current_device_info();
 
 // exl3_kernels.cu
-int launch_repack(const uint16_t* trellis, int k, int n, int K, uint32_t* packed, cudaStream_t st);
+constexpr int REPACK_MATRICES = 8, REPACK_COPY = 2048;        // matrices of a group; vector elements per copying CTA
+struct RepackGroup {
+    const uint16_t* trellis[REPACK_MATRICES];
+    const uint16_t* suh[REPACK_MATRICES];      // [k] each -> suh_cat [matrices][k]; null suh_cat: no vectors
+    const uint16_t* svh[REPACK_MATRICES];
+    uint16_t *suh_cat, *svh_cat;
+    int nb_end[REPACK_MATRICES];               // column blocks up to and including each matrix
+    int matrices, KG;
+};
+int launch_repack(const RepackGroup& g, int K, uint32_t* packed, cudaStream_t st);
 int launch_unpack(const uint32_t* packed, int k, int n, int K, uint16_t* trellis, cudaStream_t st);
 int launch_reconstruct_stored(const uint16_t* trellis, int kt, int nt, int K, int cb, __half* w, cudaStream_t st);
 int launch_reconstruct_packed(const uint32_t* packed, int k, int n, int K, int cb, __half* w, cudaStream_t st);
@@ -114,7 +123,7 @@ inline int rotated_layout(int gemv_mode) { return gemv_mode == GEMV_SPLIT ? 1 : 
 struct MoeGemmLaunch;
 int moe_init_device();
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* counters, cudaStream_t st);
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st);
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
                       const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st);
 int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids, const int* expert_ids,

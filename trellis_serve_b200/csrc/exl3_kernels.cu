@@ -17,12 +17,35 @@ namespace exl3 {
 // 16-byte loads, a lane cuts its K bytes out of each tile with funnel shifts of whole stream words and joins four of them into
 // its K resident words, stored as full 128-byte lines.  Bound by DRAM: one matrix of the 27B shape's gate|up (K = 3, 33 MB
 // in, 33 MB out) takes 15.7 us = 4.3 TB/s; one thread per output word that fetched its 32 bits one by one took 420 us.
+// A whole group is one launch: the CTAs behind the units copy the matrices' sign and scale vectors side by side.
 template <int K>
-__global__ void __launch_bounds__(256) repack_kernel(const uint16_t* __restrict__ trellis, uint32_t* __restrict__ packed, int KG, int NB, int vec)
+__global__ void __launch_bounds__(256) repack_kernel(const __grid_constant__ RepackGroup g, uint32_t* __restrict__ packed)
 {
     constexpr int TILE_WORDS = 8 * K, ROW_WORDS = 8 * TILE_WORDS;            // words of a tile, of a row of eight tiles
     __shared__ __align__(16) uint32_t sm[8 * ROW_WORDS];
-    const int kg = blockIdx.x % KG, nb = blockIdx.x / KG;
+    const int KG = g.KG, units = KG * g.nb_end[g.matrices - 1];
+    if ((int)blockIdx.x >= units) {
+        const long long first = (long long)((int)blockIdx.x - units) * REPACK_COPY;
+        for (int i = threadIdx.x; i < REPACK_COPY; i += 256) {
+            const long long at = first + i, suh_all = (long long)g.matrices * KG * 128;
+            if (at < suh_all) {
+                const int s = (int)(at / (KG * 128));
+                g.suh_cat[at] = g.suh[s][at - (long long)s * KG * 128];
+            } else if (at - suh_all < 128ll * g.nb_end[g.matrices - 1]) {
+                const long long c = at - suh_all;
+                int s = 0;
+                while (c >= 128ll * g.nb_end[s]) s++;
+                g.svh_cat[c] = g.svh[s][c - (s > 0 ? 128ll * g.nb_end[s - 1] : 0)];
+            }
+        }
+        return;
+    }
+    const int kg = blockIdx.x % KG, all_nb = blockIdx.x / KG;
+    int m = 0;
+    while (all_nb >= g.nb_end[m]) m++;
+    const int nb0 = m > 0 ? g.nb_end[m - 1] : 0, NB = g.nb_end[m] - nb0, nb = all_nb - nb0;
+    const uint16_t* trellis = g.trellis[m];
+    const bool vec = reinterpret_cast<uintptr_t>(trellis) % 16 == 0;
     // row tile r of the unit: ROW_WORDS consecutive words; 16 K chunks of 16 bytes each
     const uint4* src = reinterpret_cast<const uint4*>(trellis) + ((long long)kg * 8 * NB + nb) * (ROW_WORDS / 4);
     if (vec) {
@@ -37,7 +60,7 @@ __global__ void __launch_bounds__(256) repack_kernel(const uint16_t* __restrict_
     __syncthreads();
     const int nt = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int word = (K * lane) >> 2, sh = ((K * lane) & 3) * 8;              // where the lane's bytes start in a tile's stream
-    uint32_t* dst = packed + ((((long long)nb * KG + kg) * 8 + nt) * 2) * K * 32 + lane;
+    uint32_t* dst = packed + ((((long long)all_nb * KG + kg) * 8 + nt) * 2) * K * 32 + lane;
 #pragma unroll
     for (int kq = 0; kq < 2; kq++) {
         uint32_t out[K];
@@ -364,14 +387,14 @@ __global__ void had_out_sum_kernel(const float* __restrict__ part, int parts, lo
 
 static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
-int launch_repack(const uint16_t* trellis, int k, int n, int K, uint32_t* packed, cudaStream_t st)
+int launch_repack(const RepackGroup& g, int K, uint32_t* packed, cudaStream_t st)
 {
-    const long long units = (long long)(k / 128) * (n / 128);
+    const long long NB = g.nb_end[g.matrices - 1], units = g.KG * NB, copies = g.suh_cat ? 128ll * g.KG * g.matrices + 128 * NB : 0;
     if (units == 0) return EXL3_OK;
-    if (units >= (1ll << 31)) return EXL3_ERR_BAD_SHAPE;
+    if (units + copies >= (1ll << 31)) return EXL3_ERR_BAD_SHAPE;
     auto kernel = K == 2 ? repack_kernel<2> : K == 3 ? repack_kernel<3> : K == 4 ? repack_kernel<4> : K == 5 ? repack_kernel<5>
                 : K == 6 ? repack_kernel<6> : K == 7 ? repack_kernel<7> : repack_kernel<8>;
-    kernel<<<(unsigned)units, 256, 0, st>>>(trellis, packed, k / 128, n / 128, reinterpret_cast<uintptr_t>(trellis) % 16 == 0);
+    kernel<<<(unsigned)units + blocks_for(copies, REPACK_COPY), 256, 0, st>>>(g, packed);
     return cuda_status(cudaGetLastError());
 }
 

@@ -16,13 +16,13 @@ namespace exl3 {
 // mixed-bitrate expert set gets the blocks of its own slots only, with local expert ids.
 // With `items`: every expert's rows are also cut into items of up to item_blocks blocks of eight rows; items[i] = (expert, first block,
 // blocks, 0), blk[b] = (first block of the item of block b, its blocks), num_post[1] = items, num_post[2] = rows of the largest one; and
-// the counters of the grouped GEMM, and its error word ahead of them, are cleared.  One CTA: bound by latency, so the ids are requested
+// the workspace's header (error word) is cleared.  One CTA: bound by latency, so the ids are requested
 // KEEP at a time per thread.  If they fit into one such pass they stay in registers, each with its rank among its expert's slots from
 // the counting pass (16384 slots 24 us with a second pass of loads and atomics, 20 without).
 template <int KEEP>
 __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
                                  int* __restrict__ expert_ids, int* __restrict__ num_post, const int* __restrict__ expert_map,
-                                 int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ counters)
+                                 int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ header)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
         fill[e] = 0;
     }
     if (items)
-        for (int i = threadIdx.x; i < MOE_MAX_GRID + MOE_ERR_WORDS; i += blockDim.x) counters[i - MOE_ERR_WORDS] = 0;      // and the error word ahead of them
+        for (int i = threadIdx.x; i < MOE_ERR_WORDS; i += blockDim.x) header[i] = 0;
     __syncthreads();
     for (int i0 = 0; i0 < numel; i0 += KEEP * blockDim.x) {
         if (i0 > 0) load_ids(i0);
@@ -487,10 +487,10 @@ int moe_init_device()
 static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* counters, cudaStream_t st)
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st)
 {
     return launch_chained(numel <= 2048 ? moe_align_kernel<2> : moe_align_kernel<16>, dim3(1), dim3(1024), (3 * E + 1) * sizeof(int), st, topk_ids, numel, E, block, cap, sorted_ids, expert_ids,
-                          num_post, expert_map, E_global, item_blocks, items, blk, counters);
+                          num_post, expert_map, E_global, item_blocks, items, blk, header);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -571,7 +571,7 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     l.stages = (int)stages;
     l.x_off = MOE_BAR_BYTES + stages * ups * unit;
     l.p_off = l.x_off + l.x_bytes;
-    if (l.p_off + tail > all || l.x_bytes < (uint32_t)l.slab_rows * row) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (l.p_off + tail > all || l.x_bytes < (uint32_t)(l.items ? moe_item_rows(mode) : MOE_BLOCK_ROWS) * row) return EXL3_ERR_UNSUPPORTED_ROWS;
     const CodebookConst c = codebook_const(codebook);
     l.mul = c.mul;
     l.add = c.add;

@@ -27,7 +27,7 @@ namespace exl3 {
 
 constexpr int MOE_BLOCK_ROWS = 8;
 constexpr int MOE_MAX_GRID = 192;                                // CTAs of a launch (one per SM)
-constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word, then the counters
+constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word
 constexpr int MOE_X_SLOTS = 4, MOE_X_UNITS = 4;                  // most slots of the activation ring, and units of a slot
 constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, then the constants of the decode loop
 // Largest expert count of one routing alignment: its single CTA keeps three counters per expert in the default 48 KB of
@@ -47,11 +47,11 @@ struct MoeGemmLaunch {
     const int* expert_ids;           // expert of each block of eight rows
     const int4* items;               // (expert, first block, blocks, 0), or null: every block of eight rows is an item
     const int* counts;               // device: [0] rows; with items: [1] items, [2] rows of the largest item
-    float* partials;                 // [2 * grid][slab_rows][128]
-    int* counters;                   // [grid]
+    float* partials;                 // without items: [2 * grid][8][128]
+    int* counters;                   // without items: [grid]
     int* err;
     int KG, NB, n_total, numel, shard_end_block;   // shard_end_block: first column block of shard 1 (NB if one shard)
-    int stages, units_per_stage, slab_rows;
+    int stages, units_per_stage;
     uint32_t x_off, x_bytes, p_off;
     uint32_t mul, add;
     int rotated;                     // 1: no output Hadamard / svh (identity read-out)
@@ -172,7 +172,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     const int UB = p.NB * p.KG;                                             // units per item
     // Values read from memory go through a reduction where MMA operands depend on them: its result is a uniform register.
     const int n_items = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)(LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS));
-    const long long total = (long long)n_items * UB;
+    // What is split over the CTAs: units, or (LIST) whole column blocks -- a row's sums are then the same whatever item the alignment,
+    // whose order inside an expert is not fixed, put it into.
+    const int grain = LIST ? p.KG : 1;
+    const long long total = (long long)n_items * (UB / grain);
     int units_q, units_r;
     if (total < (1ll << 31)) {                                              // the 64-bit division is a few hundred clocks of everyone's start
         units_q = (int)((unsigned)total / gridDim.x);
@@ -181,8 +184,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         units_q = (int)(total / gridDim.x);
         units_r = (int)(total % gridDim.x);
     }
-    const long long u0 = gemv_first_unit(cta, units_q, units_r);
-    const int units = units_q + (cta < units_r ? 1 : 0), fills = (units + ups - 1) / ups;
+    const long long u0 = gemv_first_unit(cta, units_q, units_r) * grain;
+    const int units = (units_q + (cta < units_r ? 1 : 0)) * grain, fills = (units + ups - 1) / ups;
     // LIST, activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory
     // (a bulk copy costs a few hundred nanoseconds whatever its size).
     const uint32_t x_unit = LIST ? __reduce_max_sync(0xFFFFFFFFu, (unsigned)p.counts[2]) * F_ROW : 0u;
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
     }
     [[maybe_unused]] const uint32_t slot_bytes = x_unit * x_units;
-    int item = units <= 0 ? 0 : total < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
+    int item = units <= 0 ? 0 : (long long)n_items * UB < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
     int in_item = units > 0 ? (int)(u0 - (long long)item * UB) : 0;
     auto item_of = [&](int i) {                                             // expert, first row, rows
         if constexpr (LIST) {
@@ -529,7 +532,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             if (fresh) it = item_of(item);
             const bool shared = count < p.KG;                               // the column block is cut between CTAs
             int c_first = cta, c_last = cta;
-            if (shared) {
+            if (!LIST && shared) {
                 const long long first = u0 + done - kg;                     // its first unit
                 c_first = gemv_cta_of_unit(first, units_q, units_r);
                 c_last = gemv_cta_of_unit(first + p.KG - 1, units_q, units_r);
@@ -584,8 +587,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             };
             ptx::named_bar_sync(SK_BAR_ACC + d, (ACCS + 4) * 32);
             sk_fence_after();
-            if (shared) {
-                const size_t slab = (size_t)p.slab_rows * 128;
+            if (!LIST && shared) {
+                constexpr size_t slab = MOE_BLOCK_ROWS * 128;
                 read_rows(it.z, p.partials + (size_t)(2 * cta + (cta == c_first)) * slab + ew * 32 + lane);
                 release();
                 ptx::named_bar_sync(SK_BAR_EPI, 128);
@@ -596,23 +599,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                     *flag = last;
                 }
                 ptx::named_bar_sync(SK_BAR_EPI, 128);
-                if (!LIST && *flag) {
-                    moe_finish_eight(p, p.partials, c_first, c_last, sv, slots, nb, ew, lane);
-                } else if (*flag) {
-#pragma unroll 1
-                    for (int r0 = 0; r0 < it.z; r0 += 8) {
-                        float v[8];
-#pragma unroll
-                        for (int e = 0; e < 8; e++) v[e] = 0.f;
-#pragma unroll 1
-                        for (int c = c_first; c <= c_last; c++) {
-                            const float* src = p.partials + (size_t)(2 * c + (c == c_first)) * slab + r0 * 128 + ew * 32 + lane;
-#pragma unroll
-                            for (int e = 0; e < 8; e++) v[e] += __ldcg(src + e * 128);
-                        }
-                        store8(r0, v);
-                    }
-                }
+                if (*flag) moe_finish_eight(p, p.partials, c_first, c_last, sv, slots, nb, ew, lane);
                 ptx::named_bar_sync(SK_BAR_EPI, 128);                       // the flag may be overwritten
             } else if (!LIST) {
                 read_rows(MOE_BLOCK_ROWS, P + ew * 32 + lane);

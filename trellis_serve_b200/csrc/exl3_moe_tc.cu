@@ -23,7 +23,7 @@ namespace exl3 {
 static inline size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct MoeTcLayout {
-    size_t sorted, experts, counts, counters, items, blk, xf13, gu, xf2, yd_rot, partials, total;
+    size_t sorted, experts, counts, items, blk, xf13, gu, xf2, yd_rot, total;
     int cap;
 };
 
@@ -38,7 +38,6 @@ static MoeTcLayout moe_tc_layout(int slots, int num_local, int hidden, int inter
         off += up256(bytes);
         return at;
     };
-    l.counters = take(MOE_MAX_GRID * 4);
     const size_t blocks = (size_t)l.cap / MOE_BLOCK_ROWS + 1;
     l.sorted = take((size_t)l.cap * 4);
     l.experts = take(blocks * 4);
@@ -49,7 +48,6 @@ static MoeTcLayout moe_tc_layout(int slots, int num_local, int hidden, int inter
     l.gu = take((size_t)l.cap * 2 * inter * 2);
     l.xf2 = take((size_t)l.cap * inter * 2);
     l.yd_rot = take((size_t)l.cap * hidden * 2);
-    l.partials = take((size_t)2 * MOE_MAX_GRID * moe_item_rows(GEMV_PAIRED) * 128 * 4);
     l.total = off;
     return l;
 }
@@ -80,15 +78,12 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
     l.expert_ids = expert_ids;
     l.items = items;
     l.counts = counts;
-    l.partials = reinterpret_cast<float*>(ws + w.partials);
-    l.counters = reinterpret_cast<int*>(ws + w.counters);
     l.err = reinterpret_cast<int*>(ws);
     l.numel = slots;
-    l.slab_rows = ROWS;
     l.rotated = 1;
 
     if (int rc = launch_moe_align(topk_ids, slots, num_local, MOE_BLOCK_ROWS, w.cap, sorted_ids, expert_ids, counts, expert_map,
-                                  expert_map ? num_experts : 0, ROWS / MOE_BLOCK_ROWS, items, blk, l.counters, st))
+                                  expert_map ? num_experts : 0, ROWS / MOE_BLOCK_ROWS, items, blk, l.err, st))
         return rc;
     const long long stride = (long long)w.cap * hidden * 2;
     if (int rc = launch_moe_had_in_items(x, x_bf16, suh13, hidden, top_k, slots, w.cap, sorted_ids, expert_ids, counts, blk, ws + w.xf13, stride, st))

@@ -200,12 +200,41 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> prepare_group(at::TensorList trel
     at::Tensor packed = at::empty({nt / 8, kt / 8, 8, 2, words / 16, 32}, trellis[0].options().dtype(at::kInt));
     const auto stream = c10::cuda::getCurrentCUDAStream(device.index());
     uint32_t* dst = static_cast<uint32_t*>(packed.mutable_data_ptr());
-    for (const at::Tensor& t : trellis) {
-        const at::Tensor c = t.contiguous();
-        check(exl3_repack(u16(c), (int)kt * 16, (int)c.size(1) * 16, (int)(words / 16), dst, stream.stream()), "exl3_repack");
-        dst += c.numel() / 2;
+    // Vectors as the kernel can copy them: 16-bit, contiguous, one per matrix; anything else goes through torch.
+    const int64_t count = (int64_t)trellis.size();
+    bool plain = count <= 8 && (int64_t)suh.size() == count && (int64_t)svh.size() == count;
+    for (int64_t i = 0; plain && i < count; i++) {
+        const auto fits = [&](const at::Tensor& v, int64_t n) {
+            return v.device() == device && v.dim() == 1 && v.size(0) == n && v.is_contiguous() && v.element_size() == 2 && v.scalar_type() == suh[0].scalar_type();
+        };
+        plain = fits(suh[i], kt * 16) && fits(svh[i], trellis[i].size(1) * 16);
     }
-    at::Tensor suh_cat = at::stack(suh), svh_cat = at::cat(svh);
+    at::Tensor suh_cat, svh_cat;
+    if (plain) {
+        const uint16_t *t[8], *u[8], *v[8];
+        int ns[8];
+        std::vector<at::Tensor> keep;
+        suh_cat = at::empty({count, kt * 16}, suh[0].options());
+        svh_cat = at::empty({nt * 16}, svh[0].options());
+        for (int64_t i = 0; i < count; i++) {
+            keep.push_back(trellis[i].contiguous());
+            t[i] = u16(keep.back());
+            u[i] = u16(suh[i]);
+            v[i] = u16(svh[i]);
+            ns[i] = (int)trellis[i].size(1) * 16;
+        }
+        check(exl3_repack_group(t, u, v, ns, (int)count, (int)kt * 16, (int)(words / 16), dst, static_cast<uint16_t*>(suh_cat.mutable_data_ptr()),
+                                static_cast<uint16_t*>(svh_cat.mutable_data_ptr()), stream.stream()),
+              "exl3_repack_group");
+    } else {
+        for (const at::Tensor& t : trellis) {
+            const at::Tensor c = t.contiguous();
+            check(exl3_repack(u16(c), (int)kt * 16, (int)c.size(1) * 16, (int)(words / 16), dst, stream.stream()), "exl3_repack");
+            dst += c.numel() / 2;
+        }
+        suh_cat = at::stack(suh);
+        svh_cat = at::cat(svh);
+    }
     scratch(0, device.index(), (int64_t)exl3_linear_workspace_bytes((int)max_rows, (int)kt * 16, (int)nt * 16, (int)trellis.size()));
     stream.synchronize();
     return {packed, suh_cat, svh_cat};

@@ -346,7 +346,8 @@ def _up256(n: int) -> int:
 
 
 @functools.lru_cache(maxsize=256)
-def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: int, codebook: int, tokens: int, top_k: int):
+def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: int, codebook: int, tokens: int, top_k: int,
+                   blocks: tuple[int, ...]):
     """{name: (offset, nbytes)} of one layer's temporaries and their total; per class: routing triple and activation buffers."""
     lib = _lib.load()
     slots = tokens * top_k
@@ -358,7 +359,7 @@ def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: i
                     (f"xf13_{c}", int(lib.exl3_moe_fragment_bytes(cap, hidden, 2, codebook))),
                     (f"xf2_{c}", int(lib.exl3_moe_fragment_bytes(cap, inter, 1, codebook)))]
         gemv = max(gemv, int(lib.exl3_moe_workspace_bytes(cap, 2 * inter)), int(lib.exl3_moe_workspace_bytes(cap, hidden)))
-        if moe_block_size(tokens, top_k, e) == BLOCK_SIZES[1]:
+        if blocks[c] == BLOCK_SIZES[1]:
             regions.append((f"tc{c}", int(lib.exl3_moe_tc_workspace_bytes(slots, e, hidden, inter))))
     plan, off = {}, 0
     for name, n in [("gemv", gemv)] + regions:       # the GEMV workspace first: its header and counters must stay zero
@@ -367,9 +368,14 @@ def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: i
     return plan, off
 
 
+def _plan(num_experts_per_class: list[int], hidden: int, inter: int, codebook: int, tokens: int, top_k: int):
+    return _layer_regions(tuple(num_experts_per_class), hidden, inter, codebook, tokens, top_k,
+                          tuple(moe_block_size(tokens, top_k, e) for e in num_experts_per_class))
+
+
 def layer_workspace_bytes(num_experts_per_class: list[int], hidden: int, inter: int, codebook: int, tokens: int, top_k: int) -> int:
     """Bytes `run_layer` needs for up to `tokens` tokens (zero-filled once by the caller)."""
-    return _layer_regions(tuple(num_experts_per_class), hidden, inter, codebook, tokens, top_k)[1]
+    return _plan(num_experts_per_class, hidden, inter, codebook, tokens, top_k)[1]
 
 
 def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, workspace: torch.Tensor,
@@ -387,7 +393,7 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
         return out
     dev, st = x.device, _stream(x.device)
     maps = expert_maps if expert_maps is not None else pack.expert_maps
-    plan, need = _layer_regions(tuple(p.num_experts for p in pack.packs), hidden, inter, pack.codebook, tokens, top_k)
+    plan, need = _plan([p.num_experts for p in pack.packs], hidden, inter, pack.codebook, tokens, top_k)
     if need > workspace.numel():
         raise RuntimeError(f"MoE workspace holds {workspace.numel()} bytes, this call needs {need}")
     base = workspace.data_ptr()
@@ -415,7 +421,7 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
             xf13, xf2 = at(f"xf13_{c}"), at(f"xf2_{c}")
             cap = plan[f"sorted{c}"][1] // 4
             K = pk.bits
-            if moe_block_size(tokens, top_k, pk.num_experts) == BLOCK_SIZES[1]:
+            if f"tc{c}" in plan:
                 _lib.check(lib.exl3_moe_tc_experts(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
                                                    pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
                                                    _ptr(pk.svh2), K, pk.codebook, yd, at(f"tc{c}"), plan[f"tc{c}"][1], st), "exl3_moe_tc_experts")
