@@ -9,18 +9,19 @@ namespace exl3 {
 
 // ------------------------------------------------------------------------------------------------ align
 
-// One CTA.  Slots (token, k) are grouped by expert into blocks of `block` rows: sorted_ids holds the slot of every
+// One cluster of CL CTAs.  Slots (token, k) are grouped by expert into blocks of `block` rows: sorted_ids holds the slot of every
 // row (numel = padding), expert_ids the expert of every block, num_post the padded row count.  Ids outside
 // [0, E) are dropped.  The order of slots inside an expert is not specified (rows are independent).
 // With expert_map (int [E_global]: global id -> id in [0, E), or -1) the ids are translated first, so one class of a
 // mixed-bitrate expert set gets the blocks of its own slots only, with local expert ids.
 // With `items`: every expert's rows are also cut into items of up to item_blocks blocks of eight rows; items[i] = (expert, first block,
 // blocks, 0), blk[b] = (first block of the item of block b, its blocks), num_post[1] = items, num_post[2] = rows of the largest one; and
-// the workspace's header (error word) is cleared.  One CTA: bound by latency, so the ids are requested
-// KEEP at a time per thread.  If they fit into one such pass they stay in registers, each with its rank among its expert's slots from
-// the counting pass (16384 slots 24 us with a second pass of loads and atomics, 20 without).
-template <int KEEP>
-__global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
+// the workspace's header (error word) is cleared.  Bound by latency and by shared-memory
+// atomics: a CTA counts its share of the slots, reads the other CTAs' counts through distributed shared memory and lays out the experts
+// itself; KEEP slots per thread are requested together and, if that takes them all, stay in registers with their rank from the
+// counting (16384 slots, 256 experts: 24 us in one CTA with two passes of loads and atomics, 20 with one).
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
                                  int* __restrict__ expert_ids, int* __restrict__ num_post, const int* __restrict__ expert_map,
                                  int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ header)
 {
@@ -30,12 +31,14 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
     int* count = sh;              // [E]
     int* offset = sh + E;         // [E + 1]
     int* fill = sh + 2 * E + 1;   // [E]
-    const bool one = numel <= KEEP * (int)blockDim.x;
+    constexpr int KEEP = 2;
+    const int rank_cta = blockIdx.x, threads = CL * blockDim.x, thread = rank_cta * blockDim.x + threadIdx.x;      // of the cluster
+    const bool one = numel <= KEEP * threads;
     int e_of[KEEP], rank[KEEP];
     auto load_ids = [&](int i0) {                       // experts of slots i0 + thread + j * threads, -1 outside [0, E)
 #pragma unroll
         for (int j = 0; j < KEEP; j++) {
-            const int i = i0 + threadIdx.x + j * blockDim.x;
+            const int i = i0 + thread + j * threads;
             e_of[j] = i < numel ? topk_ids[i] : -1;
         }
         if (expert_map) {
@@ -51,13 +54,45 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
         count[e] = 0;
         fill[e] = 0;
     }
-    if (items)
+    if (items && rank_cta == 0)
         for (int i = threadIdx.x; i < MOE_ERR_WORDS; i += blockDim.x) header[i] = 0;
     __syncthreads();
-    for (int i0 = 0; i0 < numel; i0 += KEEP * blockDim.x) {
+    for (int i0 = 0; i0 < numel; i0 += KEEP * threads) {
         if (i0 > 0) load_ids(i0);
 #pragma unroll
         for (int j = 0; j < KEEP; j++) rank[j] = e_of[j] >= 0 ? atomicAdd(&count[e_of[j]], 1) : 0;
+    }
+    int* before = fill + E;       // CL > 1: [E], slots of the CTAs ahead; count becomes the total
+    if constexpr (CL > 1) {
+        ptx::cluster_sync_all();
+        int sums[2] = {0, 0};
+        auto gather = [&](int e) {
+            sums[0] = sums[1] = 0;
+            int c[CL];
+#pragma unroll
+            for (int r = 0; r < CL; r++) c[r] = ptx::ld_shared_cluster_s32(&count[e], r);
+#pragma unroll
+            for (int r = 0; r < CL; r++) {
+                if (r < rank_cta) sums[0] += c[r];
+                sums[1] += c[r];
+            }
+        };
+        int total[(MOE_MAX_EXPERTS + 1023) / 1024];
+#pragma unroll
+        for (int i = 0; i < (MOE_MAX_EXPERTS + 1023) / 1024; i++) {
+            const int e = threadIdx.x + i * 1024;
+            if (e < E) {
+                gather(e);
+                before[e] = sums[0];
+                total[i] = sums[1];
+            }
+        }
+        ptx::cluster_sync_all();                       // every CTA has read the counts: they may change, and CTAs may leave
+#pragma unroll
+        for (int i = 0; i < (MOE_MAX_EXPERTS + 1023) / 1024; i++) {
+            const int e = threadIdx.x + i * 1024;
+            if (e < E) count[e] = total[i];
+        }
     }
     // Exclusive prefix sums of the padded counts and (high word) of the items: warp scans by shuffle, warp totals through shared
     // memory; experts are taken in chunks of blockDim.x with a running carry.
@@ -98,39 +133,43 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
         if (e < E) {
             const int b0 = (int)(excl & 0xFFFFFFFFu) / block;
             offset[e] = b0 * block;
-            for (int r = 0; r < blocks; r++) expert_ids[b0 + r] = e;
-            for (int r = count[e]; r < blocks * block; r++) sorted_ids[b0 * block + r] = numel;
-            if (items) {
-                // the expert's blocks in nearly even items
-                int at = (int)(excl >> 32), first = 0;
-                for (int i = 0; i < n_items; i++) {
-                    const int len = (blocks - first + n_items - i - 1) / (n_items - i);
-                    items[at + i] = make_int4(e, b0 + first, len, 0);
-                    for (int r = 0; r < len; r++) blk[b0 + first + r] = make_int2(b0 + first, len);
-                    if (i == 0) atomicMax(&largest, len * block);      // the first is the largest
-                    first += len;
+            if (CL == 1 || e % CL == rank_cta) {       // the CTAs share the writing
+                for (int r = 0; r < blocks; r++) expert_ids[b0 + r] = e;
+                for (int r = count[e]; r < blocks * block; r++) sorted_ids[b0 * block + r] = numel;
+                if (items) {
+                    // the expert's blocks in nearly even items
+                    int at = (int)(excl >> 32), first = 0;
+                    for (int i = 0; i < n_items; i++) {
+                        const int len = (blocks - first + n_items - i - 1) / (n_items - i);
+                        items[at + i] = make_int4(e, b0 + first, len, 0);
+                        for (int r = 0; r < len; r++) blk[b0 + first + r] = make_int2(b0 + first, len);
+                        first += len;
+                    }
                 }
             }
+            if (n_items > 0) atomicMax(&largest, (blocks + n_items - 1) / n_items * block);
         }
         __syncthreads();
         if (threadIdx.x == blockDim.x - 1) carry_sh = base + incl;
         __syncthreads();
     }
     const int total = (int)(carry_sh & 0xFFFFFFFFu);
-    if (threadIdx.x == 0) {
+    if (thread == 0) {
         num_post[0] = total;
         if (items) {
             num_post[1] = (int)(carry_sh >> 32);
             num_post[2] = largest;
         }
     }
-    for (int i = total / block + threadIdx.x; i < cap / block; i += blockDim.x) expert_ids[i] = -1;
-    for (int i = total + threadIdx.x; i < cap; i += blockDim.x) sorted_ids[i] = numel;
-    for (int i0 = 0; i0 < numel; i0 += KEEP * blockDim.x) {
+    for (int i = total / block + thread; i < cap / block; i += threads) expert_ids[i] = -1;
+    for (int i = total + thread; i < cap; i += threads) sorted_ids[i] = numel;
+    for (int i0 = 0; i0 < numel; i0 += KEEP * threads) {
         if (!one) load_ids(i0);
 #pragma unroll
-        for (int j = 0; j < KEEP; j++)
-            if (e_of[j] >= 0) sorted_ids[offset[e_of[j]] + (one ? rank[j] : atomicAdd(&fill[e_of[j]], 1))] = i0 + threadIdx.x + j * blockDim.x;
+        for (int j = 0; j < KEEP; j++) {
+            const int e = e_of[j];
+            if (e >= 0) sorted_ids[offset[e] + (CL > 1 ? before[e] : 0) + (one ? rank[j] : atomicAdd(&fill[e], 1))] = i0 + thread + j * threads;
+        }
     }
 }
 
@@ -474,7 +513,8 @@ int moe_init_device()
 {
     const DeviceInfo* d = current_device_info();
     if (!d) return EXL3_ERR_NOT_INITIALISED;
-    int rc = moe_set_attributes_for_k<2>(d->max_smem_optin);
+    int rc = cuda_status(cudaFuncSetAttribute(moe_align_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (4 * MOE_MAX_EXPERTS + 1) * (int)sizeof(int)));
+    if (rc == EXL3_OK) rc = moe_set_attributes_for_k<2>(d->max_smem_optin);
     if (rc == EXL3_OK) rc = moe_set_attributes_for_k<3>(d->max_smem_optin);
     if (rc == EXL3_OK) rc = moe_set_attributes_for_k<4>(d->max_smem_optin);
     if (rc == EXL3_OK) rc = moe_set_attributes_for_k<5>(d->max_smem_optin);
@@ -489,8 +529,10 @@ static inline unsigned blocks_for(long long items, int per_block) { return (unsi
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
                      const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st)
 {
-    return launch_chained(numel <= 2048 ? moe_align_kernel<2> : moe_align_kernel<16>, dim3(1), dim3(1024), (3 * E + 1) * sizeof(int), st, topk_ids, numel, E, block, cap, sorted_ids, expert_ids,
-                          num_post, expert_map, E_global, item_blocks, items, blk, header);
+    // Up to two slots per thread of one CTA; more are shared by a cluster (the largest portable one).
+    const bool many = numel > 2048;
+    return launch_chained(many ? moe_align_kernel<8> : moe_align_kernel<1>, dim3(many ? 8 : 1), dim3(1024), (size_t)((many ? 4 : 3) * E + 1) * sizeof(int), st,
+                          topk_ids, numel, E, block, cap, sorted_ids, expert_ids, num_post, expert_map, E_global, item_blocks, items, blk, header);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -30,8 +30,8 @@ constexpr int MOE_MAX_GRID = 192;                                // CTAs of a la
 constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word
 constexpr int MOE_X_SLOTS = 4, MOE_X_UNITS = 4;                  // most slots of the activation ring, and units of a slot
 constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, then the constants of the decode loop
-// Largest expert count of one routing alignment: its single CTA keeps three counters per expert in the default 48 KB of
-// shared memory ((3 * E + 1) * 4 bytes + 280 static).
+// Largest expert count of one routing alignment: one CTA keeps three counters per expert in the default 48 KB of shared memory
+// ((3 * E + 1) * 4 bytes + 280 static).
 constexpr int MOE_MAX_EXPERTS = 4064;
 
 __host__ __device__ constexpr int moe_item_rows(int mode) { return mode == GEMV_SPLIT ? 32 : 128; }

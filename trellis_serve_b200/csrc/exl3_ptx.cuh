@@ -100,6 +100,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta)
                  : "memory");
 }
 
+// The word at the same shared-memory offset in CTA `cta` of the cluster.
+__device__ __forceinline__ int ld_shared_cluster_s32(const int* p, uint32_t cta)
+{
+    int v;
+    asm volatile("{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %1, %2;\n ld.shared::cluster.s32 %0, [ra];\n}" : "=r"(v) : "r"(smem_addr(p)), "r"(cta) : "memory");
+    return v;
+}
+
 // Bounded wait on a barrier of this CTA that threads of the other CTA arrive on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity)
 {
