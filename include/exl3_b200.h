@@ -112,10 +112,10 @@ exl3_status exl3_linear(const void *x, int x_dtype, const uint32_t *packed, int 
  * In a decode step every EXL3 linear is preceded by an element-wise kernel (residual add + RMSNorm ahead of q|k|v and
  * gate|up, SiLU(gate) * up ahead of down, nothing but the rotation ahead of o).  These entry points fuse the linear's input
  * rotation into that kernel: it writes Had128(fp16(activation) * suh[s]) for every matrix s of the following fused group as
- * tensor-core fragments into `workspace`, once, and exl3_linear_prerotated runs the group from there (up to two rows its
- * CTAs copy the fragments of their units into shared memory with bulk copies; 3..16 rows read them tile by tile).  The
- * fragments, and so the results, are bit-identical to exl3_linear on the same activation.  rows <= 16; the workspace is the
- * one exl3_linear_workspace_bytes(rows, k, n_total, n_shards) sizes, shared by the whole chain in stream order.
+ * the B operand of the decode kernel into `workspace`, once, and exl3_linear_prerotated runs the group from there (its CTAs
+ * copy the rotated rows of their units into shared memory with bulk copies).  The rotated rows, and so the results, are
+ * bit-identical to exl3_linear on the same activation.  rows <= 16; the workspace is the one
+ * exl3_linear_workspace_bytes(rows, k, n_total, n_shards) sizes, shared by the whole chain in stream order.
  * The reference runs these steps as separate kernels ahead of had_in_group_marlin (cuda/csrc/exl3_marlin.cu:283-290,
  * group launch :507-527); the fusion has no counterpart there.
  *   exl3_rotate_fragments   activation x [rows, k] as it is.
@@ -303,7 +303,7 @@ exl3_status exl3_allreduce(void *data, int dtype, size_t n, void *const *peer_re
  *                      experts per alignment (EXL3_ERR_BAD_SHAPE beyond).  The later steps index the expert tensors
  *                      with these lists unchecked: pass only lists written by exl3_moe_align / exl3_moe_align_mapped.
  * exl3_moe_had_in      replaces moe_had_in (exl3_marlin_moe.cu:210-225): per position Had128(fp16(x[token]) * suh[e, s])
- *                      for `shards` input rotations (gate and up), written as MMA fragments.  suh is [E, shards, hidden].
+ *                      for `shards` input rotations (gate and up), written as MMA operands.  suh is [E, shards, hidden].
  * exl3_moe_gemm        replaces moe_gemm (exl3_marlin_moe.cu:376-408): per moe block, rows @ W[e] -> Had128 * svh[e] ->
  *                      out[slot, :] fp16.  packed = [E] resident matrices; svh [E, n_total] (NULL: rotated basis, no
  *                      output transform); shard_end: first column fed by input rotation 1 (0 = single rotation).
@@ -339,14 +339,13 @@ exl3_status exl3_moe_combine(const uint16_t *yd, const float *topk_weights, cons
 /* Routed experts with many rows per expert (prefill-sized batches) on the tensor cores.  The reference serves such batches
  * with the same grouped kernel and larger moe blocks (moe_block_size picks 8..64 rows from T * top_k / E,
  * cuda/src/sglang_exl3/kernels/marlin_moe.py:52-57; launch at cuda/csrc/exl3_marlin_moe.cu:376-408); here the routing is
- * aligned to blocks of exl3_moe_tc_block_rows() = 128 rows and up to two blocks of one expert (four when hidden or inter is
- * not a multiple of 256) share every decoded weight block in a grouped tcgen05 GEMM.  x, yd and the sign vectors must be
- * 16-byte aligned.  One call runs one bitrate class from the routing to the per-slot outputs:
+ * aligned to blocks of eight rows and up to exl3_moe_tc_block_rows() = 128 rows of one expert share every decoded weight in
+ * a grouped tcgen05 GEMM.  x, yd and the sign vectors must be 16-byte aligned.  One call runs one bitrate class from the routing to the per-slot outputs:
  *   align (expert_map as in exl3_moe_align_mapped, or NULL with num_local == num_experts) -> gate|up -> SiLU(gate) * up
  *   -> down -> yd[slot, :] (fp16 [tokens * top_k, hidden]; slots of experts outside the class are not written).
  * exl3_moe_combine then closes the layer.  w13 / suh13 / svh13 / w2 / suh2 / svh2 are the resident expert stacks of
  * exl3_moe_gemm ([E][2I/128][H/128]..., [E][2][H], [E][2I], [E][H/128][I/128]..., [E][I], [E][H]).  The workspace holds
- * exl3_moe_tc_workspace_bytes(tokens * top_k, num_local, hidden, inter) bytes, 256-byte aligned, first 256 bytes zero. */
+ * exl3_moe_tc_workspace_bytes(tokens * top_k, num_local, hidden, inter) bytes, 256-byte aligned. */
 int exl3_moe_tc_block_rows(void);
 size_t exl3_moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter);
 exl3_status exl3_moe_tc_experts(const void *x, int x_dtype, int tokens, int top_k, int hidden, int inter, const int32_t *topk_ids,

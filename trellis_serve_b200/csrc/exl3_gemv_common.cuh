@@ -7,7 +7,7 @@
 
 namespace exl3 {
 
-enum { GEMV_ERR_FULL_WAIT = 1, GEMV_ERR_EMPTY_WAIT = 2, GEMV_ERR_PEER_WAIT = 3 };    // 2: the grouped MoE kernel's copy warp
+enum { GEMV_ERR_FULL_WAIT = 1, GEMV_ERR_PEER_WAIT = 3 };
 constexpr uint32_t GEMV_PEER_MAX_POLLS = 1u << 20;       // bounded wait for a peer's words: about a second
 
 #ifdef EXL3_TIMELINE

@@ -165,15 +165,8 @@ __host__ __device__ inline long long tc_a_offset(int row, int col, int KB)
     return ((((((long long)ms * KB + kb) * 4 + mt) * 8 + c) * 16 + j) * 8 + rr) * 8 + e0;
 }
 
-// The grouped instances: the wide tiling where column blocks pair up inside every shard -- 16 decode warps on a 64 x 256 weight
-// block per step (routed experts have few rows each, so the decode bounds the kernel and needs the warps), items of up to
-// TC_GROUPED_MT blocks of 128 rows of one expert -- else 128-column tiles with 8 decode warps and items of up to 4 blocks.
-constexpr int TC_GROUPED_MT = 2;
-int launch_gemm_tc_grouped(const uint32_t* packed, long long expert_stride, int K, int codebook, const int* shard_end_blocks, int n_shards,
-                           int k, int n_total, const __half* xa, int cap512, __half* out, const int4* items, const int* n_items, bool wide,
-                           int* err, cudaStream_t st);
-// exl3_moe_tc.cu: routed experts through the grouped tensor-core GEMM (many rows per expert)
-constexpr int MOE_TC_BLOCK_ROWS = 128;
+// exl3_moe_tc.cu: routed experts with many rows per expert
+constexpr int MOE_TC_BLOCK_ROWS = 128;             // largest item: rows of one expert that share a decoded weight
 
 size_t moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter);
 int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int inter, const int* topk_ids, int slots, int num_experts,
