@@ -80,7 +80,7 @@ def workspace_bytes(rows: int, k: int, n_total: int, shards: int) -> int:
 
 
 def reserve_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Zero-filled, reused per-device scratch (activation fragments, split-k partial sums, counters).  Sized at load
+    """Zero-filled, reused per-device scratch (rotated activations, split-k partial sums, counters).  Sized at load
     time so the run path never allocates and CUDA graphs see a fixed address."""
     return _workspace.reserve(device.index if device.index is not None else torch.cuda.current_device(), nbytes)
 
@@ -241,10 +241,10 @@ def run_tc(x: torch.Tensor, b: torch.Tensor, suh_cat: torch.Tensor, svh_cat: tor
 
 # ---------------------------------------------------------------------------------------------------------------
 # Decode step: the kernel ahead of a linear writes the linear's rotated input (residual / normalisation / activation fused
-# with the input rotation), the linear runs from those fragments.  All four share one workspace in stream order.
+# with the input rotation), the linear runs from those rotated rows.  All four share one workspace in stream order.
 
 def _step_workspace(device: torch.device, rows: int, k: int, shards: int, workspace: torch.Tensor) -> torch.Tensor:
-    """The chain's workspace is the caller's (zero-filled once, `workspace_bytes` of the largest group): the fragments one
+    """The chain's workspace is the caller's (zero-filled once, `workspace_bytes` of the largest group): the rotated rows one
     call leaves there are what the next call reads, so no call may swap the buffer for a larger one on its own."""
     if workspace is None:
         raise RuntimeError("the decode-step calls share one caller-owned workspace: pass it to every call of the chain")
@@ -265,7 +265,7 @@ def rotate_fragments(x: torch.Tensor, suh_cat: torch.Tensor, codebook: int, work
 
 def rmsnorm_rotate(x: torch.Tensor, residual: torch.Tensor | None, weight: torch.Tensor, eps: float, suh_cat: torch.Tensor,
                    codebook: int, workspace: torch.Tensor, normed: torch.Tensor | None = None) -> None:
-    """residual += x (in place, when given); a = rmsnorm(residual or x) * weight; fragments of a for the following group;
+    """residual += x (in place, when given); a = rmsnorm(residual or x) * weight; rotated rows of a for the following group;
     `normed` receives a when given.  All tensors share x's dtype (fp16 / bf16)."""
     _require_cuda(x, "x")
     rows, k = x.shape
@@ -279,7 +279,7 @@ def rmsnorm_rotate(x: torch.Tensor, residual: torch.Tensor | None, weight: torch
 
 def silu_mul_rotate(gate_up: torch.Tensor, suh: torch.Tensor, codebook: int, workspace: torch.Tensor,
                     act: torch.Tensor | None = None) -> None:
-    """a = silu(gate) * up of gate_up [rows, 2 * inter]; fragments of a for the following (down) matrix."""
+    """a = silu(gate) * up of gate_up [rows, 2 * inter]; rotated rows of a for the following (down) matrix."""
     _require_cuda(gate_up, "gate_up")
     rows, two = gate_up.shape
     inter = two // 2
@@ -299,7 +299,7 @@ def _residual_ptrs(residual):
 
 def run_prerotated(rows: int, b: torch.Tensor, svh_cat: torch.Tensor, shard_ends: list[int], codebook: int, out: torch.Tensor | None,
                    workspace: torch.Tensor, exchange=None, residual=None, out_dtype: torch.dtype | None = None) -> torch.Tensor | None:
-    """The fused group on the fragments the kernel ahead left in the workspace; `out` [rows, n_total] fp16 / bf16 (fp32:
+    """The fused group on the rotated rows the kernel ahead left in the workspace; `out` [rows, n_total] fp16 / bf16 (fp32:
     unrounded accumulators).  `exchange`: row-parallel shard, summed over the ranks inside the kernel.  `residual` =
     (stream in, stream out, sums of squares out float32 [rows, n_total / 128]): the epilogue carries the residual stream;
     `out` may then be None (give `out_dtype`)."""
@@ -308,7 +308,7 @@ def run_prerotated(rows: int, b: torch.Tensor, svh_cat: torch.Tensor, shard_ends
     k, n_total, K = _geometry(b)
     shards = len(shard_ends) + 1
     if workspace is None:
-        raise RuntimeError("run_prerotated reads the fragments from the workspace the producing call wrote: pass that workspace")
+        raise RuntimeError("run_prerotated reads the rotated rows from the workspace the producing call wrote: pass that workspace")
     ws = _own_or_given(workspace, b.device, workspace_bytes(rows, k, n_total, shards), _workspace)
     ex = exchange if exchange is not None and exchange.world > 1 else None
     with torch.cuda.device(b.device):

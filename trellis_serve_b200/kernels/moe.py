@@ -25,8 +25,9 @@ from .base import BackendStatus
 from .linear import _dtype_code, _ptr, _require_cuda, _stream, supports_matrix
 
 BLOCK_SIZES = (8, 128)
-# Average routed rows per expert from which a class goes through the grouped tensor-core GEMM (128-row blocks, every
-# expert decoded once per up to 512 rows) instead of the grouped GEMV (8-row blocks, decoded once per block).
+# Average routed rows per expert from which a class goes through the grouped tensor-core GEMM (items of up to 128 rows of an
+# expert, decoded once each) instead of blocks of eight rows (decoded once per block).  Measured crossover: 8 rows for 256 experts of
+# 2048 x 512, 11 for 64 of 2048 x 768, more for layers so small that the two further launches show.
 TC_ROWS_PER_EXPERT = 10
 _workspace: dict[int, torch.Tensor] = {}
 
@@ -41,8 +42,8 @@ def probe() -> BackendStatus:
 
 def moe_block_size(tokens: int, top_k: int, num_experts: int) -> int:
     """Rows per moe block.  The reference picks from a ladder 8..64 by T * top_k / E (marlin_moe.py:52-57); here decode-sized
-    batches use the grouped GEMV on 8-row blocks and batches with many rows per expert the grouped tensor-core GEMM on
-    128-row blocks (`run_layer` switches by this value)."""
+    batches use the grouped GEMV on 8-row blocks and batches with many rows per expert the grouped GEMM on
+    longer items (`run_layer` switches by this value)."""
     return BLOCK_SIZES[1] if tokens * top_k >= TC_ROWS_PER_EXPERT * num_experts else BLOCK_SIZES[0]
 
 
@@ -237,7 +238,7 @@ def align(topk_ids: torch.Tensor, num_experts: int, block: int = 8):
 
 def gemm_rotated(xf, stack, out, sorted_ids, expert_ids, num_post_padded, slots: int, shard_end: int, codebook: int,
                  svh=None) -> torch.Tensor:
-    """Grouped product (svh=None: rotated basis, no output transform).  xf = activation fragments of the blocks."""
+    """Grouped product (svh=None: rotated basis, no output transform).  xf = rotated rows of the blocks."""
     lib = _lib.load()
     e, nb, kg, _, _, K, _ = stack.shape
     k, n_total, cap = kg * 128, nb * 128, sorted_ids.numel()
