@@ -69,3 +69,24 @@ def test_long_items_agree_with_blocks_of_eight(monkeypatch, rows, top_k, K, cb):
     scale = out[1].pow(2).mean().sqrt()
     assert float((out[0] - out[1]).norm() / out[1].norm()) <= 6e-3
     assert float((out[0] - out[1]).abs().max() / scale) <= 8e-2
+
+
+@pytest.mark.parametrize("rows", [65, 128, 129, 255, 257, 384, 513, 700, 1025])
+@pytest.mark.parametrize("k,n,K,cb", [(384, 384, 4, 1), (1024, 1024, 2, 2)])
+def test_row_tiles_that_hold_no_rows_are_left_out(rows, k, n, K, cb):
+    """Many-row kernels with stale data behind the last row: the same bits as when the activation buffer was zeroed."""
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(rows + k)
+    packed, suh_cat, svh_cat, ends = lin.prepare([_trellis(k, n, K, gen)], [random_signs(k, gen, DEV).view(-1)],
+                                                 [(random_signs(n, gen, DEV).view(-1) / 16).half()])
+    x = torch.randn((rows, k), device=DEV, generator=gen).half()
+    need = lin.tc_workspace_bytes(rows, k, n, 1)
+    out = []
+    for fill in (0, 0x7F):                                   # 0x7F7F is a NaN in fp16
+        ws = torch.full((need,), fill, dtype=torch.uint8, device=DEV)
+        ws[:256] = 0
+        y = torch.empty((rows, n), dtype=torch.float16, device=DEV)
+        lin.run_tc(x, packed, suh_cat, svh_cat, ends, cb, out=y, workspace=ws)
+        torch.cuda.synchronize()
+        out.append(y)
+    assert torch.equal(out[0], out[1]) and bool(torch.isfinite(out[0]).all())

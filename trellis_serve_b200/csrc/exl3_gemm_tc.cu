@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    ptx::grid_launch_dependents();
 
     const int KB = p.KG * 2;                           // reduction blocks of 64
     const int MT = (p.rows + TT::ROWS - 1) / TT::ROWS;   // row tiles
@@ -197,6 +198,11 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
     const long long n_tiles = (long long)MT * NT * KS;
     auto kb_begin = [&](long long t) { return (int)((long long)KB * (t % KS) / KS); };
     auto kb_end = [&](long long t) { return (int)((long long)KB * (t % KS + 1) / KS); };
+    // 128-row tiles of row tile ms that hold rows: the others are neither fetched nor multiplied nor read out.
+    auto tiles_present = [&](int ms) {
+        const int left = (p.rows - ms * TT::ROWS + 127) / 128;
+        return left < TT::M_TILES ? left : TT::M_TILES;
+    };
     bool failed = false;
     auto fail = [&]() {
         if (!failed) {
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
             for (int i = 0; i < K; i++) Lnext[i] = __ldg(src + i * 32);
         }
         for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            const int ct = (int)((t / KS) / MT), row0 = (int)((t / KS) % MT) * TT::ROWS, present = TT::M_TILES;
+            const int ct = (int)((t / KS) / MT), ms = (int)((t / KS) % MT), row0 = ms * TT::ROWS, present = tiles_present(ms);
             const int sp = (int)(t % KS);
             const int kb0 = kb_begin(t), kb1 = kb_end(t);
             const long long t_next = t + gridDim.x;
@@ -296,12 +302,14 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
                 if (lane == 0) ptx::mbar_arrive(&b_full[s]);
             }
             // The decode warps read out the tile themselves (each the 32 tensor-memory lanes of its quarter and 64 of the
-            // tile's columns).
+            // tile's columns).  Decoding needs weights alone; what is written below may still be read by kernels ahead.
+            ptx::grid_dependency_wait();
             epilogue(warp, DW, row0, ct, sp, present, acc_round);
             acc_round++;
         }
     } else if (warp == DW) {
         // ------------------------------------------------------------------ A producer
+        ptx::grid_dependency_wait();
         if (lane == 0) {
             uint32_t it = 0;
             for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x) {
@@ -310,11 +318,8 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
                 int shard = 0;
                 while (shard < p.n_shards - 1 && nb >= p.shard_end_block[shard]) shard++;
                 // The A layout in global memory is in super tiles of 512 rows = four 128-row tiles of 16 KB per reduction
-                // block; the tile's 128-row tiles are fetched one by one (a 384-row tile may straddle two super tiles, and
-                // its last 128-row tiles may lie beyond the padded rows: those are not fetched, their products are never stored).
-                int t128 = ms * TT::M_TILES;
-                int present = p.MS * 4 - t128;
-                if (present > TT::M_TILES) present = TT::M_TILES;
+                // block; the tile's 128-row tiles are fetched one by one (a 384-row tile may straddle two super tiles).
+                const int t128 = ms * TT::M_TILES, present = tiles_present(ms);
                 for (int kb = kb0; kb < kb1; kb++, it++) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
@@ -330,12 +335,13 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
         }
     } else if (warp == DW + 1) {
         // ------------------------------------------------------------------ MMA issue
+        ptx::grid_dependency_wait();
         if (lane == 0) {
             uint32_t it = 0, acc_round = 0;
             for (long long t = blockIdx.x; t < n_tiles; t += gridDim.x) {
                 if (acc_round > 0 && !failed && !ptx::mbar_wait(acc_empty, (acc_round - 1) & 1)) fail();
                 tc_fence_after();
-                const int kb0 = kb_begin(t), kb1 = kb_end(t);
+                const int kb0 = kb_begin(t), kb1 = kb_end(t), present = tiles_present((int)((t / KS) % MT));
                 for (int kb = kb0; kb < kb1; kb++, it++) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
@@ -348,8 +354,9 @@ __global__ void __launch_bounds__(TcTile<MT_, WIDE>::THREADS, 1) gemm_tc_kernel(
                     for (int mt = 0; mt < TT::M_TILES; mt++)
 #pragma unroll
                         for (int ks = 0; ks < TC_KB / 16; ks++)
-                            tc_mma(tmem_base + (uint32_t)(mt * TT::NCOLS), tc_smem_desc(a_addr + mt * TC_A_TILE_BYTES + ks * 4096, 2048),
-                                   tc_smem_desc(b_addr + ks * 2 * TT::B_LBO, TT::B_LBO), TT::IDESC, (kb > kb0 || ks > 0) ? 1u : 0u);
+                            if (mt < present)
+                                tc_mma(tmem_base + (uint32_t)(mt * TT::NCOLS), tc_smem_desc(a_addr + mt * TC_A_TILE_BYTES + ks * 4096, 2048),
+                                       tc_smem_desc(b_addr + ks * 2 * TT::B_LBO, TT::B_LBO), TT::IDESC, (kb > kb0 || ks > 0) ? 1u : 0u);
                     tc_commit(&empty[s]);               // stage reusable once these MMAs have read it
                 }
                 tc_commit(acc_full);                    // accumulators complete
@@ -466,6 +473,8 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
     auto part_of = [&](long long t) { return t < n_whole ? 0 : (int)((t - n_whole) % KS); };
     auto kb_begin = [&](long long t) { return t < n_whole ? 0 : (int)((long long)KB * part_of(t) / KS); };
     auto kb_end = [&](long long t) { return t < n_whole ? KB : (int)((long long)KB * (part_of(t) + 1) / KS); };
+    // Row halves of 256 of a tile that hold rows (the same for both CTAs): the other is neither fetched nor multiplied nor read out.
+    auto halves_present = [&](long long t) { return p.rows - (int)(tile_of(t) % MT) * TT::ROWS > 256 ? TT::M_TILES : 1; };
     bool failed = false;
     auto fail = [&]() {
         if (!failed) {
@@ -515,21 +524,24 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
                 if (lane == 0) ptx::mbar_arrive(&b_full[s]);
             }
         }
+        ptx::grid_launch_dependents();                  // the rotation of cut tiles may take its place: not before, it shares the SM
+        ptx::grid_dependency_wait();
     } else if (warp == DW) {
         // ------------------------------------------------------------------ activation producer: rows 128 rank .. + 127 of each MMA
+        ptx::grid_dependency_wait();
         if (lane == 0) {
             uint32_t it = 0;
             for (long long t = first; t < n_tiles; t += step) {
                 const int ms = (int)(tile_of(t) % MT), nb = (int)(tile_of(t) / MT) * 2;
-                const int kb0 = kb_begin(t), kb1 = kb_end(t);
+                const int kb0 = kb_begin(t), kb1 = kb_end(t), present = halves_present(t);
                 int shard = 0;
                 while (shard < p.n_shards - 1 && nb >= p.shard_end_block[shard]) shard++;
                 for (int kb = kb0; kb < kb1; kb++, it++) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
                     if (round > 0 && !failed && !ptx::mbar_wait_relaxed(&empty[s], (round - 1) & 1)) fail();
-                    ptx::mbar_arrive_expect_tx(&a_full[s], TT::A_STAGE_BYTES);
-                    for (int mt = 0; mt < TT::M_TILES; mt++) {
+                    ptx::mbar_arrive_expect_tx(&a_full[s], (uint32_t)present * TC_A_TILE_BYTES);
+                    for (int mt = 0; mt < present; mt++) {
                         // 128-row tile 2 mt + rank of the 512-row super tile ms
                         const __half* src = p.xa + shard * p.xa_shard_stride + (((long long)ms * KB + kb) * 4 + 2 * mt + (int)rank) * (TC_A_TILE_BYTES / 2);
                         ptx::bulk_g2s(stage0 + (size_t)s * TT::STAGE_BYTES + (size_t)mt * TC_A_TILE_BYTES, src, TC_A_TILE_BYTES, &a_full[s]);
@@ -542,6 +554,7 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
         }
     } else if (warp >= DW + 2) {
         // ------------------------------------------------------------------ epilogue
+        ptx::grid_dependency_wait();
         const int quarter = warp & 3, cgroup = (warp - (DW + 2)) >> 2;
         unsigned char* slice = out_stage + (size_t)(warp - (DW + 2)) * TT::OUT_WARP_BYTES;
         unsigned char* my_row = slice + (size_t)lane * TT::OUT_PITCH;
@@ -555,8 +568,9 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
             // handed back as soon as it has been read.  Parts of a cut tile store their fp32 accumulators directly.
             if (!failed && !ptx::mbar_wait(acc_full, acc_round & 1)) fail();
             tc_fence_after();
+            const int present = halves_present(t);
 #pragma unroll 1
-            for (int mt = 0; mt < TT::M_TILES; mt++) {
+            for (int mt = 0; mt < present; mt++) {
                 const int row_in = mt * 256 + (int)rank * 128 + quarter * 32 + lane, row = ms * TT::ROWS + row_in;
                 ptx::bulk_wait_read_all();              // the lane's previous copy has left its staging row ...
                 __syncwarp();                           // ... and so has every other lane's (a row is rotated by four lanes)
@@ -588,7 +602,7 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
                         }
                     }
                 }
-                if (mt == TT::M_TILES - 1) {
+                if (mt == present - 1) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
@@ -620,14 +634,15 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
             acc_round++;
         }
         ptx::bulk_wait_all();                           // the lane's output copies have completed
-    } else if (lane == 0) {
+    } else {
+        ptx::grid_dependency_wait();
         uint32_t it = 0, acc_round = 0;
-        if (rank == 0) {
+        if (lane == 0 && rank == 0) {
             // -------------------------------------------------------------- MMA issue for the pair
             for (long long t = first; t < n_tiles; t += step) {
                 if (acc_round > 0 && !failed && !ptx::mbar_wait_cluster(acc_empty, (acc_round - 1) & 1)) fail();
                 tc_fence_after();
-                const int kb0 = kb_begin(t), kb1 = kb_end(t);
+                const int kb0 = kb_begin(t), kb1 = kb_end(t), present = halves_present(t);
                 for (int kb = kb0; kb < kb1; kb++, it++) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
@@ -641,14 +656,15 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
                     for (int mt = 0; mt < TT::M_TILES; mt++)
 #pragma unroll
                         for (int ks = 0; ks < TC_KB / 16; ks++)
-                            tc_mma_pair(tmem_base + (uint32_t)(mt * 256), tc_smem_desc(a_addr + mt * TC_A_TILE_BYTES + ks * 4096, 2048),
-                                        tc_smem_desc(b_addr + ks * 2 * TT::B_LBO, TT::B_LBO), TT::IDESC, (kb > kb0 || ks > 0) ? 1u : 0u);
+                            if (mt < present)
+                                tc_mma_pair(tmem_base + (uint32_t)(mt * 256), tc_smem_desc(a_addr + mt * TC_A_TILE_BYTES + ks * 4096, 2048),
+                                            tc_smem_desc(b_addr + ks * 2 * TT::B_LBO, TT::B_LBO), TT::IDESC, (kb > kb0 || ks > 0) ? 1u : 0u);
                     tc_commit_pair(&empty[s]);          // the stage is reusable in both CTAs once these MMAs have read it
                 }
                 tc_commit_pair(acc_full);               // accumulators complete in both CTAs
                 acc_round++;
             }
-        } else {
+        } else if (lane == 0) {
             // -------------------------------------------------------------- this CTA's stages reported to rank 0
             for (long long t = first; t < n_tiles; t += step) {
                 const int kb0 = kb_begin(t), kb1 = kb_end(t);
@@ -674,13 +690,15 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
 }
 
 // Rotated activations in the A-operand layout of gemm_tc_kernel.  One warp per (shard, group of 8 rows, 128-block), four lanes
-// per row with 32 columns each (fwht128_quad): a lane's 32 results are four whole 16-byte core-matrix rows, and the eight
-// lanes that share a column range fill a 128-byte core matrix.  Rows beyond `rows` inside the last group are written as
-// zeros; those up to the next multiple of 512 must have been zero-filled by the caller.
+// per row (fwht128_turn): a lane's 32 results are four whole 16-byte core-matrix rows, and the eight lanes that share a
+// column range fill a 128-byte core matrix.  Rows beyond `rows` inside the last group are written as zeros.
 constexpr int HAD_IN_TC_ROWS = 8;
 __global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_cols, const __half* __restrict__ suh, int shards, int rows, int k,
                                  __half* __restrict__ xa, long long shard_stride)
 {
+    // The GEMM behind this one reads weights before its own wait: it may start once everything ahead of this kernel is done.
+    ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int kgs = k >> 7;
     const int groups = (rows + HAD_IN_TC_ROWS - 1) / HAD_IN_TC_ROWS;
@@ -694,10 +712,11 @@ __global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_c
     if (row < rows) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
+            const int c = kg * 128 + 32 * i + 8 * (lane & 3);
             // rows of x are x_cols (a multiple of 8) long, zeros from there to k
-            const uint4 raw = col + 8 * i < x_cols ? reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * x_cols + col)[i]
-                                                   : make_uint4(0u, 0u, 0u, 0u);
-            const uint4 sraw = reinterpret_cast<const uint4*>(suh + (long long)s * k + col)[i];
+            const uint4 raw = c < x_cols ? *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * x_cols + c)
+                                         : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 sraw = *reinterpret_cast<const uint4*>(suh + (long long)s * k + c);
             const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w}, sw[4] = {sraw.x, sraw.y, sraw.z, sraw.w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -720,7 +739,7 @@ __global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_c
 #pragma unroll
         for (int i = 0; i < 32; i++) v[i] = 0.f;
     }
-    fwht128_quad(v, lane);
+    fwht128_turn(v, lane);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         uint32_t o[4];
@@ -739,8 +758,7 @@ static int launch_tc_kernel(const GemmTcLaunch& l, int sm_count, cudaStream_t st
     using TT = TcTile<MT, WIDE>;
     const long long work = (long long)((l.rows + TT::ROWS - 1) / TT::ROWS) * (l.NB / TT::NBLK) * l.ksplit;
     const int grid = work < sm_count ? (int)work : sm_count;
-    gemm_tc_kernel<K, FAM, MT, WIDE, SPLIT><<<grid, TT::THREADS, TT::SMEM_BYTES, st>>>(l);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(gemm_tc_kernel<K, FAM, MT, WIDE, SPLIT>, dim3(grid), dim3(TT::THREADS), TT::SMEM_BYTES, st, l);
 }
 
 template <int K, int FAM, int MT, bool WIDE>
@@ -764,13 +782,15 @@ static int launch_tc_pair(const GemmTcLaunch& l, cudaStream_t st)
     cfg.blockDim = dim3(TcPair::THREADS);
     cfg.dynamicSmemBytes = TcPair::SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cuda_status(cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<K, FAM>, l));
 }
 
@@ -896,12 +916,12 @@ int launch_gemm_tc(const void* x, int x_bf16, int x_cols, const __half* suh_cat,
     l.mul = c.mul;
     l.add = c.add;
     l.pw = make_pow2();
-    // Rows beyond `rows` inside the last 512-row super tile must read as zeros; with whole super tiles there are none.
-    if (rows % TC_ROWS != 0)
-        if (int rc = cuda_status(cudaMemsetAsync(xa, 0, gemm_tc_activation_bytes(rows, k, n_shards), st))) return rc;
+    // Rows beyond `rows` inside the last super tile hold whatever was there: a product row depends on its own row of A only, and
+    // theirs are never stored (zeroing them was a pass over the whole buffer, 4 us at 74 rows of 2 x 7168).
     const long long items = (long long)n_shards * ((rows + HAD_IN_TC_ROWS - 1) / HAD_IN_TC_ROWS) * (k / 128);
-    had_in_tc_kernel<<<(unsigned)((items + 7) / 8), 256, 0, st>>>(x, x_bf16, x_cols, suh_cat, n_shards, rows, k, xa, l.xa_shard_stride);
-    if (int rc = cuda_status(cudaGetLastError())) return rc;
+    if (int rc = launch_chained(had_in_tc_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, st, x, x_bf16, x_cols, suh_cat, n_shards, rows, k, xa,
+                                l.xa_shard_stride))
+        return rc;
     // Wide tiles (256 x 256) need column blocks that pair up inside every shard.  They halve the rows that share a decoded
     // weight block, which makes the decode the limiter at large row counts (measured: 823 against 851 TFLOP/s at 2048
     // rows), but they waste no rows when there are at most 256 (703 against 457 TFLOP/s): chosen only then.  Above that,

@@ -6,6 +6,7 @@
 //   had_in / had_out       128-point rotations with the suh / svh vectors
 //                          (cuda/csrc/exl3_marlin.cu:257-306, cuda/csrc/exl3_had.cuh:20-84)
 #include "exl3_internal.h"
+#include "exl3_ptx.cuh"
 
 namespace exl3 {
 
@@ -185,8 +186,6 @@ __global__ void reconstruct_packed_kernel(const uint32_t* __restrict__ packed, _
 
 // ------------------------------------------------------------------------------------------------ Hadamard
 
-__device__ __forceinline__ void ptx_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void ptx_grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ float load_as_f16_value(const void* p, long long idx, bool bf16)
 {
@@ -221,8 +220,8 @@ template <int MODE>
 __global__ void had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int shards, int rows, int k,
                               void* __restrict__ out, int x_cols)
 {
-    ptx_grid_launch_dependents();              // the GEMV behind this kernel may start streaming weights already
-    ptx_grid_dependency_wait();                // x may be the output of the kernel ahead
+    ptx::grid_launch_dependents();              // the GEMV behind this kernel may start streaming weights already
+    ptx::grid_dependency_wait();                // x may be the output of the kernel ahead
     const int lane = threadIdx.x & 31;
     const int kgs = k >> 7;
     long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -288,6 +287,8 @@ template <bool IN_F32>
 __global__ void had_out_kernel(const void* __restrict__ y, const __half* __restrict__ svh, int rows, int n, void* __restrict__ out,
                                long long out_stride, int out_bf16)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     const int nbs = n >> 7;
     const int groups = (rows + HAD_OUT_ROWS - 1) / HAD_OUT_ROWS;
@@ -324,6 +325,8 @@ __global__ void had_out_kernel(const void* __restrict__ y, const __half* __restr
 __global__ void had_out_tiles_kernel(const float* __restrict__ part, int parts, int tail_first, int row_tiles, int cut_tiles,
                                      const __half* __restrict__ svh, int rows, int n, void* __restrict__ out, int out_bf16)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)cut_tiles * 128) return;
@@ -357,6 +360,8 @@ __global__ void had_out_tiles_kernel(const float* __restrict__ part, int parts, 
 __global__ void had_out_sum_kernel(const float* __restrict__ part, int parts, long long slab, const __half* __restrict__ svh, int rows,
                                    int n, void* __restrict__ out, int out_bf16)
 {
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     const int nbs = n >> 7;
     long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -471,9 +476,8 @@ int launch_had_out(const void* y, int y_f32, const __half* svh, int rows, int n,
 {
     long long items = (long long)((rows + HAD_OUT_ROWS - 1) / HAD_OUT_ROWS) * (n / 128);
     if (items == 0) return EXL3_OK;
-    if (y_f32) had_out_kernel<true><<<blocks_for(items, 8), 256, 0, st>>>(y, svh, rows, n, out, out_stride, out_bf16);
-    else had_out_kernel<false><<<blocks_for(items, 8), 256, 0, st>>>(y, svh, rows, n, out, out_stride, out_bf16);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(y_f32 ? had_out_kernel<true> : had_out_kernel<false>, dim3(blocks_for(items, 8)), dim3(256), 0, st, y, svh, rows, n, out, out_stride,
+                          out_bf16);
 }
 
 int launch_had_out_tiles(const float* part, int parts, int tail_first, int row_tiles, const __half* svh, int rows, int n, void* out,
@@ -481,9 +485,8 @@ int launch_had_out_tiles(const float* part, int parts, int tail_first, int row_t
 {
     const int cut_tiles = row_tiles * (n / 256) - tail_first;
     if (cut_tiles <= 0) return EXL3_OK;
-    had_out_tiles_kernel<<<blocks_for((long long)cut_tiles * 128, 8), 256, 0, st>>>(part, parts, tail_first, row_tiles, cut_tiles, svh, rows, n, out,
-                                                                                  out_bf16);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(had_out_tiles_kernel, dim3(blocks_for((long long)cut_tiles * 128, 8)), dim3(256), 0, st, part, parts, tail_first, row_tiles, cut_tiles,
+                          svh, rows, n, out, out_bf16);
 }
 
 int launch_had_out_sum(const float* part, int parts, long long slab, const __half* svh, int rows, int n, void* out, int out_bf16,
@@ -491,8 +494,7 @@ int launch_had_out_sum(const float* part, int parts, long long slab, const __hal
 {
     long long items = (long long)rows * (n / 128);
     if (items == 0) return EXL3_OK;
-    had_out_sum_kernel<<<blocks_for(items, 8), 256, 0, st>>>(part, parts, slab, svh, rows, n, out, out_bf16);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(had_out_sum_kernel, dim3(blocks_for(items, 8)), dim3(256), 0, st, part, parts, slab, svh, rows, n, out, out_bf16);
 }
 
 }  // namespace exl3
