@@ -149,7 +149,7 @@ def packed_bytes_per_step(layers: int, K: int) -> float:
 def traffic_ratio() -> tuple[float | None, str]:
     """DRAM bytes moved per algorithmic byte of the dominant kernel, from the ncu capture whose figures sit beside its
     summary (read + write of one gate|up launch over its packed-weight bytes)."""
-    path = os.path.join(ROOT, "profiles", "gemv_kernel_27b_k3_batch1.traffic.json")
+    path = os.path.join(ROOT, "profiles", "skinny_kernel_27b_k3_batch1.traffic.json")
     if not os.path.exists(path):
         return None, "no capture recorded"
     with open(path) as f:
@@ -362,7 +362,7 @@ def run_c1(args) -> None:
                       "config": {"workload": "single EXL3 linear 4096x4096, K=4 3INST, batch 1, ring of 64 distinct matrices in one graph",
                                  "l2": "ring of 64 x 8.4 MB = 537 MB, larger than L2"},
                       "roofline": {"bound": "hbm", "achieved": r["gbs"], "peak": peak, "unit": "GB/s", "frac": r["gbs"] / peak,
-                                   "traffic": None, "peak_source": f"of {kind}", "kernel": "gemv_kernel"},
+                                   "traffic": None, "peak_source": f"of {kind}", "kernel": "skinny_kernel"},
                       "gpu_launches": r["ring"], "clocks": clocks.summary()}))
 
 
@@ -694,7 +694,7 @@ def main() -> None:
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                              "traffic": traffic, "traffic_unit": "bytes per launch, from one ncu capture scaled by units",
                              "traffic_source": traffic_source,
-                             "peak_source": f"of {peak_kind}", "kernel": "gemv_kernel",
+                             "peak_source": f"of {peak_kind}", "kernel": "skinny_kernel",
                              "launches_per_step": gemv_launches, "avg_launch_ms_upper_bound": avg_launch_ms},
                 "e2e": {"value": e2e_value, "unit": UNIT, "ms_per_step": ms_e2e / args.steps,
                         "h2d_bytes_per_step": sum(h.numel() * h.element_size() for h in hx),
