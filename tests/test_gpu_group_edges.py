@@ -90,3 +90,27 @@ def test_row_tiles_that_hold_no_rows_are_left_out(rows, k, n, K, cb):
         torch.cuda.synchronize()
         out.append(y)
     assert torch.equal(out[0], out[1]) and bool(torch.isfinite(out[0]).all())
+
+
+def test_plain_calls_equal_the_operator_and_the_rest_goes_through_it():
+    from trellis_serve_b200.runtime import ops
+
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(3)
+    k, n, K = 256, 384, 3
+    weights = lin.prepare([_trellis(k, n, K, gen)], [random_signs(k, gen, DEV).view(-1)], [(random_signs(n, gen, DEV).view(-1) / 16).half()])
+    rest = ([], [], [], [], [], 0, list(weights[:3]), weights[3], [0], [n])
+    op = torch.ops.exl3_b200.linear
+    for x in (torch.randn((3, k), device=DEV, generator=gen).half(), torch.randn((2, 5, k), device=DEV, generator=gen), torch.zeros((0, k), device=DEV).half()):
+        assert torch.equal(ops.linear(x, *rest), op(x, *rest))
+        assert ops._direct(x, *rest) is not None
+    assert ops._direct(x, *rest[:-1], (n,)) is None and ops._direct(x) is None          # a tuple, too few arguments
+    assert torch.equal(ops.linear(x, *rest[:-1], (n,)), op(x, *rest))
+    assert ops._direct(torch.nn.Parameter(x), *rest) is None
+    with pytest.raises(RuntimeError, match="exceeds the stored width"):
+        ops.linear(torch.zeros((1, k + 1), device=DEV), *rest)
+    with torch.inference_mode():
+        assert torch.equal(ops.linear(x, *rest), op(x, *rest))
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        assert ops._direct(x, *rest) is None

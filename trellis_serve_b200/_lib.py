@@ -5,6 +5,7 @@ There is no fallback: if the library is missing or a call fails, an exception sa
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -120,6 +121,15 @@ def native():
         torch.ops.load_library(TORCH_LIB_PATH)
         _native = torch.ops.exl3_b200
     return _native
+
+
+def direct():
+    """Module of plain Python functions over the same library (no dispatcher): `linear`, see runtime/ops.py."""
+    native()
+    spec = importlib.util.spec_from_file_location("exl3_b200_direct", TORCH_LIB_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
 
 
 def check(status: int, where: str) -> None:

@@ -52,14 +52,16 @@ def _sources_mtime() -> float:
 
 def build_torch() -> str:
     """libexl3_b200_torch.so: csrc/exl3_torch.cpp against the installed torch and the C-ABI library beside it."""
+    import sysconfig
+
     import torch
     from torch.utils.cpp_extension import include_paths
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda = os.path.join(os.path.dirname(os.path.dirname(nvcc())), "include")
-    includes = [f"-I{p}" for p in dict.fromkeys([*include_paths(), cuda])]
+    includes = [f"-I{p}" for p in dict.fromkeys([*include_paths(), cuda, sysconfig.get_paths()["include"]])]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *includes,
            os.path.join(HERE, "exl3_torch.cpp"), "-o", TORCH_OUT, f"-L{os.path.dirname(OUT)}", f"-l:{os.path.basename(OUT)}", f"-L{lib}",
-           "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-Wl,-rpath,$ORIGIN"]
+           "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
