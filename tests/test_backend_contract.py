@@ -34,6 +34,31 @@ def test_protocol_and_load_time_refusals():
         assert callable(getattr(be, method))
 
 
+@pytest.mark.parametrize("codebook,halves", [(0, True), (1, True), (2, False)])
+@pytest.mark.parametrize("tokens", [1, 64, 2048])
+def test_routed_expert_plans_follow_the_weight_mode(codebook, halves, tokens):
+    """The rotated rows of an expert's block take 512 bytes per 128 columns when weights enter as two summands, 256 when paired (always
+    with MUL1): a plan made in one mode must not serve the other, whichever came first."""
+    from trellis_serve_b200.kernels import linear as lin
+    from trellis_serve_b200.kernels import moe
+
+    experts, hidden, inter, top_k = 256, 2048, 512, 8
+    cap = moe.sorted_ids_capacity(tokens, top_k, experts)
+    need = {512: None, 256: None}
+    try:
+        for mode, row in ((1, 256), (-1, 512 if halves else 256), (1, 256), (0, 512 if halves else 256)):
+            lin.set_gemv_mode(mode)
+            plan, total = moe._plan([experts], hidden, inter, codebook, tokens, top_k)
+            assert plan["xf13_0"][1] == 2 * cap * (hidden // 128) * row and plan["xf2_0"][1] == cap * (inter // 128) * row
+            spans = sorted(plan.values())
+            assert all(a + n <= b for (a, n), (b, _) in zip(spans, spans[1:])) and spans[-1][0] + spans[-1][1] <= total
+            assert moe.layer_workspace_bytes([experts], hidden, inter, codebook, tokens, top_k) == total
+            assert need[row] in (None, total)
+            need[row] = total
+    finally:
+        lin.set_gemv_mode(-1)
+
+
 @pytest.mark.gpu
 def test_prepare_warm_run_matches_the_oracle():
     K, cb, k, ns, rows = 3, 0, 512, [256, 128], 2

@@ -347,9 +347,11 @@ def _up256(n: int) -> int:
 
 
 @functools.lru_cache(maxsize=256)
-def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: int, codebook: int, tokens: int, top_k: int,
+def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: int, row_bytes: int, tokens: int, top_k: int,
                    blocks: tuple[int, ...]):
-    """{name: (offset, nbytes)} of one layer's temporaries and their total; per class: routing triple and activation buffers."""
+    """{name: (offset, nbytes)} of one layer's temporaries and their total; per class: routing triple and activation buffers.  Kept
+    between calls, so the plan may depend on nothing but the arguments: `row_bytes`, the rotated activations of one row and 128
+    columns, changes with `set_gemv_mode`."""
     lib = _lib.load()
     slots = tokens * top_k
     regions = [("ids32", slots * 4), ("wts", slots * 4), ("gu", slots * 2 * inter * 2), ("yd", slots * hidden * 2)]
@@ -357,8 +359,7 @@ def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: i
     for c, e in enumerate(num_experts_per_class):
         cap = int(lib.exl3_moe_sorted_capacity(slots, e))
         regions += [(f"sorted{c}", cap * 4), (f"experts{c}", max(cap // 8, 1) * 4), (f"post{c}", 4),
-                    (f"xf13_{c}", int(lib.exl3_moe_fragment_bytes(cap, hidden, 2, codebook))),
-                    (f"xf2_{c}", int(lib.exl3_moe_fragment_bytes(cap, inter, 1, codebook)))]
+                    (f"xf13_{c}", 2 * cap * (hidden // 128) * row_bytes), (f"xf2_{c}", cap * (inter // 128) * row_bytes)]
         gemv = max(gemv, int(lib.exl3_moe_workspace_bytes(cap, 2 * inter)), int(lib.exl3_moe_workspace_bytes(cap, hidden)))
         if blocks[c] == BLOCK_SIZES[1]:
             regions.append((f"tc{c}", int(lib.exl3_moe_tc_workspace_bytes(slots, e, hidden, inter))))
@@ -370,7 +371,8 @@ def _layer_regions(num_experts_per_class: tuple[int, ...], hidden: int, inter: i
 
 
 def _plan(num_experts_per_class: list[int], hidden: int, inter: int, codebook: int, tokens: int, top_k: int):
-    return _layer_regions(tuple(num_experts_per_class), hidden, inter, codebook, tokens, top_k,
+    row_bytes = int(_lib.load().exl3_moe_fragment_bytes(1, 128, 1, codebook))
+    return _layer_regions(tuple(num_experts_per_class), hidden, inter, row_bytes, tokens, top_k,
                           tuple(moe_block_size(tokens, top_k, e) for e in num_experts_per_class))
 
 
