@@ -114,3 +114,44 @@ def test_plain_calls_equal_the_operator_and_the_rest_goes_through_it():
     from torch._subclasses.fake_tensor import FakeTensorMode
     with FakeTensorMode(allow_non_fake_inputs=True):
         assert ops._direct(x, *rest) is None
+
+
+def test_plain_calls_are_seen_by_whatever_watches():
+    """Function modes, the profiler, gradients of any operand and tensors that are not what their storage holds: as through the operator."""
+    from torch.overrides import TorchFunctionMode
+    from torch.profiler import ProfilerActivity, profile
+
+    from trellis_serve_b200.runtime import ops
+
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(4)
+    k, n, K = 256, 128, 3
+    packed, suh, svh, ends = lin.prepare([_trellis(k, n, K, gen)], [random_signs(k, gen, DEV).view(-1)], [(random_signs(n, gen, DEV).view(-1) / 16).half()])
+    rest = ([], [], [], [], [], 0, [packed, suh, svh], ends, [0], [n])
+    op = torch.ops.exl3_b200.linear
+    x = torch.randn((3, k), device=DEV, generator=gen).half()
+    want = op(x, *rest)
+
+    class Watch(TorchFunctionMode):
+        def __init__(self):
+            super().__init__()
+            self.seen = []
+
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Watch() as watch:
+        y = ops.linear(x, *rest)
+        assert any("exl3_b200" in name for name in watch.seen) and ops._direct(x, *rest) is None
+    assert torch.equal(y, want)
+    with profile(activities=[ProfilerActivity.CPU]) as prof:
+        y = ops.linear(x, *rest)
+    assert "exl3_b200::linear" in {e.key for e in prof.key_averages()} and torch.equal(y, want)
+    assert ops._direct(x, *rest) is not None                            # nothing watches any more
+    learned = rest[:6] + ([packed, suh.clone().requires_grad_(), svh],) + rest[7:]
+    assert ops._direct(x, *learned) is None
+    with torch.no_grad():
+        assert torch.equal(ops._direct(x, *learned), want)
+    negated = torch._neg_view(x)
+    assert torch.equal(ops.linear(negated, *rest), op(-x, *rest))

@@ -14,7 +14,9 @@
 #include <vector>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/record_function.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -265,7 +267,17 @@ void repack_experts(at::TensorList trellis, at::Tensor& out, int64_t nb0)
 
 // ------------------------------------------------------------------------------------------------ plain eager calls
 
-bool plain_tensor(PyObject* o) { return THPVariable_CheckExact(o) && THPVariable_Unpack(o).is_cuda(); }
+// A dense CUDA tensor that asks nothing of the dispatcher: no subclass, no wrapper or lazy negation (keys beyond the ordinary ones), no
+// gradient wanted.
+bool plain_tensor(PyObject* o)
+{
+    if (!THPVariable_CheckExact(o)) return false;
+    using c10::DispatchKey;
+    static const uint64_t plain =
+        c10::DispatchKeySet({DispatchKey::CUDA, DispatchKey::AutogradCUDA, DispatchKey::ADInplaceOrView, DispatchKey::AutocastCUDA}).raw_repr();
+    const at::Tensor& t = THPVariable_Unpack(o);
+    return t.is_cuda() && (t.key_set().raw_repr() & ~plain) == 0 && !(t.requires_grad() && c10::GradMode::is_enabled());
+}
 
 bool unpack_tensors(PyObject* o, std::vector<at::Tensor>& out)
 {
@@ -294,15 +306,16 @@ bool unpack_ints(PyObject* o, std::vector<int64_t>& out)
     return true;
 }
 
-// The operator for what eager code passes: positional plain CUDA tensors, lists and ints, no gradients, and nothing watching the
-// dispatcher (modes, tracing, functional transforms).  None: not such a call, take the operator.
+// The operator for what eager code passes: positional plain CUDA tensors, lists and ints, no gradients, and nothing that wants to see
+// the call: dispatch modes, tracing and functional transforms (thread-local dispatch keys), modes over torch functions, profiler and
+// other record-function callbacks.  None: not such a call, take the operator.
 PyObject* direct_linear(PyObject*, PyObject* const* args, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
     if (n != 11 || !plain_tensor(args[0]) || !PyLong_CheckExact(args[6])) Py_RETURN_NONE;
     if (!(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty()) Py_RETURN_NONE;
+    if (at::impl::torch_function_mode_enabled() || at::hasCallbacks()) Py_RETURN_NONE;
     const at::Tensor x = THPVariable_Unpack(args[0]);
-    if (c10::GradMode::is_enabled() && x.requires_grad()) Py_RETURN_NONE;
     std::vector<at::Tensor> trellis, suh, svh, dense, sliced, weights;
     std::vector<int64_t> ends, codebooks, widths;
     if (!unpack_tensors(args[1], trellis) || !unpack_tensors(args[2], suh) || !unpack_tensors(args[3], svh) || !unpack_tensors(args[4], dense) ||

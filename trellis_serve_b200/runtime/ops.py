@@ -111,8 +111,8 @@ _direct = _native_lib.direct().linear
 
 
 def linear(*args, **kwargs):
-    """`torch.ops.exl3_b200.linear`.  Plain eager calls (positional CUDA tensors, no gradients, no mode or tracer watching) skip the
-    dispatcher, which is two thirds of the host time of a small call; everything else goes through it."""
+    """`torch.ops.exl3_b200.linear`.  Plain eager calls (positional CUDA tensors, no gradients, no mode, tracer or profiler watching)
+    skip the dispatcher, which is two thirds of the host time of a small call; everything else goes through it."""
     if not kwargs and not torch.compiler.is_compiling():
         y = _direct(*args)
         if y is not None:
