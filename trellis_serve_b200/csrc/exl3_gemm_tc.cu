@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
                 if (lane == 0) ptx::mbar_arrive(&b_full[s]);
             }
         }
-        ptx::grid_launch_dependents();                  // the rotation of cut tiles may take its place: not before, it shares the SM
+        ptx::grid_launch_dependents();                  // a chained kernel behind this one: not before, it shares the SM
         ptx::grid_dependency_wait();
     } else if (warp == DW) {
         // ------------------------------------------------------------------ activation producer: rows 128 rank .. + 127 of each MMA

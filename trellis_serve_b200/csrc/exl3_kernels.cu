@@ -322,11 +322,13 @@ __global__ void had_out_kernel(const void* __restrict__ y, const __half* __restr
 // column tile x row_tiles + row tile; the tiles before `tail_first` leave that kernel finished): the sum of `parts` fp32
 // slabs part[(tile - tail_first) * parts + s][512][256], added in part order and rounded to fp16 once, as the kernel rounds
 // the accumulators of a tile it did not cut.  One warp per (cut tile, 8 rows, 128 columns).
+// Not chained to the GEMM: its 96 to 450 blocks do not fit beside a CTA of that kernel, so those let in early pile up, four to an SM, on
+// the SMs whose pairs are through first, and read all the slabs from there (2048 rows, cut tiles of 12 parts, K = 4: 5120 x 5120 208
+// us against 138, 17408 x 5120 470 against 398).
 __global__ void had_out_tiles_kernel(const float* __restrict__ part, int parts, int tail_first, int row_tiles, int cut_tiles,
                                      const __half* __restrict__ svh, int rows, int n, void* __restrict__ out, int out_bf16)
 {
     ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)cut_tiles * 128) return;
@@ -485,8 +487,9 @@ int launch_had_out_tiles(const float* part, int parts, int tail_first, int row_t
 {
     const int cut_tiles = row_tiles * (n / 256) - tail_first;
     if (cut_tiles <= 0) return EXL3_OK;
-    return launch_chained(had_out_tiles_kernel, dim3(blocks_for((long long)cut_tiles * 128, 8)), dim3(256), 0, st, part, parts, tail_first, row_tiles, cut_tiles,
-                          svh, rows, n, out, out_bf16);
+    had_out_tiles_kernel<<<blocks_for((long long)cut_tiles * 128, 8), 256, 0, st>>>(part, parts, tail_first, row_tiles, cut_tiles, svh, rows, n, out,
+                                                                                  out_bf16);
+    return cuda_status(cudaGetLastError());
 }
 
 int launch_had_out_sum(const float* part, int parts, long long slab, const __half* svh, int rows, int n, void* out, int out_bf16,
