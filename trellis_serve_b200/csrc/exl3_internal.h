@@ -72,7 +72,7 @@ struct TpExchange {
 struct GemvArgs {
     const uint32_t* packed;     // resident weights, n-blocks of all shards concatenated
     const uint32_t* xf;         // rotated activations, layout of had_in_kernel modes 1 / 2 (unless x is set)
-    const void* x;              // in-kernel rotation (rows <= 2): raw activations [rows, k], else nullptr
+    const void* x;              // in-kernel rotation (up to eight rows, see skinny_rotates_input): raw activations [rows, k], else nullptr
     const __half* suh;          //   and the input sign vectors [n_shards][k]
     int x_bf16;
     int x_glu;                  // x is gate | up [rows, 2k]: the input is silu(gate) * up (a down projection's activation)

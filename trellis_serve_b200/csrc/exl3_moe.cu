@@ -613,7 +613,7 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     l.stages = (int)stages;
     l.x_off = MOE_BAR_BYTES + stages * ups * unit;
     l.p_off = l.x_off + l.x_bytes;
-    if (l.p_off + tail > all || l.x_bytes < (uint32_t)(l.items ? moe_item_rows(mode) : MOE_BLOCK_ROWS) * row) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (l.p_off + tail > all || l.x_bytes < (uint32_t)(l.items ? MOE_TC_BLOCK_ROWS : MOE_BLOCK_ROWS) * row) return EXL3_ERR_UNSUPPORTED_ROWS;
     const CodebookConst c = codebook_const(codebook);
     l.mul = c.mul;
     l.add = c.add;

@@ -2,8 +2,8 @@
 //
 // Every (token, expert) slot is its own row because every expert has its own suh
 // (cuda/src/sglang_exl3/kernels/marlin_moe.py:11-13 of 0xSero/trellis-serve).  The routing step sorts the slots by expert; an ITEM is a
-// run of up to 32 (split) or 128 (paired) rows of one expert, a multiple of eight: either the "moe blocks" of eight rows of the engine's
-// contract (cuda/csrc/exl3_marlin_moe.cu:542-594), or the longer runs that launch_moe_align lists.  This kernel multiplies each item by
+// run of up to 128 rows of one expert, a multiple of eight: either the "moe blocks" of eight rows of the engine's contract
+// (cuda/csrc/exl3_marlin_moe.cu:542-594), or the longer runs that launch_moe_align lists.  This kernel multiplies each item by
 // its expert's matrix.  It replaces the reference's grouped Marlin instances (cuda/csrc/exl3_marlin_moe_template.h, launch at
 // exl3_marlin_moe.cu:376-408), for decode batches and for prefill alike.
 //
@@ -15,7 +15,7 @@
 //     expert's svh and the scattering of rows to their slots;
 //   * LIST, longer items: N and the pitch of B are run-time values, the activations have a ring of their own whose slot size follows
 //     the largest item, ONE warp issues the MMAs of the three decode groups in unit order into one accumulator, so that 128 rows
-//     fit into tensor memory twice.  Rotating such rows in the epilogue would be a third of all instructions on four of 32 warps
+//     fit into tensor memory twice; weights in paired mode only.  Rotating such rows in the epilogue would be a third of all instructions on four of 32 warps
 //     (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): they leave in the rotated basis, as fp16, and the kernels
 //     behind rotate them.
 //
@@ -33,8 +33,6 @@ constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, th
 // Largest expert count of one routing alignment: one CTA keeps three counters per expert in the default 48 KB of shared memory
 // ((3 * E + 1) * 4 bytes + 280 static).
 constexpr int MOE_MAX_EXPERTS = 4064;
-
-__host__ __device__ constexpr int moe_item_rows(int mode) { return mode == GEMV_SPLIT ? 32 : 128; }
 
 struct MoeGemmLaunch {
     const uint32_t* packed;          // [E][NB][KG][...] resident expert stack
@@ -119,7 +117,8 @@ __device__ __forceinline__ void moe_finish_eight(const MoeGemmLaunch& p, const f
 template <int K, int MODE, int FAM, bool LIST>
 __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_constant__ MoeGemmLaunch p)
 {
-    constexpr int ACCS = LIST ? 1 : SK_GROUPS, NMAX = LIST ? moe_item_rows(MODE) : 16;      // accumulators of a column block, and their columns
+    static_assert(!LIST || MODE == GEMV_PAIRED, "long items come with paired weights");
+    constexpr int ACCS = LIST ? 1 : SK_GROUPS, NMAX = LIST ? MOE_TC_BLOCK_ROWS : 16;        // accumulators of a column block, and their columns
     constexpr uint32_t W_BYTES = 2048u * K, HALF_BYTES = K * 128u;
     constexpr uint32_t F_ROW = MODE == GEMV_SPLIT ? 512u : 256u;            // bytes of a row in a unit's activations
     constexpr int A_COLS = MODE == GEMV_SPLIT ? 64 : 32, A_OFF = 2 * ACCS * NMAX, MMAS = MODE == GEMV_SPLIT ? 8 : 4;

@@ -62,7 +62,7 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
                           const uint32_t* w2, const __half* suh2, const __half* svh2, int K, int codebook, __half* yd, unsigned char* ws,
                           cudaStream_t st)
 {
-    constexpr int MODE = GEMV_PAIRED, ROWS = moe_item_rows(MODE);
+    constexpr int MODE = GEMV_PAIRED;
     const MoeTcLayout w = moe_tc_layout(slots, num_local, hidden, inter);
     int* sorted_ids = reinterpret_cast<int*>(ws + w.sorted);
     int* expert_ids = reinterpret_cast<int*>(ws + w.experts);
@@ -83,7 +83,7 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
     l.rotated = 1;
 
     if (int rc = launch_moe_align(topk_ids, slots, num_local, MOE_BLOCK_ROWS, w.cap, sorted_ids, expert_ids, counts, expert_map,
-                                  expert_map ? num_experts : 0, ROWS / MOE_BLOCK_ROWS, items, blk, l.err, st))
+                                  expert_map ? num_experts : 0, MOE_TC_BLOCK_ROWS / MOE_BLOCK_ROWS, items, blk, l.err, st))
         return rc;
     const long long stride = (long long)w.cap * hidden * 2;
     if (int rc = launch_moe_had_in_items(x, x_bf16, suh13, hidden, top_k, slots, w.cap, sorted_ids, expert_ids, counts, blk, ws + w.xf13, stride, st))

@@ -1,6 +1,6 @@
 // Thin wrappers over the sm_90+/sm_100 PTX used by the kernels: mbarrier, 1-D bulk async copy (TMA engine,
-// no multicast), warp-level MMA, named barriers.  Every wait is bounded: it returns false after a fixed number
-// of polls instead of spinning forever, and the caller records the failure in the device error word.
+// no multicast), clusters, counters, named barriers.  Every wait is bounded: it returns false after a fixed time (MBAR_MAX_NS) instead
+// of spinning forever, and the caller records the failure in the device error word.
 #pragma once
 #include <cstdint>
 
@@ -124,14 +124,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     return false;
 }
 
-// Shared-memory counter update with acquire-release semantics inside the CTA.
-__device__ __forceinline__ int atom_add_acq_rel_cta_shared(int* addr, int v)
-{
-    int old;
-    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_addr(addr)), "r"(v) : "memory");
-    return old;
-}
-
 // Global counter update with acquire-release semantics between the CTAs of the device.
 __device__ __forceinline__ int atom_add_acq_rel_gpu(int* addr, int v)
 {
@@ -173,9 +165,6 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
                  : "memory");
 }
 
-// Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may start before
-// the kernel ahead of it in the stream has finished.  `grid_dependency_wait` blocks until that kernel has completed
-// and its writes are visible; `grid_launch_dependents` lets the next kernel in the stream start its own prologue.
 // 1-D bulk copy shared -> global (16-byte aligned on both sides, size a multiple of 16), tracked by the issuing thread's
 // bulk groups: commit, then wait until the source may be overwritten (.read) or until the copies have completed.
 __device__ __forceinline__ void bulk_s2g(void* gmem_dst, const void* smem_src, uint32_t bytes)
@@ -186,21 +175,15 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Programmatic dependent launch: a kernel launched with the programmatic-serialization attribute may start before
+// the kernel ahead of it in the stream has finished.  `grid_dependency_wait` blocks until that kernel has completed
+// and its writes are visible; `grid_launch_dependents` lets the next kernel in the stream start its own prologue.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(int id, int threads)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// D(16x8, f32) += A(16x16, f16, row) * B(16x8, f16, col)
-__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr)

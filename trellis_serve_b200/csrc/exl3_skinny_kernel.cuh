@@ -264,53 +264,50 @@ __device__ __forceinline__ void sk_rotate_input(const SkinnyLaunch& p, const uns
     }
 }
 
-// The same for more rows (RP >= 8): a warp takes eight rows of a unit, four lanes per row (fwht128_quad), so that a unit costs 64
+// The same for three to eight rows: a warp takes all rows of a unit, four lanes per row (fwht128_quad), so that a unit costs 64
 // shuffles instead of 160 and the stores of eight rows fill whole core matrices.
-template <int MODE, int RP>
+template <int MODE>
 __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsigned char* raw, uint32_t plane, unsigned char* xs, int units,
                                                int warp, int lane)
 {
     const int rows = p.a.rows;
     const bool bf16 = p.a.x_bf16 != 0;
-    const int q = lane & 3;
+    constexpr int RP = SK_ROTATE_ROWS;
+    const int q = lane & 3, row = lane >> 2;
 #pragma unroll 1
-    for (int r0 = 0; r0 < rows; r0 += 8) {
-        const int row = r0 + (lane >> 2);
-#pragma unroll 1
-        for (int i = warp; i < units; i += SK_DECODE_WARPS) {
-            float v[32];
-            const unsigned char* signs = raw + i * 256 + q * 64;
-            const unsigned char* x = raw + (uint32_t)(1 + (row < rows ? row : 0)) * plane + i * 256 + q * 64;
+    for (int i = warp; i < units; i += SK_DECODE_WARPS) {
+        float v[32];
+        const unsigned char* signs = raw + i * 256 + q * 64;
+        const unsigned char* x = raw + (uint32_t)(1 + (row < rows ? row : 0)) * plane + i * 256 + q * 64;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const uint4 xw = reinterpret_cast<const uint4*>(x)[j], sw = reinterpret_cast<const uint4*>(signs)[j];
-                const uint32_t xv[4] = {xw.x, xw.y, xw.z, xw.w}, sv[4] = {sw.x, sw.y, sw.z, sw.w};
+        for (int j = 0; j < 4; j++) {
+            const uint4 xw = reinterpret_cast<const uint4*>(x)[j], sw = reinterpret_cast<const uint4*>(signs)[j];
+            const uint32_t xv[4] = {xw.x, xw.y, xw.z, xw.w}, sv[4] = {sw.x, sw.y, sw.z, sw.w};
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    __half2 h = *reinterpret_cast<const __half2*>(&xv[e]);
-                    if (bf16) {
-                        const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xv[e]);
-                        h = __floats2half2_rn(__low2float(bb), __high2float(bb));
-                    }
-                    const __half2 s = *reinterpret_cast<const __half2*>(&sv[e]);
-                    v[8 * j + 2 * e] = __low2float(s) * __low2float(h);
-                    v[8 * j + 2 * e + 1] = __high2float(s) * __high2float(h);
+            for (int e = 0; e < 4; e++) {
+                __half2 h = *reinterpret_cast<const __half2*>(&xv[e]);
+                if (bf16) {
+                    const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xv[e]);
+                    h = __floats2half2_rn(__low2float(bb), __high2float(bb));
                 }
+                const __half2 s = *reinterpret_cast<const __half2*>(&sv[e]);
+                v[8 * j + 2 * e] = __low2float(s) * __low2float(h);
+                v[8 * j + 2 * e + 1] = __high2float(s) * __high2float(h);
             }
-            fwht128_quad(v, lane);
-            if (row < rows) {
-                unsigned char* slot = xs + (uint32_t)i * (RP * (MODE == GEMV_SPLIT ? 512u : 256u)) + row * 16;
+        }
+        fwht128_quad(v, lane);
+        if (row < rows) {
+            unsigned char* slot = xs + (uint32_t)i * (RP * (MODE == GEMV_SPLIT ? 512u : 256u)) + row * 16;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    uint32_t hv[4];
+            for (int j = 0; j < 8; j++) {
+                uint32_t hv[4];
 #pragma unroll
-                    for (int e = 0; e < 4; e++) hv[e] = __half_as_ushort(__float2half_rn(v[4 * j + e] * HAD_SCALE));
-                    if constexpr (MODE == GEMV_SPLIT)
-                        *reinterpret_cast<uint4*>(slot + (q * 8 + j) * (RP * 16)) =
-                            make_uint4(hv[0] * 0x10001u, hv[1] * 0x10001u, hv[2] * 0x10001u, hv[3] * 0x10001u);
-                    else
-                        *reinterpret_cast<uint2*>(slot + (q * 4 + (j >> 1)) * (RP * 16) + (j & 1) * 8) = make_uint2(hv[0] | (hv[1] << 16), hv[2] | (hv[3] << 16));
-                }
+                for (int e = 0; e < 4; e++) hv[e] = __half_as_ushort(__float2half_rn(v[4 * j + e] * HAD_SCALE));
+                if constexpr (MODE == GEMV_SPLIT)
+                    *reinterpret_cast<uint4*>(slot + (q * 8 + j) * (RP * 16)) =
+                        make_uint4(hv[0] * 0x10001u, hv[1] * 0x10001u, hv[2] * 0x10001u, hv[3] * 0x10001u);
+                else
+                    *reinterpret_cast<uint2*>(slot + (q * 4 + (j >> 1)) * (RP * 16) + (j & 1) * 8) = make_uint2(hv[0] | (hv[1] << 16), hv[2] | (hv[3] << 16));
             }
         }
     }
@@ -380,6 +377,7 @@ template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_constant__ SkinnyLaunch p)
 {
     static_assert((X != SK_NORM && EPI == 0) || RP == SK_FUSED_ROWS, "the kernel normalises, and carries the residual stream of, one or two rows");
+    static_assert(X != SK_ROTATE || RP <= SK_ROTATE_ROWS, "the kernel rotates up to eight rows");
     constexpr int RB = RP <= 8 ? 1 : RP <= 16 ? 2 : 4;                      // rows that a warp finishes together
     constexpr bool ALL_FINISH = RP >= 16;
     constexpr int N = RP < 16 ? 16 : RP;                                    // MMA columns; those behind the real rows are never looked at
@@ -541,7 +539,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                     EXL3_STAMP_LANE(dw == 0, 1);
                     sk_wait(ptx::smem_addr(&x_full[1]), 0, failed);
                     sk_wait(ptx::smem_addr(&x_full[0]), 0, failed);
-                    if constexpr (RP > SK_FUSED_ROWS) sk_rotate_rows<MODE, RP>(p, smem + p.r_off, p.r_plane, xs, u1 - u0, dw, lane);
+                    if constexpr (RP > SK_FUSED_ROWS) sk_rotate_rows<MODE>(p, smem + p.r_off, p.r_plane, xs, u1 - u0, dw, lane);
                     else sk_rotate_input<MODE, X>(p, smem + p.r_off, p.r_plane, xs, u1 - u0, dw, lane);
                     EXL3_STAMP_LANE(dw == 0, 2);
                     fence_async_shared();                                   // -> visible to the tensor core's reads
