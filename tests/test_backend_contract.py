@@ -59,6 +59,42 @@ def test_routed_expert_plans_follow_the_weight_mode(codebook, halves, tokens):
         lin.set_gemv_mode(-1)
 
 
+@pytest.mark.parametrize("max_rows", [1, 16, 17, 64, 65, 2048])
+def test_dense_workspaces_hold_many_row_scratch_only_where_it_is_used(max_rows):
+    from trellis_serve_b200.kernels import linear as lin
+    from trellis_serve_b200.runtime.ops import prefers_decode
+
+    k, n = 512, 384
+    nbytes = B200Backend().workspace(_key([(k, 256, 6, "3inst"), (k, 128, 6, "3inst")]), max_rows).nbytes
+    decode = (lin.workspace_bytes(max_rows if max_rows <= 16 else lin.MAX_ROWS, k, n, 2) + 255) & ~255
+    assert nbytes == decode + (0 if prefers_decode(max_rows, k, n) else lin.tc_workspace_bytes(max_rows, k, n, 2))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_rows", [16, 17, 64, 65, 130])
+def test_dense_calls_fit_the_workspace_of_their_rows(max_rows):
+    from trellis_serve_b200.kernels import linear as lin
+    from trellis_serve_b200.runtime.layerset import random_packed, random_signs
+
+    dev, K, k, ns = torch.device("cuda", 0), 3, 512, [256, 128]
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(max_rows)
+    handle = (torch.cat([random_packed(k, n, K, gen, dev) for n in ns]), random_signs(k, gen, dev, 2), random_signs(sum(ns), gen, dev).view(-1), [256], 0, ns)
+    be = B200Backend()
+    nbytes = be.workspace(_key([(k, n, 2 * K, "3inst") for n in ns]), max_rows).nbytes
+    guarded = torch.zeros(nbytes + 4096, dtype=torch.uint8, device=dev)
+    guarded[nbytes:] = 0x5A
+    for rows in (max_rows, 1, max_rows):
+        x = torch.randn((rows, k), device=dev, generator=gen).half()
+        got, want = (torch.empty((rows, sum(ns)), dtype=torch.float16, device=dev) for _ in range(2))
+        be.run_linear(handle, x, got, guarded[:nbytes])
+        be.run_linear(handle, x, want, None)
+        assert torch.equal(got, want)
+    torch.cuda.synchronize()
+    lin.device_error(dev)
+    assert bool((guarded[nbytes:] == 0x5A).all())
+
+
 @pytest.mark.gpu
 def test_prepare_warm_run_matches_the_oracle():
     K, cb, k, ns, rows = 3, 0, 512, [256, 128], 2

@@ -148,12 +148,6 @@ def init_device(index: int) -> None:
         _initialised.add(index)
 
 
-def sm_count(index: int) -> int:
-    """Multiprocessors of device `index` as recorded at initialisation."""
-    init_device(index)
-    return int(load().exl3_device_sm_count(index))
-
-
 def int_array(values):
     values = list(values)
     return (ctypes.c_int * max(len(values), 1))(*values) if values else None
