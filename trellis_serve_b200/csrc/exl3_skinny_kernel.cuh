@@ -555,6 +555,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         // ------------------------------------------------------------------ MMA issue, one warp per group
         ptx::grid_dependency_wait();
         if constexpr (X != SK_STREAM) ptx::named_bar_sync(SK_BAR_X, (SK_DECODE_WARPS + SK_GROUPS) * 32);
+        else EXL3_STAMP_LANE(warp == SK_MMA_WARP, 1);
         // The group is a constant of each warp's code, so that every operand of the MMAs is warp-uniform to the compiler.
         auto multiply = [&](auto gconst) {
             constexpr int group = decltype(gconst)::value;
@@ -563,6 +564,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 if constexpr (X == SK_STREAM) sk_wait(x_bar + slot8, parity, failed);
             };
             SkWalk at(group, ups, fills, enter);
+            if constexpr (X == SK_STREAM && group == 0) EXL3_STAMP_LANE(true, 2);
             uint32_t xa = ptx::smem_addr(xs) + (group >> 1) * F_BYTES + (group & 1) * (F_BYTES / 2);
             constexpr uint32_t chunk = RP;                                  // 16-byte rows between chunks of 8 k slots
             constexpr uint32_t b_hi = (128u >> 4) | (1u << 14);             // 8-row groups 128 bytes apart; descriptor version

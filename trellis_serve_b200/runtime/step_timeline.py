@@ -7,8 +7,8 @@ Build a second copy of the library with the stamps compiled in and point this mo
     python -m trellis_serve_b200.runtime.step_timeline --lib /tmp/libexl3_timeline.so --layers 8
 
 In that build thread 0 of every CTA of the decode GEMV and of the attention kernel writes the time at a few points
-(kernel entry, dependency wait resolved, own input rotated, first weights landed, loop end, kernel end; attention: scores,
-values, hand-over count, merge end).  The report gives, per linear of a layer, those points relative to the end of the GEMV
+(kernel entry, dependency wait resolved, own input rotated or first streamed rows landed, first weights landed, loop end, kernel end;
+attention: scores, values, hand-over count, merge end).  The report gives, per linear of a layer, those points relative to the end of the GEMV
 launch ahead of it (median over layers), i.e. what sits on the critical path between two linears.  The stamps cost a few
 stores per CTA; the normal build has none of this code.
 """
