@@ -263,7 +263,7 @@ def run_moe(args) -> None:
         moe.TC_ROWS_PER_EXPERT = 0 if args.moe_path == "tc" else 1 << 30
     tensor_core = moe.moe_block_size(T, top_k, E) == 128
     if tensor_core:
-        # many rows per expert: the allocation-free layer entry, which sends the class through the grouped tcgen05 GEMM
+        # many rows per expert: the allocation-free layer entry, which sends the class through the kernels for long items
         mixed = moe.MixedPack([pack], [torch.arange(E, dtype=torch.int32, device=dev)], E, H, I, cb)
         ws = torch.zeros(moe.layer_workspace_bytes([E], H, I, cb, T, top_k), dtype=torch.uint8, device=dev)
         layer = lambda: moe.run_layer(x, wts, ids, mixed, out, ws)
@@ -294,12 +294,14 @@ def run_moe(args) -> None:
                       "dtype": "f16", "data": "synthetic",
                       "config": {"workload": f"MoE layer hidden 2048, 256 experts, intermediate 512, top-8, K=3 3INST, {T} tokens",
                                  "tokens": T, "distinct_experts": distinct, "touched_bytes": nbytes,
-                                 "path": "grouped tcgen05 GEMM, 128-row moe blocks" if tensor_core else "grouped GEMV, 8-row moe blocks",
+                                 "path": "items of up to 128 rows of an expert" if tensor_core else "blocks of eight rows",
                                  "tflops": 2.0 * T * top_k * 3 * H * I / ms / 1e9,
-                                 "l2": "the layer's working set is L2-resident on replay (302 MB of experts, touched subset smaller)"},
+                                 "l2": "touched experts' weights larger than L2, no flush" if nbytes > 126e6
+                                 else "touched experts' weights stay in L2 between replays"},
                       "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None,
-                                   "peak_source": f"of {kind}", "kernel": "gemm_tc_kernel (grouped)" if tensor_core else "moe_gemm_kernel"},
-                      "gpu_launches": (11 if tensor_core else 6) * args.steps, "clocks": clocks.summary()}))
+                                   "peak_source": f"of {kind}", "kernel": "moe_gemm_kernel"},
+                      # align, input rotation, gate|up, activation, down, combine; with long items an output rotation before the combine
+                      "gpu_launches": (7 if tensor_core else 6) * args.steps, "clocks": clocks.summary()}))
 
 
 def _graph_ring_time(run_one, ring: int, reps: int = 5) -> float:
