@@ -213,7 +213,8 @@ exl3_status exl3_rope_decode_attention(const void *qkv, int dtype, int rows, int
  * library GEMM sequence `dense_group` (cuda/src/sglang_exl3/runtime/ops.py:36-59).  The workspace
  * (exl3_gemm_tc_workspace_bytes) holds the rotated activations, the rotated-basis product and the fp32 slabs of cut
  * reductions; its first 256 bytes must be zero (error word).
- * exl3_linear_tc_padded: x is [rows, x_cols] with x_cols <= k a multiple of 8, read as zeros from there on.  x, suh_cat, svh_cat and y must be 16-byte aligned. */
+ * exl3_linear_tc_padded: x is [rows, x_cols] with x_cols <= k a multiple of 8, read as zeros from there on.  x, suh_cat, svh_cat and y
+ * must be 16-byte aligned. */
 /* exl3_linear for modules whose true sizes are not the stored, 128-padded ones: x is [rows, x_cols] (x_cols <= k, read as zeros from
  * there on), y [rows, sum(out_widths)] holds the first out_widths[s] columns of every matrix of the group, side by side.  fp16 / bf16
  * outputs. */
@@ -222,8 +223,8 @@ exl3_status exl3_linear_ragged(const void *x, int x_dtype, int x_cols, const uin
                                int n_shards, int rows, int k, int n_total, void *y, int y_dtype, void *workspace,
                                size_t workspace_bytes, void *stream);
 
-/* Cost model of the switch between exl3_linear and exl3_linear_tc for a fused group of n_total columns: 1 when exl3_linear is
- * expected to be the faster one on `sms` multiprocessors.  Pure host arithmetic. */
+/* The switch between exl3_linear and exl3_linear_tc for a fused group of n_total columns on `sms` multiprocessors: 1 when the call
+ * belongs to exl3_linear.  Today that is up to 64 rows, one pass over the weights, whatever the sizes.  Pure host arithmetic. */
 int exl3_prefers_decode(int rows, int k, int n_total, int sms);
 size_t exl3_gemm_tc_workspace_bytes(int rows, int k, int n_total, int n_shards);
 exl3_status exl3_linear_tc_padded(const void *x, int x_dtype, int x_cols, const uint32_t *packed, int K, int codebook,

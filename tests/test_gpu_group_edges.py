@@ -145,7 +145,7 @@ def test_plain_calls_are_seen_by_whatever_watches():
         y = ops.linear(x, *rest)
         assert any("exl3_b200" in name for name in watch.seen) and ops._direct(x, *rest) is None
     assert torch.equal(y, want)
-    with profile(activities=[ProfilerActivity.CPU]) as prof:
+    with profile(activities=[ProfilerActivity.CPU], acc_events=True) as prof:
         y = ops.linear(x, *rest)
     assert "exl3_b200::linear" in {e.key for e in prof.key_averages()} and torch.equal(y, want)
     assert ops._direct(x, *rest) is not None                            # nothing watches any more

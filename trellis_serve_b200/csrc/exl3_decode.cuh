@@ -163,12 +163,12 @@ __device__ __forceinline__ uint32_t window(const LaneTile<K>& t)
 // ---------------------------------------------------------------------------------------------- pipe-balanced windows
 //
 // On sm_100 shifts, logic ops and byte permutes all issue on the ALU pipe (16 lanes per scheduler) while integer
-// multiply-add issues on the equally wide FMA pipe, and the ALU pipe is what bounds the decode.  A shift-and-mask
+// multiply-add issues on the equally wide FMA pipe, and the ALU pipe would be the busier of the two.  A shift-and-mask
 // extraction costs two ALU slots per weight on top of the codebook's logic op.  Here a window is instead cut out with one
 // multiply by a power of two (drops the bits above the window, FMA pipe) and one shift right by 16 (drops the bits below,
 // ALU pipe): E is re-read as 32-bit registers R_j = E[16j, 16j+32), so every window lies inside one of them.  Windows
 // that start on a byte boundary (all of them at K = 8, half at K = 4) take a single mask or byte permute.  The powers of
-// two come from kernel parameters (constant bank) so that the multiply stays a multiply.
+// two come from kernel parameters (constant bank) or from shared memory so that the multiply stays a multiply.
 
 struct Pow2 {
     uint32_t v[32];          // v[c] = 1 << c

@@ -9,14 +9,14 @@
 //               level decode of exl3_decode.cuh, weights rounded to fp16 exactly as the reference decoder) and stores
 //               it K-major, in 8x8 core matrices, as the B operand; after the main loop the same warps read the
 //               accumulators back from tensor memory (tcgen05.ld) and store fp16 rows
-//   warp 8      A producer: one 64 KB bulk async copy per stage; the rotated activations are laid out in global
-//               memory by had_in_tc_kernel exactly as the A operand wants them (four 128 x 64 K-major tiles)
+//   warp 8      A producer: a 16 KB bulk async copy per 128-row tile that holds rows; the rotated activations are laid out in
+//               global memory by had_in_tc_kernel exactly as the A operand wants them (four 128 x 64 K-major tiles)
 //   warp 9      allocates tensor memory (512 columns = four 128 x 128 fp32 accumulators), issues
 //               tcgen05.mma.cta_group::1.kind::f16 (M 128, N 128, K 16) from one elected lane and commits to the
 //               mbarriers that release the stage / publish the accumulators
 //
-// Each weight block is decoded once per 512 rows and reused by 16 MMAs, so the kernel is bound by the tensor pipe,
-// not by the decode.  Every wait is bounded (exl3_ptx.cuh); on a time-out the error word is set and the control flow
+// Each weight block is decoded once per 512 rows and reused by 16 MMAs, so at hundreds of rows the kernel is bound by the tensor pipe,
+// not by the decode; above 256 rows most shapes go to the CTA pairs of gemm_tc_pair_kernel below.  Every wait is bounded (exl3_ptx.cuh); on a time-out the error word is set and the control flow
 // continues unchanged to the common exit, where tensor memory is released.
 #include <cstring>
 

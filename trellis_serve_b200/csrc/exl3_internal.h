@@ -76,7 +76,7 @@ struct GemvArgs {
     const __half* suh;          //   and the input sign vectors [n_shards][k]
     int x_bf16;
     int x_glu;                  // x is gate | up [rows, 2k]: the input is silu(gate) * up (a down projection's activation)
-    // Normalised input (consumer side of a residual block, XR > 0): x is the residual stream z [rows, k], its sums of squares
+    // Normalised input (consumer side of a residual block, SK_NORM): x is the residual stream z [rows, k], its sums of squares
     // per 128 columns are in ssq [rows, k/128] (written by the epilogue of the linear ahead or by the stats kernel), and the
     // input proper is z * rsqrt(mean square + eps) * norm_weight.
     const void* norm_weight;

@@ -19,7 +19,7 @@
 //     (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): they leave in the rotated basis, as fp16, and the kernels
 //     behind rotate them.
 //
-// Bound by the ALU pipe of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.
+// Bound by the issue of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.
 #pragma once
 #include "exl3_skinny_kernel.cuh"
 
@@ -30,8 +30,8 @@ constexpr int MOE_MAX_GRID = 192;                                // CTAs of a la
 constexpr int MOE_ERR_WORDS = 64;                                // header of the many-row workspace: error word
 constexpr int MOE_X_SLOTS = 4, MOE_X_UNITS = 4;                  // most slots of the activation ring, and units of a slot
 constexpr uint32_t MOE_BAR_BYTES = 640, MOE_TABLE_OFF = 384;     // barriers, then the constants of the decode loop
-// Largest expert count of one routing alignment: one CTA keeps three counters per expert in the default 48 KB of shared memory
-// ((3 * E + 1) * 4 bytes + 280 static).
+// Largest expert count of one routing alignment: the form of one CTA keeps three counters per expert in the default 48 KB of shared
+// memory ((3 * E + 1) * 4 bytes + 280 static), that of a cluster four in the larger size it opts in to.
 constexpr int MOE_MAX_EXPERTS = 4064;
 
 struct MoeGemmLaunch {

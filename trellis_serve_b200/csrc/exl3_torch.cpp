@@ -71,7 +71,7 @@ void scratch_clear(int64_t kind)
     for (auto& t : g_scratch[kind]) t = at::Tensor();
 }
 
-// Measurement knobs of runtime/ops.py: [0] row count from which the many-row path is taken (0: by cost), [1] 1: the many-row
+// Measurement knobs of runtime/ops.py: [0] row count from which the many-row path is taken (0: exl3_prefers_decode), [1] 1: the many-row
 // path decodes the weights and calls the library GEMM.
 int64_t g_knob[2] = {0, 0};
 int64_t knob(int64_t which, int64_t value)

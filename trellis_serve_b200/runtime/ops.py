@@ -42,8 +42,7 @@ _lib = torch.library.Library("exl3_b200", "FRAGMENT")       # must stay alive at
 class _Module(types.ModuleType):
     """Measurement knobs, module attributes that live in the native operator.
 
-    DENSE_ROWS: row count from which the many-row path is taken; 0 = decide per call with `prefers_decode` (the crossover depends
-    on the shape).  PREFILL: "tc" = fused tcgen05 kernel; "library" = decode to fp16 + library GEMM (the reference's sequence), for
+    DENSE_ROWS: row count from which the many-row path is taken; 0 = decide per call with `prefers_decode`.  PREFILL: "tc" = fused tcgen05 kernel; "library" = decode to fp16 + library GEMM (the reference's sequence), for
     comparisons."""
 
     @property
@@ -69,8 +68,8 @@ _ops.knob(1, int(os.environ.get("EXL3_B200_PREFILL", "tc") == "library"))
 
 
 def prefers_decode(rows: int, k: int, n_total: int, sms: int = 148) -> bool:
-    """Whether the decode kernel is expected to be faster than the tensor-core kernel for these sizes; `sms` is the device's
-    multiprocessor count."""
+    """Whether a call goes through the decode kernel: up to 64 rows, one pass over the weights.  The sizes and the device's multiprocessor
+    count `sms` are part of the interface; the rule does not look at them today."""
     return bool(_native_lib.load().exl3_prefers_decode(rows, k, n_total, sms))
 
 
