@@ -26,8 +26,8 @@
 // for MUL1 at K = 6), are 12 to 16 clk of a SM's four schedulers.  The loop takes 16.3 / 14.4 / 16.2 / 14.1 clk per tile and SM at K =
 // 3 / 4 / 6 / 8 (stamps in chained launches at 1.965 GHz; 15.5 / 16.3 / 17.7 at K = 2 / 5 / 7), 18.5 for MUL1 at K = 3 and 6; the ALU
 // pipe is busy in 60 to 64 % of the active cycles at every K (MUL1: the FMA pipe in 72 %).  The MMAs take 4 clk per tile of the tensor
-// pipe at N = 16 and 8 at N = 64, so the rate does not depend on the row count up to 32; at N = 64, where half units are handed over
-// in two pieces, it is 27.  Against the register-level kernel on mma.sync that it replaces (two CTAs of 16 warps, 8 rows per MMA),
+// pipe at N = 16 and 8 at N = 64 and run beside it: 15.2 to 16.3 clk (K = 3) up to 16 rows, 17.6 at 32, 22.5 at 33 to 64, where half
+// units are handed over in two pieces (27 in short launches).  Against the register-level kernel on mma.sync that it replaces (two CTAs of 16 warps, 8 rows per MMA),
 // chained launches over distinct weights, K = 3: 5120 x 34816 48.8 -> 46.3 us at one row and 51 -> 47.1 at four; 17408 x 5120 28.5 ->
 // 26.6; 5120 x 5120 12.1 -> 11.3; 17408 x 5120, K = 6, MUL1, 16 rows 45.6 -> 35.0.  What is not the loop, per launch at one row: 1.8
 // to 3.5 us from the end of the launch ahead until the input is rotated, 1.7 to 2.2 us by which CTAs that could not become resident
