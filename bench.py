@@ -559,7 +559,7 @@ def main() -> None:
     ap.add_argument("--workload", default="decode", choices=["decode", "prefill", "moe", "c1", "step"],
                     help="decode = the headline 27B-shape layer set (default); prefill / moe / c1 = secondary single-GPU workloads; "
                          "step = the whole transformer decode step (attention and KV cache included), any N")
-    ap.add_argument("--moe-path", choices=["auto", "gemv", "tc"], default="auto", help="--workload moe: force the grouped GEMV or the grouped tensor-core path")
+    ap.add_argument("--moe-path", choices=["auto", "gemv", "tc"], default="auto", help="--workload moe: force blocks of eight rows (gemv) or long items (tc)")
     ap.add_argument("--no-sweep", action="store_true", help="skip the batch and bit-rate sweep appended to the default line")
     args = ap.parse_args()
     if args.warmup < 3:
