@@ -160,15 +160,19 @@ __device__ __forceinline__ uint32_t window(const LaneTile<K>& t)
     }
 }
 
-// ---------------------------------------------------------------------------------------------- pipe-balanced windows
+// ---------------------------------------------------------------------------------------------- windows in few instructions
 //
-// On sm_100 shifts, logic ops and byte permutes all issue on the ALU pipe (16 lanes per scheduler) while integer
-// multiply-add issues on the equally wide FMA pipe, and the ALU pipe would be the busier of the two.  A shift-and-mask
-// extraction costs two ALU slots per weight on top of the codebook's logic op.  Here a window is instead cut out with one
-// multiply by a power of two (drops the bits above the window, FMA pipe) and one shift right by 16 (drops the bits below,
-// ALU pipe): E is re-read as 32-bit registers R_j = E[16j, 16j+32), so every window lies inside one of them.  Windows
-// that start on a byte boundary (all of them at K = 8, half at K = 4) take a single mask or byte permute.  The powers of
-// two come from kernel parameters (constant bank) or from shared memory so that the multiply stays a multiply.
+// The decode loops are bound by instruction issue, so a window is cut out of 32-bit registers of E that are chosen per bit rate:
+//
+//   * a window at bit 0, 8 or 16 of a register costs one instruction (mask, byte permute, shift);
+//   * any other costs two: one multiply by a power of two (drops the bits above the window, FMA pipe) and one shift right by 16 (drops
+//     those below, ALU pipe) -- shift and mask would put both on the ALU pipe, the busier of the two;
+//   * a register costs one instruction (permute or funnel shift) unless the lane's words are it already.
+//
+// Registers and windows together: 12 / 16 / 11 / 16 / 16 / 16 / 10 instructions per tile and lane at K = 2 .. 8, against 15 / 17 / 13 / 17 /
+// 16 / 19 / 10 with registers at E[16 j, 16 j + 32) (17408 x 5120, one row, chained launches: K = 5 27.2 -> 25.8 us, K = 7 29.4 -> 27.0, K =
+// 3, 4 and 6 1 to 2 % less, K = 2 and 8 the same).  The powers of two come from kernel parameters (constant bank) or from shared memory
+// so that the multiply stays a multiply.
 
 struct Pow2 {
     uint32_t v[32];          // v[c] = 1 << c
@@ -181,32 +185,56 @@ __host__ inline Pow2 make_pow2()
     return p;
 }
 
-template <int K>
-struct LaneRegs {
-    uint32_t r[4];           // r[j] = E bits [16j, 16j + 32)
+// Register and bit offset at which the window of E bits [lo, lo + 16) is found.
+struct WindowAt {
+    int reg, sh;
 };
 
+template <int K>
+__host__ __device__ constexpr WindowAt window_at(int lo)
+{
+    if (K == 2) return {(lo & 7) >> 1, lo & 8};
+    if (K == 3) return lo < 8 ? WindowAt{0, lo} : WindowAt{1, lo - 8};
+    if (K == 4) return lo == 12 || lo >= 20 ? WindowAt{1, lo - 12} : WindowAt{0, lo};
+    if (K == 5) return lo < 20 ? WindowAt{0, lo} : WindowAt{1, lo - 20};
+    if (K == 6) return lo < 18 ? WindowAt{0, lo} : lo < 36 ? WindowAt{1, lo - 18} : WindowAt{2, lo - 32};
+    if (K == 7) return lo < 21 ? WindowAt{0, lo} : lo < 42 ? WindowAt{1, lo - 21} : WindowAt{2, lo - 40};
+    return lo <= 16 ? WindowAt{0, lo} : lo == 24 ? WindowAt{1, 8} : lo <= 48 ? WindowAt{2, lo - 32} : WindowAt{3, 8};
+}
+
+template <int K>
+struct LaneRegs {
+    uint32_t r[4];           // see window_at
+};
+
+// own: this lane's right-aligned words; prev0: word 0 of the previous lane's right-aligned share of the same tile.
 template <int K>
 __device__ __forceinline__ LaneRegs<K> lane_regs(const uint32_t (&own)[2], uint32_t prev0)
 {
     LaneRegs<K> R;
-    if constexpr (K == 2) {
+    R.r[0] = own[0];
+    R.r[1] = R.r[2] = R.r[3] = 0;
+    if constexpr (K == 2) {                                  // own 16 bits
         R.r[0] = prmt(own[0], prev0, 0x5410);
-        R.r[1] = R.r[2] = R.r[3] = 0;
-    } else if constexpr (K == 3) {
-        R.r[0] = prmt(own[0], prev0, 0x4210);
-        R.r[1] = prmt(own[0], prev0, 0x6542);
-        R.r[2] = R.r[3] = 0;
-    } else if constexpr (K == 4) {
-        R.r[0] = own[0];
-        R.r[1] = prmt(own[0], prev0, 0x5432);
-        R.r[2] = R.r[3] = 0;
-    } else {
-        const LaneTile<K> t = assemble<K>(own, prev0);
-        R.r[0] = t.e[0];
-        R.r[1] = prmt(t.e[0], t.e[1], 0x5432);
-        R.r[2] = t.e[1];
-        R.r[3] = (K >= 7) ? prmt(t.e[1], t.e[2], 0x5432) : 0u;
+        R.r[1] = R.r[0] >> 2;
+        R.r[2] = R.r[0] >> 4;
+        R.r[3] = R.r[0] >> 6;
+    } else if constexpr (K == 3) {                           // own 24
+        R.r[1] = prmt(own[0], prev0, 0x5421);                // E[8, 40)
+    } else if constexpr (K == 4) {                           // own 32
+        R.r[1] = __funnelshift_r(own[0], prev0, 12);
+    } else if constexpr (K == 5) {                           // own 40
+        R.r[1] = __funnelshift_r(own[0], prmt(own[1], prev0, 0x6540), 20);
+    } else if constexpr (K == 6) {                           // own 48
+        R.r[1] = __funnelshift_r(own[0], own[1], 18);
+        R.r[2] = prmt(own[1], prev0, 0x5410);                // E[32, 64)
+    } else if constexpr (K == 7) {                           // own 56
+        R.r[1] = __funnelshift_r(own[0], own[1], 21);
+        R.r[2] = prmt(own[1], prev0, 0x5421);                // E[40, 72)
+    } else {                                                 // own 64
+        R.r[1] = prmt(own[0], own[1], 0x5432);               // E[16, 48)
+        R.r[2] = own[1];
+        R.r[3] = prmt(own[1], prev0, 0x5432);                // E[48, 80)
     }
     return R;
 }
@@ -215,17 +243,12 @@ __device__ __forceinline__ LaneRegs<K> lane_regs(const uint32_t (&own)[2], uint3
 template <int K, int P, typename Powers>
 __device__ __forceinline__ uint32_t window_low(const LaneRegs<K>& R, const Powers& pw)
 {
-    constexpr int lo = K * (7 - P);
-    constexpr int j = lo / 16;
-    constexpr int sh = lo % 16;
-    static_assert(j < 4, "window outside the lane registers");
-    if constexpr (sh == 0) {
-        return R.r[j] & 0xFFFFu;
-    } else if constexpr (sh == 8) {
-        return prmt(R.r[j], 0u, 0x4421);          // byte-aligned window (K = 2, 4, 6, 8): one permute
-    } else {
-        return (R.r[j] * pw.v[16 - sh]) >> 16;
-    }
+    constexpr WindowAt at = window_at<K>(K * (7 - P));
+    static_assert(at.sh >= 0 && at.sh <= 16, "window outside its register");
+    if constexpr (at.sh == 0) return R.r[at.reg] & 0xFFFFu;
+    else if constexpr (at.sh == 8) return prmt(R.r[at.reg], 0u, 0x4421);
+    else if constexpr (at.sh == 16) return R.r[at.reg] >> 16;
+    else return (R.r[at.reg] * pw.v[16 - at.sh]) >> 16;
 }
 
 // ---------------------------------------------------------------------------------------------- codebooks

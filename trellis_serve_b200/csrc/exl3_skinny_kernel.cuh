@@ -163,8 +163,8 @@ struct SkPow2 {
     {
 #pragma unroll
         for (int P = 0; P < 8; P++) {
-            const int sh = (K * (7 - P)) % 16;
-            if (sh != 0 && sh != 8) v[16 - sh] = ptx::lds32(table + (16 - sh) * 4);
+            const int sh = window_at<K>(K * (7 - P)).sh;
+            if (sh % 8 != 0) v[16 - sh] = ptx::lds32(table + (16 - sh) * 4);
         }
     }
 };
