@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (threadIdx.x < 34)
-        reinterpret_cast<uint32_t*>(smem + SK_TABLE_OFF)[threadIdx.x] = threadIdx.x < 32 ? 1u << threadIdx.x : threadIdx.x == 32 ? p.mul : p.add;
+    if (threadIdx.x < 35)
+        reinterpret_cast<uint32_t*>(smem + SK_TABLE_OFF)[threadIdx.x] = threadIdx.x < 32 ? 1u << threadIdx.x : threadIdx.x == 32 ? p.mul : threadIdx.x == 33 ? p.add : HASH_FLIP;
     sk_fence_before();
     __syncthreads();
     sk_fence_after();
@@ -464,7 +464,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         // ------------------------------------------------------------------ decode
         const int dw = warp - SK_DECODE_WARP, group = dw >> 3, nt = 2 * (dw & 3) + ((dw >> 2) & 1);  // columns 16 nt .. = tensor-memory lanes of this warp's quarter
         const uint32_t table = ptx::smem_addr(smem + SK_TABLE_OFF);
-        const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132)};
+        const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132), ptx::lds32(table + 136)};
+        const int source = __shfl_sync(0xFFFFFFFFu, lane, (lane + 31) & 31);      // from a shuffle, or the addition is made again per tile
         const SkPow2<K> pw(table);
         const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
         auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 constexpr int T = decltype(tconst)::value;
                 uint32_t own[2];
                 own_words<K, T>(L, own);
-                const uint32_t prev0 = __shfl_sync(0xFFFFFFFFu, own[0], (lane + 31) & 31);
+                const uint32_t prev0 = __shfl_sync(0xFFFFFFFFu, own[0], source);
                 const LaneRegs<K> R = lane_regs<K>(own, prev0);
                 uint32_t w[8];
                 decode_tile_regs<K, MODE, FAM>(R, pw, cbc, w);
