@@ -242,8 +242,10 @@ __device__ __forceinline__ LaneRegs<K> lane_regs(const uint32_t (&own)[2], uint3
     return R;
 }
 
-// 16-bit trellis state of element P (0..7) of the lane, bits above it cleared.
-template <int K, int P, typename Powers>
+// 16-bit trellis state of element P (0..7) of the lane, bits above it cleared.  MUL1 spends two multiplies and half an fp16 multiply-add
+// per weight on the FMA pipe already, so its windows are cut with shift and mask (17408 x 5120, one row, K = 3 / 6: 28.6 -> 26.4 and
+// 29.6 -> 28.0 us); for the hash codebooks the same costs 2 us.
+template <int K, int P, int FAM, typename Powers>
 __device__ __forceinline__ uint32_t window_low(const LaneRegs<K>& R, const Powers& pw)
 {
     constexpr WindowAt at = window_at<K>(K * (7 - P));
@@ -251,6 +253,7 @@ __device__ __forceinline__ uint32_t window_low(const LaneRegs<K>& R, const Power
     if constexpr (at.sh == 0) return R.r[at.reg] & 0xFFFFu;
     else if constexpr (at.sh == 8) return prmt(R.r[at.reg], 0u, 0x4421);
     else if constexpr (at.sh == 16) return R.r[at.reg] >> 16;
+    else if constexpr (FAM == FAM_MUL1) return (R.r[at.reg] >> at.sh) & 0xFFFFu;
     else return (R.r[at.reg] * pw.v[16 - at.sh]) >> 16;
 }
 

@@ -129,9 +129,9 @@ __device__ __forceinline__ void tc_decode_tile(const uint32_t (&L)[K], unsigned 
     const uint32_t prev0 = __shfl_sync(0xFFFFFFFFu, own[0], (lane + 31) & 31);
     const LaneRegs<K> R = lane_regs<K>(own, prev0);
     uint32_t st[8];
-    st[0] = window_low<K, 0>(R, pw); st[1] = window_low<K, 1>(R, pw); st[2] = window_low<K, 2>(R, pw);
-    st[3] = window_low<K, 3>(R, pw); st[4] = window_low<K, 4>(R, pw); st[5] = window_low<K, 5>(R, pw);
-    st[6] = window_low<K, 6>(R, pw); st[7] = window_low<K, 7>(R, pw);
+    st[0] = window_low<K, 0, FAM>(R, pw); st[1] = window_low<K, 1, FAM>(R, pw); st[2] = window_low<K, 2, FAM>(R, pw);
+    st[3] = window_low<K, 3, FAM>(R, pw); st[4] = window_low<K, 4, FAM>(R, pw); st[5] = window_low<K, 5, FAM>(R, pw);
+    st[6] = window_low<K, 6, FAM>(R, pw); st[7] = window_low<K, 7, FAM>(R, pw);
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) w[j] = FAM == FAM_HASH ? hash_pair_rounded(st[2 * j], st[2 * j + 1], cbc) : mul1_pair(st[2 * j], st[2 * j + 1], cbc);

@@ -39,8 +39,8 @@ template <int K, int MODE, int FAM, typename Powers>
 __device__ __forceinline__ void decode_tile_regs(const LaneRegs<K>& R, const Powers& pw, CodebookConst cbc, uint32_t (&w)[8])
 {
     uint32_t s[8];
-    s[0] = window_low<K, 0>(R, pw); s[1] = window_low<K, 1>(R, pw); s[2] = window_low<K, 2>(R, pw); s[3] = window_low<K, 3>(R, pw);
-    s[4] = window_low<K, 4>(R, pw); s[5] = window_low<K, 5>(R, pw); s[6] = window_low<K, 6>(R, pw); s[7] = window_low<K, 7>(R, pw);
+    s[0] = window_low<K, 0, FAM>(R, pw); s[1] = window_low<K, 1, FAM>(R, pw); s[2] = window_low<K, 2, FAM>(R, pw); s[3] = window_low<K, 3, FAM>(R, pw);
+    s[4] = window_low<K, 4, FAM>(R, pw); s[5] = window_low<K, 5, FAM>(R, pw); s[6] = window_low<K, 6, FAM>(R, pw); s[7] = window_low<K, 7, FAM>(R, pw);
     if constexpr (MODE == GEMV_SPLIT) {
 #pragma unroll
         for (int j = 0; j < 8; j++) w[j] = hash_pair(s[j], cbc);

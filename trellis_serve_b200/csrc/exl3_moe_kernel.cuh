@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         const uint32_t table = ptx::smem_addr(smem + MOE_TABLE_OFF);
         const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132), ptx::lds32(table + 136)};
         const int source = __shfl_sync(0xFFFFFFFFu, lane, (lane + 31) & 31);
-        const SkPow2<K> pw(table);
+        const SkPow2<K, FAM> pw(table);
         const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
         const int halves = 2 * units;
         if (halves > 0) {

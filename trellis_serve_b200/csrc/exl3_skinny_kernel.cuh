@@ -156,7 +156,7 @@ __device__ __forceinline__ void sk_bar_arrive(int id, int threads) { asm volatil
 // The decode loop's constants: the codebook's multiplier and addend and the powers of two of the windows of a bit rate (see
 // window_low), read once per warp from shared memory.  Taken from the kernel's parameters they are fetched again for every half unit
 // (7 loads of uniform registers per warp, 1.7 per tile): a shared-memory read is one that the compiler does not repeat.
-template <int K>
+template <int K, int FAM>
 struct SkPow2 {
     uint32_t v[32];
     __device__ __forceinline__ SkPow2(uint32_t table)
@@ -164,7 +164,7 @@ struct SkPow2 {
 #pragma unroll
         for (int P = 0; P < 8; P++) {
             const int sh = window_at<K>(K * (7 - P)).sh;
-            if (sh % 8 != 0) v[16 - sh] = ptx::lds32(table + (16 - sh) * 4);
+            if (FAM == FAM_HASH && sh % 8 != 0) v[16 - sh] = ptx::lds32(table + (16 - sh) * 4);
         }
     }
 };
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         const uint32_t table = ptx::smem_addr(smem + SK_TABLE_OFF);
         const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132), ptx::lds32(table + 136)};
         const int source = __shfl_sync(0xFFFFFFFFu, lane, (lane + 31) & 31);      // from a shuffle, or the addition is made again per tile
-        const SkPow2<K> pw(table);
+        const SkPow2<K, FAM> pw(table);
         const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
         auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
         SkWalk at(group, ups, fills, enter);
