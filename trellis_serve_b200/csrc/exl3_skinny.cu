@@ -66,8 +66,11 @@ static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaun
     if (l.grid > GEMV_MAX_GRID) l.grid = GEMV_MAX_GRID;
     l.units_q = (int)(units / l.grid);
     l.units_r = (int)(units % l.grid);
-    // Stages of whole units.  A bulk copy costs a few hundred nanoseconds whatever its size: copies of 24 KB of weights or a little
-    // more, as long as three such stages fit; a short range travels as one copy.
+    // Stages of whole units, as long as three fit; a short range travels as one copy.  A bulk copy costs a few hundred nanoseconds whatever
+    // its size (24 KB of weights or more), and a group of decode warps changes stages every 2 units / 3 steps: six units where the
+    // rows are resident (17408 x 5120, one row, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1, K
+    // = 8 25.4 -> 24.7), no more than 24 KB where they travel with the weights and the first stage is waited for (5120 x 5120, 16 rows: 18.5
+    // us against 19.1 with six units).
     const size_t w = 2048u * (size_t)a.K, f = (size_t)operand_pitch(a.rows) * (a.mode == GEMV_SPLIT ? 512 : 256);
     const size_t most = (size_t)(l.units_q + (l.units_r ? 1 : 0));
     const SkRaw raw = sk_raw_planes(x, a.x_glu);
@@ -76,6 +79,7 @@ static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaun
     if (fixed >= (size_t)d->max_smem_optin) return EXL3_ERR_UNSUPPORTED_ROWS;
     const size_t budget = (size_t)d->max_smem_optin - fixed, unit = w + (x == SK_STREAM ? f : 0);
     size_t ups = (24 * 1024 + w - 1) / w;
+    if (x != SK_STREAM && ups < 6) ups = 6;
     if (ups > most) ups = most;
     while (ups > 2 && budget / (ups * unit) < 3) ups--;      // a ring needs stages of two units or more (see SkWalk)
     size_t stages = budget / (ups * unit);
