@@ -175,11 +175,11 @@ exl3_status exl3_rmsnorm_linear(const void *x, int x_dtype, const void *residual
  *                          `*position` (device int, so a captured graph can move on): q in place, k into slot `*position` of
  *                          k_cache [rows, kv_heads, t_max, 128], v copied into v_cache.
  *   exl3_decode_attention  softmax(q k^T * scale) v over cache positions 0..*position for every query head (q_heads a
- *                          multiple of kv_heads, ratio 1, 2, 4, 5 or 8), split over the cache in chunks of 128 positions
- *                          and merged in a fixed order by the last CTA of each (row, KV head) to finish (one launch);
+ *                          multiple of kv_heads, ratio 1, 2, 4, 5 or 8), split over the CTAs of a cluster per (row, KV head)
+ *                          and merged in a fixed order (one launch);
  *                          out [rows, q_heads * 128] in `dtype` (may be NULL).  scratch: exl3_attention_scratch_bytes(),
- *                          256-byte aligned, zero-filled once before its first use (an error word that exl3_device_error reads,
- *                          then arrival counters that every call leaves zero); exl3_init_device must have run.  suh_next != NULL: a head is one rotation block of the o
+ *                          256-byte aligned, zero-filled once before its first use (an error word that exl3_device_error
+ *                          reads); exl3_init_device must have run.  suh_next != NULL: a head is one rotation block of the o
  *                          projection's input, so the merge also writes that linear's rotated fragments into `workspace`
  *                          (as exl3_rotate_fragments would from `out`) and exl3_linear_prerotated can follow directly.
  *   exl3_rope_decode_attention  the two above in one call and one launch: the attention kernel rotates
@@ -187,9 +187,8 @@ exl3_status exl3_rmsnorm_linear(const void *x, int x_dtype, const void *residual
  *                          rotates the new key into k_cache and copies the new value into v_cache before it reads them; same
  *                          roundings, same bits.  qkv must be 8-byte aligned.
  * Before it waits for the kernel ahead of it in the stream, an attention call reads `*position` and requests the cache rows
- * below it (like weights: they must be complete in memory before the call is enqueued behind this library's kernels; rows
- * written by earlier steps are), and walks through its merge code once on what the scratch buffer holds, storing nothing
- * (instruction-cache warm-up).  Row `*position` and qkv are read after the wait.
+ * below it and suh_next (like weights: they must be complete in memory before the call is enqueued behind this library's
+ * kernels; rows written by earlier steps are).  Row `*position`, the tables and qkv are read after the wait.
  * The reference leaves attention to its engine; no counterpart there. */
 size_t exl3_attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max);
 exl3_status exl3_rope_append(void *qkv, int dtype, int rows, int q_heads, int kv_heads, int head_dim, const float *cos_table,

@@ -284,3 +284,47 @@ def test_rope_inside_the_attention_kernel_gives_the_bits_of_the_separate_launch(
     assert torch.equal(results[0][1], results[1][1])
     assert torch.equal(results[0][2], results[1][2])
     assert torch.isfinite(results[1][0].float()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,q_heads,kv_heads,t_max,pos", [
+    (1, 5, 1, 1, 0),                # one position, one CTA
+    (1, 8, 8, 200, 63),             # a tile's last position; clusters of two and of four CTAs, some without positions
+    (2, 10, 2, 300, 64),
+    (1, 8, 1, 1100, 1023),          # clusters of eight, one round of the warps and a second one of few
+    (1, 16, 4, 1100, 1030),
+    (3, 20, 10, 600, 599),          # clusters of four
+    (20, 8, 8, 450, 440),           # one CTA per head: the ring goes around once
+    (1, 5, 1, 4000, 3999),          # eight CTAs whose rings go around
+])
+def test_decode_attention_against_float64(dtype, rows, q_heads, kv_heads, t_max, pos):
+    """exl3_decode_attention against softmax(q k^T scale) v in float64 over positions 0..pos; rows behind `pos` hold infinities and must not
+    be seen.  A result is one rounding of fp32 sums of up to 4000 probabilities, whose relative errors (scores of 128 exact products,
+    __expf) are a few 1e-6: half a unit of the type, and 2e-5 of the largest value."""
+    import math
+    from trellis_serve_b200 import _lib
+    from trellis_serve_b200.kernels import linear as lin
+    lib = _lib.load()
+    _lib.init_device(0)
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(pos + q_heads)
+    qkv = torch.randn((rows, (q_heads + 2 * kv_heads) * 128), device=DEV, generator=gen).to(dtype)
+    cache = torch.randn((2, rows, kv_heads, t_max, 128), device=DEV, generator=gen).to(dtype)
+    cache[:, :, :, pos + 1:] = float("inf")
+    position = torch.tensor([pos], dtype=torch.int32, device=DEV)
+    scratch = torch.zeros(int(lib.exl3_attention_scratch_bytes(rows, q_heads, kv_heads, t_max)), dtype=torch.uint8, device=DEV)
+    out = torch.empty((rows, q_heads * 128), dtype=dtype, device=DEV)
+    p, scale = lin._ptr, 1.0 / math.sqrt(128)
+    for _ in range(2):
+        first = out.clone()
+        _lib.check(lib.exl3_decode_attention(p(qkv), lin._dtype_code(qkv), rows, q_heads, kv_heads, 128, p(cache[0]), p(cache[1]), t_max, p(position),
+                                             scale, p(scratch), scratch.numel(), p(out), None, 0, None, 0, lin._stream(torch.device(DEV))),
+                   "exl3_decode_attention")
+    torch.cuda.synchronize()
+    assert int(scratch[:4].view(torch.int32)) == 0
+    assert torch.equal(first, out)
+    q = qkv[:, :q_heads * 128].double().view(rows, kv_heads, q_heads // kv_heads, 128)
+    k, v = cache[0, :, :, :pos + 1].double(), cache[1, :, :, :pos + 1].double()
+    want = (torch.softmax(q @ k.transpose(-1, -2) * scale, dim=-1) @ v).view(rows, q_heads * 128)
+    half_ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert bool(((out.double() - want).abs() <= want.abs() * half_ulp + 2e-5 * want.abs().max()).all())

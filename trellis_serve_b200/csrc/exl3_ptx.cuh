@@ -100,6 +100,21 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta)
                  : "memory");
 }
 
+// Floats at the same shared-memory offset in CTA `cta` of the cluster.
+__device__ __forceinline__ float ld_shared_cluster_f32(const float* p, uint32_t cta)
+{
+    float v;
+    asm volatile("{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %1, %2;\n ld.shared::cluster.f32 %0, [ra];\n}" : "=f"(v) : "r"(smem_addr(p)), "r"(cta) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_shared_cluster_f32x4(const float* p, uint32_t cta)
+{
+    float4 v;
+    asm volatile("{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %4, %5;\n ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_addr(p)), "r"(cta) : "memory");
+    return v;
+}
+
 // The word at the same shared-memory offset in CTA `cta` of the cluster.
 __device__ __forceinline__ int ld_shared_cluster_s32(const int* p, uint32_t cta)
 {

@@ -53,14 +53,15 @@ __device__ __forceinline__ void load_act4(const void* p, long long i, bool bf16,
     }
 }
 
+// A lane's four signs of a 128-column block.
+__device__ __forceinline__ uint2 lane_signs(const __half* suh_blk, int lane) { return *reinterpret_cast<const uint2*>(suh_blk + 4 * lane); }
+
 // One warp, one (shard, row, 128 block): a[e] are activation values already rounded to the activation type.  They are
 // converted to fp16 as the rotation kernel does, scaled by suh, rotated and stored as fragments.
 // mode 1: split (every value twice), mode 2: paired; layouts of had_in_kernel.
-__device__ __forceinline__ void rotate_store(const float (&a)[4], const __half* suh_blk, uint32_t* xf, int mode, int s, int kts, int rows,
-                                             int row, int kg, int lane)
+__device__ __forceinline__ void rotate_store(const float (&a)[4], uint2 sw, uint32_t* xf, int mode, int s, int kts, int rows, int row, int kg, int lane)
 {
     float v[4];
-    const uint2 sw = *reinterpret_cast<const uint2*>(suh_blk + 4 * lane);
     const __half2 s01 = *reinterpret_cast<const __half2*>(&sw.x), s23 = *reinterpret_cast<const __half2*>(&sw.y);
     v[0] = __half2float(__float2half_rn(a[0])) * __low2float(s01);
     v[1] = __half2float(__float2half_rn(a[1])) * __high2float(s01);
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(STEP_THREADS) rmsnorm_rotate_kernel(const void
 #pragma unroll
             for (int e = 0; e < 4; e++) a[e] = round_act(h[j][e] * rstd * wv[j][e], b);
             if (normed) store_act4(normed, i0, a, b);
-            for (int s = 0; s < shards; s++) rotate_store(a, suh + (long long)s * k + kg * 128, xf, mode, s, k >> 4, rows, row, kg, lane);
+            for (int s = 0; s < shards; s++) rotate_store(a, lane_signs(suh + (long long)s * k + kg * 128, lane), xf, mode, s, k >> 4, rows, row, kg, lane);
         }
     }
 }
@@ -167,7 +168,7 @@ __global__ void silu_mul_rotate_kernel(const void* __restrict__ gu, int bf16, co
 #pragma unroll
     for (int e = 0; e < 4; e++) a[e] = round_act(gv[e] / (1.0f + __expf(-gv[e])) * uv[e], b);
     if (act) store_act4(act, (long long)row * inter + kg * 128 + 4 * lane, a, b);
-    rotate_store(a, suh + kg * 128, xf, mode, 0, inter >> 4, rows, row, kg, lane);
+    rotate_store(a, lane_signs(suh + kg * 128, lane), xf, mode, 0, inter >> 4, rows, row, kg, lane);
 }
 
 // z = x (+ res_in, rounded to the activation type) -> res_out, and the sums of squares of z per (row, 128 columns) -> ssq.
@@ -236,9 +237,11 @@ namespace exl3 {
 
 constexpr int ATT_D = 128;
 constexpr int ATT_MAX_GROUP = 8;          // query heads per KV head
-constexpr int ATT_WARPS = 4;
-constexpr int ATT_CHUNK = ATT_WARPS * 32; // cache positions per CTA
-constexpr int ATT_PART = ATT_D + 4;       // floats of one partial result: 128 weighted sums, maximum, normaliser (16-byte rows)
+constexpr int ATT_WARPS = 16;
+constexpr int ATT_TILE = 8;               // cache positions that a warp takes at a time: columns of an m16n8k16 MMA
+constexpr int ATT_STAGE = ATT_WARPS * ATT_TILE;          // cache positions of a stage of the ring
+constexpr int ATT_MAX_STAGES = 3, ATT_MAX_CLUSTER = 8;
+constexpr int ATT_CHUNK = 128, ATT_PART = ATT_D + 4;     // what a call's scratch is sized by: positions and floats of a partial result
 
 // One thread per (row, head, pair i < 64): x1' = x1 cos - x2 sin, x2' = x2 cos + x1 sin with x1 = x[i], x2 = x[i + 64]
 // (the "rotate half" convention).  Query heads are rotated in place in qkv; key heads are rotated into the cache slot
@@ -295,392 +298,347 @@ extern "C" int exl3_debug_att_timeline(unsigned long long* host_out) { return (i
 #define ATT_STAMP(i) do { } while (0)
 #endif
 
-// One warp, one (row, query head): lane l merges columns 4l..4l+3 of every partial of the head (fixed order: the same bits
-// every time), writes the output and -- a head is exactly one 128-wide rotation block of the o projection's input --
-// optionally the rotated fragments of that block for the linear that follows (suh != null).  The partials were written by
-// other CTAs of the same launch, so they are read past the L1 cache.
-__device__ __forceinline__ void attention_merge_head(const float* base, long long stride, int parts, int rows, int q_heads, int row, int qh,
-                                                     int lane, void* out, bool bf16, const __half* suh, uint32_t* xf, int mode)
+// Dynamic shared memory of a CTA: the ring, then what the warps exchange.
+constexpr uint32_t ATT_ROW = ATT_D * 2, ATT_STAGE_BYTES = 2 * ATT_STAGE * ATT_ROW;      // a stage's keys, then its values
+struct AttShared {
+    float p[ATT_WARPS][ATT_TILE][ATT_MAX_GROUP + 4];     // a warp's probabilities (rows of 48 bytes: the stores of a warp meet all banks)
+    float keep[ATT_WARPS][ATT_MAX_GROUP];                // factor of what earlier tiles added
+    float m[ATT_WARPS][ATT_MAX_GROUP], l[ATT_WARPS][ATT_MAX_GROUP];
+    float sum[ATT_MAX_GROUP][ATT_D];                     // the CTA's result: weighted sums, maxima and normalisers per head
+    float max[ATT_MAX_GROUP], den[ATT_MAX_GROUP];
+    uint16_t q[ATT_MAX_GROUP][ATT_D + 8];                // queries; rows 16 bytes apart in the banks
+    uint16_t row[2][ATT_D];                              // key and value of position `pos`
+    uint64_t full[ATT_MAX_STAGES], empty[ATT_MAX_STAGES];
+};
+
+template <bool BF16>
+__device__ __forceinline__ void att_mma(float (&c)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1)
 {
-    // Sixteen partials per round of loads (one round up to 2048 cache positions), added in split order under a running
-    // maximum.
-    float mx = -INFINITY, num[4] = {0.f, 0.f, 0.f, 0.f}, den = 0.f;
-    for (int s0 = 0; s0 < parts; s0 += 16) {
-        float4 a[16];
-        float ms[16], ls[16];
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const bool in = s0 + u < parts;
-            const float* ps = base + (long long)(in ? s0 + u : s0) * stride;
-            a[u] = __ldcg(reinterpret_cast<const float4*>(ps + 4 * lane));
-            ms[u] = in ? __ldcg(ps + ATT_D) : -INFINITY;
-            ls[u] = __ldcg(ps + ATT_D + 1);
-        }
-        float bm = mx;
-#pragma unroll
-        for (int u = 0; u < 16; u++) bm = fmaxf(bm, ms[u]);
-        const float keep = mx == -INFINITY ? 0.f : __expf(mx - bm);   // rescale what earlier rounds added
-        mx = bm;
-        den *= keep;
-#pragma unroll
-        for (int e = 0; e < 4; e++) num[e] *= keep;
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const float w = ms[u] == -INFINITY ? 0.f : __expf(ms[u] - mx);
-            num[0] += w * a[u].x;
-            num[1] += w * a[u].y;
-            num[2] += w * a[u].z;
-            num[3] += w * a[u].w;
-            den += w * ls[u];
-        }
-    }
-    float y[4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) y[e] = round_act(num[e] / den, bf16);
-    if (out) store_act4(out, ((long long)row * q_heads + qh) * ATT_D + 4 * lane, y, bf16);
-    if (suh) rotate_store(y, suh + qh * ATT_D, xf, mode, 0, (q_heads * ATT_D) >> 4, rows, row, qh, lane);
+    const uint32_t zero = 0;                             // rows 8 .. 15 of A
+    if constexpr (BF16)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(zero), "r"(a2), "r"(b0), "r"(b1));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %5}, {%7, %8}, {%0, %1, %2, %3};"
+                     : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(zero), "r"(a2), "r"(b0), "r"(b1));
 }
 
-// The merge of all splits of one (row, KV head) by a whole CTA (ATT_WARPS warps).  `dry`: same instructions, no stores -- run
-// once before the wait for the kernel ahead, while the CTA has nothing else to do, so that the real pass at the very end of
-// the launch finds its code in the instruction cache.
-template <int G>
-static __device__ __noinline__ void attention_merge_cta(const float* part, float (*red)[G][ATT_PART], int row, int kvh, int kv_heads, int q_heads,
-                                                        int splits, int rows, void* y_out, bool b, const __half* suh, uint32_t* xf, int mode,
-                                                        bool dry)
+// Two 16-bit activations <-> floats.
+template <bool BF16>
+__device__ __forceinline__ float2 att_unpack(uint32_t w)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float* base = part + ((long long)row * kv_heads + kvh) * splits * (G * ATT_PART);
-    const long long stride = (long long)G * ATT_PART;
-    if (splits > 32) {                                            // more than 4096 cache positions: one warp per head, split after split
-        if (!dry)
-            for (int g = warp; g < G; g += ATT_WARPS)
-                attention_merge_head(base + g * ATT_PART, stride, splits, rows, q_heads, row, kvh * G + g, lane, y_out, b, suh, xf, mode);
-        return;
-    }
-    // Up to 32 splits: the whole CTA merges all G heads together, in three short phases with one round of loads each, so the
-    // tail of the launch is a few dependent memory round trips instead of one per head and warp.  Every sum has a fixed order.
-    __shared__ float sm_ms[ATT_MAX_GROUP * 32], sm_ls[ATT_MAX_GROUP * 32], sm_w[ATT_MAX_GROUP * 32];
-    // (1) maxima and normalisers of every (head, split)
-    for (int i = threadIdx.x; i < G * splits; i += ATT_WARPS * 32) {
-        const int g = i / splits, sp = i - g * splits;
-        const float* ps = base + sp * stride + g * ATT_PART;
-        sm_ms[g * 32 + sp] = __ldcg(ps + ATT_D);
-        sm_ls[g * 32 + sp] = __ldcg(ps + ATT_D + 1);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < G * splits; i += ATT_WARPS * 32) {
-        const int g = i / splits, sp = i - g * splits;
-        float mx = -INFINITY;
-#pragma unroll 1
-        for (int t2 = 0; t2 < splits; t2++) mx = fmaxf(mx, sm_ms[g * 32 + t2]);
-        const float ms = sm_ms[g * 32 + sp];
-        sm_w[g * 32 + sp] = ms == -INFINITY ? 0.f : __expf(ms - mx);
-    }
-    __syncthreads();
-    // (2) warp w adds the splits w, w + 4, ... of every head
-    constexpr int JB = G <= 5 ? 5 : (G <= 6 ? 4 : 3);            // splits in flight per warp: JB x G 16-byte loads per lane
-    float sum[G][4];
-#pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) sum[g][e] = 0.f;
-    const int per_warp = (splits + ATT_WARPS - 1) / ATT_WARPS;
-#pragma unroll 1
-    for (int j0 = 0; j0 < per_warp; j0 += JB) {
-        float4 a[JB][G];
-#pragma unroll
-        for (int j = 0; j < JB; j++) {
-            const int sp = warp + ATT_WARPS * (j0 + j);
-#pragma unroll
-            for (int g = 0; g < G; g++)
-                a[j][g] = sp < splits ? __ldcg(reinterpret_cast<const float4*>(base + sp * stride + g * ATT_PART + 4 * lane)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < JB; j++) {
-            const int sp = warp + ATT_WARPS * (j0 + j);
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                const float w = sp < splits ? sm_w[g * 32 + sp] : 0.f;
-                sum[g][0] += w * a[j][g].x;
-                sum[g][1] += w * a[j][g].y;
-                sum[g][2] += w * a[j][g].z;
-                sum[g][3] += w * a[j][g].w;
-            }
-        }
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++) *reinterpret_cast<float4*>(&red[warp][g][4 * lane]) = make_float4(sum[g][0], sum[g][1], sum[g][2], sum[g][3]);
-    __syncthreads();
-    // (3) one warp per head: the warps' sums in warp order, the normaliser, the output and the next linear's fragments
-    for (int g = warp; g < G; g += ATT_WARPS) {
-        float num[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int w = 0; w < ATT_WARPS; w++) {
-            const float4 v = *reinterpret_cast<const float4*>(&red[w][g][4 * lane]);
-            num[0] += v.x;
-            num[1] += v.y;
-            num[2] += v.z;
-            num[3] += v.w;
-        }
-        float den = lane < splits ? sm_w[g * 32 + lane] * sm_ls[g * 32 + lane] : 0.f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);
-        const int qh = kvh * G + g;
-        float y[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) y[e] = round_act(num[e] / den, b);
-        if (y_out && !dry) store_act4(y_out, ((long long)row * q_heads + qh) * ATT_D + 4 * lane, y, b);
-        if (suh && !dry) rotate_store(y, suh + qh * ATT_D, xf, mode, 0, (q_heads * ATT_D) >> 4, rows, row, qh, lane);
-    }
+    if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+    else return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <bool BF16>
+__device__ __forceinline__ uint16_t att_round(float v)
+{
+    if constexpr (BF16) return __bfloat16_as_ushort(__float2bfloat16_rn(v));
+    else return __half_as_ushort(__float2half_rn(v));
 }
 
-// Split-KV decode attention.  grid = (splits, kv_heads, rows); a CTA attends positions [split * ATT_CHUNK ...) of one KV
-// head for its G query heads: every lane owns ONE position (reads its key row, G dot products against the queries held in
-// shared memory, no shuffles), the warp then walks its 32 positions for the values (each lane four of the 128 columns).
-// Partial results (running maximum, normaliser, G x 128 weighted sums per split) go to scratch; the last CTA of a (row, KV
-// head) to arrive merges them.
+// Decode attention of one new token per row.  grid = (CTAs of a cluster, kv_heads, rows): the CTAs of a cluster share the positions of one
+// (row, KV head) and its G query heads, evenly and contiguously in tiles of eight.
+//
+//   * scores by m16n8k16 MMAs: A = the query heads (rows G .. 15 are zero), B = eight keys.  Both are 16-bit values as stored, so the
+//     products are exact and the sums fp32; the order of the 128 columns inside the MMAs is the one in which a lane reads 32 consecutive
+//     bytes of a key;
+//   * probabilities, normalisers and weighted sums in fp32: a lane owns four of the 128 columns and walks the warp's eight values, the
+//     probabilities come from shared memory as broadcasts (once each: a 16-byte broadcast takes four cycles of the return path);
+//   * every warp keeps its own running maximum; the warps of a CTA are merged in warp order, the CTAs of a cluster in rank order over
+//     distributed shared memory: the same bits every time.  The output of a head -- one rotation block of the o projection's input -- is
+//     finished by one warp, which also writes the rotated fragments of the linear that follows (suh != null).
+//
+// Latency bounds it: 2048 positions of 8 KV heads are 8.4 MB, 1.3 us of memory time that passes before the wait for the kernel ahead.  Of
+// the 8 us between the end of q|k|v and the start of o (27B shape, 2048 positions, one row) 0.9 are the wait, 0.6 queries and new row, 3.3
+// scores and values (17 positions per warp), 0.9 the merge in the CTA, 0.6 the cluster barrier, 1.2 the merge of the cluster and o's
+// rotation, 0.8 o's wait.  With one CTA of four warps per 128 positions, a lane per key and a merge through memory by the last CTA to
+// count itself in they were 15.6 (scores 4.4, values 2.3, hand-over 2.4, merge 4.6): 8 layers 960 -> 901 us, at 4096 positions 1049 -> 925,
+// at 4096 positions and 8 rows 1662 -> 1206.  Running the code once ahead of the wait, for the instruction cache, gained nothing; all of a
+// warp's tiles in one pass (scores of three stages, then one maximum) 0.3 % at one row, and lost 9 % at 8 rows and 4096 positions.
 // With cos_t / sin_t the kernel also does what rope_append_kernel does, with the same roundings: the queries are rotated as
 // they are loaded (qkv itself is left as it is), and the warp that owns cache position `pos` rotates the new key into the
-// cache and copies the new value there before it reads them back like any other position.
-template <int G>
-__global__ void __launch_bounds__(ATT_WARPS * 32) decode_attention_kernel(const void* __restrict__ qkv, int bf16, int q_heads, int kv_heads,
-                                                                           void* k_cache, void* v_cache, int t_max,
-                                                                           const int* __restrict__ pos_ptr, float scale,
-                                                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                                           float* part, int* counters, int* err, int rows, void* __restrict__ y_out,
-                                                                           const __half* __restrict__ suh, uint32_t* __restrict__ xf, int mode)
+// cache and copies the new value there before it reads them like any other position.
+template <int G, bool BF16>
+__global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(const void* __restrict__ qkv, int q_heads, int kv_heads, void* k_cache, void* v_cache,
+                                                                              int t_max, const int* __restrict__ pos_ptr, float scale,
+                                                                              const float* __restrict__ cos_t, const float* __restrict__ sin_t, int* err,
+                                                                              int rows, void* __restrict__ y_out, const __half* __restrict__ suh,
+                                                                              uint32_t* __restrict__ xf, int mode, int stages)
 {
-    // Dynamic shared memory: the CTA's chunk of keys and of values (ATT_CHUNK rows of 256 bytes each), brought in by two bulk
-    // copies.  The loops over them are short and rolled: a kernel whose every instruction runs once is bound by instruction
-    // fetch, not by arithmetic.
     extern __shared__ __align__(128) unsigned char att_smem[];
-    unsigned char* ks = att_smem;
-    unsigned char* vs = att_smem + ATT_CHUNK * ATT_D * 2;
-    // queries, chunk-major: qs[g][half][chunk of 8 columns][4] so that lanes reading different chunks hit different banks
-    __shared__ __align__(16) float qs[G][2][16][4];
-    __shared__ __align__(16) float red[ATT_WARPS][G][ATT_PART];
-    __shared__ __align__(8) uint64_t bar;
+    AttShared& sh = *reinterpret_cast<AttShared*>(att_smem + (size_t)stages * ATT_STAGE_BYTES);
     ATT_STAMP(0);
     ptx::grid_launch_dependents();
-    const int split = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pos = *pos_ptr;
-    const int T = pos + 1;                                        // valid cache positions
+    const int rank = blockIdx.x, ctas = gridDim.x, kvh = blockIdx.y, row = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q4 = lane & 3, n8 = lane >> 2;
+    const int pos = *pos_ptr, T = pos + 1;                        // valid cache positions
     const int heads = q_heads + 2 * kv_heads;
-    const bool b = bf16 != 0;
-    const int chunk0 = split * ATT_CHUNK;
-    const int t0 = chunk0 + warp * 32;
-    const int t = t0 + lane;
-    const long long rowbase = (((long long)row * kv_heads + kvh) * t_max) * ATT_D;
+    const int all_tiles = (T + ATT_TILE - 1) / ATT_TILE, share = (all_tiles + ctas - 1) / ctas, tile0 = rank * share;
+    const int tiles = all_tiles - tile0 < 0 ? 0 : all_tiles - tile0 < share ? all_tiles - tile0 : share;
+    const int fills = (tiles + ATT_WARPS - 1) / ATT_WARPS;
+    const long long rowbase = ((long long)row * kv_heads + kvh) * t_max;
     // Cache rows below `pos` were written by earlier steps: like weights they are constants of this launch and are requested
     // before the wait for the kernel ahead, so their trip from memory overlaps that kernel's tail; row `pos` itself comes from
     // the kernel ahead or from this kernel's own append and is put in place after the wait.
-    int old_rows = pos - chunk0;
-    old_rows = old_rows < 0 ? 0 : (old_rows > ATT_CHUNK ? ATT_CHUNK : old_rows);
-    if (threadIdx.x == 0) {
-        ptx::mbar_init(&bar, 1);
-        ptx::mbar_fence_init();
-        if (old_rows > 0) {
-            const uint32_t bytes = (uint32_t)old_rows * ATT_D * 2;
-            ptx::mbar_arrive_expect_tx(&bar, 2 * bytes);
-            ptx::bulk_g2s(ks, reinterpret_cast<const unsigned char*>(k_cache) + (rowbase + (long long)chunk0 * ATT_D) * 2, bytes, &bar);
-            ptx::bulk_g2s(vs, reinterpret_cast<const unsigned char*>(v_cache) + (rowbase + (long long)chunk0 * ATT_D) * 2, bytes, &bar);
+    auto fetch = [&](int j, int slot) {
+        const int first = (tile0 + j * ATT_WARPS) * ATT_TILE, left = (tiles - j * ATT_WARPS) * ATT_TILE;
+        int n = left < ATT_STAGE ? left : ATT_STAGE;
+        if (n > pos - first) n = pos - first;
+        if (n <= 0) {
+            ptx::mbar_arrive(&sh.full[slot]);
+            return;
         }
+        unsigned char* ks = att_smem + (size_t)slot * ATT_STAGE_BYTES;
+        const long long at = (rowbase + first) * ATT_ROW;
+        ptx::mbar_arrive_expect_tx(&sh.full[slot], 2u * (uint32_t)n * ATT_ROW);
+        ptx::bulk_g2s(ks, reinterpret_cast<const unsigned char*>(k_cache) + at, (uint32_t)n * ATT_ROW, &sh.full[slot]);
+        ptx::bulk_g2s(ks + ATT_STAGE * ATT_ROW, reinterpret_cast<const unsigned char*>(v_cache) + at, (uint32_t)n * ATT_ROW, &sh.full[slot]);
+    };
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < stages; i++) {
+            ptx::mbar_init(&sh.full[i], 1);
+            ptx::mbar_init(&sh.empty[i], ATT_WARPS);
+        }
+        ptx::mbar_fence_init();
+        for (int j = 0; j < stages && j < fills; j++) fetch(j, j);
     }
-    // Nothing else to do until the kernel ahead has finished: walk through the merge code once without storing anything, so
-    // that the CTA that ends up merging runs it from the instruction cache (it looks at last step's partials).
-    attention_merge_cta<G>(part, red, row, kvh, kv_heads, q_heads, gridDim.x, rows, y_out, b, suh, xf, mode, true);
+    const bool owner = tiles > 0 && pos / ATT_TILE >= tile0 && pos / ATT_TILE < tile0 + tiles;       // of position `pos`
+    const int with = tiles < ATT_WARPS ? tiles : ATT_WARPS;       // warps that have positions
+    const int mine = rank + ctas * warp;                          // heads are dealt to the CTAs, one warp each, to be finished
+    uint2 signs = make_uint2(0u, 0u);                             // constants: requested before the wait
+    if (suh && mine < G) signs = lane_signs(suh + (kvh * G + mine) * ATT_D, lane);
+    bool failed = false;
+    __syncthreads();
     ptx::grid_dependency_wait();
     ATT_STAMP(1);
-    // queries (rotated here when the tables are given), scaled
-    for (int e = threadIdx.x; e < G * (ATT_D / 2); e += ATT_WARPS * 32) {
-        const int g = e / (ATT_D / 2), i = e % (ATT_D / 2);
-        const long long at = ((long long)row * heads + kvh * G + g) * ATT_D;
-        const float x1 = to_f32(qkv, at + i, b), x2 = to_f32(qkv, at + i + 64, b);
-        float y1 = x1, y2 = x2;
+    // Queries, and the new row: a thread per pair (i, i + 64) of a head.
+    {
+        const int i = threadIdx.x & 63;
+        const uint16_t* src = reinterpret_cast<const uint16_t*>(qkv) + (long long)row * heads * ATT_D;
+        float c = 1.f, sn = 0.f;
         if (cos_t) {
-            const float c = cos_t[(long long)pos * 64 + i], sn = sin_t[(long long)pos * 64 + i];
-            y1 = round_act(x1 * c - x2 * sn, b);
-            y2 = round_act(x2 * c + x1 * sn, b);
+            c = cos_t[(long long)pos * 64 + i];
+            sn = sin_t[(long long)pos * 64 + i];
         }
-        qs[g][(i >> 2) & 1][i >> 3][i & 3] = y1 * scale;
-        qs[g][((i + 64) >> 2) & 1][(i + 64) >> 3][i & 3] = y2 * scale;
-    }
-    // the new row: rotated key and value into the cache (with the tables) and, either way, into this CTA's chunk
-    if (pos >= t0 && pos < t0 + 32) {                             // warp-uniform: the warp that owns position `pos`
-        const long long cat = rowbase + (long long)pos * ATT_D;
-        const int r = pos - chunk0;
-        if (cos_t) {
-            const long long kat = ((long long)row * heads + q_heads + kvh) * ATT_D, vat = kat + (long long)kv_heads * ATT_D;
-            for (int i = lane; i < 64; i += 32) {
-                const float x1 = to_f32(qkv, kat + i, b), x2 = to_f32(qkv, kat + i + 64, b);
-                const float c = cos_t[(long long)pos * 64 + i], sn = sin_t[(long long)pos * 64 + i];
-                const float y1 = x1 * c - x2 * sn, y2 = x2 * c + x1 * sn;
-                uint16_t h1, h2;
-                if (b) {
-                    h1 = __bfloat16_as_ushort(__float2bfloat16_rn(y1));
-                    h2 = __bfloat16_as_ushort(__float2bfloat16_rn(y2));
-                } else {
-                    h1 = __half_as_ushort(__float2half_rn(y1));
-                    h2 = __half_as_ushort(__float2half_rn(y2));
-                }
-                reinterpret_cast<uint16_t*>(k_cache)[cat + i] = h1;
-                reinterpret_cast<uint16_t*>(k_cache)[cat + i + 64] = h2;
-                reinterpret_cast<uint16_t*>(ks)[r * ATT_D + i] = h1;
-                reinterpret_cast<uint16_t*>(ks)[r * ATT_D + i + 64] = h2;
+        auto rotate = [&](uint32_t a, uint32_t b, uint16_t* to) {
+            if (cos_t) {
+                const float x1 = att_unpack<BF16>(a).x, x2 = att_unpack<BF16>(b).x;
+                to[i] = att_round<BF16>(x1 * c - x2 * sn);
+                to[i + 64] = att_round<BF16>(x2 * c + x1 * sn);
+            } else {
+                to[i] = (uint16_t)a;
+                to[i + 64] = (uint16_t)b;
             }
-            const uint2 vv = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(qkv) + vat * 2)[lane];
-            reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(v_cache) + cat * 2)[lane] = vv;
-            reinterpret_cast<uint2*>(vs + (size_t)r * ATT_D * 2)[lane] = vv;
-        } else {
-            reinterpret_cast<uint2*>(ks + (size_t)r * ATT_D * 2)[lane] = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(k_cache) + cat * 2)[lane];
-            reinterpret_cast<uint2*>(vs + (size_t)r * ATT_D * 2)[lane] = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(v_cache) + cat * 2)[lane];
+        };
+        const int g = threadIdx.x >> 6;                       // ATT_MAX_GROUP heads of 64 threads
+        const uint16_t* at = src + (kvh * G + (g < G ? g : 0)) * ATT_D;
+        const uint32_t a = at[i], b = at[i + 64];
+        if (g < 2 && owner) {                                 // the new key (rotated with the tables), the new value
+            const long long cat = (rowbase + pos) * ATT_D;
+            uint16_t* cache = reinterpret_cast<uint16_t*>(g == 0 ? k_cache : v_cache) + cat;
+            const uint16_t* kv = cos_t ? src + (q_heads + kvh + g * kv_heads) * ATT_D : cache;
+            const uint32_t ka = kv[i], kb = kv[i + 64];
+            if (g == 0) rotate(ka, kb, sh.row[0]);
+            else {
+                sh.row[1][i] = (uint16_t)ka;
+                sh.row[1][i + 64] = (uint16_t)kb;
+            }
+            if (cos_t) {
+                cache[i] = sh.row[g][i];
+                cache[i + 64] = sh.row[g][i + 64];
+            }
         }
+        rotate(g < G ? a : 0u, g < G ? b : 0u, sh.q[g]);
     }
     __syncthreads();
-    if (old_rows > 0 && !ptx::mbar_wait(&bar, 0) && lane == 0) atomicExch(err, 1);
-    const int splits = gridDim.x;
-    float* out = part + (((long long)row * kv_heads + kvh) * splits + split) * (G * ATT_PART);
-    // scores: lane = position; its key row in 16 chunks of 8 columns, taken in an order rotated by the lane number so that
-    // the lanes of a quarter warp read different banks (rows are 256 bytes apart); the query chunk follows the same order
-    float sc[G];
+    // As A fragments: lane = head n8, columns 64 i + 16 q4 .. + 15 as eight pairs.
+    uint32_t qa[2][8];
 #pragma unroll
-    for (int g = 0; g < G; g++) sc[g] = 0.f;
-    if (t < T) {
-        const uint32_t krow = ptx::smem_addr(ks) + (uint32_t)(warp * 32 + lane) * (ATT_D * 2);
-#pragma unroll 2
-        for (int j = 0; j < 16; j++) {
-            const int c = (j + lane) & 15;
-            const uint4 w = ptx::lds128(krow + c * 16);
-            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-            float kf[8];
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-            for (int h2 = 0; h2 < 4; h2++) {
-                if (b) {
-                    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&ww[h2]);
-                    kf[2 * h2] = __low2float(v);
-                    kf[2 * h2 + 1] = __high2float(v);
-                } else {
-                    const __half2 v = *reinterpret_cast<const __half2*>(&ww[h2]);
-                    kf[2 * h2] = __low2float(v);
-                    kf[2 * h2 + 1] = __high2float(v);
+        for (int j = 0; j < 2; j++) {
+            const uint4 w = ptx::lds128(ptx::smem_addr(&sh.q[n8][64 * i + 16 * q4 + 8 * j]));
+            qa[i][4 * j] = w.x;
+            qa[i][4 * j + 1] = w.y;
+            qa[i][4 * j + 2] = w.z;
+            qa[i][4 * j + 3] = w.w;
+        }
+    ATT_STAMP(2);
+    float m = -INFINITY, l = 0.f;                             // of head n8; l: this lane's positions only
+    float acc[G][4] = {};                                         // columns 4 lane .. + 3 of every head
+    int slot = 0;
+    uint32_t parity = 0;
+#pragma unroll 1
+    for (int j = 0; j < fills; j++) {
+        const int tile = j * ATT_WARPS + warp;
+        if (tile < tiles) {
+            const int p0 = (tile0 + tile) * ATT_TILE, n = T - p0 < ATT_TILE ? T - p0 : ATT_TILE;      // positions that exist
+            unsigned char* ks = att_smem + (size_t)slot * ATT_STAGE_BYTES + warp * (ATT_TILE * ATT_ROW);
+            unsigned char* vs = ks + ATT_STAGE * ATT_ROW;
+            if (pos - p0 < ATT_TILE) {                            // this warp owns position `pos`
+                reinterpret_cast<uint2*>(ks + (pos - p0) * ATT_ROW)[lane] = reinterpret_cast<const uint2*>(sh.row[0])[lane];
+                reinterpret_cast<uint2*>(vs + (pos - p0) * ATT_ROW)[lane] = reinterpret_cast<const uint2*>(sh.row[1])[lane];
+                __syncwarp();
+            }
+            if (!failed && !ptx::mbar_wait(&sh.full[slot], parity)) failed = true;
+            // Scores.  Rows of keys are 256 bytes apart: lanes of odd rows read the halves of their 32 bytes in the other order, so that
+            // the eight lanes of a quarter warp meet different banks.
+            float c[2][4] = {};
+            const uint32_t krow = ptx::smem_addr(ks) + n8 * ATT_ROW + q4 * 32, odd = n8 & 1;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const uint4 u = ptx::lds128(krow + i * 128 + odd * 16), v = ptx::lds128(krow + i * 128 + (odd ^ 1) * 16);
+                const uint4 lo = odd ? v : u, hi = odd ? u : v;
+                att_mma<BF16>(c[i], qa[i][0], qa[i][1], lo.x, lo.y);
+                att_mma<BF16>(c[i], qa[i][2], qa[i][3], lo.z, lo.w);
+                att_mma<BF16>(c[i], qa[i][4], qa[i][5], hi.x, hi.y);
+                att_mma<BF16>(c[i], qa[i][6], qa[i][7], hi.z, hi.w);
+            }
+            // This lane: head n8, positions 2 q4 and 2 q4 + 1 of the tile.
+            const float s0 = 2 * q4 < n ? (c[0][0] + c[1][0]) * scale : -INFINITY, s1 = 2 * q4 + 1 < n ? (c[0][1] + c[1][1]) * scale : -INFINITY;
+            float mx = fmaxf(s0, s1);
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+            mx = fmaxf(m, mx);
+            const float keep = m == -INFINITY ? 0.f : __expf(m - mx);
+            const float e0 = 2 * q4 < n ? __expf(s0 - mx) : 0.f, e1 = 2 * q4 + 1 < n ? __expf(s1 - mx) : 0.f;
+            m = mx;
+            l = l * keep + (e0 + e1);
+            sh.p[warp][2 * q4][n8] = e0;
+            sh.p[warp][2 * q4 + 1][n8] = e1;
+            if (q4 == 0) sh.keep[warp][n8] = keep;
+            __syncwarp();
+            if (j > 0) {
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const float k = sh.keep[warp][g];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) acc[g][e] *= k;
                 }
             }
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                const float4 qa = *reinterpret_cast<const float4*>(&qs[g][0][c][0]), qb = *reinterpret_cast<const float4*>(&qs[g][1][c][0]);
-                sc[g] += kf[0] * qa.x + kf[1] * qa.y + kf[2] * qa.z + kf[3] * qa.w + kf[4] * qb.x + kf[5] * qb.y + kf[6] * qb.z + kf[7] * qb.w;
-            }
-        }
-    }
-    ATT_STAMP(2);
-    float m[G], l[G], p[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        float v = t < T ? sc[g] : -INFINITY;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-        m[g] = v;
-        p[g] = (t < T) ? __expf(sc[g] - v) : 0.f;
-        float s = p[g];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-        l[g] = s;
-    }
-    // values: the warp walks its positions, each lane four of the 128 columns
-    float acc[G][4];
-#pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) acc[g][e] = 0.f;
-    const int n = T - t0 < 32 ? (T - t0 < 0 ? 0 : T - t0) : 32;   // warp-uniform: positions of this warp that exist
-    const uint32_t vrow = ptx::smem_addr(vs) + (uint32_t)(warp * 32) * (ATT_D * 2) + lane * 8;
+            const uint32_t vrow = ptx::smem_addr(vs) + lane * 8;
 #pragma unroll 4
-    for (int u = 0; u < n; u++) {
-        const uint2 w = ptx::lds64(vrow + u * (ATT_D * 2));
-        float v[4];
-        if (b) {
-            const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&w.x), c = *reinterpret_cast<const __nv_bfloat162*>(&w.y);
-            v[0] = __low2float(a); v[1] = __high2float(a); v[2] = __low2float(c); v[3] = __high2float(c);
-        } else {
-            const __half2 a = *reinterpret_cast<const __half2*>(&w.x), c = *reinterpret_cast<const __half2*>(&w.y);
-            v[0] = __low2float(a); v[1] = __high2float(a); v[2] = __low2float(c); v[3] = __high2float(c);
-        }
+            for (int u = 0; u < n; u++) {
+                const uint2 w = ptx::lds64(vrow + u * ATT_ROW);
+                const float2 va = att_unpack<BF16>(w.x), vb = att_unpack<BF16>(w.y);
+                float e[ATT_MAX_GROUP];
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            const float pj = __shfl_sync(0xFFFFFFFFu, p[g], u);
+                for (int g = 0; g < G; g += 4) {
+                    if (G - g == 1) {
+                        e[g] = sh.p[warp][u][g];
+                    } else {
+                        const float4 f = *reinterpret_cast<const float4*>(&sh.p[warp][u][g]);
+                        e[g] = f.x;
+                        e[g + 1] = f.y;
+                        if (G - g > 2) {
+                            e[g + 2] = f.z;
+                            e[g + 3] = f.w;
+                        }
+                    }
+                }
 #pragma unroll
-            for (int e = 0; e < 4; e++) acc[g][e] += pj * v[e];
+                for (int g = 0; g < G; g++) {
+                    acc[g][0] += e[g] * va.x;
+                    acc[g][1] += e[g] * va.y;
+                    acc[g][2] += e[g] * vb.x;
+                    acc[g][3] += e[g] * vb.y;
+                }
+            }
+            __syncwarp();                                     // the next tile overwrites the probabilities
         }
+        if (j + stages < fills) {                     // the ring goes around: more positions than it holds
+            if (lane == 0) ptx::mbar_arrive(&sh.empty[slot]);
+            if (threadIdx.x == 0) {
+                if (!failed && !ptx::mbar_wait(&sh.empty[slot], parity)) failed = true;
+                fetch(j + stages, slot);
+            }
+            __syncwarp();
+        }
+        if (++slot == stages) {
+            slot = 0;
+            parity ^= 1;
+        }
+    }
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
+    l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
+    if (q4 == 0) {
+        sh.m[warp][n8] = m;
+        sh.l[warp][n8] = l;
     }
     ATT_STAMP(3);
-    __shared__ float wgt[G][ATT_WARPS];
-    __shared__ int last_s;
-    // The four warps' partial results are merged inside the CTA (fixed warp order), so one partial per split goes out.
+    __syncthreads();                                          // every copy has been waited for and read: the ring's first stage is free
+    float* red = reinterpret_cast<float*>(att_smem);              // [warp][G][128]
 #pragma unroll
-    for (int g = 0; g < G; g++) {
-        *reinterpret_cast<float4*>(&red[warp][g][4 * lane]) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+    for (int g = 0; g < G; g++)
+        *reinterpret_cast<float4*>(red + ((warp * G + g) * ATT_D + 4 * lane)) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+    __syncthreads();
+    // Weight of part `lane` (a warp of the CTA, a CTA of the cluster) from its maximum; returns the common maximum.
+    auto weigh = [&](float part_max, float part_den, float& weight, float& den) {
+        float mx = part_max;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        weight = part_max == -INFINITY ? 0.f : __expf(part_max - mx);
+        den = weight * part_den;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xFFFFFFFFu, den, o);
+        return mx;
+    };
+    if (warp < G) {
+        float weight, den;
+        const float mx = weigh(lane < with ? sh.m[lane][warp] : -INFINITY, lane < with ? sh.l[lane][warp] : 0.f, weight, den);
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int w = 0; w < with; w++) {
+            const float f = __shfl_sync(0xFFFFFFFFu, weight, w);
+            const float4 a = *reinterpret_cast<const float4*>(red + ((w * G + warp) * ATT_D + 4 * lane));
+            sum[0] += f * a.x;
+            sum[1] += f * a.y;
+            sum[2] += f * a.z;
+            sum[3] += f * a.w;
+        }
+        *reinterpret_cast<float4*>(&sh.sum[warp][4 * lane]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
         if (lane == 0) {
-            red[warp][g][ATT_D] = n > 0 ? m[g] : -INFINITY;
-            red[warp][g][ATT_D + 1] = n > 0 ? l[g] : 0.f;
+            sh.max[warp] = mx;
+            sh.den[warp] = den;
         }
     }
-    __syncthreads();
-    if (threadIdx.x < G) {
-        const int g = threadIdx.x;
-        float mx = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < ATT_WARPS; w++) mx = fmaxf(mx, red[w][g][ATT_D]);
-        float den = 0.f;
-#pragma unroll
-        for (int w = 0; w < ATT_WARPS; w++) {
-            const float mw = red[w][g][ATT_D];
-            const float f = mw == -INFINITY ? 0.f : __expf(mw - mx);
-            wgt[g][w] = f;
-            den += f * red[w][g][ATT_D + 1];
-        }
-        out[g * ATT_PART + ATT_D] = mx;
-        out[g * ATT_PART + ATT_D + 1] = den;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < G * (ATT_D / 4); e += ATT_WARPS * 32) {
-        const int g = e / (ATT_D / 4), c = (e % (ATT_D / 4)) * 4;
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < ATT_WARPS; w++) {
-            const float f = wgt[g][w];
-            const float4 a = *reinterpret_cast<const float4*>(&red[w][g][c]);
-            sum.x += f * a.x;
-            sum.y += f * a.y;
-            sum.z += f * a.z;
-            sum.w += f * a.w;
-        }
-        *reinterpret_cast<float4*>(out + g * ATT_PART + c) = sum;
-    }
-    // The CTA that is last to deliver its split for this (row, KV head) merges all of them: no second launch.  Its partial
-    // stores are fenced before the count, the others' are read after it.
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int* cnt = counters + row * kv_heads + kvh;
-        const int arrived = atomicAdd(cnt, 1);
-        last_s = arrived == splits - 1;
-        if (last_s) *cnt = 0;                                     // everyone has counted: zero again for the next launch
-    }
-    __syncthreads();
     ATT_STAMP(4);
-    if (!last_s) return;
-    __threadfence();
+    if (ctas > 1) ptx::cluster_sync_all();
+    else __syncthreads();
     ATT_STAMP(5);
-    attention_merge_cta<G>(part, red, row, kvh, kv_heads, q_heads, splits, rows, y_out, b, suh, xf, mode, false);
+    if (mine < G) {
+        float4 a[ATT_MAX_CLUSTER];
+#pragma unroll
+        for (int c = 0; c < ATT_MAX_CLUSTER; c++)
+            if (c < ctas) a[c] = ptx::ld_shared_cluster_f32x4(&sh.sum[mine][4 * lane], c);
+        float weight, den;
+        weigh(lane < ctas ? ptx::ld_shared_cluster_f32(&sh.max[mine], lane) : -INFINITY, lane < ctas ? ptx::ld_shared_cluster_f32(&sh.den[mine], lane) : 0.f, weight, den);
+        float num[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < ATT_MAX_CLUSTER; c++)
+            if (c < ctas) {
+                const float f = __shfl_sync(0xFFFFFFFFu, weight, c);
+                num[0] += f * a[c].x;
+                num[1] += f * a[c].y;
+                num[2] += f * a[c].z;
+                num[3] += f * a[c].w;
+            }
+        const int qh = kvh * G + mine;
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) y[e] = round_act(num[e] / den, BF16);
+        if (y_out) store_act4(y_out, ((long long)row * q_heads + qh) * ATT_D + 4 * lane, y, BF16);
+        if (suh) rotate_store(y, signs, xf, mode, 0, (q_heads * ATT_D) >> 4, rows, row, qh, lane);
+    }
     ATT_STAMP(7);
+    if (failed && lane == 0) atomicExch(err, 1);
+    if (ctas > 1) ptx::cluster_sync_all();                        // no CTA leaves while its shared memory is being read
 }
 
-// Scratch: an error word (set when the bounded wait for the cache copies gives up; exl3_device_error reads it), one arrival
-// counter per (row, KV head) -- zero before the first launch, left zero by every launch -- then the partials.
+// Scratch: an error word (set when the bounded wait for the cache copies gives up; exl3_device_error reads it).  Callers hold as much as a
+// merge through memory would take.
 constexpr size_t ATT_SCRATCH_HEADER = 256;
-constexpr size_t ATT_DYN_SMEM = 2 * (size_t)ATT_CHUNK * ATT_D * 2;
 static size_t attention_counter_bytes(int rows, int kv_heads) { return ((size_t)rows * kv_heads * sizeof(int) + 255) & ~(size_t)255; }
 
 size_t attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max)
@@ -690,14 +648,22 @@ size_t attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max)
     return ATT_SCRATCH_HEADER + attention_counter_bytes(rows, kv_heads) + (size_t)rows * kv_heads * splits * G * ATT_PART * sizeof(float);
 }
 
-// The kernels keep their cache chunk in dynamic shared memory beyond the default limit: opted in once per device.
+// The kernels keep their part of the cache in dynamic shared memory beyond the default limit: opted in once per device.
+template <int G>
+static int attention_opt_in()
+{
+    const int most = (int)(ATT_MAX_STAGES * ATT_STAGE_BYTES + sizeof(AttShared));
+    const int rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return rc != EXL3_OK ? rc : cuda_status(cudaFuncSetAttribute(decode_attention_kernel<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+}
+
 int attention_init_device()
 {
-    int rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_DYN_SMEM));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_DYN_SMEM));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_DYN_SMEM));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_DYN_SMEM));
-    if (rc == EXL3_OK) rc = cuda_status(cudaFuncSetAttribute(decode_attention_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATT_DYN_SMEM));
+    int rc = attention_opt_in<1>();
+    if (rc == EXL3_OK) rc = attention_opt_in<2>();
+    if (rc == EXL3_OK) rc = attention_opt_in<4>();
+    if (rc == EXL3_OK) rc = attention_opt_in<5>();
+    if (rc == EXL3_OK) rc = attention_opt_in<8>();
     return rc;
 }
 
@@ -715,13 +681,34 @@ static int launch_attention_g(const void* qkv, int bf16, int rows, int q_heads, 
                               const int* pos, float scale, const float* cos_t, const float* sin_t, float* part, void* out, const __half* suh,
                               uint32_t* xf, int mode, cudaStream_t st)
 {
-    const int splits = (t_max + ATT_CHUNK - 1) / ATT_CHUNK;
-    unsigned char* base = reinterpret_cast<unsigned char*>(part);
-    int* err = reinterpret_cast<int*>(base);
-    int* counters = reinterpret_cast<int*>(base + ATT_SCRATCH_HEADER);
-    float* partials = reinterpret_cast<float*>(base + ATT_SCRATCH_HEADER + attention_counter_bytes(rows, kv_heads));
-    return launch_chained(decode_attention_kernel<G>, dim3(splits, kv_heads, rows), dim3(ATT_WARPS * 32), ATT_DYN_SMEM, st, qkv, bf16, q_heads,
-                          kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, partials, counters, err, rows, out, suh, xf, mode);
+    const DeviceInfo* d = current_device_info();
+    if (!d) return EXL3_ERR_NOT_INITIALISED;
+    // CTAs that share a (row, KV head): as many as a portable cluster holds, while every one has 64 positions and more to look at and all
+    // CTAs of the launch fit on the chip together (a CTA with a full ring has an SM for itself).
+    const int tiles = (t_max + ATT_TILE - 1) / ATT_TILE;
+    int ctas = ATT_MAX_CLUSTER;
+    while (ctas > 1 && ((long long)rows * kv_heads * ctas > d->sm_count || tiles < 8 * ctas)) ctas /= 2;
+    const int share = (tiles + ctas - 1) / ctas;
+    int stages = (share + ATT_WARPS - 1) / ATT_WARPS;
+    if (stages > ATT_MAX_STAGES) stages = ATT_MAX_STAGES;
+    int* err = reinterpret_cast<int*>(part);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas, kv_heads, rows);
+    cfg.blockDim = dim3(ATT_WARPS * 32);
+    cfg.dynamicSmemBytes = stages * (size_t)ATT_STAGE_BYTES + sizeof(AttShared);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    auto* const kernel = bf16 ? decode_attention_kernel<G, true> : decode_attention_kernel<G, false>;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, qkv, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, rows, out, suh, xf, mode,
+                                          stages));
 }
 
 int launch_decode_attention(const void* qkv, int bf16, int rows, int q_heads, int kv_heads, void* k_cache, void* v_cache, int t_max,

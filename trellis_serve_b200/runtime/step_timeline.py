@@ -8,7 +8,7 @@ Build a second copy of the library with the stamps compiled in and point this mo
 
 In that build thread 0 of every CTA of the decode GEMV and of the attention kernel writes the time at a few points
 (kernel entry, dependency wait resolved, own input rotated or first streamed rows landed, first weights landed, loop end, kernel end;
-attention: scores, values, hand-over count, merge end).  The report gives, per linear of a layer, those points relative to the end of the GEMV
+attention: queries ready, positions done, CTA merged, cluster met, heads merged).  The report gives, per linear of a layer, those points relative to the end of the GEMV
 launch ahead of it (median over layers), i.e. what sits on the critical path between two linears.  The stamps cost a few
 stores per CTA; the normal build has none of this code.
 """
@@ -100,10 +100,11 @@ def main() -> None:
         def mx(pt):
             v = a[:, pt][a[:, pt] > 0]
             return (v.max() - base) if len(v) else float("nan")
-        res.append([a[:, 0].min() - base, a[:, 1].max() - base, np.median(a[:, 2]) - base, mx(2), np.median(a[:, 3]) - base, mx(3), mx(4), mx(5),
-                    mx(7), (nxt_o[0] - base) if nxt_o else float("nan")])
+        med = lambda pt: np.median(a[:, pt]) - base
+        res.append([a[:, 0].min() - base, med(0), mx(0), mx(1), med(2), mx(2), med(3), mx(3), mx(4), mx(5), mx(7), (nxt_o[0] - base) if nxt_o else float("nan")])
     if res:
-        hdr2 = ["entry.min", "wait.max", "scores.med", "scores.max", "values.med", "values.max", "count.max", "fence.max", "merge.end", "o.wait"]
+        hdr2 = ["entry.min", "entry.med", "entry.max", "wait.max", "queries.med", "queries.max", "tiles.med", "tiles.max", "cta.max", "cluster.max", "merge.end",
+                "o.wait"]
         r = np.median(np.array(res, dtype=np.float64), axis=0)
         print("attention, ns after the end of the q|k|v launch ahead (median over layers):")
         print("  " + "  ".join(f"{h}={v:.0f}" for h, v in zip(hdr2, r)))
