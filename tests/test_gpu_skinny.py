@@ -71,3 +71,32 @@ def test_true_sizes_below_the_stored_ones(rows, x_cols, widths):
     lin.device_error(DEV)
     want = torch.cat([whole[:, sum(ns[:i]):sum(ns[:i]) + w] for i, w in enumerate(widths)], 1)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [1, 5, 16, 40])
+@pytest.mark.parametrize("k,n,K,cb", [
+    (1024, 640, 3, 0),          # a unit per CTA
+    (1280, 5120, 4, 1),         # three parts of three and four units; whole column blocks from nine rows up
+    (896, 4736, 2, 2),          # a column block per CTA, 37 CTAs
+    (128, 19200, 8, 0),         # one unit deep, 150 column blocks: two for two of the CTAs
+    (512, 38016, 5, 1),         # 297 column blocks of four units: two or three per CTA
+    (9600, 512, 3, 0),          # 37 parts of two and three units
+    (16384, 256, 6, 2),         # 74 parts
+])
+def test_column_blocks_and_parts_of_them(rows, k, n, K, cb):
+    """The ways of dealing units to CTAs other than even ranges: whole column blocks, equal parts of one, remainders of both, against a plain
+    fp32 product on the decoded weights (bounds of the test above)."""
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(rows + n)
+    packed, suh, svh = random_packed(k, n, K, gen, DEV), random_signs(k, gen, DEV, 1), (random_signs(n, gen, DEV).view(-1) / 64).half()
+    x = torch.randn((rows, k), device=DEV, generator=gen).half()
+    y, again = (torch.empty((rows, n), dtype=torch.float32, device=DEV) for _ in range(2))
+    lin.run(x, packed, suh, svh, [], cb, out=y)
+    lin.run(x, packed, suh, svh, [], cb, out=again)
+    torch.cuda.synchronize()
+    lin.device_error(DEV)
+    assert torch.equal(y, again)
+    torch.backends.cuda.matmul.allow_tf32 = False
+    want = _had128(lin.had_in_group(x, suh).float() @ lin.reconstruct_packed(packed, cb).float()) * svh.float()
+    assert float((y - want).norm() / want.norm()) <= 1e-3
+    assert float((y - want).abs().max() / want.pow(2).mean().sqrt()) <= 2e-3

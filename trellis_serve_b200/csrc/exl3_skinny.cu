@@ -54,25 +54,61 @@ int skinny_init_device()
     return rc;
 }
 
-// Work split and shared-memory plan of one launch; `x`: SK_STREAM or one of the modes that keep a slot of activations per unit.
-static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaunch& l, size_t& smem)
+// Work split and shared-memory plan of one launch; `x`: SK_STREAM or one of the modes that keep a slot of activations per unit.  aligned: CTAs
+// may get column blocks or equal parts of them instead of even ranges.
+static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligned, SkinnyLaunch& l, size_t& smem)
 {
     memset(&l, 0, sizeof(l));
     l.a = a;
     l.KG = a.k / 128;
     l.NB = a.n_total / 128;
     const long long units = (long long)l.KG * l.NB;
-    l.grid = units < d->sm_count ? (int)units : d->sm_count;
-    if (l.grid > GEMV_MAX_GRID) l.grid = GEMV_MAX_GRID;
-    l.units_q = (int)(units / l.grid);
-    l.units_r = (int)(units % l.grid);
+    const int ctas = d->sm_count < GEMV_MAX_GRID ? d->sm_count : GEMV_MAX_GRID;
+    size_t most = (size_t)((units + ctas - 1) / ctas);       // units of the busiest CTA
+    l.piece = 1;
+    if (aligned) {
+        // Every way of dealing the units has a cost, counted in units of the busiest CTA (0.5 us each up to 16 rows).  Partial sums that
+        // CTAs exchange take 2.5 us on top of whole column blocks; a range that starts and ends inside column blocks, evenly as it is, hands
+        // over twice: 1 us, 2 and more from nine rows up, where the hand-over is longer.  Chained launches, us, even ranges against the
+        // choice here: whole blocks, K = 3: 1024 x 8192 8.9 / 6.7 at one row, 1024 x 17408 10.7 / 8.6, 16.3 / 11.1 at 16, 21.2 / 17.6 at 57;
+        // parts: 4096 x 4096, K = 4 9.6 / 8.8, 1792 x 4096 8.7 / 6.9 at one row, 18.6 / 10.1 at 16, 27.5 / 16.0 at 57, 5120 x 5120 18.6 / 15.9
+        // at 16.  Where the rule stays with even ranges: 5120 x 5120, one row 11.2, in three parts (14 units for 11) 11.7; 17408 x 5120 24.9,
+        // 27.5; 2048 x 25088, whole blocks (32 units for 22) 18.0, 18.8.  In a long range of few rows all hand-overs but the last are hidden:
+        // 5120 x 34816, one row 43.3, whole blocks (80 units for 74) 44.1, but 50.0 / 46.8 at 16 rows.
+        constexpr int EXCHANGE = 5;
+        const int uneven = a.rows > 8 ? 4 : 2, hidden = a.rows <= 8 && most > 12 ? 3 : 0;
+        const bool few = x == SK_ROTATE && a.rows > SK_FUSED_ROWS;           // rows rotated inside in one pass of the decode warps
+        long long best = (long long)most + EXCHANGE + uneven;
+        const long long whole = (long long)((l.NB + ctas - 1) / ctas) * l.KG;
+        if (whole + hidden < best && !(few && whole > SK_DECODE_WARPS)) {
+            best = whole + hidden;
+            l.piece = l.KG;
+        }
+        for (int parts = 2; parts <= l.KG && (long long)parts * l.NB <= ctas; parts++) {
+            const int part = (l.KG + parts - 1) / parts;
+            if (part + EXCHANGE < best && !(few && part > SK_DECODE_WARPS)) {
+                best = part + EXCHANGE;
+                l.parts = parts;
+                l.piece = 1;
+            }
+        }
+    }
+    if (l.parts) {
+        l.grid = l.parts * l.NB;
+        most = (size_t)((l.KG + l.parts - 1) / l.parts);
+    } else {
+        const long long pieces = units / l.piece;
+        l.grid = pieces < ctas ? (int)pieces : ctas;
+        l.units_q = (int)(pieces / l.grid);
+        l.units_r = (int)(pieces % l.grid);
+        most = (size_t)(l.units_q + (l.units_r ? 1 : 0)) * l.piece;
+    }
     // Stages of whole units, as long as three fit; a short range travels as one copy.  A bulk copy costs a few hundred nanoseconds whatever
     // its size (24 KB of weights or more), and a group of decode warps changes stages every 2 units / 3 steps: six units where the
     // rows are resident (17408 x 5120, one row, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1, K
     // = 8 25.4 -> 24.7), no more than 24 KB where they travel with the weights and the first stage is waited for (5120 x 5120, 16 rows: 18.5
     // us against 19.1 with six units).
     const size_t w = 2048u * (size_t)a.K, f = (size_t)operand_pitch(a.rows) * (a.mode == GEMV_SPLIT ? 512 : 256);
-    const size_t most = (size_t)(l.units_q + (l.units_r ? 1 : 0));
     const SkRaw raw = sk_raw_planes(x, a.x_glu);
     const size_t planes = x == SK_STREAM ? 0 : (size_t)(raw.planes_const + a.rows * raw.planes_row);
     const size_t fixed = SK_BAR_BYTES + (x == SK_STREAM ? 0 : most * f + planes * (most * 256 + 16)) + (size_t)a.rows * 512 + 1024;
@@ -103,6 +139,12 @@ static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaun
     l.add = c.add;
     l.xf_shard_stride = (long long)l.KG * (long long)f;
     return EXL3_OK;
+}
+
+static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaunch& l, size_t& smem)
+{
+    const int rc = plan_split(a, d, x, true, l, smem);
+    return rc == EXL3_OK || (l.piece == 1 && l.parts == 0) ? rc : plan_split(a, d, x, false, l, smem);      // the busiest CTA's rows may not fit
 }
 
 bool skinny_rotates_input(const GemvArgs& a)

@@ -76,7 +76,9 @@ struct SkTmem {
 struct SkinnyLaunch {
     GemvArgs a;
     int KG, NB, grid;
-    int units_q, units_r;       // units per CTA: the first units_r CTAs take units_q + 1
+    // How the units are dealt to the CTAs.  parts == 0: pieces of `piece` units (one, or a whole column block) evenly and contiguously, the
+    // first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.
+    int units_q, units_r, piece, parts;
     int stages, units_per_stage;
     uint32_t x_off, p_off;      // bytes: activations behind the weights, staged rows of the epilogue
     uint32_t r_off, r_plane;    // raw input of the in-kernel rotation (see SkRaw), bytes per plane
@@ -404,7 +406,26 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
     const int cta = blockIdx.x, rows = p.a.rows;
-    const int u0 = (int)gemv_first_unit(cta, p.units_q, p.units_r), u1 = (int)gemv_first_unit(cta + 1, p.units_q, p.units_r);
+    int u0, u1;
+    if (p.parts > 0) {
+        const int nb = cta / p.parts, part = cta - nb * p.parts;
+        u0 = nb * p.KG + part * p.KG / p.parts;
+        u1 = nb * p.KG + (part + 1) * p.KG / p.parts;
+    } else {
+        u0 = (int)gemv_first_unit(cta, p.units_q, p.units_r) * p.piece;
+        u1 = (int)gemv_first_unit(cta + 1, p.units_q, p.units_r) * p.piece;
+    }
+    auto sharers = [&](int nb, int& first, int& last) {                     // CTAs that share column block nb
+        if (p.parts > 0) {
+            first = nb * p.parts;
+            last = first + p.parts - 1;
+        } else if (p.piece > 1) {
+            first = last = cta;
+        } else {
+            first = gemv_cta_of_unit((long long)nb * p.KG, p.units_q, p.units_r);
+            last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, p.units_q, p.units_r);
+        }
+    };
     const int ups = p.units_per_stage, stages = p.stages;
     const int halves = 2 * (u1 - u0), fills = (u1 - u0 + ups - 1) / ups;
 
@@ -695,8 +716,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         for (int ub = u0; ub < u1;) {
             const int nb = ub / p.KG, left = (nb + 1) * p.KG - ub, ue = ub + left < u1 ? ub + left : u1;
             const int hb = 2 * (ub - u0), he = 2 * (ue - u0);
-            const int c_first = gemv_cta_of_unit((long long)nb * p.KG, p.units_q, p.units_r);
-            const int c_last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, p.units_q, p.units_r);
+            int c_first, c_last;
+            sharers(nb, c_first, c_last);
             const bool shared = c_first != c_last;
             const size_t nelem = (size_t)rows * 128;
             float* dst = (shared ? p.a.partials + (size_t)(cta + nb) * nelem : P) + ew * 32 + lane;
@@ -767,8 +788,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     const uint32_t tp_epoch = p.a.tp.world > 1 ? (uint32_t)*reinterpret_cast<volatile int*>(p.a.tp.state) + 1u : 0u;
     if (ALL_FINISH && *flag) {
         const int nb = (u1 - 1) / p.KG;
-        const int c_first = gemv_cta_of_unit((long long)nb * p.KG, p.units_q, p.units_r);
-        const int c_last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, p.units_q, p.units_r);
+        int c_first, c_last;
+        sharers(nb, c_first, c_last);
         sk_finish_block_call<RB, EPI>(p.a, tp_epoch, P, c_first != c_last, c_first, c_last, nb, warp, SK_THREADS / 32, lane);
     }
     EXL3_STAMP(5);
