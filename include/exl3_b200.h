@@ -336,6 +336,19 @@ exl3_status exl3_moe_gemm(const uint32_t *xf, const uint32_t *packed, int K, int
 exl3_status exl3_moe_combine(const uint16_t *yd, const float *topk_weights, const int32_t *topk_ids, int tokens, int top_k,
                              int hidden, int num_experts, void *y, int y_dtype, void *stream);
 
+/* Routed experts of a few slots -- one decoded token, or a few -- without alignment and without rotation launches: every slot is a row
+ * with a matrix of its own, two launches of the decode kernel, which rotates its input itself (the second one SiLU(gate) * up).
+ * exl3_moe_prefers_slots: 1 where that is the faster way (no more slots than experts, and no more than 16 units of 128 x 128 weights per SM
+ * and launch).  A layer of one token, 256 experts of 2048 x 512, top-8, K = 3, takes 21.6 us for 30.2; two tokens 29.9 for 36.
+ * exl3_moe_slots_experts: topk_ids -> yd[slot, :] as exl3_moe_tc_experts gives it (expert_map as there), gu: scratch fp16 [slots, 2 *
+ * inter]; x, gu, weights and suh 16-byte aligned; workspace as for exl3_moe_gemm.  The launch structure this replaces for one token is that of
+ * cuda/src/sglang_exl3/kernels/marlin_moe.py:272-294. */
+int exl3_moe_prefers_slots(int slots, int num_local, int hidden, int inter, int K, int codebook);
+exl3_status exl3_moe_slots_experts(const void *x, int x_dtype, int slots, int top_k, int hidden, int inter, const int32_t *topk_ids,
+                                   int num_experts, const int32_t *expert_map, int num_local, const uint32_t *w13, const uint16_t *suh13,
+                                   const uint16_t *svh13, const uint32_t *w2, const uint16_t *suh2, const uint16_t *svh2, int K, int codebook,
+                                   uint16_t *gu, uint16_t *yd, void *workspace, size_t workspace_bytes, void *stream);
+
 /* Routed experts with many rows per expert (prefill-sized batches) on the tensor cores.  The reference serves such batches
  * with the same grouped kernel and larger moe blocks (moe_block_size picks 8..64 rows from T * top_k / E,
  * cuda/src/sglang_exl3/kernels/marlin_moe.py:52-57; launch at cuda/csrc/exl3_marlin_moe.cu:376-408); here the routing is

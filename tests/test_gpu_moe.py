@@ -205,3 +205,57 @@ def test_expert_parallel_shares_add_up_to_the_layer(world):
     got = total.cpu().numpy()
     assert orc.rel_norm(got, ref) <= 3e-3, orc.rel_norm(got, ref)
     assert orc.max_over_rms(got, ref) <= 8e-3, orc.max_over_rms(got, ref)
+
+
+def _layer(pack, x, w, ids, maps=None):
+    need = moe.layer_workspace_bytes([p.num_experts for p in pack.packs], pack.hidden, pack.inter, pack.codebook, *ids.shape)
+    out, ws = torch.empty_like(x), torch.zeros(need, dtype=torch.uint8, device=DEV)
+    moe.run_layer(x, w, ids, pack, out, ws, maps)
+    again = torch.empty_like(x)
+    moe.run_layer(x, w, ids, pack, again, ws, maps)
+    torch.cuda.synchronize()
+    assert torch.equal(out, again)
+    return out
+
+
+@pytest.mark.parametrize("tokens,top_k,Ks,hidden,inter,cb,dtype", [
+    (1, 8, [3] * 16, 2048, 512, 0, torch.bfloat16),
+    (1, 1, [2] * 3, 128, 128, 2, torch.float16),            # one slot, one unit deep
+    (2, 3, [5] * 8, 384, 640, 2, torch.bfloat16),           # experts shared by two slots
+    (2, 4, [8] * 12, 1024, 384, 1, torch.float16),
+    (1, 4, [3, 4, 3, 4, 3, 3, 4, 3], 256, 256, 0, torch.float16),       # two bitrate classes
+])
+def test_few_slots_agree_with_the_aligned_form(tokens, top_k, Ks, hidden, inter, cb, dtype):
+    """One token or two: a row and a matrix per slot (exl3_moe_slots_experts) against blocks of eight rows, whose arithmetic differs by the
+    order of the fp32 sums only, so by single roundings of the fp16 values between and of the result; also with ids out of range, with an
+    expert map that leaves experts out, and for rows that are not 16-byte aligned, which go the other way."""
+    from trellis_serve_b200 import _lib
+    E = len(Ks)
+    gate, up, down = _mixed_experts(9000, Ks, hidden, inter)
+    for proj, scale in ((gate, hidden), (up, hidden), (down, inter)):
+        proj[2][:] = [(s.astype(np.float32) / (1.24 * scale ** 0.5)).astype(np.float16) for s in proj[2]]
+    pack = moe.prepare_mixed(_to_dev(gate), _to_dev(up), _to_dev(down), cb)
+    slots = tokens * top_k
+    assert all(_lib.load().exl3_moe_prefers_slots(slots, max(p.num_experts, slots), hidden, inter, p.bits, cb) for p in pack.packs)
+    ids, w = _routing(tokens, top_k, E, 7 + tokens)
+    if tokens > 1:
+        ids[1] = ids[0]
+    x = torch.randn((tokens, hidden), device=DEV, generator=torch.Generator(device=DEV).manual_seed(3)).to(dtype)
+    wt, it = torch.from_numpy(w).to(DEV), torch.from_numpy(ids).to(DEV)
+
+    def close(got, want):
+        got, want = got.float(), want.float()
+        assert float((got - want).norm() / want.norm()) <= (4e-3 if dtype == torch.bfloat16 else 1e-3)
+    close(_layer(pack, x, wt, it), moe.forward_mixed(x, wt, it, pack))
+    odd = torch.empty(tokens * hidden + 1, dtype=dtype, device=DEV)[1:].view(tokens, hidden)
+    odd.copy_(x)
+    assert torch.equal(_layer(pack, odd, wt, it), moe.forward_mixed(odd, wt, it, pack))
+    if slots > 2:
+        bad = it.clone()
+        bad.view(-1)[0], bad.view(-1)[1] = -1, E
+        close(_layer(pack, x, wt, bad), moe.forward_mixed(x, wt, bad, pack))
+        maps = [m.clone() for m in pack.expert_maps]
+        for m in maps:
+            m[it.view(-1)[0].long()] = -1
+        gone = torch.where(it == it.view(-1)[0], -1, it)
+        close(_layer(pack, x, wt, it, maps), moe.forward_mixed(x, wt, gone, pack))

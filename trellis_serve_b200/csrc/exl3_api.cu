@@ -885,6 +885,39 @@ exl3_status exl3_moe_combine(const uint16_t* yd, const float* topk_weights, cons
                               y_dtype == EXL3_BF16, (cudaStream_t)stream);
 }
 
+int exl3_moe_prefers_slots(int slots, int num_local, int hidden, int inter, int K, int codebook)
+{
+    if (slots < 1 || slots > num_local || hidden < 128 || (hidden % 128) || inter < 128 || (inter % 128) || K < 2 || K > 8 || codebook < 0 || codebook > 2) return 0;
+    return skinny_serves_slots(slots, hidden, inter, K, codebook);
+}
+
+exl3_status exl3_moe_slots_experts(const void* x, int x_dtype, int slots, int top_k, int hidden, int inter, const int32_t* topk_ids, int num_experts,
+                                   const int32_t* expert_map, int num_local, const uint32_t* w13, const uint16_t* suh13, const uint16_t* svh13,
+                                   const uint32_t* w2, const uint16_t* suh2, const uint16_t* svh2, int K, int codebook, uint16_t* gu, uint16_t* yd,
+                                   void* workspace, size_t workspace_bytes, void* stream)
+{
+    if (int rc = check_matrix(hidden, 2 * inter, K, codebook)) return rc;
+    if (slots < 1 || top_k < 1 || (inter % 128) || num_experts < 1 || num_local < 1) return EXL3_ERR_BAD_SHAPE;
+    if (x_dtype != EXL3_F16 && x_dtype != EXL3_BF16) return EXL3_ERR_UNSUPPORTED_DTYPE;
+    if (!current_device_info()) return EXL3_ERR_NOT_INITIALISED;
+    if (!skinny_serves_slots(slots, hidden, inter, K, codebook)) return EXL3_ERR_UNSUPPORTED_ROWS;
+    if (!aligned(x, 16) || !aligned(w13, 16) || !aligned(suh13, 16) || !aligned(svh13, 8) || !aligned(w2, 16) || !aligned(suh2, 16) || !aligned(svh2, 8) ||
+        !aligned(gu, 16) || !aligned(yd, 8) || !aligned(topk_ids, 4) || (expert_map && !aligned(expert_map, 4)))
+        return EXL3_ERR_BAD_POINTER;
+    const MoeWorkspace wl = moe_workspace();
+    if (!aligned(workspace, 256) || workspace_bytes < wl.total) return EXL3_ERR_WORKSPACE;
+    unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+    float* partials = reinterpret_cast<float*>(ws + wl.partials_off);
+    int *counters = reinterpret_cast<int*>(ws + wl.counters_off), *err = reinterpret_cast<int*>(ws);
+    cudaStream_t st = (cudaStream_t)stream;
+    auto half = [](const uint16_t* p) { return reinterpret_cast<const __half*>(p); };
+    if (int rc = launch_skinny_slots(x, x_dtype == EXL3_BF16, top_k, topk_ids, expert_map, num_experts, num_local, 0, slots, hidden, 2 * inter, 2, 0, w13,
+                                     half(suh13), half(svh13), K, codebook, reinterpret_cast<__half*>(gu), partials, counters, err, st))
+        return rc;
+    return launch_skinny_slots(gu, 0, 1, topk_ids, expert_map, num_experts, num_local, 1, slots, inter, hidden, 1, 1, w2, half(suh2), half(svh2), K, codebook,
+                               reinterpret_cast<__half*>(yd), partials, counters, err, st);
+}
+
 int exl3_moe_tc_block_rows(void) { return MOE_TC_BLOCK_ROWS; }
 
 size_t exl3_moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter)

@@ -191,14 +191,15 @@ static __device__ __noinline__ void gemv_residual_store(const GemvArgs& a, uint3
 }
 
 // One row's block of 128 outputs (one warp, four columns per lane) from the fp32 sums: the rotated-basis product as it is, or
-// Had128 * svh in the output type, summed over the ranks where there is an exchange.  EPI 1: with the residual stream.
+// Had128 * svh in the output type, summed over the ranks where there is an exchange.  EPI 1: with the residual stream.  svh: a.svh, or so
+// that svh + 128 nb are the block's.
 template <int EPI>
-__device__ __forceinline__ void gemv_finish_row(const GemvArgs& a, uint32_t tp_epoch, float4 v, int m, int nb, int lane)
+__device__ __forceinline__ void gemv_finish_row(const GemvArgs& a, const __half* svh, uint32_t tp_epoch, float4 v, int m, int nb, int lane)
 {
     const long long o = (long long)m * a.n_total + nb * 128 + 4 * lane;
     if (EPI == 1 || !a.rotated) {
         fwht128(v.x, v.y, v.z, v.w, lane);
-        const uint2 sv = *reinterpret_cast<const uint2*>(a.svh + nb * 128 + 4 * lane);
+        const uint2 sv = *reinterpret_cast<const uint2*>(svh + nb * 128 + 4 * lane);
         const __half2 s01 = *reinterpret_cast<const __half2*>(&sv.x), s23 = *reinterpret_cast<const __half2*>(&sv.y);
         v.x *= HAD_SCALE * __low2float(s01);
         v.y *= HAD_SCALE * __high2float(s01);

@@ -112,6 +112,13 @@ void gemv_set_mode_override(int mode);      // -1 = default; test / measurement 
 // variant can serve the problem (row count, alignment, shared-memory budget) and launch_skinny() then requires it to.
 bool skinny_rotates_input(const GemvArgs& a);
 int launch_skinny(const GemvArgs& a, cudaStream_t st);
+// Routed experts of a few slots, two launches (SkSlots): whether the kernel serves a layer of these sizes, and one of its products; `known`:
+// the ids were there before the kernel ahead began.  partials: 2560 x 128 floats, counters: slots * n / 128 zeros.
+constexpr int SK_SLOTS_UNITS = 16;         // most units per SM: beyond, the launches saved are outweighed by experts decoded once per slot
+bool skinny_serves_slots(int slots, int hidden, int inter, int K, int codebook);
+int launch_skinny_slots(const void* x, int x_bf16, int per_row, const int* ids, const int* map, int experts, int local, int known, int slots, int k, int n,
+                        int shards, int glu, const uint32_t* packed, const __half* suh, const __half* svh, int K, int codebook, __half* out,
+                        float* partials, int* counters, int* err, cudaStream_t st);
 int skinny_init_device();
 // Rows that a core-matrix column of the rotated input is laid out for (the kernels' B operand; the padding rows are never written and
 // their products never looked at): a constant of each kernel instance, so that descriptors advance by constants.

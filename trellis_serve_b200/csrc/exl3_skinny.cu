@@ -159,6 +159,81 @@ bool skinny_rotates_input(const GemvArgs& a)
     return plan_skinny(a, d, a.norm_weight ? SK_NORM : SK_ROTATE, l, smem) == EXL3_OK;
 }
 
+static int launch_planned(SkinnyLaunch& l, int x, size_t smem, cudaStream_t st)
+{
+#ifdef EXL3_TIMELINE
+    if (!g_tl_base) cudaGetSymbolAddress(reinterpret_cast<void**>(&g_tl_base), g_timeline);
+    l.tl = g_tl_base + (size_t)(g_tl_next_slot++ % TL_SLOTS) * TL_CTAS * TL_POINTS;
+#endif
+    const int pitch = operand_pitch(l.a.rows);
+    switch (l.a.K) {
+        case 2: return launch_skinny_for_k<2>(l, pitch, x, smem, st);
+        case 3: return launch_skinny_for_k<3>(l, pitch, x, smem, st);
+        case 4: return launch_skinny_for_k<4>(l, pitch, x, smem, st);
+        case 5: return launch_skinny_for_k<5>(l, pitch, x, smem, st);
+        case 6: return launch_skinny_for_k<6>(l, pitch, x, smem, st);
+        case 7: return launch_skinny_for_k<7>(l, pitch, x, smem, st);
+        case 8: return launch_skinny_for_k<8>(l, pitch, x, smem, st);
+    }
+    return EXL3_ERR_UNSUPPORTED_K;
+}
+
+// One of the two products of a routed-expert layer, every slot with a matrix of its own (see SkSlots): rows of k values -> n columns per slot.
+static GemvArgs slots_args(int slots, int k, int n, int glu, int K, int codebook)
+{
+    GemvArgs a;
+    memset(&a, 0, sizeof(a));
+    a.K = K;
+    a.codebook = codebook;
+    a.mode = gemv_default_mode(codebook);
+    a.rows = 1;
+    a.k = k;
+    a.n_total = slots * n;
+    a.n_shards = 1;
+    a.shard_end_blocks[0] = a.n_total / 128;
+    a.out_dtype = EXL3_F16;
+    a.x_glu = glu;
+    return a;
+}
+
+bool skinny_serves_slots(int slots, int hidden, int inter, int K, int codebook)
+{
+    const DeviceInfo* d = current_device_info();
+    if (!d || slots < 1 || hidden < 128 || inter < 128 || K < 2 || K > 8) return false;
+    for (int down = 0; down < 2; down++) {
+        const int k = down ? inter : hidden, n = down ? hidden : 2 * inter;
+        const long long blocks = (long long)slots * (n / 128), units = blocks * (k / 128);
+        if (blocks * 128 >= (1ll << 31) || blocks > (long long)WS_MAX_COUNTERS || blocks > 2048 || units > (long long)SK_SLOTS_UNITS * d->sm_count) return false;
+        SkinnyLaunch l;
+        size_t smem;
+        if (plan_skinny(slots_args(slots, k, n, down, K, codebook), d, SK_ROTATE, l, smem) != EXL3_OK) return false;
+    }
+    return true;
+}
+
+int launch_skinny_slots(const void* x, int x_bf16, int per_row, const int* ids, const int* map, int experts, int local, int known, int slots, int k, int n,
+                        int shards, int glu, const uint32_t* packed, const __half* suh, const __half* svh, int K, int codebook, __half* out,
+                        float* partials, int* counters, int* err, cudaStream_t st)
+{
+    const DeviceInfo* d = current_device_info();
+    if (!d) return EXL3_ERR_NOT_INITIALISED;
+    GemvArgs a = slots_args(slots, k, n, glu, K, codebook);
+    a.packed = packed;
+    a.x = x;
+    a.x_bf16 = x_bf16;
+    a.suh = suh;
+    a.svh = svh;
+    a.out = out;
+    a.partials = partials;
+    a.counters = counters;
+    a.err = err;
+    SkinnyLaunch l;
+    size_t smem = 0;
+    if (int rc = plan_skinny(a, d, SK_ROTATE, l, smem)) return rc;
+    l.s = {ids, map, experts, local, n / 128, n / 128 / shards, per_row, known, (long long)k * n * K / 32};
+    return launch_planned(l, SK_ROTATE, smem, st);
+}
+
 int launch_skinny(const GemvArgs& a, cudaStream_t st)
 {
     const DeviceInfo* d = current_device_info();
@@ -171,21 +246,7 @@ int launch_skinny(const GemvArgs& a, cudaStream_t st)
     size_t smem = 0;
     const int x = !a.x ? SK_STREAM : a.norm_weight ? SK_NORM : SK_ROTATE;
     if (int rc = plan_skinny(a, d, x, l, smem)) return rc;
-#ifdef EXL3_TIMELINE
-    if (!g_tl_base) cudaGetSymbolAddress(reinterpret_cast<void**>(&g_tl_base), g_timeline);
-    l.tl = g_tl_base + (size_t)(g_tl_next_slot++ % TL_SLOTS) * TL_CTAS * TL_POINTS;
-#endif
-    const int pitch = operand_pitch(a.rows);
-    switch (a.K) {
-        case 2: return launch_skinny_for_k<2>(l, pitch, x, smem, st);
-        case 3: return launch_skinny_for_k<3>(l, pitch, x, smem, st);
-        case 4: return launch_skinny_for_k<4>(l, pitch, x, smem, st);
-        case 5: return launch_skinny_for_k<5>(l, pitch, x, smem, st);
-        case 6: return launch_skinny_for_k<6>(l, pitch, x, smem, st);
-        case 7: return launch_skinny_for_k<7>(l, pitch, x, smem, st);
-        case 8: return launch_skinny_for_k<8>(l, pitch, x, smem, st);
-    }
-    return EXL3_ERR_UNSUPPORTED_K;
+    return launch_planned(l, x, smem, st);
 }
 
 }  // namespace exl3

@@ -33,10 +33,19 @@ static SkinnyKernel instance_for(int mode, int family, int pitch, int x, int res
     return mode == GEMV_SPLIT ? instance<K, GEMV_SPLIT, FAM_HASH>(pitch, x, residual) : instance<K, GEMV_PAIRED, FAM_HASH>(pitch, x, residual);
 }
 
+template <int K>
+static SkinnyKernel slots_instance(int mode, int family)
+{
+    if (family == FAM_MUL1) return skinny_kernel<K, GEMV_PAIRED, FAM_MUL1, 2, SK_ROTATE, 0, true>;
+    return mode == GEMV_SPLIT ? skinny_kernel<K, GEMV_SPLIT, FAM_HASH, 2, SK_ROTATE, 0, true> : skinny_kernel<K, GEMV_PAIRED, FAM_HASH, 2, SK_ROTATE, 0, true>;
+}
+
 template <>
 int launch_skinny_for_k<EXL3_SKINNY_K>(const SkinnyLaunch& l, int pitch, int x, size_t smem, cudaStream_t st)
 {
-    const SkinnyKernel kernel = instance_for<EXL3_SKINNY_K>(l.a.mode, codebook_family(l.a.codebook), pitch, x, l.a.res_out != nullptr);
+    const int family = codebook_family(l.a.codebook);
+    const SkinnyKernel kernel = l.s.ids ? slots_instance<EXL3_SKINNY_K>(l.a.mode, family)
+                                        : instance_for<EXL3_SKINNY_K>(l.a.mode, family, pitch, x, l.a.res_out != nullptr);
     if (!kernel) return EXL3_ERR_UNSUPPORTED_ROWS;
     // Programmatic stream serialization: prologue, weight copies and the first half units overlap the tail of the kernel ahead; the
     // kernel waits (griddepcontrol.wait) before touching anything that kernel wrote.
@@ -46,16 +55,20 @@ int launch_skinny_for_k<EXL3_SKINNY_K>(const SkinnyLaunch& l, int pitch, int x, 
 template <>
 int skinny_set_attributes_for_k<EXL3_SKINNY_K>(int max_smem)
 {
+    auto opt_in = [&](SkinnyKernel kernel) {
+        return cuda_status(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    };
     for (int family : {FAM_HASH, FAM_MUL1})
-        for (int mode : {GEMV_SPLIT, GEMV_PAIRED})
+        for (int mode : {GEMV_SPLIT, GEMV_PAIRED}) {
+            if (int rc = opt_in(slots_instance<EXL3_SKINNY_K>(mode, family))) return rc;
             for (int pitch : {2, 8, 16, 32, 64})
                 for (int x : {SK_STREAM, SK_ROTATE, SK_NORM})
                     for (int residual : {0, 1}) {
                         const SkinnyKernel kernel = instance_for<EXL3_SKINNY_K>(mode, family, pitch, x, residual);
                         if (!kernel) continue;
-                        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-                        if (int rc = cuda_status(e)) return rc;
+                        if (int rc = opt_in(kernel)) return rc;
                     }
+        }
     return EXL3_OK;
 }
 

@@ -73,8 +73,27 @@ struct SkTmem {
     static_assert(A_OFF + SK_GROUPS * A_BUFS * A_COLS <= SK_TMEM_COLS, "tensor memory");
 };
 
+// Routed experts of a few slots as one matrix: NB column blocks are `slots` runs of `blocks`, run s is the expert of slot s.
+struct SkSlots {
+    const int* ids;             // expert of each slot (a router's), `map`: -> this rank's or class's expert, or -1; null: as it is
+    const int* map;
+    int experts, local;         // ids in [0, experts); experts behind the pointers
+    int blocks, shard_blocks;   // column blocks of an expert, of one of its matrices with sign vectors of their own (gate, up)
+    int per_row;                // slots that share a row of x (top-k, or 1)
+    int known;                  // the ids were there before the kernel ahead began: read ahead of the wait
+    long long stride;           // 32-bit words between experts
+
+    __device__ __forceinline__ int expert(int s) const
+    {
+        int e = __ldcg(ids + s);
+        if (map) e = e >= 0 && e < experts ? __ldcg(map + e) : -1;
+        return e >= 0 && e < local ? e : -1;
+    }
+};
+
 struct SkinnyLaunch {
     GemvArgs a;
+    SkSlots s;
     int KG, NB, grid;
     // How the units are dealt to the CTAs.  parts == 0: pieces of `piece` units (one, or a whole column block) evenly and contiguously, the
     // first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.
@@ -320,9 +339,10 @@ __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsi
 
 // The finished sums of column block nb -> output, rows w, w + nw, ... of a warp.  shared: the block's partial sums of CTAs c_first ..
 // c_last are added in CTA order; several rows and CTAs are requested together, so that their round trips overlap.
+// svh: so that svh + 128 nb are the block's.
 template <int RB, int EPI>
-__device__ __forceinline__ void sk_finish_block(const GemvArgs& a, uint32_t tp_epoch, const float* P, bool shared, int c_first, int c_last, int nb,
-                                                int w, int nw, int lane)
+__device__ __forceinline__ void sk_finish_block(const GemvArgs& a, const __half* svh, uint32_t tp_epoch, const float* P, bool shared, int c_first, int c_last,
+                                                int nb, int w, int nw, int lane)
 {
     constexpr int CB = 8 / RB;
     const int rows = a.rows;
@@ -361,7 +381,7 @@ __device__ __forceinline__ void sk_finish_block(const GemvArgs& a, uint32_t tp_e
         }
 #pragma unroll 1
         for (int i = 0; i < RB; i++) {
-            if (m + nw * i < rows) gemv_finish_row<EPI>(a, tp_epoch, make_float4(v[0][0], v[0][1], v[0][2], v[0][3]), m + nw * i, nb, lane);
+            if (m + nw * i < rows) gemv_finish_row<EPI>(a, svh, tp_epoch, make_float4(v[0][0], v[0][1], v[0][2], v[0][3]), m + nw * i, nb, lane);
 #pragma unroll
             for (int j = 0; j + 1 < RB; j++)
 #pragma unroll
@@ -374,14 +394,16 @@ template <int RB, int EPI>
 static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint32_t tp_epoch, const float* P, bool shared, int c_first, int c_last,
                                                          int nb, int w, int nw, int lane)
 {
-    sk_finish_block<RB, EPI>(a, tp_epoch, P, shared, c_first, c_last, nb, w, nw, lane);
+    sk_finish_block<RB, EPI>(a, a.svh, tp_epoch, P, shared, c_first, c_last, nb, w, nw, lane);
 }
 
 // RP: operand pitch, the rows rounded up (operand_pitch).
-template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0>
+// SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.
+template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0, bool SLOTS = false>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_constant__ SkinnyLaunch p)
 {
     static_assert((X != SK_NORM && EPI == 0) || RP == SK_FUSED_ROWS, "the kernel normalises, and carries the residual stream of, one or two rows");
+    static_assert(!SLOTS || (X == SK_ROTATE && RP == SK_FUSED_ROWS && EPI == 0), "slots come one row each");
     static_assert(X != SK_ROTATE || RP <= SK_ROTATE_ROWS, "the kernel rotates up to eight rows");
     constexpr int RB = RP <= 8 ? 1 : RP <= 16 ? 2 : 4;                      // rows that a warp finishes together
     constexpr bool ALL_FINISH = RP >= 16;
@@ -432,7 +454,35 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     auto weights = [&](int j, int slot) {                                   // one thread: fill number j, units [u0 + j * ups, ...)
         const int u = u0 + j * ups, n = u1 - u < ups ? u1 - u : ups;
         ptx::mbar_arrive_expect_tx(&w_full[slot], (uint32_t)n * W_BYTES);
-        ptx::bulk_g2s(wring + (size_t)(slot * ups) * W_BYTES, p.a.packed + (long long)u * (512 * K), (uint32_t)n * W_BYTES, &w_full[slot]);
+        if constexpr (SLOTS) {
+            const int per = p.s.blocks * p.KG;                              // units of an expert
+            unsigned char* dst = wring + (size_t)(slot * ups) * W_BYTES;
+            for (int at = u; at < u + n;) {
+                const int sl = at / per, in = at - sl * per, run = per - in < u + n - at ? per - in : u + n - at, e = p.s.expert(sl);
+                ptx::bulk_g2s(dst, p.a.packed + (e < 0 ? 0 : e) * p.s.stride + (long long)in * (512 * K), (uint32_t)run * W_BYTES, &w_full[slot]);
+                dst += (size_t)run * W_BYTES;
+                at += run;
+            }
+        } else {
+            ptx::bulk_g2s(wring + (size_t)(slot * ups) * W_BYTES, p.a.packed + (long long)u * (512 * K), (uint32_t)n * W_BYTES, &w_full[slot]);
+        }
+    };
+    // One thread: the CTA's units' 256 bytes of sign vectors, or (row >= 0) of plane `row` of the input, of the slots' experts.
+    [[maybe_unused]] auto rows_of_slots = [&](unsigned char* dst, int row, uint64_t* bar) {
+        for (int u = u0; u < u1;) {
+            const int unb = u / p.KG, ukg = u - unb * p.KG, run = p.KG - ukg < u1 - u ? p.KG - ukg : u1 - u;
+            const int sl = unb / p.s.blocks, nb = unb - sl * p.s.blocks;
+            const unsigned char* src;
+            if (row >= 0) {
+                src = reinterpret_cast<const unsigned char*>(p.a.x) + ((long long)(sl / p.s.per_row) * sk_raw_planes(X, p.a.x_glu).planes_row + row) * 2 * p.a.k;
+            } else {
+                const int e = p.s.expert(sl);
+                src = reinterpret_cast<const unsigned char*>(p.a.suh) + ((long long)(e < 0 ? 0 : e) * (p.s.blocks / p.s.shard_blocks) + nb / p.s.shard_blocks) * 2 * p.a.k;
+            }
+            ptx::bulk_g2s(dst, src + ukg * 256, (uint32_t)run * 256u, bar);
+            dst += (size_t)run * 256;
+            u += run;
+        }
     };
     // One thread: n units from u on, `bytes` per row block of a column block (consecutive in memory), a source per shard.
     auto rows_of = [&](int u, int n, unsigned char* dst, const void* src, uint32_t bytes, long long shard_stride, uint64_t* bar) {
@@ -459,11 +509,15 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             for (int g = 0; g < SK_GROUPS; g++) ptx::mbar_init(&acc_done[g], 1);
             for (int d = 0; d < TM::ACC_BUFS; d++) ptx::mbar_init(&acc_empty[d], 4);
             ptx::mbar_fence_init();
+            if constexpr (SLOTS) {
+                if (!p.s.known) ptx::grid_dependency_wait();                // the ids
+            }
             for (int j = 0; j < stages && j < fills; j++) weights(j, j);    // constants: before the kernel ahead has finished
             if constexpr (X != SK_STREAM) {
                 const int n = u1 - u0;
                 ptx::mbar_arrive_expect_tx(&x_full[1], (uint32_t)(n * sk_raw_planes(X, 0).planes_const) * 256u);
-                rows_of(u0, n, smem + p.r_off, p.a.suh, 256, 2ll * p.a.k, &x_full[1]);
+                if constexpr (SLOTS) rows_of_slots(smem + p.r_off, -1, &x_full[1]);
+                else rows_of(u0, n, smem + p.r_off, p.a.suh, 256, 2ll * p.a.k, &x_full[1]);
                 if constexpr (X == SK_NORM) rows_of(u0, n, smem + p.r_off + p.r_plane, p.a.norm_weight, 256, 0, &x_full[1]);
             }
         }
@@ -479,6 +533,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     sk_fence_after();
     // All 512 columns are this CTA's: tensor memory starts at address 0, which keeps the addresses warp-uniform constants.
     uint32_t failed = *tmem_slot != 0;
+    if constexpr (SLOTS) {
+        // The kernel behind may look at the ids as soon as it begins: not before the kernel that wrote them has finished.
+        if (!p.s.known) ptx::grid_dependency_wait();
+    }
     ptx::grid_launch_dependents();                                          // the next kernel in the stream may begin its prologue
 
     if (warp >= SK_DECODE_WARP) {
@@ -679,7 +737,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 const unsigned char* x = reinterpret_cast<const unsigned char*>(p.a.x);
                 unsigned char* dst = smem + p.r_off + sk_raw_planes(X, p.a.x_glu).planes_const * p.r_plane;
                 ptx::mbar_arrive_expect_tx(&x_full[0], (uint32_t)(n * rows * row_planes) * 256u);
-                for (int q = 0; q < rows * row_planes; q++, x += 2 * p.a.k, dst += p.r_plane) rows_of(u0, n, dst, x, 256, 0, &x_full[0]);
+                for (int q = 0; q < rows * row_planes; q++, x += 2 * p.a.k, dst += p.r_plane) {
+                    if constexpr (SLOTS) rows_of_slots(dst, q, &x_full[0]);
+                    else rows_of(u0, n, dst, x, 256, 0, &x_full[0]);
+                }
             }
             int slot = 0;
             uint32_t phase = 0;
@@ -721,6 +782,13 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             const bool shared = c_first != c_last;
             const size_t nelem = (size_t)rows * 128;
             float* dst = (shared ? p.a.partials + (size_t)(cta + nb) * nelem : P) + ew * 32 + lane;
+            const __half* svh = p.a.svh;
+            [[maybe_unused]] bool held = true;                              // SLOTS: the slot's expert is one of these
+            if constexpr (SLOTS) {
+                const int sl = nb / p.s.blocks, e = p.s.expert(sl);
+                held = e >= 0;
+                svh += (long long)(e - sl) * p.s.blocks * 128;
+            }
             ptx::named_bar_sync(SK_BAR_ACC + d, (SK_GROUPS + 4) * 32);
             sk_fence_after();
 #pragma unroll 1
@@ -768,9 +836,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 if (tid == 0) *flag = finish;
                 break;
             }
-            if (finish) {
+            if (finish && held) {
                 if constexpr (ALL_FINISH) sk_finish_block_call<RB, EPI>(p.a, tp_epoch, P, shared, c_first, c_last, nb, ew, 4, lane);
-                else sk_finish_block<RB, EPI>(p.a, tp_epoch, P, shared, c_first, c_last, nb, ew, 4, lane);
+                else sk_finish_block<RB, EPI>(p.a, svh, tp_epoch, P, shared, c_first, c_last, nb, ew, 4, lane);
             }
             EXL3_STAMP_LANE(ew == 0, 7);
             ptx::named_bar_sync(SK_BAR_EPI, 128);                           // staged rows and flag may be overwritten

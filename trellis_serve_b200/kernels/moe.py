@@ -381,12 +381,17 @@ def layer_workspace_bytes(num_experts_per_class: list[int], hidden: int, inter: 
     return _plan(num_experts_per_class, hidden, inter, codebook, tokens, top_k)[1]
 
 
+def _aligned16(*tensors) -> bool:
+    return all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
 def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, workspace: torch.Tensor,
               expert_maps: list[torch.Tensor] | None = None) -> torch.Tensor:
     """One MoE layer (alignment included) that allocates nothing: `workspace` is a zero-filled uint8 tensor of at least
     `layer_workspace_bytes(...)`; `expert_maps` replaces the pack's per-class maps (expert parallelism with an engine's
     global -> local map composed in).  Same kernels and the same bits as `forward_mixed` for decode-sized batches; a class
-    whose experts see `TC_ROWS_PER_EXPERT` rows or more on average goes through the grouped tensor-core GEMM."""
+    whose experts see `TC_ROWS_PER_EXPERT` rows or more on average goes through the grouped tensor-core GEMM, and the few slots of
+    one decoded token or two through two launches of the dense decode kernel (`exl3_moe_slots_experts`)."""
     _require_cuda(x, "x")
     lib = _lib.load()
     tokens, hidden = x.shape
@@ -428,6 +433,12 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
                 _lib.check(lib.exl3_moe_tc_experts(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
                                                    pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
                                                    _ptr(pk.svh2), K, pk.codebook, yd, at(f"tc{c}"), plan[f"tc{c}"][1], st), "exl3_moe_tc_experts")
+                continue
+            if (lib.exl3_moe_prefers_slots(slots, pk.num_experts, hidden, inter, K, pk.codebook)
+                    and _aligned16(x, pk.w13, pk.w2, pk.suh13, pk.suh2)):
+                _lib.check(lib.exl3_moe_slots_experts(_ptr(x), _dtype_code(x), slots, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
+                                                      pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
+                                                      _ptr(pk.svh2), K, pk.codebook, gu, yd, ws, ws_bytes, st), "exl3_moe_slots_experts")
                 continue
             _lib.check(lib.exl3_moe_align_mapped(_ptr(ids32), slots, emap.numel(), _ptr(emap), pk.num_experts, sorted_ids, cap,
                                                  expert_ids, num_post, st), "exl3_moe_align_mapped")
