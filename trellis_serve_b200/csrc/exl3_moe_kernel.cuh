@@ -171,9 +171,15 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     const int UB = p.NB * p.KG;                                             // units per item
     // Values read from memory go through a reduction where MMA operands depend on them: its result is a uniform register.
     const int n_items = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)(LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS));
-    // What is split over the CTAs: units, or (LIST) whole column blocks -- a row's sums are then the same whatever item the alignment,
-    // whose order inside an expert is not fixed, put it into.
-    const int grain = LIST ? p.KG : 1;
+    // What is split over the CTAs: units, or whole column blocks -- with LIST always: a row's sums are then the same whatever item the
+    // alignment, whose order inside an expert is not fixed, put it into; otherwise where the exchange of partial sums that it saves is worth
+    // more than what the busiest CTA takes on (the costs of the dense kernel's split, in units).
+    int grain = LIST ? p.KG : 1;
+    if (!LIST && (long long)n_items * UB < (1ll << 30)) {
+        const unsigned blocks = (unsigned)(n_items * p.NB), cut = (blocks * p.KG + gridDim.x - 1) / gridDim.x;
+        const unsigned whole = (blocks + gridDim.x - 1) / gridDim.x * p.KG;
+        if (whole + (cut > 12 ? 3 : 0) < cut + 7) grain = p.KG;
+    }
     const long long total = (long long)n_items * (UB / grain);
     int units_q, units_r;
     if (total < (1ll << 31)) {                                              // the 64-bit division is a few hundred clocks of everyone's start
