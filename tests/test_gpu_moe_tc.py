@@ -125,3 +125,34 @@ def test_graph_replay_with_fresh_routing_allocates_nothing():
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, out2)
+
+
+@pytest.mark.parametrize("top_k,tokens,dtype", [(1, 90, torch.float16), (2, 61, torch.bfloat16), (3, 57, torch.float16), (5, 33, torch.bfloat16),
+                                               (8, 30, torch.float16), (11, 17, torch.bfloat16)])
+def test_last_rotation_and_sum_in_one_launch(top_k, tokens, dtype):
+    """exl3_moe_tc_layer against exl3_moe_tc_experts + exl3_moe_combine, which an output that is not 16-byte aligned takes: the same roundings
+    of the slots' rows, their fp32 sum in another order -- at most a unit in the last place of the result, and at 2^-22 of the summed values
+    in all.  Top-k from one to more than a warp's eight rows, tokens that do not fill the last warp, ids out of range and an expert that
+    the map leaves out."""
+    E, hidden, inter, K, cb = 12 if top_k == 11 else 8, 384, 128, 3, 0
+    gate, up, down = _experts(51 + top_k, E, hidden, inter, K, out_scale=1 / 8)
+    pack = moe.prepare_mixed(_to_dev(gate), _to_dev(up), _to_dev(down), cb)
+    assert moe.moe_block_size(tokens, top_k, E) == 128
+    ids, w = _routing(tokens, top_k, E, 5 + top_k)
+    ids[0, 0], ids[1, 0] = -1, E
+    emap = pack.expert_maps[0].clone()
+    emap[3] = -1
+    x = torch.randn((tokens, hidden), device=DEV, generator=torch.Generator(device=DEV).manual_seed(2)).to(dtype)
+    wt, it = torch.from_numpy(w).to(DEV), torch.from_numpy(ids).to(DEV)
+    ws = torch.zeros(moe.layer_workspace_bytes([E], hidden, inter, cb, tokens, top_k), dtype=torch.uint8, device=DEV)
+    one, again = torch.empty_like(x), torch.empty_like(x)
+    two = torch.empty(tokens * hidden + 2, dtype=dtype, device=DEV)[2:].view(tokens, hidden)
+    for maps in (None, [emap]):
+        for out in (one, again, two):
+            moe.run_layer(x, wt, it, pack, out, ws, maps)
+        torch.cuda.synchronize()
+        assert torch.equal(one, again)
+        ulp = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
+        a, b = one.float(), two.float()
+        assert bool(((a - b).abs() <= ulp * b.abs() + 2.0 ** -22 * b.abs().max()).all())
+        assert float((a != b).float().mean()) <= 0.02

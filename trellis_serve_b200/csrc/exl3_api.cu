@@ -926,10 +926,10 @@ size_t exl3_moe_tc_workspace_bytes(int slots, int num_local, int hidden, int int
     return moe_tc_workspace_bytes(slots, num_local, hidden, inter);
 }
 
-exl3_status exl3_moe_tc_experts(const void* x, int x_dtype, int tokens, int top_k, int hidden, int inter, const int32_t* topk_ids,
-                                int num_experts, const int32_t* expert_map, int num_local, const uint32_t* w13, const uint16_t* suh13,
-                                const uint16_t* svh13, const uint32_t* w2, const uint16_t* suh2, const uint16_t* svh2, int K, int codebook,
-                                uint16_t* yd, void* workspace, size_t workspace_bytes, void* stream)
+static int moe_tc_common(const void* x, int x_dtype, int tokens, int top_k, int hidden, int inter, const int32_t* topk_ids, int num_experts,
+                         const int32_t* expert_map, int num_local, const uint32_t* w13, const uint16_t* suh13, const uint16_t* svh13, const uint32_t* w2,
+                         const uint16_t* suh2, const uint16_t* svh2, int K, int codebook, void* yd, void* workspace, size_t workspace_bytes, void* stream,
+                         const float* weights, int* place, int y_bf16)
 {
     if (int rc = check_matrix(hidden, 2 * inter, K, codebook)) return rc;
     if (int rc = check_matrix(inter, hidden, K, codebook)) return rc;
@@ -947,7 +947,26 @@ exl3_status exl3_moe_tc_experts(const void* x, int x_dtype, int tokens, int top_
     return launch_moe_tc_experts(x, x_dtype == EXL3_BF16, top_k, hidden, inter, topk_ids, slots, num_experts, expert_map, num_local, w13,
                                  reinterpret_cast<const __half*>(suh13), reinterpret_cast<const __half*>(svh13), w2,
                                  reinterpret_cast<const __half*>(suh2), reinterpret_cast<const __half*>(svh2), K, codebook,
-                                 reinterpret_cast<__half*>(yd), reinterpret_cast<unsigned char*>(workspace), (cudaStream_t)stream);
+                                 reinterpret_cast<__half*>(yd), reinterpret_cast<unsigned char*>(workspace), (cudaStream_t)stream, weights, place, y_bf16);
+}
+
+exl3_status exl3_moe_tc_experts(const void* x, int x_dtype, int tokens, int top_k, int hidden, int inter, const int32_t* topk_ids,
+                                int num_experts, const int32_t* expert_map, int num_local, const uint32_t* w13, const uint16_t* suh13,
+                                const uint16_t* svh13, const uint32_t* w2, const uint16_t* suh2, const uint16_t* svh2, int K, int codebook,
+                                uint16_t* yd, void* workspace, size_t workspace_bytes, void* stream)
+{
+    return moe_tc_common(x, x_dtype, tokens, top_k, hidden, inter, topk_ids, num_experts, expert_map, num_local, w13, suh13, svh13, w2, suh2, svh2, K, codebook,
+                         yd, workspace, workspace_bytes, stream, nullptr, nullptr, 0);
+}
+
+exl3_status exl3_moe_tc_layer(const void* x, int dtype, int tokens, int top_k, int hidden, int inter, const int32_t* topk_ids, const float* topk_weights,
+                              int num_experts, const int32_t* expert_map, int num_local, const uint32_t* w13, const uint16_t* suh13, const uint16_t* svh13,
+                              const uint32_t* w2, const uint16_t* suh2, const uint16_t* svh2, int K, int codebook, void* y, int32_t* place, void* workspace,
+                              size_t workspace_bytes, void* stream)
+{
+    if (tokens > 0 && (!aligned(topk_weights, 4) || !aligned(place, 4))) return EXL3_ERR_BAD_POINTER;
+    return moe_tc_common(x, dtype, tokens, top_k, hidden, inter, topk_ids, num_experts, expert_map, num_local, w13, suh13, svh13, w2, suh2, svh2, K, codebook,
+                         y, workspace, workspace_bytes, stream, topk_weights, place, dtype == EXL3_BF16);
 }
 
 /* ---- exl3_linear_static: the fused linear for callers that cannot bring a workspace ---------------------------

@@ -130,7 +130,7 @@ inline int rotated_layout(int gemv_mode) { return gemv_mode == GEMV_SPLIT ? 1 : 
 struct MoeGemmLaunch;
 int moe_init_device();
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st);
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st, int* place = nullptr);
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
                       const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st);
 int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids, const int* expert_ids,
@@ -142,6 +142,8 @@ int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half
                          const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st);
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
                          const int* num_post, const int2* blk, __half* yd, cudaStream_t st);
+int launch_moe_out_combine(const __half* yd_rot, const __half* svh2, const float* weights, const int* place, const int* expert_ids, const int2* blk, int tokens,
+                           int top_k, int hidden, void* y, int y_bf16, cudaStream_t st);
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,
                        int y_bf16, cudaStream_t st);
 
@@ -179,7 +181,7 @@ size_t moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter);
 int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int inter, const int* topk_ids, int slots, int num_experts,
                           const int* expert_map, int num_local, const uint32_t* w13, const __half* suh13, const __half* svh13,
                           const uint32_t* w2, const __half* suh2, const __half* svh2, int K, int codebook, __half* yd, unsigned char* ws,
-                          cudaStream_t st);
+                          cudaStream_t st, const float* weights = nullptr, int* place = nullptr, int y_bf16 = 0);      // weights: yd is y [tokens, hidden]
 // How launch_gemm_tc left its result: !tile_slabs: parts == 1: fp16 in `out` in the rotated basis (launch_had_out), parts > 1:
 // `parts` fp32 slabs [rows][n_total] (launch_had_out_sum); tile_slabs (the CTA-pair tiling): the 512 x 256 tiles before
 // tail_first are final in y, the others are `parts` fp32 slabs per tile (launch_had_out_tiles; row_tiles = 512-row tiles per

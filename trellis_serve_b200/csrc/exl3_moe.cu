@@ -16,14 +16,15 @@ namespace exl3 {
 // mixed-bitrate expert set gets the blocks of its own slots only, with local expert ids.
 // With `items`: every expert's rows are also cut into items of up to item_blocks blocks of eight rows; items[i] = (expert, first block,
 // blocks, 0), blk[b] = (first block of the item of block b, its blocks), num_post[1] = items, num_post[2] = rows of the largest one; and
-// the workspace's header (error word) is cleared.  Bound by latency and by shared-memory
+// the workspace's header (error word) is cleared.  place (or null): the row of every slot, -1 for dropped ones.  Bound by latency and by shared-memory
 // atomics: a CTA counts its share of the slots, reads the other CTAs' counts through distributed shared memory and lays out the experts
 // itself; KEEP slots per thread are requested together and, if that takes them all, stay in registers with their rank from the
 // counting (16384 slots, 256 experts: 24 us in one CTA with two passes of loads and atomics, 20 with one).
 template <int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ topk_ids, int numel, int E, int block, int cap, int* __restrict__ sorted_ids,
                                  int* __restrict__ expert_ids, int* __restrict__ num_post, const int* __restrict__ expert_map,
-                                 int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ header)
+                                 int E_global, int item_blocks, int4* __restrict__ items, int2* __restrict__ blk, int* __restrict__ header,
+                                 int* __restrict__ place)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
@@ -167,8 +168,13 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(1024) moe_align_ker
         if (!one) load_ids(i0);
 #pragma unroll
         for (int j = 0; j < KEEP; j++) {
-            const int e = e_of[j];
-            if (e >= 0) sorted_ids[offset[e] + (CL > 1 ? before[e] : 0) + (one ? rank[j] : atomicAdd(&fill[e], 1))] = i0 + thread + j * threads;
+            const int e = e_of[j], i = i0 + thread + j * threads;
+            int at = -1;
+            if (e >= 0) {
+                at = offset[e] + (CL > 1 ? before[e] : 0) + (one ? rank[j] : atomicAdd(&fill[e], 1));
+                sorted_ids[at] = i;
+            }
+            if (place && i < numel) place[i] = at;
         }
     }
 }
@@ -447,6 +453,87 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
     }
 }
 
+// y[t, :] = sum_j w[t, j] * fp16( Had128(yd_rot[place of slot t * top_k + j]) * svh2[its expert] ), in fp32, one rounding: moe_out_kernel and
+// moe_combine_kernel in one, without the slots' rows in memory between.  A warp takes 8 / G tokens, G rows each (top_k rounded up to a power
+// of two, at most eight; more come in rounds), four lanes per row; the rows of a token are added by exchanging halves, so that every lane ends
+// with 32 / G of the 128 columns, its own.  Traffic bounds it (2048 tokens, top-8, 2048 columns: 67 MB, 10.4 us).
+template <int G>
+__global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2,
+                                                                 const float* __restrict__ weights, const int* __restrict__ place,
+                                                                 const int* __restrict__ expert_ids, const int2* __restrict__ blk, int tokens, int top_k,
+                                                                 int hidden, void* __restrict__ y, int y_bf16)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    constexpr int N = 32 / G;
+    const int lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2, kgs = hidden >> 7, spans = (kgs + MOE_SPAN - 1) / MOE_SPAN;
+    const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), group = id / spans, kg0 = (id - group * spans) * MOE_SPAN;
+    const int t = group * (8 / G) + r / G, kg1 = kg0 + MOE_SPAN < kgs ? kg0 + MOE_SPAN : kgs;
+    if (group * (8 / G) >= tokens) return;
+    const __half *src = yd_rot, *sv = svh2;
+    long long pitch = 0;
+    float wt = 0.f;
+    bool valid = false;
+    auto look = [&](int j0) {                                     // this lane's slot of a round
+        const int j = j0 + r % G, slot = t * top_k + j, at = t < tokens && j < top_k ? place[slot] : -1;
+        valid = at >= 0;
+        src = yd_rot;
+        sv = svh2;
+        pitch = 0;
+        if (!valid) return;
+        const int b = at / MOE_BLOCK_ROWS;
+        const int2 run = blk[b];
+        wt = weights[slot];
+        src += (long long)run.x * MOE_BLOCK_ROWS * hidden + (at - run.x * MOE_BLOCK_ROWS) * 128;            // [column block][row][128]
+        pitch = (long long)run.y * MOE_BLOCK_ROWS * 128;
+        sv += (long long)expert_ids[b] * hidden;
+    };
+    look(0);
+#pragma unroll 1
+    for (int kg = kg0; kg < kg1; kg++) {
+        float sum[N] = {};
+#pragma unroll 1
+        for (int j0 = 0; j0 < top_k; j0 += G) {
+            if (top_k > G) look(j0);
+            uint32_t w[16], sw[16];
+            moe_load32<false>(src, kg * pitch, q, w);
+            moe_load32<true>(sv, kg * 128, q, sw);
+            float v[32];
+            moe_unrotate32(w, sw, lane, v);
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = valid ? v[i] * wt : 0.f;
+#pragma unroll
+            for (int m = 2 * G, n = 32; m >= 4; m >>= 1, n >>= 1) {           // lanes m apart exchange halves of n values
+                const bool upper = (lane & m) != 0;
+#pragma unroll
+                for (int i = 0; i < n / 2; i++) {
+                    const float keep = upper ? v[i + n / 2] : v[i], send = upper ? v[i] : v[i + n / 2];
+                    v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, m);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < N; i++) sum[i] += v[i];
+        }
+        if (t >= tokens) continue;
+        uint32_t o[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; i++) {
+            const __half2 h = __floats2half2_rn(sum[2 * i], sum[2 * i + 1]);
+            const __nv_bfloat162 bb = __floats2bfloat162_rn(__low2float(h), __high2float(h));
+            o[i] = y_bf16 ? *reinterpret_cast<const uint32_t*>(&bb) : *reinterpret_cast<const uint32_t*>(&h);
+        }
+        const int at = (r % G) * N;                                // of the 32 values, whose i-th is column 32 (i / 8) + 8 q + i % 8
+        uint16_t* dst = reinterpret_cast<uint16_t*>(y) + (long long)t * hidden + kg * 128 + 8 * q;
+        if constexpr (N >= 8) {
+#pragma unroll
+            for (int i = 0; i < N / 8; i++)
+                *reinterpret_cast<uint4*>(dst + 32 * (at / 8 + i)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        } else {
+            *reinterpret_cast<uint2*>(dst + 32 * (at / 8) + at % 8) = make_uint2(o[0], o[1]);
+        }
+    }
+}
+
 // y[t, :] = sum_j w[t, j] * yd[t*top_k + j, :] in fp32, slot order, one rounding; ids outside [0, E) are skipped.  V columns per
 // thread; the rows of up to eight slots are requested together (16384 slots of 2048 columns: 40 us with two columns per thread
 // and one slot at a time).
@@ -527,12 +614,12 @@ int moe_init_device()
 static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
 int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, int* sorted_ids, int* expert_ids, int* num_post,
-                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st)
+                     const int* expert_map, int E_global, int item_blocks, int4* items, int2* blk, int* header, cudaStream_t st, int* place)
 {
     // Up to two slots per thread of one CTA; more are shared by a cluster (the largest portable one).
     const bool many = numel > 2048;
     return launch_chained(many ? moe_align_kernel<8> : moe_align_kernel<1>, dim3(many ? 8 : 1), dim3(1024), (size_t)((many ? 4 : 3) * E + 1) * sizeof(int), st,
-                          topk_ids, numel, E, block, cap, sorted_ids, expert_ids, num_post, expert_map, E_global, item_blocks, items, blk, header);
+                          topk_ids, numel, E, block, cap, sorted_ids, expert_ids, num_post, expert_map, E_global, item_blocks, items, blk, header, place);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -577,6 +664,16 @@ int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, i
 {
     return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden, MOE_SPAN)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
                           num_post, blk, yd);
+}
+
+int launch_moe_out_combine(const __half* yd_rot, const __half* svh2, const float* weights, const int* place, const int* expert_ids, const int2* blk, int tokens,
+                           int top_k, int hidden, void* y, int y_bf16, cudaStream_t st)
+{
+    const int g = top_k > 4 ? 8 : top_k > 2 ? 4 : top_k;
+    auto* const kernel = g == 8 ? moe_out_combine_kernel<8> : g == 4 ? moe_out_combine_kernel<4> : g == 2 ? moe_out_combine_kernel<2> : moe_out_combine_kernel<1>;
+    const long long groups = (tokens + 8 / g - 1) / (8 / g), spans = (hidden / 128 + MOE_SPAN - 1) / MOE_SPAN;
+    return launch_chained(kernel, dim3(blocks_for(groups * spans, 8)), dim3(256), 0, st, yd_rot, svh2, weights, place, expert_ids, blk, tokens, top_k, hidden, y,
+                          y_bf16);
 }
 
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,

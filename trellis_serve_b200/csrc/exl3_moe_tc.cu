@@ -60,7 +60,7 @@ size_t moe_tc_workspace_bytes(int slots, int num_local, int hidden, int inter)
 int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int inter, const int* topk_ids, int slots, int num_experts,
                           const int* expert_map, int num_local, const uint32_t* w13, const __half* suh13, const __half* svh13,
                           const uint32_t* w2, const __half* suh2, const __half* svh2, int K, int codebook, __half* yd, unsigned char* ws,
-                          cudaStream_t st)
+                          cudaStream_t st, const float* weights, int* place, int y_bf16)
 {
     constexpr int MODE = GEMV_PAIRED;
     const MoeTcLayout w = moe_tc_layout(slots, num_local, hidden, inter);
@@ -83,7 +83,7 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
     l.rotated = 1;
 
     if (int rc = launch_moe_align(topk_ids, slots, num_local, MOE_BLOCK_ROWS, w.cap, sorted_ids, expert_ids, counts, expert_map,
-                                  expert_map ? num_experts : 0, MOE_TC_BLOCK_ROWS / MOE_BLOCK_ROWS, items, blk, l.err, st))
+                                  expert_map ? num_experts : 0, MOE_TC_BLOCK_ROWS / MOE_BLOCK_ROWS, items, blk, l.err, st, place))
         return rc;
     const long long stride = (long long)w.cap * hidden * 2;
     if (int rc = launch_moe_had_in_items(x, x_bf16, suh13, hidden, top_k, slots, w.cap, sorted_ids, expert_ids, counts, blk, ws + w.xf13, stride, st))
@@ -109,6 +109,7 @@ int launch_moe_tc_experts(const void* x, int x_bf16, int top_k, int hidden, int 
     l.n_total = hidden;
     l.shard_end_block = l.NB;
     if (int rc = launch_moe_gemm(l, K, codebook, MODE, st)) return rc;
+    if (weights) return launch_moe_out_combine(yd_rot, svh2, weights, place, expert_ids, blk, slots / top_k, top_k, hidden, yd, y_bf16, st);
     return launch_moe_out_items(yd_rot, svh2, hidden, slots, w.cap, sorted_ids, expert_ids, counts, blk, yd, st);
 }
 

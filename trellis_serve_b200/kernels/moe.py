@@ -421,6 +421,13 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
         wts = view("wts").view(torch.float32)
         wts.copy_(topk_weights.reshape(-1))
     gu, yd, ws, ws_bytes = at("gu"), at("yd"), at("gemv"), plan["gemv"][1]
+    if len(pack.packs) == 1 and "tc0" in plan and out.dtype == x.dtype and _aligned16(out):      # one class: rotated back and summed in one launch
+        pk, emap = pack.packs[0], maps[0]
+        with torch.cuda.device(dev):
+            _lib.check(lib.exl3_moe_tc_layer(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), _ptr(wts), emap.numel(), _ptr(emap),
+                                             pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2), _ptr(pk.svh2),
+                                             pk.bits, pk.codebook, _ptr(out), yd, at("tc0"), plan["tc0"][1], st), "exl3_moe_tc_layer")
+        return out
     if not pack.covers_all or expert_maps is not None:
         view("yd").zero_()                # slots of experts held elsewhere are never written and must add nothing
     with torch.cuda.device(dev):
