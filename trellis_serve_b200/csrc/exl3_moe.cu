@@ -312,23 +312,22 @@ __device__ __forceinline__ void moe_unrotate32(const uint32_t (&w)[16], const ui
     for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] * (HAD_SCALE * moe_half(sw, i))));
 }
 
-// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_turn), and up to MOE_SPAN column blocks of
-// 128 of it: 16-byte loads and full-line stores, and the chain of dependent loads (block -> expert and slot -> values) is walked once
+// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_turn), and a span of up to four column blocks
+// of 128 of it: 16-byte loads and full-line stores, and the chain of dependent loads (block -> expert and slot -> values) is walked once
 // per span -- with one column block per warp it is what bounds these kernels (70 us instead of 22 us of traffic for 2048 tokens, top-8,
-// 2048 columns).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
-constexpr int MOE_SPAN = 4, MOE_MID_SPAN = 2;
-template <int SPAN>
+// 2048 columns).  The span is halved while the warps are not enough for two full loads of the chip (span_of; a layer of 2048 tokens, 32
+// experts of 1024 x 384, top-2: 86 us with four, 76 with two, and the middle step of 2048 x 512, top-8, 8 us less with one than with two).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
 struct MoeSpan {
     int b, kg0, kg1, slot, ex;
     bool valid, any;
-    __device__ __forceinline__ MoeSpan(int kgs, int cap, int numel, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
+    __device__ __forceinline__ MoeSpan(int span, int kgs, int cap, int numel, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                        const int* __restrict__ num_post)
     {
-        const int lane = threadIdx.x & 31, spans = (kgs + SPAN - 1) / SPAN;
+        const int lane = threadIdx.x & 31, spans = (kgs + span - 1) / span;
         const int at = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
         b = at / spans;
-        kg0 = (at - b * spans) * SPAN;
-        kg1 = kg0 + SPAN < kgs ? kg0 + SPAN : kgs;
+        kg0 = (at - b * spans) * span;
+        kg1 = kg0 + span < kgs ? kg0 + span : kgs;
         any = false;
         if (b >= cap / MOE_BLOCK_ROWS) return;
         const int post = *num_post;
@@ -344,12 +343,12 @@ struct MoeSpan {
 __global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
                                                             int numel, int cap, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                                             const int* __restrict__ num_post, const int2* __restrict__ blk,
-                                                            unsigned char* __restrict__ xf, long long shard_stride)
+                                                            unsigned char* __restrict__ xf, long long shard_stride, int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3, kgs = hidden >> 7;
-    const MoeSpan<MOE_SPAN> at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan at(span, kgs, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
@@ -381,12 +380,12 @@ __global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restri
 __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restrict__ gu_rot, const __half* __restrict__ svh13,
                                                          const __half* __restrict__ suh2, int inter, int numel, int cap,
                                                          const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
-                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, unsigned char* __restrict__ xf)
+                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, unsigned char* __restrict__ xf, int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3, kgs = inter >> 7;
-    const MoeSpan<MOE_MID_SPAN> at(kgs, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan at(span, kgs, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
@@ -420,12 +419,13 @@ __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restric
 // yd[slot(row), :] = fp16( Had128(yd_rot[row]) * svh2[expert] ).
 __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
                                                          const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
-                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, __half* __restrict__ yd)
+                                                         const int* __restrict__ num_post, const int2* __restrict__ blk, __half* __restrict__ yd,
+                                                         int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     const int lane = threadIdx.x & 31, q = lane & 3;
-    const MoeSpan<MOE_SPAN> at(hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
+    const MoeSpan at(span, hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
     const int2 run = blk[at.b];
     const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
@@ -461,14 +461,14 @@ template <int G>
 __global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2,
                                                                  const float* __restrict__ weights, const int* __restrict__ place,
                                                                  const int* __restrict__ expert_ids, const int2* __restrict__ blk, int tokens, int top_k,
-                                                                 int hidden, void* __restrict__ y, int y_bf16)
+                                                                 int hidden, void* __restrict__ y, int y_bf16, int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     constexpr int N = 32 / G;
-    const int lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2, kgs = hidden >> 7, spans = (kgs + MOE_SPAN - 1) / MOE_SPAN;
-    const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), group = id / spans, kg0 = (id - group * spans) * MOE_SPAN;
-    const int t = group * (8 / G) + r / G, kg1 = kg0 + MOE_SPAN < kgs ? kg0 + MOE_SPAN : kgs;
+    const int lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2, kgs = hidden >> 7, spans = (kgs + span - 1) / span;
+    const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), group = id / spans, kg0 = (id - group * spans) * span;
+    const int t = group * (8 / G) + r / G, kg1 = kg0 + span < kgs ? kg0 + span : kgs;
     if (group * (8 / G) >= tokens) return;
     const __half *src = yd_rot, *sv = svh2;
     long long pitch = 0;
@@ -624,10 +624,17 @@ int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, 
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-static unsigned span_blocks(int cap, int cols, int span)      // CTAs of eight warps, a warp per (block of eight rows, span)
+// Column blocks per warp for `groups` groups of eight rows, and the CTAs of eight warps that this takes: up to four, as long as the warps fill the
+// chip (24 per SM) twice.
+static int span_of(long long groups, int cols)
 {
-    return blocks_for((long long)(cap / MOE_BLOCK_ROWS) * ((cols / 128 + span - 1) / span), 8);
+    const DeviceInfo* d = current_device_info();
+    const long long enough = 2 * 24 * (long long)(d ? d->sm_count : 148);
+    int span = 4;
+    while (span > 1 && groups * ((cols / 128 + span - 1) / span) < enough) span /= 2;
+    return span;
 }
+static unsigned span_blocks(long long groups, int cols, int span) { return blocks_for(groups * ((cols / 128 + span - 1) / span), 8); }
 
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
                       const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st)
@@ -648,22 +655,25 @@ int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int n
 int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
                             const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st)
 {
-    return launch_chained(moe_had_in_kernel, dim3(span_blocks(cap, hidden, MOE_SPAN), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
-                          expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride);
+    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(2 * groups, hidden);
+    return launch_chained(moe_had_in_kernel, dim3(span_blocks(groups, hidden, span), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
+                          expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride, span);
 }
 
 int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half* suh2, int inter, int numel, int cap, const int* sorted_ids,
                          const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st)
 {
-    return launch_chained(moe_mid_kernel, dim3(span_blocks(cap, inter, MOE_MID_SPAN)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
-                          num_post, blk, reinterpret_cast<unsigned char*>(xf));
+    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(groups, inter);
+    return launch_chained(moe_mid_kernel, dim3(span_blocks(groups, inter, span)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
+                          num_post, blk, reinterpret_cast<unsigned char*>(xf), span);
 }
 
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
                          const int* num_post, const int2* blk, __half* yd, cudaStream_t st)
 {
-    return launch_chained(moe_out_kernel, dim3(span_blocks(cap, hidden, MOE_SPAN)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
-                          num_post, blk, yd);
+    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(groups, hidden);
+    return launch_chained(moe_out_kernel, dim3(span_blocks(groups, hidden, span)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
+                          num_post, blk, yd, span);
 }
 
 int launch_moe_out_combine(const __half* yd_rot, const __half* svh2, const float* weights, const int* place, const int* expert_ids, const int2* blk, int tokens,
@@ -671,9 +681,9 @@ int launch_moe_out_combine(const __half* yd_rot, const __half* svh2, const float
 {
     const int g = top_k > 4 ? 8 : top_k > 2 ? 4 : top_k;
     auto* const kernel = g == 8 ? moe_out_combine_kernel<8> : g == 4 ? moe_out_combine_kernel<4> : g == 2 ? moe_out_combine_kernel<2> : moe_out_combine_kernel<1>;
-    const long long groups = (tokens + 8 / g - 1) / (8 / g), spans = (hidden / 128 + MOE_SPAN - 1) / MOE_SPAN;
-    return launch_chained(kernel, dim3(blocks_for(groups * spans, 8)), dim3(256), 0, st, yd_rot, svh2, weights, place, expert_ids, blk, tokens, top_k, hidden, y,
-                          y_bf16);
+    const int groups = (tokens + 8 / g - 1) / (8 / g), span = span_of(groups, hidden);
+    return launch_chained(kernel, dim3(span_blocks(groups, hidden, span)), dim3(256), 0, st, yd_rot, svh2, weights, place, expert_ids, blk, tokens, top_k, hidden,
+                          y, y_bf16, span);
 }
 
 int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, int tokens, int top_k, int hidden, int E, void* y,
