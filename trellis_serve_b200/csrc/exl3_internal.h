@@ -31,8 +31,9 @@ struct RepackGroup {
     uint16_t *suh_cat, *svh_cat;
     int nb_end[REPACK_MATRICES];               // column blocks up to and including each matrix
     int matrices, KG;
+    int pieces;                                // launch_repack: CTAs per row block
 };
-int launch_repack(const RepackGroup& g, int K, uint32_t* packed, cudaStream_t st);
+int launch_repack(RepackGroup g, int K, uint32_t* packed, cudaStream_t st);
 int launch_unpack(const uint32_t* packed, int k, int n, int K, uint16_t* trellis, cudaStream_t st);
 int launch_reconstruct_stored(const uint16_t* trellis, int kt, int nt, int K, int cb, __half* w, cudaStream_t st);
 int launch_reconstruct_packed(const uint32_t* packed, int k, int n, int K, int cb, __half* w, cudaStream_t st);

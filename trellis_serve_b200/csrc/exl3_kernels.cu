@@ -13,20 +13,26 @@ namespace exl3 {
 // ------------------------------------------------------------------------------------------------ repack
 
 // The permutation is one of bytes: a lane's share of a tile is K whole bytes of the tile's stream (big-endian inside each
-// little-endian 32-bit word), so the lane stream of four tiles is four runs of K bytes.  One CTA per (column block, row block)
-// unit, warp nt = its column tile: the unit's eight tile rows (256K contiguous bytes each) are brought into shared memory with
-// 16-byte loads, a lane cuts its K bytes out of each tile with funnel shifts of whole stream words and joins four of them into
-// its K resident words, stored as full 128-byte lines.  Bound by DRAM: one matrix of the 27B shape's gate|up (K = 3, 33 MB
-// in, 33 MB out) takes 15.7 us = 4.3 TB/s; one thread per output word that fetched its 32 bits one by one took 420 us.
+// little-endian 32-bit word), so the lane stream of four tiles is four runs of K bytes.  One CTA per row block and up to two
+// neighbouring column blocks of a matrix (units), warp nt = its column tile: their eight tile rows (256K contiguous bytes per unit each) are
+// brought into shared memory with 16-byte loads, K per thread and all in flight together, a lane cuts its K bytes out of each tile with
+// funnel shifts of whole stream words and joins four of them into its K resident words, stored as full 128-byte lines.  Bound by DRAM: the
+// 27B shape's gate|up (K = 3, 67 MB in, 67 MB out) takes 25.0 us = 5.3 TB/s, with one unit per CTA 31.1; one thread per output word that
+// fetched its 32 bits one by one took 15 times as long.
 // A whole group is one launch: the CTAs behind the units copy the matrices' sign and scale vectors side by side.
+// At K = 8 one unit is 16 KB and enough in flight (31.1 us for 5120 x 17408, 36.2 with two).
+constexpr int repack_units(int K) { return K < 8 ? 2 : 1; }
 template <int K>
 __global__ void __launch_bounds__(256) repack_kernel(const __grid_constant__ RepackGroup g, uint32_t* __restrict__ packed)
 {
     constexpr int TILE_WORDS = 8 * K, ROW_WORDS = 8 * TILE_WORDS;            // words of a tile, of a row of eight tiles
-    __shared__ __align__(16) uint32_t sm[8 * ROW_WORDS];
-    const int KG = g.KG, units = KG * g.nb_end[g.matrices - 1];
-    if ((int)blockIdx.x >= units) {
-        const long long first = (long long)((int)blockIdx.x - units) * REPACK_COPY;
+    constexpr int REPACK_UNITS = repack_units(K);
+    constexpr int SPAN = REPACK_UNITS * ROW_WORDS / 4, LOADS = 8 * SPAN / 256;       // 16-byte words of a row of the units; of a thread
+    static_assert(LOADS * 256 == 8 * SPAN, "every thread loads as much");
+    __shared__ __align__(16) uint32_t sm[8 * REPACK_UNITS * ROW_WORDS];      // [tile row][unit]
+    const int KG = g.KG;
+    if ((int)blockIdx.x >= KG * g.pieces) {
+        const long long first = (long long)((int)blockIdx.x - KG * g.pieces) * REPACK_COPY;
         for (int i = threadIdx.x; i < REPACK_COPY; i += 256) {
             const long long at = first + i, suh_all = (long long)g.matrices * KG * 128;
             if (at < suh_all) {
@@ -41,27 +47,41 @@ __global__ void __launch_bounds__(256) repack_kernel(const __grid_constant__ Rep
         }
         return;
     }
-    const int kg = blockIdx.x % KG, all_nb = blockIdx.x / KG;
-    int m = 0;
-    while (all_nb >= g.nb_end[m]) m++;
-    const int nb0 = m > 0 ? g.nb_end[m - 1] : 0, NB = g.nb_end[m] - nb0, nb = all_nb - nb0;
+    const int kg = blockIdx.x % KG;
+    int m = 0, piece = blockIdx.x / KG, nb0 = 0, NB = g.nb_end[0];
+    while (piece >= (NB + REPACK_UNITS - 1) / REPACK_UNITS) {
+        piece -= (NB + REPACK_UNITS - 1) / REPACK_UNITS;
+        nb0 = g.nb_end[m++];
+        NB = g.nb_end[m] - nb0;
+    }
+    const int nb = piece * REPACK_UNITS, here = NB - nb < REPACK_UNITS ? NB - nb : REPACK_UNITS;
     const uint16_t* trellis = g.trellis[m];
     const bool vec = reinterpret_cast<uintptr_t>(trellis) % 16 == 0;
-    // row tile r of the unit: ROW_WORDS consecutive words; 16 K chunks of 16 bytes each
+    // row tile r of the units: `here` x ROW_WORDS consecutive words
     const uint4* src = reinterpret_cast<const uint4*>(trellis) + ((long long)kg * 8 * NB + nb) * (ROW_WORDS / 4);
     if (vec) {
-        for (int c = threadIdx.x; c < 8 * (ROW_WORDS / 4); c += 256) {
-            const int r = c / (ROW_WORDS / 4), o = c % (ROW_WORDS / 4);
-            reinterpret_cast<uint4*>(sm)[c] = __ldcs(src + (long long)r * NB * (ROW_WORDS / 4) + o);
+        uint4 v[LOADS];
+#pragma unroll
+        for (int i = 0; i < LOADS; i++) {
+            const int c = threadIdx.x + i * 256, r = c / SPAN, o = c % SPAN;
+            if (o < here * (ROW_WORDS / 4)) v[i] = __ldg(src + (long long)r * NB * (ROW_WORDS / 4) + o);
+        }
+#pragma unroll
+        for (int i = 0; i < LOADS; i++) {
+            const int c = threadIdx.x + i * 256;
+            if (c % SPAN < here * (ROW_WORDS / 4)) reinterpret_cast<uint4*>(sm)[c] = v[i];
         }
     } else {                                                                  // a checkpoint view that starts between 16-byte boundaries
         const uint32_t* src4 = reinterpret_cast<const uint32_t*>(src);
-        for (int c = threadIdx.x; c < 8 * ROW_WORDS; c += 256) sm[c] = __ldcs(src4 + (long long)(c / ROW_WORDS) * NB * ROW_WORDS + c % ROW_WORDS);
+        for (int c = threadIdx.x; c < 8 * 4 * SPAN; c += 256)
+            if (c % (4 * SPAN) < here * ROW_WORDS) sm[c] = __ldcs(src4 + (long long)(c / (4 * SPAN)) * NB * ROW_WORDS + c % (4 * SPAN));
     }
     __syncthreads();
     const int nt = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int word = (K * lane) >> 2, sh = ((K * lane) & 3) * 8;              // where the lane's bytes start in a tile's stream
-    uint32_t* dst = packed + ((((long long)all_nb * KG + kg) * 8 + nt) * 2) * K * 32 + lane;
+    uint32_t* dst = packed + ((((long long)(nb0 + nb) * KG + kg) * 8 + nt) * 2) * K * 32 + lane;
+#pragma unroll 1
+    for (int unit = 0; unit < here; unit++, dst += (long long)KG * 512 * K)
 #pragma unroll
     for (int kq = 0; kq < 2; kq++) {
         uint32_t out[K];
@@ -69,7 +89,7 @@ __global__ void __launch_bounds__(256) repack_kernel(const __grid_constant__ Rep
         for (int i = 0; i < K; i++) out[i] = 0;
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            const uint32_t* tw = sm + (kq * 4 + t) * ROW_WORDS + nt * TILE_WORDS;
+            const uint32_t* tw = sm + ((kq * 4 + t) * REPACK_UNITS + unit) * ROW_WORDS + nt * TILE_WORDS;
             constexpr int N = (K + 3) / 4;                                    // shifted words that hold the K bytes, left-aligned
             uint32_t w[N + 1];
 #pragma unroll
@@ -394,14 +414,17 @@ __global__ void had_out_sum_kernel(const float* __restrict__ part, int parts, lo
 
 static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
-int launch_repack(const RepackGroup& g, int K, uint32_t* packed, cudaStream_t st)
+int launch_repack(RepackGroup g, int K, uint32_t* packed, cudaStream_t st)
 {
     const long long NB = g.nb_end[g.matrices - 1], units = g.KG * NB, copies = g.suh_cat ? 128ll * g.KG * g.matrices + 128 * NB : 0;
     if (units == 0) return EXL3_OK;
+    g.pieces = 0;
+    const int per = repack_units(K);
+    for (int m = 0; m < g.matrices; m++) g.pieces += (g.nb_end[m] - (m > 0 ? g.nb_end[m - 1] : 0) + per - 1) / per;
     if (units + copies >= (1ll << 31)) return EXL3_ERR_BAD_SHAPE;
     auto kernel = K == 2 ? repack_kernel<2> : K == 3 ? repack_kernel<3> : K == 4 ? repack_kernel<4> : K == 5 ? repack_kernel<5>
                 : K == 6 ? repack_kernel<6> : K == 7 ? repack_kernel<7> : repack_kernel<8>;
-    kernel<<<(unsigned)units + blocks_for(copies, REPACK_COPY), 256, 0, st>>>(g, packed);
+    kernel<<<(unsigned)(g.KG * g.pieces) + blocks_for(copies, REPACK_COPY), 256, 0, st>>>(g, packed);
     return cuda_status(cudaGetLastError());
 }
 
