@@ -150,7 +150,7 @@ exl3_status exl3_linear_prerotated(const uint32_t *packed, int K, int codebook, 
  * (no exchange, up to two rows).  exl3_normed_linear is the consumer: the fused group on rmsnorm(z) * norm_weight, where z is
  * such a stream and ssq its sums of squares; up to two rows the GEMV normalises on the way into its own rotation, so a
  * transformer block is four launches plus attention.  exl3_residual_ssq starts a chain (z = x + residual_in, or x itself, and
- * its sums of squares); exl3_rmsnorm_linear = exl3_residual_ssq + exl3_normed_linear for a caller without a producer.
+ * its sums of squares), exl3_normed ends one (out = rmsnorm(z) * weight from z and its sums of squares, in fp32, one rounding); exl3_rmsnorm_linear = exl3_residual_ssq + exl3_normed_linear for a caller without a producer.
  * From three rows up the library runs its normalisation / stream kernels around a plain GEMV (y must then be given).
  * The reference's engine runs residual add and RMSNorm as kernels of its own ahead of had_in; no counterpart there. */
 exl3_status exl3_glu_linear(const void *gate_up, int x_dtype, const uint32_t *packed, int K, int codebook, const uint16_t *suh,
@@ -158,6 +158,7 @@ exl3_status exl3_glu_linear(const void *gate_up, int x_dtype, const uint32_t *pa
                             int y_dtype, void *workspace, size_t workspace_bytes, void *const *peer_regions, int rank, int world,
                             size_t max_elems, int *state, const void *residual_in, void *residual_out, float *ssq_out,
                             void *stream);
+exl3_status exl3_normed(const void *z, int dtype, const float *ssq, const void *weight, float eps, int rows, int k, void *out, void *stream);
 exl3_status exl3_residual_ssq(const void *x, const void *residual_in, int dtype, int rows, int k, void *residual_out, float *ssq,
                               void *stream);
 exl3_status exl3_normed_linear(const void *z, int x_dtype, const float *ssq, const void *norm_weight, float eps,

@@ -328,3 +328,19 @@ def test_decode_attention_against_float64(dtype, rows, q_heads, kv_heads, t_max,
     want = (torch.softmax(q @ k.transpose(-1, -2) * scale, dim=-1) @ v).view(rows, q_heads * 128)
     half_ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
     assert bool(((out.double() - want).abs() <= want.abs() * half_ulp + 2e-5 * want.abs().max()).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,k", [(1, 128), (3, 5120), (2, 4224)])
+def test_end_of_the_residual_chain(dtype, rows, k):
+    """exl3_normed against float64: one rounding of an fp32 product of three factors (a few 2^-24)."""
+    gen = torch.Generator(device=DEV).manual_seed(rows + k)
+    z = torch.randn((rows, k), device=DEV, generator=gen).to(dtype)
+    weight = (1.0 + 0.1 * torch.randn(k, device=DEV, generator=gen)).to(dtype)
+    ssq, out = torch.empty((rows, k // 128), dtype=torch.float32, device=DEV), torch.empty_like(z)
+    lin.residual_ssq(z, None, None, ssq)
+    lin.normed(z, ssq, weight, 1e-6, out)
+    torch.cuda.synchronize()
+    want = z.double() / (z.double().pow(2).mean(1, keepdim=True) + 1e-6).sqrt() * weight.double()
+    half_ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert bool(((out.double() - want).abs() <= want.abs() * (half_ulp + 2.0 ** -21) + 2.0 ** -25).all())

@@ -46,6 +46,7 @@ SIGNATURES = {
                                     _vp]),
     "exl3_rmsnorm_linear": (_i, [_vp, _i, _vp, _vp, _vp, ctypes.c_float, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_residual_ssq": (_i, [_vp, _vp, _i, _i, _i, _vp, _vp, _vp]),
+    "exl3_normed": (_i, [_vp, _i, _vp, _vp, ctypes.c_float, _i, _i, _vp, _vp]),
     "exl3_normed_linear": (_i, [_vp, _i, _vp, _vp, ctypes.c_float, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, _vp]),
     "exl3_glu_linear": (_i, [_vp, _i, _vp, _i, _i, _vp, _vp, _ip, _i, _i, _i, _i, _vp, _i, _vp, _sz, ctypes.POINTER(_vp), _i, _i, _sz, _vp, _vp, _vp, _vp,
                              _vp]),

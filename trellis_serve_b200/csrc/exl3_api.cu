@@ -568,6 +568,15 @@ exl3_status exl3_residual_ssq(const void* x, const void* residual_in, int dtype,
     return launch_residual_ssq(x, residual_in, dtype == EXL3_BF16, rows, k, residual_out, ssq, (cudaStream_t)stream);
 }
 
+exl3_status exl3_normed(const void* z, int dtype, const float* ssq, const void* weight, float eps, int rows, int k, void* out, void* stream)
+{
+    if (dtype != EXL3_F16 && dtype != EXL3_BF16) return EXL3_ERR_UNSUPPORTED_DTYPE;
+    if (rows < 0 || k <= 0 || k % 128) return EXL3_ERR_BAD_SHAPE;
+    if (rows == 0) return EXL3_OK;
+    if (!aligned(z, 8) || !aligned(weight, 8) || !aligned(out, 8) || !aligned(ssq, 4)) return EXL3_ERR_BAD_POINTER;
+    return launch_normed(z, ssq, weight, eps, dtype == EXL3_BF16, rows, k, out, (cudaStream_t)stream);
+}
+
 exl3_status exl3_normed_linear(const void* z, int x_dtype, const float* ssq, const void* norm_weight, float eps, const uint32_t* packed, int K,
                                int codebook, const uint16_t* suh_cat, const uint16_t* svh_cat, const int* shard_ends, int n_shards, int rows,
                                int k, int n_total, void* y, int y_dtype, void* workspace, size_t workspace_bytes, void* stream)

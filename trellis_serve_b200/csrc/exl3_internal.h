@@ -151,6 +151,7 @@ int launch_moe_combine(const __half* yd, const float* w, const int* topk_ids, in
 // exl3_step.cu ------------------------------------------------------------------------------------------
 int launch_rmsnorm_rotate(const void* x, void* residual, const void* weight, float eps, int bf16, const __half* suh, int shards, int rows,
                           int k, void* normed, uint32_t* xf, int mode, cudaStream_t st, void* residual_out = nullptr);
+int launch_normed(const void* z, const float* ssq, const void* weight, float eps, int bf16, int rows, int k, void* out, cudaStream_t st);
 int launch_residual_ssq(const void* x, const void* res_in, int bf16, int rows, int k, void* res_out, float* ssq, cudaStream_t st);
 int launch_silu_mul_rotate(const void* gu, int bf16, const __half* suh, int rows, int inter, void* act, uint32_t* xf, int mode,
                            cudaStream_t st);

@@ -198,6 +198,37 @@ __global__ void residual_ssq_kernel(const void* __restrict__ x, const void* __re
     if (lane == 0) ssq[item] = ss;
 }
 
+// out = z * rsqrt(mean square + eps) * weight, one warp per (row, 128 columns), the mean square from the sums in ssq [rows, k / 128]: the end
+// of a chain of residual blocks.  Latency bounds it (5 elementwise and normalisation launches of a framework in its place took 11 us).
+__global__ void normed_kernel(const void* __restrict__ z, const float* __restrict__ ssq, const void* __restrict__ weight, float eps, int bf16, int rows, int k,
+                              void* __restrict__ out)
+{
+    ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    const int lane = threadIdx.x & 31, kgs = k >> 7;
+    const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (item >= (long long)rows * kgs) return;
+    const bool b = bf16 != 0;
+    const int col = (int)(item % kgs) * 128 + 4 * lane;
+    float v[4], w[4], sum = 0.f;
+    load_act4(z, (item / kgs) * k + col, b, v);
+    load_act4(weight, col, b, w);
+    for (int i = lane; i < kgs; i += 32) sum += ssq[(item / kgs) * kgs + i];
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, m);
+    const float rstd = rsqrtf(sum / (float)k + eps);
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = v[e] * rstd * w[e];
+    store_act4(out, (item / kgs) * k + col, v, b);
+}
+
+int launch_normed(const void* z, const float* ssq, const void* weight, float eps, int bf16, int rows, int k, void* out, cudaStream_t st)
+{
+    const long long items = (long long)rows * (k / 128);
+    if (items == 0) return EXL3_OK;
+    return launch_chained(normed_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, st, z, ssq, weight, eps, bf16, rows, k, out);
+}
+
 int launch_residual_ssq(const void* x, const void* res_in, int bf16, int rows, int k, void* res_out, float* ssq, cudaStream_t st)
 {
     const long long items = (long long)rows * (k / 128);

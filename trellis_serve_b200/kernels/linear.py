@@ -349,6 +349,16 @@ def residual_ssq(x: torch.Tensor, residual_in: torch.Tensor | None, residual_out
                                                  _stream(x.device)), "exl3_residual_ssq")
 
 
+def normed(z: torch.Tensor, ssq: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor) -> torch.Tensor:
+    """out = rmsnorm(z) * weight, in fp32 and rounded once, with the sums of squares of z per 128 columns that a linear's residual epilogue
+    (or `residual_ssq`) left in ssq: the end of such a chain."""
+    _require_cuda(z, "z")
+    rows, k = z.shape
+    with torch.cuda.device(z.device):
+        _lib.check(_lib.load().exl3_normed(_ptr(z), _dtype_code(z), _ptr(ssq), _ptr(weight), float(eps), rows, k, _ptr(out), _stream(z.device)), "exl3_normed")
+    return out
+
+
 def run_normed(z: torch.Tensor, ssq: torch.Tensor, weight: torch.Tensor, eps: float, b: torch.Tensor, suh_cat: torch.Tensor,
                svh_cat: torch.Tensor, shard_ends: list[int], codebook: int, out: torch.Tensor, workspace: torch.Tensor | None = None) -> torch.Tensor:
     """The fused group on rmsnorm(z) * weight, z a residual stream and ssq its sums of squares per 128 columns (from a linear's

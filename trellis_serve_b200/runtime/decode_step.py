@@ -122,7 +122,7 @@ class DecodeStep:
         self.graph: torch.cuda.CUDAGraph | None = None
         self.linear_launches = s.layers * 4
         small = 0 if rows <= 2 else 5                                 # normalisation x2, activation and stream x2 kernels: only from three rows up
-        self.fused_launches = 1 + s.layers * ((0 if attention == "library" else 1) + small)   # the stream's start (+ rotation ahead of o with stock attention)
+        self.fused_launches = 2 + s.layers * ((0 if attention == "library" else 1) + small)   # the stream's start and end (+ rotation ahead of o with stock attention)
         self.attention_launches = s.layers if attention == "library" else None   # RoPE, append, attention and merge in one
 
     # ---- bytes
@@ -193,8 +193,7 @@ class DecodeStep:
                 lin.run_glu(self.gu, down.packed, down.suh, down.svh, cb, self.h, ws)
                 self._reduce(self.h)
                 lin.residual_ssq(self.h, z2, z, ssq)
-        self.out.copy_(torch.nn.functional.rms_norm(z.float(), (self.shape.hidden,), self.final_norm.float(), self.shape.eps).to(self.dtype))
-        return self.out
+        return lin.normed(z, ssq, self.final_norm, self.shape.eps, self.out)
 
     def capture(self, warmup: int = 2) -> None:
         side = torch.cuda.Stream(device=self.device)
