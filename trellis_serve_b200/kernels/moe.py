@@ -144,6 +144,7 @@ class MixedPack:
     codebook: int
     expert_ids: list[torch.Tensor] = field(default_factory=list)    # int32 [E_c] per class: local id -> global id
     covers_all: bool = True             # False: some experts belong to no class (another rank holds them)
+    identity: bool = False              # one class whose map is 0, 1, ..: kernels need not look ids up
 
     def __post_init__(self):
         if not self.expert_ids:
@@ -175,7 +176,8 @@ def prepare_mixed(gate, up, down, codebook: int, experts=None) -> MixedPack:
         m = torch.full((e,), -1, dtype=torch.int32)
         m[ids] = torch.arange(len(ids), dtype=torch.int32)
         maps.append(m.to(packs[-1].w13.device))
-    return MixedPack(packs, maps, e, packs[0].hidden, packs[0].inter, codebook, covers_all=len(keep) == e)
+    return MixedPack(packs, maps, e, packs[0].hidden, packs[0].inter, codebook, covers_all=len(keep) == e,
+                     identity=len(classes) == 1 and len(keep) == e)
 
 
 def expert_partition(num_experts: int, rank: int, world: int) -> range:
@@ -401,6 +403,7 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
         return out
     dev, st = x.device, _stream(x.device)
     maps = expert_maps if expert_maps is not None else pack.expert_maps
+    lookup = [None] if expert_maps is None and pack.identity else maps           # for the calls that take ids as they are
     plan, need = _plan([p.num_experts for p in pack.packs], hidden, inter, pack.codebook, tokens, top_k)
     if need > workspace.numel():
         raise RuntimeError(f"MoE workspace holds {workspace.numel()} bytes, this call needs {need}")
@@ -424,26 +427,26 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
     if len(pack.packs) == 1 and "tc0" in plan and out.dtype == x.dtype and _aligned16(out):      # one class: rotated back and summed in one launch
         pk, emap = pack.packs[0], maps[0]
         with torch.cuda.device(dev):
-            _lib.check(lib.exl3_moe_tc_layer(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), _ptr(wts), emap.numel(), _ptr(emap),
+            _lib.check(lib.exl3_moe_tc_layer(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), _ptr(wts), emap.numel(), _ptr(lookup[0]),
                                              pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2), _ptr(pk.svh2),
                                              pk.bits, pk.codebook, _ptr(out), yd, at("tc0"), plan["tc0"][1], st), "exl3_moe_tc_layer")
         return out
     if not pack.covers_all or expert_maps is not None:
         view("yd").zero_()                # slots of experts held elsewhere are never written and must add nothing
     with torch.cuda.device(dev):
-        for c, (pk, emap) in enumerate(zip(pack.packs, maps)):
+        for c, (pk, emap, given) in enumerate(zip(pack.packs, maps, lookup)):
             sorted_ids, expert_ids, num_post = at(f"sorted{c}"), at(f"experts{c}"), at(f"post{c}")
             xf13, xf2 = at(f"xf13_{c}"), at(f"xf2_{c}")
             cap = plan[f"sorted{c}"][1] // 4
             K = pk.bits
             if f"tc{c}" in plan:
-                _lib.check(lib.exl3_moe_tc_experts(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
+                _lib.check(lib.exl3_moe_tc_experts(_ptr(x), _dtype_code(x), tokens, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(given),
                                                    pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
                                                    _ptr(pk.svh2), K, pk.codebook, yd, at(f"tc{c}"), plan[f"tc{c}"][1], st), "exl3_moe_tc_experts")
                 continue
             if (lib.exl3_moe_prefers_slots(slots, pk.num_experts, hidden, inter, K, pk.codebook)
                     and _aligned16(x, pk.w13, pk.w2, pk.suh13, pk.suh2)):
-                _lib.check(lib.exl3_moe_slots_experts(_ptr(x), _dtype_code(x), slots, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(emap),
+                _lib.check(lib.exl3_moe_slots_experts(_ptr(x), _dtype_code(x), slots, top_k, hidden, inter, _ptr(ids32), emap.numel(), _ptr(given),
                                                       pk.num_experts, _ptr(pk.w13), _ptr(pk.suh13), _ptr(pk.svh13), _ptr(pk.w2), _ptr(pk.suh2),
                                                       _ptr(pk.svh2), K, pk.codebook, gu, yd, ws, ws_bytes, st), "exl3_moe_slots_experts")
                 continue
