@@ -262,13 +262,11 @@ def run_moe(args) -> None:
     if args.moe_path != "auto":           # measurement knob: force one path to find the crossover
         moe.TC_ROWS_PER_EXPERT = 0 if args.moe_path == "tc" else 1 << 30
     tensor_core = moe.moe_block_size(T, top_k, E) == 128
-    if tensor_core:
-        # many rows per expert: the allocation-free layer entry, which sends the class through the kernels for long items
-        mixed = moe.MixedPack([pack], [torch.arange(E, dtype=torch.int32, device=dev)], E, H, I, cb)
-        ws = torch.zeros(moe.layer_workspace_bytes([E], H, I, cb, T, top_k), dtype=torch.uint8, device=dev)
-        layer = lambda: moe.run_layer(x, wts, ids, mixed, out, ws)
-    else:
-        layer = lambda: moe.forward(x, wts, ids, pack, out=out)
+    slots = not tensor_core and args.moe_path == "auto" and bool(_lib.load().exl3_moe_prefers_slots(T * top_k, E, H, I, K, cb))
+    # The allocation-free layer entry; --moe-path gemv: the aligned form whatever the batch.
+    mixed = moe.MixedPack([pack], [torch.arange(E, dtype=torch.int32, device=dev)], E, H, I, cb, identity=True)
+    ws = torch.zeros(moe.layer_workspace_bytes([E], H, I, cb, T, top_k), dtype=torch.uint8, device=dev)
+    layer = (lambda: moe.forward(x, wts, ids, pack, out=out)) if args.moe_path == "gemv" else (lambda: moe.run_layer(x, wts, ids, mixed, out, ws))
     for _ in range(args.warmup):
         layer()
     torch.cuda.synchronize()
@@ -294,14 +292,15 @@ def run_moe(args) -> None:
                       "dtype": "f16", "data": "synthetic",
                       "config": {"workload": f"MoE layer hidden 2048, 256 experts, intermediate 512, top-8, K=3 3INST, {T} tokens",
                                  "tokens": T, "distinct_experts": distinct, "touched_bytes": nbytes,
-                                 "path": "items of up to 128 rows of an expert" if tensor_core else "blocks of eight rows",
+                                 "path": "items of up to 128 rows of an expert" if tensor_core else "a row and a matrix per slot" if slots else "blocks of eight rows",
                                  "tflops": 2.0 * T * top_k * 3 * H * I / ms / 1e9,
                                  "l2": "touched experts' weights larger than L2, no flush" if nbytes > 126e6
                                  else "touched experts' weights stay in L2 between replays"},
                       "roofline": {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": None,
-                                   "peak_source": f"of {kind}", "kernel": "moe_gemm_kernel"},
-                      # align, input rotation, gate|up, activation, down, combine; with long items an output rotation before the combine
-                      "gpu_launches": (7 if tensor_core else 6) * args.steps, "clocks": clocks.summary()}))
+                                   "peak_source": f"of {kind}", "kernel": "skinny_kernel" if slots else "moe_gemm_kernel"},
+                      # align, input rotation, gate|up, activation, down, combine (with long items the output rotation is part of it); gate|up,
+                      # down, combine for a few slots
+                      "gpu_launches": (3 if slots else 6) * args.steps, "clocks": clocks.summary()}))
 
 
 def _graph_ring_time(run_one, ring: int, reps: int = 5) -> float:

@@ -672,15 +672,9 @@ static size_t tc_up(size_t v) { return (v + 255) & ~(size_t)255; }
 // The decode kernel up to the 64 rows that one pass over the weights serves, whatever the sizes.  It is the more exact of the two
 // (weights as two exact summands, fp32 sums to the end; the tensor-core kernel rounds weights and rotated product to fp16), and the
 // faster one for large groups.  For small ones it is not, from 17 to 33 rows on: the line stays at 64 for the results' sake.  Chained
-// graph launches, K = 3, microseconds, decode kernel / tensor-core kernel (K = 4 and 8 within 8 %):
-//     rows             17           33           64           65           96
-//     17408 x 5120     35.0 / 43.5  41.9 / 45.2  44.5 / 48.4  71.0 / 48.6  84 / 51
-//     5120 x 34816     58.8 / 75.8  72.5 / 77.5  78.3 / 78.6  126 / 78.6   144 / 80.5
-//     5120 x 7168      22.5 / 23.0  26.4 / 24.7  28.4 / 26.6  42.7 / 26.9  54.7 / 28.8
-//     5120 x 5120      -            24.3 / 22.0  26.1 / 24.4  37.3 / 24.4  51.4 / 27.0
-//     2048 x 1024      -            16.4 / 11.4  20.3 / 12.6  27.2 / 12.7  38.4 / 13.9
-//     1024 x 640       -            13.0 / 8.9   14.5 / 9.5   19.8 / 9.7   27.6 / 10.3
-// From 65 rows up the decode kernel passes twice and loses at every size.
+// graph launches of 64 rows, K = 3, microseconds, decode kernel / tensor-core kernel: 17408 x 5120 42.5 / 48.4, 5120 x 34816 66 / 78.6, 5120 x
+// 5120 23.9 / 24.4, 2048 x 1024 18.0 / 12.6, 1024 x 640 12.9 / 9.5.  From 65 rows up the decode kernel passes twice and loses at every
+// size (17408 x 5120 71 / 48.6, 5120 x 5120 37 / 24.4).
 int exl3_prefers_decode(int rows, int k, int n_total, int sms)
 {
     (void)k;                     // part of the interface, not of today's rule

@@ -9,7 +9,7 @@
 //
 // The machinery of the dense decode GEMV (exl3_skinny_kernel.cuh): decoded registers go to tensor memory as the A operand, the rotated
 // rows are the B operand (N = rows of the item), persistent CTAs split the unit list (item, column block, row block) evenly and
-// contiguously, partial sums of column blocks cut between CTAs are added in CTA order by the last one to arrive.  Two forms:
+// contiguously, or by whole column blocks, partial sums of column blocks cut between CTAs are added in CTA order by the last one to arrive.  Two forms:
 //
 //   * blocks of eight rows (decode batches): the dense kernel, but for the item list that is read on the device (CUDA-graph safe), the
 //     expert's svh and the scattering of rows to their slots;

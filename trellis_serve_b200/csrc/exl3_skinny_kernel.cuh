@@ -2,9 +2,10 @@
 // W_inner decoded on the fly from the resident trellis.  The B200 counterpart of the reference's fused dense kernel
 // (cuda/csrc/exl3_marlin.cu:489-527 -> cuda/csrc/exl3_marlin_template.h:271 of 0xSero/trellis-serve), built around the hardware:
 //
-//   * persistent grid, one CTA per SM; the (column block, row block) units of the matrix are split evenly and contiguously over the
-//     CTAs ("stream-K"), so every CTA streams ONE contiguous byte range of the weights, in stages of several units, with 1-D bulk
-//     async copies (TMA engine, mbarrier byte counting, no multicast) issued by a copy warp;
+//   * persistent grid, one CTA per SM; the (column block, row block) units of the matrix are dealt to the CTAs evenly and contiguously
+//     ("stream-K"), or by column blocks or equal parts of them where that is cheaper (plan_split), so every CTA streams ONE contiguous byte
+//     range of the weights, in stages of several units, with 1-D bulk async copies (TMA engine, mbarrier byte counting, no multicast)
+//     issued by a copy warp;
 //   * the work is the decode of the trellis, so the product must cost the decoding warps nothing: decoded registers go straight to
 //     TENSOR MEMORY as the A operand of tcgen05.mma (M = 128 output columns of a column block), the rotated activations are the B
 //     operand (N = rows) in shared memory.  The lane that decodes a 16x16 tile holds exactly its share of a tcgen05.st 16x256b
@@ -22,16 +23,17 @@
 //     normalising it on the way -- so the linear is ONE launch.  Weights are constants: copies start, and the first half units of
 //     every group are decoded, before the kernel ahead in the stream has finished.
 //
-// Bound by the issue of the decode: 46 to 54 instructions per 16x16 tile, whatever K (51.7 at K = 3, 48.1 at K = 4, 46.5 at K = 8, 62.1
-// for MUL1 at K = 6), are 12 to 16 clk of a SM's four schedulers.  The loop takes 16.3 / 14.4 / 16.2 / 14.1 clk per tile and SM at K =
-// 3 / 4 / 6 / 8 (stamps in chained launches at 1.965 GHz; 15.5 / 16.3 / 17.7 at K = 2 / 5 / 7), 18.5 for MUL1 at K = 3 and 6; the ALU
-// pipe is busy in 60 to 64 % of the active cycles at every K (MUL1: the FMA pipe in 72 %).  The MMAs take 4 clk per tile of the tensor
-// pipe at N = 16 and 8 at N = 64 and run beside it: 15.2 to 16.3 clk (K = 3) up to 16 rows, 17.6 at 32, 22.5 at 33 to 64, where half
-// units are handed over in two pieces (27 in short launches).  Against the register-level kernel on mma.sync that it replaces (two CTAs of 16 warps, 8 rows per MMA),
-// chained launches over distinct weights, K = 3: 5120 x 34816 48.8 -> 46.3 us at one row and 51 -> 47.1 at four; 17408 x 5120 28.5 ->
-// 26.6; 5120 x 5120 12.1 -> 11.3; 17408 x 5120, K = 6, MUL1, 16 rows 45.6 -> 35.0.  What is not the loop, per launch at one row: 1.8
-// to 3.5 us from the end of the launch ahead until the input is rotated, 1.7 to 2.2 us by which CTAs that could not become resident
-// early finish later than the median, 3.2 to 4.6 us from there to the stored outputs (tensor memory -> partial sums -> counter -> sums).
+// Bound by the issue of the decode and by the register ports that its pipes share: 44 to 52 instructions per 16x16 tile, whatever K (49.7 at K =
+// 3, 44.5 at K = 4, 51.8 at K = 6, 46.5 at K = 8, 61.2 for MUL1 at K = 6), are 11 to 13 clk of a SM's four schedulers.  The loop takes 15.1 /
+// 13.3 / 15.7 / 14.0 clk per tile and SM at K = 3 / 4 / 6 / 8 (stamps in chained launches at 1.965 GHz; 14.6 / 15.4 / 15.8 at K = 2 / 5 / 7),
+// 16.0 and 16.2 for MUL1 at K = 3 and 6; issue slots are used in 70 to 75 % of a launch's active cycles, the ALU pipe in 62 to 65 %.  The
+// MMAs take 4 clk per tile of the tensor pipe at N = 16 and 8 at N = 64 and run beside it: 15.1 to 15.4 clk (K = 3) up to 16 rows, 16.4 at 32,
+// 21.9 at 33 to 64, where half units are handed over in two pieces.  Chained launches over distinct weights, K = 3, one row, us: 5120 x 34816
+// 43.2, 17408 x 5120 24.8, 5120 x 5120 11.3, 4096 x 4096 (K = 4) 8.7; 17408 x 5120, K = 6, MUL1, 16 rows 33.2.  What is not the loop, per
+// launch at one row: 1.8 to 4 us from the end of the launch ahead until the input is rotated, 1.8 to 2.4 us by which CTAs that could not
+// become resident early finish later than the median, 3.1 to 4.3 us from there to the stored outputs (tensor memory -> partial sums ->
+// counter -> sums).  Fewer instructions in the loop's bookkeeping (one counter for stage and range) changed nothing at K = 3 and lost 2 %
+// at K = 4 to 8; a copy of the loop per group lost 7 % to instruction fetch.
 #pragma once
 #include "exl3_gemv_common.cuh"
 
