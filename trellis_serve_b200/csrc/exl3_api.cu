@@ -672,8 +672,8 @@ static size_t tc_up(size_t v) { return (v + 255) & ~(size_t)255; }
 // The decode kernel up to the 64 rows that one pass over the weights serves, whatever the sizes.  It is the more exact of the two
 // (weights as two exact summands, fp32 sums to the end; the tensor-core kernel rounds weights and rotated product to fp16), and the
 // faster one for large groups.  For small ones it is not, from 17 to 33 rows on: the line stays at 64 for the results' sake.  Chained
-// graph launches of 64 rows, K = 3, microseconds, decode kernel / tensor-core kernel: 17408 x 5120 42.5 / 48.4, 5120 x 34816 66 / 78.6, 5120 x
-// 5120 23.9 / 24.4, 2048 x 1024 18.0 / 12.6, 1024 x 640 12.9 / 9.5.  From 65 rows up the decode kernel passes twice and loses at every
+// graph launches of 64 rows, K = 3, microseconds, decode kernel / tensor-core kernel: 17408 x 5120 42.5 / 48.4, 5120 x 5120 23.9 /
+// 24.4, 2048 x 1024 18.0 / 12.6, 1024 x 640 12.9 / 9.5.  From 65 rows up the decode kernel passes twice and loses at every
 // size (17408 x 5120 71 / 48.6, 5120 x 5120 37 / 24.4).
 int exl3_prefers_decode(int rows, int k, int n_total, int sms)
 {

@@ -26,8 +26,9 @@ from .linear import _dtype_code, _ptr, _require_cuda, _stream, supports_matrix
 
 BLOCK_SIZES = (8, 128)
 # Average routed rows per expert from which a class goes through the grouped tensor-core GEMM (items of up to 128 rows of an
-# expert, decoded once each) instead of blocks of eight rows (decoded once per block).  Measured crossover: 8 rows for 256 experts of
-# 2048 x 512, 11 for 64 of 2048 x 768, more for layers so small that the two further launches show.
+# expert, decoded once each) instead of blocks of eight rows (decoded once per block).  By time the line would lie between 2 and 8 rows (256 experts
+# of 2048 x 512, graph, blocks / items: 179 / 221 us at 2 rows, 289 / 257 at 8, 344 / 260 at 10); it lies at 10 because items round the
+# decoded weights to fp16 and blocks of eight do not.
 TC_ROWS_PER_EXPERT = 10
 _workspace: dict[int, torch.Tensor] = {}
 
