@@ -78,17 +78,19 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
         constexpr int EXCHANGE = 5;
         const int uneven = a.rows > 8 ? 4 : 2, hidden = a.rows <= 8 && most > 12 ? 3 : 0;
         const bool few = x == SK_ROTATE && a.rows > SK_FUSED_ROWS;           // rows rotated inside in one pass of the decode warps
-        long long best = (long long)most + EXCHANGE + uneven;
         const long long whole = (long long)((l.NB + ctas - 1) / ctas) * l.KG;
+        long long best = (long long)most + EXCHANGE + uneven;
         if (whole + hidden < best && !(few && whole > SK_DECODE_WARPS)) {
             best = whole + hidden;
             l.piece = l.KG;
         }
-        for (int parts = 2; parts <= l.KG && (long long)parts * l.NB <= ctas; parts++) {
-            const int part = (l.KG + parts - 1) / parts;
+        // Parts get shorter with their number: the fewest of the shortest that the grid has room for.  Trying each number in turn, twice per
+        // call, showed in the smallest calls.
+        const int room = l.NB < ctas ? (ctas / l.NB < l.KG ? ctas / l.NB : l.KG) : 1;
+        if (room > 1) {
+            const int part = (l.KG + room - 1) / room;
             if (part + EXCHANGE < best && !(few && part > SK_DECODE_WARPS)) {
-                best = part + EXCHANGE;
-                l.parts = parts;
+                l.parts = (l.KG + part - 1) / part;
                 l.piece = 1;
             }
         }
