@@ -190,6 +190,8 @@ exl3_status exl3_rmsnorm_linear(const void *x, int x_dtype, const void *residual
  * Before it waits for the kernel ahead of it in the stream, an attention call reads `*position` and requests the cache rows
  * below it and suh_next (like weights: they must be complete in memory before the call is enqueued behind this library's
  * kernels; rows written by earlier steps are).  Row `*position`, the tables and qkv are read after the wait.
+ * `*position` is the caller's to keep within 0 .. t_max - 1.  Outside, nothing is read or written beyond the cache and nothing is appended;
+ * an attention call then reports EXL3_ERR_BAD_SHAPE through exl3_device_error on its scratch.
  * The reference leaves attention to its engine; no counterpart there. */
 size_t exl3_attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max);
 exl3_status exl3_rope_append(void *qkv, int dtype, int rows, int q_heads, int kv_heads, int head_dim, const float *cos_table,
@@ -376,7 +378,8 @@ exl3_status exl3_moe_tc_layer(const void *x, int dtype, int tokens, int top_k, i
 
 /* Reads and clears the device-side error word kept in a workspace (set when a bounded wait in a kernel gave up).
  * workspace == NULL with workspace_bytes == 0 means the built-in scratch of exl3_linear_static on the current device.
- * Synchronises `stream`.  Returns EXL3_OK or EXL3_ERR_DEVICE_WAIT. */
+ * Synchronises `stream`.  Returns EXL3_OK, EXL3_ERR_DEVICE_WAIT or, on the scratch of an attention call whose position lay outside
+ * the cache, EXL3_ERR_BAD_SHAPE. */
 exl3_status exl3_device_error(void *workspace, size_t workspace_bytes, void *stream);
 
 /* Measurement / test knob: how weights of the 3INST and MCG codebooks enter the tensor-core product.

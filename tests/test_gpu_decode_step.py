@@ -344,3 +344,45 @@ def test_end_of_the_residual_chain(dtype, rows, k):
     want = z.double() / (z.double().pow(2).mean(1, keepdim=True) + 1e-6).sqrt() * weight.double()
     half_ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
     assert bool(((out.double() - want).abs() <= want.abs() * (half_ulp + 2.0 ** -21) + 2.0 ** -25).all())
+
+
+@pytest.mark.parametrize("dtype,rows,q_heads,kv_heads,t_max", [(torch.float16, 2, 10, 2, 64), (torch.bfloat16, 1, 4, 1, 203)])
+def test_positions_outside_the_cache_are_reported_and_write_nothing(dtype, rows, q_heads, kv_heads, t_max):
+    """A position at or behind `t_max`, or below zero: the cache and what lies around it stay as they are, the call reports it, and the next
+    call works.  Without the rotary part a position behind the cache attends over all of it, as the last position does.  The tables and
+    the memory around the cache are there, so that the call would stay within this test's tensors even without the check."""
+    import math
+    from trellis_serve_b200 import _lib
+    lib = _lib.load()
+    _lib.init_device(0)
+    gen = torch.Generator(device=DEV).manual_seed(t_max)
+    room = 64                                                   # positions of slack before, between and behind keys and values
+    flat = torch.randn((room + rows * kv_heads * t_max + room, 2, 128), device=DEV, generator=gen).to(dtype).transpose(0, 1).contiguous()
+    cache = flat[:, room:-room]
+    qkv = torch.randn((rows, (q_heads + 2 * kv_heads) * 128), device=DEV, generator=gen).to(dtype)
+    tables = torch.randn((2, 1 + t_max + room, 64), device=DEV, generator=gen)[:, 1:]
+    scratch = torch.zeros(int(lib.exl3_attention_scratch_bytes(rows, q_heads, kv_heads, t_max)), dtype=torch.uint8, device=DEV)
+    p, st, code, scale = lin._ptr, lin._stream(DEV), lin._dtype_code(qkv), 1.0 / math.sqrt(128)
+
+    def call(name, pos, rope):
+        position, out = torch.tensor([pos], dtype=torch.int32, device=DEV), torch.zeros((rows, q_heads * 128), dtype=dtype, device=DEV)
+        head = (p(qkv), code, rows, q_heads, kv_heads, 128) + ((p(tables[0]), p(tables[1])) if rope else ()) + (p(cache[0]), p(cache[1]), t_max, p(position))
+        tail = () if name == "exl3_rope_append" else (scale, p(scratch), scratch.numel(), p(out), None, 0, None, 0)
+        _lib.check(getattr(lib, name)(*head, *tail, st), name)
+        torch.cuda.synchronize()
+        return out, lib.exl3_device_error(p(scratch), scratch.numel(), st)
+
+    last, rc = call("exl3_decode_attention", t_max - 1, False)
+    assert rc == 0
+    before, q_before = flat.clone(), qkv.clone()
+    for pos in (t_max, t_max + 1, t_max + room - 1, -1):
+        out, rc = call("exl3_decode_attention", pos, False)
+        assert rc == 1                                          # EXL3_ERR_BAD_SHAPE
+        if pos > 0:
+            assert torch.equal(out, last)
+        _, rc = call("exl3_rope_decode_attention", pos, True)
+        assert rc == 1
+        call("exl3_rope_append", pos, True)
+        assert torch.equal(flat, before) and torch.equal(qkv, q_before)
+    again, rc = call("exl3_decode_attention", t_max - 1, False)
+    assert rc == 0 and torch.equal(again, last)

@@ -437,7 +437,7 @@ exl3_status exl3_device_error(void* workspace, size_t workspace_bytes, void* str
     if (int rc = cuda_status(cudaStreamSynchronize(st))) return rc;
     if (code == 0) return EXL3_OK;
     if (int rc = cuda_status(cudaMemsetAsync(workspace, 0, sizeof(int), st))) return rc;
-    return EXL3_ERR_DEVICE_WAIT;
+    return code == ATT_ERR_POSITION ? EXL3_ERR_BAD_SHAPE : EXL3_ERR_DEVICE_WAIT;
 }
 
 /* ---- decode step: rotated fragments written by the kernel ahead of the linear -------------------------------------- */

@@ -155,6 +155,7 @@ int launch_normed(const void* z, const float* ssq, const void* weight, float eps
 int launch_residual_ssq(const void* x, const void* res_in, int bf16, int rows, int k, void* res_out, float* ssq, cudaStream_t st);
 int launch_silu_mul_rotate(const void* gu, int bf16, const __half* suh, int rows, int inter, void* act, uint32_t* xf, int mode,
                            cudaStream_t st);
+enum { ATT_ERR_WAIT = 1, ATT_ERR_POSITION = 2 };     // error word of the attention kernel: a wait gave up; `*position` is outside the cache
 size_t attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max);
 int attention_init_device();
 int launch_rope_append(void* qkv, int bf16, int rows, int q_heads, int kv_heads, const float* cos_t, const float* sin_t, void* k_cache,

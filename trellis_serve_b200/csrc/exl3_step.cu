@@ -288,6 +288,7 @@ __global__ void rope_append_kernel(void* __restrict__ qkv, int bf16, int rows, i
     if (idx >= (long long)rows * heads * 64) return;
     const int i = (int)(idx & 63), head = (int)((idx >> 6) % heads), row = (int)((idx >> 6) / heads);
     const int pos = *pos_ptr;
+    if (pos < 0 || pos >= t_max) return;                          // a caller's error: no such cache slot
     const long long base = ((long long)row * heads + head) * ATT_D;
     const bool b = bf16 != 0;
     const float x1 = to_f32(qkv, base + i, b), x2 = to_f32(qkv, base + i + 64, b);
@@ -403,7 +404,10 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
     ptx::grid_launch_dependents();
     const int rank = blockIdx.x, ctas = gridDim.x, kvh = blockIdx.y, row = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q4 = lane & 3, n8 = lane >> 2;
-    const int pos = *pos_ptr, T = pos + 1;                        // valid cache positions
+    // A position outside the cache is a caller's error: it is reported, the rows that exist are attended over, nothing is appended.
+    const int given = *pos_ptr;
+    const bool inside = given >= 0 && given < t_max;
+    const int pos = inside ? given : given < 0 ? -1 : t_max, T = pos < t_max ? pos + 1 : t_max;       // T: valid cache positions
     const int heads = q_heads + 2 * kv_heads;
     const int all_tiles = (T + ATT_TILE - 1) / ATT_TILE, share = (all_tiles + ctas - 1) / ctas, tile0 = rank * share;
     const int tiles = all_tiles - tile0 < 0 ? 0 : all_tiles - tile0 < share ? all_tiles - tile0 : share;
@@ -434,7 +438,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
         ptx::mbar_fence_init();
         for (int j = 0; j < stages && j < fills; j++) fetch(j, j);
     }
-    const bool owner = tiles > 0 && pos / ATT_TILE >= tile0 && pos / ATT_TILE < tile0 + tiles;       // of position `pos`
+    const bool owner = inside && tiles > 0 && pos / ATT_TILE >= tile0 && pos / ATT_TILE < tile0 + tiles;       // of position `pos`
     const int with = tiles < ATT_WARPS ? tiles : ATT_WARPS;       // warps that have positions
     const int mine = rank + ctas * warp;                          // heads are dealt to the CTAs, one warp each, to be finished
     uint2 signs = make_uint2(0u, 0u);                             // constants: requested before the wait
@@ -448,7 +452,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
         const int i = threadIdx.x & 63;
         const uint16_t* src = reinterpret_cast<const uint16_t*>(qkv) + (long long)row * heads * ATT_D;
         float c = 1.f, sn = 0.f;
-        if (cos_t) {
+        if (cos_t && inside) {
             c = cos_t[(long long)pos * 64 + i];
             sn = sin_t[(long long)pos * 64 + i];
         }
@@ -663,7 +667,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
         if (suh) rotate_store(y, signs, xf, mode, 0, (q_heads * ATT_D) >> 4, rows, row, qh, lane);
     }
     ATT_STAMP(7);
-    if (failed && lane == 0) atomicExch(err, 1);
+    if (failed && lane == 0) atomicExch(err, ATT_ERR_WAIT);
+    if (!inside && threadIdx.x == 0) atomicExch(err, ATT_ERR_POSITION);
     if (ctas > 1) ptx::cluster_sync_all();                        // no CTA leaves while its shared memory is being read
 }
 
