@@ -386,3 +386,42 @@ def test_positions_outside_the_cache_are_reported_and_write_nothing(dtype, rows,
         assert torch.equal(flat, before) and torch.equal(qkv, q_before)
     again, rc = call("exl3_decode_attention", t_max - 1, False)
     assert rc == 0 and torch.equal(again, last)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("t_max,pos,masked", [
+    (200, 199, [(0, 8)]),                       # a warp's only tile
+    (200, 150, [(0, 8), (64, 104), (144, 151)]),
+    (2048, 2047, [(0, 1024)]),                  # whole CTAs of a cluster
+    (4000, 3999, [(0, 500), (1000, 1016), (2048, 3999)]),
+    (64, 63, [(0, 64)]),                        # nothing left: NaN, as softmax gives
+])
+def test_scores_of_minus_infinity_and_nan(dtype, t_max, pos, masked):
+    """Positions whose scores are -inf (an infinite key component against queries that are negative there) have no weight, be they a single
+    one, a warp's tile or all that a CTA has; a score that is not a number makes the heads that see it so.  Bounds of the test above."""
+    import math
+    from trellis_serve_b200 import _lib
+    lib = _lib.load()
+    _lib.init_device(0)
+    rows, q_heads, kv_heads = 2, 10, 2
+    gen = torch.Generator(device=DEV).manual_seed(pos)
+    qkv = torch.randn((rows, (q_heads + 2 * kv_heads) * 128), device=DEV, generator=gen).to(dtype)
+    qkv[:, :q_heads * 128].view(rows, q_heads, 128)[:, :, 5] = -1.0
+    cache = torch.randn((2, rows, kv_heads, t_max, 128), device=DEV, generator=gen).to(dtype)
+    for lo, hi in masked:
+        cache[0, :, :, lo:hi, 5] = float("inf")
+    cache[0, 1, 0, 3, 7] = float("nan")
+    position = torch.tensor([pos], dtype=torch.int32, device=DEV)
+    scratch = torch.zeros(int(lib.exl3_attention_scratch_bytes(rows, q_heads, kv_heads, t_max)), dtype=torch.uint8, device=DEV)
+    out = torch.zeros((rows, q_heads * 128), dtype=dtype, device=DEV)
+    p, scale = lin._ptr, 1.0 / math.sqrt(128)
+    _lib.check(lib.exl3_decode_attention(p(qkv), lin._dtype_code(qkv), rows, q_heads, kv_heads, 128, p(cache[0]), p(cache[1]), t_max, p(position),
+                                         scale, p(scratch), scratch.numel(), p(out), None, 0, None, 0, lin._stream(DEV)), "exl3_decode_attention")
+    torch.cuda.synchronize()
+    q = qkv[:, :q_heads * 128].double().view(rows, kv_heads, q_heads // kv_heads, 128)
+    k, v = cache[0, :, :, :pos + 1].double(), cache[1, :, :, :pos + 1].double()
+    want = (torch.softmax(q @ k.transpose(-1, -2) * scale, dim=-1) @ v).view(rows, q_heads * 128)
+    assert torch.equal(out.isnan(), want.isnan())
+    got, want = out.double().nan_to_num(), want.nan_to_num()
+    half_ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert bool(((got - want).abs() <= want.abs() * half_ulp + 2e-5 * want.abs().max()).all())

@@ -537,7 +537,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
             mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
             mx = fmaxf(m, mx);
             const float keep = m == -INFINITY ? 0.f : __expf(m - mx);
-            const float e0 = 2 * q4 < n ? __expf(s0 - mx) : 0.f, e1 = 2 * q4 + 1 < n ? __expf(s1 - mx) : 0.f;
+            const float base = mx == -INFINITY ? 0.f : mx;        // scores that are all -inf so far have no weight, rather than NaN
+            const float e0 = 2 * q4 < n ? __expf(s0 - base) : 0.f, e1 = 2 * q4 + 1 < n ? __expf(s1 - base) : 0.f;
             m = mx;
             l = l * keep + (e0 + e1);
             sh.p[warp][2 * q4][n8] = e0;
