@@ -610,7 +610,7 @@ exl3_status exl3_rmsnorm_linear(const void* x, int x_dtype, const void* residual
 size_t exl3_attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max)
 {
     if (rows < 0 || q_heads < 1 || kv_heads < 1 || t_max < 1) return 0;
-    return attention_scratch_bytes(rows, q_heads, kv_heads, t_max);
+    return ATT_SCRATCH_BYTES;
 }
 
 exl3_status exl3_rope_append(void* qkv, int dtype, int rows, int q_heads, int kv_heads, int head_dim, const float* cos_table,
@@ -639,10 +639,10 @@ static int attention_common(const void* qkv, int dtype, int rows, int q_heads, i
     if (rows < 0 || q_heads < 1 || kv_heads < 1 || head_dim != 128 || t_max < 1 || q_heads % kv_heads) return EXL3_ERR_BAD_SHAPE;
     if (!aligned(qkv, 8) || !aligned(k_cache, 16) || !aligned(v_cache, 16) || !aligned(position, 4) || (out && !aligned(out, 8)) || (!out && !suh_next))
         return EXL3_ERR_BAD_POINTER;
-    if (!aligned(scratch, 256) || scratch_bytes < attention_scratch_bytes(rows, q_heads, kv_heads, t_max)) return EXL3_ERR_WORKSPACE;
+    if (!aligned(scratch, 256) || scratch_bytes < ATT_SCRATCH_BYTES) return EXL3_ERR_WORKSPACE;
     if (!current_device_info()) return EXL3_ERR_NOT_INITIALISED;
     return launch_decode_attention(qkv, dtype == EXL3_BF16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, position, scale, cos_table,
-                                   sin_table, reinterpret_cast<float*>(scratch), out, reinterpret_cast<const __half*>(suh_next), xf,
+                                   sin_table, reinterpret_cast<int*>(scratch), out, reinterpret_cast<const __half*>(suh_next), xf,
                                    suh_next ? fragment_mode(codebook) : 0, (cudaStream_t)stream);
 }
 

@@ -156,12 +156,12 @@ int launch_residual_ssq(const void* x, const void* res_in, int bf16, int rows, i
 int launch_silu_mul_rotate(const void* gu, int bf16, const __half* suh, int rows, int inter, void* act, uint32_t* xf, int mode,
                            cudaStream_t st);
 enum { ATT_ERR_WAIT = 1, ATT_ERR_POSITION = 2 };     // error word of the attention kernel: a wait gave up; `*position` is outside the cache
-size_t attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max);
+constexpr size_t ATT_SCRATCH_BYTES = 256;             // that word, and nothing else: the CTAs of a head merge over shared memory
 int attention_init_device();
 int launch_rope_append(void* qkv, int bf16, int rows, int q_heads, int kv_heads, const float* cos_t, const float* sin_t, void* k_cache,
                        void* v_cache, int t_max, const int* pos, cudaStream_t st);
 int launch_decode_attention(const void* qkv, int bf16, int rows, int q_heads, int kv_heads, void* k_cache, void* v_cache, int t_max,
-                            const int* pos, float scale, const float* cos_t, const float* sin_t, float* part, void* out, const __half* suh,
+                            const int* pos, float scale, const float* cos_t, const float* sin_t, int* err, void* out, const __half* suh,
                             uint32_t* xf, int mode, cudaStream_t st);
 
 // exl3_gemm_tc.cu ---------------------------------------------------------------------------------------

@@ -272,7 +272,6 @@ constexpr int ATT_WARPS = 16;
 constexpr int ATT_TILE = 8;               // cache positions that a warp takes at a time: columns of an m16n8k16 MMA
 constexpr int ATT_STAGE = ATT_WARPS * ATT_TILE;          // cache positions of a stage of the ring
 constexpr int ATT_MAX_STAGES = 3, ATT_MAX_CLUSTER = 8;
-constexpr int ATT_CHUNK = 128, ATT_PART = ATT_D + 4;     // what a call's scratch is sized by: positions and floats of a partial result
 
 // One thread per (row, head, pair i < 64): x1' = x1 cos - x2 sin, x2' = x2 cos + x1 sin with x1 = x[i], x2 = x[i + 64]
 // (the "rotate half" convention).  Query heads are rotated in place in qkv; key heads are rotated into the cache slot
@@ -673,18 +672,6 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 1) decode_attention_kernel(con
     if (ctas > 1) ptx::cluster_sync_all();                        // no CTA leaves while its shared memory is being read
 }
 
-// Scratch: an error word (set when the bounded wait for the cache copies gives up; exl3_device_error reads it).  Callers hold as much as a
-// merge through memory would take.
-constexpr size_t ATT_SCRATCH_HEADER = 256;
-static size_t attention_counter_bytes(int rows, int kv_heads) { return ((size_t)rows * kv_heads * sizeof(int) + 255) & ~(size_t)255; }
-
-size_t attention_scratch_bytes(int rows, int q_heads, int kv_heads, int t_max)
-{
-    const int splits = (t_max + ATT_CHUNK - 1) / ATT_CHUNK;
-    const int G = q_heads / (kv_heads > 0 ? kv_heads : 1);
-    return ATT_SCRATCH_HEADER + attention_counter_bytes(rows, kv_heads) + (size_t)rows * kv_heads * splits * G * ATT_PART * sizeof(float);
-}
-
 // The kernels keep their part of the cache in dynamic shared memory beyond the default limit: opted in once per device.
 template <int G>
 static int attention_opt_in()
@@ -715,7 +702,7 @@ int launch_rope_append(void* qkv, int bf16, int rows, int q_heads, int kv_heads,
 
 template <int G>
 static int launch_attention_g(const void* qkv, int bf16, int rows, int q_heads, int kv_heads, void* k_cache, void* v_cache, int t_max,
-                              const int* pos, float scale, const float* cos_t, const float* sin_t, float* part, void* out, const __half* suh,
+                              const int* pos, float scale, const float* cos_t, const float* sin_t, int* err, void* out, const __half* suh,
                               uint32_t* xf, int mode, cudaStream_t st)
 {
     const DeviceInfo* d = current_device_info();
@@ -728,7 +715,6 @@ static int launch_attention_g(const void* qkv, int bf16, int rows, int q_heads, 
     const int share = (tiles + ctas - 1) / ctas;
     int stages = (share + ATT_WARPS - 1) / ATT_WARPS;
     if (stages > ATT_MAX_STAGES) stages = ATT_MAX_STAGES;
-    int* err = reinterpret_cast<int*>(part);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, kv_heads, rows);
     cfg.blockDim = dim3(ATT_WARPS * 32);
@@ -749,17 +735,17 @@ static int launch_attention_g(const void* qkv, int bf16, int rows, int q_heads, 
 }
 
 int launch_decode_attention(const void* qkv, int bf16, int rows, int q_heads, int kv_heads, void* k_cache, void* v_cache, int t_max,
-                            const int* pos, float scale, const float* cos_t, const float* sin_t, float* part, void* out, const __half* suh,
+                            const int* pos, float scale, const float* cos_t, const float* sin_t, int* err, void* out, const __half* suh,
                             uint32_t* xf, int mode, cudaStream_t st)
 {
     if (rows == 0) return EXL3_OK;
     if (kv_heads < 1 || q_heads % kv_heads) return EXL3_ERR_BAD_SHAPE;
     switch (q_heads / kv_heads) {
-        case 1: return launch_attention_g<1>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, part, out, suh, xf, mode, st);
-        case 2: return launch_attention_g<2>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, part, out, suh, xf, mode, st);
-        case 4: return launch_attention_g<4>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, part, out, suh, xf, mode, st);
-        case 5: return launch_attention_g<5>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, part, out, suh, xf, mode, st);
-        case 8: return launch_attention_g<8>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, part, out, suh, xf, mode, st);
+        case 1: return launch_attention_g<1>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, out, suh, xf, mode, st);
+        case 2: return launch_attention_g<2>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, out, suh, xf, mode, st);
+        case 4: return launch_attention_g<4>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, out, suh, xf, mode, st);
+        case 5: return launch_attention_g<5>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, out, suh, xf, mode, st);
+        case 8: return launch_attention_g<8>(qkv, bf16, rows, q_heads, kv_heads, k_cache, v_cache, t_max, pos, scale, cos_t, sin_t, err, out, suh, xf, mode, st);
     }
     return EXL3_ERR_BAD_SHAPE;
 }
