@@ -176,8 +176,8 @@ exl3_status exl3_rmsnorm_linear(const void *x, int x_dtype, const void *residual
  *                          `*position` (device int, so a captured graph can move on): q in place, k into slot `*position` of
  *                          k_cache [rows, kv_heads, t_max, 128], v copied into v_cache.
  *   exl3_decode_attention  softmax(q k^T * scale) v over cache positions 0..*position for every query head (q_heads a
- *                          multiple of kv_heads, ratio 1, 2, 4, 5 or 8), split over the CTAs of a cluster per (row, KV head)
- *                          and merged in a fixed order (one launch);
+ *                          multiple of kv_heads, ratio 1, 2, 4, 5 or 8), split over the CTAs of a cluster per (row, KV head), at most
+ *                          eight, and merged in a fixed order (one launch);
  *                          out [rows, q_heads * 128] in `dtype` (may be NULL).  scratch: exl3_attention_scratch_bytes(),
  *                          256-byte aligned, zero-filled once before its first use (an error word that exl3_device_error
  *                          reads); exl3_init_device must have run.  suh_next != NULL: a head is one rotation block of the o

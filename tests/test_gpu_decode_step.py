@@ -331,6 +331,13 @@ def test_decode_attention_against_float64(dtype, rows, q_heads, kv_heads, t_max,
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,q_heads,kv_heads,t_max,pos", [(1, 8, 1, 8192, 8191), (3, 10, 2, 9001, 8500), (1, 5, 1, 40000, 39990), (1, 4, 1, 131072, 131071)])
+def test_decode_attention_of_long_contexts(dtype, rows, q_heads, kv_heads, t_max, pos):
+    """8192 positions and more, of which eight CTAs have to take everything: the rings go around up to 43 times.  Bounds as above."""
+    test_decode_attention_against_float64(dtype, rows, q_heads, kv_heads, t_max, pos)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("rows,k", [(1, 128), (3, 5120), (2, 4224)])
 def test_end_of_the_residual_chain(dtype, rows, k):
     """exl3_normed against float64: one rounding of an fp32 product of three factors (a few 2^-24)."""

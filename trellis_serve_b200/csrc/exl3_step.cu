@@ -708,7 +708,11 @@ static int launch_attention_g(const void* qkv, int bf16, int rows, int q_heads, 
     const DeviceInfo* d = current_device_info();
     if (!d) return EXL3_ERR_NOT_INITIALISED;
     // CTAs that share a (row, KV head): as many as a portable cluster holds, while every one has 64 positions and more to look at and all
-    // CTAs of the launch fit on the chip together (a CTA with a full ring has an SM for itself).
+    // CTAs of the launch fit on the chip together (a CTA with a full ring has an SM for itself).  No more than eight, however long the
+    // context: one row of one KV head keeps 8 of the SMs busy and grows by 1.37 us per 1024 positions (5 query heads; 1.68 with 8).  Chained
+    // launches, us, against one CTA per 128 positions merged through memory, whose merge grew with the context as well: one KV head, 5
+    // query heads, 4096 / 8192 / 32768 / 131072 positions 8.6 / 14.1 / 47.0 / 178 (12.8 / 23.0 / 73.4 / 285), 8 query heads 9.8 / 16.7 /
+    // 57.1 / 219 (18.3 / 28.2 / 82.9 / 324), 8 KV heads of 5 9.1 / 14.7 / 48.1 / 181 (16.6 / 37.0 / 144 / 587).
     const int tiles = (t_max + ATT_TILE - 1) / ATT_TILE;
     int ctas = ATT_MAX_CLUSTER;
     while (ctas > 1 && ((long long)rows * kv_heads * ctas > d->sm_count || tiles < 8 * ctas)) ctas /= 2;

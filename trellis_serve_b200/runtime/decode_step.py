@@ -2,17 +2,16 @@
 
     per layer:  a = RMSNorm(residual)                          -> inside the input rotation of q|k|v       (normed linear)
                 q|k|v = EXL3(a);  RoPE(q, k);  KV cache append;  attention over the cache
-                o = EXL3(attention)                             -> rotation launch, then the GEMV
+                o = EXL3(attention)                             -> rotated by the attention kernel (rotation launch with stock attention)
                 residual += o                                   -> in the epilogue of o (with the stream's sums of squares)
                 a = RMSNorm(residual)                           -> inside the input rotation of gate|up
                 g|u = EXL3(a);  act = SiLU(g) * u               -> computed inside down's own input rotation (glu linear; from three
                 h = EXL3(act);  residual += h                      rows up: silu_mul_rotate ahead of the GEMV); the sum in down's epilogue
 
-Every linear is ONE decode-GEMV launch whose activations were rotated by the kernel ahead of it; rotary embedding, cache
-append and attention are stock torch (`scaled_dot_product_attention`): they are not part of the quantized-linear path and
-their bytes (the KV read) are reported separately.  `attention="library"` (default) runs the library's own kernel for that part (RoPE + cache append + split-KV attention, merged
-by the last CTA to arrive); `attention="torch"` keeps the stock torch ops.  The whole step is captured in one CUDA graph, as an engine captures
-it (cuda/src/sglang_exl3/sglang_glue/moe.py:202-213 warms for that purpose; cuda/src/sglang_exl3/tools/decode_microbench.py
+Every linear is ONE decode-GEMV launch; rotary embedding, cache append and attention are not part of the quantized-linear path and
+their bytes (the KV read) are reported separately.  `attention="library"` (default) runs the library's own kernel for that part (RoPE +
+cache append + attention by a cluster per row and KV head); `attention="torch"` takes stock torch ops (`scaled_dot_product_attention`).
+The whole step is captured in one CUDA graph, as an engine captures it (cuda/src/sglang_exl3/sglang_glue/moe.py:202-213 warms for that purpose; cuda/src/sglang_exl3/tools/decode_microbench.py
 :27-41 times launches the same way).
 
 Tensor parallelism: query and KV heads are split over the ranks (with more ranks than KV heads every head is held by
@@ -143,7 +142,7 @@ class DecodeStep:
 
     def _attention(self, layer: int, suh_next: torch.Tensor | None = None) -> bool:
         """RoPE, cache append and attention of one layer into `self.attn`.  True when the rotated input of the o projection
-        was written as well (the library's merge kernel does that when handed the projection's sign vector)."""
+        was written as well (the library's kernel does that when handed the projection's sign vector)."""
         s, q, kv = self.shape, self.q_heads * self.shape.head_dim, self.kv_heads * self.shape.head_dim
         if self.attention == "library":
             from .. import _lib
