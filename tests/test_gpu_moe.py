@@ -259,3 +259,54 @@ def test_few_slots_agree_with_the_aligned_form(tokens, top_k, Ks, hidden, inter,
             m[it.view(-1)[0].long()] = -1
         gone = torch.where(it == it.view(-1)[0], -1, it)
         close(_layer(pack, x, wt, it, maps), moe.forward_mixed(x, wt, gone, pack))
+
+
+@pytest.mark.parametrize("tokens,top_k,E,hidden,inter,K,cb,dtype", [
+    (1, 8, 16, 2048, 512, 3, 0, torch.bfloat16),            # whole column blocks and even ranges with all slots, parts with few
+    (2, 8, 16, 1024, 384, 4, 1, torch.float16),
+    (1, 4, 9, 640, 1152, 5, 2, torch.float16),              # odd numbers of units, parts with remainders
+    (2, 3, 6, 128, 128, 2, 0, torch.float16),               # fewer units than CTAs
+    (40, 4, 160, 128, 128, 3, 1, torch.bfloat16),           # 160 slots: more than one look at the ids
+])
+def test_slots_without_an_expert_take_no_part(tokens, top_k, E, hidden, inter, K, cb, dtype):
+    """The form for few slots with an expert map that holds none, one, a few, all but one and all of the slots' experts, in one captured graph
+    whose map changes between replays (a rank's share of the experts): the units of the slots that are left are dealt anew each time.
+    Against blocks of eight rows on ids without the others, bound of the test above."""
+    from trellis_serve_b200 import _lib
+    gate, up, down = _mixed_experts(400 + E, [K] * E, hidden, inter)
+    for proj, scale in ((gate, hidden), (up, hidden), (down, inter)):
+        proj[2][:] = [(s.astype(np.float32) / (1.24 * scale ** 0.5)).astype(np.float16) for s in proj[2]]
+    pack = moe.prepare_mixed(_to_dev(gate), _to_dev(up), _to_dev(down), cb)
+    assert _lib.load().exl3_moe_prefers_slots(tokens * top_k, E, hidden, inter, K, cb)
+    ids, w = _routing(tokens, top_k, E, 50 + tokens)
+    x = torch.randn((tokens, hidden), device=DEV, generator=torch.Generator(device=DEV).manual_seed(6)).to(dtype)
+    wt, it = torch.from_numpy(w).to(DEV), torch.from_numpy(ids).to(DEV)
+    emap = pack.expert_maps[0].clone()
+    ws = torch.zeros(moe.layer_workspace_bytes([E], hidden, inter, cb, tokens, top_k), dtype=torch.uint8, device=DEV)
+    out = torch.empty_like(x)
+    moe.run_layer(x, wt, it, pack, out, ws, [emap])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        moe.run_layer(x, wt, it, pack, out, ws, [emap])
+    used = np.unique(ids)
+    for hold in (used, used[:0], used[:1], used[-1:], used[1:], used[::2], used[: len(used) // 2], used):
+        keep = torch.zeros(E, dtype=torch.bool, device=DEV)
+        keep[torch.from_numpy(hold).long().to(DEV)] = True
+        emap.copy_(torch.where(keep, torch.arange(E, dtype=torch.int32, device=DEV), -1))
+        out.fill_(float("nan"))
+        graph.replay()
+        got = out.clone()
+        out.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(out, got)
+        moe.run_layer(x, wt, it, pack, out, ws, [emap])
+        assert torch.equal(out, got)
+        want = moe.forward_mixed(x, wt, torch.where(keep[it.long()], it, -1), pack).float()
+        torch.cuda.synchronize()
+        if len(hold) == 0:
+            assert not got.any()
+            continue
+        assert float((got.float() - want).norm() / want.norm()) <= (4e-3 if dtype == torch.bfloat16 else 1e-3)
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    assert lib.exl3_device_error(ws.data_ptr(), ws.numel(), st) == 0

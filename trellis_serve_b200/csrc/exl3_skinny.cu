@@ -1,4 +1,5 @@
 // Host side of the decode GEMV / skinny GEMM: work split, shared-memory plan, dispatch on K.
+#include <climits>
 #include <cstring>
 
 #include "exl3_skinny_kernel.cuh"
@@ -55,8 +56,8 @@ int skinny_init_device()
 }
 
 // Work split and shared-memory plan of one launch; `x`: SK_STREAM or one of the modes that keep a slot of activations per unit.  aligned: CTAs
-// may get column blocks or equal parts of them instead of even ranges.
-static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligned, SkinnyLaunch& l, size_t& smem)
+// may get column blocks or equal parts of them instead of even ranges.  slots: of routed experts, or 0.
+static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligned, int slots, SkinnyLaunch& l, size_t& smem)
 {
     memset(&l, 0, sizeof(l));
     l.a = a;
@@ -64,47 +65,8 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.NB = a.n_total / 128;
     const long long units = (long long)l.KG * l.NB;
     const int ctas = d->sm_count < GEMV_MAX_GRID ? d->sm_count : GEMV_MAX_GRID;
-    size_t most = (size_t)((units + ctas - 1) / ctas);       // units of the busiest CTA
-    l.piece = 1;
-    if (aligned) {
-        // Every way of dealing the units has a cost, counted in units of the busiest CTA (0.5 us each up to 16 rows).  Partial sums that
-        // CTAs exchange take 2.5 us on top of whole column blocks; a range that starts and ends inside column blocks, evenly as it is, hands
-        // over twice: 1 us, 2 and more from nine rows up, where the hand-over is longer.  Chained launches, us, even ranges against the
-        // choice here: whole blocks, K = 3: 1024 x 8192 8.9 / 6.7 at one row, 1024 x 17408 10.7 / 8.6, 16.3 / 11.1 at 16, 21.2 / 17.6 at 57;
-        // parts: 4096 x 4096, K = 4 9.6 / 8.8, 1792 x 4096 8.7 / 6.9 at one row, 18.6 / 10.1 at 16, 27.5 / 16.0 at 57, 5120 x 5120 18.6 / 15.9
-        // at 16.  Where the rule stays with even ranges: 5120 x 5120, one row 11.2, in three parts (14 units for 11) 11.7; 17408 x 5120 24.9,
-        // 27.5; 2048 x 25088, whole blocks (32 units for 22) 18.0, 18.8.  In a long range of few rows all hand-overs but the last are hidden:
-        // 5120 x 34816, one row 43.3, whole blocks (80 units for 74) 44.1, but 50.0 / 46.8 at 16 rows.
-        constexpr int EXCHANGE = 5;
-        const int uneven = a.rows > 8 ? 4 : 2, hidden = a.rows <= 8 && most > 12 ? 3 : 0;
-        const bool few = x == SK_ROTATE && a.rows > SK_FUSED_ROWS;           // rows rotated inside in one pass of the decode warps
-        const long long whole = (long long)((l.NB + ctas - 1) / ctas) * l.KG;
-        long long best = (long long)most + EXCHANGE + uneven;
-        if (whole + hidden < best && !(few && whole > SK_DECODE_WARPS)) {
-            best = whole + hidden;
-            l.piece = l.KG;
-        }
-        // Parts get shorter with their number: the fewest of the shortest that the grid has room for.  Trying each number in turn, twice per
-        // call, showed in the smallest calls.
-        const int room = l.NB < ctas ? (ctas / l.NB < l.KG ? ctas / l.NB : l.KG) : 1;
-        if (room > 1) {
-            const int part = (l.KG + room - 1) / room;
-            if (part + EXCHANGE < best && !(few && part > SK_DECODE_WARPS)) {
-                l.parts = (l.KG + part - 1) / part;
-                l.piece = 1;
-            }
-        }
-    }
-    if (l.parts) {
-        l.grid = l.parts * l.NB;
-        most = (size_t)((l.KG + l.parts - 1) / l.parts);
-    } else {
-        const long long pieces = units / l.piece;
-        l.grid = pieces < ctas ? (int)pieces : ctas;
-        l.units_q = (int)(pieces / l.grid);
-        l.units_r = (int)(pieces % l.grid);
-        most = (size_t)(l.units_q + (l.units_r ? 1 : 0)) * l.piece;
-    }
+    l.deal = sk_deal(l.NB, l.KG, ctas, a.rows, x == SK_ROTATE && a.rows > SK_FUSED_ROWS, INT_MAX, aligned);
+    const size_t most = (size_t)l.deal.most;
     // Stages of whole units, as long as three fit; a short range travels as one copy.  A bulk copy costs a few hundred nanoseconds whatever
     // its size (24 KB of weights or more), and a group of decode warps changes stages every 2 units / 3 steps: six units where the
     // rows are resident (17408 x 5120, one row, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1, K
@@ -113,7 +75,7 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     const size_t w = 2048u * (size_t)a.K, f = (size_t)operand_pitch(a.rows) * (a.mode == GEMV_SPLIT ? 512 : 256);
     const SkRaw raw = sk_raw_planes(x, a.x_glu);
     const size_t planes = x == SK_STREAM ? 0 : (size_t)(raw.planes_const + a.rows * raw.planes_row);
-    const size_t fixed = SK_BAR_BYTES + (x == SK_STREAM ? 0 : most * f + planes * (most * 256 + 16)) + (size_t)a.rows * 512 + 1024;
+    const size_t fixed = SK_BAR_BYTES + (x == SK_STREAM ? 0 : most * f + planes * (most * 256 + 16)) + (size_t)a.rows * 512 + 1024 + slots * sizeof(int2);
     if (fixed >= (size_t)d->max_smem_optin) return EXL3_ERR_UNSUPPORTED_ROWS;
     const size_t budget = (size_t)d->max_smem_optin - fixed, unit = w + (x == SK_STREAM ? f : 0);
     size_t ups = (24 * 1024 + w - 1) / w;
@@ -134,8 +96,9 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.r_off = (uint32_t)(l.x_off + (x == SK_STREAM ? stages * ups : most) * f);
     l.r_plane = (uint32_t)(most * 256 + 16);              // 16 bytes apart in the banks: eight rows are read together
     l.p_off = (uint32_t)(l.r_off + planes * l.r_plane);
+    l.s.list_off = (uint32_t)(l.p_off + (size_t)a.rows * 512);
     // Rows behind the last real one are read from whatever follows (their products are dropped): never past the allocation.
-    smem = l.p_off + (size_t)a.rows * 512 + 1024;
+    smem = l.s.list_off + slots * sizeof(int2) + 1024;
     const CodebookConst c = codebook_const(a.codebook);
     l.mul = c.mul;
     l.add = c.add;
@@ -143,10 +106,10 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     return EXL3_OK;
 }
 
-static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaunch& l, size_t& smem)
+static int plan_skinny(const GemvArgs& a, const DeviceInfo* d, int x, SkinnyLaunch& l, size_t& smem, int slots = 0)
 {
-    const int rc = plan_split(a, d, x, true, l, smem);
-    return rc == EXL3_OK || (l.piece == 1 && l.parts == 0) ? rc : plan_split(a, d, x, false, l, smem);      // the busiest CTA's rows may not fit
+    const int rc = plan_split(a, d, x, true, slots, l, smem);
+    return rc == EXL3_OK || (l.deal.piece == 1 && l.deal.parts == 0) ? rc : plan_split(a, d, x, false, slots, l, smem);      // the busiest CTA's rows may not fit
 }
 
 bool skinny_rotates_input(const GemvArgs& a)
@@ -208,7 +171,7 @@ bool skinny_serves_slots(int slots, int hidden, int inter, int K, int codebook)
         if (blocks * 128 >= (1ll << 31) || blocks > (long long)WS_MAX_COUNTERS || blocks > 2048 || units > (long long)SK_SLOTS_UNITS * d->sm_count) return false;
         SkinnyLaunch l;
         size_t smem;
-        if (plan_skinny(slots_args(slots, k, n, down, K, codebook), d, SK_ROTATE, l, smem) != EXL3_OK) return false;
+        if (plan_skinny(slots_args(slots, k, n, down, K, codebook), d, SK_ROTATE, l, smem, slots) != EXL3_OK) return false;
     }
     return true;
 }
@@ -231,8 +194,8 @@ int launch_skinny_slots(const void* x, int x_bf16, int per_row, const int* ids, 
     a.err = err;
     SkinnyLaunch l;
     size_t smem = 0;
-    if (int rc = plan_skinny(a, d, SK_ROTATE, l, smem)) return rc;
-    l.s = {ids, map, experts, local, n / 128, n / 128 / shards, per_row, known, (long long)k * n * K / 32};
+    if (int rc = plan_skinny(a, d, SK_ROTATE, l, smem, slots)) return rc;
+    l.s = {ids, map, experts, local, n / 128, n / 128 / shards, per_row, known, slots, l.s.list_off, (long long)k * n * K / 32};
     return launch_planned(l, SK_ROTATE, smem, st);
 }
 

@@ -33,23 +33,24 @@ static SkinnyKernel instance_for(int mode, int family, int pitch, int x, int res
     return mode == GEMV_SPLIT ? instance<K, GEMV_SPLIT, FAM_HASH>(pitch, x, residual) : instance<K, GEMV_PAIRED, FAM_HASH>(pitch, x, residual);
 }
 
-template <int K>
+template <int K, int SLOTS>
 static SkinnyKernel slots_instance(int mode, int family)
 {
-    if (family == FAM_MUL1) return skinny_kernel<K, GEMV_PAIRED, FAM_MUL1, 2, SK_ROTATE, 0, true>;
-    return mode == GEMV_SPLIT ? skinny_kernel<K, GEMV_SPLIT, FAM_HASH, 2, SK_ROTATE, 0, true> : skinny_kernel<K, GEMV_PAIRED, FAM_HASH, 2, SK_ROTATE, 0, true>;
+    if (family == FAM_MUL1) return skinny_kernel<K, GEMV_PAIRED, FAM_MUL1, 2, SK_ROTATE, 0, SLOTS>;
+    return mode == GEMV_SPLIT ? skinny_kernel<K, GEMV_SPLIT, FAM_HASH, 2, SK_ROTATE, 0, SLOTS> : skinny_kernel<K, GEMV_PAIRED, FAM_HASH, 2, SK_ROTATE, 0, SLOTS>;
 }
 
 template <>
 int launch_skinny_for_k<EXL3_SKINNY_K>(const SkinnyLaunch& l, int pitch, int x, size_t smem, cudaStream_t st)
 {
     const int family = codebook_family(l.a.codebook);
-    const SkinnyKernel kernel = l.s.ids ? slots_instance<EXL3_SKINNY_K>(l.a.mode, family)
-                                        : instance_for<EXL3_SKINNY_K>(l.a.mode, family, pitch, x, l.a.res_out != nullptr);
+    const SkinnyKernel kernel = l.s.map   ? slots_instance<EXL3_SKINNY_K, SK_HELD>(l.a.mode, family)
+                                : l.s.ids ? slots_instance<EXL3_SKINNY_K, SK_EACH>(l.a.mode, family)
+                                          : instance_for<EXL3_SKINNY_K>(l.a.mode, family, pitch, x, l.a.res_out != nullptr);
     if (!kernel) return EXL3_ERR_UNSUPPORTED_ROWS;
     // Programmatic stream serialization: prologue, weight copies and the first half units overlap the tail of the kernel ahead; the
     // kernel waits (griddepcontrol.wait) before touching anything that kernel wrote.
-    return launch_chained(kernel, dim3(l.grid), dim3(SK_THREADS), smem, st, l);
+    return launch_chained(kernel, dim3(l.deal.grid), dim3(SK_THREADS), smem, st, l);
 }
 
 template <>
@@ -60,7 +61,8 @@ int skinny_set_attributes_for_k<EXL3_SKINNY_K>(int max_smem)
     };
     for (int family : {FAM_HASH, FAM_MUL1})
         for (int mode : {GEMV_SPLIT, GEMV_PAIRED}) {
-            if (int rc = opt_in(slots_instance<EXL3_SKINNY_K>(mode, family))) return rc;
+            if (int rc = opt_in(slots_instance<EXL3_SKINNY_K, SK_EACH>(mode, family))) return rc;
+            if (int rc = opt_in(slots_instance<EXL3_SKINNY_K, SK_HELD>(mode, family))) return rc;
             for (int pitch : {2, 8, 16, 32, 64})
                 for (int x : {SK_STREAM, SK_ROTATE, SK_NORM})
                     for (int residual : {0, 1}) {

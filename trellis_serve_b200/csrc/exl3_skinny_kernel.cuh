@@ -50,7 +50,7 @@ constexpr int SK_THREADS = (SK_DECODE_WARP + SK_DECODE_WARPS) * 32;
 static_assert(SK_EPI_WARP % 4 == 0 && SK_DECODE_WARP % 4 == 0 && SK_THREADS == 1024, "roles of the skinny GEMM");
 constexpr int SK_MAX_STAGES = 8;
 constexpr int SK_TMEM_COLS = 512;
-constexpr uint32_t SK_BAR_BYTES = 512, SK_TABLE_OFF = 320;      // barriers, then the constants of the decode loop
+constexpr uint32_t SK_BAR_BYTES = 512, SK_TABLE_OFF = 320, SK_DEAL_OFF = 464;      // barriers, the constants of the decode loop, the deal of the slots
 // Named barriers (0 is __syncthreads): the epilogue warps among themselves, "input rotated", "buffer decoded" (group x buffer),
 // "column block multiplied".
 constexpr int SK_BAR_EPI = 1, SK_BAR_X = 2, SK_BAR_BUF = 3, SK_BAR_ACC = 12;
@@ -60,6 +60,8 @@ constexpr int SK_ROTATE_ROWS = 8;                               // largest row c
 // Where the B operand comes from: the workspace, streamed with the weights (written by a rotation or producer kernel ahead); x or
 // gate | up, rotated by this kernel; the residual stream, normalised and rotated by this kernel.
 enum { SK_STREAM = 0, SK_ROTATE = 1, SK_NORM = 2 };
+// Which matrices: the launch's own; routed experts of every slot, or of those that have one here (see SkSlots).
+enum { SK_DENSE = 0, SK_EACH = 1, SK_HELD = 2 };
 
 // Tensor memory: accumulators [buffers][group][N columns], then the A buffers.  Every group cycles through buffers of its own: a
 // wait by parity tells one fill of a barrier from the next, not from the one after, so a buffer must not pass between groups
@@ -75,31 +77,93 @@ struct SkTmem {
     static_assert(A_OFF + SK_GROUPS * A_BUFS * A_COLS <= SK_TMEM_COLS, "tensor memory");
 };
 
-// Routed experts of a few slots as one matrix: NB column blocks are `slots` runs of `blocks`, run s is the expert of slot s.
+// How column blocks of KG units are dealt to the CTAs.  parts == 0: pieces of `piece` units (one, or a whole column block) evenly and
+// contiguously, the first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.  most: units of
+// the busiest CTA.
+struct SkDeal {
+    int units_q, units_r, piece, parts, most, grid;
+};
+
+// The cheapest of the three ways for `ctas` CTAs, `limit` units at most in one of them (even ranges aside).  few: rows rotated inside in one
+// pass of the decode warps.
+//
+// Every way of dealing the units has a cost, counted in units of the busiest CTA (0.5 us each up to 16 rows).  Partial sums that
+// CTAs exchange take 2.5 us on top of whole column blocks; a range that starts and ends inside column blocks, evenly as it is, hands
+// over twice: 1 us, 2 and more from nine rows up, where the hand-over is longer.  Chained launches, us, even ranges against the
+// choice here: whole blocks, K = 3: 1024 x 8192 8.9 / 6.7 at one row, 1024 x 17408 10.7 / 8.6, 16.3 / 11.1 at 16, 21.2 / 17.6 at 57;
+// parts: 4096 x 4096, K = 4 9.6 / 8.8, 1792 x 4096 8.7 / 6.9 at one row, 18.6 / 10.1 at 16, 27.5 / 16.0 at 57, 5120 x 5120 18.6 / 15.9
+// at 16.  Where the rule stays with even ranges: 5120 x 5120, one row 11.2, in three parts (14 units for 11) 11.7; 17408 x 5120 24.9,
+// 27.5; 2048 x 25088, whole blocks (32 units for 22) 18.0, 18.8.  In a long range of few rows all hand-overs but the last are hidden:
+// 5120 x 34816, one row 43.3, whole blocks (80 units for 74) 44.1, but 50.0 / 46.8 at 16 rows.
+__host__ __device__ inline SkDeal sk_deal(int NB, int KG, int ctas, int rows, bool few, int limit, bool aligned)
+{
+#ifdef __CUDA_ARCH__
+    using Count = int;                                                      // of slots: far below 2^31
+#else
+    using Count = long long;
+#endif
+    const Count units = (Count)NB * KG;
+    SkDeal t = {0, 0, 1, 0, (int)((units + ctas - 1) / ctas), ctas};
+    if (aligned) {
+        constexpr int EXCHANGE = 5;
+        const int uneven = rows > 8 ? 4 : 2, hidden = rows <= 8 && t.most > 12 ? 3 : 0;
+        const Count whole = (Count)((NB + ctas - 1) / ctas) * KG;
+        Count best = (Count)t.most + EXCHANGE + uneven;
+        if (whole + hidden < best && whole <= limit && !(few && whole > SK_DECODE_WARPS)) {
+            best = whole + hidden;
+            t.piece = KG;
+        }
+        // Parts get shorter with their number: the fewest of the shortest that the grid has room for.  Trying each number in turn, twice per
+        // call, showed in the smallest calls.
+        const int room = NB < ctas ? (ctas / NB < KG ? ctas / NB : KG) : 1;
+        if (room > 1) {
+            const int part = (KG + room - 1) / room;
+            if (part + EXCHANGE < best && part <= limit && !(few && part > SK_DECODE_WARPS)) {
+                t.parts = (KG + part - 1) / part;
+                t.piece = 1;
+            }
+        }
+    }
+    if (t.parts) {
+        t.grid = t.parts * NB;
+        t.most = (KG + t.parts - 1) / t.parts;
+    } else {
+        const Count pieces = units / t.piece;
+        t.grid = pieces < ctas ? (int)pieces : ctas;
+        t.units_q = (int)(pieces / t.grid);
+        t.units_r = (int)(pieces % t.grid);
+        t.most = (t.units_q + (t.units_r ? 1 : 0)) * t.piece;
+    }
+    return t;
+}
+
+// Routed experts of a few slots as one matrix: the column blocks are runs of `blocks`, run v is the expert of slot v -- or, with a map, of the
+// v-th slot that has an expert here.
 struct SkSlots {
-    const int* ids;             // expert of each slot (a router's), `map`: -> this rank's or class's expert, or -1; null: as it is
-    const int* map;
+    const int* ids;             // expert of each slot (a router's)
+    const int* map;             // -> this rank's or class's expert, or -1; null: as it is
     int experts, local;         // ids in [0, experts); experts behind the pointers
     int blocks, shard_blocks;   // column blocks of an expert, of one of its matrices with sign vectors of their own (gate, up)
     int per_row;                // slots that share a row of x (top-k, or 1)
     int known;                  // the ids were there before the kernel ahead began: read ahead of the wait
+    int slots;
+    uint32_t list_off;          // with a map, bytes: the slots that have an expert here, (slot, expert) each
     long long stride;           // 32-bit words between experts
 
-    __device__ __forceinline__ int expert(int s) const
+    __device__ __forceinline__ int expert(int s) const                      // without a map
     {
-        int e = __ldcg(ids + s);
-        if (map) e = e >= 0 && e < experts ? __ldcg(map + e) : -1;
+        const int e = __ldcg(ids + s);
         return e >= 0 && e < local ? e : -1;
     }
 };
 
+static_assert(SK_DEAL_OFF >= SK_TABLE_OFF + 35 * 4 && SK_DEAL_OFF + sizeof(SkDeal) + sizeof(int2) <= SK_BAR_BYTES, "head of the shared memory");
+
 struct SkinnyLaunch {
     GemvArgs a;
     SkSlots s;
-    int KG, NB, grid;
-    // How the units are dealt to the CTAs.  parts == 0: pieces of `piece` units (one, or a whole column block) evenly and contiguously, the
-    // first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.
-    int units_q, units_r, piece, parts;
+    int KG, NB;
+    SkDeal deal;
     int stages, units_per_stage;
     uint32_t x_off, p_off;      // bytes: activations behind the weights, staged rows of the epilogue
     uint32_t r_off, r_plane;    // raw input of the in-kernel rotation (see SkRaw), bytes per plane
@@ -341,10 +405,10 @@ __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsi
 
 // The finished sums of column block nb -> output, rows w, w + nw, ... of a warp.  shared: the block's partial sums of CTAs c_first ..
 // c_last are added in CTA order; several rows and CTAs are requested together, so that their round trips overlap.
-// svh: so that svh + 128 nb are the block's.
+// svh: so that svh + 128 nb_out are the block's; nb_out: where it stands in the output.
 template <int RB, int EPI>
 __device__ __forceinline__ void sk_finish_block(const GemvArgs& a, const __half* svh, uint32_t tp_epoch, const float* P, bool shared, int c_first, int c_last,
-                                                int nb, int w, int nw, int lane)
+                                                int nb, int nb_out, int w, int nw, int lane)
 {
     constexpr int CB = 8 / RB;
     const int rows = a.rows;
@@ -383,7 +447,7 @@ __device__ __forceinline__ void sk_finish_block(const GemvArgs& a, const __half*
         }
 #pragma unroll 1
         for (int i = 0; i < RB; i++) {
-            if (m + nw * i < rows) gemv_finish_row<EPI>(a, svh, tp_epoch, make_float4(v[0][0], v[0][1], v[0][2], v[0][3]), m + nw * i, nb, lane);
+            if (m + nw * i < rows) gemv_finish_row<EPI>(a, svh, tp_epoch, make_float4(v[0][0], v[0][1], v[0][2], v[0][3]), m + nw * i, nb_out, lane);
 #pragma unroll
             for (int j = 0; j + 1 < RB; j++)
 #pragma unroll
@@ -396,16 +460,22 @@ template <int RB, int EPI>
 static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint32_t tp_epoch, const float* P, bool shared, int c_first, int c_last,
                                                          int nb, int w, int nw, int lane)
 {
-    sk_finish_block<RB, EPI>(a, a.svh, tp_epoch, P, shared, c_first, c_last, nb, w, nw, lane);
+    sk_finish_block<RB, EPI>(a, a.svh, tp_epoch, P, shared, c_first, c_last, nb, nb, w, nw, lane);
 }
 
 // RP: operand pitch, the rows rounded up (operand_pitch).
-// SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.
-template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0, bool SLOTS = false>
+// SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.  SK_EACH: every slot as it stands; one whose id is out of range decodes
+// expert 0 and drops the result.  SK_HELD, for ids with a map (a rank's share of the experts, bitrate classes): every CTA makes the same list of
+// the slots that have an expert here, and where that is not all of them their units are dealt anew, so that the others cost nothing: 256
+// experts of 2048 x 512, top-8, K = 3, us per layer in a chain, a rank with 128 / 64 / 32 of them: one token 22.0 / 16.7 / 14.4, two tokens
+// 25.5 / 21.3 / 16.1 (every slot decoded 23.3 / 23.0 / 22.5 and 31.4 / 31.2 / 30.7, blocks of eight rows 29.9 / 23.5 / 19.3 and 32.5 / 29.5 /
+// 24.1); four classes of 64, two tokens 71 (108).  Where every slot has an expert the list costs 0.3 us a layer (20.8, 21.1 with it), which is
+// why SK_EACH stays.
+template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0, int SLOTS = SK_DENSE>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_constant__ SkinnyLaunch p)
 {
     static_assert((X != SK_NORM && EPI == 0) || RP == SK_FUSED_ROWS, "the kernel normalises, and carries the residual stream of, one or two rows");
-    static_assert(!SLOTS || (X == SK_ROTATE && RP == SK_FUSED_ROWS && EPI == 0), "slots come one row each");
+    static_assert(SLOTS == SK_DENSE || (X == SK_ROTATE && RP == SK_FUSED_ROWS && EPI == 0), "slots come one row each");
     static_assert(X != SK_ROTATE || RP <= SK_ROTATE_ROWS, "the kernel rotates up to eight rows");
     constexpr int RB = RP <= 8 ? 1 : RP <= 16 ? 2 : 4;                      // rows that a warp finishes together
     constexpr bool ALL_FINISH = RP >= 16;
@@ -430,37 +500,59 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
     const int cta = blockIdx.x, rows = p.a.rows;
-    int u0, u1;
-    if (p.parts > 0) {
-        const int nb = cta / p.parts, part = cta - nb * p.parts;
-        u0 = nb * p.KG + part * p.KG / p.parts;
-        u1 = nb * p.KG + (part + 1) * p.KG / p.parts;
-    } else {
-        u0 = (int)gemv_first_unit(cta, p.units_q, p.units_r) * p.piece;
-        u1 = (int)gemv_first_unit(cta + 1, p.units_q, p.units_r) * p.piece;
-    }
-    auto sharers = [&](int nb, int& first, int& last) {                     // CTAs that share column block nb
-        if (p.parts > 0) {
-            first = nb * p.parts;
-            last = first + p.parts - 1;
-        } else if (p.piece > 1) {
+    const int ups = p.units_per_stage, stages = p.stages;
+    int u0, u1, halves, fills;                                              // units [u0, u1)
+    auto take = [&](const SkDeal& t) {
+        if (t.parts > 0) {
+            const int nb = cta / t.parts, part = cta - nb * t.parts;
+            u0 = nb * p.KG + part * p.KG / t.parts;
+            u1 = nb * p.KG + (part + 1) * p.KG / t.parts;
+        } else {
+            u0 = (int)gemv_first_unit(cta, t.units_q, t.units_r) * t.piece;
+            u1 = (int)gemv_first_unit(cta + 1, t.units_q, t.units_r) * t.piece;
+        }
+        if (SLOTS == SK_HELD && cta >= t.grid) u1 = u0;                                // fewer slots than the grid was launched for
+    };
+    auto count = [&]() {
+        halves = 2 * (u1 - u0);
+        fills = (u1 - u0 + ups - 1) / ups;
+    };
+    // SK_HELD: what the copy warp made of the ids.
+    [[maybe_unused]] SkDeal* dealt = reinterpret_cast<SkDeal*>(smem + SK_DEAL_OFF);
+    [[maybe_unused]] int2* range = reinterpret_cast<int2*>(dealt + 1);
+    [[maybe_unused]] int2* list = reinterpret_cast<int2*>(smem + p.s.list_off);
+    [[maybe_unused]] auto run_of = [&](int v) { return SLOTS == SK_HELD ? list[v] : make_int2(v, p.s.expert(v)); };      // (slot, expert or -1)
+    take(p.deal);
+    count();
+    auto sharers_in = [&](const SkDeal& t, int nb, int& first, int& last) {
+        if (t.parts > 0) {
+            first = nb * t.parts;
+            last = first + t.parts - 1;
+        } else if (t.piece > 1) {
             first = last = cta;
         } else {
-            first = gemv_cta_of_unit((long long)nb * p.KG, p.units_q, p.units_r);
-            last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, p.units_q, p.units_r);
+            first = gemv_cta_of_unit((long long)nb * p.KG, t.units_q, t.units_r);
+            last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, t.units_q, t.units_r);
         }
     };
-    const int ups = p.units_per_stage, stages = p.stages;
-    const int halves = 2 * (u1 - u0), fills = (u1 - u0 + ups - 1) / ups;
+    auto sharers = [&](int nb, int& first, int& last) {                     // CTAs that share column block nb
+        if constexpr (SLOTS == SK_HELD) {
+            sharers_in(*dealt, nb, first, last);
+            first = __shfl_sync(0xFFFFFFFFu, first, 0);
+            last = __shfl_sync(0xFFFFFFFFu, last, 0);
+        } else {
+            sharers_in(p.deal, nb, first, last);
+        }
+    };
 
     auto weights = [&](int j, int slot) {                                   // one thread: fill number j, units [u0 + j * ups, ...)
         const int u = u0 + j * ups, n = u1 - u < ups ? u1 - u : ups;
         ptx::mbar_arrive_expect_tx(&w_full[slot], (uint32_t)n * W_BYTES);
-        if constexpr (SLOTS) {
+        if constexpr (SLOTS != SK_DENSE) {
             const int per = p.s.blocks * p.KG;                              // units of an expert
             unsigned char* dst = wring + (size_t)(slot * ups) * W_BYTES;
             for (int at = u; at < u + n;) {
-                const int sl = at / per, in = at - sl * per, run = per - in < u + n - at ? per - in : u + n - at, e = p.s.expert(sl);
+                const int sl = at / per, in = at - sl * per, run = per - in < u + n - at ? per - in : u + n - at, e = run_of(sl).y;
                 ptx::bulk_g2s(dst, p.a.packed + (e < 0 ? 0 : e) * p.s.stride + (long long)in * (512 * K), (uint32_t)run * W_BYTES, &w_full[slot]);
                 dst += (size_t)run * W_BYTES;
                 at += run;
@@ -473,12 +565,13 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     [[maybe_unused]] auto rows_of_slots = [&](unsigned char* dst, int row, uint64_t* bar) {
         for (int u = u0; u < u1;) {
             const int unb = u / p.KG, ukg = u - unb * p.KG, run = p.KG - ukg < u1 - u ? p.KG - ukg : u1 - u;
-            const int sl = unb / p.s.blocks, nb = unb - sl * p.s.blocks;
+            const int v = unb / p.s.blocks, nb = unb - v * p.s.blocks;
             const unsigned char* src;
             if (row >= 0) {
-                src = reinterpret_cast<const unsigned char*>(p.a.x) + ((long long)(sl / p.s.per_row) * sk_raw_planes(X, p.a.x_glu).planes_row + row) * 2 * p.a.k;
+                const int slot = SLOTS == SK_HELD ? list[v].x : v;
+                src = reinterpret_cast<const unsigned char*>(p.a.x) + ((long long)(slot / p.s.per_row) * sk_raw_planes(X, p.a.x_glu).planes_row + row) * 2 * p.a.k;
             } else {
-                const int e = p.s.expert(sl);
+                const int e = run_of(v).y;
                 src = reinterpret_cast<const unsigned char*>(p.a.suh) + ((long long)(e < 0 ? 0 : e) * (p.s.blocks / p.s.shard_blocks) + nb / p.s.shard_blocks) * 2 * p.a.k;
             }
             ptx::bulk_g2s(dst, src + ukg * 256, (uint32_t)run * 256u, bar);
@@ -501,6 +594,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     };
     EXL3_STAMP(0);
     if (warp == SK_COPY_WARP) {
+        auto constants = [&]() {                                            // one thread: before the kernel ahead has finished
+            for (int j = 0; j < stages && j < fills; j++) weights(j, j);
+            if constexpr (X != SK_STREAM) {
+                const int n = u1 - u0;
+                ptx::mbar_arrive_expect_tx(&x_full[1], (uint32_t)(n * sk_raw_planes(X, 0).planes_const) * 256u);
+                if constexpr (SLOTS != SK_DENSE) rows_of_slots(smem + p.r_off, -1, &x_full[1]);
+                else rows_of(u0, n, smem + p.r_off, p.a.suh, 256, 2ll * p.a.k, &x_full[1]);
+                if constexpr (X == SK_NORM) rows_of(u0, n, smem + p.r_off + p.r_plane, p.a.norm_weight, 256, 0, &x_full[1]);
+            }
+        };
         if (lane == 0) {
             for (int s = 0; s < SK_MAX_STAGES; s++) {
                 ptx::mbar_init(&w_full[s], 1);
@@ -511,16 +614,47 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             for (int g = 0; g < SK_GROUPS; g++) ptx::mbar_init(&acc_done[g], 1);
             for (int d = 0; d < TM::ACC_BUFS; d++) ptx::mbar_init(&acc_empty[d], 4);
             ptx::mbar_fence_init();
-            if constexpr (SLOTS) {
+            if constexpr (SLOTS == SK_EACH) {
                 if (!p.s.known) ptx::grid_dependency_wait();                // the ids
             }
-            for (int j = 0; j < stages && j < fills; j++) weights(j, j);    // constants: before the kernel ahead has finished
-            if constexpr (X != SK_STREAM) {
-                const int n = u1 - u0;
-                ptx::mbar_arrive_expect_tx(&x_full[1], (uint32_t)(n * sk_raw_planes(X, 0).planes_const) * 256u);
-                if constexpr (SLOTS) rows_of_slots(smem + p.r_off, -1, &x_full[1]);
-                else rows_of(u0, n, smem + p.r_off, p.a.suh, 256, 2ll * p.a.k, &x_full[1]);
-                if constexpr (X == SK_NORM) rows_of(u0, n, smem + p.r_off + p.r_plane, p.a.norm_weight, 256, 0, &x_full[1]);
+            if constexpr (SLOTS != SK_HELD) constants();
+        }
+        if constexpr (SLOTS == SK_HELD) {
+            SkDeal t = p.deal;
+            int held = 0;
+            auto look = [&](int s0, auto count) {                           // 32 `count` slots whose round trips overlap
+                constexpr int C = decltype(count)::value;
+                int e[C];
+#pragma unroll
+                for (int i = 0; i < C; i++) e[i] = s0 + 32 * i + lane < p.s.slots ? __ldcg(p.s.ids + s0 + 32 * i + lane) : -1;
+#pragma unroll
+                for (int i = 0; i < C; i++) e[i] = e[i] >= 0 && e[i] < p.s.experts ? __ldcg(p.s.map + e[i]) : -1;
+#pragma unroll
+                for (int i = 0; i < C; i++) {
+                    const bool has = e[i] >= 0 && e[i] < p.s.local;
+                    const uint32_t have = __ballot_sync(0xFFFFFFFFu, has);
+                    if (has) list[held + __popc(have & ((1u << lane) - 1))] = make_int2(s0 + 32 * i + lane, e[i]);
+                    held += __popc(have);
+                }
+            };
+            if (!p.s.known) ptx::grid_dependency_wait();                    // the ids
+            if (p.s.slots <= 32) {
+                look(0, std::integral_constant<int, 1>{});
+            } else {
+#pragma unroll 1
+                for (int s0 = 0; s0 < p.s.slots; s0 += 128) look(s0, std::integral_constant<int, 4>{});
+            }
+            if (held < p.s.slots) {
+                t = {0, 0, 1, 0, 0, 0};
+                if (held > 0) t = sk_deal(held * p.s.blocks, p.KG, (int)gridDim.x, 1, false, p.deal.most, true);
+                take(t);
+                count();
+            }
+            __syncwarp();
+            if (lane == 0) {
+                if (u0 < u1) constants();
+                *dealt = t;
+                *range = make_int2(u0, u1);
             }
         }
     } else if (warp == SK_MMA_WARP) {
@@ -535,13 +669,22 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     sk_fence_after();
     // All 512 columns are this CTA's: tensor memory starts at address 0, which keeps the addresses warp-uniform constants.
     uint32_t failed = *tmem_slot != 0;
-    if constexpr (SLOTS) {
+    if constexpr (SLOTS == SK_HELD) {
+        // Warp-uniform to the compiler, as the host's deal is: the loops of the MMA warps run over these (1.3 us a layer otherwise).
+        const int2 mine = *range;
+        u0 = __shfl_sync(0xFFFFFFFFu, mine.x, 0);
+        u1 = __shfl_sync(0xFFFFFFFFu, mine.y, 0);
+        count();
+    }
+    if constexpr (SLOTS != SK_DENSE) {
         // The kernel behind may look at the ids as soon as it begins: not before the kernel that wrote them has finished.
         if (!p.s.known) ptx::grid_dependency_wait();
     }
     ptx::grid_launch_dependents();                                          // the next kernel in the stream may begin its prologue
 
-    if (warp >= SK_DECODE_WARP) {
+    if (SLOTS == SK_HELD && u0 >= u1) {
+        ptx::grid_dependency_wait();                                        // nothing for this CTA
+    } else if (warp >= SK_DECODE_WARP) {
         // ------------------------------------------------------------------ decode
         const int dw = warp - SK_DECODE_WARP, group = dw >> 3, nt = 2 * (dw & 3) + ((dw >> 2) & 1);  // columns 16 nt .. = tensor-memory lanes of this warp's quarter
         const uint32_t table = ptx::smem_addr(smem + SK_TABLE_OFF);
@@ -740,7 +883,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 unsigned char* dst = smem + p.r_off + sk_raw_planes(X, p.a.x_glu).planes_const * p.r_plane;
                 ptx::mbar_arrive_expect_tx(&x_full[0], (uint32_t)(n * rows * row_planes) * 256u);
                 for (int q = 0; q < rows * row_planes; q++, x += 2 * p.a.k, dst += p.r_plane) {
-                    if constexpr (SLOTS) rows_of_slots(dst, q, &x_full[0]);
+                    if constexpr (SLOTS != SK_DENSE) rows_of_slots(dst, q, &x_full[0]);
                     else rows_of(u0, n, dst, x, 256, 0, &x_full[0]);
                 }
             }
@@ -785,11 +928,14 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             const size_t nelem = (size_t)rows * 128;
             float* dst = (shared ? p.a.partials + (size_t)(cta + nb) * nelem : P) + ew * 32 + lane;
             const __half* svh = p.a.svh;
-            [[maybe_unused]] bool held = true;                              // SLOTS: the slot's expert is one of these
-            if constexpr (SLOTS) {
-                const int sl = nb / p.s.blocks, e = p.s.expert(sl);
-                held = e >= 0;
-                svh += (long long)(e - sl) * p.s.blocks * 128;
+            int nb_out = nb;
+            [[maybe_unused]] bool held = true;                              // SLOTS: the slot has an expert
+            if constexpr (SLOTS != SK_DENSE) {
+                const int v = nb / p.s.blocks;
+                const int2 run = run_of(v);
+                held = run.y >= 0;
+                nb_out += (run.x - v) * p.s.blocks;
+                svh += (long long)(run.y - run.x) * p.s.blocks * 128;
             }
             ptx::named_bar_sync(SK_BAR_ACC + d, (SK_GROUPS + 4) * 32);
             sk_fence_after();
@@ -840,7 +986,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             }
             if (finish && held) {
                 if constexpr (ALL_FINISH) sk_finish_block_call<RB, EPI>(p.a, tp_epoch, P, shared, c_first, c_last, nb, ew, 4, lane);
-                else sk_finish_block<RB, EPI>(p.a, svh, tp_epoch, P, shared, c_first, c_last, nb, ew, 4, lane);
+                else sk_finish_block<RB, EPI>(p.a, svh, tp_epoch, P, shared, c_first, c_last, nb, nb_out, ew, 4, lane);
             }
             EXL3_STAMP_LANE(ew == 0, 7);
             ptx::named_bar_sync(SK_BAR_EPI, 128);                           // staged rows and flag may be overwritten
