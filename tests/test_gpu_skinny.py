@@ -100,3 +100,15 @@ def test_column_blocks_and_parts_of_them(rows, k, n, K, cb):
     want = _had128(lin.had_in_group(x, suh).float() @ lin.reconstruct_packed(packed, cb).float()) * svh.float()
     assert float((y - want).norm() / want.norm()) <= 1e-3
     assert float((y - want).abs().max() / want.pow(2).mean().sqrt()) <= 2e-3
+
+
+@pytest.mark.parametrize("rows,k,n,K,cb", [
+    (1, 8576, 36864, 3, 0),     # 134 units in whole column blocks, 131 in even ranges
+    (2, 10368, 36992, 3, 2),    # 162 and 159
+    (5, 1024, 47488, 8, 0),     # 24 and 21
+    (8, 896, 46080, 8, 1),      # 21 and 18
+])
+def test_even_ranges_where_the_rows_of_whole_column_blocks_do_not_fit(rows, k, n, K, cb):
+    """Sizes for which whole column blocks cost less but the busiest CTA's rotated and raw rows (1792 bytes a unit for two rows split, 6400 for
+    eight) leave no room for a ring of stages in 227 KB, while those of even ranges do."""
+    test_column_blocks_and_parts_of_them(rows, k, n, K, cb)
