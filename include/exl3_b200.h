@@ -343,7 +343,7 @@ exl3_status exl3_moe_combine(const uint16_t *yd, const float *topk_weights, cons
  * with a matrix of its own, two launches of the decode kernel, which rotates its input itself (the second one SiLU(gate) * up).
  * exl3_moe_prefers_slots: 1 where that is the faster way (no more slots than experts, and no more than 16 units of 128 x 128 weights per SM
  * and launch).  A layer of one token, 256 experts of 2048 x 512, top-8, K = 3, takes 21.6 us for 30.2; two tokens 29.9 for 36.  With an
- * expert_map the slots whose expert it leaves out cost nothing (a rank with 32 of the 256 experts: 14.4 us for 19.3, two tokens 16.1 for
+ * expert_map the slots whose expert it leaves out cost nothing (a rank with 32 of the 256 experts: 13.6 us for 19.3, two tokens 16.0 for
  * 24.1); their rows of yd are not written.
  * exl3_moe_slots_experts: topk_ids -> yd[slot, :] as exl3_moe_tc_experts gives it (expert_map as there), gu: scratch fp16 [slots, 2 *
  * inter]; x, gu, weights and suh 16-byte aligned; workspace as for exl3_moe_gemm.  The launch structure this replaces for one token is that of

@@ -65,8 +65,8 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.NB = a.n_total / 128;
     const long long units = (long long)l.KG * l.NB;
     const int ctas = d->sm_count < GEMV_MAX_GRID ? d->sm_count : GEMV_MAX_GRID;
-    l.deal = sk_deal(l.NB, l.KG, ctas, a.rows, x == SK_ROTATE && a.rows > SK_FUSED_ROWS, INT_MAX, aligned);
-    const size_t most = (size_t)l.deal.most;
+    l.deal = sk_deal(l.NB, l.KG, ctas, a.rows, x == SK_ROTATE && a.rows > SK_FUSED_ROWS, INT_MAX, aligned, l.most);
+    const size_t most = (size_t)l.most;
     // Stages of whole units, as long as three fit; a short range travels as one copy.  A bulk copy costs a few hundred nanoseconds whatever
     // its size (24 KB of weights or more), and a group of decode warps changes stages every 2 units / 3 steps: six units where the
     // rows are resident (17408 x 5120, one row, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1, K
@@ -96,12 +96,13 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.r_off = (uint32_t)(l.x_off + (x == SK_STREAM ? stages * ups : most) * f);
     l.r_plane = (uint32_t)(most * 256 + 16);              // 16 bytes apart in the banks: eight rows are read together
     l.p_off = (uint32_t)(l.r_off + planes * l.r_plane);
-    l.s.list_off = (uint32_t)(l.p_off + (size_t)a.rows * 512);
+    l.list_off = (uint32_t)(l.p_off + (size_t)a.rows * 512);
     // Rows behind the last real one are read from whatever follows (their products are dropped): never past the allocation.
-    smem = l.s.list_off + slots * sizeof(int2) + 1024;
+    smem = l.list_off + slots * sizeof(int2) + 1024;
     const CodebookConst c = codebook_const(a.codebook);
     l.mul = c.mul;
     l.add = c.add;
+    l.slots = slots;
     l.xf_shard_stride = (long long)l.KG * (long long)f;
     return EXL3_OK;
 }
@@ -195,7 +196,7 @@ int launch_skinny_slots(const void* x, int x_bf16, int per_row, const int* ids, 
     SkinnyLaunch l;
     size_t smem = 0;
     if (int rc = plan_skinny(a, d, SK_ROTATE, l, smem, slots)) return rc;
-    l.s = {ids, map, experts, local, n / 128, n / 128 / shards, per_row, known, slots, l.s.list_off, (long long)k * n * K / 32};
+    l.s = {ids, map, experts, local, n / 128, n / 128 / shards, per_row, known, (long long)k * n * K / 32};
     return launch_planned(l, SK_ROTATE, smem, st);
 }
 

@@ -50,7 +50,8 @@ constexpr int SK_THREADS = (SK_DECODE_WARP + SK_DECODE_WARPS) * 32;
 static_assert(SK_EPI_WARP % 4 == 0 && SK_DECODE_WARP % 4 == 0 && SK_THREADS == 1024, "roles of the skinny GEMM");
 constexpr int SK_MAX_STAGES = 8;
 constexpr int SK_TMEM_COLS = 512;
-constexpr uint32_t SK_BAR_BYTES = 512, SK_TABLE_OFF = 320, SK_DEAL_OFF = 464;      // barriers, the constants of the decode loop, the deal of the slots
+constexpr uint32_t SK_BAR_BYTES = 512, SK_TABLE_OFF = 320, SK_RANGE_OFF = 464, SK_DEAL_OFF = 472;
+                                                                // barriers, the constants of the decode loop, a CTA's units and their deal (SK_HELD)
 // Named barriers (0 is __syncthreads): the epilogue warps among themselves, "input rotated", "buffer decoded" (group x buffer),
 // "column block multiplied".
 constexpr int SK_BAR_EPI = 1, SK_BAR_X = 2, SK_BAR_BUF = 3, SK_BAR_ACC = 12;
@@ -78,13 +79,12 @@ struct SkTmem {
 };
 
 // How column blocks of KG units are dealt to the CTAs.  parts == 0: pieces of `piece` units (one, or a whole column block) evenly and
-// contiguously, the first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.  most: units of
-// the busiest CTA.
+// contiguously, the first units_r CTAs take units_q + 1.  parts > 0: every column block is cut into that many parts, one per CTA.
 struct SkDeal {
-    int units_q, units_r, piece, parts, most, grid;
+    int grid, units_q, units_r, piece, parts;
 };
 
-// The cheapest of the three ways for `ctas` CTAs, `limit` units at most in one of them (even ranges aside).  few: rows rotated inside in one
+// The cheapest of the three ways for `ctas` CTAs, `limit` units at most in one of them (even ranges aside); most: units of the busiest.  few: rows rotated inside in one
 // pass of the decode warps.
 //
 // Every way of dealing the units has a cost, counted in units of the busiest CTA (0.5 us each up to 16 rows).  Partial sums that
@@ -95,7 +95,7 @@ struct SkDeal {
 // at 16.  Where the rule stays with even ranges: 5120 x 5120, one row 11.2, in three parts (14 units for 11) 11.7; 17408 x 5120 24.9,
 // 27.5; 2048 x 25088, whole blocks (32 units for 22) 18.0, 18.8.  In a long range of few rows all hand-overs but the last are hidden:
 // 5120 x 34816, one row 43.3, whole blocks (80 units for 74) 44.1, but 50.0 / 46.8 at 16 rows.
-__host__ __device__ inline SkDeal sk_deal(int NB, int KG, int ctas, int rows, bool few, int limit, bool aligned)
+__host__ __device__ inline SkDeal sk_deal(int NB, int KG, int ctas, int rows, bool few, int limit, bool aligned, int& most)
 {
 #ifdef __CUDA_ARCH__
     using Count = int;                                                      // of slots: far below 2^31
@@ -103,12 +103,13 @@ __host__ __device__ inline SkDeal sk_deal(int NB, int KG, int ctas, int rows, bo
     using Count = long long;
 #endif
     const Count units = (Count)NB * KG;
-    SkDeal t = {0, 0, 1, 0, (int)((units + ctas - 1) / ctas), ctas};
+    SkDeal t = {ctas, 0, 0, 1, 0};
+    most = (int)((units + ctas - 1) / ctas);
     if (aligned) {
         constexpr int EXCHANGE = 5;
-        const int uneven = rows > 8 ? 4 : 2, hidden = rows <= 8 && t.most > 12 ? 3 : 0;
+        const int uneven = rows > 8 ? 4 : 2, hidden = rows <= 8 && most > 12 ? 3 : 0;
         const Count whole = (Count)((NB + ctas - 1) / ctas) * KG;
-        Count best = (Count)t.most + EXCHANGE + uneven;
+        Count best = (Count)most + EXCHANGE + uneven;
         if (whole + hidden < best && whole <= limit && !(few && whole > SK_DECODE_WARPS)) {
             best = whole + hidden;
             t.piece = KG;
@@ -126,15 +127,44 @@ __host__ __device__ inline SkDeal sk_deal(int NB, int KG, int ctas, int rows, bo
     }
     if (t.parts) {
         t.grid = t.parts * NB;
-        t.most = (KG + t.parts - 1) / t.parts;
+        most = (KG + t.parts - 1) / t.parts;
     } else {
         const Count pieces = units / t.piece;
         t.grid = pieces < ctas ? (int)pieces : ctas;
         t.units_q = (int)(pieces / t.grid);
         t.units_r = (int)(pieces % t.grid);
-        t.most = (t.units_q + (t.units_r ? 1 : 0)) * t.piece;
+        most = (t.units_q + (t.units_r ? 1 : 0)) * t.piece;
     }
     return t;
+}
+
+// The units of a CTA (none for those behind a grid smaller than the one that was launched), and the CTAs that share column block nb: what the
+// kernel does with the host's deal, for one that it made itself; warp-uniform to the compiler.
+__device__ __forceinline__ void sk_range(const SkDeal& t, int KG, int cta, int& u0, int& u1)
+{
+    if (t.parts > 0) {
+        const int nb = cta / t.parts, part = cta - nb * t.parts;
+        u0 = nb * KG + part * KG / t.parts;
+        u1 = nb * KG + (part + 1) * KG / t.parts;
+    } else {
+        u0 = (int)gemv_first_unit(cta, t.units_q, t.units_r) * t.piece;
+        u1 = (int)gemv_first_unit(cta + 1, t.units_q, t.units_r) * t.piece;
+    }
+    if (cta >= t.grid) u1 = u0;
+}
+__device__ __forceinline__ void sk_sharers(const SkDeal& t, int KG, int cta, int nb, int& first, int& last)
+{
+    if (t.parts > 0) {
+        first = nb * t.parts;
+        last = first + t.parts - 1;
+    } else if (t.piece > 1) {
+        first = last = cta;
+    } else {
+        first = gemv_cta_of_unit((long long)nb * KG, t.units_q, t.units_r);
+        last = gemv_cta_of_unit((long long)nb * KG + KG - 1, t.units_q, t.units_r);
+    }
+    first = __shfl_sync(0xFFFFFFFFu, first, 0);
+    last = __shfl_sync(0xFFFFFFFFu, last, 0);
 }
 
 // Routed experts of a few slots as one matrix: the column blocks are runs of `blocks`, run v is the expert of slot v -- or, with a map, of the
@@ -146,8 +176,6 @@ struct SkSlots {
     int blocks, shard_blocks;   // column blocks of an expert, of one of its matrices with sign vectors of their own (gate, up)
     int per_row;                // slots that share a row of x (top-k, or 1)
     int known;                  // the ids were there before the kernel ahead began: read ahead of the wait
-    int slots;
-    uint32_t list_off;          // with a map, bytes: the slots that have an expert here, (slot, expert) each
     long long stride;           // 32-bit words between experts
 
     __device__ __forceinline__ int expert(int s) const                      // without a map
@@ -157,7 +185,9 @@ struct SkSlots {
     }
 };
 
-static_assert(SK_DEAL_OFF >= SK_TABLE_OFF + 35 * 4 && SK_DEAL_OFF + sizeof(SkDeal) + sizeof(int2) <= SK_BAR_BYTES, "head of the shared memory");
+static_assert(SK_RANGE_OFF >= SK_TABLE_OFF + 35 * 4 && SK_RANGE_OFF % sizeof(int2) == 0 && SK_DEAL_OFF >= SK_RANGE_OFF + sizeof(int2) &&
+                  SK_DEAL_OFF % sizeof(int) == 0 && SK_DEAL_OFF + sizeof(SkDeal) <= SK_BAR_BYTES,
+              "head of the shared memory");
 
 struct SkinnyLaunch {
     GemvArgs a;
@@ -170,6 +200,8 @@ struct SkinnyLaunch {
     long long xf_shard_stride;  // bytes between shards in xf
     unsigned long long* tl;     // measurement builds only: where this launch stamps its timeline
     uint32_t mul, add;
+    int slots, most;            // slots of s; units of the busiest CTA
+    uint32_t list_off;          // SK_HELD, bytes: the slots that have an expert here, (slot, expert) each
 };
 
 __device__ __forceinline__ bool sk_elect()
@@ -467,9 +499,9 @@ static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint
 // SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.  SK_EACH: every slot as it stands; one whose id is out of range decodes
 // expert 0 and drops the result.  SK_HELD, for ids with a map (a rank's share of the experts, bitrate classes): every CTA makes the same list of
 // the slots that have an expert here, and where that is not all of them their units are dealt anew, so that the others cost nothing: 256
-// experts of 2048 x 512, top-8, K = 3, us per layer in a chain, a rank with 128 / 64 / 32 of them: one token 22.0 / 16.7 / 14.4, two tokens
-// 25.5 / 21.3 / 16.1 (every slot decoded 23.3 / 23.0 / 22.5 and 31.4 / 31.2 / 30.7, blocks of eight rows 29.9 / 23.5 / 19.3 and 32.5 / 29.5 /
-// 24.1); four classes of 64, two tokens 71 (108).  Where every slot has an expert the list costs 0.3 us a layer (20.8, 21.1 with it), which is
+// experts of 2048 x 512, top-8, K = 3, us per layer in a chain, a rank with 128 / 64 / 32 of them: one token 21.8 / 16.7 / 13.6, two tokens
+// 25.4 / 21.2 / 16.0 (every slot decoded 23.3 / 23.0 / 22.5 and 31.4 / 31.2 / 30.7, blocks of eight rows 29.9 / 23.5 / 19.3 and 32.5 / 29.5 /
+// 24.1); four classes of 64, two tokens 70 (108).  Where every slot has an expert the list costs 0.3 us a layer (20.8, 21.1 with it), which is
 // why SK_EACH stays.
 template <int K, int MODE, int FAM, int RP, int X = SK_STREAM, int EPI = 0, int SLOTS = SK_DENSE>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_constant__ SkinnyLaunch p)
@@ -500,50 +532,35 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
 
     const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
     const int cta = blockIdx.x, rows = p.a.rows;
-    const int ups = p.units_per_stage, stages = p.stages;
-    int u0, u1, halves, fills;                                              // units [u0, u1)
-    auto take = [&](const SkDeal& t) {
-        if (t.parts > 0) {
-            const int nb = cta / t.parts, part = cta - nb * t.parts;
-            u0 = nb * p.KG + part * p.KG / t.parts;
-            u1 = nb * p.KG + (part + 1) * p.KG / t.parts;
-        } else {
-            u0 = (int)gemv_first_unit(cta, t.units_q, t.units_r) * t.piece;
-            u1 = (int)gemv_first_unit(cta + 1, t.units_q, t.units_r) * t.piece;
-        }
-        if (SLOTS == SK_HELD && cta >= t.grid) u1 = u0;                                // fewer slots than the grid was launched for
-    };
-    auto count = [&]() {
-        halves = 2 * (u1 - u0);
-        fills = (u1 - u0 + ups - 1) / ups;
-    };
-    // SK_HELD: what the copy warp made of the ids.
+    int u0, u1;                                                             // units [u0, u1)
+    if (p.deal.parts > 0) {
+        const int nb = cta / p.deal.parts, part = cta - nb * p.deal.parts;
+        u0 = nb * p.KG + part * p.KG / p.deal.parts;
+        u1 = nb * p.KG + (part + 1) * p.KG / p.deal.parts;
+    } else {
+        u0 = (int)gemv_first_unit(cta, p.deal.units_q, p.deal.units_r) * p.deal.piece;
+        u1 = (int)gemv_first_unit(cta + 1, p.deal.units_q, p.deal.units_r) * p.deal.piece;
+    }
+    // SK_HELD: the slots that have an expert here, and what the copy warp made of them.
+    [[maybe_unused]] int2* list = reinterpret_cast<int2*>(smem + p.list_off);
     [[maybe_unused]] SkDeal* dealt = reinterpret_cast<SkDeal*>(smem + SK_DEAL_OFF);
-    [[maybe_unused]] int2* range = reinterpret_cast<int2*>(dealt + 1);
-    [[maybe_unused]] int2* list = reinterpret_cast<int2*>(smem + p.s.list_off);
+    [[maybe_unused]] int2* range = reinterpret_cast<int2*>(smem + SK_RANGE_OFF);
     [[maybe_unused]] auto run_of = [&](int v) { return SLOTS == SK_HELD ? list[v] : make_int2(v, p.s.expert(v)); };      // (slot, expert or -1)
-    take(p.deal);
-    count();
-    auto sharers_in = [&](const SkDeal& t, int nb, int& first, int& last) {
-        if (t.parts > 0) {
-            first = nb * t.parts;
-            last = first + t.parts - 1;
-        } else if (t.piece > 1) {
-            first = last = cta;
-        } else {
-            first = gemv_cta_of_unit((long long)nb * p.KG, t.units_q, t.units_r);
-            last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, t.units_q, t.units_r);
-        }
-    };
     auto sharers = [&](int nb, int& first, int& last) {                     // CTAs that share column block nb
         if constexpr (SLOTS == SK_HELD) {
-            sharers_in(*dealt, nb, first, last);
-            first = __shfl_sync(0xFFFFFFFFu, first, 0);
-            last = __shfl_sync(0xFFFFFFFFu, last, 0);
+            sk_sharers(*dealt, p.KG, cta, nb, first, last);
+        } else if (p.deal.parts > 0) {
+            first = nb * p.deal.parts;
+            last = first + p.deal.parts - 1;
+        } else if (p.deal.piece > 1) {
+            first = last = cta;
         } else {
-            sharers_in(p.deal, nb, first, last);
+            first = gemv_cta_of_unit((long long)nb * p.KG, p.deal.units_q, p.deal.units_r);
+            last = gemv_cta_of_unit((long long)nb * p.KG + p.KG - 1, p.deal.units_q, p.deal.units_r);
         }
     };
+    const int ups = p.units_per_stage, stages = p.stages;
+    int halves = 2 * (u1 - u0), fills = (u1 - u0 + ups - 1) / ups;
 
     auto weights = [&](int j, int slot) {                                   // one thread: fill number j, units [u0 + j * ups, ...)
         const int u = u0 + j * ups, n = u1 - u < ups ? u1 - u : ups;
@@ -626,7 +643,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 constexpr int C = decltype(count)::value;
                 int e[C];
 #pragma unroll
-                for (int i = 0; i < C; i++) e[i] = s0 + 32 * i + lane < p.s.slots ? __ldcg(p.s.ids + s0 + 32 * i + lane) : -1;
+                for (int i = 0; i < C; i++) e[i] = s0 + 32 * i + lane < p.slots ? __ldcg(p.s.ids + s0 + 32 * i + lane) : -1;
 #pragma unroll
                 for (int i = 0; i < C; i++) e[i] = e[i] >= 0 && e[i] < p.s.experts ? __ldcg(p.s.map + e[i]) : -1;
 #pragma unroll
@@ -638,17 +655,18 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 }
             };
             if (!p.s.known) ptx::grid_dependency_wait();                    // the ids
-            if (p.s.slots <= 32) {
+            if (p.slots <= 32) {
                 look(0, std::integral_constant<int, 1>{});
             } else {
 #pragma unroll 1
-                for (int s0 = 0; s0 < p.s.slots; s0 += 128) look(s0, std::integral_constant<int, 4>{});
+                for (int s0 = 0; s0 < p.slots; s0 += 128) look(s0, std::integral_constant<int, 4>{});
             }
-            if (held < p.s.slots) {
-                t = {0, 0, 1, 0, 0, 0};
-                if (held > 0) t = sk_deal(held * p.s.blocks, p.KG, (int)gridDim.x, 1, false, p.deal.most, true);
-                take(t);
-                count();
+            if (held < p.slots) {
+                int most;
+                t = {0, 0, 0, 1, 0};
+                if (held > 0) t = sk_deal(held * p.s.blocks, p.KG, (int)gridDim.x, 1, false, p.most, true, most);
+                sk_range(t, p.KG, cta, u0, u1);
+                fills = (u1 - u0 + ups - 1) / ups;
             }
             __syncwarp();
             if (lane == 0) {
@@ -674,7 +692,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         const int2 mine = *range;
         u0 = __shfl_sync(0xFFFFFFFFu, mine.x, 0);
         u1 = __shfl_sync(0xFFFFFFFFu, mine.y, 0);
-        count();
+        halves = 2 * (u1 - u0);
+        fills = (u1 - u0 + ups - 1) / ups;
     }
     if constexpr (SLOTS != SK_DENSE) {
         // The kernel behind may look at the ids as soon as it begins: not before the kernel that wrote them has finished.
