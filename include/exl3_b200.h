@@ -313,7 +313,7 @@ exl3_status exl3_allreduce(void *data, int dtype, size_t n, void *const *peer_re
  * exl3_moe_glu_had_in  replaces moe_glu_had_in (exl3_marlin_moe.cu:237-258): Had128(fp16(silu(g) * u) * suh2[e]);
  *                      gu is [slots, 2*inter] fp16 (gate | up).
  * exl3_moe_combine     replaces moe_combine (exl3_marlin_moe.cu:262-292): y[t] = sum_j w[t,j] * yd[t*top_k+j] in fp32,
- *                      slot order, one rounding; expert ids outside [0, E) are skipped.
+ *                      slot order, rounded to fp16 (a bf16 y: that value converted); expert ids outside [0, E) are skipped.
  * The fragment buffers hold exl3_moe_fragment_bytes(); the GEMV workspace holds exl3_moe_workspace_bytes() and must be
  * zero-filled once. */
 int exl3_moe_block_rows(void);
@@ -370,8 +370,8 @@ exl3_status exl3_moe_tc_experts(const void *x, int x_dtype, int tokens, int top_
                                 int num_experts, const int32_t *expert_map, int num_local, const uint32_t *w13, const uint16_t *suh13,
                                 const uint16_t *svh13, const uint32_t *w2, const uint16_t *suh2, const uint16_t *svh2, int K,
                                 int codebook, uint16_t *yd, void *workspace, size_t workspace_bytes, void *stream);
-/* The same for a layer of one bitrate class, to the end: y[t, :] = sum_j topk_weights[t, j] * (the slot's output), in fp32, in `dtype` (that of
- * x), with the last rotation and the sum in one launch; slots without an expert add nothing.  place: scratch int32 [tokens * top_k]; y
+/* The same for a layer of one bitrate class, to the end: y[t, :] = sum_j topk_weights[t, j] * (the slot's output), in fp32, rounded as by
+ * exl3_moe_combine to `dtype` (that of x), with the last rotation and the sum in one launch; slots without an expert add nothing.  place: scratch int32 [tokens * top_k]; y
  * 16-byte aligned.  2048 tokens, 256 experts of 2048 x 512, top-8: 386 -> 374 us. */
 exl3_status exl3_moe_tc_layer(const void *x, int dtype, int tokens, int top_k, int hidden, int inter, const int32_t *topk_ids,
                               const float *topk_weights, int num_experts, const int32_t *expert_map, int num_local, const uint32_t *w13,

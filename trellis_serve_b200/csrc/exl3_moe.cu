@@ -453,7 +453,8 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
     }
 }
 
-// y[t, :] = sum_j w[t, j] * fp16( Had128(yd_rot[place of slot t * top_k + j]) * svh2[its expert] ), in fp32, one rounding: moe_out_kernel and
+// y[t, :] = sum_j w[t, j] * fp16( Had128(yd_rot[place of slot t * top_k + j]) * svh2[its expert] ), in fp32, rounded to fp16 (and, for a bf16 y, from there: values
+// beyond 65504 are infinite in it as well, as with explicit casts around an fp16 layer): moe_out_kernel and
 // moe_combine_kernel in one, without the slots' rows in memory between.  A warp takes 8 / G tokens, G rows each (top_k rounded up to a power
 // of two, at most eight; more come in rounds), four lanes per row; the rows of a token are added by exchanging halves, so that every lane ends
 // with 32 / G of the 128 columns, its own.  Traffic bounds it (2048 tokens, top-8, 2048 columns: 67 MB, 10.4 us).
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* _
     }
 }
 
-// y[t, :] = sum_j w[t, j] * yd[t*top_k + j, :] in fp32, slot order, one rounding; ids outside [0, E) are skipped.  V columns per
+// y[t, :] = sum_j w[t, j] * yd[t*top_k + j, :] in fp32, slot order, rounded to fp16 and, for a bf16 y, from there; ids outside [0, E) are skipped.  V columns per
 // thread; the rows of up to eight slots are requested together (16384 slots of 2048 columns: 40 us with two columns per thread
 // and one slot at a time).
 template <int V>

@@ -392,9 +392,10 @@ def run_layer(x, topk_weights, topk_ids, pack: MixedPack, out: torch.Tensor, wor
               expert_maps: list[torch.Tensor] | None = None) -> torch.Tensor:
     """One MoE layer (alignment included) that allocates nothing: `workspace` is a zero-filled uint8 tensor of at least
     `layer_workspace_bytes(...)`; `expert_maps` replaces the pack's per-class maps (expert parallelism with an engine's
-    global -> local map composed in).  Same kernels and the same bits as `forward_mixed` for decode-sized batches; a class
-    whose experts see `TC_ROWS_PER_EXPERT` rows or more on average goes through the grouped tensor-core GEMM, and the few slots of
-    one decoded token or two through two launches of the dense decode kernel (`exl3_moe_slots_experts`)."""
+    global -> local map composed in).  Decode-sized batches take the kernels of `forward_mixed` and give the same bits.  The few slots
+    of one decoded token or two go through two launches of the dense decode kernel (`exl3_moe_slots_experts`), whose fp32 sums are
+    added in another order, one that depends on how many slots have an expert here; a class whose experts see
+    `TC_ROWS_PER_EXPERT` rows or more on average goes through the grouped tensor-core GEMM, on weights rounded to fp16."""
     _require_cuda(x, "x")
     lib = _lib.load()
     tokens, hidden = x.shape
