@@ -702,18 +702,18 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     const DeviceInfo* d = current_device_info();
     if (!d) return EXL3_ERR_NOT_INITIALISED;
     const int grid = d->sm_count < MOE_MAX_GRID ? d->sm_count : MOE_MAX_GRID;
-    // Stages of about 24 KB of weights (a bulk copy costs a few hundred nanoseconds whatever its size), two units or more per stage (see
-    // SkWalk).  Single blocks of eight rows: their activations ride with the weights, as many stages as fit; four units per stage where
+    // Stages of about 24 KB of weights (a bulk copy costs a few hundred nanoseconds whatever its size), a unit or more per group of decode
+    // warps (see SkWalk).  Single blocks of eight rows: their activations ride with the weights, as many stages as fit; four units per stage where
     // three such stages fit, as the decode groups change stages less often (64 tokens, 256 experts: K = 4 172 -> 169 us, K = 5 191 -> 187).
     // Long items: three stages of weights, the rest for activations (three units of 128 rows and more; larger stages take from those).
     const uint32_t unit = 2048u * (uint32_t)K, row = mode == GEMV_SPLIT ? 512u : 256u, tail = MOE_BLOCK_ROWS * 128 * 4, all = (uint32_t)d->max_smem_optin;
     uint32_t ups = (24u * 1024u + unit - 1) / unit;
-    if (ups < 2) ups = 2;
+    if (ups < SK_GROUPS) ups = SK_GROUPS;
     uint32_t stages = 3;
     if (!l.items) {
         const uint32_t with_rows = unit + MOE_BLOCK_ROWS * row;
         if (ups < 4) ups = 4;
-        while (ups > 2 && 3 * ups * with_rows > all - MOE_BAR_BYTES - tail) ups--;
+        while (ups > SK_GROUPS && 3 * ups * with_rows > all - MOE_BAR_BYTES - tail) ups--;
         stages = (all - MOE_BAR_BYTES - tail) / (ups * with_rows);
         if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
         l.x_bytes = stages * ups * MOE_BLOCK_ROWS * row;

@@ -19,7 +19,11 @@
 //     (measured: 2.2 us per 32 rows, 512 x 2048 of 256 experts 192 us): they leave in the rotated basis, as fp16, and the kernels
 //     behind rotate them.
 //
-// Bound by the issue of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.
+// Bound by the issue of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.  Groups take whole units
+// (three half units apart before): 256 experts of 2048 x 512, top-8, K = 3, 64 tokens 178.5 -> 175.2 us, 2048 tokens 366 -> 359.  Long items: 16.9 clk
+// per tile for gate|up, most of it on the scheduler that the MMA warp is on (62 instructions per tile there, 55 on the others): the loop that
+// issues them frees a buffer after its own half's MMAs (not both after the unit's: 355 -> 350 us), knows its loop bounds as uniform (349), and
+// is one piece of code for all groups (347).
 #pragma once
 #include "exl3_skinny_kernel.cuh"
 
@@ -143,7 +147,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         if (lane == 0) {
             for (int s = 0; s < SK_MAX_STAGES; s++) {
                 ptx::mbar_init(&w_full[s], 1);
-                ptx::mbar_init(&stage_empty[s], LIST ? 1 : 2 * ups);
+                ptx::mbar_init(&stage_empty[s], LIST ? 1 : ups);
             }
             for (int s = 0; s < MOE_X_SLOTS; s++) {
                 ptx::mbar_init(&x_full[s], 1);
@@ -169,6 +173,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     ptx::grid_dependency_wait();                                            // the item list comes from kernels ahead in the stream
 
     const int UB = p.NB * p.KG;                                             // units per item
+    auto uniform = [](int v) { return (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)v); };     // v >= 0, the same in every lane
     // Values read from memory go through a reduction where MMA operands depend on them: its result is a uniform register.
     const int n_items = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)(LIST ? p.counts[1] : p.counts[0] / MOE_BLOCK_ROWS));
     // What is split over the CTAs: units, or whole column blocks -- with LIST always: a row's sums are then the same whatever item the
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         units_r = (int)(total % gridDim.x);
     }
     const long long u0 = gemv_first_unit(cta, units_q, units_r) * grain;
-    const int units = (units_q + (cta < units_r ? 1 : 0)) * grain, fills = (units + ups - 1) / ups;
+    const int units = uniform((units_q + (cta < units_r ? 1 : 0)) * grain), fills = uniform((units + ups - 1) / ups);
     // LIST, activation ring: a slot holds the activations of a run of up to x_units row blocks of a column block, consecutive in memory
     // (a bulk copy costs a few hundred nanoseconds whatever its size).
     const uint32_t x_unit = LIST ? __reduce_max_sync(0xFFFFFFFFu, (unsigned)p.counts[2]) * F_ROW : 0u;
@@ -200,9 +205,11 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         x_slots = (int)(p.x_bytes / (x_unit * x_units));
         if (x_slots > MOE_X_SLOTS) x_slots = MOE_X_SLOTS;
     }
+    x_units = uniform(x_units);
+    x_slots = uniform(x_slots);
     [[maybe_unused]] const uint32_t slot_bytes = x_unit * x_units;
-    int item = units <= 0 ? 0 : (long long)n_items * UB < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB);
-    int in_item = units > 0 ? (int)(u0 - (long long)item * UB) : 0;
+    int item = uniform(units <= 0 ? 0 : (long long)n_items * UB < (1ll << 31) ? (int)((unsigned)u0 / (unsigned)UB) : (int)(u0 / UB));
+    int in_item = uniform(units > 0 ? (int)(u0 - (long long)item * UB) : 0);
     auto item_of = [&](int i) {                                             // expert, first row, rows
         if constexpr (LIST) {
             const int4 t = p.items[i];
@@ -212,31 +219,26 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
     };
 
     if (warp >= SK_DECODE_WARP) {
-        // ------------------------------------------------------------------ decode: as in the dense kernel
+        // ------------------------------------------------------------------ decode: as in the dense kernel, whole units
         const int dw = warp - SK_DECODE_WARP, group = dw >> 3, nt = 2 * (dw & 3) + ((dw >> 2) & 1);
         const uint32_t table = ptx::smem_addr(smem + MOE_TABLE_OFF);
         const CodebookConst cbc = {ptx::lds32(table + 128), ptx::lds32(table + 132), ptx::lds32(table + 136)};
         const int source = __shfl_sync(0xFFFFFFFFu, lane, (lane + 31) & 31);
         const SkPow2<K, FAM> pw(table);
         const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
-        const int halves = 2 * units;
-        if (halves > 0) {
+        if (units > 0) {
             auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
             SkWalk at(group, ups, fills, enter);
-            uint32_t wa = ptx::smem_addr(wring) + (uint32_t)(nt * 2) * HALF_BYTES + lane * 4u + (group >> 1) * W_BYTES + (group & 1) * HALF_BYTES;
+            uint32_t wa = ptx::smem_addr(wring) + (uint32_t)(nt * 2) * HALF_BYTES + lane * 4u + group * W_BYTES;
             const uint32_t t_base = ((uint32_t)(nt * 16) << 16) + A_OFF + (uint32_t)(group * 2) * A_COLS;
             const uint32_t empty0 = ptx::smem_addr(&buf_empty[group * 2]);
             const int bar0 = SK_BAR_BUF + group * 2;
             uint32_t parity = 1;
-            int h = group;
-            const uint32_t move0 = group & 1 ? 2 * W_BYTES - HALF_BYTES : W_BYTES + HALF_BYTES, move1 = 3 * W_BYTES - move0;
-            const int adv0 = 1 + (group & 1);
-            auto step = [&](auto which) {
+            auto half = [&](auto which) {
                 constexpr int S = decltype(which)::value;
-                if (at.left <= 0 && at.settle(ups, stages, enter)) wa -= ring;
                 uint32_t L[K];
 #pragma unroll
-                for (int i = 0; i < K; i++) L[i] = ptx::lds32(wa + i * 128u);
+                for (int i = 0; i < K; i++) L[i] = ptx::lds32(wa + S * HALF_BYTES + i * 128u);
                 constexpr int TCOLS = MODE == GEMV_SPLIT ? 16 : 8;
                 const uint32_t ta = t_base + S * A_COLS;
                 auto tile = [&](auto tconst) {
@@ -259,14 +261,14 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 sk_fence_before();
                 sk_bar_arrive(bar0 + S, (8 + 1) * 32);
-                wa += S == 0 ? move0 : move1;
-                at.left -= S == 0 ? adv0 : 3 - adv0;
-                h += SK_GROUPS;
             };
 #pragma unroll 1
-            while (h < halves) {
-                step(std::integral_constant<int, 0>{});
-                if (h < halves) step(std::integral_constant<int, 1>{});
+            for (int u = group; u < units; u += SK_GROUPS) {
+                if (at.left <= 0 && at.settle(ups, stages, enter)) wa -= ring;
+                half(std::integral_constant<int, 0>{});
+                half(std::integral_constant<int, 1>{});
+                wa += SK_GROUPS * W_BYTES;
+                at.left -= SK_GROUPS;
                 parity ^= 1;
             }
         }
@@ -280,52 +282,40 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             const uint32_t w_bar = ptx::smem_addr(w_full), s_bar = ptx::smem_addr(stage_empty), ring = (uint32_t)(stages * ups) * F_BYTES;
             auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
             SkWalk at(group, ups, fills, enter);
-            uint32_t xa = ptx::smem_addr(xs) + (group >> 1) * F_BYTES + (group & 1) * (F_BYTES / 2);
+            uint32_t xa = ptx::smem_addr(xs) + group * F_BYTES;
             const uint32_t empty0 = ptx::smem_addr(&buf_empty[group * 2]), done_bar = ptx::smem_addr(&acc_done[group]);
-            uint32_t d = 0, acc_parity = 1, done_parity = 0, acc = 0, accumulate = 0;
-            int h = group, done = 0, kg = in_item % p.KG;
-            auto step = [&](auto which) {
-                constexpr int S = decltype(which)::value;
-                constexpr uint32_t half = S == 0 ? group & 1 : 1 - (group & 1);
-                if (at.left <= 0 && at.settle(ups, stages, enter)) xa -= ring;
-                const uint64_t b = ((uint64_t)b_hi << 32) | (chunk << 16) | (xa >> 4);
-                ptx::named_bar_sync(SK_BAR_BUF + group * 2 + S, (8 + 1) * 32);
-                sk_fence_after();
-                if (sk_elect()) {
-#pragma unroll
-                    for (int m = 0; m < MMAS; m++) sk_mma(acc, a_base + S * A_COLS + m * 8, b + m * 2u * chunk, IDESC, m > 0 ? 1u : accumulate);
-                    sk_commit_addr(empty0 + S * 8u);
-                    sk_commit_addr(s_bar + at.slot8);
-                }
-                __syncwarp();
-                accumulate = 1;
-                xa += half ? 2 * F_BYTES - F_BYTES / 2 : F_BYTES + F_BYTES / 2;
-                at.left -= 1 + half;
-                h += SK_GROUPS;
-            };
-            bool second = false;                                            // which of the two steps comes next
+            uint32_t d = 0, acc_parity = 1, done_parity = 0;
+            int u = group, done = 0, kg = uniform(in_item % p.KG);
 #pragma unroll 1
             while (done < units) {                                          // column blocks of the CTA
                 done += p.KG - kg < units - done ? p.KG - kg : units - done;
                 kg = 0;
-                const int he = 2 * done;
                 sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
                 sk_fence_after();
-                acc = (d * SK_GROUPS + group) * NMAX;
-                accumulate = 0;
+                const uint32_t acc = (d * SK_GROUPS + group) * NMAX;
+                uint32_t accumulate = 0;
 #pragma unroll 1
-                while (h < he) {
-                    if (!second) {
-                        step(std::integral_constant<int, 0>{});
-                        if (h >= he) {
-                            second = true;
-                            break;
+                for (; u < done; u += SK_GROUPS) {
+                    if (at.left <= 0 && at.settle(ups, stages, enter)) xa -= ring;
+                    const uint64_t b = ((uint64_t)b_hi << 32) | (chunk << 16) | (xa >> 4);
+#pragma unroll
+                    for (int S = 0; S < 2; S++) {
+                        ptx::named_bar_sync(SK_BAR_BUF + group * 2 + S, (8 + 1) * 32);
+                        sk_fence_after();
+                        if (sk_elect()) {
+#pragma unroll
+                            for (int m = 0; m < MMAS; m++)
+                                sk_mma(acc, a_base + S * A_COLS + m * 8, b + (S * MMAS + m) * 2u * chunk, IDESC, m > 0 ? 1u : accumulate);
+                            sk_commit_addr(empty0 + S * 8u);
+                            if (S == 1) sk_commit_addr(s_bar + at.slot8);
                         }
+                        __syncwarp();
+                        accumulate = 1;
                     }
-                    step(std::integral_constant<int, 1>{});
-                    second = false;
+                    xa += SK_GROUPS * F_BYTES;
+                    at.left -= SK_GROUPS;
                 }
-                if (accumulate) {                                           // else the group had no half unit of this block
+                if (accumulate) {                                           // else the group had no unit of this block
                     if (sk_elect()) sk_commit_addr(done_bar);
                     __syncwarp();
                     sk_wait(done_bar, done_parity, failed);
@@ -347,64 +337,55 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         // ------------------------------------------------------------------ MMA issue, all groups in unit order
         const uint32_t s_bar = ptx::smem_addr(stage_empty), xe_bar = ptx::smem_addr(x_empty), xf_bar = ptx::smem_addr(x_full);
         const uint32_t empty0 = ptx::smem_addr(buf_empty), done0 = ptx::smem_addr(acc_done), xs_addr = ptx::smem_addr(xs);
-        uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, accumulate = 0, acc = 0, idesc = 0, pitch = MOE_BLOCK_ROWS, b_lo = 0;
-        int left = ups, third = 0;
-        // A unit whose number is `C` modulo three: groups and buffers of its two halves are constants of the code.  A unit at a time, with as
-        // few instructions as possible: this warp gets an eighth of its scheduler's issue slots.
-        auto unit = [&](auto cconst, bool run_end, bool stage_end) {
-            constexpr int C = decltype(cconst)::value, G0 = (2 * C) % 3, B0 = (2 * C) / 3, G1 = (2 * C + 1) % 3, B1 = (2 * C + 1) / 3;
-            ptx::named_bar_sync(SK_BAR_BUF + G0 * 2 + B0, (8 + 1) * 32);
-            ptx::named_bar_sync(SK_BAR_BUF + G1 * 2 + B1, (8 + 1) * 32);
-            sk_fence_after();
-            const uint64_t b = ((uint64_t)((128u >> 4) | (1u << 14)) << 32) | b_lo;
-            if (sk_elect()) {
-#pragma unroll
-                for (int m = 0; m < 2 * MMAS; m++)
-                    sk_mma(acc, A_OFF + (m < MMAS ? (G0 * 2 + B0) * A_COLS + m * 8 : (G1 * 2 + B1) * A_COLS + (m - MMAS) * 8), b + m * 2u * pitch, idesc,
-                           m > 0 ? 1u : accumulate);
-                sk_commit_addr(empty0 + (G0 * 2 + B0) * 8u);
-                sk_commit_addr(empty0 + (G1 * 2 + B1) * 8u);
-                if (run_end) sk_commit_addr(xe_bar + x_slot * 8u);
-                if (stage_end) sk_commit_addr(s_bar + stage8);
-            }
-            __syncwarp();
-            accumulate = 1;
-        };
+        uint32_t stage8 = 0, x_slot = 0, x_parity = 0, d = 0, acc_parity = 1, g = 0;
+        int left = ups;
+        // A unit at a time with as few instructions as possible: this warp shares its scheduler with six decode warps, whose groups wait for the
+        // slowest of their members.  A half's MMAs free its buffer while the group decodes the other one.
         int done = 0;
 #pragma unroll 1
         while (done < units) {                                              // column blocks of the CTA
-            const int kg = in_item % p.KG, count = p.KG - kg < units - done ? p.KG - kg : units - done;
-            if constexpr (LIST) pitch = __reduce_max_sync(0xFFFFFFFFu, (unsigned)item_of(item).z);
-            const uint32_t cols = (pitch + 15u) & ~15u;
-            idesc = (1u << 4) | ((cols >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> fp32, M = 128, N = cols
+            const int kg = uniform(in_item % p.KG), count = p.KG - kg < units - done ? p.KG - kg : units - done;
+            const uint32_t pitch = __reduce_max_sync(0xFFFFFFFFu, (unsigned)item_of(item).z), chunk2 = 2u * pitch, cols = (pitch + 15u) & ~15u;
+            const uint32_t idesc = (1u << 4) | ((cols >> 3) << 17) | ((128u >> 4) << 24);  // fp16 x fp16 -> fp32, M = 128, N = cols
             sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
             sk_fence_after();
-            acc = d * NMAX;
-            accumulate = 0;
+            const uint32_t acc = d * NMAX;
+            uint32_t accumulate = 0;
 #pragma unroll 1
-            for (int u = 0, r = 0; u < count; u++) {
-                if (r == 0) {
-                    sk_wait(xf_bar + x_slot * 8u, x_parity, failed);
-                    b_lo = (pitch << 16) | ((xs_addr + x_slot * slot_bytes) >> 4);
-                }
-                left--;
-                const bool stage_end = left == 0, run_end = r + 1 == x_units || u + 1 == count;
-                if (third == 0) unit(std::integral_constant<int, 0>{}, run_end, stage_end);
-                else if (third == 1) unit(std::integral_constant<int, 1>{}, run_end, stage_end);
-                else unit(std::integral_constant<int, 2>{}, run_end, stage_end);
-                third = third == 2 ? 0 : third + 1;
-                if (stage_end) {
-                    left = ups;
-                    stage8 = stage8 + 8 == (uint32_t)stages * 8u ? 0 : stage8 + 8;
-                }
-                b_lo += pitch * (F_ROW / 16);
-                r++;
-                if (run_end) {
-                    r = 0;
-                    if (++x_slot == (uint32_t)x_slots) {
-                        x_slot = 0;
-                        x_parity ^= 1;
+            for (int todo = count; todo > 0;) {                             // runs of the activation ring
+                const int run = todo < x_units ? todo : x_units;
+                todo -= run;
+                sk_wait(xf_bar + x_slot * 8u, x_parity, failed);
+                uint32_t lo = (pitch << 16) | ((xs_addr + x_slot * slot_bytes) >> 4);
+#pragma unroll 1
+                for (int r = run; r > 0; r--) {
+                    left--;
+                    const uint32_t a = A_OFF + g * (2 * A_COLS), empty = empty0 + g * 16u;
+#pragma unroll
+                    for (int S = 0; S < 2; S++) {
+                        ptx::named_bar_sync(SK_BAR_BUF + g * 2 + S, (8 + 1) * 32);
+                        sk_fence_after();
+                        if (sk_elect()) {
+#pragma unroll
+                            for (int m = 0; m < MMAS; m++)
+                                sk_mma_at(acc, a + S * A_COLS + m * 8, lo + m * chunk2, (128u >> 4) | (1u << 14), idesc, S + m > 0 ? 1u : accumulate);
+                            sk_commit_addr(empty + S * 8u);
+                            if (S == 1 && r == 1) sk_commit_addr(xe_bar + x_slot * 8u);
+                            if (S == 1 && left == 0) sk_commit_addr(s_bar + stage8);
+                        }
+                        __syncwarp();
+                        lo += MMAS * chunk2;
                     }
+                    accumulate = 1;
+                    g = g == SK_GROUPS - 1 ? 0 : g + 1;
+                    if (left == 0) {
+                        left = ups;
+                        stage8 = stage8 + 8 == (uint32_t)stages * 8u ? 0 : stage8 + 8;
+                    }
+                }
+                if (++x_slot == (uint32_t)x_slots) {
+                    x_slot = 0;
+                    x_parity ^= 1;
                 }
             }
             if (sk_elect()) sk_commit_addr(done0 + d * 8u);
@@ -424,7 +405,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
         int done = 0, kg = units > 0 ? in_item % p.KG : 0;
 #pragma unroll 1
         while (done < units) {
-            if (!failed && !ptx::mbar_wait_relaxed(&acc_done[d], parity, 60)) failed = 1;
+            if (!failed && !ptx::mbar_wait_relaxed(&acc_done[d], parity, done + p.KG < units ? 400 : 60)) failed = 1;
             sk_fence_after();
             sk_fence_before();
             sk_bar_arrive(SK_BAR_ACC + (int)d, (1 + 4) * 32);
@@ -445,7 +426,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 if (n > x_units) n = x_units;
                 const uint32_t unit = (uint32_t)it.z * F_ROW, bytes = (uint32_t)n * unit;
                 const unsigned char* src = p.xf + (nb >= p.shard_end_block ? p.xf_shard_stride : 0) + ((long long)it.y * p.KG * F_ROW + (long long)kg * unit);
-                if (!failed && !ptx::mbar_wait_relaxed(&x_empty[slot], phase, 50)) failed = 1;
+                if (!failed && !ptx::mbar_wait_relaxed(&x_empty[slot], phase, 200)) failed = 1;
                 ptx::mbar_arrive_expect_tx(&x_full[slot], bytes);
                 ptx::bulk_g2s(xs + (size_t)slot * slot_bytes, src, bytes, &x_full[slot]);
                 if (++slot == x_slots) {
@@ -477,7 +458,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
             int e = item_of(item).x;
             [[maybe_unused]] int x_item = item, x_nb = in_item / p.KG, x_kg = in_item - x_nb * p.KG;
             for (int j = 0; j < fills; j++) {
-                if (!failed && !ptx::mbar_wait_relaxed(&stage_empty[slot], phase, 100)) failed = 1;
+                if (!failed && !ptx::mbar_wait_relaxed(&stage_empty[slot], phase, 400)) failed = 1;
                 int n = todo < ups ? todo : ups;
                 todo -= n;
                 unsigned char* dst = wring + (size_t)(slot * ups) * W_BYTES;
@@ -557,7 +538,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 for (int e = 0; e < 8; e++) dst[r0 * 128 + e * 128] = __float2half_rn(v[e]);
             };
             // Tensor memory -> shared memory or the CTA's slab: lane = output column.
-            const int hb = 2 * done, he = 2 * (done + count);
+            const int hb = done, he = done + count;
             auto load_rows = [&](int c, float (&v)[8]) {
                 uint32_t r[ACCS][8];
 #pragma unroll
@@ -572,7 +553,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 if constexpr (!LIST) {
 #pragma unroll
                     for (int g = 0; g < ACCS; g++)
-                        if (hb + (g + 3 - hb % 3) % 3 < he)                 // else the group had no half unit of this block
+                        if (hb + (g + 3 - hb % 3) % 3 < he)                 // else the group had no unit of this block
 #pragma unroll
                             for (int e = 0; e < 8; e++) v[e] += __uint_as_float(r[g][e]);
                 }

@@ -63,7 +63,6 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.a = a;
     l.KG = a.k / 128;
     l.NB = a.n_total / 128;
-    const long long units = (long long)l.KG * l.NB;
     const int ctas = d->sm_count < GEMV_MAX_GRID ? d->sm_count : GEMV_MAX_GRID;
     l.deal = sk_deal(l.NB, l.KG, ctas, a.rows, x == SK_ROTATE && a.rows > SK_FUSED_ROWS, INT_MAX, aligned, l.most);
     const size_t most = (size_t)l.most;
@@ -81,7 +80,10 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     size_t ups = (24 * 1024 + w - 1) / w;
     if (x != SK_STREAM && ups < 6) ups = 6;
     if (ups > most) ups = most;
-    while (ups > 2 && budget / (ups * unit) < 3) ups--;      // a ring needs stages of two units or more (see SkWalk)
+    const size_t least = a.rows <= SK_FUSED_ROWS || (a.rows > SK_ROTATE_ROWS && a.rows <= 16) ? SK_GROUPS : 2;      // see SkWalk
+    if (ups < least) ups = least;
+    if (ups > most) ups = most;
+    while (ups > least && budget / (ups * unit) < 3) ups--;
     size_t stages = budget / (ups * unit);
     if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
     const size_t fills = (most + ups - 1) / ups;

@@ -11,9 +11,10 @@
 //     operand (N = rows) in shared memory.  The lane that decodes a 16x16 tile holds exactly its share of a tcgen05.st 16x256b
 //     fragment: one store of eight registers per tile, no repacking.  Split mode keeps the two fp16 summands of a weight as two k
 //     slots (the accumulator adds them), so every activation stands twice in a row of B; paired mode (MUL1) stores fp16 pairs;
-//   * 24 decode warps in three groups of eight (one column tile each); a group decodes one half unit (64 k x 128 columns) at a time
-//     into one of its tensor-memory buffers; one MMA warp per group issues the MMAs of a half unit into accumulators of its own
-//     (fixed order of additions; the epilogue adds the groups' accumulators in group order).  MMAs are issued by an elected lane of
+//   * 24 decode warps in three groups of eight (one column tile each) that take whole units in turn (WHOLE; half units from three rows to
+//     eight and above 16); a group decodes one half unit (64 k x 128 columns) at a time into one of its tensor-memory buffers; one MMA
+//     warp per group issues the MMAs of a half unit into accumulators of its own (fixed order of additions; the epilogue adds the
+//     groups' accumulators in group order).  MMAs are issued by an elected lane of
 //     a CONVERGED warp with warp-uniform operands: 16 clk per MMA (N <= 32) against 47 from one thread of a diverged warp;
 //   * warps that wait long wait on named barriers, which cost no issue slots: polls of mbarriers by the waiting warps were 12 of
 //     67 executed instructions per tile;
@@ -226,6 +227,15 @@ __device__ __forceinline__ void sk_mma(uint32_t d, uint32_t a, uint64_t b, uint3
         "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with B's descriptor as two words.
+__device__ __forceinline__ void sk_mma_at(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}\n" ::"r"(d),
+        "r"(a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // Rows of the operand = the tile's columns (lane / 4 and + 8), 32-bit columns = k (split) or pairs of k (paired).
 __device__ __forceinline__ void sk_store_tile_split(uint32_t taddr, const uint32_t (&w)[8])
 {
@@ -288,18 +298,18 @@ struct SkPow2 {
     }
 };
 
-// A group's walk over its half units h = group, group + 3, ... through the stage ring.  `left`: units left in the current stage, the
-// current one included.  settle() follows it into the stage of its unit and calls enter(barrier offset, parity) for the fill.  A ring
-// that is used more than once has stages of two units or more (four halves), so every group has a half in every fill: none can be
-// passed over, and none can be refilled before each group has seen it -- waits by parity need both.
+// A group's walk over its units or half units group, group + 3, ... through the stage ring, from unit `first` on.  `left`: units left in the
+// current stage, the current one included.  settle() follows it into the stage of its unit and calls enter(barrier offset, parity) for the fill.
+// A ring that is used more than once has stages of three units or more (two where groups take half units), so every group has a part of
+// every fill: none can be passed over, and none can be refilled before each group has seen it -- waits by parity need both.
 struct SkWalk {
     int left, fills;            // units left in the stage; fills still to come
     uint32_t slot8, parity;
     template <typename F>
-    __device__ __forceinline__ SkWalk(int group, int ups, int fills_, F enter) : left(ups), fills(fills_ - 1), slot8(0), parity(0)
+    __device__ __forceinline__ SkWalk(int first, int ups, int fills_, F enter) : left(ups), fills(fills_ - 1), slot8(0), parity(0)
     {
         enter(0u, 0u);
-        left -= group >> 1;
+        left -= first;
     }
     // True when the walk has wrapped around to the first slot.
     template <typename F>
@@ -496,6 +506,13 @@ static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint
 }
 
 // RP: operand pitch, the rows rounded up (operand_pitch).
+// WHOLE: a group takes whole units, not every third half unit: one walk through the stages, one loop test and addresses that are constants for eight
+// tiles instead of four (49.7 -> 46.7 instructions per tile at K = 3, the loop 14.9 -> 13.8 clk).  Chained launches over distinct weights, K = 3, one
+// row, us: 5120 x 34816 42.7 -> 41.7, 17408 x 5120 24.7 -> 24.2, 2048 x 25088 17.3 -> 17.0, 4096 x 4096 8.8 -> 8.6; K = 4, 5, 8 17408 x 5120 23.4 ->
+// 22.6, 25.8 -> 24.9, 25.2 -> 24.7; 16 rows 30.6 -> 30.1.  What it costs: at the end of a column block a group may be a unit behind the others
+// instead of half of one, which shows where a CTA has few units in two blocks (5120 x 7168, 15 units: one row 13.65 -> 13.75, but five rows 17.7 ->
+// 18.4, as its sums of the first block then hold up the second: hence not for three to eight rows).  Above 16 rows a stage of three units takes too
+// much shared memory.
 // SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.  SK_EACH: every slot as it stands; one whose id is out of range decodes
 // expert 0 and drops the result.  SK_HELD, for ids with a map (a rank's share of the experts, bitrate classes): every CTA makes the same list of
 // the slots that have an expert here, and where that is not all of them their units are dealt anew, so that the others cost nothing: 256
@@ -510,7 +527,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
     static_assert(SLOTS == SK_DENSE || (X == SK_ROTATE && RP == SK_FUSED_ROWS && EPI == 0), "slots come one row each");
     static_assert(X != SK_ROTATE || RP <= SK_ROTATE_ROWS, "the kernel rotates up to eight rows");
     constexpr int RB = RP <= 8 ? 1 : RP <= 16 ? 2 : 4;                      // rows that a warp finishes together
-    constexpr bool ALL_FINISH = RP >= 16;
+    constexpr bool ALL_FINISH = RP >= 16, WHOLE = RP != SK_ROTATE_ROWS && RP <= 16;
     constexpr int N = RP < 16 ? 16 : RP;                                    // MMA columns; those behind the real rows are never looked at
     using TM = SkTmem<MODE, N>;
     constexpr uint32_t W_BYTES = 2048u * K, HALF_BYTES = K * 128u;
@@ -560,7 +577,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         }
     };
     const int ups = p.units_per_stage, stages = p.stages;
-    int halves = 2 * (u1 - u0), fills = (u1 - u0 + ups - 1) / ups;
+    int units = u1 - u0, halves = 2 * units, fills = (u1 - u0 + ups - 1) / ups;
 
     auto weights = [&](int j, int slot) {                                   // one thread: fill number j, units [u0 + j * ups, ...)
         const int u = u0 + j * ups, n = u1 - u < ups ? u1 - u : ups;
@@ -625,7 +642,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             for (int s = 0; s < SK_MAX_STAGES; s++) {
                 ptx::mbar_init(&w_full[s], 1);
                 ptx::mbar_init(&x_full[s], 1);
-                ptx::mbar_init(&stage_empty[s], 2 * ups);
+                ptx::mbar_init(&stage_empty[s], WHOLE ? ups : 2 * ups);
             }
             for (int b = 0; b < TM::A_BUFS * SK_GROUPS; b++) ptx::mbar_init(&buf_empty[b], 1);
             for (int g = 0; g < SK_GROUPS; g++) ptx::mbar_init(&acc_done[g], 1);
@@ -692,7 +709,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         const int2 mine = *range;
         u0 = __shfl_sync(0xFFFFFFFFu, mine.x, 0);
         u1 = __shfl_sync(0xFFFFFFFFu, mine.y, 0);
-        halves = 2 * (u1 - u0);
+        units = u1 - u0;
+        halves = 2 * units;
         fills = (u1 - u0 + ups - 1) / ups;
     }
     if constexpr (SLOTS != SK_DENSE) {
@@ -712,8 +730,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         const SkPow2<K, FAM> pw(table);
         const uint32_t w_bar = ptx::smem_addr(w_full), ring = (uint32_t)(stages * ups) * W_BYTES;
         auto enter = [&](uint32_t slot8, uint32_t parity) { sk_wait(w_bar + slot8, parity, failed); };
-        SkWalk at(group, ups, fills, enter);
-        uint32_t wa = ptx::smem_addr(wring) + (uint32_t)(nt * 2) * HALF_BYTES + lane * 4u + (group >> 1) * W_BYTES + (group & 1) * HALF_BYTES;
+        SkWalk at(WHOLE ? group : group >> 1, ups, fills, enter);
+        uint32_t wa = ptx::smem_addr(wring) + (uint32_t)(nt * 2) * HALF_BYTES + lane * 4u +
+                      (WHOLE ? group * W_BYTES : (group >> 1) * W_BYTES + (group & 1) * HALF_BYTES);
         const uint32_t t_base = ((uint32_t)(nt * 16) << 16) + TM::A_OFF + (uint32_t)(group * TM::A_BUFS) * TM::A_COLS;
         const uint32_t empty0 = ptx::smem_addr(&buf_empty[group * TM::A_BUFS]);
         const int bar0 = SK_BAR_BUF + group * TM::A_BUFS;
@@ -724,12 +743,12 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         const int adv0 = 1 + (group & 1);
         auto step = [&](auto which) {
             constexpr int S = decltype(which)::value;
-            // A stage is waited for when its first half unit is wanted, not before: stages behind the first lap come only once halves
-            // have been multiplied, and with the rotation inside that takes every decode warp.
-            if (at.left <= 0 && at.settle(ups, stages, enter)) wa -= ring;
+            // A stage is waited for when its first unit is wanted, not before: stages behind the first lap come only once units have been
+            // multiplied, and with the rotation inside that takes every decode warp.
+            if ((!WHOLE || S == 0) && at.left <= 0 && at.settle(ups, stages, enter)) wa -= ring;
             uint32_t L[K];
 #pragma unroll
-            for (int i = 0; i < K; i++) L[i] = ptx::lds32(wa + i * 128u);
+            for (int i = 0; i < K; i++) L[i] = ptx::lds32(wa + (WHOLE ? S * HALF_BYTES : 0u) + i * 128u);
             auto tile = [&](auto tconst, uint32_t ta) {
                 constexpr int T = decltype(tconst)::value;
                 uint32_t own[2];
@@ -767,17 +786,24 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                 close(1);
                 if (S == 0) parity ^= 1;
             }
-            wa += S == 0 ? move0 : move1;
-            at.left -= S == 0 ? adv0 : 3 - adv0;
-            h += SK_GROUPS;
+            if constexpr (!WHOLE) {
+                wa += S == 0 ? move0 : move1;
+                at.left -= S == 0 ? adv0 : 3 - adv0;
+                h += SK_GROUPS;
+            } else if constexpr (S == 1) {
+                wa += SK_GROUPS * W_BYTES;
+                at.left -= SK_GROUPS;
+                h += SK_GROUPS;
+            }
         };
+        const int n = WHOLE ? units : halves;
         EXL3_STAMP_LANE(dw == 0, 3);
         [[maybe_unused]] bool rotated = false;
 #pragma unroll 1
         while (true) {
-            if (h < halves) {
+            if (h < n) {
                 step(std::integral_constant<int, 0>{});
-                if (h < halves) step(std::integral_constant<int, 1>{});
+                if (WHOLE || h < n) step(std::integral_constant<int, 1>{});
                 parity ^= 1;
             }
             if constexpr (X != SK_STREAM) {
@@ -794,7 +820,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                     rotated = true;
                 }
             }
-            if (h >= halves) break;
+            if (h >= n) break;
         }
         EXL3_STAMP_LANE(dw == 0, 4);
         ptx::grid_dependency_wait();
@@ -810,9 +836,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             auto enter = [&](uint32_t slot8, uint32_t parity) {
                 if constexpr (X == SK_STREAM) sk_wait(x_bar + slot8, parity, failed);
             };
-            SkWalk at(group, ups, fills, enter);
+            SkWalk at(WHOLE ? group : group >> 1, ups, fills, enter);
             if constexpr (X == SK_STREAM && group == 0) EXL3_STAMP_LANE(true, 2);
-            uint32_t xa = ptx::smem_addr(xs) + (group >> 1) * F_BYTES + (group & 1) * (F_BYTES / 2);
+            uint32_t xa = ptx::smem_addr(xs) + (WHOLE ? group * F_BYTES : (group >> 1) * F_BYTES + (group & 1) * (F_BYTES / 2));
             constexpr uint32_t chunk = RP;                                  // 16-byte rows between chunks of 8 k slots
             constexpr uint32_t b_hi = (128u >> 4) | (1u << 14);             // 8-row groups 128 bytes apart; descriptor version
             constexpr uint32_t a_base = TM::A_OFF + (uint32_t)(group * TM::A_BUFS) * TM::A_COLS;
@@ -823,11 +849,12 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
             auto step = [&](auto which) {                                   // the steps of the decode warps (see there)
                 constexpr int S = decltype(which)::value;
                 constexpr uint32_t half = S == 0 ? group & 1 : 1 - (group & 1);
+                constexpr int PIECES = WHOLE ? 2 : TM::PARTS;
                 if (at.left <= 0 && at.settle(ups, stages, enter) && X == SK_STREAM) xa -= ring;
                 uint64_t b = ((uint64_t)b_hi << 32) | (chunk << 16) | (xa >> 4);
 #pragma unroll
-                for (int part = 0; part < TM::PARTS; part++) {
-                    constexpr int B0 = TM::PARTS == 1 ? S : 0;
+                for (int part = 0; part < PIECES; part++) {
+                    constexpr int B0 = PIECES == 1 ? S : 0;
                     const int buf = B0 + part;
                     ptx::named_bar_sync(SK_BAR_BUF + group * TM::A_BUFS + buf, (8 + 1) * 32);
                     sk_fence_after();
@@ -836,26 +863,30 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
                         for (int m = 0; m < MMAS; m++)
                             sk_mma(acc, a_base + buf * TM::A_COLS + m * 8, b + m * 2u * chunk, IDESC, m > 0 ? 1u : accumulate);
                         sk_commit_addr(empty0 + buf * 8u);
-                        if (part == TM::PARTS - 1) sk_commit_addr(s_bar + at.slot8);
+                        if (part == PIECES - 1) sk_commit_addr(s_bar + at.slot8);
                     }
                     __syncwarp();
                     accumulate = 1;
                     b += MMAS * 2u * chunk;
                 }
-                xa += half ? 2 * F_BYTES - F_BYTES / 2 : F_BYTES + F_BYTES / 2;
-                at.left -= 1 + half;
+                xa += WHOLE ? SK_GROUPS * F_BYTES : half ? 2 * F_BYTES - F_BYTES / 2 : F_BYTES + F_BYTES / 2;
+                at.left -= WHOLE ? SK_GROUPS : 1 + half;
                 h += SK_GROUPS;
             };
-            bool second = false;                                            // which of the two steps comes next
+            [[maybe_unused]] bool second = false;                                            // which of the two steps comes next
 #pragma unroll 1
             for (int ub = u0; ub < u1;) {                                   // column blocks of the CTA
-                const int left = p.KG - ub % p.KG, ue = ub + left < u1 ? ub + left : u1, he = 2 * (ue - u0);
+                const int left = p.KG - ub % p.KG, ue = ub + left < u1 ? ub + left : u1, he = (WHOLE ? 1 : 2) * (ue - u0);
                 sk_wait(ptx::smem_addr(&acc_empty[d]), acc_parity, failed);
                 sk_fence_after();
                 acc = (d * SK_GROUPS + group) * N;
                 accumulate = 0;
 #pragma unroll 1
                 while (h < he) {
+                    if constexpr (WHOLE) {
+                        step(std::integral_constant<int, 0>{});
+                        continue;
+                    }
                     if (!second) {
                         step(std::integral_constant<int, 0>{});
                         if (h >= he) {
@@ -940,7 +971,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_kernel(const __grid_cons
         int d = 0;
         for (int ub = u0; ub < u1;) {
             const int nb = ub / p.KG, left = (nb + 1) * p.KG - ub, ue = ub + left < u1 ? ub + left : u1;
-            const int hb = 2 * (ub - u0), he = 2 * (ue - u0);
+            const int hb = (WHOLE ? 1 : 2) * (ub - u0), he = (WHOLE ? 1 : 2) * (ue - u0);     // units, or half units
             int c_first, c_last;
             sharers(nb, c_first, c_last);
             const bool shared = c_first != c_last;
