@@ -156,3 +156,31 @@ def test_last_rotation_and_sum_in_one_launch(top_k, tokens, dtype):
         a, b = one.float(), two.float()
         assert bool(((a - b).abs() <= ulp * b.abs() + 2.0 ** -22 * b.abs().max()).all())
         assert float((a != b).float().mean()) <= 0.02
+
+
+@pytest.mark.parametrize("hidden,inter", [(640, 384), (128, 128), (1152, 256)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_rotations_of_pairs_of_row_blocks(hidden, inter, dtype):
+    """The rotations take two neighbouring blocks of eight rows or two column blocks at a time: experts with one row, exactly one block, an odd
+    and an even number of blocks and more than an item's 128 rows, so that pairs lie within an item, across two and at the end; odd numbers of
+    column blocks, and one alone.  fp16: the bars of this file; bf16 adds the rounding of the result, 2^-9 of a value."""
+    K, cb, E = 3, 0, 6
+    counts = [1, 8, 24, 9, 133, 17]
+    gate, up, down = _experts(77 + hidden, E, hidden, inter, K, out_scale=1 / 8)
+    pack = moe.prepare_mixed(_to_dev(gate), _to_dev(up), _to_dev(down), cb)
+    rng = np.random.default_rng(hidden)
+    ids = rng.permutation(np.repeat(np.arange(E), counts)).astype(np.int32)[:, None]
+    tokens = len(ids)
+    assert moe.moe_block_size(tokens, 1, E) == 128
+    w = rng.uniform(0.5, 1.0, (tokens, 1)).astype(np.float32)
+    x = rng.standard_normal((tokens, hidden)).astype(np.float16)
+    xt = torch.from_numpy(x).to(DEV).to(dtype)
+    ref = orc.np_moe_layer(xt.to(torch.float16).cpu().numpy(), ids, w, gate, up, down, K, cb)
+    ws = torch.zeros(moe.layer_workspace_bytes([E], hidden, inter, cb, tokens, 1), dtype=torch.uint8, device=DEV)
+    out = torch.empty_like(xt)
+    moe.run_layer(xt, torch.from_numpy(w).to(DEV), torch.from_numpy(ids).to(DEV), pack, out, ws, None)
+    got = out.float().cpu().numpy()
+    if dtype == torch.float16:
+        _check(out, ref)
+    else:
+        assert orc.rel_norm(got, ref) <= 3e-3 + 2.0 ** -9

@@ -442,6 +442,65 @@ __device__ __forceinline__ void fwht128_turn(float (&v)[32], int lane)
     for (int i = 0; i < 16; i++) f32x2_split(p[i], v[2 * i], v[2 * i + 1]);
 }
 
+// The transform of 16 rows on tensor cores, inputs in fp16: rows g and g + 8 of lane 4 g + t, its elements the 16-byte chunks t, t + 4, t + 8, t + 12 of
+// a row (a[.][4 j + w]: elements 2 w, 2 w + 1 of chunk 4 j + t) -- what 16-byte loads of 64 consecutive bytes give.  Four of the seven index bits
+// (0, 1, and the lane's 3, 4) are the k of m16n8k16 MMAs, whose right operand is the signs of a 16-point transform, or (SIGNED) these
+// times a sign vector: products of two fp16 numbers, exact, so the vector costs nothing.  The other three bits are butterflies between a lane's own
+// registers: no shuffles, half the additions, and results in the layout that the inputs had: p[2 j + b][h][row] is elements 4 b + 2 h, 4 b + 2 h + 1
+// of chunk 4 j + t.  Unnormalised, sums in fp32; 21 million warp instructions where fwht128_turn takes 36 (moe_had_in_kernel, 16384 rows of 2048).
+struct Had128Rows {
+    unsigned long long p[8][2][2];                           // [group][h][row]: packed pairs
+
+    // s: the sign vector's words, laid out as a row; TWO: there are rows g + 8.
+    template <bool SIGNED, bool TWO>
+    __device__ __forceinline__ void run(const uint32_t (&a0)[16], const uint32_t (&a1)[16], const uint32_t (&s)[16], int lane)
+    {
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t mask = (__popc(t & (g >> 1)) & 1 ? 0x80008000u : 0u) ^ (g & 1 ? 0x80000000u : 0u);
+        const uint32_t one = 0x3C003C00u ^ mask;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int w = 4 * (i >> 1) + 2 * (i & 1);        // group 2 j + b: words 2 b, 2 b + 1 of chunk j
+            const uint32_t b0 = SIGNED ? s[w] ^ mask : one, b1 = SIGNED ? s[w + 1] ^ mask : one;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float c[4];
+                asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                    : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                    : "r"(a0[w]), "r"(TWO ? a1[w] : 0u), "r"(a0[w + 1]), "r"(TWO ? a1[w + 1] : 0u), "r"(b0), "r"(h ? b1 ^ 0x80008000u : b1), "f"(0.f));
+                p[i][h][0] = f32x2(c[0], c[1]);
+                p[i][h][1] = f32x2(c[2], c[3]);
+            }
+        }
+        const unsigned long long minus = f32x2(-1.f, -1.f);
+#pragma unroll
+        for (int stride = 1; stride < 8; stride <<= 1) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (i & stride) continue;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+#pragma unroll
+                    for (int r = 0; r < (TWO ? 2 : 1); r++) {
+                        const unsigned long long lo = p[i][h][r], hi = p[i + stride][h][r];
+                        p[i][h][r] = f32x2_add(lo, hi);
+                        p[i + stride][h][r] = f32x2_fma(hi, minus, lo);
+                    }
+                }
+            }
+        }
+    }
+    // Element pair w (0..3) of chunk j of a row.
+    __device__ __forceinline__ void pair(int row, int j, int w, float& x, float& y) const { f32x2_split(p[2 * j + (w >> 1)][w & 1][row], x, y); }
+    // All 32 elements of a row, chunk by chunk.
+    __device__ __forceinline__ void row(int r, float (&v)[32]) const
+    {
+#pragma unroll
+        for (int i = 0; i < 16; i++) pair(r, i >> 2, i & 3, v[2 * i], v[2 * i + 1]);
+    }
+};
+
 constexpr float HAD_SCALE = 0.08838834764831845f;   // 1 / sqrt(128)
 
 // 32 consecutive halves (64 bytes, 16-byte aligned) as floats.

@@ -182,8 +182,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(1024) moe_align_ker
 // ------------------------------------------------------------------------------------------------ rotations
 
 // A lane's 32 values of a row in the B-operand layout of the grouped GEMM (k chunk by k chunk of eight, a 16-byte word per row, `rows`
-// rows): the warp's stores fill 128-byte lines.  DEALT: the lane holds chunks q, q + 4, ... (see fwht128_turn), else 4 q, 4 q + 1, ...
-template <bool DEALT>
+// rows): the warp's stores fill 128-byte lines.  The lane holds chunks q, q + 4, ...
 __device__ __forceinline__ void moe_store_rows(unsigned char* unit, int rows, int row, int q, const float (&v)[32])
 {
 #pragma unroll
@@ -194,24 +193,66 @@ __device__ __forceinline__ void moe_store_rows(unsigned char* unit, int rows, in
             const __half2 h = __floats2half2_rn(v[8 * j + 2 * i] * HAD_SCALE, v[8 * j + 2 * i + 1] * HAD_SCALE);
             w[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        *reinterpret_cast<uint4*>(unit + ((size_t)(DEALT ? 4 * j + q : 4 * q + j) * rows + row) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(unit + ((size_t)(4 * j + q) * rows + row) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// A lane's 32 halves of 128 (16-byte aligned) as packed words: 32 consecutive ones, or (DEALT) 16-byte chunks q, q + 4, ...
-template <bool DEALT>
+// A lane's 32 halves of 128 (16-byte aligned) as packed words: 16-byte chunks q, q + 4, ...
 __device__ __forceinline__ void moe_load32(const void* base, long long at, int q, uint32_t (&w)[16])
 {
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at) + (DEALT ? q : 4 * q);
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at) + q;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const uint4 r = src[DEALT ? 4 * i : i];
+        const uint4 r = src[4 * i];
         w[4 * i] = r.x;
         w[4 * i + 1] = r.y;
         w[4 * i + 2] = r.z;
         w[4 * i + 3] = r.w;
     }
 }
+// The same through shared memory, requested one column block ahead without holding registers: with 16 warps per SM (a lane's transform takes half
+// of its registers) the latency of plain loads was three quarters of these kernels' time.  A warp's own: two rows per lane group, and up to three
+// vectors that are the same for all its rows.  CTAs of four warps keep this within the shared memory that needs no opting in.
+constexpr int MOE_HAD_WARPS = 4;
+template <int ROWS>
+struct MoeStage {
+    uint4 row[2 * ROWS][4][32];                                          // ... and their vectors, where every row has its own (ROWS = 2)
+    uint4 vec[3][16];
+
+    static __device__ __forceinline__ void copy16(void* to, const void* from)
+    {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_addr(to)), "l"(from) : "memory");
+    }
+    __device__ __forceinline__ void fetch_row(int r, const void* base, long long at, int lane)
+    {
+        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at) + (lane & 3);
+#pragma unroll
+        for (int i = 0; i < 4; i++) copy16(&row[r][i][lane], src + 4 * i);
+    }
+    __device__ __forceinline__ void fetch_vec(int i, const void* base, long long at, int lane)
+    {
+        if (lane < 16) copy16(&vec[i][lane], reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + at) + lane);
+    }
+    static __device__ __forceinline__ void arrived()                    // what was fetched is there, for the whole warp
+    {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+    }
+    static __device__ __forceinline__ void words(const uint4* at, int step, uint32_t (&w)[16])
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint4 r = at[i * step];
+            w[4 * i] = r.x;
+            w[4 * i + 1] = r.y;
+            w[4 * i + 2] = r.z;
+            w[4 * i + 3] = r.w;
+        }
+    }
+    __device__ __forceinline__ void load_row(int r, int lane, uint32_t (&w)[16]) const { words(&row[r][0][lane], 32, w); }
+    __device__ __forceinline__ void load_vec(int i, int lane, uint32_t (&w)[16]) const { words(&vec[i][lane & 3], 4, w); }
+};
+
 __device__ __forceinline__ float moe_half(const uint32_t (&w)[16], int i)
 {
     const __half2 h = *reinterpret_cast<const __half2*>(&w[i >> 1]);
@@ -302,21 +343,23 @@ __global__ void __launch_bounds__(256) moe_glu_had_in_rows_kernel(const __half* 
     moe_store_row<MODE>(xf + ((long long)b * kgs + kg) * MOE_BLOCK_ROWS * F_ROW, MOE_BLOCK_ROWS, row % MOE_BLOCK_ROWS, lane, v);
 }
 
-// 32 columns of a rotated-basis row back in the true basis: Had128(y) * svh, rounded to fp16 like the output of the linear.
-__device__ __forceinline__ void moe_unrotate32(const uint32_t (&w)[16], const uint32_t (&sw)[16], int lane, float (&v)[32])
+// 32 values of a row (Had128Rows) back in the true basis: times svh, rounded to fp16 like the output of the linear.
+__device__ __forceinline__ void moe_unrotate32(const Had128Rows& had, int r, const uint32_t (&sw)[16], float (&v)[32])
 {
-#pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = moe_half(w, i);
-    fwht128_turn(v, lane);
+    had.row(r, v);
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] * (HAD_SCALE * moe_half(sw, i))));
 }
 
-// The kernels for long items.  A warp takes a block of eight rows, four lanes per row (fwht128_turn), and a span of up to four column blocks
-// of 128 of it: 16-byte loads and full-line stores, and the chain of dependent loads (block -> expert and slot -> values) is walked once
-// per span -- with one column block per warp it is what bounds these kernels (70 us instead of 22 us of traffic for 2048 tokens, top-8,
-// 2048 columns).  The span is halved while the warps are not enough for two full loads of the chip (span_of; a layer of 2048 tokens, 32
-// experts of 1024 x 384, top-2: 86 us with four, 76 with two, and the middle step of 2048 x 512, top-8, 8 us less with one than with two).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
+// The kernels for long items: the transforms of 16 rows by tensor-core MMAs (Had128Rows), their inputs one column block ahead in shared memory
+// (MoeStage).  A warp takes a block of eight rows (the way in: two neighbouring blocks; behind the GEMMs two column blocks, or gate and up, are
+// the 16 rows) and a span of up to four column blocks, so that the chain of dependent loads (block -> expert and slot -> values) is walked once
+// per span.  The span is halved while the warps are not enough for two full loads of the chip (span_of).  Bound by latency and issue together:
+// 2048 tokens, 256 experts of 2048 x 512, top-8, the three kernels, thousands of cycles and millions of warp instructions, before (fwht128_turn,
+// eight rows per warp, 24 warps per SM, plain loads) / with MMAs alone / one column block ahead: way in 98, 36 / 75, 21 / 71, 22; middle 61, 19 / 56, 14 /
+// 48, 14; out and sum 60, 24 / 54, 17 / 49, 18.  The layer: 347 us -> 348 -> 321, 700 tokens, 64 experts of 1536 x 768, top-6 131 -> 124, 2048 tokens,
+// 32 experts of 1024 x 384, top-2 67 -> 63.5.  Rows through L1 lose it again (338 us), and so does one row that all lanes without a slot ask for (700
+// tokens: 137).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.
 struct MoeSpan {
     int b, kg0, kg1, slot, ex;
     bool valid, any;
@@ -338,52 +381,93 @@ struct MoeSpan {
     }
 };
 
-// xf[shard][item][row block] = Had128(fp16(x[token(p)]) * suh[expert(p), shard]) in the B-operand layout; blockIdx.y = shard (both
-// shards from one load of x cost 128 registers and a third of the warps in flight).
-__global__ void __launch_bounds__(256, 3) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
+// xf[shard][item][row block] = Had128(fp16(x[token(p)]) * suh[expert(p), shard]) in the B-operand layout; blockIdx.y = shard.  A warp takes two
+// neighbouring blocks of eight rows, together where they are of one item and one after the other where not.
+__global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_had_in_kernel(const void* __restrict__ x, int x_bf16, const __half* __restrict__ suh, int hidden, int top_k,
                                                             int numel, int cap, const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                                             const int* __restrict__ num_post, const int2* __restrict__ blk,
                                                             unsigned char* __restrict__ xf, long long shard_stride, int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
-    const int lane = threadIdx.x & 31, q = lane & 3, kgs = hidden >> 7;
-    const MoeSpan at(span, kgs, cap, numel, sorted_ids, expert_ids, num_post);
-    if (!at.any) return;
-    const int2 run = blk[at.b];
-    const int rows = run.y * MOE_BLOCK_ROWS, row = (at.b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
-    const long long x_row = (long long)(at.valid ? at.slot / top_k : 0) * hidden;
-    const __half* signs = suh + ((long long)at.ex * gridDim.y + blockIdx.y) * hidden;
-    unsigned char* unit = xf + blockIdx.y * shard_stride + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
+    __shared__ MoeStage<1> stages[MOE_HAD_WARPS];
+    MoeStage<1>& st = stages[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, q = lane & 3, kgs = hidden >> 7, spans = (kgs + span - 1) / span;
+    const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), pair = id / spans;
+    const int kg0 = (id - pair * spans) * span, kg1 = kg0 + span < kgs ? kg0 + span : kgs;
+    const int b0 = 2 * pair, blocks = cap / MOE_BLOCK_ROWS;
+    if (b0 >= blocks) return;
+    const int2 first = blk[b0];                                                   // beside the number of blocks in use, not behind it
+    int2 second = blk[b0 + 1 < blocks ? b0 + 1 : b0];
+    const int post = *num_post / MOE_BLOCK_ROWS;
+    if (b0 >= post) return;
+    if (b0 + 1 >= post) second.x = -1;
+    const bool both = first.x == second.x;
 #pragma unroll 1
-    for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
-        uint32_t xw[16], sw[16];
-        moe_load32<true>(x, x_row + kg * 128, q, xw);
-        moe_load32<true>(signs, kg * 128, q, sw);
-        if (x_bf16) {
+    for (int pass = 0; pass < (both || b0 + 1 >= post ? 1 : 2); pass++) {
+        const int b = b0 + pass, ex = expert_ids[b];
+        const int2 run = pass ? second : first;
+        const int rows = run.y * MOE_BLOCK_ROWS, row = (b - run.x) * MOE_BLOCK_ROWS + (lane >> 2);
+        int slot[2];
+        slot[0] = sorted_ids[b * MOE_BLOCK_ROWS + (lane >> 2)];
+        slot[1] = both ? sorted_ids[(b + 1) * MOE_BLOCK_ROWS + (lane >> 2)] : -1;
+        long long x_row[2];
+        bool valid[2];
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xw[i]);
-                const __half2 h = __floats2half2_rn(__low2float(bb), __high2float(bb));
-                xw[i] = *reinterpret_cast<const uint32_t*>(&h);
+        for (int r = 0; r < 2; r++) {
+            valid[r] = slot[r] >= 0 && slot[r] < numel;
+            x_row[r] = (long long)(valid[r] ? slot[r] / top_k : 0) * hidden;
+        }
+        const __half* signs = suh + ((long long)ex * gridDim.y + blockIdx.y) * hidden;
+        unsigned char* unit = xf + blockIdx.y * shard_stride + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)kg0 * rows) * 256;
+        auto fetch = [&](int kg) {
+            if (valid[0]) st.fetch_row(0, x, x_row[0] + kg * 128, lane);     // not one row that every padded one would ask the same cache line for
+            if (valid[1]) st.fetch_row(1, x, x_row[1] + kg * 128, lane);
+            st.fetch_vec(0, signs, kg * 128, lane);
+        };
+        __syncwarp();
+        fetch(kg0);
+#pragma unroll 1
+        for (int kg = kg0; kg < kg1; kg++, unit += rows * 256) {
+            uint32_t xw[2][16], sw[16];
+            st.arrived();
+            st.load_row(0, lane, xw[0]);
+            st.load_row(1, lane, xw[1]);
+            st.load_vec(0, lane, sw);
+            __syncwarp();
+            if (kg + 1 < kg1) fetch(kg + 1);
+            if (x_bf16) {
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xw[r][i]);
+                        const __half2 h = __floats2half2_rn(__low2float(bb), __high2float(bb));
+                        xw[r][i] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+            }
+            Had128Rows had;
+            had.run<true, true>(xw[0], xw[1], sw, lane);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float v[32];
+                had.row(r, v);
+                if (valid[r]) moe_store_rows(unit, rows, row + 8 * r, q, v);
             }
         }
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = moe_half(xw, i) * moe_half(sw, i);
-        fwht128_turn(v, lane);
-        if (at.valid) moe_store_rows<false>(unit, rows, row, q, v);
     }
 }
 
 // The input of the down projection: Had128( fp16( silu(gate) * up ) * suh2[expert] ) with gate | up = Had128(gu_rot[row]) * svh13[expert].
-__global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restrict__ gu_rot, const __half* __restrict__ svh13,
+__global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_mid_kernel(const __half* __restrict__ gu_rot, const __half* __restrict__ svh13,
                                                          const __half* __restrict__ suh2, int inter, int numel, int cap,
                                                          const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                                          const int* __restrict__ num_post, const int2* __restrict__ blk, unsigned char* __restrict__ xf, int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
+    __shared__ MoeStage<1> stages[MOE_HAD_WARPS];
+    MoeStage<1>& st = stages[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, q = lane & 3, kgs = inter >> 7;
     const MoeSpan at(span, kgs, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
@@ -393,37 +477,57 @@ __global__ void __launch_bounds__(256, 2) moe_mid_kernel(const __half* __restric
     const __half* sv = svh13 + (long long)at.ex * 2 * inter;
     const __half* s2 = suh2 + (long long)at.ex * inter;
     unsigned char* unit = xf + ((long long)run.x * MOE_BLOCK_ROWS * kgs + (long long)at.kg0 * rows) * 256;
+    auto fetch = [&](int kg) {
+        st.fetch_row(0, gu, (long long)kg * rows * 128, lane);
+        st.fetch_row(1, gu, (long long)(kgs + kg) * rows * 128, lane);
+        st.fetch_vec(0, sv, kg * 128, lane);
+        st.fetch_vec(1, sv, inter + kg * 128, lane);
+        st.fetch_vec(2, s2, kg * 128, lane);
+    };
+    fetch(at.kg0);
 #pragma unroll 1
     for (int kg = at.kg0; kg < at.kg1; kg++, unit += rows * 256) {
-        uint32_t w[16], sw[16], u[16];                        // up is fp16 by now: packed again, it leaves room for gate
+        uint32_t g[16], u[16], sw[16];
+        st.arrived();
+        st.load_row(0, lane, g);
+        st.load_row(1, lane, u);
+        Had128Rows had;                                       // gate and up are its two rows
+        had.run<false, true>(g, u, g, lane);
         float v[32];
-        moe_load32<true>(gu, (long long)(kgs + kg) * rows * 128, q, w);
-        moe_load32<false>(sv, inter + kg * 128, q, sw);
-        moe_unrotate32(w, sw, lane, v);
+        st.load_vec(1, lane, sw);
+        moe_unrotate32(had, 1, sw, v);
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
             u[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        moe_load32<true>(gu, (long long)kg * rows * 128, q, w);
-        moe_load32<false>(sv, kg * 128, q, sw);
-        moe_unrotate32(w, sw, lane, v);
-        moe_load32<false>(s2, kg * 128, q, sw);
+        st.load_vec(0, lane, sw);
+        moe_unrotate32(had, 0, sw, v);
+        st.load_vec(2, lane, sw);
+        __syncwarp();
+        if (kg + 1 < at.kg1) fetch(kg + 1);
 #pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = __half2float(__float2half_rn(v[i] / (1.0f + __expf(-v[i])) * moe_half(u, i))) * moe_half(sw, i);
-        fwht128_turn(v, lane);
-        if (at.valid) moe_store_rows<true>(unit, rows, row, q, v);
+        for (int i = 0; i < 16; i++) {
+            const __half2 h = __floats2half2_rn(v[2 * i] / (1.0f + __expf(-v[2 * i])) * moe_half(u, 2 * i),
+                                                v[2 * i + 1] / (1.0f + __expf(-v[2 * i + 1])) * moe_half(u, 2 * i + 1));
+            g[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        had.run<true, false>(g, g, sw, lane);
+        had.row(0, v);
+        if (at.valid) moe_store_rows(unit, rows, row, q, v);
     }
 }
 
 // yd[slot(row), :] = fp16( Had128(yd_rot[row]) * svh2[expert] ).
-__global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
+__global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_out_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2, int hidden, int numel, int cap,
                                                          const int* __restrict__ sorted_ids, const int* __restrict__ expert_ids,
                                                          const int* __restrict__ num_post, const int2* __restrict__ blk, __half* __restrict__ yd,
                                                          int span)
 {
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
+    __shared__ MoeStage<1> stages[MOE_HAD_WARPS];
+    MoeStage<1>& st = stages[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, q = lane & 3;
     const MoeSpan at(span, hidden >> 7, cap, numel, sorted_ids, expert_ids, num_post);
     if (!at.any) return;
@@ -432,23 +536,40 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
     const __half* src = yd_rot + (long long)run.x * MOE_BLOCK_ROWS * hidden + row * 128;                     // [column block][row][128]
     const __half* sv = svh2 + (long long)at.ex * hidden;
     __half* dst = yd + (long long)(at.valid ? at.slot : 0) * hidden + 8 * q;
+    auto fetch = [&](int kg) {
+        const int next = kg + 1 < at.kg1 ? kg + 1 : kg;
+        st.fetch_row(0, src, (long long)kg * rows * 128, lane);
+        st.fetch_row(1, src, (long long)next * rows * 128, lane);
+    };
+    fetch(at.kg0);
 #pragma unroll 1
-    for (int kg = at.kg0; kg < at.kg1; kg++) {
-        uint32_t w[16], sw[16];
-        moe_load32<false>(src, (long long)kg * rows * 128, q, w);
-        moe_load32<true>(sv, kg * 128, q, sw);
-        float v[32];
-        moe_unrotate32(w, sw, lane, v);
-        if (!at.valid) continue;
+    for (int kg = at.kg0; kg < at.kg1; kg += 2) {             // two column blocks are the transform's two rows
+        const bool two = kg + 1 < at.kg1;
+        uint32_t w[2][16];
+        st.arrived();
+        st.load_row(0, lane, w[0]);
+        st.load_row(1, lane, w[1]);
+        __syncwarp();
+        if (kg + 2 < at.kg1) fetch(kg + 2);
+        Had128Rows had;
+        had.run<false, true>(w[0], w[1], w[0], lane);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint32_t o[4];
+        for (int r = 0; r < 2; r++) {
+            if (!at.valid || (r && !two)) break;
+            uint32_t sw[16];
+            moe_load32(sv, (kg + r) * 128, q, sw);
+            float v[32];
+            moe_unrotate32(had, r, sw, v);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const __half2 h = __floats2half2_rn(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
-                o[j] = *reinterpret_cast<const uint32_t*>(&h);
+            for (int i = 0; i < 4; i++) {
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const __half2 h = __floats2half2_rn(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
+                    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                reinterpret_cast<uint4*>(dst + (kg + r) * 128)[4 * i] = make_uint4(o[0], o[1], o[2], o[3]);
             }
-            reinterpret_cast<uint4*>(dst + kg * 128)[4 * i] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
 }
@@ -459,7 +580,7 @@ __global__ void __launch_bounds__(256, 3) moe_out_kernel(const __half* __restric
 // of two, at most eight; more come in rounds), four lanes per row; the rows of a token are added by exchanging halves, so that every lane ends
 // with 32 / G of the 128 columns, its own.  Traffic bounds it (2048 tokens, top-8, 2048 columns: 67 MB, 10.4 us).
 template <int G>
-__global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2,
+__global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_out_combine_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2,
                                                                  const float* __restrict__ weights, const int* __restrict__ place,
                                                                  const int* __restrict__ expert_ids, const int2* __restrict__ blk, int tokens, int top_k,
                                                                  int hidden, void* __restrict__ y, int y_bf16, int span)
@@ -467,6 +588,8 @@ __global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* _
     ptx::grid_launch_dependents();
     ptx::grid_dependency_wait();
     constexpr int N = 32 / G;
+    __shared__ MoeStage<2> stages[MOE_HAD_WARPS];
+    MoeStage<2>& st = stages[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, q = lane & 3, r = lane >> 2, kgs = hidden >> 7, spans = (kgs + span - 1) / span;
     const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), group = id / spans, kg0 = (id - group * spans) * span;
     const int t = group * (8 / G) + r / G, kg1 = kg0 + span < kgs ? kg0 + span : kgs;
@@ -478,59 +601,82 @@ __global__ void __launch_bounds__(256, 3) moe_out_combine_kernel(const __half* _
     auto look = [&](int j0) {                                     // this lane's slot of a round
         const int j = j0 + r % G, slot = t * top_k + j, at = t < tokens && j < top_k ? place[slot] : -1;
         valid = at >= 0;
-        src = yd_rot;
-        sv = svh2;
-        pitch = 0;
         if (!valid) return;
         const int b = at / MOE_BLOCK_ROWS;
         const int2 run = blk[b];
         wt = weights[slot];
-        src += (long long)run.x * MOE_BLOCK_ROWS * hidden + (at - run.x * MOE_BLOCK_ROWS) * 128;            // [column block][row][128]
+        src = yd_rot + (long long)run.x * MOE_BLOCK_ROWS * hidden + (at - run.x * MOE_BLOCK_ROWS) * 128;            // [column block][row][128]
         pitch = (long long)run.y * MOE_BLOCK_ROWS * 128;
-        sv += (long long)expert_ids[b] * hidden;
+        sv = svh2 + (long long)expert_ids[b] * hidden;
     };
     look(0);
+    auto fetch = [&](int kg) {
+        if (!valid) return;                                       // not one row that every such lane would ask the same cache line for
+        const int next = kg + 1 < kg1 ? kg + 1 : kg;
+        st.fetch_row(0, src, kg * pitch, lane);
+        st.fetch_row(1, src, next * pitch, lane);
+        st.fetch_row(2, sv, kg * 128, lane);
+        st.fetch_row(3, sv, next * 128, lane);
+    };
+    if (top_k <= G) fetch(kg0);
 #pragma unroll 1
-    for (int kg = kg0; kg < kg1; kg++) {
-        float sum[N] = {};
+    for (int kg = kg0; kg < kg1; kg += 2) {                       // two column blocks are the transform's two rows
+        const bool two = kg + 1 < kg1;
+        float sum[2][N] = {};
 #pragma unroll 1
         for (int j0 = 0; j0 < top_k; j0 += G) {
-            if (top_k > G) look(j0);
-            uint32_t w[16], sw[16];
-            moe_load32<false>(src, kg * pitch, q, w);
-            moe_load32<true>(sv, kg * 128, q, sw);
-            float v[32];
-            moe_unrotate32(w, sw, lane, v);
-#pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = valid ? v[i] * wt : 0.f;
-#pragma unroll
-            for (int m = 2 * G, n = 32; m >= 4; m >>= 1, n >>= 1) {           // lanes m apart exchange halves of n values
-                const bool upper = (lane & m) != 0;
-#pragma unroll
-                for (int i = 0; i < n / 2; i++) {
-                    const float keep = upper ? v[i + n / 2] : v[i], send = upper ? v[i] : v[i + n / 2];
-                    v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, m);
-                }
+            if (top_k > G) {
+                look(j0);
+                fetch(kg);
             }
+            uint32_t w[2][16];
+            st.arrived();
+            st.load_row(0, lane, w[0]);
+            st.load_row(1, lane, w[1]);
+            Had128Rows had;
+            had.run<false, true>(w[0], w[1], w[0], lane);
 #pragma unroll
-            for (int i = 0; i < N; i++) sum[i] += v[i];
+            for (int b = 0; b < 2; b++) {
+                if (b && !two) break;
+                uint32_t sw[16];
+                st.load_row(2 + b, lane, sw);
+                if (top_k <= G && b == 1 && kg + 2 < kg1) fetch(kg + 2);      // what a lane fetches it alone reads
+                float v[32];
+                moe_unrotate32(had, b, sw, v);
+#pragma unroll
+                for (int i = 0; i < 32; i++) v[i] = valid ? v[i] * wt : 0.f;
+#pragma unroll
+                for (int m = 2 * G, n = 32; m >= 4; m >>= 1, n >>= 1) {       // lanes m apart exchange halves of n values
+                    const bool upper = (lane & m) != 0;
+#pragma unroll
+                    for (int i = 0; i < n / 2; i++) {
+                        const float keep = upper ? v[i + n / 2] : v[i], send = upper ? v[i] : v[i + n / 2];
+                        v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, m);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < N; i++) sum[b][i] += v[i];
+            }
         }
-        if (t >= tokens) continue;
-        uint32_t o[N / 2];
 #pragma unroll
-        for (int i = 0; i < N / 2; i++) {
-            const __half2 h = __floats2half2_rn(sum[2 * i], sum[2 * i + 1]);
-            const __nv_bfloat162 bb = __floats2bfloat162_rn(__low2float(h), __high2float(h));
-            o[i] = y_bf16 ? *reinterpret_cast<const uint32_t*>(&bb) : *reinterpret_cast<const uint32_t*>(&h);
-        }
-        const int at = (r % G) * N;                                // of the 32 values, whose i-th is column 32 (i / 8) + 8 q + i % 8
-        uint16_t* dst = reinterpret_cast<uint16_t*>(y) + (long long)t * hidden + kg * 128 + 8 * q;
-        if constexpr (N >= 8) {
+        for (int b = 0; b < 2; b++) {
+            if (t >= tokens || (b && !two)) break;
+            uint32_t o[N / 2];
 #pragma unroll
-            for (int i = 0; i < N / 8; i++)
-                *reinterpret_cast<uint4*>(dst + 32 * (at / 8 + i)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-        } else {
-            *reinterpret_cast<uint2*>(dst + 32 * (at / 8) + at % 8) = make_uint2(o[0], o[1]);
+            for (int i = 0; i < N / 2; i++) {
+                const __half2 h = __floats2half2_rn(sum[b][2 * i], sum[b][2 * i + 1]);
+                const __nv_bfloat162 bb = __floats2bfloat162_rn(__low2float(h), __high2float(h));
+                o[i] = y_bf16 ? *reinterpret_cast<const uint32_t*>(&bb) : *reinterpret_cast<const uint32_t*>(&h);
+            }
+            const int at = (r % G) * N;                            // of the 32 values, whose i-th is column 32 (i / 8) + 8 q + i % 8
+            uint16_t* dst = reinterpret_cast<uint16_t*>(y) + (long long)t * hidden + (kg + b) * 128 + 8 * q;
+            if constexpr (N >= 8) {
+#pragma unroll
+                for (int i = 0; i < N / 8; i++)
+                    *reinterpret_cast<uint4*>(dst + 32 * (at / 8 + i)) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            } else {
+                *reinterpret_cast<uint2*>(dst + 32 * (at / 8) + at % 8) = make_uint2(o[0], o[1]);
+            }
         }
     }
 }
@@ -626,16 +772,16 @@ int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Column blocks per warp for `groups` groups of eight rows, and the CTAs of eight warps that this takes: up to four, as long as the warps fill the
-// chip (24 per SM) twice.
-static int span_of(long long groups, int cols)
+// chip (16 per SM) twice.
+static int span_of(long long groups, int cols, int least = 1)
 {
     const DeviceInfo* d = current_device_info();
-    const long long enough = 2 * 24 * (long long)(d ? d->sm_count : 148);
+    const long long enough = 2 * 16 * (long long)(d ? d->sm_count : 148);
     int span = 4;
-    while (span > 1 && groups * ((cols / 128 + span - 1) / span) < enough) span /= 2;
+    while (span > least && groups * ((cols / 128 + span - 1) / span) < enough) span /= 2;
     return span;
 }
-static unsigned span_blocks(long long groups, int cols, int span) { return blocks_for(groups * ((cols / 128 + span - 1) / span), 8); }
+static unsigned span_blocks(long long groups, int cols, int span) { return blocks_for(groups * ((cols / 128 + span - 1) / span), MOE_HAD_WARPS); }
 
 int launch_moe_had_in(const void* x, int x_bf16, const __half* suh, int shards, int hidden, int top_k, int numel, int cap,
                       const int* sorted_ids, const int* expert_ids, const int* num_post, void* xf, long long shard_stride, int mode, cudaStream_t st)
@@ -656,8 +802,8 @@ int launch_moe_glu_had_in(const __half* gu, const __half* suh2, int inter, int n
 int launch_moe_had_in_items(const void* x, int x_bf16, const __half* suh13, int hidden, int top_k, int numel, int cap, const int* sorted_ids,
                             const int* expert_ids, const int* num_post, const int2* blk, void* xf, long long shard_stride, cudaStream_t st)
 {
-    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(2 * groups, hidden);
-    return launch_chained(moe_had_in_kernel, dim3(span_blocks(groups, hidden, span), 2), dim3(256), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
+    const int pairs = (cap / MOE_BLOCK_ROWS + 1) / 2, span = span_of(2 * pairs, hidden);
+    return launch_chained(moe_had_in_kernel, dim3(span_blocks(pairs, hidden, span), 2), dim3(MOE_HAD_WARPS * 32), 0, st, x, x_bf16, suh13, hidden, top_k, numel, cap, sorted_ids,
                           expert_ids, num_post, blk, reinterpret_cast<unsigned char*>(xf), shard_stride, span);
 }
 
@@ -665,15 +811,15 @@ int launch_moe_mid_items(const __half* gu_rot, const __half* svh13, const __half
                          const int* expert_ids, const int* num_post, const int2* blk, void* xf, cudaStream_t st)
 {
     const int groups = cap / MOE_BLOCK_ROWS, span = span_of(groups, inter);
-    return launch_chained(moe_mid_kernel, dim3(span_blocks(groups, inter, span)), dim3(256), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
+    return launch_chained(moe_mid_kernel, dim3(span_blocks(groups, inter, span)), dim3(MOE_HAD_WARPS * 32), 0, st, gu_rot, svh13, suh2, inter, numel, cap, sorted_ids, expert_ids,
                           num_post, blk, reinterpret_cast<unsigned char*>(xf), span);
 }
 
 int launch_moe_out_items(const __half* yd_rot, const __half* svh2, int hidden, int numel, int cap, const int* sorted_ids, const int* expert_ids,
                          const int* num_post, const int2* blk, __half* yd, cudaStream_t st)
 {
-    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(groups, hidden);
-    return launch_chained(moe_out_kernel, dim3(span_blocks(groups, hidden, span)), dim3(256), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
+    const int groups = cap / MOE_BLOCK_ROWS, span = span_of(groups, hidden, 2);
+    return launch_chained(moe_out_kernel, dim3(span_blocks(groups, hidden, span)), dim3(MOE_HAD_WARPS * 32), 0, st, yd_rot, svh2, hidden, numel, cap, sorted_ids, expert_ids,
                           num_post, blk, yd, span);
 }
 
@@ -682,8 +828,8 @@ int launch_moe_out_combine(const __half* yd_rot, const __half* svh2, const float
 {
     const int g = top_k > 4 ? 8 : top_k > 2 ? 4 : top_k;
     auto* const kernel = g == 8 ? moe_out_combine_kernel<8> : g == 4 ? moe_out_combine_kernel<4> : g == 2 ? moe_out_combine_kernel<2> : moe_out_combine_kernel<1>;
-    const int groups = (tokens + 8 / g - 1) / (8 / g), span = span_of(groups, hidden);
-    return launch_chained(kernel, dim3(span_blocks(groups, hidden, span)), dim3(256), 0, st, yd_rot, svh2, weights, place, expert_ids, blk, tokens, top_k, hidden,
+    const int groups = (tokens + 8 / g - 1) / (8 / g), span = span_of(groups, hidden, 2);
+    return launch_chained(kernel, dim3(span_blocks(groups, hidden, span)), dim3(MOE_HAD_WARPS * 32), 0, st, yd_rot, svh2, weights, place, expert_ids, blk, tokens, top_k, hidden,
                           y, y_bf16, span);
 }
 
