@@ -364,6 +364,8 @@ __device__ __forceinline__ unsigned long long f32x2_fma(unsigned long long a, un
     return r;
 }
 
+// APART: lanes between the four of a row (1: lane l holds elements of row l >> 2, as above; 8: of row l & 7, elements 32 * (l >> 3) ..).
+template <int APART = 1>
 __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane)
 {
     unsigned long long p[16];
@@ -382,7 +384,7 @@ __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane)
         }
     }
 #pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
+    for (int m = APART; m < 4 * APART; m <<= 1) {
         const float sign = (lane & m) != 0 ? -1.f : 1.f;
         const unsigned long long sign2 = f32x2(sign, sign);
 #pragma unroll

@@ -405,7 +405,9 @@ __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsi
     const int rows = p.a.rows;
     const bool bf16 = p.a.x_bf16 != 0;
     constexpr int RP = SK_ROTATE_ROWS;
-    const int q = lane & 3, row = lane >> 2;
+    // Eight rows side by side in a quarter warp: its loads (planes are 16 bytes apart in the banks) and stores are conflict-free.  With
+    // the four lanes of a row side by side the stores of a unit were 128 cycles of shared memory instead of 32.
+    const int q = lane >> 3, row = lane & 7;
 #pragma unroll 1
     for (int i = warp; i < units; i += SK_DECODE_WARPS) {
         float v[32];
@@ -427,7 +429,7 @@ __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsi
                 v[8 * j + 2 * e + 1] = __high2float(s) * __high2float(h);
             }
         }
-        fwht128_quad(v, lane);
+        fwht128_quad<8>(v, lane);
         if (row < rows) {
             unsigned char* slot = xs + (uint32_t)i * (RP * (MODE == GEMV_SPLIT ? 512u : 256u)) + row * 16;
 #pragma unroll
