@@ -689,66 +689,77 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
     }
 }
 
-// Rotated activations in the A-operand layout of gemm_tc_kernel.  One warp per (shard, group of 8 rows, 128-block), four lanes
-// per row (fwht128_turn): a lane's 32 results are four whole 16-byte core-matrix rows, and the eight lanes that share a
-// column range fill a 128-byte core matrix.  Rows beyond `rows` inside the last group are written as zeros.
-constexpr int HAD_IN_TC_ROWS = 8;
-__global__ void had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_cols, const __half* __restrict__ suh, int shards, int rows, int k,
-                                 __half* __restrict__ xa, long long shard_stride)
+// Rotated activations in the A-operand layout of gemm_tc_kernel.  One warp per (shard, 16 rows, 128-block), the transform on tensor cores
+// (Had128Rows): a lane's results are whole 16-byte core-matrix rows, and the eight lanes with the same chunk fill a 128-byte core matrix.
+// Rows beyond `rows` inside the last group of eight are written as zeros.  With fwht128_turn on eight rows per warp before / now, the whole call in
+// bursts, us: 2048 rows, 5120 x 2 x 17408, K = 4 643.7 / 639.2, 5120 x (5120 + 2 x 1024), bf16 202.6 / 193.4, 1024 rows, 17408 x 5120 269.0 / 265.5,
+// 100 rows, 5120 x 7168 32.8 / 31.2, 70 rows, 2048 x 1024 14.0 / 13.7.  The output rotation in the epilogue of the CTA-pair kernel stays as it is: with
+// the same transform it takes tensor-pipe time from the tcgen05 MMAs and registers that spill (631 -> 646 us).
+constexpr int HAD_IN_TC_ROWS = 16, HAD_IN_TC_WARPS = 4;
+__global__ void __launch_bounds__(HAD_IN_TC_WARPS * 32, 4) had_in_tc_kernel(const void* __restrict__ x, int x_bf16, int x_cols, const __half* __restrict__ suh,
+                                                                            int shards, int rows, int k, __half* __restrict__ xa, long long shard_stride)
 {
     // The GEMM behind this one reads weights before its own wait: it may start once everything ahead of this kernel is done.
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, t = lane & 3;
     const int kgs = k >> 7;
     const int groups = (rows + HAD_IN_TC_ROWS - 1) / HAD_IN_TC_ROWS;
     const long long item = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= (long long)shards * groups * kgs) return;
     const int kg = (int)(item % kgs);
-    const int row = (int)((item / kgs) % groups) * HAD_IN_TC_ROWS + (lane >> 2);
+    const int row0 = (int)((item / kgs) % groups) * HAD_IN_TC_ROWS + (lane >> 2);
     const int s = (int)(item / ((long long)kgs * groups));
-    const int col = kg * 128 + 32 * (lane & 3);
-    float v[32];
-    if (row < rows) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int c = kg * 128 + 32 * i + 8 * (lane & 3);
-            // rows of x are x_cols (a multiple of 8) long, zeros from there to k
-            const uint4 raw = c < x_cols ? *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * x_cols + c)
-                                         : make_uint4(0u, 0u, 0u, 0u);
-            const uint4 sraw = *reinterpret_cast<const uint4*>(suh + (long long)s * k + c);
-            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w}, sw[4] = {sraw.x, sraw.y, sraw.z, sraw.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                float x0, x1;
-                if (x_bf16) {
-                    const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-                    x0 = __half2float(__float2half_rn(__low2float(bb)));
-                    x1 = __half2float(__float2half_rn(__high2float(bb)));
-                } else {
-                    const __half2 h = *reinterpret_cast<const __half2*>(&w[j]);
-                    x0 = __low2float(h);
-                    x1 = __high2float(h);
-                }
-                const __half2 sh = *reinterpret_cast<const __half2*>(&sw[j]);
-                v[8 * i + 2 * j] = x0 * __low2float(sh);
-                v[8 * i + 2 * j + 1] = x1 * __high2float(sh);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = 0.f;
-    }
-    fwht128_turn(v, lane);
+    uint32_t xw[2][16], sw[16];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        uint32_t o[4];
+        const int c = kg * 128 + 32 * i + 8 * t;
+        const uint4 sraw = *reinterpret_cast<const uint4*>(suh + (long long)s * k + c);
+        sw[4 * i] = sraw.x;
+        sw[4 * i + 1] = sraw.y;
+        sw[4 * i + 2] = sraw.z;
+        sw[4 * i + 3] = sraw.w;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const __half2 h = __floats2half2_rn(v[8 * i + 2 * j] * HAD_SCALE, v[8 * i + 2 * j + 1] * HAD_SCALE);
-            o[j] = *reinterpret_cast<const uint32_t*>(&h);
+        for (int r = 0; r < 2; r++) {
+            // rows of x are x_cols (a multiple of 8) long, zeros from there to k
+            const int row = row0 + 8 * r;
+            const uint4 raw = row < rows && c < x_cols ? *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + (long long)row * x_cols + c)
+                                                       : make_uint4(0u, 0u, 0u, 0u);
+            xw[r][4 * i] = raw.x;
+            xw[r][4 * i + 1] = raw.y;
+            xw[r][4 * i + 2] = raw.z;
+            xw[r][4 * i + 3] = raw.w;
         }
-        *reinterpret_cast<uint4*>(xa + s * shard_stride + tc_a_offset(row, col + 8 * i, kgs * 2)) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    if (x_bf16) {
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const __nv_bfloat162 bb = *reinterpret_cast<const __nv_bfloat162*>(&xw[r][i]);
+                const __half2 h = __floats2half2_rn(__low2float(bb), __high2float(bb));
+                xw[r][i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+    }
+    Had128Rows had;
+    had.run<true, true>(xw[0], xw[1], sw, lane);
+    __half* out = xa + s * shard_stride;
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int row = row0 + 8 * r;
+        if ((row & ~7) >= rows) break;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                float a, b;
+                had.pair(r, i, j, a, b);
+                const __half2 h = __floats2half2_rn(a * HAD_SCALE, b * HAD_SCALE);
+                o[j] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            *reinterpret_cast<uint4*>(out + tc_a_offset(row, kg * 128 + 32 * i + 8 * t, kgs * 2)) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
     }
 }
 
@@ -919,7 +930,7 @@ int launch_gemm_tc(const void* x, int x_bf16, int x_cols, const __half* suh_cat,
     // Rows beyond `rows` inside the last super tile hold whatever was there: a product row depends on its own row of A only, and
     // theirs are never stored (zeroing them was a pass over the whole buffer, 4 us at 74 rows of 2 x 7168).
     const long long items = (long long)n_shards * ((rows + HAD_IN_TC_ROWS - 1) / HAD_IN_TC_ROWS) * (k / 128);
-    if (int rc = launch_chained(had_in_tc_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, st, x, x_bf16, x_cols, suh_cat, n_shards, rows, k, xa,
+    if (int rc = launch_chained(had_in_tc_kernel, dim3((unsigned)((items + HAD_IN_TC_WARPS - 1) / HAD_IN_TC_WARPS)), dim3(HAD_IN_TC_WARPS * 32), 0, st, x, x_bf16, x_cols, suh_cat, n_shards, rows, k, xa,
                                 l.xa_shard_stride))
         return rc;
     // Wide tiles (256 x 256) need column blocks that pair up inside every shard.  They halve the rows that share a decoded
