@@ -398,58 +398,13 @@ __device__ __forceinline__ void fwht128_quad(float (&v)[32], int lane)
     for (int i = 0; i < 16; i++) f32x2_split(p[i], v[2 * i], v[2 * i + 1]);
 }
 
-// The transform over four lanes with half the shuffles: in a cross-lane stage the two lanes of a pair exchange HALF of their values each,
-// so that every lane holds both operands of its butterflies, 32 shuffles for eight rows.  The exchange turns the layout: a row comes in
-// as 16-byte chunks dealt to the lanes in turn (v[8 i + e] of lane q is element 32 i + 8 q + e: loads of 64 consecutive bytes) and goes
-// out with 32 consecutive elements per lane (v[i] is element 32 q + i), or the other way round -- the same code.  The stages run in a
-// different order from fwht128's, with the same rounding of every sum.  Shuffles and loads share a pipe (207 of its cycles per eight rows
-// and 128 columns with fwht128_quad and 64-byte lanes, 83 % busy) that bounds the rotations of routed experts.
-__device__ __forceinline__ void fwht128_turn(float (&v)[32], int lane)
-{
-    unsigned long long p[16];
-    const unsigned long long minus = f32x2(-1.f, -1.f);
-#pragma unroll
-    for (int i = 0; i < 16; i++) p[i] = f32x2(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
-#pragma unroll
-    for (int stride = 1; stride < 16; stride <<= 1) {
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            if ((i & stride) == 0) {
-                const unsigned long long lo = p[i], hi = p[i + stride];
-                p[i] = f32x2_add(lo, hi);
-                p[i + stride] = f32x2_fma(hi, minus, lo);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-        const bool upper = (lane & m) != 0;
-        const float sign = upper ? -1.f : 1.f;
-        const unsigned long long sign2 = f32x2(sign, sign), other2 = f32x2(-sign, -sign);
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            if ((i & (4 * m)) == 0) {
-                const unsigned long long send = upper ? p[i] : p[i + 4 * m], keep = upper ? p[i + 4 * m] : p[i];
-                float a, b;
-                f32x2_split(send, a, b);
-                const unsigned long long got = f32x2(__shfl_xor_sync(0xFFFFFFFFu, a, m), __shfl_xor_sync(0xFFFFFFFFu, b, m));
-                unsigned long long t;
-                asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(keep), "l"(sign2));
-                p[i] = f32x2_add(keep, got);
-                p[i + 4 * m] = f32x2_fma(got, other2, t);
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 16; i++) f32x2_split(p[i], v[2 * i], v[2 * i + 1]);
-}
-
 // The transform of 16 rows on tensor cores, inputs in fp16: rows g and g + 8 of lane 4 g + t, its elements the 16-byte chunks t, t + 4, t + 8, t + 12 of
 // a row (a[.][4 j + w]: elements 2 w, 2 w + 1 of chunk 4 j + t) -- what 16-byte loads of 64 consecutive bytes give.  Four of the seven index bits
 // (0, 1, and the lane's 3, 4) are the k of m16n8k16 MMAs, whose right operand is the signs of a 16-point transform, or (SIGNED) these
 // times a sign vector: products of two fp16 numbers, exact, so the vector costs nothing.  The other three bits are butterflies between a lane's own
 // registers: no shuffles, half the additions, and results in the layout that the inputs had: p[2 j + b][h][row] is elements 4 b + 2 h, 4 b + 2 h + 1
-// of chunk 4 j + t.  Unnormalised, sums in fp32; 21 million warp instructions where fwht128_turn takes 36 (moe_had_in_kernel, 16384 rows of 2048).
+// of chunk 4 j + t.  Unnormalised, sums in fp32; 21 million warp instructions where the same transform by
+// butterflies over four lanes per row takes 36 (moe_had_in_kernel, 16384 rows of 2048).
 struct Had128Rows {
     unsigned long long p[8][2][2];                           // [group][h][row]: packed pairs
 

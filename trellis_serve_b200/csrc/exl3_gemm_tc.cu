@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(TcPair::THREADS, 1) gemm_tc_pair_kernel(const 
 
 // Rotated activations in the A-operand layout of gemm_tc_kernel.  One warp per (shard, 16 rows, 128-block), the transform on tensor cores
 // (Had128Rows): a lane's results are whole 16-byte core-matrix rows, and the eight lanes with the same chunk fill a 128-byte core matrix.
-// Rows beyond `rows` inside the last group of eight are written as zeros.  With fwht128_turn on eight rows per warp before / now, the whole call in
+// Rows beyond `rows` inside the last group of eight are written as zeros.  With butterflies over four lanes per row, eight rows per warp, before / now, the whole call in
 // bursts, us: 2048 rows, 5120 x 2 x 17408, K = 4 643.7 / 639.2, 5120 x (5120 + 2 x 1024), bf16 202.6 / 193.4, 1024 rows, 17408 x 5120 269.0 / 265.5,
 // 100 rows, 5120 x 7168 32.8 / 31.2, 70 rows, 2048 x 1024 14.0 / 13.7.  The output rotation in the epilogue of the CTA-pair kernel stays as it is: with
 // the same transform it takes tensor-pipe time from the tcgen05 MMAs and registers that spill (631 -> 646 us).

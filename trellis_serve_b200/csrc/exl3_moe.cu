@@ -355,8 +355,8 @@ __device__ __forceinline__ void moe_unrotate32(const Had128Rows& had, int r, con
 // (MoeStage).  A warp takes a block of eight rows (the way in: two neighbouring blocks; behind the GEMMs two column blocks, or gate and up, are
 // the 16 rows) and a span of up to four column blocks, so that the chain of dependent loads (block -> expert and slot -> values) is walked once
 // per span.  The span is halved while the warps are not enough for two full loads of the chip (span_of).  Bound by latency and issue together:
-// 2048 tokens, 256 experts of 2048 x 512, top-8, the three kernels, thousands of cycles and millions of warp instructions, before (fwht128_turn,
-// eight rows per warp, 24 warps per SM, plain loads) / with MMAs alone / one column block ahead: way in 98, 36 / 75, 21 / 71, 22; middle 61, 19 / 56, 14 /
+// 2048 tokens, 256 experts of 2048 x 512, top-8, the three kernels, thousands of cycles and millions of warp instructions, before (butterflies
+// over four lanes per row, eight rows per warp, 24 warps per SM, plain loads) / with MMAs alone / one column block ahead: way in 98, 36 / 75, 21 / 71, 22; middle 61, 19 / 56, 14 /
 // 48, 14; out and sum 60, 24 / 54, 17 / 49, 18.  The layer: 347 us -> 348 -> 321, 700 tokens, 64 experts of 1536 x 768, top-6 131 -> 124, 2048 tokens,
 // 32 experts of 1024 x 384, top-2 67 -> 63.5.  Rows through L1 lose it again (338 us), and so does one row that all lanes without a slot ask for (700
 // tokens: 137).  Padding rows are left as they are: a column of the product depends on its own row only and nothing looks at theirs.

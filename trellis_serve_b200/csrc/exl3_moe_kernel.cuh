@@ -116,6 +116,15 @@ __device__ __forceinline__ void moe_finish_eight(const MoeGemmLaunch& p, const f
     }
 }
 
+// Sixteen tensor-memory lanes x sixteen columns: r[4 s .. 4 s + 3] are columns 8 s + 2 (lane % 4) and the next, of tensor-memory lane (lane / 4) and that + 8.
+__device__ __forceinline__ void moe_load_turned(uint32_t taddr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
 // LIST: items of several blocks from the align kernel's list; otherwise every block of eight rows is an item, and row count and pitch are
 // constants of the code.
 template <int K, int MODE, int FAM, bool LIST>
@@ -531,15 +540,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 slots[0] = p.sorted_ids[it.y + ew];
                 slots[1] = p.sorted_ids[it.y + ew + 4];
             }
-            // LIST: rows of a column block of an item are consecutive, [item][column block][row][128]; this lane's column.
-            __half* dst = p.out + (long long)it.y * p.n_total + (long long)nb * it.z * 128 + ew * 32 + lane;
-            auto store8 = [&](int r0, const float (&v)[8]) {
-#pragma unroll
-                for (int e = 0; e < 8; e++) dst[r0 * 128 + e * 128] = __float2half_rn(v[e]);
-            };
             // Tensor memory -> shared memory or the CTA's slab: lane = output column.
             const int hb = done, he = done + count;
-            auto load_rows = [&](int c, float (&v)[8]) {
+            [[maybe_unused]] auto load_rows = [&](int c, float (&v)[8]) {
                 uint32_t r[ACCS][8];
 #pragma unroll
                 for (int g = 0; g < ACCS; g++) sk_load8(((uint32_t)(ew * 32) << 16) + (uint32_t)((d * ACCS + g) * NMAX + c), r[g]);
@@ -549,7 +552,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
 #pragma unroll
                     for (int e = 0; e < 8; e++) asm volatile("" : "+r"(r[g][e]));       // no use of the registers moves ahead of the wait
 #pragma unroll
-                for (int e = 0; e < 8; e++) v[e] = LIST ? __uint_as_float(r[0][e]) : 0.f;
+                for (int e = 0; e < 8; e++) v[e] = 0.f;
                 if constexpr (!LIST) {
 #pragma unroll
                     for (int g = 0; g < ACCS; g++)
@@ -558,7 +561,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                             for (int e = 0; e < 8; e++) v[e] += __uint_as_float(r[g][e]);
                 }
             };
-            auto read_rows = [&](int rows, float* to) {
+            [[maybe_unused]] auto read_rows = [&](int rows, float* to) {
 #pragma unroll 1
                 for (int c = 0; c < rows; c += 8) {
                     float v[8];
@@ -595,11 +598,46 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                 moe_finish_eight(p, P, 0, -1, sv, slots, nb, ew, lane);
                 ptx::named_bar_sync(SK_BAR_EPI, 128);
             } else {
+                // Rows of a column block of an item are consecutive, [item][column block][row][128].  A warp has 32 columns of them, which come
+                // out of tensor memory as pieces of rows' pairs: turned in shared memory by transposing stores of 8x8 matrices (64 bytes per
+                // row, its 16-byte chunks xor-ed with the row pair: no bank conflicts) they leave as 16-byte stores.  With a column per lane and
+                // two bytes per store this was 6 of 68 instructions per tile of 512 x 2048.
+                const uint32_t turn = ptx::smem_addr(smem + p.p_off + ew * 1024);
+                const uint32_t put = turn + (lane & 7) * 64u + (((lane >> 3) ^ (lane >> 1)) & 3) * 16u;        // row, matrix
+                const uint32_t get = turn + (lane >> 2) * 64u + (((lane & 3) ^ (lane >> 3)) & 3) * 16u;        // row, chunk
+                const uint32_t from = ((uint32_t)(ew * 32) << 16) + (uint32_t)(d * NMAX);
+                __half* dst = p.out + (long long)it.y * p.n_total + (long long)nb * it.z * 128 + (lane >> 2) * 128 + ew * 32 + (lane & 3) * 8;
 #pragma unroll 1
-                for (int r0 = 0; r0 < it.z; r0 += 8) {
-                    float v[8];
-                    load_rows(r0, v);
-                    store8(r0, v);
+                for (int r0 = 0; r0 < it.z; r0 += 16) {
+                    uint32_t a[2][8];                                       // columns 0 - 15 and 16 - 31 of the warp's, rows r0 .. r0 + 15
+#pragma unroll
+                    for (int i = 0; i < 2; i++) moe_load_turned(from + ((uint32_t)(16 * i) << 16) + r0, a[i]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+#pragma unroll
+                        for (int e = 0; e < 8; e++) asm volatile("" : "+r"(a[i][e]));       // no use of the registers moves ahead of the wait
+#pragma unroll
+                    for (int s = 0; s < 2; s++) {
+                        uint32_t m[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const __half2 h = __floats2half2_rn(__uint_as_float(a[j >> 1][4 * s + 2 * (j & 1)]), __uint_as_float(a[j >> 1][4 * s + 2 * (j & 1) + 1]));
+                            m[j] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(put + s * 512u), "r"(m[0]), "r"(m[1]),
+                                     "r"(m[2]), "r"(m[3])
+                                     : "memory");
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int s = 0; s < 2; s++)
+                        if (r0 + 8 * s < it.z) {
+                            uint4 v;
+                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(get + s * 512u));
+                            *reinterpret_cast<uint4*>(dst + (r0 + 8 * s) * 128) = v;
+                        }
+                    __syncwarp();
                 }
                 release();
             }

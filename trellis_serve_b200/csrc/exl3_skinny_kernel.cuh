@@ -510,8 +510,9 @@ static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint
 // RP: operand pitch, the rows rounded up (operand_pitch).
 // WHOLE: a group takes whole units, not every third half unit: one walk through the stages, one loop test and addresses that are constants for eight
 // tiles instead of four (49.7 -> 46.7 instructions per tile at K = 3, the loop 14.9 -> 13.8 clk).  Chained launches over distinct weights, K = 3, one
-// row, us: 5120 x 34816 42.7 -> 41.7, 17408 x 5120 24.7 -> 24.2, 2048 x 25088 17.3 -> 17.0, 4096 x 4096 8.8 -> 8.6; K = 4, 5, 8 17408 x 5120 23.4 ->
-// 22.6, 25.8 -> 24.9, 25.2 -> 24.7; 16 rows 30.6 -> 30.1.  What it costs: at the end of a column block a group may be a unit behind the others
+// row, us: 5120 x 34816 42.7 -> 41.7, 17408 x 5120 24.7 -> 24.2, 2048 x 25088 17.3 -> 17.0, 4096 x 4096 8.8 -> 8.6; 17408 x 5120 at K = 2, 4, 5, 6, 7, 8
+// 24.5 -> 23.9, 23.6 -> 23.2, 26.0 -> 25.7, 25.9 -> 25.3, 26.7 -> 26.4, 25.4 -> 25.1, MUL1 26.4 -> 25.5; 16 rows 30.6 -> 30.1, MUL1 at K = 6 33.0 ->
+// 32.0.  What it costs: at the end of a column block a group may be a unit behind the others
 // instead of half of one, which shows where a CTA has few units in two blocks (5120 x 7168, 15 units: one row 13.65 -> 13.75, but five rows 17.7 ->
 // 18.4, as its sums of the first block then hold up the second: hence not for three to eight rows).  Above 16 rows a stage of three units takes too
 // much shared memory.
