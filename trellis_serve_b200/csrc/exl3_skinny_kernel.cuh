@@ -24,17 +24,17 @@
 //     normalising it on the way -- so the linear is ONE launch.  Weights are constants: copies start, and the first half units of
 //     every group are decoded, before the kernel ahead in the stream has finished.
 //
-// Bound by the issue of the decode and by the register ports that its pipes share: 44 to 52 instructions per 16x16 tile, whatever K (49.7 at K =
-// 3, 44.5 at K = 4, 51.8 at K = 6, 46.5 at K = 8, 61.2 for MUL1 at K = 6), are 11 to 13 clk of a SM's four schedulers.  The loop takes 15.1 /
-// 13.3 / 15.7 / 14.0 clk per tile and SM at K = 3 / 4 / 6 / 8 (stamps in chained launches at 1.965 GHz; 14.6 / 15.4 / 15.8 at K = 2 / 5 / 7),
-// 16.0 and 16.2 for MUL1 at K = 3 and 6; issue slots are used in 70 to 75 % of a launch's active cycles, the ALU pipe in 62 to 65 %.  The
-// MMAs take 4 clk per tile of the tensor pipe at N = 16 and 8 at N = 64 and run beside it: 15.1 to 15.4 clk (K = 3) up to 16 rows, 16.4 at 32,
-// 21.9 at 33 to 64, where half units are handed over in two pieces.  Chained launches over distinct weights, K = 3, one row, us: 5120 x 34816
-// 43.2, 17408 x 5120 24.8, 5120 x 5120 11.3, 4096 x 4096 (K = 4) 8.7; 17408 x 5120, K = 6, MUL1, 16 rows 33.2.  What is not the loop, per
-// launch at one row: 1.8 to 4 us from the end of the launch ahead until the input is rotated, 1.8 to 2.4 us by which CTAs that could not
-// become resident early finish later than the median, 3.1 to 4.3 us from there to the stored outputs (tensor memory -> partial sums ->
-// counter -> sums).  Fewer instructions in the loop's bookkeeping (one counter for stage and range) changed nothing at K = 3 and lost 2 %
-// at K = 4 to 8; a copy of the loop per group lost 7 % to instruction fetch.
+// Bound by the issue of the decode and by the register ports that its pipes share: 42 to 52 instructions per 16x16 tile, whatever K (46.7 at K =
+// 3, 41.7 at K = 4), are 11 to 13 clk of a SM's four schedulers; three to four more where groups take half units (49.7, 44.5).  The loop takes
+// 13.8 clk per tile and SM at K = 3 (stamps in chained launches at 1.965 GHz); with half units 14.9, and 13.3 / 15.7 / 14.0 at K = 4 / 6 / 8, 16.0 and
+// 16.2 for MUL1 at K = 3 and 6; 12.6 is what it takes alone, over weights that stay in shared memory and without the input rotation.  Issue
+// slots are used in 64 to 72 % of a launch's active cycles.  The MMAs take 4 clk per tile of the tensor pipe at N = 16 and 8 at N = 64 and run
+// beside it: 16.4 clk (K = 3) at 32 rows, 21.9 at 33 to 64, where half units are handed over in two pieces.  Chained launches over distinct
+// weights, K = 3, one row, us: 5120 x 34816 41.7, 17408 x 5120 24.2, 5120 x 5120 11.0, 4096 x 4096 (K = 4) 8.5; 17408 x 5120, K = 6, MUL1, 16 rows
+// 32.0.  What is not the loop, per launch at one row: 1.6 to 3.7 us from the end of the launch ahead until the input is rotated, 2.1 to 2.4 us by
+// which CTAs that could not become resident early finish later than the median, 2.9 to 4.2 us from there to the stored outputs (tensor memory
+// -> partial sums -> counter -> sums).  Fewer instructions in the loop's bookkeeping (one counter for stage and range, half units) changed
+// nothing at K = 3 and lost 2 % at K = 4 to 8; a copy of the loop per group lost 7 % to instruction fetch.
 #pragma once
 #include "exl3_gemv_common.cuh"
 
