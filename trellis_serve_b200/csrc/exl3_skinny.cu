@@ -80,7 +80,10 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     size_t ups = (24 * 1024 + w - 1) / w;
     if (x != SK_STREAM && ups < 6) ups = 6;
     if (ups > most) ups = most;
-    const size_t least = a.rows <= SK_FUSED_ROWS || (a.rows > SK_ROTATE_ROWS && a.rows <= 16) ? SK_GROUPS : 2;      // see SkWalk
+    // Three units per stage where groups take whole units (see SkWalk).  Ranges so long that two such stages do not fit beside the resident rows
+    // are rotated by a launch of their own, which is the faster way anyway: 5120 x 34816, K = 8, two rows (74 units per CTA) 47.6 us, inside with
+    // two stages of three units, for which it takes a KB less of everything else, 48.6, with two stages of two units 55.5.
+    const size_t least = a.rows <= SK_FUSED_ROWS || (a.rows > SK_ROTATE_ROWS && a.rows <= 16) ? SK_GROUPS : 2;
     if (ups < least) ups = least;
     if (ups > most) ups = most;
     while (ups > least && budget / (ups * unit) < 3) ups--;
