@@ -423,9 +423,10 @@ struct Had128Rows {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 float c[4];
-                asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                    : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-                    : "r"(a0[w]), "r"(TWO ? a1[w] : 0u), "r"(a0[w + 1]), "r"(TWO ? a1[w + 1] : 0u), "r"(b0), "r"(h ? b1 ^ 0x80008000u : b1), "f"(0.f));
+                // volatile: of the whole warp, it must not sink into a branch that only lanes with a result take
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                             : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                             : "r"(a0[w]), "r"(TWO ? a1[w] : 0u), "r"(a0[w + 1]), "r"(TWO ? a1[w + 1] : 0u), "r"(b0), "r"(h ? b1 ^ 0x80008000u : b1), "f"(0.f));
                 p[i][h][0] = f32x2(c[0], c[1]);
                 p[i][h][1] = f32x2(c[2], c[3]);
             }
