@@ -155,8 +155,11 @@ static __device__ __noinline__ void gemv_exchange_store(const TpExchange& tp, ui
 
 // Residual epilogue of one row's block of 128 outputs (one warp, four columns per lane): y -- summed over the ranks first, if
 // there is an exchange -- rounded as it would be stored, plus the residual stream: the new stream goes to res_out, this block's
-// share of its mean square to ssq_out, y itself to `out` only if that is set.  Out of line: once per 128 outputs.
-static __device__ __noinline__ void gemv_residual_store(const GemvArgs& a, uint32_t tp_epoch, float4 vv, long long o, int m, int fnb,
+// share of its mean square to ssq_out, y itself to `out` only if that is set.  Inlined into the one place that uses it: called, it made its caller
+// keep nine registers in memory (36 bytes stored, 96 to 100 loaded), all at the end of a launch, where the last CTA's epilogue is what the
+// kernel behind waits for.  Without them, chained launches, one row, us: 5120 x 5120 streamed, K = 3 12.4 -> 10.85, K = 6 13.3 -> 11.9; 17408 x 5120 from
+// gate | up, K = 8, two rows 29.6 -> 27.9; a step of four layers of hidden 5120 437.5 -> 423.
+__device__ __forceinline__ void gemv_residual_store(const GemvArgs& a, uint32_t tp_epoch, float4 vv, long long o, int m, int fnb,
                                                         int lane)
 {
     const float v[4] = {vv.x, vv.y, vv.z, vv.w};
