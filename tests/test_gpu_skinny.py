@@ -3,6 +3,8 @@ one unit, ranges that wrap the ring several times), with and without the rotatio
 weights."""
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 
@@ -112,3 +114,38 @@ def test_even_ranges_where_the_rows_of_whole_column_blocks_do_not_fit(rows, k, n
     """Sizes for which whole column blocks cost less but the busiest CTA's rotated and raw rows (1792 bytes a unit for two rows split, 6400 for
     eight) leave no room for a ring of stages in 227 KB, while those of even ranges do."""
     test_column_blocks_and_parts_of_them(rows, k, n, K, cb)
+
+
+def _launches(call):
+    """Kernels that `call` launches: the nodes of its captured graph."""
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    count = ctypes.c_size_t(0)
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(count)) == 0
+    return count.value
+
+
+@pytest.mark.parametrize("rows,k,n,K,cb,launches", [
+    (1, 5120, 34816, 8, 0, 1),      # 74 units per CTA: a ring of two stages of three units, 96 KB
+    (2, 5120, 34816, 8, 2, 1),      # the same beside two rows of paired weights
+    (1, 5120, 34816, 7, 0, 2),      # two of three would hold 84 KB
+    (2, 5120, 34816, 6, 0, 2),      # ... 72 KB
+    (2, 5120, 34816, 8, 0, 2),      # two do not fit
+    (1, 8576, 36864, 3, 0, 2),      # neither do they in even ranges of 131 units
+    (2, 6272, 36352, 3, 0, 1),      # 98 units in whole column blocks do not fit, 95 in even ranges do: three stages of three
+    (1, 5504, 36224, 8, 0, 1),      # 86 and 83: two of three
+    (2, 4736, 35968, 8, 0, 1),      # 74 and 71: two of three
+])
+def test_rings_of_long_ranges(rows, k, n, K, cb, launches):
+    """One or two rows over ranges that leave room for few stages: the smallest rings, many laps of them, even ranges where whole column blocks
+    do not fit, and the lines beyond which a launch of its own rotates the rows."""
+    test_column_blocks_and_parts_of_them(rows, k, n, K, cb)
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(1)
+    packed, suh, svh = random_packed(k, n, K, gen, DEV), random_signs(k, gen, DEV, 1), random_signs(n, gen, DEV).view(-1)
+    x, y = torch.randn((rows, k), device=DEV, generator=gen).half(), torch.empty((rows, n), dtype=torch.float16, device=DEV)
+    ws = torch.zeros(lin.workspace_bytes(rows, k, n, 1), dtype=torch.uint8, device=DEV)
+    assert _launches(lambda: lin.run(x, packed, suh, svh, [], cb, out=y, workspace=ws)) == launches

@@ -67,10 +67,10 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     l.deal = sk_deal(l.NB, l.KG, ctas, a.rows, x == SK_ROTATE && a.rows > SK_FUSED_ROWS, INT_MAX, aligned, l.most);
     const size_t most = (size_t)l.most;
     // Stages of whole units, as long as three fit; a short range travels as one copy.  A bulk copy costs a few hundred nanoseconds whatever
-    // its size (24 KB of weights or more), and a group of decode warps changes stages every 2 units / 3 steps: six units where the
-    // rows are resident (17408 x 5120, one row, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1, K
-    // = 8 25.4 -> 24.7), no more than 24 KB where they travel with the weights and the first stage is waited for (5120 x 5120, 16 rows: 18.5
-    // us against 19.1 with six units).
+    // its size (24 KB of weights or more), and a group of decode warps changes stages every ups / 3 units (2 ups / 3 half units): six units where
+    // the rows are resident (17408 x 5120, one row, with half units, against stages of 24 KB: K = 3 25.2 -> 24.6 us, K = 4 23.6 -> 22.9, K = 6 27.1 -> 26.1,
+    // K = 8 25.4 -> 24.7), no more than 24 KB, or three units, where they travel with the weights and the first stage is waited for (5120 x 5120, 16 rows,
+    // with half units: 18.5 us against 19.1 with six units).
     const size_t w = 2048u * (size_t)a.K, f = (size_t)operand_pitch(a.rows) * (a.mode == GEMV_SPLIT ? 512 : 256);
     const SkRaw raw = sk_raw_planes(x, a.x_glu);
     const size_t planes = x == SK_STREAM ? 0 : (size_t)(raw.planes_const + a.rows * raw.planes_row);
@@ -80,9 +80,7 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     size_t ups = (24 * 1024 + w - 1) / w;
     if (x != SK_STREAM && ups < 6) ups = 6;
     if (ups > most) ups = most;
-    // Three units per stage where groups take whole units (see SkWalk).  Ranges so long that two such stages do not fit beside the resident rows
-    // are rotated by a launch of their own, which is the faster way anyway: 5120 x 34816, K = 8, two rows (74 units per CTA) 47.6 us, inside with
-    // two stages of three units, for which it takes a KB less of everything else, 48.6, with two stages of two units 55.5.
+    // Three units per stage where groups take whole units (see SkWalk).
     const size_t least = a.rows <= SK_FUSED_ROWS || (a.rows > SK_ROTATE_ROWS && a.rows <= 16) ? SK_GROUPS : 2;
     if (ups < least) ups = least;
     if (ups > most) ups = most;
@@ -90,6 +88,15 @@ static int plan_split(const GemvArgs& a, const DeviceInfo* d, int x, bool aligne
     size_t stages = budget / (ups * unit);
     if (stages > SK_MAX_STAGES) stages = SK_MAX_STAGES;
     const size_t fills = (most + ups - 1) / ups;
+    // One or two rows over a range so long that three stages do not fit beside them: two, if they hold 96 KB or more; with less the weights do not
+    // keep up and a rotation launch of its own is the faster way.  5120 x 34816 (74 units per CTA), us, two stages of three units / rotation launch /
+    // half units in as many stages of two units as fit: K = 5, two rows normalised 51.6 / 49.9 / 52.0; K = 6, one row normalised 52.8 / 50.8 / 50.1,
+    // two rows 51.1 / 48.0 / 50.8, normalised 55.4 / 51.6 / 52.5; K = 7, one row 51.9 / 47.7 / 48.2, normalised 53.5 / 51.0 / 51.4, two rows 53.5 / 47.8 /
+    // 51.5; two stages do not fit for two normalised rows at K = 7, 51.4 with the launch, 62.6 with half units, and at K = 8 (47.6 / 57.5 for one, 48.2 / 60.1).
+    // A step of four such layers, one row: K = 6 484 / 465 / 472, K = 7 490 / 471 / 478.  With 96 KB (K = 8, one row) the launch takes as long
+    // alone and more in a stack of four layers: 380 / 387.5 / 379; K = 7, one row there 418 / 414 / 407.  Two stages of four units (K = 7 50.0, 411 in the
+    // stack; 17408 x 5120 from gate | up, K = 8, two rows 29.0 against 27.6 with three) are no better.
+    if (x != SK_STREAM && a.rows <= SK_FUSED_ROWS && stages < 3 && stages < fills && stages * ups * w < 96 * 1024) return EXL3_ERR_UNSUPPORTED_ROWS;
     if (stages < 2 && stages < fills) return EXL3_ERR_UNSUPPORTED_ROWS;
     // From three rows up the rotation inside saves a launch (3 us) as long as it is one pass of the decode warps and leaves the ring
     // its three stages: 5120 x 5120, 4 rows: 13.3 against 15.9 us; 17408 x 5120, 4 rows: 34.1 against 29.1 us.
