@@ -184,3 +184,18 @@ def test_rotations_of_pairs_of_row_blocks(hidden, inter, dtype):
         _check(out, ref)
     else:
         assert orc.rel_norm(got, ref) <= 3e-3 + 2.0 ** -9
+
+
+@pytest.mark.parametrize("K,cb", [(6, 0), (7, 1), (8, 2), (8, 0)])
+def test_long_items_at_high_bit_rates(K, cb):
+    """Three stages of three units leave the activations of 128 rows three slots of shared memory at 6 and 7 bits and two at 8: items of all 128 rows,
+    of few and of 64, six units deep, so that both rings are lapped many times (the bars of this file)."""
+    hidden, inter, E = 768, 640, 5
+    gate, up, down = _experts(7 * K + cb, E, hidden, inter, K, out_scale=1 / 8)
+    pack = moe.prepare_mixed(_to_dev(gate), _to_dev(up), _to_dev(down), cb)
+    rng = np.random.default_rng(K)
+    ids = rng.permutation(np.repeat(np.arange(E), [300, 128, 64, 3, 17])).astype(np.int32)[:, None]
+    assert moe.moe_block_size(len(ids), 1, E) == 128
+    w = rng.uniform(0.5, 1.0, ids.shape).astype(np.float32)
+    x = rng.standard_normal((len(ids), hidden)).astype(np.float16)
+    _check(_run_layer(pack, x, w, ids), orc.np_moe_layer(x, ids, w, gate, up, down, K, cb))

@@ -851,7 +851,10 @@ int launch_moe_gemm(MoeGemmLaunch l, int K, int codebook, int mode, cudaStream_t
     // Stages of about 24 KB of weights (a bulk copy costs a few hundred nanoseconds whatever its size), a unit or more per group of decode
     // warps (see SkWalk).  Single blocks of eight rows: their activations ride with the weights, as many stages as fit; four units per stage where
     // three such stages fit, as the decode groups change stages less often (64 tokens, 256 experts: K = 4 172 -> 169 us, K = 5 191 -> 187).
-    // Long items: three stages of weights, the rest for activations (three units of 128 rows and more; larger stages take from those).
+    // Long items: three stages of weights, the rest for activations (larger stages take from those): of 128 rows four units and more up to K = 5, three at 6
+    // and 7, two at 8.  Two stages of three units would leave them four and three there and lose all the same: 2048 tokens, 256 experts of 2048 x
+    // 512, top-8, K = 6 / 7 / 8 392 / 408 / 396 us against 372 / 376 / 371; 700 tokens, 64 experts of 1536 x 768, top-6, K = 6 / 8 143.5 / 136.4 against 131 / 123
+    // (half units, three stages of two: 402 / 431 / 411, 140 / 138).
     const uint32_t unit = 2048u * (uint32_t)K, row = mode == GEMV_SPLIT ? 512u : 256u, tail = MOE_BLOCK_ROWS * 128 * 4, all = (uint32_t)d->max_smem_optin;
     uint32_t ups = (24u * 1024u + unit - 1) / unit;
     if (ups < SK_GROUPS) ups = SK_GROUPS;
