@@ -578,7 +578,9 @@ __global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_out_kernel(const __
 // beyond 65504 are infinite in it as well, as with explicit casts around an fp16 layer): moe_out_kernel and
 // moe_combine_kernel in one, without the slots' rows in memory between.  A warp takes 8 / G tokens, G rows each (top_k rounded up to a power
 // of two, at most eight; more come in rounds), four lanes per row; the rows of a token are added by exchanging halves, so that every lane ends
-// with 32 / G of the 128 columns, its own.  Traffic bounds it (2048 tokens, top-8, 2048 columns: 67 MB, 10.4 us).
+// with 32 / G of the 128 columns, its own.  Latency and
+// issue bound it (2048 tokens, top-8, 2048 columns: 31 us under ncu for 67 MB, which are 10.4 us of traffic).  One and two rows per token spill (352 and 28
+// bytes stored); top-1 gained all the same (2048 tokens, 32 experts of 2048 x 512: a layer 81 -> 74 us with the transforms on tensor cores, top-2 109 -> 99).
 template <int G>
 __global__ void __launch_bounds__(MOE_HAD_WARPS * 32, 4) moe_out_combine_kernel(const __half* __restrict__ yd_rot, const __half* __restrict__ svh2,
                                                                  const float* __restrict__ weights, const int* __restrict__ place,
@@ -771,8 +773,8 @@ int launch_moe_align(const int* topk_ids, int numel, int E, int block, int cap, 
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Column blocks per warp for `groups` groups of eight rows, and the CTAs of eight warps that this takes: up to four, as long as the warps fill the
-// chip (16 per SM) twice.
+// Column blocks per warp for `groups` groups of eight rows, and (span_blocks) the CTAs that this takes: up to four, as long as the warps
+// fill the chip (16 per SM) twice.
 static int span_of(long long groups, int cols, int least = 1)
 {
     const DeviceInfo* d = current_device_info();

@@ -20,10 +20,10 @@
 //     behind rotate them.
 //
 // Bound by the issue of the decode (see exl3_skinny_kernel.cuh); the MMAs of a 16x16 tile take 8 clk at 128 paired rows.  Groups take whole units
-// (three half units apart before): 256 experts of 2048 x 512, top-8, K = 3, 64 tokens 178.5 -> 175.2 us, 2048 tokens 366 -> 359.  Long items: 16.9 clk
-// per tile for gate|up, most of it on the scheduler that the MMA warp is on (62 instructions per tile there, 55 on the others): the loop that
-// issues them frees a buffer after its own half's MMAs (not both after the unit's: 355 -> 350 us), knows its loop bounds as uniform (349), and
-// is one piece of code for all groups (347).
+// (three half units apart before): 256 experts of 2048 x 512, top-8, K = 3, 64 tokens 178.5 -> 175.2 us, 2048 tokens 366 -> 359.  Long items: 16.6 clk
+// per tile for gate|up (16.9 before their rows left through shared memory), most of it on the scheduler that the MMA warp is on (62 instructions per tile there,
+// 55 on the others): the loop that issues them frees a buffer after its own half's MMAs (not both after the unit's: 355 -> 350 us), knows
+// its loop bounds as uniform (349), and is one piece of code for all groups (347).
 #pragma once
 #include "exl3_skinny_kernel.cuh"
 
@@ -553,13 +553,11 @@ __global__ void __launch_bounds__(SK_THREADS, 1) moe_gemm_kernel(const __grid_co
                     for (int e = 0; e < 8; e++) asm volatile("" : "+r"(r[g][e]));       // no use of the registers moves ahead of the wait
 #pragma unroll
                 for (int e = 0; e < 8; e++) v[e] = 0.f;
-                if constexpr (!LIST) {
 #pragma unroll
-                    for (int g = 0; g < ACCS; g++)
-                        if (hb + (g + 3 - hb % 3) % 3 < he)                 // else the group had no unit of this block
+                for (int g = 0; g < ACCS; g++)
+                    if (hb + (g + 3 - hb % 3) % 3 < he)                     // else the group had no unit of this block
 #pragma unroll
-                            for (int e = 0; e < 8; e++) v[e] += __uint_as_float(r[g][e]);
-                }
+                        for (int e = 0; e < 8; e++) v[e] += __uint_as_float(r[g][e]);
             };
             [[maybe_unused]] auto read_rows = [&](int rows, float* to) {
 #pragma unroll 1

@@ -405,8 +405,9 @@ __device__ __forceinline__ void sk_rotate_rows(const SkinnyLaunch& p, const unsi
     const int rows = p.a.rows;
     const bool bf16 = p.a.x_bf16 != 0;
     constexpr int RP = SK_ROTATE_ROWS;
-    // Eight rows side by side in a quarter warp: its loads (planes are 16 bytes apart in the banks) and stores are conflict-free.  With
-    // the four lanes of a row side by side the stores of a unit were 128 cycles of shared memory instead of 32.
+    // Eight rows side by side in a quarter warp: its loads (planes are 16 bytes apart in the banks) are conflict-free, and so are its stores of split
+    // activations; paired ones are stored eight bytes at a time, two quarter warps to the same banks.  With the four lanes of a row side by side
+    // the split stores of a unit were 128 cycles of shared memory instead of 32 (5120 x 7168, five rows, K = 3 17.9 -> 17.5 us; MUL1, K = 6 18.1 -> 17.8).
     const int q = lane >> 3, row = lane & 7;
 #pragma unroll 1
     for (int i = warp; i < units; i += SK_DECODE_WARPS) {
@@ -514,7 +515,8 @@ static __device__ __noinline__ void sk_finish_block_call(const GemvArgs& a, uint
 // 24.5 -> 23.9, 23.6 -> 23.2, 26.0 -> 25.7, 25.9 -> 25.3, 26.7 -> 26.4, 25.4 -> 25.1, MUL1 26.4 -> 25.5; 16 rows 30.6 -> 30.1, MUL1 at K = 6 33.0 ->
 // 32.0.  What it costs: at the end of a column block a group may be a unit behind the others
 // instead of half of one, which shows where a CTA has few units in two blocks (5120 x 7168, 15 units: one row 13.65 -> 13.75, but five rows 17.7 ->
-// 18.4, as its sums of the first block then hold up the second: hence not for three to eight rows).  Above 16 rows a stage of three units takes too
+// 18.4, as its sums of the first block then hold up the second).  Hence not for three to eight rows, most of whose launches, those that rotate inside, have such
+// ranges; longer ones of that many rows, whose activations are streamed, were not tried.  Above 16 rows a stage of three units takes too
 // much shared memory.
 // SLOTS: the matrix is that of SkSlots, one row per slot, rotated inside.  SK_EACH: every slot as it stands; one whose id is out of range decodes
 // expert 0 and drops the result.  SK_HELD, for ids with a map (a rank's share of the experts, bitrate classes): every CTA makes the same list of
