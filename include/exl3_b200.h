@@ -139,7 +139,8 @@ exl3_status exl3_linear_prerotated(const uint32_t *packed, int K, int codebook, 
 
 /* A down projection fed straight from the gate | up output: y = linear(fp16(silu(gate) * up)) with gate_up [rows, 2k] in
  * x_dtype, suh [k], n_shards = 1.  Up to two rows the activation is computed inside the GEMV's own input rotation (one launch,
- * no activation buffer); above that the library runs the activation kernel ahead of it.  Same bits as exl3_silu_mul_rotate
+ * no activation buffer) unless a CTA's range leaves too little shared memory beside the rows; above that, and then, the library runs the
+ * activation kernel ahead of it.  Same bits as exl3_silu_mul_rotate
  * followed by exl3_linear_prerotated.  The exchange arguments are those of exl3_linear_prerotated (world <= 1: none).
  * The reference's engine runs its activation kernel between the two launches; no counterpart there.
  *
@@ -149,7 +150,7 @@ exl3_status exl3_linear_prerotated(const uint32_t *packed, int K, int codebook, 
  * (a second buffer) and the sum of its squares per (row, 128 columns) to ssq_out [rows, n_total / 128]; y may then be NULL
  * (no exchange, up to two rows).  exl3_normed_linear is the consumer: the fused group on rmsnorm(z) * norm_weight, where z is
  * such a stream and ssq its sums of squares; up to two rows the GEMV normalises on the way into its own rotation, so a
- * transformer block is four launches plus attention.  exl3_residual_ssq starts a chain (z = x + residual_in, or x itself, and
+ * transformer block is four launches plus attention (one more for a range that leaves too little shared memory beside the rows).  exl3_residual_ssq starts a chain (z = x + residual_in, or x itself, and
  * its sums of squares), exl3_normed ends one (out = rmsnorm(z) * weight from z and its sums of squares, in fp32, one rounding); exl3_rmsnorm_linear = exl3_residual_ssq + exl3_normed_linear for a caller without a producer.
  * From three rows up the library runs its normalisation / stream kernels around a plain GEMV (y must then be given).
  * The reference's engine runs residual add and RMSNorm as kernels of its own ahead of had_in; no counterpart there. */

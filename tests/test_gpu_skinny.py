@@ -149,3 +149,29 @@ def test_rings_of_long_ranges(rows, k, n, K, cb, launches):
     x, y = torch.randn((rows, k), device=DEV, generator=gen).half(), torch.empty((rows, n), dtype=torch.float16, device=DEV)
     ws = torch.zeros(lin.workspace_bytes(rows, k, n, 1), dtype=torch.uint8, device=DEV)
     assert _launches(lambda: lin.run(x, packed, suh, svh, [], cb, out=y, workspace=ws)) == launches
+
+
+@pytest.mark.parametrize("rows,K,cb,launches", [(1, 3, 0, 1), (2, 5, 0, 2), (1, 6, 0, 2), (2, 7, 2, 2), (1, 8, 2, 1), (2, 8, 0, 2)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_rings_of_long_ranges_normalised(rows, K, cb, launches, dtype):
+    """The normalising form beside 74 units per CTA, on either side of the line, against the normalisation on its own and a plain linear: they
+    differ by the last bit of the normalisation factor, which flips the rounding of an activation here and there (the bar of the decode step's
+    tests for the same pair)."""
+    k, n = 5120, 34816
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(rows + K)
+    packed, suh, svh = random_packed(k, n, K, gen, DEV), random_signs(k, gen, DEV, 2), (random_signs(n, gen, DEV).view(-1) / 64).half()
+    z = torch.randn((rows, k), device=DEV, generator=gen).to(dtype)
+    weight = (1.0 + 0.1 * torch.randn(k, device=DEV, generator=gen)).to(dtype)
+    ssq = z.float().view(rows, k // 128, 128).pow(2).sum(-1).contiguous()
+    got, act = torch.empty((rows, n), dtype=torch.float32, device=DEV), torch.empty_like(z)
+    ws = torch.zeros(lin.workspace_bytes(rows, k, n, 2), dtype=torch.uint8, device=DEV)
+    assert _launches(lambda: lin.run_normed(z, ssq, weight, 1e-6, packed, suh, svh, [n // 2], cb, got, ws)) == launches
+    got.zero_()
+    lin.run_normed(z, ssq, weight, 1e-6, packed, suh, svh, [n // 2], cb, got, ws)
+    lin.normed(z, ssq, weight, 1e-6, act)
+    want = lin.run(act, packed, suh, svh, [n // 2], cb, out=torch.empty_like(got))
+    torch.cuda.synchronize()
+    lin.device_error(DEV)
+    scale = float(want.pow(2).mean().sqrt())
+    assert float((got - want).abs().max()) <= 2e-3 * scale * (1 if dtype == torch.float16 else 8)      # bf16 activations: eight times the step

@@ -362,7 +362,8 @@ def normed(z: torch.Tensor, ssq: torch.Tensor, weight: torch.Tensor, eps: float,
 def run_normed(z: torch.Tensor, ssq: torch.Tensor, weight: torch.Tensor, eps: float, b: torch.Tensor, suh_cat: torch.Tensor,
                svh_cat: torch.Tensor, shard_ends: list[int], codebook: int, out: torch.Tensor, workspace: torch.Tensor | None = None) -> torch.Tensor:
     """The fused group on rmsnorm(z) * weight, z a residual stream and ssq its sums of squares per 128 columns (from a linear's
-    residual epilogue or `residual_ssq`): up to two rows the GEMV normalises on the way into its own rotation (one launch)."""
+    residual epilogue or `residual_ssq`): up to two rows the GEMV normalises on the way into its own rotation (one launch;
+    two for ranges that leave too little shared memory beside the rows)."""
     _require_cuda(z, "z")
     lib = _lib.load()
     _lib.init_device(b.device.index if b.device.index is not None else torch.cuda.current_device())
@@ -379,7 +380,8 @@ def run_normed(z: torch.Tensor, ssq: torch.Tensor, weight: torch.Tensor, eps: fl
 def run_glu(gate_up: torch.Tensor, b: torch.Tensor, suh: torch.Tensor, svh_cat: torch.Tensor, codebook: int, out: torch.Tensor | None,
             workspace: torch.Tensor | None = None, exchange=None, residual=None) -> torch.Tensor | None:
     """Down projection of silu(gate) * up straight from `gate_up` [rows, 2k]: up to two rows the activation is computed inside
-    the GEMV's own input rotation (one launch, no activation buffer).  `exchange` and `residual` as in `run_prerotated`."""
+    the GEMV's own input rotation (one launch, no activation buffer; two launches for ranges that leave too little shared memory beside
+    the rows).  `exchange` and `residual` as in `run_prerotated`."""
     _require_cuda(gate_up, "gate_up")
     lib = _lib.load()
     _lib.init_device(b.device.index if b.device.index is not None else torch.cuda.current_device())

@@ -97,8 +97,8 @@ class DecodeLayerSet:
         self.y_gu = torch.empty((rows, 2 * f), dtype=dtype, device=self.device)
         self.y_down = torch.empty((rows, h), dtype=dtype, device=self.device)
         self.graph: torch.cuda.CUDAGraph | None = None
-        # up to two rows the GEMV rotates its own input: one launch per group; otherwise rotation + GEMV (from three to eight rows an
-        # upper bound: groups whose ranges are one pass of a CTA's decode warps still rotate inside)
+        # up to two rows the GEMV rotates its own input: one launch per group (a lower bound: wide groups of 6 to 8 bits can take two); otherwise
+        # rotation + GEMV (from three to eight rows an upper bound: groups whose ranges are one pass of a CTA's decode warps still rotate inside)
         self.launches_per_step = layers * 4 * (1 if rows <= 2 else 2)
         if tp_size > 1 and allreduce is not None and not self.fused_exchange:
             self.launches_per_step += layers * 2             # the stand-alone exchange kernel after o and down
